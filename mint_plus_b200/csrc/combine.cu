@@ -1,239 +1,729 @@
-// Combine from materialised logits: select by chain mask -> row softmax -> split -> two weighted sums, and its
-// backward.  HBM-bound on the two (B,H,T,T) logit tensors; one warp per query row, fixed summation order.
+// Combine from materialised logits: select by chain mask -> row softmax -> split -> two weighted sums, and its backward.
+//
+// Bound by HBM on the (B,H,T,T) logits, their gradients and the mask; the sums over keys, queries and head dimensions run on
+// the warp-level matrix instruction (16x8x16, bf16 operands, fp32 accumulators), because as scalar loops they and not the
+// memory set the pace (B2 H20 T360 D32 bf16, 47 MB, forward + backward: 996 us with one dot product per lane and key, 75 us so;
+// what remains is the latency of mask -> logits -> products in warps that live for three chunks).
+// Operands keep their precision: a value is split into bf16 pieces (v = v0 + v1 + ...; one piece for a bf16 tensor, three for an
+// fp32 one, two / three for the fp32 probabilities) and the products of pieces that matter in fp32 are added, smallest first.
+//
+// A CTA of four warps owns 16 query rows (or one block of keys) and its warps take turns on the chunks of the other axis, each
+// with a private online-softmax state, merged in a fixed order at the end: with T / 16 * B * H CTAs even one short pair fills
+// the chip, and no warp waits for another inside its loop.  All results are bit-reproducible.
+#include <initializer_list>
+
 #include "common.cuh"
 
 namespace mintb {
+namespace {
 
-template <typename T>
-__device__ __forceinline__ float sel_logit(const T* il, const T* el, const uint8_t* m, int j) {
-  return m[j] ? ld_f(el + j) : ld_f(il + j);
+constexpr int kWarps = 4;
+
+template <typename T> struct Num;
+template <> struct Num<__nv_bfloat16> { static constexpr int kV = 1, kP = 2, kKeys = 32; };   // pieces of a tensor / of a probability
+template <> struct Num<float> { static constexpr int kV = 3, kP = 3, kKeys = 32; };
+
+__device__ __forceinline__ uint32_t pack2(float lo, float hi) {
+  uint32_t r;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+  return r;
 }
-
-__device__ __forceinline__ float warp_max(float v) {
+// The first N bf16 pieces of the pair (a, b), most significant first.
+template <int N>
+__device__ __forceinline__ void split2(float a, float b, uint32_t (&out)[N]) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
-}
-__device__ __forceinline__ float warp_sum(float v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
-// Row statistics shared by forward and backward: m = max_j logit, l = sum_j exp(logit - m).
-template <typename T>
-__device__ __forceinline__ void row_stats(const T* il, const T* el, const uint8_t* m, int Tn, int lane, float& mx,
-                                          float& l) {
-  mx = -INFINITY;
-  for (int j = lane; j < Tn; j += 32) mx = fmaxf(mx, sel_logit(il, el, m, j));
-  mx = warp_max(mx);
-  l = 0.f;
-  for (int j = lane; j < Tn; j += 32) l += expf(sel_logit(il, el, m, j) - mx);
-  l = warp_sum(l);
-}
-
-template <typename T, int D>
-__global__ void __launch_bounds__(128) combine_fwd_kernel(const T* __restrict__ il, const T* __restrict__ el,
-                                                           const uint8_t* __restrict__ mask,
-                                                           const T* __restrict__ iv, const T* __restrict__ ev,
-                                                           T* __restrict__ out, int B, int H, int Tn) {
-  constexpr int NV = (D + 31) / 32;
-  const size_t row = size_t(blockIdx.x) * 4 + threadIdx.x / 32;
-  const int lane = threadIdx.x % 32;
-  if (row >= size_t(B) * H * Tn) return;
-  const int i = int(row % Tn);
-  const size_t bh = row / Tn;
-  const int b = int(bh / H);
-  const T* ilr = il + row * Tn;
-  const T* elr = el + row * Tn;
-  const uint8_t* mr = mask + (size_t(b) * Tn + i) * Tn;
-  const T* ivh = iv + bh * Tn * D;
-  const T* evh = ev + bh * Tn * D;
-  float mx, l;
-  row_stats(ilr, elr, mr, Tn, lane, mx, l);
-  const float inv = 1.f / l;
-  float acc[NV];
-#pragma unroll
-  for (int k = 0; k < NV; ++k) acc[k] = 0.f;
-  for (int j0 = 0; j0 < Tn; j0 += 32) {
-    const int j = j0 + lane;
-    float pj = 0.f;
-    bool x = false;
-    if (j < Tn) {
-      x = mr[j] != 0;
-      pj = expf((x ? ld_f(elr + j) : ld_f(ilr + j)) - mx) * inv;
+  for (int k = 0; k < N; ++k) {
+    out[k] = pack2(a, b);
+    if (k + 1 < N) {
+      a -= __uint_as_float(out[k] << 16);
+      b -= __uint_as_float(out[k] & 0xffff0000u);
     }
-    const unsigned xs = __ballot_sync(0xffffffffu, x);
-    const int n = min(32, Tn - j0);
-    for (int jj = 0; jj < n; ++jj) {
-      const float pb = __shfl_sync(0xffffffffu, pj, jj);
-      const T* v = ((xs >> jj) & 1u) ? evh + size_t(j0 + jj) * D : ivh + size_t(j0 + jj) * D;
+  }
+}
+__device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], const __nv_bfloat16* p) {
+  const uint32_t a = uint32_t(__cvta_generic_to_shared(p));
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
+}
+__device__ __forceinline__ void ldsm4t(uint32_t (&r)[4], const __nv_bfloat16* p) {
+  const uint32_t a = uint32_t(__cvta_generic_to_shared(p));
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
+}
+
+// Rows [r0, r0 + ROWS) of src[n][D] (zeros from row n on) as bf16 pieces in shared memory, dst[piece][ROWS][D + 8]; one warp.
+// The 16-byte pad makes the eight rows of an ldmatrix start in different banks.  stage() only starts the copies of a bf16 tensor
+// (asynchronous, so that they share one trip to memory with the loads issued after them); staged() waits for them.
+template <typename T, int D, int ROWS>
+__device__ __forceinline__ void stage(const T* __restrict__ src, int r0, int n, __nv_bfloat16* __restrict__ dst, int lane) {
+  constexpr int LD = D + 8, NV = Num<T>::kV;
+  if (reinterpret_cast<uintptr_t>(src) % 16 != 0) {   // a contiguous view that starts off a 16-byte boundary
+    for (int i = lane; i < ROWS * D / 2; i += 32) {
+      const int r = i / (D / 2), d = i % (D / 2) * 2;
+      const T* p = src + size_t(r0 + r) * D + d;
+      uint32_t w[NV];
+      split2<NV>(r0 + r < n ? ld_f(p) : 0.f, r0 + r < n ? ld_f(p + 1) : 0.f, w);
 #pragma unroll
-      for (int k = 0; k < NV; ++k) {
-        const int d = lane + 32 * k;
-        if (d < D) acc[k] = fmaf(pb, ld_f(v + d), acc[k]);
+      for (int k = 0; k < NV; ++k) *reinterpret_cast<uint32_t*>(dst + (k * ROWS + r) * LD + d) = w[k];
+    }
+  } else if constexpr (NV == 1) {
+#pragma unroll
+    for (int i0 = 0; i0 < ROWS * D / 8; i0 += 32) {
+      const int i = i0 + lane, r = i / (D / 8), d = i % (D / 8) * 8, row = r0 + r < n ? r0 + r : n - 1;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(uint32_t(__cvta_generic_to_shared(dst + r * LD + d))), "l"(src + size_t(row) * D + d),
+                   "r"(r0 + r < n ? 16 : 0) : "memory");   // a source size of 0 fills with zeros
+    }
+  } else {
+    constexpr int N = ROWS * D / 4 / 32, NB = N < 8 ? N : 8;   // 16-byte loads per lane, in batches of at most eight
+#pragma unroll
+    for (int b0 = 0; b0 < N; b0 += NB) {
+      float4 v[NB];
+#pragma unroll
+      for (int k = 0; k < NB; ++k) {
+        const int i = (b0 + k) * 32 + lane, r = i / (D / 4), d = i % (D / 4) * 4, row = r0 + r < n ? r0 + r : n - 1;
+        v[k] = *reinterpret_cast<const float4*>(src + size_t(row) * D + d);
+      }
+#pragma unroll
+      for (int k = 0; k < NB; ++k) {
+        const int i = (b0 + k) * 32 + lane, r = i / (D / 4), d = i % (D / 4) * 4;
+        if (r0 + r >= n) v[k] = make_float4(0, 0, 0, 0);
+        uint32_t p0[NV], p1[NV];
+        split2<NV>(v[k].x, v[k].y, p0); split2<NV>(v[k].z, v[k].w, p1);
+#pragma unroll
+        for (int q = 0; q < NV; ++q) *reinterpret_cast<uint2*>(dst + (q * ROWS + r) * LD + d) = make_uint2(p0[q], p1[q]);
       }
     }
   }
-#pragma unroll
-  for (int k = 0; k < NV; ++k) {
-    const int d = lane + 32 * k;
-    if (d < D) st_f(out + row * D + d, acc[k]);
-  }
+}
+__device__ __forceinline__ void staged() {
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncwarp();
 }
 
-// Backward kernel 1, one warp per query row: stats -> dP_ij = dO_i . V_sel(j) -> delta = sum_j p dP -> dS = p (dP - delta),
-// written to the selected pathway's logit gradient (zero in the other).  Stores (m, 1/l) for kernel 2.
-template <typename T, int D>
-__global__ void __launch_bounds__(128) combine_bwd_rows_kernel(const T* __restrict__ il, const T* __restrict__ el,
-                                                                const uint8_t* __restrict__ mask,
-                                                                const T* __restrict__ iv, const T* __restrict__ ev,
-                                                                const T* __restrict__ dO, T* __restrict__ d_il,
-                                                                T* __restrict__ d_el, float* __restrict__ stats, int B,
-                                                                int H, int Tn) {
-  const size_t row = size_t(blockIdx.x) * 4 + threadIdx.x / 32;
-  const int lane = threadIdx.x % 32;
-  if (row >= size_t(B) * H * Tn) return;
-  const int i = int(row % Tn);
-  const size_t bh = row / Tn;
-  const int b = int(bh / H);
-  const T* ilr = il + row * Tn;
-  const T* elr = el + row * Tn;
-  const uint8_t* mr = mask + (size_t(b) * Tn + i) * Tn;
-  const T* ivh = iv + bh * Tn * D;
-  const T* evh = ev + bh * Tn * D;
-  float go[D];
-#pragma unroll
-  for (int d = 0; d < D; ++d) go[d] = ld_f(dO + row * D + d);
-  float mx, l;
-  row_stats(ilr, elr, mr, Tn, lane, mx, l);
-  const float inv = 1.f / l;
-  if (lane == 0) {
-    stats[row * 2] = mx;
-    stats[row * 2 + 1] = inv;
-  }
-  float delta = 0.f;
-  for (int j = lane; j < Tn; j += 32) {
-    const bool x = mr[j] != 0;
-    const T* v = x ? evh + size_t(j) * D : ivh + size_t(j) * D;
-    float dp = 0.f;
-#pragma unroll
-    for (int d = 0; d < D; ++d) dp = fmaf(go[d], ld_f(v + d), dp);
-    delta = fmaf(expf((x ? ld_f(elr + j) : ld_f(ilr + j)) - mx) * inv, dp, delta);
-  }
-  delta = warp_sum(delta);
-  for (int j = lane; j < Tn; j += 32) {
-    const bool x = mr[j] != 0;
-    const T* v = x ? evh + size_t(j) * D : ivh + size_t(j) * D;
-    float dp = 0.f;
-#pragma unroll
-    for (int d = 0; d < D; ++d) dp = fmaf(go[d], ld_f(v + d), dp);
-    const float pj = expf((x ? ld_f(elr + j) : ld_f(ilr + j)) - mx) * inv;
-    const float ds = pj * (dp - delta);
-    st_f(d_il + row * Tn + j, x ? 0.f : ds);
-    st_f(d_el + row * Tn + j, x ? ds : 0.f);
+// Elements j and k of a row; PAIR: neighbours in one aligned access (even T and aligned tensors).
+template <bool PAIR>
+__device__ __forceinline__ float2 ld_pair(const __nv_bfloat16* p, int j, int k) {
+  if constexpr (PAIR) {
+    const uint32_t u = *reinterpret_cast<const uint32_t*>(p + j);
+    return make_float2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u));
+  } else {
+    return make_float2(ld_f(p + j), ld_f(p + k));
   }
 }
+template <bool PAIR>
+__device__ __forceinline__ float2 ld_pair(const float* p, int j, int k) {
+  if constexpr (PAIR) return *reinterpret_cast<const float2*>(p + j);
+  else return make_float2(p[j], p[k]);
+}
+template <bool PAIR>
+__device__ __forceinline__ void st_pair(__nv_bfloat16* p, float a, float b, bool second) {
+  if constexpr (PAIR) *reinterpret_cast<uint32_t*>(p) = pack2(a, b);
+  else { st_f(p, a); if (second) st_f(p + 1, b); }
+}
+template <bool PAIR>
+__device__ __forceinline__ void st_pair(float* p, float a, float b, bool second) {
+  if constexpr (PAIR) *reinterpret_cast<float2*>(p) = make_float2(a, b);
+  else { p[0] = a; if (second) p[1] = b; }
+}
 
-// Backward kernel 2: dV_intra[j] = sum_i (p o ~M)_ij dO_i, dV_inter[j] = sum_i (p o M)_ij dO_i.
-// Block = 32 keys x 4 slices of D; walks the query rows in order (deterministic).
-template <typename T, int D>
-__global__ void __launch_bounds__(128) combine_bwd_values_kernel(const T* __restrict__ il, const T* __restrict__ el,
-                                                                  const uint8_t* __restrict__ mask,
-                                                                  const T* __restrict__ dO,
-                                                                  const float* __restrict__ stats,
-                                                                  T* __restrict__ d_iv, T* __restrict__ d_ev, int B,
-                                                                  int H, int Tn) {
-  constexpr int DS = D / 4;
-  const int jj = threadIdx.x % 32, q = threadIdx.x / 32;
-  const int j = blockIdx.x * 32 + jj;
-  const size_t bh = blockIdx.y;
-  const int b = int(bh / H);
-  float ai[DS], ae[DS];
+// One warp's 16 x KC block of the logits, in the accumulator layout of the matrix instruction: lane (g, t) holds rows g and g + 8,
+// columns 8 nt + 2 t and the next.
+template <typename T, int KC, bool PAIR>
+struct Block {
+  bool any_i, any_x;   // (of the whole warp) some element takes the intra / the cross pathway
+  bool edge;           // the block sticks out of the matrix
+  uint32_t cross;      // bit 4 nt + 2 h + e: row g + 8 h, column e of tile nt is of the cross pathway; set only where both occur
+  uint32_t inside;     // the elements inside the matrix; set only at the edge
+
+  // Addresses outside are clamped, so that no load waits behind a branch.
+  template <bool EDGE>
+  __device__ __forceinline__ void mask_words(const uint8_t* __restrict__ mask, int i0, int j0, int n, int lane, uint32_t (&w)[KC / 8]) {
+    const int g = lane / 4, t = lane % 4;
+    const uint8_t* r0 = mask + size_t(EDGE ? min(i0 + g, n - 1) : i0 + g) * n;
+    const uint8_t* r1 = mask + size_t(EDGE ? min(i0 + g + 8, n - 1) : i0 + g + 8) * n;
+    uint32_t lo[KC / 8], hi[KC / 8];
 #pragma unroll
-  for (int d = 0; d < DS; ++d) ai[d] = ae[d] = 0.f;
-  if (j < Tn) {
-    for (int i = 0; i < Tn; ++i) {
-      const size_t row = bh * Tn + i;
-      const bool x = mask[(size_t(b) * Tn + i) * Tn + j] != 0;
-      const float lg = x ? ld_f(el + row * Tn + j) : ld_f(il + row * Tn + j);
-      const float pj = expf(lg - stats[row * 2]) * stats[row * 2 + 1];
-      const T* g = dO + row * D + q * DS;
-      if (x) {
-#pragma unroll
-        for (int d = 0; d < DS; ++d) ae[d] = fmaf(pj, ld_f(g + d), ae[d]);
+    for (int nt = 0; nt < KC / 8; ++nt) {
+      const int j = j0 + 8 * nt + 2 * t;
+      if constexpr (PAIR) {
+        const int c = EDGE ? min(j, n - 2) : j;
+        lo[nt] = *reinterpret_cast<const uint16_t*>(r0 + c);
+        hi[nt] = *reinterpret_cast<const uint16_t*>(r1 + c);
       } else {
-#pragma unroll
-        for (int d = 0; d < DS; ++d) ai[d] = fmaf(pj, ld_f(g + d), ai[d]);
+        const int c = EDGE ? min(j, n - 1) : j, d = EDGE ? min(j + 1, n - 1) : j + 1;
+        lo[nt] = r0[c] | uint32_t(r0[d]) << 8;
+        hi[nt] = r1[c] | uint32_t(r1[d]) << 8;
       }
     }
-    const size_t off = (bh * Tn + j) * D + q * DS;
 #pragma unroll
-    for (int d = 0; d < DS; ++d) {
-      st_f(d_iv + off + d, ai[d]);
-      st_f(d_ev + off + d, ae[d]);
+    for (int nt = 0; nt < KC / 8; ++nt) w[nt] = lo[nt] | hi[nt] << 16;
+  }
+
+  __device__ __forceinline__ void load_mask(const uint8_t* __restrict__ mask, int i0, int j0, int n, int lane) {
+    const int g = lane / 4, t = lane % 4;
+    uint32_t w[KC / 8];
+    edge = i0 + 16 > n || j0 + KC > n;
+    if (edge) mask_words<true>(mask, i0, j0, n, lane, w);
+    else mask_words<false>(mask, i0, j0, n, lane, w);
+    uint32_t some = 0, zero = 0;
+#pragma unroll
+    for (int nt = 0; nt < KC / 8; ++nt) {
+      some |= w[nt];
+      zero |= (w[nt] - 0x01010101u) & ~w[nt] & 0x80808080u;   // not 0 iff a byte is 0
+    }
+    any_x = __any_sync(0xffffffffu, some != 0);
+    any_i = __any_sync(0xffffffffu, zero != 0);
+    cross = inside = 0;
+    if (any_i && any_x) {
+#pragma unroll
+      for (int nt = 0; nt < KC / 8; ++nt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) cross |= ((w[nt] >> (8 * e)) & 0xffu ? 1u : 0u) << (4 * nt + e);
+    }
+    if (edge) {
+#pragma unroll
+      for (int nt = 0; nt < KC / 8; ++nt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          inside |= (i0 + g + 8 * (e / 2) < n && j0 + 8 * nt + 2 * t + (e & 1) < n ? 1u : 0u) << (4 * nt + e);
+    }
+  }
+
+  template <bool EDGE>
+  __device__ __forceinline__ void read(const T* __restrict__ p, int i0, int j0, int n, int lane, float (&s)[KC / 8][4]) {
+    const int g = lane / 4, t = lane % 4;
+    const T* r[2] = {p + size_t(EDGE ? min(i0 + g, n - 1) : i0 + g) * n, p + size_t(EDGE ? min(i0 + g + 8, n - 1) : i0 + g + 8) * n};
+#pragma unroll
+    for (int nt = 0; nt < KC / 8; ++nt)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int j = j0 + 8 * nt + 2 * t;
+        const float2 v = ld_pair<PAIR>(r[h], EDGE ? min(j, PAIR ? n - 2 : n - 1) : j, EDGE ? min(j + 1, n - 1) : j + 1);
+        s[nt][2 * h] = v.x;
+        s[nt][2 * h + 1] = v.y;
+      }
+  }
+
+  // The selected logits (-inf outside).  A tensor that no element of the block selects is not read.
+  __device__ __forceinline__ void load_logits(const T* __restrict__ il, const T* __restrict__ el, int i0, int j0, int n, int lane, float (&s)[KC / 8][4]) {
+    if (edge) read<true>(any_x ? el : il, i0, j0, n, lane, s);
+    else read<false>(any_x ? el : il, i0, j0, n, lane, s);
+    if (any_i && any_x) {
+      float v[KC / 8][4];
+      read<true>(il, i0, j0, n, lane, v);
+#pragma unroll
+      for (int nt = 0; nt < KC / 8; ++nt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (!((cross >> (4 * nt + e)) & 1u)) s[nt][e] = v[nt][e];
+    }
+    if (edge) {
+#pragma unroll
+      for (int nt = 0; nt < KC / 8; ++nt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (!((inside >> (4 * nt + e)) & 1u)) s[nt][e] = -INFINITY;
+    }
+  }
+};
+
+// s with the elements of the other pathway set to zero.
+template <int N>
+__device__ __forceinline__ void keep(float (&out)[N][4], const float (&s)[N][4], uint32_t sel) {
+#pragma unroll
+  for (int nt = 0; nt < N; ++nt)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) out[nt][e] = (sel >> (4 * nt + e)) & 1u ? s[nt][e] : 0.f;
+}
+
+// exp(s - ref), for which bf16 logits take the hardware's exp2 as it is (2 ulp of fp32).
+template <typename T>
+__device__ __forceinline__ float exp_from(float s, float ref) {
+  if constexpr (Num<T>::kV == 1) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"((s - ref) * kLog2e));
+    return y;
+  } else {
+    return expf(s - ref);
+  }
+}
+
+// c += a b summed over the pieces whose product reaches fp32, smallest first.  B fragments of piece `q` come from frag(q).
+template <int NA, int NB, typename F>
+__device__ __forceinline__ void mma_pieces(float (&c)[4], const uint32_t (&a)[NA][4], F frag) {
+  constexpr int NM = NA > NB ? NA : NB;
+#pragma unroll
+  for (int sum = NM - 1; sum >= 0; --sum)
+#pragma unroll
+    for (int q = 0; q < NB; ++q) {
+      const int p = sum - q;
+      if (p >= 0 && p < NA) {
+        const uint2 b = frag(q);
+        mma16816(c, a[p], b.x, b.y);
+      }
+    }
+}
+
+// dp[nt] = (dO V^T) of 16 rows against KC staged keys; `go` holds dO's A fragments [D / 16][piece].
+template <typename T, int D, int KC>
+__device__ __forceinline__ void grad_dot(float (&dp)[KC / 8][4], const uint32_t (&go)[D / 16][Num<T>::kV][4], const __nv_bfloat16* sv, int lane) {
+  constexpr int NV = Num<T>::kV, LD = D + 8;
+#pragma unroll
+  for (int nt = 0; nt < KC / 8; nt += 2) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) dp[nt][e] = dp[nt + 1][e] = 0.f;
+#pragma unroll
+    for (int k = 0; k < D / 16; ++k) {
+      uint32_t f[NV][4];   // two key tiles of eight, both halves of the 16 dimensions
+#pragma unroll
+      for (int q = 0; q < NV; ++q)
+        ldsm4(f[q], sv + (q * KC + 8 * nt + (lane & 7) + ((lane >> 4) << 3)) * LD + 16 * k + ((lane >> 3) & 1) * 8);
+      mma_pieces<NV, NV>(dp[nt], go[k], [&](int q) { return make_uint2(f[q][0], f[q][1]); });
+      mma_pieces<NV, NV>(dp[nt + 1], go[k], [&](int q) { return make_uint2(f[q][2], f[q][3]); });
     }
   }
 }
 
+__device__ __forceinline__ float quad_max(float v) {
+  v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 1));
+  return fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 2));
+}
+__device__ __forceinline__ float quad_sum(float v) {
+  v += __shfl_xor_sync(0xffffffffu, v, 1);
+  return v + __shfl_xor_sync(0xffffffffu, v, 2);
+}
+// The reference point of exp: 0 while nothing finite has been seen, so that exp(-inf - 0) = 0 and a row without any finite logit
+// ends as 0 / 0 = NaN, as the softmax of an all -inf row does in PyTorch.
+__device__ __forceinline__ float finite_or_zero(float m) { return m == -INFINITY ? 0.f : m; }
+
+// ------------------------------------------------------------------------------------------------ forward
 template <typename T, int D>
-static cudaError_t fwd_t(const void* il, const void* el, const uint8_t* mask, const void* iv, const void* ev, void* out,
-                         int B, int H, int Tn, cudaStream_t s) {
-  size_t rows = size_t(B) * H * Tn;
-  combine_fwd_kernel<T, D><<<unsigned((rows + 3) / 4), 128, 0, s>>>(
-      static_cast<const T*>(il), static_cast<const T*>(el), mask, static_cast<const T*>(iv), static_cast<const T*>(ev),
-      static_cast<T*>(out), B, H, Tn);
+constexpr int fwd_smem_bytes() {
+  constexpr int v = kWarps * Num<T>::kV * Num<T>::kKeys * (D + 8) * 2, m = kWarps * 16 * (D + 2) * 4;
+  return v > m ? v : m;   // the merge reuses the value tiles
+}
+
+template <typename T, int D, bool PAIR>
+__global__ void __launch_bounds__(32 * kWarps, 4) combine_fwd_kernel(const T* __restrict__ il, const T* __restrict__ el, const uint8_t* __restrict__ mask,
+                                                                  const T* __restrict__ iv, const T* __restrict__ ev, T* __restrict__ out, int H, int n) {
+  constexpr int KC = Num<T>::kKeys, NV = Num<T>::kV, NP = Num<T>::kP, LD = D + 8;
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, g = lane / 4, t = lane % 4;
+  const size_t bh = blockIdx.y;
+  const int i0 = blockIdx.x * 16;
+  il += bh * n * n; el += bh * n * n; mask += size_t(bh / H) * n * n;
+  iv += bh * n * D; ev += bh * n * D;
+  __nv_bfloat16* sv = reinterpret_cast<__nv_bfloat16*>(smem) + warp * NV * KC * LD;
+
+  float acc[D / 8][4], m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
+#pragma unroll
+  for (int d = 0; d < D / 8; ++d)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[d][e] = 0.f;
+
+  for (int j0 = warp * KC; j0 < n; j0 += kWarps * KC) {
+    float s[KC / 8][4];
+    Block<T, KC, PAIR> blk;
+    blk.load_mask(mask, i0, j0, n, lane);
+    __syncwarp();
+    stage<T, D, KC>(blk.any_x ? ev : iv, j0, n, sv, lane);
+    blk.load_logits(il, el, i0, j0, n, lane, s);
+    float alpha[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float mx = m[h];
+#pragma unroll
+      for (int nt = 0; nt < KC / 8; ++nt) mx = fmaxf(mx, fmaxf(s[nt][2 * h], s[nt][2 * h + 1]));
+      mx = quad_max(mx);
+      const float ref = finite_or_zero(mx);
+      alpha[h] = expf(m[h] - ref);
+      m[h] = mx;
+      l[h] *= alpha[h];
+#pragma unroll
+      for (int nt = 0; nt < KC / 8; ++nt)
+#pragma unroll
+        for (int e = 2 * h; e < 2 * h + 2; ++e) {
+          s[nt][e] = exp_from<T>(s[nt][e], ref);
+          l[h] += s[nt][e];
+        }
+    }
+#pragma unroll
+    for (int d = 0; d < D / 8; ++d)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[d][e] *= alpha[e / 2];
+#pragma unroll
+    for (int path = 1; path >= 0; --path) {
+      if (!(path ? blk.any_x : blk.any_i)) continue;   // no element of the block takes this pathway's values
+      if (path == 0 && blk.any_x) {
+        __syncwarp();
+        stage<T, D, KC>(iv, j0, n, sv, lane);
+      }
+      staged();
+      float q[KC / 8][4];
+      if (blk.any_i && blk.any_x) keep(q, s, path ? blk.cross : ~blk.cross);
+      else keep(q, s, 0xffffffffu);
+      float part[D / 8][4];   // summed apart from the running total, so that its roundings stay those of a short sum
+#pragma unroll
+      for (int d = 0; d < D / 8; ++d)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) part[d][e] = 0.f;
+#pragma unroll
+      for (int kc = 0; kc < KC / 16; ++kc) {
+        uint32_t a[NP][4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {   // A fragment register r: rows g + 8 (r & 1), keys 2 t + 8 (r >> 1)
+          const int nt = 2 * kc + (r >> 1), e = 2 * (r & 1);
+          uint32_t w[NP];
+          split2<NP>(q[nt][e], q[nt][e + 1], w);
+#pragma unroll
+          for (int k = 0; k < NP; ++k) a[k][r] = w[k];
+        }
+#pragma unroll
+        for (int d = 0; d < D / 8; d += 2) {
+          uint32_t f[NV][4];
+#pragma unroll
+          for (int q = 0; q < NV; ++q)
+            ldsm4t(f[q], sv + (q * KC + 16 * kc + (lane & 15)) * LD + 8 * d + (lane >> 4) * 8);
+          mma_pieces<NP, NV>(part[d], a, [&](int q) { return make_uint2(f[q][0], f[q][1]); });
+          mma_pieces<NP, NV>(part[d + 1], a, [&](int q) { return make_uint2(f[q][2], f[q][3]); });
+        }
+      }
+#pragma unroll
+      for (int d = 0; d < D / 8; ++d)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[d][e] += part[d][e];
+    }
+  }
+  // merge the four warps' states: [warp][16][D] accumulators, then maxima and row sums
+  l[0] = quad_sum(l[0]);
+  l[1] = quad_sum(l[1]);
+  __syncthreads();
+  float* sa = reinterpret_cast<float*>(smem);
+  float* sm = sa + kWarps * 16 * D;
+  float* sl = sm + kWarps * 16;
+#pragma unroll
+  for (int d = 0; d < D / 8; ++d)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) sa[(warp * 16 + g + 8 * (e / 2)) * D + 8 * d + 2 * t + (e & 1)] = acc[d][e];
+  if (t == 0) {
+    sm[warp * 16 + g] = m[0]; sm[warp * 16 + g + 8] = m[1];
+    sl[warp * 16 + g] = l[0]; sl[warp * 16 + g + 8] = l[1];
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < 16 * D; i += 32 * kWarps) {
+    const int r = i / D;
+    if (i0 + r >= n) break;
+    float mx = -INFINITY, sum = 0.f, v = 0.f;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) mx = fmaxf(mx, sm[w * 16 + r]);
+    const float ref = finite_or_zero(mx);
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) {
+      const float f = expf(sm[w * 16 + r] - ref);
+      sum = fmaf(sl[w * 16 + r], f, sum);
+      v = fmaf(sa[(w * 16 + r) * D + i % D], f, v);
+    }
+    st_f(out + (bh * n + i0) * D + i, v / sum);
+  }
+}
+
+// ------------------------------------------------------------------------------------------------ backward: rows
+// 16 query rows per CTA: one walk over the keys for the row maximum, the row sum and delta = sum_j p_j dP_j (dP = dO V_sel^T), a
+// second one (logits and mask now in L2) for dS = p (dP - delta), written to the selected pathway's gradient, zero to the other.
+template <typename T, int D, bool PAIR>
+__global__ void __launch_bounds__(32 * kWarps, 4) combine_bwd_rows_kernel(const T* __restrict__ il, const T* __restrict__ el, const uint8_t* __restrict__ mask,
+                                                                       const T* __restrict__ iv, const T* __restrict__ ev, const T* __restrict__ dO,
+                                                                       T* __restrict__ d_il, T* __restrict__ d_el, float* __restrict__ stats, int H, int n) {
+  constexpr int KC = Num<T>::kKeys, NV = Num<T>::kV, LD = D + 8;
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ float red[3][kWarps][16];
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, g = lane / 4, t = lane % 4;
+  const size_t bh = blockIdx.y;
+  const int i0 = blockIdx.x * 16;
+  il += bh * n * n; el += bh * n * n; mask += size_t(bh / H) * n * n;
+  d_il += bh * n * n; d_el += bh * n * n;
+  iv += bh * n * D; ev += bh * n * D;
+  __nv_bfloat16* sv = reinterpret_cast<__nv_bfloat16*>(smem) + warp * NV * KC * LD;
+
+  uint32_t go[D / 16][NV][4];
+  stage<T, D, 16>(dO + bh * n * D, i0, n, sv, lane);
+  staged();
+#pragma unroll
+  for (int k = 0; k < D / 16; ++k)
+#pragma unroll
+    for (int q = 0; q < NV; ++q) ldsm4(go[k][q], sv + (q * 16 + (lane & 15)) * LD + 16 * k + (lane >> 4) * 8);
+
+  // logits and dP of one chunk
+  Block<T, KC, PAIR> blk;
+  auto chunk = [&](int j0, float (&s)[KC / 8][4], float (&dp)[KC / 8][4]) {
+    blk.load_mask(mask, i0, j0, n, lane);
+    __syncwarp();
+    stage<T, D, KC>(blk.any_x ? ev : iv, j0, n, sv, lane);
+    blk.load_logits(il, el, i0, j0, n, lane, s);
+    staged();
+    grad_dot<T, D, KC>(dp, go, sv, lane);
+    if (blk.any_i && blk.any_x) {
+      __syncwarp();
+      stage<T, D, KC>(iv, j0, n, sv, lane);
+      staged();
+      float di[KC / 8][4];
+      grad_dot<T, D, KC>(di, go, sv, lane);
+#pragma unroll
+      for (int nt = 0; nt < KC / 8; ++nt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (!((blk.cross >> (4 * nt + e)) & 1u)) dp[nt][e] = di[nt][e];
+    }
+  };
+
+  float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f}, dl[2] = {0.f, 0.f};
+  for (int j0 = warp * KC; j0 < n; j0 += kWarps * KC) {
+    float s[KC / 8][4], dp[KC / 8][4];
+    chunk(j0, s, dp);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float mx = m[h];
+#pragma unroll
+      for (int nt = 0; nt < KC / 8; ++nt) mx = fmaxf(mx, fmaxf(s[nt][2 * h], s[nt][2 * h + 1]));
+      mx = quad_max(mx);
+      const float ref = finite_or_zero(mx), alpha = expf(m[h] - ref);
+      m[h] = mx;
+      l[h] *= alpha;
+      dl[h] *= alpha;
+#pragma unroll
+      for (int nt = 0; nt < KC / 8; ++nt)
+#pragma unroll
+        for (int e = 2 * h; e < 2 * h + 2; ++e) {
+          const float p = exp_from<T>(s[nt][e], ref);
+          l[h] += p;
+          dl[h] = fmaf(p, dp[nt][e], dl[h]);
+        }
+    }
+  }
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    l[h] = quad_sum(l[h]);
+    dl[h] = quad_sum(dl[h]);
+    if (t == 0) { red[0][warp][g + 8 * h] = m[h]; red[1][warp][g + 8 * h] = l[h]; red[2][warp][g + 8 * h] = dl[h]; }
+  }
+  __syncthreads();
+  float ref[2], inv[2], delta[2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int r = g + 8 * h;
+    float mx = -INFINITY, sum = 0.f, d = 0.f;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) mx = fmaxf(mx, red[0][w][r]);
+    ref[h] = finite_or_zero(mx);
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) {
+      const float f = expf(red[0][w][r] - ref[h]);
+      sum = fmaf(red[1][w][r], f, sum);
+      d = fmaf(red[2][w][r], f, d);
+    }
+    inv[h] = 1.f / sum;
+    delta[h] = d * inv[h];
+    if (warp == 0 && t == 0 && i0 + r < n) {
+      stats[(bh * n + i0 + r) * 2] = ref[h];
+      stats[(bh * n + i0 + r) * 2 + 1] = inv[h];
+    }
+  }
+  for (int j0 = warp * KC; j0 < n; j0 += kWarps * KC) {
+    float s[KC / 8][4], dp[KC / 8][4];
+    chunk(j0, s, dp);
+#pragma unroll
+    for (int nt = 0; nt < KC / 8; ++nt)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const uint32_t x = blk.any_i && blk.any_x ? blk.cross >> (4 * nt + 2 * h) : blk.any_x ? 3u : 0u;
+        const uint32_t in = blk.edge ? (blk.inside >> (4 * nt + 2 * h)) & 3u : 3u;
+        if (in == 0) continue;
+        const size_t off = size_t(i0 + g + 8 * h) * n + j0 + 8 * nt + 2 * t;
+        const float a = exp_from<T>(s[nt][2 * h], ref[h]) * inv[h] * (dp[nt][2 * h] - delta[h]);
+        const float b = exp_from<T>(s[nt][2 * h + 1], ref[h]) * inv[h] * (dp[nt][2 * h + 1] - delta[h]);
+        st_pair<PAIR>(d_il + off, (x & 1u) ? 0.f : a, (x & 2u) ? 0.f : b, (in & 2u) != 0);
+        st_pair<PAIR>(d_el + off, (x & 1u) ? a : 0.f, (x & 2u) ? b : 0.f, (in & 2u) != 0);
+      }
+  }
+}
+
+// ------------------------------------------------------------------------------------------------ backward: values
+// dV_intra[j] = sum_i (p o ~M)_ij dO_i, dV_inter[j] = sum_i (p o M)_ij dO_i for one block of keys: the warps take 16 query rows
+// at a time, form the probabilities in row order, and read them back from shared memory transposed.
+template <int D> constexpr int values_keys() { return 32; }
+template <typename T, int D>
+constexpr int values_smem_bytes() {
+  constexpr int w = kWarps * (Num<T>::kP * 16 * (values_keys<D>() + 8) + Num<T>::kV * 16 * (D + 8)) * 2, r = 2 * values_keys<D>() * D * 4;
+  return w > r ? w : r;
+}
+
+template <typename T, int D, bool PAIR>
+__global__ void __launch_bounds__(32 * kWarps, D == 64 ? 2 : 4) combine_bwd_values_kernel(const T* __restrict__ il, const T* __restrict__ el, const uint8_t* __restrict__ mask,
+                                                                         const T* __restrict__ dO, const float* __restrict__ stats, T* __restrict__ d_iv,
+                                                                         T* __restrict__ d_ev, int H, int n) {
+  constexpr int KB = values_keys<D>(), NV = Num<T>::kV, NP = Num<T>::kP, LD = D + 8, LP = KB + 8;
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, g = lane / 4, t = lane % 4;
+  const size_t bh = blockIdx.y;
+  const int j0 = blockIdx.x * KB;
+  il += bh * n * n; el += bh * n * n; mask += size_t(bh / H) * n * n;
+  __nv_bfloat16* sp = reinterpret_cast<__nv_bfloat16*>(smem) + warp * (NP * 16 * LP + NV * 16 * LD);
+  __nv_bfloat16* sg = sp + NP * 16 * LP;
+
+  float acc[2][KB / 16][D / 8][4];
+#pragma unroll
+  for (int p = 0; p < 2; ++p)
+#pragma unroll
+    for (int k = 0; k < KB / 16; ++k)
+#pragma unroll
+      for (int d = 0; d < D / 8; ++d)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[p][k][d][e] = 0.f;
+
+  for (int i0 = warp * 16; i0 < n; i0 += kWarps * 16) {
+    float s[KB / 8][4];
+    Block<T, KB, PAIR> blk;
+    __syncwarp();
+    stage<T, D, 16>(dO + bh * n * D, i0, n, sg, lane);
+    blk.load_mask(mask, i0, j0, n, lane);
+    blk.load_logits(il, el, i0, j0, n, lane, s);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int i = i0 + g + 8 * h;
+      const float2 st = i < n ? *reinterpret_cast<const float2*>(stats + (bh * n + i) * 2) : make_float2(0.f, 0.f);
+#pragma unroll
+      for (int nt = 0; nt < KB / 8; ++nt)
+#pragma unroll
+        for (int e = 2 * h; e < 2 * h + 2; ++e) s[nt][e] = exp_from<T>(s[nt][e], st.x) * st.y;
+    }
+#pragma unroll
+    for (int path = 0; path < 2; ++path) {
+      if (!(path ? blk.any_x : blk.any_i)) continue;
+      float pr[KB / 8][4];
+      if (blk.any_i && blk.any_x) keep(pr, s, path ? blk.cross : ~blk.cross);
+      else keep(pr, s, 0xffffffffu);
+      __syncwarp();
+#pragma unroll
+      for (int nt = 0; nt < KB / 8; ++nt)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          uint32_t w[NP];
+          split2<NP>(pr[nt][2 * h], pr[nt][2 * h + 1], w);
+#pragma unroll
+          for (int q = 0; q < NP; ++q) *reinterpret_cast<uint32_t*>(sp + (q * 16 + g + 8 * h) * LP + 8 * nt + 2 * t) = w[q];
+        }
+      staged();
+#pragma unroll
+      for (int k = 0; k < KB / 16; ++k) {
+        uint32_t a[NP][4];   // P^T: 16 keys x 16 rows
+#pragma unroll
+        for (int q = 0; q < NP; ++q)
+          ldsm4t(a[q], sp + (q * 16 + (lane & 7) + ((lane >> 4) << 3)) * LP + 16 * k + ((lane >> 3) & 1) * 8);
+#pragma unroll
+        for (int d = 0; d < D / 8; d += 2) {
+          uint32_t f[NV][4];
+#pragma unroll
+          for (int q = 0; q < NV; ++q) ldsm4t(f[q], sg + (q * 16 + (lane & 15)) * LD + 8 * d + (lane >> 4) * 8);
+          float c0[4] = {0.f, 0.f, 0.f, 0.f}, c1[4] = {0.f, 0.f, 0.f, 0.f};
+          mma_pieces<NP, NV>(c0, a, [&](int q) { return make_uint2(f[q][0], f[q][1]); });
+          mma_pieces<NP, NV>(c1, a, [&](int q) { return make_uint2(f[q][2], f[q][3]); });
+#pragma unroll
+          for (int e = 0; e < 4; ++e) { acc[path][k][d][e] += c0[e]; acc[path][k][d + 1][e] += c1[e]; }
+        }
+      }
+    }
+  }
+  __syncthreads();
+  float* red = reinterpret_cast<float*>(smem);   // [2][KB][D], the warps' sums added in turn
+  for (int w = 0; w < kWarps; ++w) {
+    if (warp == w) {
+#pragma unroll
+      for (int p = 0; p < 2; ++p)
+#pragma unroll
+        for (int k = 0; k < KB / 16; ++k)
+#pragma unroll
+          for (int d = 0; d < D / 8; ++d)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              float* r = red + (p * KB + 16 * k + g + 8 * (e / 2)) * D + 8 * d + 2 * t + (e & 1);
+              *r = w == 0 ? acc[p][k][d][e] : *r + acc[p][k][d][e];
+            }
+    }
+    __syncthreads();
+  }
+  for (int i = threadIdx.x; i < KB * D; i += 32 * kWarps) {
+    if (j0 + i / D >= n) break;
+    st_f(d_iv + (bh * n + j0) * D + i, red[i]);
+    st_f(d_ev + (bh * n + j0) * D + i, red[KB * D + i]);
+  }
+}
+
+template <typename K>
+cudaError_t need_smem(K kernel, int bytes) {
+  return bytes <= 48 * 1024 ? cudaSuccess : cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+}
+
+template <typename T, int D, bool PAIR>
+cudaError_t fwd_t(const void* il, const void* el, const uint8_t* mask, const void* iv, const void* ev, void* out, int B, int H, int n, cudaStream_t s) {
+  constexpr int bytes = fwd_smem_bytes<T, D>();
+  cudaError_t e = need_smem(combine_fwd_kernel<T, D, PAIR>, bytes);
+  if (e != cudaSuccess) return e;
+  combine_fwd_kernel<T, D, PAIR><<<dim3((n + 15) / 16, B * H), 32 * kWarps, bytes, s>>>(
+      static_cast<const T*>(il), static_cast<const T*>(el), mask, static_cast<const T*>(iv), static_cast<const T*>(ev), static_cast<T*>(out), H, n);
   count_launches(1);
   return cudaGetLastError();
 }
 
-template <typename T, int D>
-static cudaError_t bwd_t(const void* il, const void* el, const uint8_t* mask, const void* iv, const void* ev,
-                         const void* d_out, void* d_il, void* d_el, void* d_iv, void* d_ev, float* stats, int B, int H,
-                         int Tn, cudaStream_t s) {
-  size_t rows = size_t(B) * H * Tn;
-  combine_bwd_rows_kernel<T, D><<<unsigned((rows + 3) / 4), 128, 0, s>>>(
-      static_cast<const T*>(il), static_cast<const T*>(el), mask, static_cast<const T*>(iv), static_cast<const T*>(ev),
-      static_cast<const T*>(d_out), static_cast<T*>(d_il), static_cast<T*>(d_el), stats, B, H, Tn);
-  dim3 grid((Tn + 31) / 32, B * H);
-  combine_bwd_values_kernel<T, D><<<grid, 128, 0, s>>>(static_cast<const T*>(il), static_cast<const T*>(el), mask,
-                                                       static_cast<const T*>(d_out), stats, static_cast<T*>(d_iv),
-                                                       static_cast<T*>(d_ev), B, H, Tn);
+template <typename T, int D, bool PAIR>
+cudaError_t bwd_t(const void* il, const void* el, const uint8_t* mask, const void* iv, const void* ev, const void* d_out, void* d_il, void* d_el, void* d_iv,
+                  void* d_ev, float* stats, int B, int H, int n, cudaStream_t s) {
+  constexpr int rows_bytes = kWarps * Num<T>::kV * Num<T>::kKeys * (D + 8) * 2, val_bytes = values_smem_bytes<T, D>();
+  cudaError_t e = need_smem(combine_bwd_rows_kernel<T, D, PAIR>, rows_bytes);
+  if (e == cudaSuccess) e = need_smem(combine_bwd_values_kernel<T, D, PAIR>, val_bytes);
+  if (e != cudaSuccess) return e;
+  combine_bwd_rows_kernel<T, D, PAIR><<<dim3((n + 15) / 16, B * H), 32 * kWarps, rows_bytes, s>>>(
+      static_cast<const T*>(il), static_cast<const T*>(el), mask, static_cast<const T*>(iv), static_cast<const T*>(ev), static_cast<const T*>(d_out),
+      static_cast<T*>(d_il), static_cast<T*>(d_el), stats, H, n);
+  combine_bwd_values_kernel<T, D, PAIR><<<dim3((n + values_keys<D>() - 1) / values_keys<D>(), B * H), 32 * kWarps, val_bytes, s>>>(
+      static_cast<const T*>(il), static_cast<const T*>(el), mask, static_cast<const T*>(d_out), stats, static_cast<T*>(d_iv), static_cast<T*>(d_ev), H, n);
   count_launches(2);
   return cudaGetLastError();
 }
 
-cudaError_t launch_combine_fwd(const void* il, const void* el, const uint8_t* mask, const void* iv, const void* ev,
-                               void* out, int B, int H, int T, int D, int dtype, cudaStream_t s) {
-#define CASE(TT, DD) return fwd_t<TT, DD>(il, el, mask, iv, ev, out, B, H, T, s)
-  if (dtype == MINTB_F32) {
-    if (D == 16) CASE(float, 16);
-    if (D == 32) CASE(float, 32);
-    if (D == 64) CASE(float, 64);
-  } else {
-    if (D == 16) CASE(__nv_bfloat16, 16);
-    if (D == 32) CASE(__nv_bfloat16, 32);
-    if (D == 64) CASE(__nv_bfloat16, 64);
-  }
-#undef CASE
-  return cudaErrorInvalidValue;
+bool aligned(size_t to, std::initializer_list<const void*> ps) {
+  for (const void* p : ps)
+    if (reinterpret_cast<uintptr_t>(p) % to) return false;
+  return true;
 }
 
-cudaError_t launch_combine_bwd(const void* il, const void* el, const uint8_t* mask, const void* iv, const void* ev,
-                               const void* d_out, void* d_il, void* d_el, void* d_iv, void* d_ev, float* stats, int B,
-                               int H, int T, int D, int dtype, cudaStream_t s) {
-#define CASE(TT, DD) return bwd_t<TT, DD>(il, el, mask, iv, ev, d_out, d_il, d_el, d_iv, d_ev, stats, B, H, T, s)
-  if (dtype == MINTB_F32) {
-    if (D == 16) CASE(float, 16);
-    if (D == 32) CASE(float, 32);
-    if (D == 64) CASE(float, 64);
-  } else {
-    if (D == 16) CASE(__nv_bfloat16, 16);
-    if (D == 32) CASE(__nv_bfloat16, 32);
-    if (D == 64) CASE(__nv_bfloat16, 64);
-  }
-#undef CASE
+}  // namespace
+
+// Rows of an even T start on a pair boundary, so pairs are read and written whole; otherwise element by element.
+#define MINTB_COMBINE_DISPATCH(FN, ...)                                                                                       \
+  if (dtype == MINTB_F32) {                                                                                                   \
+    if (D == 16) return pair ? FN<float, 16, true>(__VA_ARGS__) : FN<float, 16, false>(__VA_ARGS__);                          \
+    if (D == 32) return pair ? FN<float, 32, true>(__VA_ARGS__) : FN<float, 32, false>(__VA_ARGS__);                          \
+    if (D == 64) return pair ? FN<float, 64, true>(__VA_ARGS__) : FN<float, 64, false>(__VA_ARGS__);                          \
+  } else {                                                                                                                    \
+    if (D == 16) return pair ? FN<__nv_bfloat16, 16, true>(__VA_ARGS__) : FN<__nv_bfloat16, 16, false>(__VA_ARGS__);          \
+    if (D == 32) return pair ? FN<__nv_bfloat16, 32, true>(__VA_ARGS__) : FN<__nv_bfloat16, 32, false>(__VA_ARGS__);          \
+    if (D == 64) return pair ? FN<__nv_bfloat16, 64, true>(__VA_ARGS__) : FN<__nv_bfloat16, 64, false>(__VA_ARGS__);          \
+  }                                                                                                                           \
   return cudaErrorInvalidValue;
+
+cudaError_t launch_combine_fwd(const void* il, const void* el, const uint8_t* mask, const void* iv, const void* ev, void* out, int B, int H, int T, int D,
+                               int dtype, cudaStream_t s) {
+  const bool pair = T % 2 == 0 && aligned(dtype == MINTB_F32 ? 8 : 4, {il, el}) && aligned(2, {mask});
+  MINTB_COMBINE_DISPATCH(fwd_t, il, el, mask, iv, ev, out, B, H, T, s)
+}
+
+cudaError_t launch_combine_bwd(const void* il, const void* el, const uint8_t* mask, const void* iv, const void* ev, const void* d_out, void* d_il, void* d_el,
+                               void* d_iv, void* d_ev, float* stats, int B, int H, int T, int D, int dtype, cudaStream_t s) {
+  const bool pair = T % 2 == 0 && aligned(dtype == MINTB_F32 ? 8 : 4, {il, el, d_il, d_el}) && aligned(2, {mask});
+  MINTB_COMBINE_DISPATCH(bwd_t, il, el, mask, iv, ev, d_out, d_il, d_el, d_iv, d_ev, stats, B, H, T, s)
 }
 
 }  // namespace mintb

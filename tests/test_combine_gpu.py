@@ -1,0 +1,35 @@
+"""Combine from materialised logits at the edges of its tiles (16 query rows, 32 / 64 keys, odd and even row lengths, tensors off a
+16-byte boundary) against the oracle."""
+import pytest
+import torch
+
+import mint_plus_b200 as M
+from oracle import multimer_attention as O
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("T,D", [(1, 16), (15, 32), (16, 64), (33, 16), (63, 64), (64, 32), (65, 64), (130, 16), (257, 32), (290, 64)])
+def test_combine_tile_edges(T, D, dtype):
+    B, H = 2, 3
+    g = torch.Generator().manual_seed(1000 * T + D)
+    il, el = (2 * torch.randn(B, H, T, T, generator=g) for _ in range(2))
+    iv, ev, grad = (torch.randn(B, H, T, D, generator=g) for _ in range(3))
+    mask = torch.rand(B, T, T, generator=g) < 0.5
+    if T > 64:
+        mask[0, :, : T // 2] = False                 # whole chunks of one pathway
+        il[:, :, :, -5:] = el[:, :, :, -5:] = float("-inf")
+    ts = [t.to(dtype) for t in (il, el, iv, ev, grad)]
+    leaves = [t.float().requires_grad_(True) for t in ts[:4]]
+    want = O.combine_from_logits(leaves[0], leaves[1], mask, leaves[2], leaves[3])
+    wg = torch.autograd.grad(want, leaves, ts[4].float())
+    off = [torch.empty(t.numel() + 1, dtype=dtype, device=DEV)[1:].view(t.shape).copy_(t) if D == 32 else t.to(DEV) for t in ts]
+    dl = [t.requires_grad_(True) for t in off[:4]]
+    out = M.fused_multimer_combine(dl[0], dl[1], mask.to(DEV), dl[2], dl[3])
+    got = torch.autograd.grad(out, dl, off[4])
+    tol = 2e-6 if dtype == torch.float32 else 6e-3
+    for a, b in zip((out, *got), (want, *wg)):
+        b = b.detach()
+        assert (a.float().cpu() - b).norm() <= tol * (b.norm() + 1e-6)
