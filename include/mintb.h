@@ -95,6 +95,9 @@ MINTB_API int mintb_reset_work_counters(void);
 MINTB_API size_t mintb_mask_meta_bytes(int B, int T);
 MINTB_API int mintb_mask_meta_from_chain_ids(const int32_t* chain_ids, const uint8_t* key_pad, void* meta, int B, int T,
                                    void* stream);
+/* the same from int64 ids, of which the low 32 bits count */
+MINTB_API int mintb_mask_meta_from_chain_ids64(const int64_t* chain_ids, const uint8_t* key_pad, void* meta, int B, int T,
+                                               void* stream);
 MINTB_API int mintb_mask_meta_from_mask(const uint8_t* chain_mask, const uint8_t* key_pad, void* meta, int B, int T,
                               void* stream);
 

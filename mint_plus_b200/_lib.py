@@ -26,6 +26,7 @@ PROTOTYPES = {
     "mintb_selftest_wait": (c_int, [c_ulonglong, _P, _P, _P]),
     "mintb_mask_meta_bytes": (c_size_t, [c_int, c_int]),
     "mintb_mask_meta_from_chain_ids": (c_int, [_P, _P, _P, c_int, c_int, _P]),
+    "mintb_mask_meta_from_chain_ids64": (c_int, [_P, _P, _P, c_int, c_int, _P]),
     "mintb_mask_meta_from_mask": (c_int, [_P, _P, _P, c_int, c_int, _P]),
     "mintb_rope_tables": (c_int, [_P, _P, _P, c_int, c_int, _P]),
     "mintb_reset_work_counters": (c_int, []),

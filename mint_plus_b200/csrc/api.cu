@@ -113,14 +113,21 @@ size_t mintb_mask_meta_bytes(int B, int T) {
   return meta_layout(B, T).total;
 }
 
-int mintb_mask_meta_from_chain_ids(const int32_t* chain_ids, const uint8_t* key_pad, void* meta, int B, int T,
-                                   void* stream) {
+static int meta_from_chain_ids(const void* chain_ids, bool ids64, const uint8_t* key_pad, void* meta, int B, int T, void* stream) {
   if (B <= 0 || T <= 0 || chain_ids == nullptr || meta == nullptr || !aligned(meta, 256)) {
     set_error("mintb_mask_meta_from_chain_ids: need B, T > 0, chain_ids, and a 256-byte aligned meta buffer");
     return MINTB_EINVAL;
   }
-  cudaError_t e = launch_meta_from_chain_ids(chain_ids, key_pad, meta, B, T, static_cast<cudaStream_t>(stream));
+  cudaError_t e = launch_meta_from_chain_ids(chain_ids, ids64, key_pad, meta, B, T, static_cast<cudaStream_t>(stream));
   return e == cudaSuccess ? MINTB_OK : cuda_fail(e, "mask metadata launch");
+}
+
+int mintb_mask_meta_from_chain_ids(const int32_t* chain_ids, const uint8_t* key_pad, void* meta, int B, int T, void* stream) {
+  return meta_from_chain_ids(chain_ids, false, key_pad, meta, B, T, stream);
+}
+
+int mintb_mask_meta_from_chain_ids64(const int64_t* chain_ids, const uint8_t* key_pad, void* meta, int B, int T, void* stream) {
+  return meta_from_chain_ids(chain_ids, true, key_pad, meta, B, T, stream);
 }
 
 int mintb_mask_meta_from_mask(const uint8_t* chain_mask, const uint8_t* key_pad, void* meta, int B, int T,

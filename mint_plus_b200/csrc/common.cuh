@@ -128,7 +128,7 @@ int check_attn_args(AttnArgs& a, const char* who, const void* q_s, const void* k
                     unsigned flags, float scale, void* stream, int* dev_status);
 
 // prep.cu
-cudaError_t launch_meta_from_chain_ids(const int32_t* chain_ids, const uint8_t* key_pad, void* meta, int B, int T,
+cudaError_t launch_meta_from_chain_ids(const void* chain_ids, bool ids64, const uint8_t* key_pad, void* meta, int B, int T,
                                        cudaStream_t s);
 cudaError_t launch_meta_from_mask(const uint8_t* mask, const uint8_t* key_pad, void* meta, int B, int T,
                                   cudaStream_t s);

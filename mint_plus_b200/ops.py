@@ -85,19 +85,21 @@ def _key_pad_u8(key_padding_mask, B, T):
         return None
     if tuple(key_padding_mask.shape) != (B, T):
         raise ValueError(f"key_padding_mask must be (B, T) = ({B}, {T}), got {tuple(key_padding_mask.shape)}")
-    return key_padding_mask.to(torch.uint8).contiguous()
+    m = key_padding_mask.contiguous()
+    return m.view(torch.uint8) if m.dtype == torch.bool else m.to(torch.uint8)
 
 
 def mask_meta_from_chain_ids(chain_ids: torch.Tensor, key_padding_mask: Optional[torch.Tensor] = None) -> MaskMeta:
     """chain_ids (B,T) integer; key_padding_mask (B,T) bool, True = padded key (esm2.py:85,89)."""
     _require_cuda(chain_ids, key_padding_mask)
     B, T = chain_ids.shape
-    cid = chain_ids.to(torch.int32).contiguous()
+    cid = (chain_ids if chain_ids.dtype in (torch.int32, torch.int64) else chain_ids.to(torch.int32)).contiguous()
     pad = _key_pad_u8(key_padding_mask, B, T)
-    buf = torch.empty(L.lib().mintb_mask_meta_bytes(B, T), dtype=torch.uint8, device=cid.device)
+    lib = L.lib()
+    build = lib.mintb_mask_meta_from_chain_ids64 if cid.dtype == torch.int64 else lib.mintb_mask_meta_from_chain_ids
+    buf = torch.empty(lib.mintb_mask_meta_bytes(B, T), dtype=torch.uint8, device=cid.device)
     with _on(cid.device):
-        L.check(L.lib().mintb_mask_meta_from_chain_ids(_ptr(cid), _ptr(pad), _ptr(buf), B, T, _stream()),
-                "mask_meta_from_chain_ids")
+        L.check(build(_ptr(cid), _ptr(pad), _ptr(buf), B, T, _stream()), "mask_meta_from_chain_ids")
     return MaskMeta(buf, B, T)
 
 
@@ -138,6 +140,7 @@ def cached_mask_meta(chain_mask: torch.Tensor, key_padding_mask: Optional[torch.
 
 # ----------------------------------------------------------------------------------------------- RoPE tables
 _rope_cache = {}
+_ROPE_TABLES = 256
 
 
 def default_inv_freq(D: int, device) -> torch.Tensor:
@@ -150,22 +153,27 @@ def rope_tables(T: int, D: int, device,
     """(cos, sin, inv_freq): the cos/sin tables (T, D/2) fp32 on `device`, cached per (T, D, device, inv_freq contents); the
     third entry is the caller's inv_freq (None for the default frequencies), held so that the cache key stays valid."""
     device = torch.device(device)
-    key = (T, D, device.index, inv_freq.data_ptr() if inv_freq is not None else 0,
-           inv_freq._version if inv_freq is not None else 0)
+    key = (D, device.index, inv_freq.data_ptr() if inv_freq is not None else 0, inv_freq._version if inv_freq is not None else 0)
     hit = _rope_cache.get(key)
-    if hit is not None:
-        return hit
-    inv = default_inv_freq(D, device) if inv_freq is None else inv_freq.detach().to(device=device, dtype=torch.float32).contiguous()
-    if inv.numel() != D // 2:
-        raise ValueError(f"inv_freq must have D/2 = {D // 2} entries")
-    cos = torch.empty(T, D // 2, dtype=torch.float32, device=device)
-    sin = torch.empty_like(cos)
-    with _on(device):
-        L.check(L.lib().mintb_rope_tables(_ptr(inv), _ptr(cos), _ptr(sin), T, D, _stream()), "rope_tables")
-    if len(_rope_cache) > 16:
-        _rope_cache.clear()
-    _rope_cache[key] = (cos, sin, inv_freq)   # keeps the buffer alive so its address cannot be reused under this key
-    return _rope_cache[key]
+    if hit is not None and T in hit[3]:
+        return hit[3][T]
+    if hit is None or T > hit[0].shape[0]:
+        # row t depends on t alone, so the table of the longest length seen so far serves the shorter ones
+        rows = (T + 255) // 256 * 256
+        inv = default_inv_freq(D, device) if inv_freq is None else inv_freq.detach().to(device=device, dtype=torch.float32).contiguous()
+        if inv.numel() != D // 2:
+            raise ValueError(f"inv_freq must have D/2 = {D // 2} entries")
+        cos = torch.empty(rows, D // 2, dtype=torch.float32, device=device)
+        sin = torch.empty_like(cos)
+        with _on(device):
+            L.check(L.lib().mintb_rope_tables(_ptr(inv), _ptr(cos), _ptr(sin), rows, D, _stream()), "rope_tables")
+        while len(_rope_cache) >= _ROPE_TABLES:      # every layer of a model brings its own inv_freq buffer
+            _rope_cache.pop(next(iter(_rope_cache)), None)
+        hit = _rope_cache[key] = (cos, sin, inv_freq, {})   # keeps the buffer alive so its address cannot be reused under this key
+    if len(hit[3]) >= 64:
+        hit[3].clear()
+    hit[3][T] = out = (hit[0][:T], hit[1][:T], inv_freq)
+    return out
 
 
 # ----------------------------------------------------------------------------------------------- attention
@@ -1104,6 +1112,8 @@ class _EmbedFn(torch.autograd.Function):
         V, E, dt, pad_idx, mask_idx, td = ctx.cfg
         B, T = tokens.shape
         d_out = d_out.contiguous()
+        if d_out.data_ptr() % 16:        # a view off the kernel's alignment
+            d_out = d_out.clone()
         dw = torch.empty(V, E, dtype=torch.float32, device=d_out.device)
         with _on(d_out.device):
             rc = L.lib().mintb_embed_bwd(_ptr(tokens), _ptr(d_out), _ptr(scales), _ptr(dw), B, T, E, V, _DTYPES[dt], pad_idx, mask_idx, td,
