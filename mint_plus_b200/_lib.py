@@ -93,6 +93,25 @@ def lib() -> ctypes.CDLL:
     return _lib
 
 
+_host = None
+
+
+def host():
+    """The C++ host side (csrc/host): launches and autograd nodes over the library.  Like the library it has no fallback."""
+    global _host
+    if _host is None:
+        lib()
+        import torch  # noqa: F401 - its libraries have to be loaded first
+        try:
+            from . import _mintb_host as mod
+        except ImportError as e:
+            raise MintbError(f"the host extension cannot be loaded ({e}): build it with `python -m mint_plus_b200.build`. "
+                             "There is no fallback path.") from e
+        mod.set_failure_class(MintbError)
+        _host = mod
+    return _host
+
+
 def check(rc: int, what: str) -> None:
     """Map a MINTB_* return code to a Python exception (ValueError for rejected arguments)."""
     if rc == OK:

@@ -1,0 +1,137 @@
+// Host side of the operators in C++: tensors in, launches of libmintb out, without the interpreter in between.
+//
+// A step of a small model is a few hundred launches of a few microseconds each, and from Python every one of them cost the host
+// 20 to 35 us (argument conversion, tensor wrappers, a Python autograd function): the 8M training step ran 11.1 ms for 2.3 ms of
+// kernels, one pair through the FP8 650M model 13.9 ms for 3.5 ms.  Here a launch costs the driver call, its tensor maps and the
+// allocator; the backward pass runs on autograd's thread without the interpreter lock.
+#pragma once
+
+#include <ATen/ATen.h>
+#include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/saved_variable.h>
+
+#include <optional>
+#include <stdexcept>
+#include <string>
+#include <utility>
+#include <vector>
+
+#include "../../../include/mintb.h"
+
+namespace mintb_host {
+
+using at::Tensor;
+using torch::autograd::SavedVariable;
+using torch::autograd::variable_list;
+using OptTensor = std::optional<Tensor>;
+
+// A CUDA failure reported by the library (the Python side maps it to MintbError).
+struct MintbFailure : std::runtime_error {
+  using std::runtime_error::runtime_error;
+};
+
+inline void check(int rc, const char* what) {
+  if (rc == MINTB_OK) return;
+  const std::string msg = std::string(what) + ": " + mintb_last_error();
+  if (rc == MINTB_EINVAL || rc == MINTB_EWORKSPACE) TORCH_CHECK_VALUE(false, msg);
+  if (rc == MINTB_EUNSUPPORTED) TORCH_CHECK_NOT_IMPLEMENTED(false, msg);
+  throw MintbFailure(msg);
+}
+
+Tensor dev_status(int device);   // the device's status word (int32 [1]), created on first use
+
+// Everything a launch needs to know about where it runs; makes the tensor's device current for its lifetime.
+struct Env {
+  explicit Env(const Tensor& t) : guard(t.device()), stream(at::cuda::getCurrentCUDAStream(t.device().index()).stream()), status(status_ptr(t.device().index())), opts(t.options()) {}
+  c10::cuda::CUDAGuard guard;
+  void* stream;
+  int* status;
+  at::TensorOptions opts;   // options of the tensor: device, layout (dtype overridden per allocation)
+
+  Tensor empty(at::IntArrayRef sizes, at::ScalarType dt) const { return at::empty(sizes, opts.dtype(dt)); }
+  Tensor bytes(size_t n) const { return n ? at::empty({int64_t(n)}, opts.dtype(at::kByte)) : Tensor(); }
+
+ private:
+  static int* status_ptr(int device);
+};
+
+inline void* ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
+inline float* fptr(const Tensor& t) { return static_cast<float*>(ptr(t)); }
+inline Tensor opt(const OptTensor& t) { return t.has_value() ? *t : Tensor(); }
+
+inline int dt_code(at::ScalarType t, const char* what) {
+  switch (t) {
+    case at::kFloat: return MINTB_F32;
+    case at::kBFloat16: return MINTB_BF16;
+    case at::kFloat8_e4m3fn: return MINTB_E4M3;
+    case at::kFloat8_e5m2: return MINTB_E5M2;
+    default: TORCH_CHECK_TYPE(false, what, " has an unsupported dtype");
+  }
+}
+inline int param_dt(const Tensor& t, const char* what) {
+  if (!t.defined()) return MINTB_F32;
+  TORCH_CHECK_TYPE(t.scalar_type() == at::kFloat || t.scalar_type() == at::kBFloat16, what, " must be float32 or bfloat16");
+  return dt_code(t.scalar_type(), what);
+}
+inline Tensor as_dtype(const Tensor& t, at::ScalarType dt) { return !t.defined() || t.scalar_type() == dt ? t : t.to(dt); }
+
+// ---- launches (no autograd) ---------------------------------------------------------------------------------------------------
+
+struct AttnInputs {   // (B,H,T,D) projections and what goes with them
+  Tensor q[6];        // q, k, v of the self pathway, then of the cross pathway
+  Tensor meta, cos, sin;
+  double scale;
+  unsigned flags;
+};
+struct AttnResult {
+  Tensor out, lse;
+  Tensor ws;          // workspace holding the rotated copies the backward pass starts from, where asked for
+};
+AttnResult attn_fwd(const AttnInputs& a, bool for_backward);
+
+struct Product {      // y = act(alpha x w^T + bias) and its variants
+  Tensor x, w, bias;
+  double alpha = 1.0;
+  bool gelu = false, save_preact = false;
+  double out_e4m3 = 0.0;         // scale of an e4m3 result, 0: bf16
+};
+std::pair<Tensor, Tensor> linear_fwd(const Product& p);     // (y, pre-activation)
+// res_a resid + res_b (alpha x w^T + bias), and with quant > 0 its e4m3 copy saturate(. / quant)
+std::pair<Tensor, Tensor> linear_res_fwd(const Product& p, const Tensor& resid, double res_a, double res_b, double quant);
+Tensor quantize(const Tensor& x, double scale);
+Tensor dgrad(const Tensor& dz, const Tensor& w, double alpha, const Tensor& dz2 = {}, const Tensor& w2 = {});
+Tensor wgrad(const Tensor& dz, const Tensor& x, double alpha, at::ScalarType out);
+// (dz, db): dz = dy gelu'(z) (dy itself without z) in bf16, db its column sums in fp32
+std::pair<Tensor, Tensor> gelu_colsum(const Tensor& dy, const Tensor& z, bool want_db);
+// (dz in e5m2, db)
+std::pair<Tensor, Tensor> gelu_colsum_f8(const Tensor& dy, const Tensor& z, bool want_db, double scale);
+
+struct NormOut {
+  Tensor s, y, stats, q8;
+};
+NormOut add_layernorm_fwd(const Tensor& x, const Tensor& r, double a, double b, const Tensor& gamma, const Tensor& beta, double eps, bool need_s, double quant);
+struct NormGrad {
+  Tensor dx, dr, dgamma, dbeta;   // parameter gradients in fp32
+};
+NormGrad add_layernorm_bwd(const Tensor& dy, const Tensor& ds, const Tensor& x, const Tensor& r, double a, double b, const Tensor& gamma, const Tensor& stats,
+                           bool want_params);
+
+// Which inputs of a call want gradients, as a node of the autograd graph; nullptr when none does.
+template <typename N>
+std::shared_ptr<N> make_node(const std::vector<Tensor>& inputs) {
+  if (!at::GradMode::is_enabled()) return nullptr;
+  bool any = false;
+  for (const Tensor& t : inputs) any = any || (t.defined() && t.requires_grad());
+  if (!any) return nullptr;
+  auto node = std::shared_ptr<N>(new N(), torch::autograd::deleteNode);
+  torch::autograd::edge_list edges;
+  edges.reserve(inputs.size());
+  for (const Tensor& t : inputs) edges.push_back(t.defined() ? torch::autograd::impl::gradient_edge(t) : torch::autograd::Edge());
+  node->set_next_edges(std::move(edges));
+  return node;
+}
+
+}  // namespace mintb_host

@@ -1,0 +1,157 @@
+// The library's calls on tensors: allocation of results and workspaces, nothing else (no autograd).
+#include <mutex>
+
+#include "common.h"
+
+namespace mintb_host {
+
+Tensor dev_status(int device) {
+  static std::mutex mu;
+  static std::vector<Tensor> words;
+  std::lock_guard<std::mutex> lock(mu);
+  if (device >= int(words.size())) words.resize(device + 1);
+  if (!words[device].defined()) words[device] = at::zeros({1}, at::TensorOptions().dtype(at::kInt).device(at::kCUDA, device));
+  return words[device];
+}
+
+int* Env::status_ptr(int device) {
+  static thread_local int last = -1;
+  static thread_local int* p = nullptr;
+  if (device != last) {
+    p = dev_status(device).data_ptr<int>();   // never replaced once created
+    last = device;
+  }
+  return p;
+}
+
+AttnResult attn_fwd(const AttnInputs& a, bool for_backward) {
+  const Tensor& q = a.q[0];
+  const int64_t B = q.size(0), H = q.size(1), T = q.size(2), D = q.size(3);
+  const int dt = dt_code(q.scalar_type(), "q");
+  Env e(q);
+  AttnResult r;
+  r.out = (a.flags & MINTB_FLAG_OUT_SEQ_FIRST) ? e.empty({T, B, H, D}, q.scalar_type()) : e.empty({B, H, T, D}, q.scalar_type());
+  r.lse = e.empty({B, H, T}, at::kFloat);
+  size_t bytes = mintb_attn_fwd_workspace_bytes(B, H, T, D, dt, a.flags);
+  // with in-kernel RoPE the forward pass leaves the rotated copies of Q_self and K_self at the start of its workspace: sized for
+  // the backward pass and kept, that pass starts from them
+  const bool keep = for_backward && (a.flags & MINTB_FLAG_ROPE) && !(a.flags & MINTB_FLAG_QK_PREROTATED);
+  if (keep) bytes = std::max(bytes, mintb_attn_bwd_workspace_bytes(B, H, T, D, dt, a.flags));
+  Tensor ws = e.bytes(bytes);
+  check(mintb_attn_fwd(ptr(a.q[0]), ptr(a.q[1]), ptr(a.q[2]), ptr(a.q[3]), ptr(a.q[4]), ptr(a.q[5]), ptr(a.meta), fptr(a.cos), fptr(a.sin), ptr(r.out),
+                       fptr(r.lse), ptr(ws), bytes, B, H, T, D, dt, a.flags, float(a.scale), e.stream, e.status),
+        "mintb_attn_fwd");
+  if (keep) r.ws = ws;
+  return r;
+}
+
+std::pair<Tensor, Tensor> linear_fwd(const Product& p) {
+  Env e(p.x);
+  const int64_t M = p.x.size(0), K = p.x.size(1), N = p.w.size(0);
+  const bool f8_out = p.out_e4m3 > 0;
+  Tensor out = e.empty({M, N}, f8_out ? at::kFloat8_e4m3fn : at::kBFloat16);
+  Tensor z = p.gelu && p.save_preact ? e.empty({M, N}, at::kBFloat16) : Tensor();
+  check(mintb_linear_fwd(ptr(p.x), ptr(p.w), ptr(p.bias), ptr(out), ptr(z), M, N, K, dt_code(p.x.scalar_type(), "x"), param_dt(p.bias, "bias"),
+                         f8_out ? MINTB_E4M3 : MINTB_BF16, p.gelu, float(p.alpha), f8_out ? float(1.0 / p.out_e4m3) : 1.f, e.stream, e.status),
+        "mintb_linear_fwd");
+  return {out, z};
+}
+
+std::pair<Tensor, Tensor> linear_res_fwd(const Product& p, const Tensor& resid, double res_a, double res_b, double quant) {
+  Env e(p.x);
+  const int64_t M = p.x.size(0), K = p.x.size(1), N = p.w.size(0);
+  Tensor out = e.empty({M, N}, at::kBFloat16);
+  Tensor q8 = quant > 0 ? e.empty({M, N}, at::kFloat8_e4m3fn) : Tensor();
+  check(mintb_linear_res_fwd(ptr(p.x), ptr(p.w), ptr(p.bias), ptr(resid), float(res_a), float(res_b), q8.defined() ? ptr(q8) : ptr(out),
+                             q8.defined() ? ptr(out) : nullptr, M, N, K, dt_code(p.x.scalar_type(), "x"), param_dt(p.bias, "bias"),
+                             q8.defined() ? MINTB_E4M3 : MINTB_BF16, float(p.alpha), quant > 0 ? float(1.0 / quant) : 1.f, e.stream, e.status),
+        "mintb_linear_res_fwd");
+  return {out, q8};
+}
+
+Tensor quantize(const Tensor& x, double scale) {
+  Env e(x);
+  Tensor out = e.empty(x.sizes(), at::kFloat8_e4m3fn);
+  check(mintb_quantize_e4m3(ptr(x), ptr(out), size_t(x.numel()), float(1.0 / scale), e.stream), "mintb_quantize_e4m3");
+  return out;
+}
+
+Tensor dgrad(const Tensor& dz, const Tensor& w, double alpha, const Tensor& dz2, const Tensor& w2) {
+  Env e(dz);
+  const int64_t M = dz.size(0), N = dz.size(1), K = w.size(1), N2 = dz2.defined() ? dz2.size(1) : 0;
+  Tensor dx = e.empty({M, K}, at::kBFloat16);
+  check(mintb_linear_dgrad(ptr(dz), ptr(w), ptr(dz2), ptr(w2), ptr(dx), M, N, K, N2, dt_code(dz.scalar_type(), "dz"), dt_code(w.scalar_type(), "w"),
+                           float(alpha), e.stream, e.status),
+        "mintb_linear_dgrad");
+  return dx;
+}
+
+Tensor wgrad(const Tensor& dz, const Tensor& x, double alpha, at::ScalarType out) {
+  Env e(dz);
+  const int64_t M = dz.size(0), N = dz.size(1), K = x.size(1);
+  const int odt = dt_code(out, "dw");
+  Tensor dw = e.empty({N, K}, out);
+  const size_t bytes = mintb_linear_wgrad_workspace_bytes(N, K, odt);
+  Tensor ws = e.bytes(bytes);
+  check(mintb_linear_wgrad(ptr(dz), ptr(x), ptr(dw), ptr(ws), bytes, M, N, K, dt_code(dz.scalar_type(), "dz"), dt_code(x.scalar_type(), "x"), odt,
+                           float(alpha), e.stream, e.status),
+        "mintb_linear_wgrad");
+  return dw;
+}
+
+std::pair<Tensor, Tensor> gelu_colsum(const Tensor& dy, const Tensor& z, bool want_db) {
+  if (!z.defined() && !want_db) return {dy, Tensor()};
+  Env e(dy);
+  const int64_t M = dy.size(0), N = dy.size(1);
+  Tensor dz = z.defined() ? e.empty({M, N}, at::kBFloat16) : dy;
+  Tensor db = want_db ? e.empty({N}, at::kFloat) : Tensor();
+  check(mintb_gelu_bwd_colsum_act(ptr(dy), ptr(z), z.defined() ? ptr(dz) : nullptr, nullptr, fptr(db), M, N, e.stream), "mintb_gelu_bwd_colsum");
+  return {dz, db};
+}
+
+std::pair<Tensor, Tensor> gelu_colsum_f8(const Tensor& dy, const Tensor& z, bool want_db, double scale) {
+  Env e(dy);
+  const int64_t M = dy.size(0), N = dy.size(1);
+  Tensor dz8 = e.empty({M, N}, at::kFloat8_e5m2);
+  Tensor db = want_db ? e.empty({N}, at::kFloat) : Tensor();
+  check(mintb_gelu_bwd_colsum_f8(ptr(dy), ptr(z), nullptr, nullptr, fptr(db), ptr(dz8), float(scale), M, N, e.stream), "mintb_gelu_bwd_colsum_f8");
+  return {dz8, db};
+}
+
+NormOut add_layernorm_fwd(const Tensor& x, const Tensor& r, double a, double b, const Tensor& gamma, const Tensor& beta, double eps, bool need_s, double quant) {
+  Env e(x);
+  const int64_t rows = x.size(0), E = x.size(1);
+  const bool norm = gamma.defined();
+  NormOut o;
+  if (need_s || !norm) o.s = e.empty({rows, E}, at::kBFloat16);
+  if (norm) {
+    o.y = e.empty({rows, E}, at::kBFloat16);
+    o.stats = e.empty({rows, 2}, at::kFloat);
+  }
+  if (quant > 0) o.q8 = e.empty({rows, E}, at::kFloat8_e4m3fn);
+  check(mintb_add_layernorm_fwd_q(ptr(x), ptr(r), float(a), float(b), ptr(gamma), ptr(beta), param_dt(gamma, "gamma"), ptr(o.s), ptr(o.y), fptr(o.stats), rows, E,
+                                  float(eps), ptr(o.q8), quant > 0 ? float(1.0 / quant) : 1.f, e.stream),
+        "mintb_add_layernorm_fwd");
+  return o;
+}
+
+NormGrad add_layernorm_bwd(const Tensor& dy, const Tensor& ds, const Tensor& x, const Tensor& r, double a, double b, const Tensor& gamma, const Tensor& stats,
+                           bool want_params) {
+  Env e(x);
+  const int64_t rows = x.size(0), E = x.size(1);
+  NormGrad g;
+  g.dx = e.empty({rows, E}, at::kBFloat16);
+  if (r.defined()) g.dr = e.empty({rows, E}, at::kBFloat16);
+  if (want_params) {
+    g.dgamma = e.empty({E}, at::kFloat);
+    g.dbeta = e.empty({E}, at::kFloat);
+  }
+  const size_t bytes = want_params ? mintb_add_layernorm_bwd_workspace_bytes(rows, E) : 0;
+  Tensor ws = e.bytes(bytes);
+  check(mintb_add_layernorm_bwd(ptr(dy), ptr(ds), ptr(x), ptr(r), float(a), float(b), ptr(gamma), param_dt(gamma, "gamma"), fptr(stats), ptr(g.dx), ptr(g.dr),
+                                fptr(g.dgamma), fptr(g.dbeta), ptr(ws), bytes, rows, E, e.stream),
+        "mintb_add_layernorm_bwd");
+  return g;
+}
+
+}  // namespace mintb_host

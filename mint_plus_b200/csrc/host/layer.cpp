@@ -1,0 +1,278 @@
+// A whole transformer layer as one node of the autograd graph: its forward pass is eight to ten launches, its backward pass about
+// twenty, and nothing but the kernels' own layouts lies between them.  Residual gradients ride in the LayerNorm passes, the
+// q/k/v weight gradients of separate projections are row ranges of one matrix.
+#include "layer.h"
+
+#include <tuple>
+
+namespace mintb_host {
+
+namespace {
+
+// Positions in LayerPlan::params.
+struct Where {
+  int64_t ws, bs, wc, bc, wo, bo, w1, b1, w2, b2, g1, be1, g2, be2, n;
+  explicit Where(const LayerPlan& p) {
+    int64_t k = 0;
+    ws = k; k += p.n_self;
+    bs = k; k += p.n_self;
+    wc = k; k += p.n_cross;
+    bc = k; k += p.n_cross;
+    wo = k++; bo = k++; w1 = k++; b1 = k++; w2 = k++; b2 = k++;
+    g1 = be1 = -1;
+    if (!p.mu) { g1 = k++; be1 = k++; }
+    g2 = k++; be2 = k++;
+    n = k;
+  }
+};
+
+enum Saved { kX, kXq, kStats1, kQ0, kQ1, kQ2, kQ3, kQ4, kQ5, kOut, kLse, kO, kX1, kH2, kStats2, kZ, kA, kY2, kNumSaved };
+
+}  // namespace
+
+struct LayerNode : public torch::autograd::Node {
+  LayerPlan plan;
+  Batch batch;
+  SavedVariable saved[kNumSaved];
+  std::vector<SavedVariable> weights;   // what the bf16 products read again
+  std::vector<int64_t> shape;
+  double xq_scale = 1.0;
+
+  variable_list apply(variable_list&& grads) override;
+  void release_variables() override {
+    for (auto& s : saved) s.reset_data();
+    for (auto& s : weights) s.reset_data();
+    plan = LayerPlan();
+    batch = Batch();
+  }
+  std::string name() const override { return "TransformerLayerBackward"; }
+};
+
+std::tuple<Tensor, OptTensor> LayerPlan::forward(const Tensor& x_in, const OptTensor& xq_in, const Batch& batch, double next_quant) {
+  const Where at(*this);
+  TORCH_CHECK(int64_t(params.size()) == at.n, "a layer plan needs ", at.n, " parameters, got ", params.size());
+  std::vector<Tensor> inputs;
+  inputs.reserve(at.n + 1);
+  inputs.push_back(x_in);
+  for (const Tensor& t : params) inputs.push_back(t);
+  auto node = make_node<LayerNode>(inputs);
+  const bool grad = node != nullptr;
+
+  const int64_t E = H * D, T = batch.T, B = batch.B;
+  const bool packed = batch.rows32.defined();
+  Tensor keep_t[kNumSaved];
+  Tensor y, y8;
+  {
+    at::AutoDispatchBelowADInplaceOrView below;
+    Env e(x_in);
+    const Tensor x = x_in.reshape({-1, E}).contiguous();
+    const int64_t rows = x.size(0);
+
+    // the operand of the QKV products
+    Tensor h = x, hq;
+    if (!mu) {
+      NormOut n = add_layernorm_fwd(x, Tensor(), 1.0, 0.0, params[at.g1], params[at.be1], eps1, false, fp8 ? qkv_self.x_scale : 0.0);
+      h = n.y;
+      hq = n.q8;
+      keep_t[kStats1] = n.stats;
+    } else if (fp8) {
+      hq = xq_in.has_value() ? xq_in->reshape({-1, E}) : quantize(x, qkv_self.x_scale);
+    }
+    const Tensor& op = fp8 ? hq : h;
+
+    // q, k, v of both pathways, head-major, the self pathway rotated.  Packed: positions without a token are not written, and keys
+    // there are masked but still multiplied by a zero probability, so they must hold finite numbers.
+    AttnInputs a;
+    Tensor all = packed ? at::zeros({6, B, H, T, D}, e.opts.dtype(at::kBFloat16)) : e.empty({6, B, H, T, D}, at::kBFloat16);
+    for (int k = 0; k < 6; ++k) a.q[k] = all.select(0, k);
+    const int32_t* map = packed ? batch.rows32.data_ptr<int32_t>() : nullptr;
+    const int in_dt = fp8 ? MINTB_E4M3 : MINTB_BF16;
+    if (qkv6.defined()) {
+      check(mintb_qkv2_fwd(ptr(op), ptr(qkv6), ptr(bias6), ptr(a.q[0]), ptr(a.q[1]), ptr(a.q[2]), ptr(a.q[3]), ptr(a.q[4]), ptr(a.q[5]), T, B, H, D, in_dt,
+                           param_dt(bias6, "bias"), float(qkv_self.alpha()), float(qkv_cross.alpha()), 1.f, fptr(batch.cos), fptr(batch.sin), map, rows, e.stream,
+                           e.status),
+            "mintb_qkv2_fwd");
+    } else {
+      for (int p = 0; p < 2; ++p) {
+        const Operand& o = p ? qkv_cross : qkv_self;
+        const Tensor& bias = p ? bias_cross : bias_self;
+        check(mintb_qkv_fwd(ptr(op), ptr(o.w), ptr(bias), ptr(a.q[3 * p]), ptr(a.q[3 * p + 1]), ptr(a.q[3 * p + 2]), T, B, H, D, in_dt, param_dt(bias, "bias"),
+                            float(o.alpha()), 1.f, p ? nullptr : fptr(batch.cos), p ? nullptr : fptr(batch.sin), map, rows, e.stream, e.status),
+              "mintb_qkv_fwd");
+      }
+    }
+    a.meta = batch.meta;
+    a.scale = scale;
+    a.flags = MINTB_FLAG_OUT_SEQ_FIRST | (sqrt_softmax ? MINTB_FLAG_SQRT_SOFTMAX : 0) | (packed ? MINTB_FLAG_SKIP_PAD_QUERIES : 0);
+    AttnResult attn = attn_fwd(a, false);
+    Tensor o = attn.out.view({T * B, E});
+    if (packed) o = o.index_select(0, batch.rows64);
+
+    // output projection with the residual sum in its epilogue
+    Product po;
+    po.x = fp8 ? quantize(o, out.x_scale) : o;
+    po.w = out.w; po.bias = params[at.bo]; po.alpha = out.alpha();
+    auto [x1, x1q] = linear_res_fwd(po, x, keep, add, fp8 && mu ? fc1.x_scale : 0.0);
+
+    Tensor h2 = x1, h2q = x1q;
+    if (!mu) {
+      NormOut n = add_layernorm_fwd(x1, Tensor(), 1.0, 0.0, params[at.g2], params[at.be2], eps2, false, fp8 ? fc1.x_scale : 0.0);
+      h2 = n.y;
+      h2q = n.q8;
+      keep_t[kStats2] = n.stats;
+    }
+    Product p1;
+    p1.x = fp8 ? h2q : h2;
+    p1.w = fc1.w; p1.bias = params[at.b1]; p1.alpha = fc1.alpha(); p1.gelu = true; p1.save_preact = grad; p1.out_e4m3 = fp8 ? fc2.x_scale : 0.0;
+    auto [act, z] = linear_fwd(p1);
+    Product p2;
+    p2.x = act;
+    p2.w = fc2.w; p2.bias = params[at.b2]; p2.alpha = fc2.alpha();
+    if (!mu) {
+      std::tie(y, y8) = linear_res_fwd(p2, x1, 1.0, 1.0, 0.0);
+    } else {
+      Tensor y2 = linear_fwd(p2).first;
+      NormOut n = add_layernorm_fwd(x1, y2, keep, add, params[at.g2], params[at.be2], eps2, false, next_quant);
+      y = n.y;
+      y8 = n.q8;
+      keep_t[kY2] = y2;
+      keep_t[kStats2] = n.stats;
+    }
+    y = y.view(x_in.sizes());
+    if (grad) {
+      keep_t[kXq] = op;
+      for (int k = 0; k < 6; ++k) keep_t[kQ0 + k] = a.q[k];
+      keep_t[kOut] = attn.out;
+      keep_t[kLse] = attn.lse;
+      keep_t[kO] = po.x;
+      keep_t[kX1] = x1;
+      keep_t[kH2] = p1.x;
+      keep_t[kZ] = z;
+      keep_t[kA] = act;
+    }
+  }
+  if (grad) {
+    torch::autograd::set_history(y, node);
+    node->plan = *this;
+    node->batch = batch;
+    node->shape = x_in.sizes().vec();
+    keep_t[kX] = x_in;
+    for (int k = 0; k < kNumSaved; ++k)
+      if (keep_t[k].defined()) node->saved[k] = SavedVariable(keep_t[k], false);
+    if (!fp8)
+      for (const Tensor& t : {qkv_self.w, qkv_cross.w, out.w, fc1.w, fc2.w}) node->weights.emplace_back(t, false);
+  }
+  return {y, y8.defined() ? OptTensor(y8) : OptTensor()};
+}
+
+variable_list LayerNode::apply(variable_list&& grads) {
+  const Where at(plan);
+  variable_list res(at.n + 1);
+  if (!grads[0].defined()) return res;
+  at::NoGradGuard no_grad;
+  const bool fp8 = plan.fp8, mu = plan.mu, packed = batch.rows32.defined();
+  const int64_t E = plan.H * plan.D, T = batch.T, B = batch.B;
+  auto wants = [&](int64_t k) { return k >= 0 && plan.params[k].defined() && task_should_compute_output(size_t(k) + 1); };
+  auto any = [&](int64_t k, int64_t n) {
+    bool w = false;
+    for (int64_t i = 0; i < n; ++i) w = w || wants(k + i);
+    return w;
+  };
+  auto give = [&](int64_t k, const Tensor& g) {
+    if (g.defined()) res[k + 1] = as_dtype(g, plan.params[k].scalar_type());
+  };
+  auto give_rows = [&](int64_t k, int64_t n, const Tensor& g) {   // the rows of q, k and v
+    if (!g.defined()) return;
+    const Tensor c = as_dtype(g, plan.params[k].scalar_type());
+    for (int64_t i = 0; i < n; ++i)
+      if (wants(k + i)) res[k + i + 1] = n == 1 ? c : c.narrow(0, i * E, E);
+  };
+  auto w_dt = [&](int64_t k) { return plan.params[k].scalar_type() == at::kFloat ? at::kFloat : at::kBFloat16; };
+  for (auto& s : weights) s.unpack();   // raises if a weight that the products read again has been written since
+  Tensor s[kNumSaved];
+  for (int k = 0; k < kNumSaved; ++k) s[k] = saved[k].unpack();
+  const Tensor x = s[kX].reshape({-1, E}).contiguous(), gy = grads[0].reshape({-1, E}).contiguous();
+  const bool p1 = wants(at.g1) || wants(at.be1), p2 = wants(at.g2) || wants(at.be2);
+
+  auto amax = [](const Tensor& t) { return t.abs().amax().item<double>(); };
+  auto settle = [&](Operand& o, auto measure) {
+    if (o.grad_scale > 0) return;
+    TORCH_CHECK(o.holder != nullptr, "an 8-bit projection without a gradient scale");
+    o.grad_scale = o.holder->current();
+    if (o.grad_scale <= 0) o.grad_scale = o.holder->fix(measure());
+  };
+  // one projection's output gradient as the operand of its products, with the bias gradient
+  auto operand = [&](Operand& o, const Tensor& dy, const Tensor& z, bool want_db) {
+    if (fp8) settle(o, [&] { return amax(z.defined() ? gelu_colsum(dy, z, false).first : dy); });
+    return fp8 ? gelu_colsum_f8(dy, z, want_db, o.grad_scale) : gelu_colsum(dy, z, want_db);
+  };
+  auto a_in = [&](const Operand& o) { return fp8 ? o.grad_scale * o.w_scale * o.out_scale : 1.0; };
+  auto a_w = [&](const Operand& o) { return fp8 ? o.grad_scale * o.x_scale * o.out_scale : 1.0; };
+
+  Tensor d_ffn = gy, d1;   // gradients of the FFN's result and of the first residual sum
+  if (mu) {
+    NormGrad g = add_layernorm_bwd(gy, Tensor(), s[kX1], s[kY2], plan.keep, plan.add, plan.params[at.g2], s[kStats2], p2);
+    if (p2) { give(at.g2, g.dgamma); give(at.be2, g.dbeta); }
+    d1 = g.dx;
+    d_ffn = g.dr;
+  }
+  {
+    auto [g2, db2] = operand(plan.fc2, d_ffn, Tensor(), wants(at.b2));
+    give(at.b2, db2);
+    if (wants(at.w2)) give(at.w2, wgrad(g2, s[kA], a_w(plan.fc2), w_dt(at.w2)));
+    Tensor da = dgrad(g2, plan.fc2.w, a_in(plan.fc2));
+    auto [g1, db1] = operand(plan.fc1, da, s[kZ], wants(at.b1));
+    give(at.b1, db1);
+    if (wants(at.w1)) give(at.w1, wgrad(g1, s[kH2], a_w(plan.fc1), w_dt(at.w1)));
+    Tensor dh2 = dgrad(g1, plan.fc1.w, a_in(plan.fc1));
+    if (mu) {
+      d1.add_(dh2);
+    } else {
+      NormGrad g = add_layernorm_bwd(dh2, gy, s[kX1], Tensor(), 1.0, 0.0, plan.params[at.g2], s[kStats2], p2);
+      if (p2) { give(at.g2, g.dgamma); give(at.be2, g.dbeta); }
+      d1 = g.dx;
+    }
+  }
+  // output projection: its result entered the sum times `add`
+  Tensor d_attn;
+  {
+    auto [go, dbo] = operand(plan.out, d1, Tensor(), wants(at.bo));
+    if (dbo.defined()) give(at.bo, plan.add == 1.0 ? dbo : dbo * plan.add);
+    if (wants(at.wo)) give(at.wo, wgrad(go, s[kO], a_w(plan.out) * plan.add, w_dt(at.wo)));
+    d_attn = dgrad(go, plan.out.w, a_in(plan.out) * plan.add);
+  }
+  if (packed) d_attn = at::zeros({T * B, E}, d_attn.options()).index_copy_(0, batch.rows64, d_attn);
+  AttnInputs a;
+  for (int k = 0; k < 6; ++k) a.q[k] = s[kQ0 + k];
+  a.meta = batch.meta;
+  a.scale = plan.scale;
+  a.flags = MINTB_FLAG_OUT_SEQ_FIRST | (plan.sqrt_softmax ? MINTB_FLAG_SQRT_SOFTMAX : 0) | (packed ? MINTB_FLAG_SKIP_PAD_QUERIES : 0);
+  RowMajor rm{x.size(0), batch.inv32, batch.cos, batch.sin};
+  auto g = attn_bwd(a, s[kOut], s[kLse], d_attn, Tensor(), &rm);
+
+  // both projections read the same rows: their input gradients are one product over the concatenated reduction, so the e5m2 casts
+  // take scales that give them one multiplier
+  Operand os = plan.qkv_self, oc = plan.qkv_cross;
+  if (fp8) settle(os, [&] { return std::max(amax(g[0]), amax(g[1]) / ((os.w_scale * os.out_scale) / (oc.w_scale * oc.out_scale))); });
+  if (fp8) oc.grad_scale = os.grad_scale * (os.w_scale * os.out_scale) / (oc.w_scale * oc.out_scale);
+  auto [gs, dbs] = operand(os, g[0], Tensor(), any(at.bs, plan.n_self));
+  auto [gc, dbc] = operand(oc, g[1], Tensor(), any(at.bc, plan.n_cross));
+  give_rows(at.bs, plan.n_self, dbs);
+  give_rows(at.bc, plan.n_cross, dbc);
+  if (any(at.ws, plan.n_self)) give_rows(at.ws, plan.n_self, wgrad(gs, s[kXq], a_w(os), w_dt(at.ws)));
+  if (any(at.wc, plan.n_cross)) give_rows(at.wc, plan.n_cross, wgrad(gc, s[kXq], a_w(oc), w_dt(at.wc)));
+  if (mu) {
+    if (task_should_compute_output(0)) {
+      Tensor dx = dgrad(gs, os.w, a_in(os), gc, oc.w);
+      res[0] = dx.add_(d1, plan.keep).view(shape);
+    }
+  } else if (task_should_compute_output(0) || p1) {
+    Tensor dh = dgrad(gs, os.w, a_in(os), gc, oc.w);
+    NormGrad n = add_layernorm_bwd(dh, d1, x, Tensor(), 1.0, 0.0, plan.params[at.g1], s[kStats1], p1);
+    if (p1) { give(at.g1, n.dgamma); give(at.be1, n.dbeta); }
+    res[0] = n.dx.view(shape);
+  }
+  return res;
+}
+
+}  // namespace mintb_host

@@ -1,0 +1,48 @@
+#pragma once
+
+#include "ops.h"
+
+namespace mintb_host {
+
+// The static scale of an e5m2 gradient cast, kept on the Python side; 0 until a first backward pass has measured it.
+struct ScaleHolder {
+  virtual ~ScaleHolder() = default;
+  virtual double current() = 0;
+  virtual double fix(double amax) = 0;   // the scale for gradients of that size, from now on
+};
+
+// One projection's operand: the bf16 weight itself, or its e4m3 copy with the scales of an 8-bit product.
+struct Operand {
+  Tensor w;
+  double w_scale = 1.0, x_scale = 1.0, out_scale = 1.0;
+  double grad_scale = 0.0;   // of the e5m2 cast of its output gradient; 0: ask the holder
+  std::shared_ptr<ScaleHolder> holder;
+  double alpha() const { return w_scale * x_scale * out_scale; }
+};
+
+// What a batch brings with it.
+struct Batch {
+  int64_t T, B;
+  Tensor meta, cos, sin;
+  Tensor rows32, rows64, inv32;   // packed tokens: (t, b) row of each token, and its inverse; undefined: the padded grid
+};
+
+// A two-pathway transformer layer laid out for calling: its parameters and the operands formed from them.  The Python layer builds
+// one and keeps it until a parameter or an operand it was made from changes.
+struct LayerPlan {
+  bool mu = false;      // x = keep x + add attn(x); x = LN(keep x + add ffn(x)); else x += attn(LN(x)); x += ffn(LN(x))
+  bool fp8 = false, sqrt_softmax = false;
+  int64_t H = 0, D = 0;
+  double scale = 1.0, keep = 1.0, add = 1.0, eps1 = 0.0, eps2 = 0.0;
+  // parameters: self q/k/v weights (one fused or three), their biases, the cross pathway's, then out, fc1, fc2 (weight, bias) and the
+  // norms (gamma, beta): the first one on Pre-LN layers only.  An absent bias is undefined.
+  std::vector<Tensor> params;
+  int64_t n_self = 1, n_cross = 1;
+  Operand qkv_self, qkv_cross, out, fc1, fc2;   // qkv operands [3E][E], rows [Q; K; V]
+  Tensor qkv6, bias6;                           // both pathways in one operand, when one product serves them
+  Tensor bias_self, bias_cross;                 // [3E] biases of separate products
+
+  std::tuple<Tensor, OptTensor> forward(const Tensor& x, const OptTensor& xq, const Batch& batch, double next_quant);
+};
+
+}  // namespace mintb_host

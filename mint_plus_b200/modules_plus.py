@@ -13,7 +13,7 @@ import torch
 import torch.nn.functional as F
 from torch import nn
 
-from . import ops
+from . import native, ops
 from .attention import MultiHeadAttention, MultimerAttention
 from .kernels import fused_multimer_combine
 
@@ -234,6 +234,9 @@ class _PreLnLayer(_TwoPathwayLayer):
         self.final_layer_norm = norm()
 
     def forward(self, x, self_attn_mask=None, self_attn_padding_mask=None, chain_ids=None, pack=None):
+        y = native.run_layer(self, x, self_attn_mask, self_attn_padding_mask, chain_ids, pack, mu=False, keep=1.0, add=1.0)
+        if y is not None:
+            return y, None
         if x.is_cuda and x.dtype == torch.bfloat16 and isinstance(self.final_layer_norm, nn.LayerNorm):
             # bf16 on the GPU: each residual add is fused with the LayerNorm that follows it (one pass over the activations)
             _, h = ops.add_layernorm(x, None, 1.0, 0.0, self.self_attn_layer_norm, need_s=False)

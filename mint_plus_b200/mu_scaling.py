@@ -18,7 +18,7 @@ from typing import Optional
 import torch
 from torch import nn
 
-from . import ops
+from . import native, ops
 from .attention import MultiHeadAttention
 from .modules_plus import VanillaFeedForward, _TwoPathwayLayer
 
@@ -397,6 +397,10 @@ class TransformerLayer_MINT_mu(_TwoPathwayLayer):
     def forward(self, x, self_attn_mask=None, self_attn_padding_mask=None, chain_ids=None, pack=None):
         tau = self._tau_f                       # host copy of the buffer: no device read-back per call
         keep, add = math.sqrt(1.0 - tau), math.sqrt(tau)
+        y = native.run_layer(self, x, self_attn_mask, self_attn_padding_mask, chain_ids, pack, mu=True, keep=keep, add=add,
+                             next_quant=self._next_x_scale)
+        if y is not None:
+            return y, None
         gpu_bf16 = x.is_cuda and x.dtype == torch.bfloat16
         fc1 = self.feed_forward.fc1
         fc1_scale = fc1.x_scale if isinstance(fc1, Fp8Linear) else None

@@ -1,0 +1,170 @@
+"""Lays the two-pathway layers out for the C++ host side (csrc/host/layer.cpp): which parameters and operands a layer's forward
+and backward pass take, formed once and kept on the layer until one of them changes.
+
+A layer is served here when it is what the builders make: bf16 activations on the GPU, nn.Linear projections with bf16 weights or
+Fp8Linear ones throughout, LayerNorms with parameters, the fused attention.  Everything else (adapters, wrapped projections, mixed
+kinds) stays on the modules' own path.
+"""
+from __future__ import annotations
+
+from typing import Optional
+
+import torch
+from torch import nn
+
+from . import _lib as L
+from . import ops
+
+
+class _Plan:
+    """The native plan of a layer and what it was made from: `slots` are (dict, key, object) that must still hold that object,
+    `tensors` (tensor, address, version) whose contents were copied into an operand."""
+
+    __slots__ = ("native", "slots", "tensors", "can_grad", "x_scale", "rot")
+
+    def valid(self) -> bool:
+        for d, k, o in self.slots:
+            if d.get(k) is not o:
+                return False
+        for t, p, v in self.tensors:
+            if t._version != v or t.data_ptr() != p:
+                return False
+        return True
+
+    # copies of a model lay their layers out themselves
+    def __deepcopy__(self, memo):
+        return None
+
+    def __reduce__(self):
+        return type(None), ()
+
+
+_ATTN_CHILDREN = ("q_proj", "k_proj", "v_proj", "fused_qkv", "out_proj", "rot_emb")
+
+
+def _attn_mods(attn):
+    fused = attn._modules.get("fused_qkv")
+    mods = [fused] if fused is not None else [attn._modules.get(n) for n in ("q_proj", "k_proj", "v_proj")]
+    return None if any(m is None for m in mods) else mods
+
+
+def _build(layer, mu: bool, keep: float, add: float) -> Optional[_Plan]:
+    from . import modules_plus as mp
+    from .mu_scaling import Fp8Linear, fused_fp8_weight
+    sa, ma, ff = layer.self_attn, layer.multimer_attn, layer.feed_forward
+    ms, mc = _attn_mods(sa), _attn_mods(ma)
+    if ms is None or mc is None or sa._modules.get("out_proj") is None:
+        return None
+    one = [sa.out_proj, ff.fc1, ff.fc2]
+    linears = ms + mc + one
+    fp8 = type(linears[0]) is Fp8Linear
+    if any(type(m) is not (Fp8Linear if fp8 else nn.Linear) for m in linears):
+        return None
+    for mods in (ms, mc):
+        if len({m.bias is None for m in mods}) != 1 or len({m.weight.dtype for m in mods}) != 1:
+            return None
+    norms = [layer.final_layer_norm] if mu else [layer.self_attn_layer_norm, layer.final_layer_norm]
+    params_dt = (torch.bfloat16, torch.float32)
+    if any(type(n) is not nn.LayerNorm or n.weight is None or n.weight.dtype not in params_dt for n in norms):
+        return None
+    if any(m.weight.dtype not in ((torch.bfloat16,) if not fp8 else params_dt) or not m.weight.is_cuda or not m.weight.is_contiguous()
+           or (m.bias is not None and (m.bias.dtype not in params_dt or not m.bias.is_contiguous())) for m in linears):
+        return None
+    E, H = sa.embed_dim, sa.num_heads
+    bias_s, bias_c = ms[0].bias is not None, mc[0].bias is not None
+
+    p = _Plan()
+    p.slots, p.tensors = [], []
+    for m, names in ((layer, ("self_attn", "multimer_attn", "feed_forward", "final_layer_norm") + (() if mu else ("self_attn_layer_norm",))),
+                     (sa, _ATTN_CHILDREN), (ma, _ATTN_CHILDREN), (ff, ("fc1", "fc2"))):
+        p.slots += [(m._modules, n, m._modules.get(n)) for n in names]
+    for m in linears + norms:
+        p.slots += [(m._parameters, "weight", m._parameters.get("weight")), (m._parameters, "bias", m._parameters.get("bias"))]
+
+    def watch(t):
+        if t is not None:
+            p.tensors.append((t, t.data_ptr(), t._version))
+
+    with torch.no_grad():
+        qkv6 = bias6 = b_self = b_cross = None
+        if fp8:
+            f8s, f8c = fused_fp8_weight(sa, ms), fused_fp8_weight(ma, mc)
+            if f8s[2] != f8c[2]:
+                return None          # one cast of the input serves both products
+            holders = [f8s[4], one[0].grad_scale, one[1].grad_scale, one[2].grad_scale]
+            p.can_grad = all(m.fp8_grads for m in linears)
+            op_s = L.host().Operand(f8s[0], f8s[1], f8s[2], f8s[3], holders[0])
+            op_c = L.host().Operand(f8c[0], f8c[1], f8c[2], f8c[3])
+            wq = [m._quantized_weight() for m in one]
+            o, f1, f2 = (L.host().Operand(w, s, m.x_scale, m.out_scale, h) for (w, s), m, h in zip(wq, one, holders[1:]))
+            for m in linears:
+                watch(m.weight)
+                p.slots += [(m.__dict__, k, m.__dict__.get(k)) for k in ("_wq", "x_scale", "out_scale", "fp8_grads", "grad_scale")]
+            p.slots += [(h.__dict__, "scale", h.scale) for h in holders if h is not None]
+            p.slots += [(a.__dict__, "_fp8_qkv_grad_scale", a.__dict__.get("_fp8_qkv_grad_scale")) for a in (sa, ma)]
+            w_s, w_c = f8s[0], f8c[0]
+            p.x_scale = f8s[2]
+        else:
+            p.can_grad, p.x_scale = True, 0.0
+            w_s, w_c = ((m[0].weight.detach() if len(m) == 1 else None) for m in (ms, mc))
+            if w_s is None or w_c is None or 12 * E * E <= mp._QKV6_MAX_BYTES:
+                for m in ms + mc:
+                    watch(m.weight)
+        if mp.FUSE_QKV6 and 6 * E * E * (1 if fp8 else 2) <= mp._QKV6_MAX_BYTES and bias_s == bias_c:
+            # both pathways' projections as one product that reads x once; a larger [6E][E] operand pushes the activation rows out
+            # of L2 between column tiles (measured slower)
+            if fp8:
+                qkv6 = torch.cat([w_s.view(torch.uint8), w_c.view(torch.uint8)]).view(torch.float8_e4m3fn)
+            else:
+                qkv6 = torch.cat([m.weight.detach() for m in ms + mc])
+            w_s, w_c = qkv6[:3 * E], qkv6[3 * E:]
+            if bias_s:
+                bias6 = torch.cat([m.bias.detach().float() for m in ms + mc])
+        elif not fp8:
+            w_s = torch.cat([m.weight.detach() for m in ms]) if w_s is None else w_s
+            w_c = torch.cat([m.weight.detach() for m in mc]) if w_c is None else w_c
+        if qkv6 is None:
+            b_self = (ms[0].bias.detach() if len(ms) == 1 else torch.cat([m.bias.detach() for m in ms])) if bias_s else None
+            b_cross = (mc[0].bias.detach() if len(mc) == 1 else torch.cat([m.bias.detach() for m in mc])) if bias_c else None
+        for m in ms + mc:
+            watch(m.bias)
+        if not fp8:
+            op_s, op_c = L.host().Operand(w_s), L.host().Operand(w_c)
+            o, f1, f2 = (L.host().Operand(m.weight) for m in one)
+    params = [m.weight for m in ms] + [m.bias for m in ms] + [m.weight for m in mc] + [m.bias for m in mc]
+    for m in one + norms:
+        params += [m.weight, m.bias]
+    p.native = L.host().LayerPlan(mu=mu, fp8=fp8, sqrt_softmax=bool(layer._use_sqrt_softmax), H=H, D=sa.head_dim, scale=sa.scaling, keep=keep, add=add,
+                                  eps1=norms[0].eps, eps2=norms[-1].eps, params=params, n_self=len(ms), n_cross=len(mc), qkv_self=op_s, qkv_cross=op_c,
+                                  out=o, fc1=f1, fc2=f2, qkv6=qkv6, bias6=bias6, bias_self=b_self, bias_cross=b_cross)
+    p.slots += [(layer.__dict__, k, layer.__dict__.get(k)) for k in ("_use_sqrt_softmax", "_tau_f")]
+    p.rot = sa.rot_emb
+    return p
+
+
+def run_layer(layer, x, chain_mask, padding_mask, chain_ids, pack, *, mu: bool, keep: float, add: float, next_quant=None):
+    """The layer's result for x (T,B,E) (or the packed rows of one), or None when the layer is not served here."""
+    from . import modules_plus as mp
+    if not (x.is_cuda and x.dtype == torch.bfloat16 and layer.use_multimer and layer._use_fused_multi_pathway and mp.FUSE_OUT_RESIDUAL):
+        return None
+    plan = layer.__dict__.get("_native_plan")
+    if plan is None or not plan.valid():
+        if layer.self_attn.head_dim not in (16, 32, 64):
+            return None
+        plan = _build(layer, mu, keep, add)
+        layer.__dict__["_native_plan"] = plan
+        if plan is None:
+            return None
+    if not plan.can_grad and torch.is_grad_enabled():
+        return None
+    T, B = (pack.T, pack.B) if pack is not None else (x.shape[0], x.shape[1])
+    meta = mp._cached_ids_meta(chain_ids, padding_mask) if chain_ids is not None and chain_mask is None else ops.cached_mask_meta(chain_mask, padding_mask)
+    cos = sin = None
+    if plan.rot is not None:
+        cos, sin, _ = ops.rope_tables(T, layer.self_attn.head_dim, x.device, plan.rot.inv_freq)
+    xq = ops.attached_e4m3(x, plan.x_scale) if mu and plan.x_scale else None
+    rows = (pack.rows32, pack.rows64, pack.inv32) if pack is not None else (None, None, None)
+    y, q8 = plan.native.forward(x, xq, T, B, meta.buf, cos, sin, *rows, next_quant or 0.0)
+    if q8 is not None:
+        ops.attach_e4m3(y, q8, next_quant)
+    return y

@@ -51,14 +51,9 @@ def _workspace(nbytes: int, device) -> Optional[torch.Tensor]:
 
 
 # ----------------------------------------------------------------------------------------------- status word
-_status = {}
-
-
 def _dev_status(device) -> torch.Tensor:
-    key = torch.device(device).index
-    if key not in _status:
-        _status[key] = torch.zeros(1, dtype=torch.int32, device=device)
-    return _status[key]
+    device = torch.device(device)
+    return L.host().dev_status(torch.cuda.current_device() if device.index is None else device.index)
 
 
 def check_device_status(device=None) -> None:
@@ -91,16 +86,8 @@ def _key_pad_u8(key_padding_mask, B, T):
 
 def mask_meta_from_chain_ids(chain_ids: torch.Tensor, key_padding_mask: Optional[torch.Tensor] = None) -> MaskMeta:
     """chain_ids (B,T) integer; key_padding_mask (B,T) bool, True = padded key (esm2.py:85,89)."""
-    _require_cuda(chain_ids, key_padding_mask)
     B, T = chain_ids.shape
-    cid = (chain_ids if chain_ids.dtype in (torch.int32, torch.int64) else chain_ids.to(torch.int32)).contiguous()
-    pad = _key_pad_u8(key_padding_mask, B, T)
-    lib = L.lib()
-    build = lib.mintb_mask_meta_from_chain_ids64 if cid.dtype == torch.int64 else lib.mintb_mask_meta_from_chain_ids
-    buf = torch.empty(lib.mintb_mask_meta_bytes(B, T), dtype=torch.uint8, device=cid.device)
-    with _on(cid.device):
-        L.check(build(_ptr(cid), _ptr(pad), _ptr(buf), B, T, _stream()), "mask_meta_from_chain_ids")
-    return MaskMeta(buf, B, T)
+    return MaskMeta(L.host().mask_meta(chain_ids, key_padding_mask), B, T)
 
 
 def mask_meta_from_mask(chain_mask: torch.Tensor, key_padding_mask: Optional[torch.Tensor] = None) -> MaskMeta:
@@ -278,11 +265,10 @@ def multimer_attention(q_self, k_self, v_self, q_cross, k_cross, v_cross, *, met
     The mask comes from exactly one of `meta`, `chain_ids` (B,T) or `chain_mask` (B,T,T).
     """
     ts = (q_self, k_self, v_self, q_cross, k_cross, v_cross)
-    _require_cuda(*ts)
-    if q_self.dim() != 4 or any(t.shape != q_self.shape for t in ts):
+    if not q_self.is_cuda:
+        _require_cuda(*ts)
+    if q_self.dim() != 4:
         raise ValueError("q/k/v of both pathways must share one (B, H, T, D) shape")
-    if q_self.dtype not in _DTYPES or any(t.dtype != q_self.dtype for t in ts):
-        raise TypeError("q/k/v must all be float32 or all be bfloat16")
     B, H, T, D = q_self.shape
     if meta is None:
         if (chain_ids is None) == (chain_mask is None):
@@ -291,7 +277,7 @@ def multimer_attention(q_self, k_self, v_self, q_cross, k_cross, v_cross, *, met
             else cached_mask_meta(chain_mask, key_padding_mask)
     elif chain_ids is not None or chain_mask is not None or key_padding_mask is not None:
         raise ValueError("meta already carries the chain and padding masks")
-    if (meta.B, meta.T) != (B, T):
+    if meta.B != B or meta.T != T:
         raise ValueError(f"mask metadata is for (B, T) = ({meta.B}, {meta.T}), tensors have ({B}, {T})")
     flags = ((L.FLAG_ROPE if rope else 0) | (L.FLAG_SQRT_SOFTMAX if sqrt_softmax else 0) | (L.FLAG_FORCE_SIMT if force_simt else 0)
              | (L.FLAG_OUT_SEQ_FIRST if out_seq_first else 0) | (L.FLAG_SKIP_PAD_QUERIES if skip_pad_queries else 0))
@@ -300,42 +286,15 @@ def multimer_attention(q_self, k_self, v_self, q_cross, k_cross, v_cross, *, met
         cos, sin, _ = rope_tables(T, D, q_self.device, inv_freq)
     if scale is None:
         scale = D ** -0.5
-    ts = tuple(t.contiguous() for t in ts)
-    if grad_rowmajor_tabs is not None and (rope or force_simt or q_self.dtype != torch.bfloat16 or D not in (16, 32, 64)):
-        grad_rowmajor_tabs = None      # served by the bf16 tensor-core kernels on pre-rotated inputs only
-    return _MultimerAttentionFn.apply(*ts, meta, cos, sin, float(scale), int(flags), grad_rowmajor_tabs)
+    if grad_rowmajor_tabs is not None and not rope and not force_simt and q_self.dtype == torch.bfloat16 and D in (16, 32, 64):
+        # served by the bf16 tensor-core kernels on pre-rotated inputs only
+        if any(t.shape != q_self.shape for t in ts):
+            raise ValueError("q/k/v of both pathways must share one (B, H, T, D) shape")
+        return _MultimerAttentionFn.apply(*(t.contiguous() for t in ts), meta, cos, sin, float(scale), int(flags), grad_rowmajor_tabs)
+    return L.host().attention(*ts, meta.buf, cos, sin, scale, flags)
 
 
 # ----------------------------------------------------------------------------------------------- combine from logits
-class _CombineFn(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, il, el, mask_u8, iv, ev):
-        B, H, T, D = iv.shape
-        out = torch.empty_like(iv)
-        with _on(iv.device):
-            rc = L.lib().mintb_combine_fwd(_ptr(il), _ptr(el), _ptr(mask_u8), _ptr(iv), _ptr(ev), _ptr(out), B, H, T, D,
-                                          _DTYPES[iv.dtype], _stream())
-        L.check(rc, "mintb_combine_fwd")
-        ctx.save_for_backward(il, el, mask_u8, iv, ev)
-        return out
-
-    @staticmethod
-    def backward(ctx, d_out):
-        il, el, mask_u8, iv, ev = ctx.saved_tensors
-        B, H, T, D = iv.shape
-        d_out = d_out.contiguous()
-        d_il, d_el, d_iv, d_ev = torch.empty_like(il), torch.empty_like(el), torch.empty_like(iv), torch.empty_like(ev)
-        lib = L.lib()
-        ws_bytes = lib.mintb_combine_bwd_workspace_bytes(B, H, T)
-        ws = _workspace(ws_bytes, iv.device)
-        with _on(iv.device):
-            rc = lib.mintb_combine_bwd(_ptr(il), _ptr(el), _ptr(mask_u8), _ptr(iv), _ptr(ev), _ptr(d_out), _ptr(d_il),
-                                       _ptr(d_el), _ptr(d_iv), _ptr(d_ev), _ptr(ws), ws_bytes, B, H, T, D,
-                                       _DTYPES[iv.dtype], _stream())
-        L.check(rc, "mintb_combine_bwd")
-        return d_il, d_el, None, d_iv, d_ev
-
-
 def multimer_combine(intra_logits, inter_logits, chain_mask, intra_values, inter_values) -> torch.Tensor:
     """Combine from materialised (B,H,T,T) logits (kernels/__init__.py:179-242 of the reference); differentiable."""
     ts = (intra_logits, inter_logits, intra_values, inter_values)
@@ -347,8 +306,7 @@ def multimer_combine(intra_logits, inter_logits, chain_mask, intra_values, inter
     if intra_values.dtype not in _DTYPES or any(t.dtype != intra_values.dtype for t in ts):
         raise TypeError("logits and values must all be float32 or all be bfloat16")
     m = chain_mask.contiguous().view(torch.uint8) if chain_mask.dtype == torch.bool else chain_mask.to(torch.uint8).contiguous()
-    return _CombineFn.apply(intra_logits.contiguous(), inter_logits.contiguous(), m, intra_values.contiguous(),
-                            inter_values.contiguous())
+    return L.host().combine(intra_logits, inter_logits, m, intra_values, inter_values)
 
 
 # ----------------------------------------------------------------------------------------------- projection GEMMs
@@ -395,12 +353,20 @@ def attach_e4m3(t: torch.Tensor, q8: torch.Tensor, scale: float) -> None:
     t._mintb_e4m3 = (q8, float(scale), t._version)
 
 
+def attached_e4m3(t: torch.Tensor, scale: float) -> Optional[torch.Tensor]:
+    """The copy attached to `t` when there is one with this scale and `t` has not been written since, else None."""
+    hit = t.__dict__.get("_mintb_e4m3")
+    if hit is not None and hit[1] == scale and hit[2] == t._version and hit[0].numel() == t.numel():
+        return hit[0]
+    return None
+
+
 def e4m3_of(t: torch.Tensor, scale: float) -> torch.Tensor:
     """The e4m3 operand of a projection that reads the (rows, E) view of `t`: the copy attached by the pass that produced `t`
     when there is one with this scale and `t` has not been written since, else a cast pass."""
-    hit = getattr(t, "_mintb_e4m3", None)
-    if hit is not None and hit[1] == float(scale) and hit[2] == t._version and hit[0].numel() == t.numel():
-        return hit[0].view(-1, t.shape[-1])
+    hit = attached_e4m3(t, float(scale))
+    if hit is not None:
+        return hit.view(-1, t.shape[-1])
     return quantize_e4m3(t.reshape(-1, t.shape[-1]), scale)
 
 
@@ -590,26 +556,6 @@ def _as_bf16(w: torch.Tensor) -> torch.Tensor:
     return (w if w.dtype == torch.bfloat16 else w.to(torch.bfloat16)).contiguous()
 
 
-class _LinearFn(torch.autograd.Function):
-    """y = act(x W^T + b) with the forward on the tcgen05 GEMM.  With GELU the pre-activation is written by the same GEMM
-    epilogue and kept for the backward pass."""
-
-    @staticmethod
-    def forward(ctx, x2d, w, bias, gelu):
-        wb = (w if w.dtype == torch.bfloat16 else w.to(torch.bfloat16)).contiguous()
-        keep = gelu and any(ctx.needs_input_grad[:3])
-        res = gemm_bf16(x2d, wb, bias, gelu, save_preact=keep)
-        out, z = res if keep else (res, None)
-        ctx.save_for_backward(x2d, w, bias, z)
-        return out
-
-    @staticmethod
-    def backward(ctx, dy):
-        x2d, w, bias, z = ctx.saved_tensors
-        dx, dw, db, _ = linear_backward(dy, x2d, w, bias, z, ctx.needs_input_grad)
-        return dx, dw, db, None
-
-
 class _LinearResFn(torch.autograd.Function):
     """s = a r + b (x W^T + bias) with the residual sum formed in the GEMM epilogue (bf16 operands); optionally also the e4m3
     copy of s for the projection that reads it next (second output, not differentiable)."""
@@ -695,9 +641,8 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias=None, gelu: bool = False)
     """nn.Linear forward (optionally followed by erf-GELU) for bf16 CUDA activations; differentiable."""
     if x.dtype != torch.bfloat16:
         raise TypeError("ops.linear takes bfloat16 activations")
-    x2d = x.reshape(-1, x.shape[-1]).contiguous()
-    y = _LinearFn.apply(x2d, weight, bias, gelu)
-    return y.view(*x.shape[:-1], weight.shape[0])
+    _require_cuda(x, weight, bias)
+    return L.host().linear(x, weight, bias, gelu)
 
 
 # ----------------------------------------------------------------------------------------------- variable-length packing
@@ -717,61 +662,6 @@ class PackInfo:
 
 
 # ----------------------------------------------------------------------------------------------- residual + LayerNorm
-class _AddLayerNormFn(torch.autograd.Function):
-    """(s, y) with s = a x + b r and y = LayerNorm(s) gamma + beta, in one pass over x and r; `need_s` False drops s,
-    gamma None drops the normalisation (then only s).  Replaces the residual add + LayerNorm pairs of the layers."""
-
-    @staticmethod
-    def forward(ctx, x, r, a, b, gamma, beta, eps, need_s, quant_scale=None):
-        E = x.shape[-1]
-        x2 = x.reshape(-1, E).contiguous()
-        r2 = r.reshape(-1, E).contiguous() if r is not None else None
-        rows = x2.shape[0]
-        norm = gamma is not None
-        s = torch.empty_like(x2) if (need_s or not norm) else None
-        y = torch.empty_like(x2) if norm else None
-        stats = torch.empty(rows, 2, dtype=torch.float32, device=x.device) if norm else None
-        pdt = _BIAS_DT[gamma.dtype] if norm else L.F32
-        # the e4m3 copy of the main result for the e4m3 projection that consumes it next (same values as quantize_e4m3)
-        q8 = torch.empty(rows, E, dtype=torch.float8_e4m3fn, device=x.device) if quant_scale else None
-        with _on(x.device):
-            rc = L.lib().mintb_add_layernorm_fwd_q(_ptr(x2), _ptr(r2), float(a), float(b), _ptr(gamma), _ptr(beta), pdt, _ptr(s), _ptr(y),
-                                                   _ptr(stats), rows, E, float(eps), _ptr(q8),
-                                                   1.0 / quant_scale if quant_scale else 1.0, _stream())
-        L.check(rc, "mintb_add_layernorm_fwd")
-        ctx.save_for_backward(x2, r2, gamma, stats)
-        ctx.cfg = (float(a), float(b), x.shape, pdt, beta is not None)
-        ctx.mark_non_differentiable(*([q8] if q8 is not None else []))
-        return s.view(x.shape) if s is not None else None, y.view(x.shape) if y is not None else None, q8
-
-    @staticmethod
-    def backward(ctx, ds_in, dy, _dq8=None):
-        x2, r2, gamma, stats = ctx.saved_tensors
-        a, b, shape, pdt, has_beta = ctx.cfg
-        rows, E = x2.shape
-        norm = gamma is not None
-        if not norm and ds_in is None:
-            return (None,) * 9
-        dy2 = dy.reshape(rows, E).contiguous() if (norm and dy is not None) else None
-        if norm and dy2 is None:
-            dy2 = torch.zeros_like(x2)
-        ds2 = ds_in.reshape(rows, E).contiguous() if ds_in is not None else None
-        dx = torch.empty_like(x2)
-        dr = torch.empty_like(x2) if r2 is not None else None
-        want_pg = norm and (ctx.needs_input_grad[4] or ctx.needs_input_grad[5])   # frozen norm parameters: no sums at all
-        dgamma = torch.empty(E, dtype=torch.float32, device=x2.device) if want_pg else None
-        dbeta = torch.empty(E, dtype=torch.float32, device=x2.device) if want_pg else None
-        lib = L.lib()
-        wsb = lib.mintb_add_layernorm_bwd_workspace_bytes(rows, E) if want_pg else 0
-        ws = torch.empty(wsb, dtype=torch.uint8, device=x2.device) if wsb else None
-        with _on(x2.device):
-            rc = lib.mintb_add_layernorm_bwd(_ptr(dy2), _ptr(ds2), _ptr(x2), _ptr(r2), a, b, _ptr(gamma), pdt, _ptr(stats), _ptr(dx),
-                                             _ptr(dr), _ptr(dgamma), _ptr(dbeta), _ptr(ws), wsb, rows, E, _stream())
-        L.check(rc, "mintb_add_layernorm_bwd")
-        return (dx.view(shape), dr.view(shape) if dr is not None else None, None, None,
-                dgamma.to(gamma.dtype) if want_pg else None, dbeta.to(gamma.dtype) if (want_pg and has_beta) else None, None, None, None)
-
-
 def add_layernorm(x, r, a: float, b: float, norm: Optional[torch.nn.LayerNorm], need_s: bool = True,
                   quant_scale: Optional[float] = None):
     """(s, y): s = a x + b r (r may be None), y = norm(s).  bf16 CUDA tensors; `norm` None returns (s, None).
@@ -781,9 +671,9 @@ def add_layernorm(x, r, a: float, b: float, norm: Optional[torch.nn.LayerNorm], 
     if x.dtype != torch.bfloat16 or not x.is_cuda:
         raise TypeError("add_layernorm takes bfloat16 CUDA tensors")
     if norm is None:
-        s, y, q8 = _AddLayerNormFn.apply(x, r, a, b, None, None, 0.0, True, quant_scale)
+        s, y, q8 = L.host().add_layernorm(x, r, a, b, None, None, 0.0, True, quant_scale or 0.0)
     else:
-        s, y, q8 = _AddLayerNormFn.apply(x, r, a, b, norm.weight, norm.bias, norm.eps, need_s, quant_scale)
+        s, y, q8 = L.host().add_layernorm(x, r, a, b, norm.weight, norm.bias, norm.eps, need_s, quant_scale or 0.0)
     if q8 is not None:
         attach_e4m3(y if y is not None else s, q8, quant_scale)
     return s, y
@@ -1090,38 +980,6 @@ def qkv_project(x: torch.Tensor, weight: torch.Tensor, bias, num_heads: int, rop
 
 
 # ----------------------------------------------------------------------------------------------- model prologue / epilogue
-class _EmbedFn(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, tokens, weight, pad_idx, mask_idx, token_dropout, mask_ratio_train):
-        B, T = tokens.shape
-        V, E = weight.shape
-        out = torch.empty(T, B, E, dtype=weight.dtype, device=weight.device)
-        scales = torch.empty(B, dtype=torch.float32, device=weight.device)
-        w = weight.contiguous()
-        with _on(weight.device):
-            rc = L.lib().mintb_embed_fwd(_ptr(tokens), _ptr(w), _ptr(out), _ptr(scales), B, T, E, V, _DTYPES[weight.dtype], int(pad_idx),
-                                         int(mask_idx), int(bool(token_dropout)), float(mask_ratio_train), _stream())
-        L.check(rc, "mintb_embed_fwd")
-        ctx.save_for_backward(tokens, scales)
-        ctx.cfg = (V, E, weight.dtype, int(pad_idx), int(mask_idx), int(bool(token_dropout)))
-        return out
-
-    @staticmethod
-    def backward(ctx, d_out):
-        tokens, scales = ctx.saved_tensors
-        V, E, dt, pad_idx, mask_idx, td = ctx.cfg
-        B, T = tokens.shape
-        d_out = d_out.contiguous()
-        if d_out.data_ptr() % 16:        # a view off the kernel's alignment
-            d_out = d_out.clone()
-        dw = torch.empty(V, E, dtype=torch.float32, device=d_out.device)
-        with _on(d_out.device):
-            rc = L.lib().mintb_embed_bwd(_ptr(tokens), _ptr(d_out), _ptr(scales), _ptr(dw), B, T, E, V, _DTYPES[dt], pad_idx, mask_idx, td,
-                                         _stream())
-        L.check(rc, "mintb_embed_bwd")
-        return None, dw.to(dt), None, None, None, None
-
-
 def embed_tokens(tokens: torch.Tensor, weight: torch.Tensor, pad_idx: int, mask_idx: int, token_dropout: bool,
                  mask_ratio_train: float = 0.12) -> torch.Tensor:
     """The model's prologue in one pass (esm2.py:91-104 of the reference): x = W[tokens]; under token dropout <mask> rows are
@@ -1131,33 +989,7 @@ def embed_tokens(tokens: torch.Tensor, weight: torch.Tensor, pad_idx: int, mask_
     _require_cuda(tokens, weight)
     if tokens.dtype != torch.int64 or tokens.dim() != 2 or weight.dtype not in _DTYPES:
         raise TypeError("embed_tokens takes int64 tokens (B, T) and an fp32 or bf16 weight (V, E)")
-    return _EmbedFn.apply(tokens.contiguous(), weight, pad_idx, mask_idx, token_dropout, mask_ratio_train)
-
-
-class _MaskedCeFn(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, rows, targets, mask_u8, V):
-        N, ld = rows.shape[0], rows.stride(0)
-        lse = torch.empty(N, dtype=torch.float32, device=rows.device)
-        sums = torch.empty(2, dtype=torch.float32, device=rows.device)
-        with _on(rows.device):
-            rc = L.lib().mintb_masked_ce_fwd(_ptr(rows), _ptr(targets), _ptr(mask_u8), _ptr(lse), _ptr(sums), N, ld, V, _stream())
-        L.check(rc, "mintb_masked_ce_fwd")
-        ctx.save_for_backward(rows, targets, mask_u8, lse, sums)
-        ctx.V = V
-        return sums[0] / sums[1]
-
-    @staticmethod
-    def backward(ctx, g):
-        rows, targets, mask_u8, lse, sums = ctx.saved_tensors
-        N, ld = rows.shape[0], rows.stride(0)
-        d_pad = torch.empty(N, ld, dtype=torch.bfloat16, device=rows.device)
-        g32 = g.detach().to(torch.float32).reshape(1).contiguous()
-        with _on(rows.device):
-            rc = L.lib().mintb_masked_ce_bwd(_ptr(rows), _ptr(targets), _ptr(mask_u8), _ptr(lse), _ptr(sums), _ptr(g32), _ptr(d_pad), N, ld,
-                                             ctx.V, _stream())
-        L.check(rc, "mintb_masked_ce_bwd")
-        return d_pad[:, :rows.shape[1]], None, None, None
+    return L.host().embed(tokens.contiguous(), weight, pad_idx, mask_idx, bool(token_dropout), mask_ratio_train)
 
 
 def masked_cross_entropy(logits: torch.Tensor, targets: torch.Tensor, target_mask: torch.Tensor) -> torch.Tensor:
@@ -1168,14 +1000,4 @@ def masked_cross_entropy(logits: torch.Tensor, targets: torch.Tensor, target_mas
     _require_cuda(logits, targets, target_mask)
     if logits.dtype != torch.bfloat16 or logits.dim() != 3 or logits.stride(-1) != 1:
         raise TypeError("masked_cross_entropy takes bfloat16 logits (B, T, V) with a contiguous last dimension")
-    B, T, V = logits.shape
-    if logits.stride(0) == T * logits.stride(1):                         # rows in (B, T) order
-        rows = torch.as_strided(logits, (B * T, V), (logits.stride(1), 1), logits.storage_offset())
-        tg, mk = targets, target_mask
-    elif logits.stride(1) == B * logits.stride(0):                       # rows in (T, B) order: a transposed view
-        rows = torch.as_strided(logits, (T * B, V), (logits.stride(0), 1), logits.storage_offset())
-        tg, mk = targets.t(), target_mask.t()
-    else:
-        c = logits.contiguous()
-        rows, tg, mk = c.view(B * T, V), targets, target_mask
-    return _MaskedCeFn.apply(rows, tg.contiguous().view(-1), mk.contiguous().view(-1).to(torch.uint8), V)
+    return L.host().masked_ce(logits, targets, target_mask)

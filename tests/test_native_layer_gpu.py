@@ -1,0 +1,135 @@
+"""The layers as the C++ host side runs them (one autograd node over the launches) against the same layers composed from the
+operators: values, input and parameter gradients, for every kind of layer it serves; operands follow the parameters."""
+import copy
+
+import pytest
+import torch
+
+import mint_plus_b200 as M
+from mint_plus_b200 import modules_plus, native, ops
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+E, H = 128, 4
+
+
+def make_layer(kind):
+    torch.manual_seed(3)
+    if kind.startswith("mu"):
+        layer = M.TransformerLayer_MINT_mu(E, 4 * E, H, use_multimer=True, num_layers=4, use_sqrt_softmax=kind != "mu")
+    elif kind.startswith("plus"):
+        layer = M.TransformerLayer_MINT_plus(E, 4 * E, H, use_multimer=True)
+    else:
+        layer = M.TransformerLayer_MINT(E, 4 * E, H, use_multimer=True)
+    for n, p in layer.named_parameters():
+        if n.endswith("bias") or "norm" in n:
+            torch.nn.init.normal_(p, 1.0 if n.endswith("norm.weight") else 0.0, 0.1)
+    layer = layer.to(DEV).to(torch.bfloat16)
+    if kind.endswith("fp8"):
+        wrap = torch.nn.Module()
+        wrap.layers = torch.nn.ModuleList([layer])
+        M.apply_fp8_to_model(wrap)
+        for m in layer.modules():
+            if isinstance(m, M.Fp8Linear):
+                m.grad_scale.scale = 2.0 ** -12
+        layer.self_attn._fp8_qkv_grad_scale = ops.GradScale(2.0 ** -12)
+        layer.multimer_attn._fp8_qkv_grad_scale = ops.GradScale(2.0 ** -12)
+    return layer
+
+
+def batch(T, B, seed=0):
+    g = torch.Generator().manual_seed(seed)
+    x = torch.randn(T, B, E, generator=g).bfloat16().to(DEV)
+    ids = torch.zeros(B, T, dtype=torch.int64)
+    pad = torch.zeros(B, T, dtype=torch.bool)
+    for b in range(B):
+        ids[b, T // 3 + b:] = 1
+        pad[b, T - 2 * b - 1:] = b > 0
+    return x, ids.to(DEV), pad.to(DEV)
+
+
+def run(layer, x, ids, pad, gy, pack=None):
+    x = x.clone().requires_grad_(True)
+    layer.zero_grad()
+    y, _ = layer(x, self_attn_padding_mask=pad, chain_ids=ids, pack=pack)
+    y.backward(gy)
+    return [y.detach(), x.grad] + [p.grad.clone() for p in layer.parameters() if p.grad is not None]
+
+
+def close(a, b, tol):
+    assert len(a) == len(b)
+    for u, v in zip(a, b):
+        assert u.dtype == v.dtype and u.shape == v.shape
+        assert (u.float() - v.float()).norm() <= tol * (v.float().norm() + 1e-6)
+
+
+@pytest.mark.parametrize("kind,T,B,two_products", [("base", 70, 3, False), ("base", 129, 1, True), ("plus", 64, 2, False), ("plus", 200, 2, True), ("mu", 65, 2, False),
+                                                   ("mu_fp8", 130, 3, False), ("mu_fp8", 33, 1, True), ("base_fp8", 96, 2, False)])
+def test_layer_equals_the_composed_operators(kind, T, B, two_products, monkeypatch):
+    if two_products:
+        monkeypatch.setattr(modules_plus, "_QKV6_MAX_BYTES", 0)
+    layer = make_layer(kind)
+    x, ids, pad = batch(T, B)
+    gy = torch.randn(T, B, E, device=DEV, generator=torch.Generator(DEV).manual_seed(1)).bfloat16()
+    got = run(layer, x, ids, pad, gy)
+    assert layer._native_plan is not None
+    with torch.no_grad():
+        assert torch.equal(layer(x, self_attn_padding_mask=pad, chain_ids=ids)[0], got[0])
+    with monkeypatch.context() as m:
+        m.setattr(native, "run_layer", lambda *a, **k: None)
+        want = run(layer, x, ids, pad, gy)
+    ops.check_device_status()
+    close(got, want, 6e-2 if kind.endswith("fp8") else 1e-2)
+
+
+@pytest.mark.parametrize("kind", ["plus", "mu_fp8"])
+def test_packed_rows_equal_the_padded_grid(kind):
+    layer = make_layer(kind)
+    T, B = 140, 3
+    x, ids, pad = batch(T, B)
+    pack = ops.PackInfo(pad)
+    keep = ~pad.t().reshape(-1)
+    gy = torch.randn(T, B, E, device=DEV).bfloat16() * keep.view(T, B, 1)
+    want = run(layer, x, ids, pad, gy)
+    got = run(layer, x.view(T * B, E)[keep].unsqueeze(1), ids, pad, gy.view(T * B, E)[keep].unsqueeze(1), pack)
+    assert torch.equal(got[0].squeeze(1), want[0].view(T * B, E)[keep])
+    close(got[2:], want[2:], 2e-2)
+
+
+@pytest.mark.parametrize("kind", ["base", "mu_fp8"])
+def test_operands_follow_the_parameters(kind):
+    layer = make_layer(kind)
+    x, ids, pad = batch(80, 2)
+    kw = dict(self_attn_padding_mask=pad, chain_ids=ids)
+    with torch.no_grad():
+        first = layer(x, **kw)[0]
+        twin = copy.deepcopy(layer)
+        assert torch.equal(twin(x, **kw)[0], first)
+        for p in layer.parameters():
+            p.mul_(0.5)
+        changed = layer(x, **kw)[0]
+        for a, b in zip(twin.parameters(), layer.parameters()):
+            a.copy_(b)
+        assert not torch.equal(changed, first)
+        assert torch.equal(make_twin_value(twin, x, kw), changed)
+        layer.feed_forward.fc1 = copy.deepcopy(layer.feed_forward.fc1)          # a replaced module
+        layer.feed_forward.fc1.weight.zero_()
+        assert not torch.equal(layer(x, **kw)[0], changed)
+
+
+def make_twin_value(twin, x, kw):
+    twin.__dict__["_native_plan"] = None
+    return twin(x, **kw)[0]
+
+
+def test_checkpointed_layer_gives_the_same_gradients():
+    from torch.utils.checkpoint import checkpoint
+    layer = make_layer("plus")
+    x, ids, pad = batch(100, 2)
+    gy = torch.randn(100, 2, E, device=DEV).bfloat16()
+    want = run(layer, x, ids, pad, gy)
+    xr = x.clone().requires_grad_(True)
+    layer.zero_grad()
+    y, _ = checkpoint(layer, xr, use_reentrant=False, self_attn_padding_mask=pad, chain_ids=ids)
+    y.backward(gy)
+    close([y.detach(), xr.grad] + [p.grad for p in layer.parameters()], want, 1e-3)
