@@ -220,6 +220,10 @@ MINTB_API int mintb_quantize_e4m3(const void* x, void* out, size_t n, float inv_
 MINTB_API int mintb_linear_res_fwd(const void* x, const void* w, const void* bias, const void* resid, float res_a, float res_b,
                                    void* out, void* bf16_copy_out, int M, int N, int K, int in_dtype, int bias_dtype,
                                    int out_dtype, float alpha, float out_scale, void* stream, int* dev_status);
+/* mintb_linear_res_fwd whose projection is, with round_first, rounded to bf16 before it enters the sum */
+MINTB_API int mintb_linear_add_fwd(const void* x, const void* w, const void* bias, const void* resid, float res_a, float res_b,
+                                   int round_first, void* out, void* bf16_copy_out, int M, int N, int K, int in_dtype, int bias_dtype,
+                                   int out_dtype, float alpha, float out_scale, void* stream, int* dev_status);
 MINTB_API int mintb_qkv2_fwd(const void* x, const void* w, const void* bias, void* q1, void* k1, void* v1, void* q2, void* k2,
                              void* v2, int T, int B, int H, int D, int in_dtype, int bias_dtype, float alpha1, float alpha2,
                              float q_scale, const float* rope_cos, const float* rope_sin, const int32_t* row_map, int n_rows,
@@ -240,6 +244,10 @@ MINTB_API int mintb_qkv2_fwd(const void* x, const void* w, const void* bias, voi
  */
 MINTB_API int mintb_linear_dgrad(const void* dz, const void* w, const void* dz2, const void* w2, void* dx, int M, int N, int K,
                                  int N2, int dz_dtype, int w_dtype, float alpha, void* stream, int* dev_status);
+/* mintb_linear_dgrad with a scaled matrix added in the epilogue: dx = alpha (dz w + dz2 w2) + beta resid[M][K], each term rounded
+ * to bf16 before the sum */
+MINTB_API int mintb_linear_dgrad_res(const void* dz, const void* w, const void* dz2, const void* w2, void* dx, const void* resid, float beta,
+                                     int M, int N, int K, int N2, int dz_dtype, int w_dtype, float alpha, void* stream, int* dev_status);
 MINTB_API size_t mintb_linear_wgrad_workspace_bytes(int N, int K, int out_dtype);
 MINTB_API int mintb_linear_wgrad(const void* dz, const void* x, void* dw, void* workspace, size_t workspace_bytes, int M, int N,
                                  int K, int dz_dtype, int x_dtype, int out_dtype, float alpha, void* stream, int* dev_status);
@@ -276,6 +284,17 @@ MINTB_API size_t mintb_add_layernorm_bwd_workspace_bytes(int rows, int E);
 MINTB_API int mintb_add_layernorm_bwd(const void* dy, const void* ds_in, const void* x, const void* r, float a, float b,
                                       const void* gamma, int param_dtype, const float* stats, void* dx, void* dr, float* dgamma,
                                       float* dbeta, void* workspace, size_t workspace_bytes, int rows, int E, void* stream);
+/* mintb_add_layernorm_bwd with dgamma and dbeta written as `grad_dtype` (f32 or bf16); ds_apart: ds_in is another gradient of the
+ * same input, added to dx = a ds after that has been rounded to bf16 (dr does not see it) */
+MINTB_API int mintb_add_layernorm_bwd_typed(const void* dy, const void* ds_in, int ds_apart, const void* x, const void* r, float a, float b,
+                                            const void* gamma, int param_dtype, const float* stats, void* dx, void* dr, void* dgamma,
+                                            void* dbeta, int grad_dtype, void* workspace, size_t workspace_bytes, int rows, int E,
+                                            void* stream);
+/* mintb_gelu_bwd_colsum / _f8 (dz or dz_e5m2, as there) with the column sums written as `db_dtype` (f32 or bf16), added in a
+ * fixed order over the workspace: no clearing pass, no conversion pass, the same bits every time */
+MINTB_API size_t mintb_bias_grad_workspace_bytes(int M, int N);
+MINTB_API int mintb_gelu_bwd_bias(const void* dy, const void* z, void* dz, void* db, int db_dtype, void* dz_e5m2, float e5m2_scale,
+                                  void* workspace, size_t workspace_bytes, int M, int N, void* stream);
 MINTB_API int mintb_gelu_bwd_colsum(const void* dy, const void* z, void* dz, float* db, int M, int N, void* stream);
 MINTB_API int mintb_gelu_bwd_colsum_act(const void* dy, const void* z, void* dz, void* act, float* db, int M, int N,
                                         void* stream);

@@ -46,8 +46,11 @@ PROTOTYPES = {
     "mintb_quantize_e4m3": (c_int, [_P, _P, c_size_t, c_float, _P]),
     "mintb_linear_res_fwd": (c_int, [_P, _P, _P, _P, c_float, c_float, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float,
                                      _P, _P]),
+    "mintb_linear_add_fwd": (c_int, [_P, _P, _P, _P, c_float, c_float, c_int, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float,
+                                     _P, _P]),
     "mintb_qkv2_fwd": (c_int, [_P] * 9 + [c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_float, _P, _P, _P, c_int, _P, _P]),
     "mintb_linear_dgrad": (c_int, [_P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_float, _P, _P]),
+    "mintb_linear_dgrad_res": (c_int, [_P, _P, _P, _P, _P, _P, c_float, c_int, c_int, c_int, c_int, c_int, c_int, c_float, _P, _P]),
     "mintb_linear_wgrad_workspace_bytes": (c_size_t, [c_int, c_int, c_int]),
     "mintb_linear_wgrad": (c_int, [_P, _P, _P, _P, c_size_t, c_int, c_int, c_int, c_int, c_int, c_int, c_float, _P, _P]),
     "mintb_add_layernorm_fwd": (c_int, [_P, _P, c_float, c_float, _P, _P, c_int, _P, _P, _P, c_int, c_int, c_float, _P]),
@@ -55,6 +58,10 @@ PROTOTYPES = {
     "mintb_add_layernorm_bwd_workspace_bytes": (c_size_t, [c_int, c_int]),
     "mintb_add_layernorm_bwd": (c_int, [_P, _P, _P, _P, c_float, c_float, _P, c_int, _P, _P, _P, _P, _P, _P, c_size_t, c_int,
                                         c_int, _P]),
+    "mintb_add_layernorm_bwd_typed": (c_int, [_P, _P, c_int, _P, _P, c_float, c_float, _P, c_int, _P, _P, _P, _P, _P, c_int, _P, c_size_t, c_int,
+                                              c_int, _P]),
+    "mintb_bias_grad_workspace_bytes": (c_size_t, [c_int, c_int]),
+    "mintb_gelu_bwd_bias": (c_int, [_P, _P, _P, _P, c_int, _P, c_float, _P, c_size_t, c_int, c_int, _P]),
     "mintb_gelu_bwd_colsum": (c_int, [_P, _P, _P, _P, c_int, c_int, _P]),
     "mintb_gelu_bwd_colsum_act": (c_int, [_P, _P, _P, _P, _P, c_int, c_int, _P]),
     "mintb_gelu_bwd_colsum_f8": (c_int, [_P, _P, _P, _P, _P, _P, c_float, c_int, c_int, _P]),

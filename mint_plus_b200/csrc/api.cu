@@ -21,33 +21,70 @@ static std::atomic<unsigned long long> g_launches{0};
 // the pool of work counters (see common.cuh); zero-initialised with the module, each pair cleared again by its last user
 static __device__ int g_tile_counters[2 * kTileCounterSlots];
 
-int next_tile_counter(int** out) {
-  constexpr int kMaxDevices = 64;
-  static std::atomic<unsigned> next{0};
-  static std::mutex mu;
-  static int* base[kMaxDevices] = {};
-  int dev = -1;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess || dev < 0 || dev >= kMaxDevices) {
+constexpr int kArrivalCounters = 1 << 16;
+static __device__ int g_arrivals[kArrivalCounters];
+
+// This thread's current device's address of a symbol of the library, looked up once per device.
+template <typename S>
+static int* device_base(S& symbol, std::atomic<int*>* cache, int n_cache) {
+  const int dev = current_device();
+  if (dev < 0 || dev >= n_cache) {
     set_error("work counters: cudaGetDevice failed or device index %d is out of range", dev);
-    return MINTB_ECUDA;
+    return nullptr;
   }
-  int* b = nullptr;
-  {
-    std::lock_guard<std::mutex> lock(mu);
-    if (base[dev] == nullptr) {   // the symbol's address differs per device; look it up once with that device current
-      void* ptr = nullptr;
-      e = cudaGetSymbolAddress(&ptr, g_tile_counters);
-      if (e != cudaSuccess || ptr == nullptr) {
-        set_error("work counters: cudaGetSymbolAddress failed: %s", cudaGetErrorString(e));
-        return MINTB_ECUDA;
-      }
-      base[dev] = static_cast<int*>(ptr);
+  int* b = cache[dev].load(std::memory_order_acquire);
+  if (b == nullptr) {
+    void* ptr = nullptr;
+    const cudaError_t e = cudaGetSymbolAddress(&ptr, symbol);
+    if (e != cudaSuccess || ptr == nullptr) {
+      set_error("work counters: cudaGetSymbolAddress failed: %s", cudaGetErrorString(e));
+      return nullptr;
     }
-    b = base[dev];
+    b = static_cast<int*>(ptr);
+    cache[dev].store(b, std::memory_order_release);
   }
+  return b;
+}
+
+int next_arrival_counters(int n, int** out) {
+  static std::atomic<unsigned> next{0};
+  static std::atomic<int*> base[64] = {};
+  if (n <= 0 || n > kArrivalCounters / 16) {
+    set_error("arrival counters: %d requested", n);
+    return MINTB_EUNSUPPORTED;
+  }
+  int* b = device_base(g_arrivals, base, 64);
+  if (b == nullptr) return MINTB_ECUDA;
+  unsigned at;
+  do at = next.fetch_add(unsigned(n), std::memory_order_relaxed) % kArrivalCounters; while (at + unsigned(n) > unsigned(kArrivalCounters));
+  *out = b + at;
+  return MINTB_OK;
+}
+
+int next_tile_counter(int** out) {
+  static std::atomic<unsigned> next{0};
+  static std::atomic<int*> base[64] = {};
+  int* b = device_base(g_tile_counters, base, 64);
+  if (b == nullptr) return MINTB_ECUDA;
   *out = b + 2 * (next.fetch_add(1, std::memory_order_relaxed) % kTileCounterSlots);
   return MINTB_OK;
+}
+
+int current_device() {
+  int dev = -1;
+  return cudaGetDevice(&dev) == cudaSuccess ? dev : -1;
+}
+
+int sm_count() {
+  static std::atomic<int> cached[64];
+  const int dev = current_device();
+  if (dev < 0 || dev >= 64) return 148;
+  int n = cached[dev].load(std::memory_order_relaxed);
+  if (n == 0) {
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+    cached[dev].store(n, std::memory_order_relaxed);
+  }
+  return n;
 }
 
 void count_launches(int n) { g_launches.fetch_add(static_cast<unsigned long long>(n), std::memory_order_relaxed); }

@@ -96,6 +96,7 @@ __global__ void __launch_bounds__(256) rope_rotate_kernel(const __nv_bfloat16* _
                                                           __nv_bfloat16* __restrict__ qr, __nv_bfloat16* __restrict__ kr,
                                                           const float* __restrict__ cos_tab, const float* __restrict__ sin_tab,
                                                           size_t rows, int T, int D) {
+  griddep_wait();
   griddep_launch();   // the attention kernel's set-up may overlap this pass
   const int h = D / 2, cpr = h / 8;  // chunks per row
   const size_t idx = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -283,7 +284,8 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  griddep_wait();   // the set-up above may overlap the rotation pass before this kernel; its copies are read from here on
+  griddep_wait();    // the set-up above may overlap the kernel before this one; what it wrote is read from here on
+  griddep_launch();  // (the next kernel's set-up may begin: this grid's tensor memory is allocated)
   const uint32_t tbase = *tmem_slot;
 
   if (warp == 0) {
@@ -797,8 +799,8 @@ static int fwd_tc_t(const AttnArgs& a, const void* q_s, const void* k_s) {
     set_error("mintb_attn_fwd: cuTensorMapEncodeTiled failed");
     return MINTB_ECUDA;
   }
-  {  // per device and cheap, so set on every call
-    cudaError_t e = cudaFuncSetAttribute(attn_fwd_tc_kernel<D, SQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(Cfg::kSmemBytes));
+  {
+    cudaError_t e = opt_in_smem<attn_fwd_tc_kernel<D, SQ>>(int(Cfg::kSmemBytes));
     if (e != cudaSuccess) { set_error("cudaFuncSetAttribute: %s", cudaGetErrorString(e)); return MINTB_ECUDA; }
   }
   int* sched = nullptr;   // the launch's work counter pair (common.cuh)
@@ -809,13 +811,7 @@ static int fwd_tc_t(const AttnArgs& a, const void* q_s, const void* k_s) {
   FwdParams p{a.meta.bits, a.meta.kpad, a.meta.cls, static_cast<__nv_bfloat16*>(a.out), a.lse, a.H, a.T, a.meta.TW, a.meta.NT,
               a.scale * kLog2e, a.dev_status, out_row_stride(a), out_bh_stride(a), a.skip_pad_queries ? 1 : 0,
               sched, NQ, int(n_items)};
-  static int n_ctas = 0;   // two persistent CTAs per SM
-  if (n_ctas == 0) {
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    n_ctas = 2 * (sms > 0 ? sms : 148);
-  }
+  const int n_ctas = 2 * sm_count();   // two persistent CTAs per SM
   const unsigned grid = unsigned(n_items < n_ctas ? n_items : n_ctas);
   cudaError_t e = launch_dependent(attn_fwd_tc_kernel<D, SQ>, dim3(grid), dim3(kTcThreads), Cfg::kSmemBytes, a.stream, mqs, mks, mvs, mqc, mkc, mvc, p);
   count_launches(1);
@@ -828,8 +824,8 @@ static int fwd_tc_t(const AttnArgs& a, const void* q_s, const void* k_s) {
 void launch_rope_rotate(const AttnArgs& a, __nv_bfloat16* qr, __nv_bfloat16* kr) {
   const size_t rows = size_t(a.B) * a.H * a.T;
   const size_t n = rows * (a.D / 16);
-  rope_rotate_kernel<<<unsigned((n + 255) / 256), 256, 0, a.stream>>>(
-      static_cast<const __nv_bfloat16*>(a.q_s), static_cast<const __nv_bfloat16*>(a.k_s), qr, kr, a.rope_cos, a.rope_sin, rows, a.T, a.D);
+  launch_dependent(rope_rotate_kernel, dim3(unsigned((n + 255) / 256)), dim3(256), 0, a.stream, static_cast<const __nv_bfloat16*>(a.q_s),
+                   static_cast<const __nv_bfloat16*>(a.k_s), qr, kr, a.rope_cos, a.rope_sin, rows, a.T, a.D);
   count_launches(1);
 }
 

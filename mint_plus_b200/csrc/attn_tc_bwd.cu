@@ -113,6 +113,7 @@ __global__ void __launch_bounds__(256) bwd_stats_kernel(const __nv_bfloat16* __r
                                                         const float* __restrict__ lse, float2* __restrict__ stats, int BH, int T,
                                                         int Tpad, int D, float factor, size_t row_stride, size_t bh_stride,
                                                         float* __restrict__ acc_s, float* __restrict__ acc_c) {
+  griddep_wait();
   griddep_launch();       // the main kernel's set-up may overlap this pass; it waits for it before it reads the statistics
   const int lpr = D / 8;  // lanes per row
   const size_t idx = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -813,7 +814,7 @@ static int bwd_tc_t(const AttnArgs& a, const void* q_s, const void* k_s, const f
     set_error("mintb_attn_bwd: cuTensorMapEncodeTiled failed for the dQ accumulators");
     return MINTB_ECUDA;
   }
-  cudaError_t e = cudaFuncSetAttribute(attn_bwd_tc_kernel<D, SQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(Cfg::kSmemBytes));
+  cudaError_t e = opt_in_smem<attn_bwd_tc_kernel<D, SQ>>(int(Cfg::kSmemBytes));
   if (e != cudaSuccess) { set_error("cudaFuncSetAttribute: %s", cudaGetErrorString(e)); return MINTB_ECUDA; }
   BwdParams p{};
   p.bitsT = a.meta.bitsT; p.kpad = a.meta.kpad; p.cls = a.meta.cls;
@@ -860,10 +861,8 @@ int launch_attn_bwd_tc(const AttnArgs& a) {
   {
     const int tpad = bwd_tpad(a.T);
     const size_t n = size_t(a.B) * a.H * tpad * (a.D / 8);
-    bwd_stats_kernel<<<unsigned((n + 255) / 256), 256, 0, a.stream>>>(static_cast<const __nv_bfloat16*>(a.out),
-                                                                     static_cast<const __nv_bfloat16*>(a.d_out), a.lse, stats,
-                                                                     a.B * a.H, a.T, tpad, a.D, a.sqrt_softmax ? 0.5f : 1.f, out_row_stride(a),
-                                                                     out_bh_stride(a), acc_s, acc_c);
+    launch_dependent(bwd_stats_kernel, dim3(unsigned((n + 255) / 256)), dim3(256), 0, a.stream, static_cast<const __nv_bfloat16*>(a.out),
+                     static_cast<const __nv_bfloat16*>(a.d_out), a.lse, stats, a.B * a.H, a.T, tpad, a.D, a.sqrt_softmax ? 0.5f : 1.f, out_row_stride(a), out_bh_stride(a), acc_s, acc_c);
     count_launches(1);
   }
   int rc = MINTB_EUNSUPPORTED;

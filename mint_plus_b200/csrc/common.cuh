@@ -6,6 +6,8 @@
 #include <stdint.h>
 #include <stddef.h>
 
+#include <atomic>
+
 #include "../../include/mintb.h"
 
 namespace mintb {
@@ -111,6 +113,18 @@ inline cudaError_t launch_dependent(void (*kern)(KArgs...), dim3 grid, dim3 bloc
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
 }
+// Lets `Kern` use `bytes` of dynamic shared memory on the current device; asks the driver once per device.
+int current_device();   // of the calling thread, or -1
+template <auto Kern>
+inline cudaError_t opt_in_smem(int bytes) {
+  static std::atomic<unsigned long long> done{0};
+  const int dev = current_device();
+  if (dev >= 0 && dev < 64 && ((done.load(std::memory_order_acquire) >> dev) & 1u)) return cudaSuccess;
+  const cudaError_t e = cudaFuncSetAttribute(Kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess && dev >= 0 && dev < 64) done.fetch_or(1ull << dev, std::memory_order_release);
+  return e;
+}
+int sm_count();         // of the current device
 void count_launches(int n);  // process-wide tally of kernels launched by this library
 
 // Work counters of the persistent kernels.  A launch takes the next {next unit, CTAs that have left} pair of a pool in the
@@ -120,6 +134,9 @@ void count_launches(int n);  // process-wide tally of kernels launched by this l
 constexpr int kTileCounterSlots = 4096;
 int next_tile_counter(int** out);      // MINTB_OK or an error code
 // (device side, in ptx.cuh: leave_tile_counter)
+// `n` neighbouring counters of a second pool of the same kind, for kernels whose last CTA of a group finishes the group's work: zero when
+// a launch gets them, cleared again by that CTA.
+int next_arrival_counters(int n, int** out);
 
 // api.cu
 int check_attn_args(AttnArgs& a, const char* who, const void* q_s, const void* k_s, const void* v_s, const void* q_c,

@@ -10,12 +10,13 @@
 // descriptor names the block stride, so tcgen05.mma reads the tile transposed.  Operands are bf16 (kind::f16) or 8-bit
 // floats (kind::f8f6f4: e5m2 gradients against e4m3 activations / weights), fp32 accumulation in TMEM.
 //
-// Persistent CTAs, one per SM, 128 x 256 output tiles, the roles of the forward GEMM: warp 0 TMA producer (4-stage ring of
-// 128-byte reduction slabs), warp 1 MMA issuer (two 256-column accumulators), warps 2-9 epilogue.  dgrad stores bf16 through
-// shared memory and bulk tensor stores.  wgrad reduces over the tokens, tens of thousands of them against a few hundred
-// output tiles, so its reduction is cut into S aligned splits (S chosen on the host so that tiles x S fills the SMs
-// evenly); every unit adds its fp32 partial tile to a zeroed fp32 matrix with bulk tensor reductions, and a small pass
-// converts that matrix when the gradient is wanted in bf16.  Units of one split run together, so the CTAs march through
+// Persistent CTAs, one per SM, 128 x BN output tiles (BN = 256, narrower where that leaves SMs idle), the roles of the forward
+// GEMM: warp 0 TMA producer (ring of 128-byte reduction slabs), warp 1 MMA issuer (two BN-column accumulators), warps 2-9
+// epilogue.  dgrad stores bf16 through shared memory and bulk tensor stores.  wgrad reduces over the tokens.  Few of them: a tile
+// per CTA over all of them, stored as the gradient wants it.  Tens of thousands against a few hundred output tiles: the
+// reduction is cut into S aligned splits (S chosen on the host so that tiles x S fills the SMs evenly); every unit adds its
+// fp32 partial tile to a zeroed fp32 matrix with bulk tensor reductions, and a small pass converts that matrix when the
+// gradient is wanted in bf16.  Units of one split run together, so the CTAs march through
 // the same token range at the same time and share their operand tiles in L2.  Every mbarrier wait is bounded.
 #include "common.cuh"
 #include "ptx.cuh"
@@ -24,12 +25,18 @@ namespace mintb {
 
 using namespace ptx;
 
-constexpr int kBM = 128, kBN = 256, kBStages = 4;
-constexpr int kBABytes = kBM * 128, kBBBytes = kBN * 128, kBStageBytes = kBABytes + kBBBytes;
+constexpr int kBM = 128;
+constexpr int kBABytes = kBM * 128;
 constexpr int kBEpiWarps = 8, kBEpiThreads = 32 * kBEpiWarps, kBThreads = 64 + kBEpiThreads;
 constexpr int kBOutStageBytes = 32 * 128;   // one epilogue warp's staging: 32 rows x 128 bytes
-constexpr size_t kBwdGemmSmem = 1024 + size_t(kBStages) * kBStageBytes + kBEpiWarps * kBOutStageBytes + 256;
+template <int BN>
+struct BwdGemmCfg {
+  static constexpr int kStages = BN == 256 ? 4 : BN == 128 ? 5 : 7;
+  static constexpr int kStageBytes = kBABytes + BN * 128;
+  static constexpr size_t kSmem = 1024 + size_t(kStages) * kStageBytes + kBEpiWarps * kBOutStageBytes + 256;
+};
 
+enum BwdGemmResult : int { kAddF32 = 0, kStoreF32 = 1, kStoreBf16 = 2 };   // what a unit of the reduction does with its tile
 enum BwdGemmMode : int { kDgrad = 0, kWgrad = 1 };
 
 struct BwdGemmParams {
@@ -39,7 +46,9 @@ struct BwdGemmParams {
   uint32_t idesc;        // instruction descriptor (formats, majors, M = 128, N = 256)
   int splits;            // aligned cuts of the reduction (wgrad); 1 for dgrad
   int n_full, pieces;    // the first n_full (split, tile) units run whole, the others in `pieces` aligned pieces (UnitMap)
-  float alpha;
+  int result;            // BwdGemmResult (dgrad: always kStoreBf16)
+  float alpha, beta;
+  const __nv_bfloat16* resid;   // dgrad: when non-null, beta * resid[rows][cols] is added to the result
   int* status;
   int* sched;            // work counter pair of this launch (common.cuh)
 };
@@ -92,11 +101,12 @@ struct UnitMap {
   }
 };
 
-template <int MODE>
+template <int MODE, int BN>
 __global__ void __launch_bounds__(kBThreads, 1)
 gemm_bwd_kernel(const __grid_constant__ CUtensorMap map_a1, const __grid_constant__ CUtensorMap map_b1,
                 const __grid_constant__ CUtensorMap map_a2, const __grid_constant__ CUtensorMap map_b2,
                 const __grid_constant__ CUtensorMap map_out, BwdGemmParams p) {
+  constexpr int kBN = BN, kBStages = BwdGemmCfg<BN>::kStages, kBStageBytes = BwdGemmCfg<BN>::kStageBytes;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   unsigned char* s_out = smem + size_t(kBStages) * kBStageBytes;   // [epilogue warp][32 rows][128 B]
@@ -124,10 +134,12 @@ gemm_bwd_kernel(const __grid_constant__ CUtensorMap map_a1, const __grid_constan
     for (int s = 0; s < kBUnitRing; ++s) { mbar_init(&ur_full[s], 1); mbar_init(&ur_empty[s], 1 + kBEpiWarps); }
     fence_mbar_init();
   }
-  if (warp == 1) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
+  if (warp == 1) { tmem_alloc(tmem_slot, 2 * BN); tmem_relinquish(); }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  griddep_wait();
+  griddep_launch();   // only now: see gemm_tc_kernel
   const uint32_t tbase = *tmem_slot;
 
   if (warp == 0) {
@@ -262,27 +274,48 @@ gemm_bwd_kernel(const __grid_constant__ CUtensorMap map_a1, const __grid_constan
         tmem_ld_wait();
         if (lane == 0) bulk_wait_read_all();   // the previous bulk operation of this warp has read the staging rows
         __syncwarp();
-        if (MODE == kDgrad) {
+        if (MODE == kDgrad && p.resid != nullptr && m0 + quarter * 32 + lane < p.rows) {
+          const __nv_bfloat16* rr = p.resid + size_t(m0 + quarter * 32 + lane) * p.cols + n0 + c0;
+#pragma unroll
+          for (int j = 0; j < 32; j += 8) {
+            if (n0 + c0 + j < p.cols) {   // (columns come in multiples of eight)
+              const uint4 q = __ldg(reinterpret_cast<const uint4*>(rr + j));
+              const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                // rounded like the two tensors whose sum this is
+                const auto sum = [&](uint32_t acc, float other) {
+                  return __float_as_uint(__bfloat162float(__float2bfloat16_rn(__uint_as_float(acc) * p.alpha)) +
+                                         __bfloat162float(__float2bfloat16_rn(p.beta * other)));
+                };
+                r[j + 2 * e] = sum(r[j + 2 * e], __uint_as_float(w[e] << 16));
+                r[j + 2 * e + 1] = sum(r[j + 2 * e + 1], __uint_as_float(w[e] & 0xffff0000u));
+              }
+            }
+          }
+        }
+        const float alpha = MODE == kDgrad && p.resid != nullptr ? 1.f : p.alpha;
+        if (MODE == kDgrad || p.result == kStoreBf16) {
           // 32 columns of this warp's 32 rows as bf16 -> shared memory (row = lane, 64-byte swizzle) -> one bulk tensor store
 #pragma unroll
           for (int j = 0; j < 32; j += 8)
             *reinterpret_cast<uint4*>(my_out + swizzled_offset(lane, j / 8, 64)) = make_uint4(
-                bwd_pack_bf16x2(__uint_as_float(r[j]) * p.alpha, __uint_as_float(r[j + 1]) * p.alpha),
-                bwd_pack_bf16x2(__uint_as_float(r[j + 2]) * p.alpha, __uint_as_float(r[j + 3]) * p.alpha),
-                bwd_pack_bf16x2(__uint_as_float(r[j + 4]) * p.alpha, __uint_as_float(r[j + 5]) * p.alpha),
-                bwd_pack_bf16x2(__uint_as_float(r[j + 6]) * p.alpha, __uint_as_float(r[j + 7]) * p.alpha));
+                bwd_pack_bf16x2(__uint_as_float(r[j]) * alpha, __uint_as_float(r[j + 1]) * alpha),
+                bwd_pack_bf16x2(__uint_as_float(r[j + 2]) * alpha, __uint_as_float(r[j + 3]) * alpha),
+                bwd_pack_bf16x2(__uint_as_float(r[j + 4]) * alpha, __uint_as_float(r[j + 5]) * alpha),
+                bwd_pack_bf16x2(__uint_as_float(r[j + 6]) * alpha, __uint_as_float(r[j + 7]) * alpha));
         } else {
-          // 32 fp32 columns (128-byte rows, 128-byte swizzle) -> one bulk tensor reduction into the fp32 matrix
+          // 32 fp32 columns (128-byte rows, 128-byte swizzle) -> one bulk tensor reduction into (or store to) the fp32 matrix
 #pragma unroll
           for (int j = 0; j < 32; j += 4)
             *reinterpret_cast<float4*>(my_out + swizzled_offset(lane, j / 4, 128)) =
-                make_float4(__uint_as_float(r[j]) * p.alpha, __uint_as_float(r[j + 1]) * p.alpha, __uint_as_float(r[j + 2]) * p.alpha,
-                            __uint_as_float(r[j + 3]) * p.alpha);
+                make_float4(__uint_as_float(r[j]) * alpha, __uint_as_float(r[j + 1]) * alpha, __uint_as_float(r[j + 2]) * alpha,
+                            __uint_as_float(r[j + 3]) * alpha);
         }
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) {
-          if (MODE == kDgrad) tma_store_2d(&map_out, my_out, n0 + c0, m0 + quarter * 32);
+          if (MODE == kDgrad || p.result != kAddF32) tma_store_2d(&map_out, my_out, n0 + c0, m0 + quarter * 32);
           else tma_reduce_add_2d(&map_out, my_out, n0 + c0, m0 + quarter * 32);
           bulk_commit_group();
         }
@@ -291,18 +324,20 @@ gemm_bwd_kernel(const __grid_constant__ CUtensorMap map_a1, const __grid_constan
       mbar_arrive(&acc_empty[ab]);
       if (++ab == 2) { ab = 0; ab_phase ^= 1; }
     }
-    if (lane == 0) bulk_wait_read_all();   // the bulk operations have read their staging rows (the kernel boundary orders their writes)
+    if (lane == 0) bulk_wait_all();   // (a dependent kernel may already be waiting for this grid)
   }
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {
     __syncwarp();
-    tmem_dealloc(tbase, 512);
+    tmem_dealloc(tbase, 2 * BN);
   }
 }
 
 // out[i] = bf16(acc[i]): the fp32 sum of the wgrad units as the bf16 gradient; 8 elements per thread.
 __global__ void __launch_bounds__(256) wgrad_convert_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ out, size_t n) {
+  griddep_wait();
+  griddep_launch();
   const size_t i = (size_t(blockIdx.x) * blockDim.x + threadIdx.x) * 8;
   if (i >= n) return;
   if (i + 8 <= n) {
@@ -357,33 +392,48 @@ static bool result_map(CUtensorMap* m, const void* ptr, int rows, int cols, bool
 }
 
 // kind::f16 / kind::f8f6f4 instruction descriptor: fp32 accumulate, operand formats (bf16: 1; e4m3: 0, e5m2: 1), majors, N, M
-static uint32_t bwd_idesc(int a_fmt, int b_fmt, bool a_mn, bool b_mn) {
+static uint32_t bwd_idesc(int a_fmt, int b_fmt, bool a_mn, bool b_mn, int bn) {
   return (1u << 4) | (uint32_t(a_fmt) << 7) | (uint32_t(b_fmt) << 10) | (uint32_t(a_mn) << 15) | (uint32_t(b_mn) << 16) |
-         (uint32_t(kBN >> 3) << 17) | (uint32_t(kBM >> 4) << 24);
-}
-
-static int sm_count() {
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return sms;
+         (uint32_t(bn >> 3) << 17) | (uint32_t(kBM >> 4) << 24);
 }
 
 static int fmt_code(int dtype) { return dtype == MINTB_E5M2 ? 1 : dtype == MINTB_E4M3 ? 0 : 1; }   // bf16 is code 1 of kind::f16
 static bool is_f8(int dtype) { return dtype == MINTB_E4M3 || dtype == MINTB_E5M2; }
 
-template <int MODE>
-static int launch_bwd_gemm(const CUtensorMap& a1, const CUtensorMap& b1, const CUtensorMap& a2, const CUtensorMap& b2,
-                           const CUtensorMap& out, const BwdGemmParams& p_in, int grid, cudaStream_t stream) {
-  cudaError_t e = cudaFuncSetAttribute(gemm_bwd_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kBwdGemmSmem));
+template <int MODE, int BN>
+static int launch_bwd_gemm_t(const CUtensorMap& a1, const CUtensorMap& b1, const CUtensorMap& a2, const CUtensorMap& b2, const CUtensorMap& out,
+                             BwdGemmParams& p, long long units, cudaStream_t stream) {
+  constexpr auto kern = gemm_bwd_kernel<MODE, BN>;
+  cudaError_t e = opt_in_smem<kern>(int(BwdGemmCfg<BN>::kSmem));
   if (e != cudaSuccess) { set_error("cudaFuncSetAttribute: %s", cudaGetErrorString(e)); return MINTB_ECUDA; }
-  BwdGemmParams p = p_in;
   if (int rc = next_tile_counter(&p.sched); rc != MINTB_OK) return rc;
-  gemm_bwd_kernel<MODE><<<grid, kBThreads, kBwdGemmSmem, stream>>>(a1, b1, a2, b2, out, p);
+  const int sms = sm_count();
+  e = launch_dependent(kern, dim3(unsigned(units < sms ? units : sms)), dim3(kBThreads), BwdGemmCfg<BN>::kSmem, stream, a1, b1, a2, b2, out, p);
   count_launches(1);
-  e = cudaGetLastError();
   if (e != cudaSuccess) { set_error("backward gemm launch: %s", cudaGetErrorString(e)); return MINTB_ECUDA; }
   return MINTB_OK;
+}
+template <int MODE>
+static int launch_bwd_gemm(int bn, const CUtensorMap& a1, const CUtensorMap& b1, const CUtensorMap& a2, const CUtensorMap& b2, const CUtensorMap& out,
+                           BwdGemmParams& p, long long units, cudaStream_t stream) {
+  return bn == 256 ? launch_bwd_gemm_t<MODE, 256>(a1, b1, a2, b2, out, p, units, stream)
+       : bn == 128 ? launch_bwd_gemm_t<MODE, 128>(a1, b1, a2, b2, out, p, units, stream)
+                   : launch_bwd_gemm_t<MODE, 64>(a1, b1, a2, b2, out, p, units, stream);
+}
+
+// Cycles of an uncut product on the busiest SM, as in the forward GEMM's pick_tile; 8-bit operands are loaded 128 columns at a time.
+static int pick_bwd_tile(int rows, int cols, int n_slabs, bool f8, int sms, long long* cost_out) {
+  const long long tm = (rows + kBM - 1) / kBM;
+  int best = 256;
+  long long best_cost = -1;
+  for (const int bn : {256, 128, 64}) {
+    if (bn == 64 && f8) break;
+    const long long rounds = (tm * ((cols + bn - 1) / bn) + sms - 1) / sms;
+    const long long cost = rounds * n_slabs * (bn == 256 ? 512 : bn == 128 ? 280 : 200) + 1500 + 8 * bn;
+    if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = bn; }
+  }
+  *cost_out = best_cost;
+  return best;
 }
 
 // Plan of a weight-gradient launch: n_tiles output tiles, a reduction of n_slabs slabs, `sms` CTAs.  A tile's reduction is cut
@@ -392,9 +442,9 @@ static int launch_bwd_gemm(const CUtensorMap& a1, const CUtensorMap& b1, const C
 // each, so that they spread over the whole grid as short units.  Cost model in slab-times on the busiest CTA: a round of
 // large units costs its slabs (the epilogue of a unit overlaps the next unit's products), a round of short units at least
 // an epilogue (six slab-times), one epilogue at the end.  At most 16 splits and 32 pieces, units of at least 8 slabs.
-struct WgradPlan { int splits, n_full, pieces; long long units; };
-static WgradPlan plan_wgrad(int n_tiles, int n_slabs, int sms) {
-  WgradPlan best{1, n_tiles, 1, n_tiles};
+struct WgradPlan { int splits, n_full, pieces; long long units, cost; };
+static WgradPlan search_wgrad_plan(int n_tiles, int n_slabs, int sms) {
+  WgradPlan best{1, n_tiles, 1, n_tiles, 0};
   long long best_cost = -1;
   for (int s = 1; s <= 16; ++s) {
     const int per = (n_slabs + s - 1) / s;
@@ -411,11 +461,19 @@ static WgradPlan plan_wgrad(int n_tiles, int n_slabs, int sms) {
       const long long units = full_rounds * sms + rem * m_eff;
       if (best_cost < 0 || cost < best_cost || (cost == best_cost && units < best.units)) {
         best_cost = cost;
-        best = WgradPlan{s_eff, int(full_rounds * sms), m_eff, units};
+        best = WgradPlan{s_eff, int(full_rounds * sms), m_eff, units, cost};
       }
     }
   }
   return best;
+}
+// The search takes the host some microseconds and a model asks for the same few shapes all the time: the last ones are kept.
+static WgradPlan plan_wgrad(int n_tiles, int n_slabs, int sms) {
+  struct Entry { int n_tiles, n_slabs, sms; WgradPlan plan; };
+  static thread_local Entry cache[32] = {};
+  Entry& c = cache[(unsigned(n_tiles) * 31u + unsigned(n_slabs)) % 32u];
+  if (c.n_tiles != n_tiles || c.n_slabs != n_slabs || c.sms != sms) c = Entry{n_tiles, n_slabs, sms, search_wgrad_plan(n_tiles, n_slabs, sms)};
+  return c.plan;
 }
 
 }  // namespace mintb
@@ -426,6 +484,11 @@ static bool bwd_aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p
 
 extern "C" int mintb_linear_dgrad(const void* dz, const void* w, const void* dz2, const void* w2, void* dx, int M, int N, int K,
                                   int N2, int dz_dtype, int w_dtype, float alpha, void* stream, int* dev_status) {
+  return mintb_linear_dgrad_res(dz, w, dz2, w2, dx, nullptr, 0.f, M, N, K, N2, dz_dtype, w_dtype, alpha, stream, dev_status);
+}
+
+extern "C" int mintb_linear_dgrad_res(const void* dz, const void* w, const void* dz2, const void* w2, void* dx, const void* resid, float beta, int M, int N,
+                                      int K, int N2, int dz_dtype, int w_dtype, float alpha, void* stream, int* dev_status) {
   const bool f8 = is_f8(dz_dtype);
   if (dz == nullptr || w == nullptr || dx == nullptr || M <= 0 || N <= 0 || K <= 0 || N2 < 0 || ((dz2 == nullptr) != (N2 == 0)) ||
       ((w2 == nullptr) != (N2 == 0))) {
@@ -438,11 +501,13 @@ extern "C" int mintb_linear_dgrad(const void* dz, const void* w, const void* dz2
   }
   const int esz = f8 ? 1 : 2;
   if ((size_t(N) * esz) % 16 || (size_t(N2) * esz) % 16 || (size_t(K) * esz) % 16 || K % 8 || !bwd_aligned16(dz) || !bwd_aligned16(w) ||
-      !bwd_aligned16(dz2) || !bwd_aligned16(w2) || !bwd_aligned16(dx)) {
+      !bwd_aligned16(dz2) || !bwd_aligned16(w2) || !bwd_aligned16(dx) || !bwd_aligned16(resid)) {
     set_error("mintb_linear_dgrad: rows of dz, w and dx must be 16-byte multiples and the pointers 16-byte aligned");
     return MINTB_EINVAL;
   }
-  const int epb = 128 / esz;
+  const int epb = 128 / esz, sms = sm_count();
+  long long cost;
+  const int bn = pick_bwd_tile(M, K, (N + epb - 1) / epb + (N2 + epb - 1) / epb, f8, sms, &cost);
   CUtensorMap a1, b1, a2, b2, mo;
   bool ok = operand_map(&a1, dz, M, N, esz, kBM) && operand_map(&b1, w, N, K, esz, epb) && result_map(&mo, dx, M, K, false);
   a2 = a1; b2 = b1;
@@ -450,12 +515,12 @@ extern "C" int mintb_linear_dgrad(const void* dz, const void* w, const void* dz2
   if (!ok) { set_error("mintb_linear_dgrad: cuTensorMapEncodeTiled failed"); return MINTB_ECUDA; }
   BwdGemmParams p{};
   p.rows = M; p.cols = K; p.red1 = N; p.red2 = N2; p.f8 = f8 ? 1 : 0;
-  p.idesc = bwd_idesc(fmt_code(dz_dtype), fmt_code(w_dtype), false, true);
-  p.splits = 1; p.pieces = 1; p.alpha = alpha; p.status = dev_status;
-  const int tiles = ((M + kBM - 1) / kBM) * ((K + kBN - 1) / kBN);
+  p.idesc = bwd_idesc(fmt_code(dz_dtype), fmt_code(w_dtype), false, true, bn);
+  p.splits = 1; p.pieces = 1; p.result = kStoreBf16; p.alpha = alpha; p.beta = beta;
+  p.resid = static_cast<const __nv_bfloat16*>(resid); p.status = dev_status;
+  const int tiles = ((M + kBM - 1) / kBM) * ((K + bn - 1) / bn);
   p.n_full = tiles;
-  const int sms = sm_count();
-  return launch_bwd_gemm<kDgrad>(a1, b1, a2, b2, mo, p, tiles < sms ? tiles : sms, static_cast<cudaStream_t>(stream));
+  return launch_bwd_gemm<kDgrad>(bn, a1, b1, a2, b2, mo, p, tiles, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" size_t mintb_linear_wgrad_workspace_bytes(int N, int K, int out_dtype) {
@@ -489,31 +554,44 @@ extern "C" int mintb_linear_wgrad(const void* dz, const void* x, void* dw, void*
     return MINTB_EWORKSPACE;
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const int epb = 128 / esz, sms = sm_count(), n_slabs = (M + epb - 1) / epb;
+  // Uncut, when the tiles over all tokens end before the cut reduction does with its clearing and conversion passes (about 3 us;
+  // the bulk reduction and its order are gone then too): up to about 2000 tokens for the 8M model's matrices.
+  long long direct_cost;
+  const int bn = pick_bwd_tile(N, K, n_slabs, f8, sms, &direct_cost);
+  const int tiles256 = ((N + kBM - 1) / kBM) * ((K + 255) / 256);
+  const WgradPlan plan = plan_wgrad(tiles256, n_slabs, sms);
+  const bool direct = K % 8 == 0 && direct_cost <= plan.cost * 512 + (out_dtype == MINTB_BF16 ? 6000 : 3500);
   float* acc = out_dtype == MINTB_F32 ? static_cast<float*>(dw) : static_cast<float*>(workspace);
-  cudaError_t e = cudaMemsetAsync(acc, 0, size_t(N) * K * 4, s);
+  cudaError_t e = direct ? cudaSuccess : cudaMemsetAsync(acc, 0, size_t(N) * K * 4, s);
   if (e != cudaSuccess) { set_error("cudaMemsetAsync: %s", cudaGetErrorString(e)); return MINTB_ECUDA; }
-  const int epb = 128 / esz;
   CUtensorMap a1, b1, mo;
-  if (!operand_map(&a1, dz, M, N, esz, epb) || !operand_map(&b1, x, M, K, esz, epb) || !result_map(&mo, acc, N, K, true)) {
+  const bool f32_result = !direct || out_dtype == MINTB_F32;
+  if (!operand_map(&a1, dz, M, N, esz, epb) || !operand_map(&b1, x, M, K, esz, epb) || !result_map(&mo, direct ? dw : acc, N, K, f32_result)) {
     set_error("mintb_linear_wgrad: cuTensorMapEncodeTiled failed");
     return MINTB_ECUDA;
   }
   BwdGemmParams p{};
   p.rows = N; p.cols = K; p.red1 = M; p.red2 = 0; p.f8 = f8 ? 1 : 0;
-  p.idesc = bwd_idesc(fmt_code(dz_dtype), fmt_code(x_dtype), true, true);
+  p.idesc = bwd_idesc(fmt_code(dz_dtype), fmt_code(x_dtype), true, true, direct ? bn : 256);
   p.alpha = alpha; p.status = dev_status;
-  const int tiles = ((N + kBM - 1) / kBM) * ((K + kBN - 1) / kBN);
-  const int sms = sm_count();
-  const WgradPlan plan = plan_wgrad(tiles, (M + epb - 1) / epb, sms);
-  p.splits = plan.splits; p.n_full = plan.n_full; p.pieces = plan.pieces;
-  const long long units = plan.units;
-  int rc = launch_bwd_gemm<kWgrad>(a1, b1, a1, b1, mo, p, units < sms ? int(units) : sms, s);
-  if (rc != MINTB_OK) return rc;
+  long long units;
+  if (direct) {
+    p.splits = 1; p.pieces = 1;
+    p.n_full = ((N + kBM - 1) / kBM) * ((K + bn - 1) / bn);
+    p.result = f32_result ? kStoreF32 : kStoreBf16;
+    units = p.n_full;
+  } else {
+    p.splits = plan.splits; p.n_full = plan.n_full; p.pieces = plan.pieces;
+    p.result = kAddF32;
+    units = plan.units;
+  }
+  int rc = launch_bwd_gemm<kWgrad>(direct ? bn : 256, a1, b1, a1, b1, mo, p, units, s);
+  if (rc != MINTB_OK || direct) return rc;
   if (out_dtype == MINTB_BF16) {
     const size_t n = size_t(N) * K;
-    wgrad_convert_kernel<<<unsigned((n / 8 + 255) / 256 + 1), 256, 0, s>>>(acc, static_cast<__nv_bfloat16*>(dw), n);
+    e = launch_dependent(wgrad_convert_kernel, dim3(unsigned((n / 8 + 255) / 256 + 1)), dim3(256), 0, s, acc, static_cast<__nv_bfloat16*>(dw), n);
     count_launches(1);
-    e = cudaGetLastError();
     if (e != cudaSuccess) { set_error("wgrad convert launch: %s", cudaGetErrorString(e)); return MINTB_ECUDA; }
   }
   return MINTB_OK;

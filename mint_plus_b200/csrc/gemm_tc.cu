@@ -1,9 +1,10 @@
 // tcgen05 GEMM for the projections around the attention: out = epilogue(alpha * x W^T + bias).
 //
 //   x [M][K] and W [N][K] are both K-contiguous (nn.Linear layout), bf16 (kind::f16) or e4m3 (kind::f8f6f4), fp32 accumulate.
-//   Persistent CTAs walk 128 x 256 output tiles (N fastest, so the CTAs running together share rows of x in L2).
-//   warp 0  TMA producer: 128-byte-wide K slabs of x (128 rows) and W (256 rows) into a 4-stage ring, 128B swizzle
-//   warp 1  MMA issuer: four tcgen05.mma (M128 N256) per slab into one of two 256-column TMEM accumulators
+//   Persistent CTAs walk 128 x BN output tiles (N fastest, so the CTAs running together share rows of x in L2), BN = 256 where
+//   they fill the chip, 128 or 64 where fewer, larger tiles would leave most SMs idle (pick_tile below).
+//   warp 0  TMA producer: 128-byte-wide K slabs of x (128 rows) and W (BN rows) into a ring of 4 to 8 stages, 128B swizzle
+//   warp 1  MMA issuer: four tcgen05.mma (M128 N = BN) per slab into one of two BN-column TMEM accumulators
 //   warps 2-9  epilogue: two threads per output row (one per half of the tile's columns); 32 columns at a time: alpha, bias, erf-GELU, cast, store —
 //              row-major, or scattered head-major into (B,H,T,D) q/k/v with optional scale and RoPE (the QKV projection),
 //              while the MMA warp already fills the other accumulator.
@@ -17,13 +18,19 @@ namespace mintb {
 
 using namespace ptx;
 
-constexpr int kGM = 128, kGN = 256, kGStages = 4;
+constexpr int kGM = 128;
 constexpr int kGEpiWarps = 8, kGEpiThreads = 32 * kGEpiWarps, kGThreads = 64 + kGEpiThreads;   // TMA warp, MMA warp, epilogue warps
 constexpr int kSlabBytes = 128;                       // bytes of K per stage and row (64 bf16 or 128 e4m3)
-constexpr int kABytes = kGM * kSlabBytes, kBBytes = kGN * kSlabBytes, kGStageBytes = kABytes + kBBytes;
+constexpr int kABytes = kGM * kSlabBytes;
 constexpr int kGStageOutBytes = 32 * 64 + 32 * 32;   // one epilogue warp's staging: 32 rows x 32 bf16 columns, then 32 rows x 32 e4m3 columns, for bulk stores
 constexpr int kGTileRing = 4;   // tile numbers travel from the loading warp to the other roles through a ring this deep
-constexpr size_t kGemmSmem = 1024 + size_t(kGStages) * kGStageBytes + kGEpiWarps * kGStageOutBytes + 256 + 2 * kGN * sizeof(float);
+// A narrower tile needs less of the ring per slab and has less work to hide a slab's latency behind: more stages.
+template <int BN>
+struct GemmCfg {
+  static constexpr int kStages = BN == 256 ? 4 : BN == 128 ? 6 : 8;
+  static constexpr int kBBytes = BN * kSlabBytes, kStageBytes = kABytes + kBBytes;
+  static constexpr size_t kSmem = 1024 + size_t(kStages) * kStageBytes + kGEpiWarps * kGStageOutBytes + 256 + 2 * BN * sizeof(float);
+};
 
 enum GemmEpilogue : int { kEpiBias = 0, kEpiBiasGelu = 1, kEpiHeadMajor = 2 };
 
@@ -37,6 +44,7 @@ struct GemmParams {
   float alpha2;                // head-major epilogue with two pathways: the multiplier of the second pathway's columns (n >= 3E)
   const __nv_bfloat16* resid;  // row-major epilogues: when non-null the result is res_a * resid[m][n] + res_b * (alpha x w^T + bias)
   float res_a, res_b;
+  int res_round;               // the projection is rounded to bf16 before it enters the residual sum, as when it was a tensor of its own
   float out_scale;             // multiplies the result before the cast to e4m3
   const void* bias;            // [N] or null
   void* out;                   // row-major [M][N]
@@ -108,11 +116,12 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   return r;
 }
 
-// EPI: epilogue kind; HD: head_dim of the head-major epilogue (0 otherwise)
-template <int EPI, int HD>
+// EPI: epilogue kind; HD: head_dim of the head-major epilogue (0 otherwise); BN: tile columns
+template <int EPI, int HD, int BN>
 __global__ void __launch_bounds__(kGThreads, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                const __grid_constant__ CUtensorMap map_out, const __grid_constant__ CUtensorMap map_pre, GemmParams p) {
+  constexpr int kGN = BN, kGStages = GemmCfg<BN>::kStages, kGStageBytes = GemmCfg<BN>::kStageBytes;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   unsigned char* s_out = smem + size_t(kGStages) * kGStageBytes;   // [epilogue warp][32 rows][64 B], 64B swizzle
@@ -140,10 +149,15 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     for (int s = 0; s < kGTileRing; ++s) { mbar_init(&tr_full[s], 1); mbar_init(&tr_empty[s], 1 + kGEpiWarps); }
     fence_mbar_init();
   }
-  if (warp == 1) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
+  if (warp == 1) { tmem_alloc(tmem_slot, 2 * BN); tmem_relinquish(); }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  // The next kernel may set itself up while this one runs: from here on only, because its CTAs may take tensor memory that a CTA of
+  // this grid has yet to allocate, and then wait for this grid; and after the wait, so that a kernel may count on everything before
+  // its direct predecessor being complete.
+  griddep_wait();
+  griddep_launch();
   const uint32_t tbase = *tmem_slot;
 
   if (warp == 0) {
@@ -392,6 +406,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         } else {
           const int n = n0 + c0;
           if (p.resid != nullptr) {   // res_a * resid + res_b * (projection): the residual sum of the layer, formed here
+            if (p.res_round) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) v[j] = __bfloat162float(__float2bfloat16_rn(v[j]));
+            }
             if (m < p.M) {
               const __nv_bfloat16* rr = p.resid + size_t(m) * p.N + n;
               if (n + 32 <= p.N) {
@@ -486,7 +504,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       };
       // The TMEM load of the next chunk is issued before the arithmetic and the stores of the current one (head size 64
       // has its own loop).
-      const int cbeg = chalf * (kGN / 2), cend = (chalf + 1) * (kGN / 2);
+      // (a 64-column tile holds one head of 64: the first half of the warps takes it whole)
+      constexpr bool kOneHead = EPI == kEpiHeadMajor && HD == 64 && BN == 64;
+      const int cbeg = kOneHead ? chalf * BN : chalf * (kGN / 2), cend = kOneHead ? BN : (chalf + 1) * (kGN / 2);
       if constexpr (EPI == kEpiHeadMajor && HD == 64) {
         // One head (64 columns: the lower and the upper half the rotation pairs up) of q, k or v per step: both halves
         // arrive with one TMEM round trip and the table rows are on their way while it lasts.  (E is a multiple of 64 and
@@ -555,9 +575,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         for (int c0 = cbeg; c0 < cend; c0 += 64) {
           if (n0 + c0 >= p.N) break;   // uniform
           tmem_ld_wait();
-          tmem_ld32(tacc + c0 + 32, rb);
+          if (BN > 64) tmem_ld32(tacc + c0 + 32, rb);
           do_chunk(c0, ra);
-          if (n0 + c0 + 32 >= p.N) break;   // uniform
+          if (BN == 64 || n0 + c0 + 32 >= p.N) break;   // uniform
           tmem_ld_wait();
           if (c0 + 64 < cend) tmem_ld32(tacc + c0 + 64, ra);
           do_chunk(c0 + 32, rb);
@@ -568,13 +588,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       mbar_arrive(&acc_empty[ab]);
       if (++ab == 2) { ab = 0; ab_phase ^= 1; }
     }
-    if (lane == 0) bulk_wait_read_all();   // the bulk stores have read their staging rows (the kernel boundary orders their writes)
+    if (lane == 0) bulk_wait_all();   // (a dependent kernel may already be waiting for this grid)
   }
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {
     __syncwarp();
-    tmem_dealloc(tbase, 512);
+    tmem_dealloc(tbase, 2 * BN);
   }
 }
 
@@ -582,6 +602,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 // finite values at +-448 and keeps a NaN a NaN (an explicit clamp would turn it into -448 and hide a diverged run).
 __global__ void __launch_bounds__(256) quantize_e4m3_kernel(const __nv_bfloat16* __restrict__ x, __nv_fp8_storage_t* __restrict__ out,
                                                             size_t n, float inv_scale) {
+  griddep_wait();
+  griddep_launch();
   const size_t i = (size_t(blockIdx.x) * blockDim.x + threadIdx.x) * 16;
   if (i >= n) return;
   if (i + 16 <= n) {
@@ -655,10 +677,42 @@ static bool gemm_out_map_f8(CUtensorMap* m, const void* ptr, int rows, int N) {
             CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// The tile width that finishes first by a count of cycles on the busiest SM: rounds of the grid times the slabs of a tile (512, 280
+// and 200 cycles at 256, 128 and 64 columns: the narrow ones are bound by the operand traffic into shared memory) plus filling
+// the ring and draining the last tile.  Whole-batch products come out at 256; M = 497 against N = K = 1280 (e4m3) at 64: 20 tiles on 148 SMs
+// and 15.9 us before, 80 tiles and 8.6 us now.
+static int pick_tile(int M, int N, int n_slabs, int sms) {
+  const long long tm = (M + kGM - 1) / kGM;
+  int best = 256;
+  long long best_cost = -1;
+  for (const int bn : {256, 128, 64}) {
+    const long long rounds = (tm * ((N + bn - 1) / bn) + sms - 1) / sms;
+    const long long cost = rounds * n_slabs * (bn == 256 ? 512 : bn == 128 ? 280 : 200) + 1500 + 8 * bn;
+    if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = bn; }
+  }
+  return best;
+}
+
+template <int EPI, int HD, int BN>
+static int launch_gemm_t(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mo, const CUtensorMap& mp, GemmParams& p, int sms, cudaStream_t stream) {
+  constexpr auto kern = gemm_tc_kernel<EPI, HD, BN>;
+  cudaError_t e = opt_in_smem<kern>(int(GemmCfg<BN>::kSmem));
+  if (e != cudaSuccess) { set_error("cudaFuncSetAttribute: %s", cudaGetErrorString(e)); return MINTB_ECUDA; }
+  const int tiles = ((p.M + kGM - 1) / kGM) * ((p.N + BN - 1) / BN);
+  if (int rc = next_tile_counter(&p.sched); rc != MINTB_OK) return rc;
+  e = launch_dependent(kern, dim3(tiles < sms ? tiles : sms), dim3(kGThreads), GemmCfg<BN>::kSmem, stream, ma, mb, mo, mp, p);
+  count_launches(1);
+  if (e != cudaSuccess) { set_error("gemm launch: %s", cudaGetErrorString(e)); return MINTB_ECUDA; }
+  return MINTB_OK;
+}
+
 int launch_gemm(const GemmParams& p_in, const void* x, const void* w, cudaStream_t stream) {
   GemmParams p = p_in;
   CUtensorMap ma, mb;
-  if (!gemm_map(&ma, x, p.M, p.K, p.in_dtype, kGM) || !gemm_map(&mb, w, p.N, p.K, p.in_dtype, kGN)) {
+  const int sms = sm_count();
+  const int per_slab = p.in_dtype == MINTB_E4M3 ? 128 : 64;
+  const int bn = pick_tile(p.M, p.N, (p.K + per_slab - 1) / per_slab, sms);
+  if (!gemm_map(&ma, x, p.M, p.K, p.in_dtype, kGM) || !gemm_map(&mb, w, p.N, p.K, p.in_dtype, bn)) {
     set_error("mintb gemm: cuTensorMapEncodeTiled failed");
     return MINTB_ECUDA;
   }
@@ -683,33 +737,23 @@ int launch_gemm(const GemmParams& p_in, const void* x, const void* w, cudaStream
     p.use_bulk_f8 = 1;
   }
   p.alt_stores = (p.use_bulk_f8 && p.use_bulk_store && p.preact != nullptr) ? 1 : 0;
-  void (*kern)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, GemmParams) = nullptr;
-  if (p.epilogue == kEpiBias) kern = gemm_tc_kernel<kEpiBias, 0>;
-  else if (p.epilogue == kEpiBiasGelu) kern = gemm_tc_kernel<kEpiBiasGelu, 0>;
-  else if (p.D == 16) kern = gemm_tc_kernel<kEpiHeadMajor, 16>;
-  else if (p.D == 32) kern = gemm_tc_kernel<kEpiHeadMajor, 32>;
-  else kern = gemm_tc_kernel<kEpiHeadMajor, 64>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kGemmSmem));
-  if (e != cudaSuccess) { set_error("cudaFuncSetAttribute: %s", cudaGetErrorString(e)); return MINTB_ECUDA; }
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int tiles = ((p.M + kGM - 1) / kGM) * ((p.N + kGN - 1) / kGN);
-  const int grid = tiles < sms ? tiles : sms;
-  if (int rc = next_tile_counter(&p.sched); rc != MINTB_OK) return rc;
-  kern<<<grid, kGThreads, kGemmSmem, stream>>>(ma, mb, mo, mp, p);
-  count_launches(1);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) { set_error("gemm launch: %s", cudaGetErrorString(e)); return MINTB_ECUDA; }
-  return MINTB_OK;
+#define MINTB_GEMM_TILE(EPI, HD)                                                              \
+  return bn == 256 ? launch_gemm_t<EPI, HD, 256>(ma, mb, mo, mp, p, sms, stream)              \
+       : bn == 128 ? launch_gemm_t<EPI, HD, 128>(ma, mb, mo, mp, p, sms, stream)              \
+                   : launch_gemm_t<EPI, HD, 64>(ma, mb, mo, mp, p, sms, stream)
+  if (p.epilogue == kEpiBias) MINTB_GEMM_TILE(kEpiBias, 0);
+  if (p.epilogue == kEpiBiasGelu) MINTB_GEMM_TILE(kEpiBiasGelu, 0);
+  if (p.D == 16) MINTB_GEMM_TILE(kEpiHeadMajor, 16);
+  if (p.D == 32) MINTB_GEMM_TILE(kEpiHeadMajor, 32);
+  MINTB_GEMM_TILE(kEpiHeadMajor, 64);
+#undef MINTB_GEMM_TILE
 }
 
 cudaError_t launch_quantize_e4m3(const void* x, void* out, size_t n, float inv_scale, cudaStream_t s) {
   const size_t threads = (n + 15) / 16;
-  quantize_e4m3_kernel<<<unsigned((threads + 255) / 256), 256, 0, s>>>(static_cast<const __nv_bfloat16*>(x),
-                                                                     static_cast<__nv_fp8_storage_t*>(out), n, inv_scale);
   count_launches(1);
-  return cudaGetLastError();
+  return launch_dependent(quantize_e4m3_kernel, dim3(unsigned((threads + 255) / 256)), dim3(256), 0, s, static_cast<const __nv_bfloat16*>(x),
+                          static_cast<__nv_fp8_storage_t*>(out), n, inv_scale);
 }
 
 }  // namespace mintb
@@ -785,6 +829,13 @@ extern "C" int mintb_qkv_fwd(const void* x, const void* w, const void* bias, voi
 extern "C" int mintb_linear_res_fwd(const void* x, const void* w, const void* bias, const void* resid, float res_a, float res_b, void* out,
                                     void* bf16_copy_out, int M, int N, int K, int in_dtype, int bias_dtype, int out_dtype, float alpha,
                                     float out_scale, void* stream, int* dev_status) {
+  return mintb_linear_add_fwd(x, w, bias, resid, res_a, res_b, 0, out, bf16_copy_out, M, N, K, in_dtype, bias_dtype, out_dtype, alpha, out_scale, stream,
+                              dev_status);
+}
+
+extern "C" int mintb_linear_add_fwd(const void* x, const void* w, const void* bias, const void* resid, float res_a, float res_b, int round_first,
+                                    void* out, void* bf16_copy_out, int M, int N, int K, int in_dtype, int bias_dtype, int out_dtype, float alpha,
+                                    float out_scale, void* stream, int* dev_status) {
   int rc = check_gemm("mintb_linear_res_fwd", x, w, M, N, K, in_dtype);
   if (rc != MINTB_OK) return rc;
   if (out == nullptr || (out_dtype != MINTB_BF16 && out_dtype != MINTB_E4M3) || (reinterpret_cast<uintptr_t>(out) & 15) || N % 8 != 0 ||
@@ -799,7 +850,7 @@ extern "C" int mintb_linear_res_fwd(const void* x, const void* w, const void* bi
   p.epilogue = kEpiBias;
   p.alpha = alpha; p.out_scale = out_scale; p.bias = bias; p.out = out; p.status = dev_status;
   p.preact = static_cast<__nv_bfloat16*>(bf16_copy_out);
-  p.resid = static_cast<const __nv_bfloat16*>(resid); p.res_a = res_a; p.res_b = res_b;
+  p.resid = static_cast<const __nv_bfloat16*>(resid); p.res_a = res_a; p.res_b = res_b; p.res_round = round_first;
   return launch_gemm(p, x, w, static_cast<cudaStream_t>(stream));
 }
 

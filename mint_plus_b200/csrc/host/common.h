@@ -99,25 +99,29 @@ struct Product {      // y = act(alpha x w^T + bias) and its variants
   double out_e4m3 = 0.0;         // scale of an e4m3 result, 0: bf16
 };
 std::pair<Tensor, Tensor> linear_fwd(const Product& p);     // (y, pre-activation)
-// res_a resid + res_b (alpha x w^T + bias), and with quant > 0 its e4m3 copy saturate(. / quant)
-std::pair<Tensor, Tensor> linear_res_fwd(const Product& p, const Tensor& resid, double res_a, double res_b, double quant);
+// res_a resid + res_b (alpha x w^T + bias), and with quant > 0 its e4m3 copy saturate(. / quant); round_first: the projection is rounded
+// to bf16 before the sum
+std::pair<Tensor, Tensor> linear_res_fwd(const Product& p, const Tensor& resid, double res_a, double res_b, double quant, bool round_first = false);
 Tensor quantize(const Tensor& x, double scale);
-Tensor dgrad(const Tensor& dz, const Tensor& w, double alpha, const Tensor& dz2 = {}, const Tensor& w2 = {});
+// alpha (dz w + dz2 w2) + beta resid
+Tensor dgrad(const Tensor& dz, const Tensor& w, double alpha, const Tensor& dz2 = {}, const Tensor& w2 = {}, const Tensor& resid = {}, double beta = 0.0);
 Tensor wgrad(const Tensor& dz, const Tensor& x, double alpha, at::ScalarType out);
-// (dz, db): dz = dy gelu'(z) (dy itself without z) in bf16, db its column sums in fp32
-std::pair<Tensor, Tensor> gelu_colsum(const Tensor& dy, const Tensor& z, bool want_db);
+// (dz, db): dz = dy gelu'(z) (dy itself without z) in bf16, db its column sums in the given type (none: not wanted)
+std::pair<Tensor, Tensor> gelu_colsum(const Tensor& dy, const Tensor& z, std::optional<at::ScalarType> db_dt);
 // (dz in e5m2, db)
-std::pair<Tensor, Tensor> gelu_colsum_f8(const Tensor& dy, const Tensor& z, bool want_db, double scale);
+std::pair<Tensor, Tensor> gelu_colsum_f8(const Tensor& dy, const Tensor& z, std::optional<at::ScalarType> db_dt, double scale);
+// Bytes that the caching allocator holds on the device without using them.
+int64_t cached_free_bytes(int device);
 
 struct NormOut {
   Tensor s, y, stats, q8;
 };
 NormOut add_layernorm_fwd(const Tensor& x, const Tensor& r, double a, double b, const Tensor& gamma, const Tensor& beta, double eps, bool need_s, double quant);
 struct NormGrad {
-  Tensor dx, dr, dgamma, dbeta;   // parameter gradients in fp32
+  Tensor dx, dr, dgamma, dbeta;   // parameter gradients in the type of gamma
 };
 NormGrad add_layernorm_bwd(const Tensor& dy, const Tensor& ds, const Tensor& x, const Tensor& r, double a, double b, const Tensor& gamma, const Tensor& stats,
-                           bool want_params);
+                           bool want_params, bool ds_apart = false);   // ds_apart: ds is added to the rounded dx
 
 // Which inputs of a call want gradients, as a node of the autograd graph; nullptr when none does.
 template <typename N>

@@ -1,4 +1,6 @@
 // The library's calls on tensors: allocation of results and workspaces, nothing else (no autograd).
+#include <c10/cuda/CUDACachingAllocator.h>
+
 #include <mutex>
 
 #include "common.h"
@@ -57,12 +59,12 @@ std::pair<Tensor, Tensor> linear_fwd(const Product& p) {
   return {out, z};
 }
 
-std::pair<Tensor, Tensor> linear_res_fwd(const Product& p, const Tensor& resid, double res_a, double res_b, double quant) {
+std::pair<Tensor, Tensor> linear_res_fwd(const Product& p, const Tensor& resid, double res_a, double res_b, double quant, bool round_first) {
   Env e(p.x);
   const int64_t M = p.x.size(0), K = p.x.size(1), N = p.w.size(0);
   Tensor out = e.empty({M, N}, at::kBFloat16);
   Tensor q8 = quant > 0 ? e.empty({M, N}, at::kFloat8_e4m3fn) : Tensor();
-  check(mintb_linear_res_fwd(ptr(p.x), ptr(p.w), ptr(p.bias), ptr(resid), float(res_a), float(res_b), q8.defined() ? ptr(q8) : ptr(out),
+  check(mintb_linear_add_fwd(ptr(p.x), ptr(p.w), ptr(p.bias), ptr(resid), float(res_a), float(res_b), round_first, q8.defined() ? ptr(q8) : ptr(out),
                              q8.defined() ? ptr(out) : nullptr, M, N, K, dt_code(p.x.scalar_type(), "x"), param_dt(p.bias, "bias"),
                              q8.defined() ? MINTB_E4M3 : MINTB_BF16, float(p.alpha), quant > 0 ? float(1.0 / quant) : 1.f, e.stream, e.status),
         "mintb_linear_res_fwd");
@@ -76,11 +78,11 @@ Tensor quantize(const Tensor& x, double scale) {
   return out;
 }
 
-Tensor dgrad(const Tensor& dz, const Tensor& w, double alpha, const Tensor& dz2, const Tensor& w2) {
+Tensor dgrad(const Tensor& dz, const Tensor& w, double alpha, const Tensor& dz2, const Tensor& w2, const Tensor& resid, double beta) {
   Env e(dz);
   const int64_t M = dz.size(0), N = dz.size(1), K = w.size(1), N2 = dz2.defined() ? dz2.size(1) : 0;
   Tensor dx = e.empty({M, K}, at::kBFloat16);
-  check(mintb_linear_dgrad(ptr(dz), ptr(w), ptr(dz2), ptr(w2), ptr(dx), M, N, K, N2, dt_code(dz.scalar_type(), "dz"), dt_code(w.scalar_type(), "w"),
+  check(mintb_linear_dgrad_res(ptr(dz), ptr(w), ptr(dz2), ptr(w2), ptr(dx), ptr(resid), float(beta), M, N, K, N2, dt_code(dz.scalar_type(), "dz"), dt_code(w.scalar_type(), "w"),
                            float(alpha), e.stream, e.status),
         "mintb_linear_dgrad");
   return dx;
@@ -99,23 +101,29 @@ Tensor wgrad(const Tensor& dz, const Tensor& x, double alpha, at::ScalarType out
   return dw;
 }
 
-std::pair<Tensor, Tensor> gelu_colsum(const Tensor& dy, const Tensor& z, bool want_db) {
-  if (!z.defined() && !want_db) return {dy, Tensor()};
+static std::pair<Tensor, Tensor> bias_pass(const Tensor& dy, const Tensor& z, std::optional<at::ScalarType> db_dt, double f8_scale) {
   Env e(dy);
   const int64_t M = dy.size(0), N = dy.size(1);
-  Tensor dz = z.defined() ? e.empty({M, N}, at::kBFloat16) : dy;
-  Tensor db = want_db ? e.empty({N}, at::kFloat) : Tensor();
-  check(mintb_gelu_bwd_colsum_act(ptr(dy), ptr(z), z.defined() ? ptr(dz) : nullptr, nullptr, fptr(db), M, N, e.stream), "mintb_gelu_bwd_colsum");
-  return {dz, db};
+  const bool f8 = f8_scale > 0;
+  Tensor dz = f8 ? e.empty({M, N}, at::kFloat8_e5m2) : z.defined() ? e.empty({M, N}, at::kBFloat16) : dy;
+  Tensor db, ws;
+  if (db_dt.has_value()) {
+    db = e.empty({N}, *db_dt == at::kBFloat16 ? at::kBFloat16 : at::kFloat);
+    ws = e.bytes(mintb_bias_grad_workspace_bytes(M, N));
+  }
+  check(mintb_gelu_bwd_bias(ptr(dy), ptr(z), !f8 && z.defined() ? ptr(dz) : nullptr, ptr(db), param_dt(db, "bias"), f8 ? ptr(dz) : nullptr, f8 ? float(f8_scale) : 1.f,
+                            ptr(ws), ws.defined() ? size_t(ws.numel()) : 0, M, N, e.stream),
+        "mintb_gelu_bwd_bias");
+  return {dz, db_dt.has_value() ? as_dtype(db, *db_dt) : db};
 }
 
-std::pair<Tensor, Tensor> gelu_colsum_f8(const Tensor& dy, const Tensor& z, bool want_db, double scale) {
-  Env e(dy);
-  const int64_t M = dy.size(0), N = dy.size(1);
-  Tensor dz8 = e.empty({M, N}, at::kFloat8_e5m2);
-  Tensor db = want_db ? e.empty({N}, at::kFloat) : Tensor();
-  check(mintb_gelu_bwd_colsum_f8(ptr(dy), ptr(z), nullptr, nullptr, fptr(db), ptr(dz8), float(scale), M, N, e.stream), "mintb_gelu_bwd_colsum_f8");
-  return {dz8, db};
+std::pair<Tensor, Tensor> gelu_colsum(const Tensor& dy, const Tensor& z, std::optional<at::ScalarType> db_dt) {
+  if (!z.defined() && !db_dt.has_value()) return {dy, Tensor()};
+  return bias_pass(dy, z, db_dt, 0.0);
+}
+
+std::pair<Tensor, Tensor> gelu_colsum_f8(const Tensor& dy, const Tensor& z, std::optional<at::ScalarType> db_dt, double scale) {
+  return bias_pass(dy, z, db_dt, scale);
 }
 
 NormOut add_layernorm_fwd(const Tensor& x, const Tensor& r, double a, double b, const Tensor& gamma, const Tensor& beta, double eps, bool need_s, double quant) {
@@ -136,22 +144,28 @@ NormOut add_layernorm_fwd(const Tensor& x, const Tensor& r, double a, double b, 
 }
 
 NormGrad add_layernorm_bwd(const Tensor& dy, const Tensor& ds, const Tensor& x, const Tensor& r, double a, double b, const Tensor& gamma, const Tensor& stats,
-                           bool want_params) {
+                           bool want_params, bool ds_apart) {
   Env e(x);
   const int64_t rows = x.size(0), E = x.size(1);
   NormGrad g;
   g.dx = e.empty({rows, E}, at::kBFloat16);
   if (r.defined()) g.dr = e.empty({rows, E}, at::kBFloat16);
   if (want_params) {
-    g.dgamma = e.empty({E}, at::kFloat);
-    g.dbeta = e.empty({E}, at::kFloat);
+    g.dgamma = e.empty({E}, gamma.scalar_type());   // (f32 or bf16: param_dt checks)
+    g.dbeta = e.empty({E}, gamma.scalar_type());
   }
   const size_t bytes = want_params ? mintb_add_layernorm_bwd_workspace_bytes(rows, E) : 0;
   Tensor ws = e.bytes(bytes);
-  check(mintb_add_layernorm_bwd(ptr(dy), ptr(ds), ptr(x), ptr(r), float(a), float(b), ptr(gamma), param_dt(gamma, "gamma"), fptr(stats), ptr(g.dx), ptr(g.dr),
-                                fptr(g.dgamma), fptr(g.dbeta), ptr(ws), bytes, rows, E, e.stream),
+  check(mintb_add_layernorm_bwd_typed(ptr(dy), ptr(ds), ds_apart, ptr(x), ptr(r), float(a), float(b), ptr(gamma), param_dt(gamma, "gamma"), fptr(stats), ptr(g.dx), ptr(g.dr),
+                                      ptr(g.dgamma), ptr(g.dbeta), param_dt(gamma, "gamma"), ptr(ws), bytes, rows, E, e.stream),
         "mintb_add_layernorm_bwd");
   return g;
+}
+
+int64_t cached_free_bytes(int device) {
+  const auto stats = c10::cuda::CUDACachingAllocator::getDeviceStats(static_cast<c10::DeviceIndex>(device));
+  constexpr size_t all = 0;   // the aggregate over the allocator's pools
+  return stats.reserved_bytes[all].current - stats.allocated_bytes[all].current;
 }
 
 }  // namespace mintb_host

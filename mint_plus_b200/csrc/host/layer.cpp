@@ -129,7 +129,7 @@ std::tuple<Tensor, OptTensor> LayerPlan::forward(const Tensor& x_in, const OptTe
     p2.x = act;
     p2.w = fc2.w; p2.bias = params[at.b2]; p2.alpha = fc2.alpha();
     if (!mu) {
-      std::tie(y, y8) = linear_res_fwd(p2, x1, 1.0, 1.0, 0.0);
+      std::tie(y, y8) = linear_res_fwd(p2, x1, 1.0, 1.0, 0.0, true);
     } else {
       Tensor y2 = linear_fwd(p2).first;
       NormOut n = add_layernorm_fwd(x1, y2, keep, add, params[at.g2], params[at.be2], eps2, false, next_quant);
@@ -202,10 +202,11 @@ variable_list LayerNode::apply(variable_list&& grads) {
     if (o.grad_scale <= 0) o.grad_scale = o.holder->fix(measure());
   };
   // one projection's output gradient as the operand of its products, with the bias gradient
-  auto operand = [&](Operand& o, const Tensor& dy, const Tensor& z, bool want_db) {
-    if (fp8) settle(o, [&] { return amax(z.defined() ? gelu_colsum(dy, z, false).first : dy); });
-    return fp8 ? gelu_colsum_f8(dy, z, want_db, o.grad_scale) : gelu_colsum(dy, z, want_db);
+  auto operand = [&](Operand& o, const Tensor& dy, const Tensor& z, std::optional<at::ScalarType> db_dt) {
+    if (fp8) settle(o, [&] { return amax(z.defined() ? gelu_colsum(dy, z, std::nullopt).first : dy); });
+    return fp8 ? gelu_colsum_f8(dy, z, db_dt, o.grad_scale) : gelu_colsum(dy, z, db_dt);
   };
+  auto bias_dt = [&](int64_t k, int64_t n = 1) { return any(k, n) ? std::optional<at::ScalarType>(plan.params[k].scalar_type()) : std::nullopt; };
   auto a_in = [&](const Operand& o) { return fp8 ? o.grad_scale * o.w_scale * o.out_scale : 1.0; };
   auto a_w = [&](const Operand& o) { return fp8 ? o.grad_scale * o.x_scale * o.out_scale : 1.0; };
 
@@ -217,18 +218,18 @@ variable_list LayerNode::apply(variable_list&& grads) {
     d_ffn = g.dr;
   }
   {
-    auto [g2, db2] = operand(plan.fc2, d_ffn, Tensor(), wants(at.b2));
+    auto [g2, db2] = operand(plan.fc2, d_ffn, Tensor(), bias_dt(at.b2));
     give(at.b2, db2);
     if (wants(at.w2)) give(at.w2, wgrad(g2, s[kA], a_w(plan.fc2), w_dt(at.w2)));
     Tensor da = dgrad(g2, plan.fc2.w, a_in(plan.fc2));
-    auto [g1, db1] = operand(plan.fc1, da, s[kZ], wants(at.b1));
+    auto [g1, db1] = operand(plan.fc1, da, s[kZ], bias_dt(at.b1));
     give(at.b1, db1);
     if (wants(at.w1)) give(at.w1, wgrad(g1, s[kH2], a_w(plan.fc1), w_dt(at.w1)));
-    Tensor dh2 = dgrad(g1, plan.fc1.w, a_in(plan.fc1));
     if (mu) {
-      d1.add_(dh2);
+      d1 = dgrad(g1, plan.fc1.w, a_in(plan.fc1), Tensor(), Tensor(), d1, 1.0);   // both ways into the first residual sum
     } else {
-      NormGrad g = add_layernorm_bwd(dh2, gy, s[kX1], Tensor(), 1.0, 0.0, plan.params[at.g2], s[kStats2], p2);
+      Tensor dh2 = dgrad(g1, plan.fc1.w, a_in(plan.fc1));
+      NormGrad g = add_layernorm_bwd(dh2, gy, s[kX1], Tensor(), 1.0, 0.0, plan.params[at.g2], s[kStats2], p2, true);
       if (p2) { give(at.g2, g.dgamma); give(at.be2, g.dbeta); }
       d1 = g.dx;
     }
@@ -236,7 +237,7 @@ variable_list LayerNode::apply(variable_list&& grads) {
   // output projection: its result entered the sum times `add`
   Tensor d_attn;
   {
-    auto [go, dbo] = operand(plan.out, d1, Tensor(), wants(at.bo));
+    auto [go, dbo] = operand(plan.out, d1, Tensor(), bias_dt(at.bo));
     if (dbo.defined()) give(at.bo, plan.add == 1.0 ? dbo : dbo * plan.add);
     if (wants(at.wo)) give(at.wo, wgrad(go, s[kO], a_w(plan.out) * plan.add, w_dt(at.wo)));
     d_attn = dgrad(go, plan.out.w, a_in(plan.out) * plan.add);
@@ -255,20 +256,17 @@ variable_list LayerNode::apply(variable_list&& grads) {
   Operand os = plan.qkv_self, oc = plan.qkv_cross;
   if (fp8) settle(os, [&] { return std::max(amax(g[0]), amax(g[1]) / ((os.w_scale * os.out_scale) / (oc.w_scale * oc.out_scale))); });
   if (fp8) oc.grad_scale = os.grad_scale * (os.w_scale * os.out_scale) / (oc.w_scale * oc.out_scale);
-  auto [gs, dbs] = operand(os, g[0], Tensor(), any(at.bs, plan.n_self));
-  auto [gc, dbc] = operand(oc, g[1], Tensor(), any(at.bc, plan.n_cross));
+  auto [gs, dbs] = operand(os, g[0], Tensor(), bias_dt(at.bs, plan.n_self));
+  auto [gc, dbc] = operand(oc, g[1], Tensor(), bias_dt(at.bc, plan.n_cross));
   give_rows(at.bs, plan.n_self, dbs);
   give_rows(at.bc, plan.n_cross, dbc);
   if (any(at.ws, plan.n_self)) give_rows(at.ws, plan.n_self, wgrad(gs, s[kXq], a_w(os), w_dt(at.ws)));
   if (any(at.wc, plan.n_cross)) give_rows(at.wc, plan.n_cross, wgrad(gc, s[kXq], a_w(oc), w_dt(at.wc)));
   if (mu) {
-    if (task_should_compute_output(0)) {
-      Tensor dx = dgrad(gs, os.w, a_in(os), gc, oc.w);
-      res[0] = dx.add_(d1, plan.keep).view(shape);
-    }
+    if (task_should_compute_output(0)) res[0] = dgrad(gs, os.w, a_in(os), gc, oc.w, d1, plan.keep).view(shape);
   } else if (task_should_compute_output(0) || p1) {
     Tensor dh = dgrad(gs, os.w, a_in(os), gc, oc.w);
-    NormGrad n = add_layernorm_bwd(dh, d1, x, Tensor(), 1.0, 0.0, plan.params[at.g1], s[kStats1], p1);
+    NormGrad n = add_layernorm_bwd(dh, d1, x, Tensor(), 1.0, 0.0, plan.params[at.g1], s[kStats1], p1, true);
     if (p1) { give(at.g1, n.dgamma); give(at.be1, n.dbeta); }
     res[0] = n.dx.view(shape);
   }

@@ -176,10 +176,10 @@ struct LinearNode : public torch::autograd::Node {
     const Tensor x2 = rows_of(x.unpack());
     const Tensor dy = grads[0].reshape({x2.size(0), -1}).contiguous();
     const bool want_db = has_bias && task_should_compute_output(2);
-    auto [dz, db] = gelu_colsum(dy, z.unpack(), want_db);
+    auto [dz, db] = gelu_colsum(dy, z.unpack(), want_db ? std::optional<at::ScalarType>(b_dt) : std::nullopt);
     if (task_should_compute_output(0)) r[0] = dgrad(dz, as_dtype(w.unpack(), at::kBFloat16).contiguous(), 1.0).view(x_shape);
     if (task_should_compute_output(1)) r[1] = as_dtype(wgrad(dz, x2, 1.0, w_dt == at::kFloat ? at::kFloat : at::kBFloat16), w_dt);
-    if (want_db) r[2] = as_dtype(db, b_dt);
+    if (want_db) r[2] = db;
     return r;
   }
   void release_variables() override {

@@ -22,7 +22,8 @@ __device__ __forceinline__ bool elect_one() {
 // Programmatic dependent launch: a kernel launched with the "programmatic stream serialization" attribute may start while
 // the kernel before it in the stream is still running; griddep_wait() returns once that kernel has completed and its writes
 // are visible (at once when the attribute was not set).  griddep_launch() in the earlier kernel says that the later one may
-// be scheduled as soon as every CTA of this grid has said so or has finished.
+// be scheduled as soon as every CTA of this grid has said so or has finished.  Kernels of this library call it after their own
+// griddep_wait(), so at any time everything before a kernel's direct predecessor is complete.
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -109,7 +109,7 @@ class MINT(nn.Module):
         """The (B,T,T) mask is only built for layers that cannot take chain ids (foreign layer classes, single-pathway
         layers, or the materialised-logits combine)."""
         for layer in self.layers:
-            for sub in (layer.layers if hasattr(layer, "layers") else [layer]):
+            for sub in (layer.layers if "layers" in layer._modules else [layer]):
                 if not (isinstance(sub, _TwoPathwayLayer) and sub.use_multimer and sub._use_fused_multi_pathway):
                     return True
         return False
@@ -202,9 +202,13 @@ class MINT(nn.Module):
         # what one layer keeps for its backward pass: about 11 tensors of the size of x (the layer input, both pathways'
         # q, k, v, the attention output twice, the two residual sums) plus two 4E-wide FFN tensors; 22 x with some margin
         per_layer = 22 * x.numel() * x.element_size()
+        need = per_layer * len(self.layers)
+        from . import _lib
+        cached = _lib.host().cached_free_bytes(x.device.index)        # held by the allocator and free: reusable
+        if need <= 0.7 * cached:
+            return False                                              # (asking the driver takes it milliseconds)
         free, _ = torch.cuda.mem_get_info(x.device)
-        free += torch.cuda.memory_reserved(x.device) - torch.cuda.memory_allocated(x.device)   # cached blocks are reusable
-        return per_layer * len(self.layers) > 0.7 * free
+        return need > 0.7 * (free + cached)
 
     @classmethod
     def from_config(cls, model_size: str, fp8: bool = False, use_erf_gelu: bool = False) -> "MINT":
