@@ -1,391 +1,527 @@
 // fp32 CUDA-core kernels for the combined-softmax multimer attention (forward, dQ, dK/dV).
 //
-// They serve the fp32 configuration (bit-level agreement with the PyTorch path to ~1e-6) and head sizes the
-// tensor-core kernels do not cover.  Every result is produced in a fixed order: no atomics.
+// They serve the fp32 configuration (agreement with the PyTorch path to ~1e-6), and bf16 tensors where a caller asks for fp32
+// arithmetic.  Every result is produced in a fixed order: no atomics.
 //
-// Work split: G = D/8 threads share one row (query row in forward and dQ, key row in dK/dV); each owns 8
-// consecutive head dimensions of the row's vectors and accumulators, dot products are completed with
-// xor-shuffles inside the group.  A block of 128 threads covers 128/G rows and walks the other sequence
-// axis in tiles of 32 staged in shared memory (32 = one word of the packed mask).
+// Bound by the fp32 multiply-adds: 2 D per query, key in the forward pass, 7 D in the backward pass.  A block of 128 threads is
+// 8 row groups x 16 column lanes: a thread owns R rows (queries in forward and dQ, keys in dK/dV) and, of every tile of 64 along
+// the other axis, the four columns lane, lane + 16, lane + 32, lane + 48.  So a 16-byte shared-memory read feeds 8 to 16 packed
+// multiply-adds, the R x D accumulators stay in registers over the whole walk (each thread sums its own columns; the 16 lanes of a
+// row group meet once, at the end), and a tile costs no reduction beyond the row maximum.  One dot product per D / 8 threads with
+// shuffles inside, as before, spent ten instructions per multiply-add of useful work: B4 H20 T401 D16 forward 222 -> 50 us, forward
+// + backward 569 -> 207 us.
+//
+// The backward kernels run per pathway (grid dimension): with the log-sum-exp known a pathway's gradients involve only its own
+// pairs, and one pathway's accumulators fit the registers.  Tiles are skipped or restricted to a pathway by the 64 x 64 class table.
 #include "common.cuh"
 
 namespace mintb {
 
 constexpr int kSimtThreads = 128;
-constexpr int kSimtTile = 32;
-
-template <int G>
-__device__ __forceinline__ float group_sum(float v) {
-#pragma unroll
-  for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
-// Loads row `t` of x[T][D] (head already selected) into dst[D] (shared), rotating it if cos/sin are given:
-// y[d] = x[d] cos - x[d+h] sin (d < h), y[d] = x[d] cos + x[d-h] sin (d >= h)   (rotary_embedding.py:16-24).
-template <typename T, int D>
-__device__ __forceinline__ void stage_row(const T* __restrict__ x, int t, int Tlen, const float* cos_tab,
-                                          const float* sin_tab, float* dst, int lane, int nlanes, size_t row_stride = D) {
-  constexpr int h = D / 2;
-  for (int d = lane; d < D; d += nlanes) {
-    float v = 0.f;
-    if (t < Tlen) {
-      v = ld_f(x + size_t(t) * row_stride + d);
-      if (cos_tab != nullptr) {
-        int f = d < h ? d : d - h;
-        float c = cos_tab[size_t(t) * h + f], s = sin_tab[size_t(t) * h + f];
-        float partner = d < h ? -ld_f(x + size_t(t) * row_stride + d + h) : ld_f(x + size_t(t) * row_stride + d - h);
-        v = v * c + partner * s;
-      }
-    }
-    dst[d] = v;
-  }
-}
+constexpr int kLanes = 16;            // column lanes
+constexpr int kGroups = 8;            // row groups
+constexpr int kSimtTile = 64;         // columns per tile: four per lane, and the granularity of the class table
+static_assert(kSimtTile == kClassTile, "a tile is one entry of the class table");
 
 struct SimtParams {
   const void *q_s, *k_s, *v_s, *q_c, *k_c, *v_c;
   const uint32_t *bits, *bitsT, *kpad;
+  const uint8_t* cls;
   const float *cos_tab, *sin_tab;
   void* out;
   float* lse;
   const void* d_out;
   void *dq_s, *dk_s, *dv_s, *dq_c, *dk_c, *dv_c;
   float* delta;  // [B][H][T]
-  int B, H, T, TW;
+  int B, H, T, TW, NT;
   float scale;
   size_t o_row, o_bh;   // element strides of out and d_out: between queries, between (batch, head) pairs
-  int sqrt_sm;  // square-root softmax: out = sum_j sqrt(p_j) v_j (mu_scaling/layer.py:162-163)
 };
 
-// ------------------------------------------------------------------------------------------------ forward
-template <typename T, int D>
-__global__ void __launch_bounds__(kSimtThreads) attn_fwd_simt_kernel(SimtParams p) {
-  constexpr int G = D / 8, R = kSimtThreads / G, KT = kSimtTile;
-  __shared__ __align__(16) float sq_s[R][D], sq_c[R][D];
-  __shared__ __align__(16) float sk_s[KT][D], sk_c[KT][D], sv_s[KT][D], sv_c[KT][D];
+namespace {
 
-  const int bh = blockIdx.y, b = bh / p.H;
-  const int r = threadIdx.x / G, g = threadIdx.x % G;
-  const int i = blockIdx.x * R + r;
-  const size_t head = size_t(bh) * p.T * D;
-  const T* q_s = static_cast<const T*>(p.q_s) + head;
-  const T* k_s = static_cast<const T*>(p.k_s) + head;
-  const T* v_s = static_cast<const T*>(p.v_s) + head;
-  const T* q_c = static_cast<const T*>(p.q_c) + head;
-  const T* k_c = static_cast<const T*>(p.k_c) + head;
-  const T* v_c = static_cast<const T*>(p.v_c) + head;
+__device__ __forceinline__ uint64_t pk(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void upk(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// Four consecutive values of a shared-memory row as two pairs.
+struct Four { uint64_t a, b; };
+__device__ __forceinline__ Four lds4(const float* p) {
+  const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p);
+  return {v.x, v.y};
+}
 
-  stage_row<T, D>(q_s, i, p.T, p.cos_tab, p.sin_tab, sq_s[r], g, G);
-  stage_row<T, D>(q_c, i, p.T, nullptr, nullptr, sq_c[r], g, G);
-  __syncwarp();
-  float qs[8], qc[8], acc[8];
-#pragma unroll
-  for (int d = 0; d < 8; ++d) {
-    qs[d] = sq_s[r][g * 8 + d];
-    qc[d] = sq_c[r][g * 8 + d];
-    acc[d] = 0.f;
-  }
-  const float c2 = p.scale * kLog2e;
-  float m = -INFINITY, l = 0.f;
-  const int irow = i < p.T ? i : p.T - 1;  // rows past T compute on a valid row and are not stored
-  const uint32_t* mrow = p.bits + (size_t(b) * p.T + irow) * p.TW;
+__device__ __forceinline__ float4 ldg4(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
+__device__ __forceinline__ float4 ldg4(const __nv_bfloat16* p) {
+  const uint2 u = __ldg(reinterpret_cast<const uint2*>(p));
+  return make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u), __uint_as_float(u.y << 16), __uint_as_float(u.y & 0xffff0000u));
+}
+__device__ __forceinline__ void stg4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ void stg4(__nv_bfloat16* p, float4 v) {
+  st_f(p, v.x); st_f(p + 1, v.y); st_f(p + 2, v.z); st_f(p + 3, v.w);
+}
 
-  for (int j0 = 0; j0 < p.T; j0 += KT) {
-    const uint32_t valid = ~p.kpad[size_t(b) * p.TW + j0 / 32];
-    if (valid == 0u) continue;  // block-uniform: every key of the tile is padded
-    __syncthreads();
-    for (int jj = threadIdx.x / 32; jj < KT; jj += kSimtThreads / 32) {
-      const int lane = threadIdx.x % 32;
-      stage_row<T, D>(k_s, j0 + jj, p.T, p.cos_tab, p.sin_tab, sk_s[jj], lane, 32);
-      stage_row<T, D>(k_c, j0 + jj, p.T, nullptr, nullptr, sk_c[jj], lane, 32);
-      stage_row<T, D>(v_s, j0 + jj, p.T, nullptr, nullptr, sv_s[jj], lane, 32);
-      stage_row<T, D>(v_c, j0 + jj, p.T, nullptr, nullptr, sv_c[jj], lane, 32);
-    }
-    __syncthreads();
-    const uint32_t cross = mrow[j0 / 32];
-    float s[KT];
-    float tmax = -INFINITY;
-#pragma unroll
-    for (int jj = 0; jj < KT; ++jj) {
-      const bool x = (cross >> jj) & 1u;
-      const float* kk = x ? &sk_c[jj][g * 8] : &sk_s[jj][g * 8];
-      float part = 0.f;
-#pragma unroll
-      for (int d = 0; d < 8; ++d) part = fmaf(x ? qc[d] : qs[d], kk[d], part);
-      part = group_sum<G>(part);
-      s[jj] = ((valid >> jj) & 1u) ? part * c2 : -INFINITY;
-      tmax = fmaxf(tmax, s[jj]);
-    }
-    const float m_new = fmaxf(m, tmax);  // tile has at least one valid key, so m_new is finite
-    // square-root softmax accumulates sqrt(p) v: the terms are exp2((s - m) / 2), the row sum stays sum exp2(s - m)
-    const float alpha = exp2f(m - m_new);
-    const float alpha_acc = p.sqrt_sm ? exp2f(0.5f * (m - m_new)) : alpha;
-    l *= alpha;
-#pragma unroll
-    for (int d = 0; d < 8; ++d) acc[d] *= alpha_acc;
-#pragma unroll
-    for (int jj = 0; jj < KT; ++jj) {
-      float pj;
-      if (p.sqrt_sm) {
-        pj = exp2f(0.5f * (s[jj] - m_new));
-        l = fmaf(pj, pj, l);
-      } else {
-        pj = exp2f(s[jj] - m_new);
-        l += pj;
+// Rows [r0, r0 + ROWS) of x[T][..] into dst[ROWS][D + 4] (zeros past T), rotated when tables are given:
+// y[d] = x[d] cos - x[d+h] sin (d < h), y[d] = x[d] cos + x[d-h] sin (d >= h)   (rotary_embedding.py:16-24).
+// The pad of four keeps the 16-byte reads of neighbouring rows in different banks.
+template <typename T, int D, int ROWS>
+__device__ __forceinline__ void stage(const T* __restrict__ x, size_t row_stride, int r0, int Tlen, const float* __restrict__ cos_tab,
+                                      const float* __restrict__ sin_tab, float* __restrict__ dst) {
+  constexpr int LD = D + 4, h = D / 2, PER = h / 4, N = ROWS * PER;
+#pragma unroll 2
+  for (int i0 = 0; i0 < N; i0 += kSimtThreads) {
+    const int i = i0 + threadIdx.x;
+    if (N % kSimtThreads != 0 && i >= N) break;
+    const int r = i / PER, c = i % PER * 4, t = r0 + r;
+    float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
+    if (t < Tlen) {
+      lo = ldg4(x + size_t(t) * row_stride + c);
+      hi = ldg4(x + size_t(t) * row_stride + c + h);
+      if (cos_tab != nullptr) {
+        const float4 cs = ldg4(cos_tab + size_t(t) * h + c), sn = ldg4(sin_tab + size_t(t) * h + c);
+        const float4 a = lo, b = hi;
+        lo = make_float4(a.x * cs.x - b.x * sn.x, a.y * cs.y - b.y * sn.y, a.z * cs.z - b.z * sn.z, a.w * cs.w - b.w * sn.w);
+        hi = make_float4(b.x * cs.x + a.x * sn.x, b.y * cs.y + a.y * sn.y, b.z * cs.z + a.z * sn.z, b.w * cs.w + a.w * sn.w);
       }
-      const float* vv = ((cross >> jj) & 1u) ? &sv_c[jj][g * 8] : &sv_s[jj][g * 8];
-#pragma unroll
-      for (int d = 0; d < 8; ++d) acc[d] = fmaf(pj, vv[d], acc[d]);
     }
-    m = m_new;
+    *reinterpret_cast<float4*>(dst + r * LD + c) = lo;
+    *reinterpret_cast<float4*>(dst + r * LD + c + h) = hi;
   }
+}
+
+// s[r][k] = a[row r] . b[column k] over D: R rows at `a` (stride LD) against the lane's four rows of `b` (16 apart).
+template <int R, int D>
+__device__ __forceinline__ void dots(const float* __restrict__ a, const float* __restrict__ b, float (&s)[R][4]) {
+  constexpr int LD = D + 4;
+  uint64_t acc[R][4];
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) acc[r][k] = 0ull;
+#pragma unroll 2
+  for (int d = 0; d < D; d += 4) {
+    Four x[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) x[r] = lds4(a + r * LD + d);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const Four y = lds4(b + k * kLanes * LD + d);
+#pragma unroll
+      for (int r = 0; r < R; ++r) acc[r][k] = fma2(x[r].b, y.b, fma2(x[r].a, y.a, acc[r][k]));
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      float u, v;
+      upk(acc[r][k], u, v);
+      s[r][k] = u + v;
+    }
+}
+
+// Keeps one phase's shared-memory reads from being moved into another's, where no registers are left for them.
+__device__ __forceinline__ void phase() { asm volatile("" ::: "memory"); }
+
+// acc[r][:] += sum_k w[r][k] * b[column k][:]
+template <int R, int D>
+__device__ __forceinline__ void axpy(uint64_t (&acc)[R][D / 2], const float (&w)[R][4], const float* __restrict__ b) {
+  constexpr int LD = D + 4;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    phase();
+    uint64_t ww[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) ww[r] = pk(w[r][k], w[r][k]);
+#pragma unroll
+    for (int d = 0; d < D; d += 4) {
+      const Four y = lds4(b + k * kLanes * LD + d);
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        acc[r][d / 2] = fma2(ww[r], y.a, acc[r][d / 2]);
+        acc[r][d / 2 + 1] = fma2(ww[r], y.b, acc[r][d / 2 + 1]);
+      }
+    }
+  }
+}
+
+// One step of the sum over the lanes: the lanes that differ in bit O exchange halves of their 2 N values and keep N sums.
+template <int O, int N, int M>
+__device__ __forceinline__ void fold(float (&v)[M], int lane) {
+  const bool up = (lane & O) != 0;
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const float send = up ? v[i] : v[i + N], keep = up ? v[i + N] : v[i];
+    v[i] = keep + __shfl_xor_sync(0xffffffffu, send, O);
+  }
+}
+// Sum over the 16 lanes of a row group: afterwards lane x holds elements [x N, (x + 1) N) of the R x D accumulators, N = R D / 16.
+template <int R, int D>
+__device__ __forceinline__ void lane_sum(const uint64_t (&acc)[R][D / 2], int lane, float (&out)[R * D / kLanes]) {
+  float v[R * D];
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+#pragma unroll
+    for (int d = 0; d < D / 2; ++d) upk(acc[r][d], v[r * D + 2 * d], v[r * D + 2 * d + 1]);
+  fold<8, R * D / 2>(v, lane);
+  fold<4, R * D / 4>(v, lane);
+  fold<2, R * D / 8>(v, lane);
+  fold<1, R * D / 16>(v, lane);
+#pragma unroll
+  for (int i = 0; i < R * D / kLanes; ++i) out[i] = v[i];
+}
+__device__ __forceinline__ float lanes_sum(float v) {
+#pragma unroll
+  for (int o = kLanes / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+__device__ __forceinline__ float lanes_max(float v) {
+#pragma unroll
+  for (int o = kLanes / 2; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+  return v;
+}
+
+// Writes the lane's N elements of its row (elements [lane N, ..) of R rows of D) scaled by f, un-rotated when tables are given:
+// R^T: dx_lo = dy_lo c + dy_hi s, dx_hi = dy_hi c - dy_lo s; the partner dimensions are half a row away, in another lane.
+template <typename T, int R, int D>
+__device__ __forceinline__ void write_rows(float (&v)[R * D / kLanes], int lane, T* __restrict__ base, size_t row_stride, int row0, int Tlen, float f,
+                                           const float* __restrict__ cos_tab, const float* __restrict__ sin_tab) {
+  constexpr int N = R * D / kLanes, h = D / 2, LPR = kLanes / R;   // lanes per row
+  const int row = row0 + lane / LPR, d0 = lane % LPR * N;
+  float o[N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) o[i] = __shfl_xor_sync(0xffffffffu, v[i], LPR / 2);
+  if (row >= Tlen) return;
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    float y = v[i];
+    if (cos_tab != nullptr) {
+      const bool low = d0 < h;
+      const int c = (low ? d0 : d0 - h) + i;
+      const float cs = __ldg(cos_tab + size_t(row) * h + c), sn = __ldg(sin_tab + size_t(row) * h + c);
+      y = low ? y * cs + o[i] * sn : y * cs - o[i] * sn;
+    }
+    o[i] = y * f;
+  }
+#pragma unroll
+  for (int i = 0; i < N; i += 4) stg4(base + size_t(row) * row_stride + d0 + i, make_float4(o[i], o[i + 1], o[i + 2], o[i + 3]));
+}
+
+// ------------------------------------------------------------------------------------------------ forward
+template <int D> constexpr int fwd_rows() { return D == 64 ? 2 : 4; }
+template <int D> constexpr int fwd_smem() { return (2 * kGroups * fwd_rows<D>() + 4 * kSimtTile) * (D + 4) * 4; }
+
+template <typename T, int D, bool SQ>
+__global__ void __launch_bounds__(kSimtThreads, D == 16 ? 3 : 2) attn_fwd_simt_kernel(SimtParams p) {
+  constexpr int R = fwd_rows<D>(), ROWS = kGroups * R, LD = D + 4;
+  extern __shared__ __align__(16) float smem_f[];
+  float *sq_s = smem_f, *sq_c = sq_s + ROWS * LD, *sk_s = sq_c + ROWS * LD, *sk_c = sk_s + kSimtTile * LD, *sv_s = sk_c + kSimtTile * LD,
+        *sv_c = sv_s + kSimtTile * LD;
+  const int bh = blockIdx.y, b = bh / p.H, i0 = blockIdx.x * ROWS;
+  const int lane = threadIdx.x % kLanes, g = threadIdx.x / kLanes;
+  const size_t head = size_t(bh) * p.T * D;
+  stage<T, D, ROWS>(static_cast<const T*>(p.q_s) + head, D, i0, p.T, p.cos_tab, p.sin_tab, sq_s);
+  stage<T, D, ROWS>(static_cast<const T*>(p.q_c) + head, D, i0, p.T, nullptr, nullptr, sq_c);
+  const float c2 = p.scale * kLog2e;
+  uint64_t acc[R][D / 2];
+  float m[R], l[R];
+  const uint32_t* mrow[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+#pragma unroll
+    for (int d = 0; d < D / 2; ++d) acc[r][d] = 0ull;
+    m[r] = -INFINITY;
+    l[r] = 0.f;
+    const int i = i0 + g * R + r;   // rows past T compute on a valid row and are not stored
+    mrow[r] = p.bits + (size_t(b) * p.T + (i < p.T ? i : p.T - 1)) * p.TW;
+  }
+  const uint8_t* cls = p.cls + (size_t(b) * p.NT + i0 / kClassTile) * p.NT;
+
+  for (int kt = 0; kt < p.NT; ++kt) {
+    const uint8_t c = cls[kt];
+    const bool intra = c & kHasIntra, inter = c & kHasInter;
+    if (!intra && !inter) continue;   // block-uniform: every key of the tile is padded
+    const int j0 = kt * kSimtTile;
+    __syncthreads();
+    if (intra) {
+      stage<T, D, kSimtTile>(static_cast<const T*>(p.k_s) + head, D, j0, p.T, p.cos_tab, p.sin_tab, sk_s);
+      stage<T, D, kSimtTile>(static_cast<const T*>(p.v_s) + head, D, j0, p.T, nullptr, nullptr, sv_s);
+    }
+    if (inter) {
+      stage<T, D, kSimtTile>(static_cast<const T*>(p.k_c) + head, D, j0, p.T, nullptr, nullptr, sk_c);
+      stage<T, D, kSimtTile>(static_cast<const T*>(p.v_c) + head, D, j0, p.T, nullptr, nullptr, sv_c);
+    }
+    uint32_t pad[2], cross[R][2];
+#pragma unroll
+    for (int w = 0; w < 2; ++w) pad[w] = (c & kHasPad) ? p.kpad[size_t(b) * p.TW + 2 * kt + w] : 0u;
+    if (intra && inter) {
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int w = 0; w < 2; ++w) cross[r][w] = mrow[r][2 * kt + w];
+    }
+    __syncthreads();
+    float s[R][4];
+    dots<R, D>((intra ? sq_s : sq_c) + g * R * LD, (intra ? sk_s : sk_c) + lane * LD, s);
+    if (intra && inter) {
+      float x[R][4];
+      dots<R, D>(sq_c + g * R * LD, sk_c + lane * LD, x);
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          if ((cross[r][k / 2] >> (lane + 16 * (k % 2))) & 1u) s[r][k] = x[r][k];
+    }
+    bool grown = false;
+    float alpha[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) s[r][k] = ((pad[k / 2] >> (lane + 16 * (k % 2))) & 1u) ? -INFINITY : s[r][k] * c2;
+      const float mx = lanes_max(fmaxf(fmaxf(s[r][0], s[r][1]), fmaxf(s[r][2], s[r][3])));
+      const float m_new = fmaxf(m[r], mx);
+      // square-root softmax accumulates sqrt(p) v: the terms are exp2((s - m) / 2), the row sum stays sum exp2(s - m)
+      alpha[r] = m_new == m[r] ? 1.f : ex2(m[r] - m_new);
+      grown = grown || m_new != m[r];
+      m[r] = m_new;
+      const float ref = m_new == -INFINITY ? 0.f : m_new;   // (only padded keys so far)
+      l[r] *= alpha[r];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        s[r][k] = ex2(SQ ? 0.5f * (s[r][k] - ref) : s[r][k] - ref);
+        l[r] = SQ ? fmaf(s[r][k], s[r][k], l[r]) : l[r] + s[r][k];
+      }
+    }
+    if (__any_sync(0xffffffffu, grown)) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const float f = SQ ? sqrtf(alpha[r]) : alpha[r];
+#pragma unroll
+        for (int d = 0; d < D / 2; ++d) acc[r][d] = mul2(acc[r][d], pk(f, f));
+      }
+    }
+    if (intra && inter) {
+      float x[R][4];
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const bool is_x = (cross[r][k / 2] >> (lane + 16 * (k % 2))) & 1u;
+          x[r][k] = is_x ? s[r][k] : 0.f;
+          if (is_x) s[r][k] = 0.f;
+        }
+      axpy<R, D>(acc, x, sv_c + lane * LD);
+    }
+    axpy<R, D>(acc, s, (intra ? sv_s : sv_c) + lane * LD);
+  }
+  constexpr int N = R * D / kLanes, LPR = kLanes / R;
+  float o[N], lsum[R];
+  lane_sum<R, D>(acc, lane, o);
+#pragma unroll
+  for (int r = 0; r < R; ++r) lsum[r] = lanes_sum(l[r]);
+  float lt = lsum[0], mt = m[0];   // of the row that this lane writes
+#pragma unroll
+  for (int r = 1; r < R; ++r)
+    if (lane / LPR == r) { lt = lsum[r]; mt = m[r]; }
+  const int i = i0 + g * R + lane / LPR, d0 = lane % LPR * N;
   if (i < p.T) {
     // A row whose keys are all padded gives 0/0 = NaN, as the softmax of an all -inf row does in PyTorch.
-    const float inv = p.sqrt_sm ? rsqrtf(l) : 1.f / l;
-    T* o = static_cast<T*>(p.out) + size_t(bh) * p.o_bh + size_t(i) * p.o_row + g * 8;
+    const float inv = SQ ? rsqrtf(lt) : 1.f / lt;
+    T* dst = static_cast<T*>(p.out) + size_t(bh) * p.o_bh + size_t(i) * p.o_row + d0;
 #pragma unroll
-    for (int d = 0; d < 8; ++d) st_f(o + d, acc[d] * inv);
-    if (g == 0) p.lse[size_t(bh) * p.T + i] = (m + log2f(l)) * kLn2;
+    for (int k = 0; k < N; k += 4) stg4(dst + k, make_float4(o[k] * inv, o[k + 1] * inv, o[k + 2] * inv, o[k + 3] * inv));
+    if (lane % LPR == 0) p.lse[size_t(bh) * p.T + i] = (mt + log2f(lt)) * kLn2;
   }
 }
 
 // ------------------------------------------------------------------------------------------------ dQ (+ delta)
-// Per query row i: delta_i = dO_i . O_i;  for each key j: p = exp(s - lse), dp = dO_i . V_sel(j),
-// ds = p (dp - delta);  dq~_sel += ds * k~_sel(j).  Then dq_self = scale * R^T dq~_self, dq_cross = scale * dq~_cross.
-template <typename T, int D>
-__global__ void __launch_bounds__(kSimtThreads) attn_bwd_dq_simt_kernel(SimtParams p) {
-  constexpr int G = D / 8, R = kSimtThreads / G, KT = kSimtTile, h = D / 2;
-  __shared__ __align__(16) float sq_s[R][D], sq_c[R][D];
-  __shared__ __align__(16) float sk_s[KT][D], sk_c[KT][D], sv_s[KT][D], sv_c[KT][D];
+// Of one pathway (blockIdx.z).  delta_i = dO_i . O_i;  for each key j of the pathway: p = exp(s - lse), dp = dO_i . V(j),
+// ds = p (dp - delta);  dq~ += ds k~(j).  Then dq_self = scale R^T dq~, dq_cross = scale dq~.
+template <int D> constexpr int dq_smem() { return (2 * kGroups * fwd_rows<D>() + 2 * kSimtTile) * (D + 4) * 4; }
 
-  const int bh = blockIdx.y, b = bh / p.H;
-  const int r = threadIdx.x / G, g = threadIdx.x % G;
-  const int i = blockIdx.x * R + r;
+template <typename T, int D, bool SQ>
+__global__ void __launch_bounds__(kSimtThreads, D == 16 ? 3 : 2) attn_bwd_dq_simt_kernel(SimtParams p) {
+  constexpr int R = fwd_rows<D>(), ROWS = kGroups * R, LD = D + 4;
+  extern __shared__ __align__(16) float smem_f[];
+  float *sq = smem_f, *sg = sq + ROWS * LD, *sk = sg + ROWS * LD, *sv = sk + kSimtTile * LD;
+  const bool path = blockIdx.z != 0;   // cross
+  const int bh = blockIdx.y, b = bh / p.H, i0 = blockIdx.x * ROWS;
+  const int lane = threadIdx.x % kLanes, g = threadIdx.x / kLanes;
   const size_t head = size_t(bh) * p.T * D;
-  const T* q_s = static_cast<const T*>(p.q_s) + head;
-  const T* k_s = static_cast<const T*>(p.k_s) + head;
-  const T* v_s = static_cast<const T*>(p.v_s) + head;
-  const T* q_c = static_cast<const T*>(p.q_c) + head;
-  const T* k_c = static_cast<const T*>(p.k_c) + head;
-  const T* v_c = static_cast<const T*>(p.v_c) + head;
-  const T* o = static_cast<const T*>(p.out) + size_t(bh) * p.o_bh;
+  const float *cos_tab = path ? nullptr : p.cos_tab, *sin_tab = path ? nullptr : p.sin_tab;
+  const T* k_g = static_cast<const T*>(path ? p.k_c : p.k_s) + head;
+  const T* v_g = static_cast<const T*>(path ? p.v_c : p.v_s) + head;
   const T* dO = static_cast<const T*>(p.d_out) + size_t(bh) * p.o_bh;
-
-  stage_row<T, D>(q_s, i, p.T, p.cos_tab, p.sin_tab, sq_s[r], g, G);
-  stage_row<T, D>(q_c, i, p.T, nullptr, nullptr, sq_c[r], g, G);
-  __syncwarp();
-  const int irow = i < p.T ? i : p.T - 1;
-  float qs[8], qc[8], go[8], dqs[8], dqc[8];
-  float dpart = 0.f;
-#pragma unroll
-  for (int d = 0; d < 8; ++d) {
-    qs[d] = sq_s[r][g * 8 + d];
-    qc[d] = sq_c[r][g * 8 + d];
-    go[d] = ld_f(dO + size_t(irow) * p.o_row + g * 8 + d);
-    dpart = fmaf(go[d], ld_f(o + size_t(irow) * p.o_row + g * 8 + d), dpart);
-    dqs[d] = 0.f;
-    dqc[d] = 0.f;
-  }
-  const float delta = group_sum<G>(dpart);
-  const float c2 = p.scale * kLog2e;
-  const float lse2 = p.lse[size_t(bh) * p.T + irow] * kLog2e;
-  if (i < p.T && g == 0) p.delta[size_t(bh) * p.T + i] = delta;
-  const uint32_t* mrow = p.bits + (size_t(b) * p.T + irow) * p.TW;
-
-  for (int j0 = 0; j0 < p.T; j0 += KT) {
-    const uint32_t valid = ~p.kpad[size_t(b) * p.TW + j0 / 32];
-    if (valid == 0u) continue;
-    __syncthreads();
-    for (int jj = threadIdx.x / 32; jj < KT; jj += kSimtThreads / 32) {
-      const int lane = threadIdx.x % 32;
-      stage_row<T, D>(k_s, j0 + jj, p.T, p.cos_tab, p.sin_tab, sk_s[jj], lane, 32);
-      stage_row<T, D>(k_c, j0 + jj, p.T, nullptr, nullptr, sk_c[jj], lane, 32);
-      stage_row<T, D>(v_s, j0 + jj, p.T, nullptr, nullptr, sv_s[jj], lane, 32);
-      stage_row<T, D>(v_c, j0 + jj, p.T, nullptr, nullptr, sv_c[jj], lane, 32);
-    }
-    __syncthreads();
-    const uint32_t cross = mrow[j0 / 32];
-#pragma unroll 4
-    for (int jj = 0; jj < KT; ++jj) {
-      if (!((valid >> jj) & 1u)) continue;  // group-uniform
-      const bool x = (cross >> jj) & 1u;
-      const float* kk = x ? &sk_c[jj][g * 8] : &sk_s[jj][g * 8];
-      const float* vv = x ? &sv_c[jj][g * 8] : &sv_s[jj][g * 8];
-      float sp = 0.f, dp = 0.f;
-#pragma unroll
-      for (int d = 0; d < 8; ++d) {
-        sp = fmaf(x ? qc[d] : qs[d], kk[d], sp);
-        dp = fmaf(go[d], vv[d], dp);
-      }
-      sp = group_sum<G>(sp);
-      dp = group_sum<G>(dp);
-      // softmax: ds = p (dp - delta).  square-root softmax, r = sqrt(p): ds = r (dp - r delta) / 2
-      float ds;
-      if (p.sqrt_sm) {
-        const float rj = exp2f(0.5f * (sp * c2 - lse2));
-        ds = 0.5f * rj * (dp - rj * delta);
-      } else {
-        ds = exp2f(sp * c2 - lse2) * (dp - delta);
-      }
-      if (x) {
-#pragma unroll
-        for (int d = 0; d < 8; ++d) dqc[d] = fmaf(ds, kk[d], dqc[d]);
-      } else {
-#pragma unroll
-        for (int d = 0; d < 8; ++d) dqs[d] = fmaf(ds, kk[d], dqs[d]);
-      }
-    }
-  }
-  // Un-rotate the self-pathway gradient through shared memory (the partner dimension lives in another thread).
+  const T* o = static_cast<const T*>(p.out) + size_t(bh) * p.o_bh;
+  stage<T, D, ROWS>(static_cast<const T*>(path ? p.q_c : p.q_s) + head, D, i0, p.T, cos_tab, sin_tab, sq);
+  stage<T, D, ROWS>(dO, p.o_row, i0, p.T, nullptr, nullptr, sg);
   __syncthreads();
+  const float c2 = p.scale * kLog2e;
+  uint64_t acc[R][D / 2];
+  float delta[R], lse2[R];
+  const uint32_t* mrow[R];
 #pragma unroll
-  for (int d = 0; d < 8; ++d) sq_s[r][g * 8 + d] = dqs[d];
-  __syncwarp();
-  if (i < p.T) {
-    T* oq_s = static_cast<T*>(p.dq_s) + head + size_t(i) * D;
-    T* oq_c = static_cast<T*>(p.dq_c) + head + size_t(i) * D;
+  for (int r = 0; r < R; ++r) {
 #pragma unroll
-    for (int d = 0; d < 8; ++d) {
-      const int dd = g * 8 + d;
-      float v = dqs[d];
-      if (p.cos_tab != nullptr) {
-        const int f = dd < h ? dd : dd - h;
-        const float c = p.cos_tab[size_t(i) * h + f], s = p.sin_tab[size_t(i) * h + f];
-        v = dd < h ? v * c + sq_s[r][dd + h] * s : v * c - sq_s[r][dd - h] * s;
-      }
-      st_f(oq_s + dd, v * p.scale);
-      st_f(oq_c + dd, dqc[d] * p.scale);
-    }
+    for (int d = 0; d < D / 2; ++d) acc[r][d] = 0ull;
+    const int i = i0 + g * R + r, ic = i < p.T ? i : p.T - 1;
+    float part = 0.f;
+#pragma unroll
+    for (int d = lane; d < D; d += kLanes) part = fmaf(sg[(g * R + r) * LD + d], ld_f(o + size_t(ic) * p.o_row + d), part);
+    delta[r] = lanes_sum(part);
+    lse2[r] = p.lse[size_t(bh) * p.T + ic] * kLog2e;
+    if (!path && lane == 0 && i < p.T) p.delta[size_t(bh) * p.T + i] = delta[r];
+    mrow[r] = p.bits + (size_t(b) * p.T + ic) * p.TW;
   }
+  const uint8_t* cls = p.cls + (size_t(b) * p.NT + i0 / kClassTile) * p.NT;
+  const uint8_t mine = path ? kHasInter : kHasIntra, other = path ? kHasIntra : kHasInter;
+
+  for (int kt = 0; kt < p.NT; ++kt) {
+    const uint8_t c = cls[kt];
+    if (!(c & mine)) continue;
+    const int j0 = kt * kSimtTile;
+    __syncthreads();
+    stage<T, D, kSimtTile>(k_g, D, j0, p.T, cos_tab, sin_tab, sk);
+    stage<T, D, kSimtTile>(v_g, D, j0, p.T, nullptr, nullptr, sv);
+    uint32_t drop[R][2];   // keys of this row that are padded or belong to the other pathway
+#pragma unroll
+    for (int w = 0; w < 2; ++w) {
+      const uint32_t pad = (c & kHasPad) ? p.kpad[size_t(b) * p.TW + 2 * kt + w] : 0u;
+#pragma unroll
+      for (int r = 0; r < R; ++r) drop[r][w] = pad | ((c & other) ? (path ? ~mrow[r][2 * kt + w] : mrow[r][2 * kt + w]) : 0u);
+    }
+    __syncthreads();
+    float s[R][4], dp[R][4];
+    dots<R, D>(sq + g * R * LD, sk + lane * LD, s);
+    phase();
+    dots<R, D>(sg + g * R * LD, sv + lane * LD, dp);
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        // softmax: ds = p (dp - delta).  square-root softmax, w = sqrt(p): ds = w (dp - w delta) / 2
+        const float x = s[r][k] * c2 - lse2[r], w = ex2(SQ ? 0.5f * x : x);
+        const float ds = SQ ? 0.5f * w * (dp[r][k] - w * delta[r]) : w * (dp[r][k] - delta[r]);
+        s[r][k] = ((drop[r][k / 2] >> (lane + 16 * (k % 2))) & 1u) ? 0.f : ds;
+      }
+    axpy<R, D>(acc, s, sk + lane * LD);
+  }
+  float v[R * D / kLanes];
+  lane_sum<R, D>(acc, lane, v);
+  write_rows<T, R, D>(v, lane, static_cast<T*>(path ? p.dq_c : p.dq_s) + head, D, i0 + g * R, p.T, p.scale, cos_tab, sin_tab);
 }
 
 // ------------------------------------------------------------------------------------------------ dK, dV
-// Per key row j, looping over query tiles:  dv_sel += p * dO_i;  dk~_sel += ds * scale * q~_sel(i).
-template <typename T, int D>
-__global__ void __launch_bounds__(kSimtThreads) attn_bwd_dkv_simt_kernel(SimtParams p) {
-  constexpr int G = D / 8, R = kSimtThreads / G, QT = kSimtTile, h = D / 2;
-  __shared__ __align__(16) float sk_s[R][D], sk_c[R][D];
-  __shared__ __align__(16) float sq_s[QT][D], sq_c[QT][D], sdo[QT][D];
-  __shared__ float slse2[QT], sdelta[QT];
+// Of one pathway, per key row j, over query tiles:  dv += p dO_i;  dk~ += ds scale q~(i).
+template <int D> constexpr int dkv_rows() { return D == 16 ? 4 : D == 32 ? 2 : 1; }
+template <int D> constexpr int dkv_smem() { return (2 * kGroups * dkv_rows<D>() + 2 * kSimtTile) * (D + 4) * 4 + 2 * kSimtTile * 4; }
 
-  const int bh = blockIdx.y, b = bh / p.H;
-  const int r = threadIdx.x / G, g = threadIdx.x % G;
-  const int j = blockIdx.x * R + r;
+template <typename T, int D, bool SQ>
+__global__ void __launch_bounds__(kSimtThreads, 2) attn_bwd_dkv_simt_kernel(SimtParams p) {
+  constexpr int R = dkv_rows<D>(), ROWS = kGroups * R, LD = D + 4;
+  extern __shared__ __align__(16) float smem_f[];
+  float *sk = smem_f, *sv = sk + ROWS * LD, *sq = sv + ROWS * LD, *sg = sq + kSimtTile * LD, *slse2 = sg + kSimtTile * LD, *sdelta = slse2 + kSimtTile;
+  const bool path = blockIdx.z != 0;
+  const int bh = blockIdx.y, b = bh / p.H, j0 = blockIdx.x * ROWS;
+  const int lane = threadIdx.x % kLanes, g = threadIdx.x / kLanes;
   const size_t head = size_t(bh) * p.T * D;
-  const T* q_s = static_cast<const T*>(p.q_s) + head;
-  const T* k_s = static_cast<const T*>(p.k_s) + head;
-  const T* v_s = static_cast<const T*>(p.v_s) + head;
-  const T* q_c = static_cast<const T*>(p.q_c) + head;
-  const T* k_c = static_cast<const T*>(p.k_c) + head;
-  const T* v_c = static_cast<const T*>(p.v_c) + head;
+  const float *cos_tab = path ? nullptr : p.cos_tab, *sin_tab = path ? nullptr : p.sin_tab;
+  const T* q_g = static_cast<const T*>(path ? p.q_c : p.q_s) + head;
   const T* dO = static_cast<const T*>(p.d_out) + size_t(bh) * p.o_bh;
-
-  stage_row<T, D>(k_s, j, p.T, p.cos_tab, p.sin_tab, sk_s[r], g, G);
-  stage_row<T, D>(k_c, j, p.T, nullptr, nullptr, sk_c[r], g, G);
-  __syncwarp();
-  const int jrow = j < p.T ? j : p.T - 1;
-  float ks[8], kc[8], vs[8], vc[8], dks[8], dkc[8], dvs[8], dvc[8];
-#pragma unroll
-  for (int d = 0; d < 8; ++d) {
-    ks[d] = sk_s[r][g * 8 + d];
-    kc[d] = sk_c[r][g * 8 + d];
-    vs[d] = ld_f(v_s + size_t(jrow) * D + g * 8 + d);
-    vc[d] = ld_f(v_c + size_t(jrow) * D + g * 8 + d);
-    dks[d] = dkc[d] = dvs[d] = dvc[d] = 0.f;
-  }
+  stage<T, D, ROWS>(static_cast<const T*>(path ? p.k_c : p.k_s) + head, D, j0, p.T, cos_tab, sin_tab, sk);
+  stage<T, D, ROWS>(static_cast<const T*>(path ? p.v_c : p.v_s) + head, D, j0, p.T, nullptr, nullptr, sv);
   const float c2 = p.scale * kLog2e;
-  const bool key_valid = (j < p.T) && !((p.kpad[size_t(b) * p.TW + jrow / 32] >> (jrow % 32)) & 1u);
-  const uint32_t* mrow = p.bitsT + (size_t(b) * p.T + jrow) * p.TW;
+  uint64_t dk[R][D / 2], dv[R][D / 2];
+  const uint32_t* mrow[R];
+  bool dead[R];   // padded keys have probability zero
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+#pragma unroll
+    for (int d = 0; d < D / 2; ++d) dk[r][d] = dv[r][d] = 0ull;
+    const int j = j0 + g * R + r, jc = j < p.T ? j : p.T - 1;
+    dead[r] = j >= p.T || ((p.kpad[size_t(b) * p.TW + jc / 32] >> (jc % 32)) & 1u);
+    mrow[r] = p.bitsT + (size_t(b) * p.T + jc) * p.TW;
+  }
+  const uint8_t* cls = p.cls + size_t(b) * p.NT * p.NT + j0 / kClassTile;
+  const uint8_t mine = path ? kHasInter : kHasIntra, other = path ? kHasIntra : kHasInter;
 
-  for (int i0 = 0; i0 < p.T; i0 += QT) {
+  for (int qt = 0; qt < p.NT; ++qt) {
+    const uint8_t c = cls[size_t(qt) * p.NT];
+    if (!(c & mine)) continue;
+    const int i0 = qt * kSimtTile;
     __syncthreads();
-    for (int ii = threadIdx.x / 32; ii < QT; ii += kSimtThreads / 32) {
-      const int lane = threadIdx.x % 32;
-      stage_row<T, D>(q_s, i0 + ii, p.T, p.cos_tab, p.sin_tab, sq_s[ii], lane, 32);
-      stage_row<T, D>(q_c, i0 + ii, p.T, nullptr, nullptr, sq_c[ii], lane, 32);
-      stage_row<T, D>(dO, i0 + ii, p.T, nullptr, nullptr, sdo[ii], lane, 32, p.o_row);
-    }
-    if (threadIdx.x < QT) {
+    stage<T, D, kSimtTile>(q_g, D, i0, p.T, cos_tab, sin_tab, sq);
+    stage<T, D, kSimtTile>(dO, p.o_row, i0, p.T, nullptr, nullptr, sg);
+    if (threadIdx.x < kSimtTile) {
       const int i = i0 + threadIdx.x;
       slse2[threadIdx.x] = i < p.T ? p.lse[size_t(bh) * p.T + i] * kLog2e : INFINITY;  // p = exp2(-inf) = 0
       sdelta[threadIdx.x] = i < p.T ? p.delta[size_t(bh) * p.T + i] : 0.f;
     }
+    uint32_t drop[R][2];
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int w = 0; w < 2; ++w)
+        drop[r][w] = dead[r] ? 0xffffffffu : (c & other) ? (path ? ~mrow[r][2 * qt + w] : mrow[r][2 * qt + w]) : 0u;
     __syncthreads();
-    const uint32_t cross = mrow[i0 / 32];
-#pragma unroll 4
-    for (int ii = 0; ii < QT; ++ii) {
-      const bool x = (cross >> ii) & 1u;
-      const float* qq = x ? &sq_c[ii][g * 8] : &sq_s[ii][g * 8];
-      const float* gg = &sdo[ii][g * 8];
-      float sp = 0.f, dp = 0.f;
+    float s[R][4], dp[R][4];
+    dots<R, D>(sk + g * R * LD, sq + lane * LD, s);
+    phase();
+    dots<R, D>(sv + g * R * LD, sg + lane * LD, dp);
 #pragma unroll
-      for (int d = 0; d < 8; ++d) {
-        sp = fmaf(qq[d], x ? kc[d] : ks[d], sp);
-        dp = fmaf(gg[d], x ? vc[d] : vs[d], dp);
-      }
-      sp = group_sum<G>(sp);
-      dp = group_sum<G>(dp);
-      // A padded key has probability zero; every thread still takes part in the shuffles above.
-      // (pj multiplies dO in dV: p for the softmax, sqrt(p) for the square-root softmax)
-      float pj, ds;
-      if (p.sqrt_sm) {
-        pj = key_valid ? exp2f(0.5f * (sp * c2 - slse2[ii])) : 0.f;
-        ds = 0.5f * pj * (dp - pj * sdelta[ii]) * p.scale;
-      } else {
-        pj = key_valid ? exp2f(sp * c2 - slse2[ii]) : 0.f;
-        ds = pj * (dp - sdelta[ii]) * p.scale;
-      }
-      if (x) {
+    for (int k = 0; k < 4; ++k) {
+      const float lse2 = slse2[lane + 16 * k], delta = sdelta[lane + 16 * k];
 #pragma unroll
-        for (int d = 0; d < 8; ++d) {
-          dvc[d] = fmaf(pj, gg[d], dvc[d]);
-          dkc[d] = fmaf(ds, qq[d], dkc[d]);
-        }
-      } else {
-#pragma unroll
-        for (int d = 0; d < 8; ++d) {
-          dvs[d] = fmaf(pj, gg[d], dvs[d]);
-          dks[d] = fmaf(ds, qq[d], dks[d]);
-        }
+      for (int r = 0; r < R; ++r) {
+        // (w multiplies dO in dV: p for the softmax, sqrt(p) for the square-root softmax)
+        const float x = s[r][k] * c2 - lse2, w = ex2(SQ ? 0.5f * x : x);
+        const float ds = (SQ ? 0.5f * w * (dp[r][k] - w * delta) : w * (dp[r][k] - delta)) * p.scale;
+        const bool no = (drop[r][k / 2] >> (lane + 16 * (k % 2))) & 1u;
+        s[r][k] = no ? 0.f : w;
+        dp[r][k] = no ? 0.f : ds;
       }
     }
+    axpy<R, D>(dv, s, sg + lane * LD);
+    axpy<R, D>(dk, dp, sq + lane * LD);
   }
-  __syncthreads();
-#pragma unroll
-  for (int d = 0; d < 8; ++d) sk_s[r][g * 8 + d] = dks[d];
-  __syncwarp();
-  if (j < p.T) {
-    const size_t off = head + size_t(j) * D;
-#pragma unroll
-    for (int d = 0; d < 8; ++d) {
-      const int dd = g * 8 + d;
-      float v = dks[d];
-      if (p.cos_tab != nullptr) {
-        const int f = dd < h ? dd : dd - h;
-        const float c = p.cos_tab[size_t(j) * h + f], s = p.sin_tab[size_t(j) * h + f];
-        v = dd < h ? v * c + sk_s[r][dd + h] * s : v * c - sk_s[r][dd - h] * s;
-      }
-      st_f(static_cast<T*>(p.dk_s) + off + dd, v);
-      st_f(static_cast<T*>(p.dk_c) + off + dd, dkc[d]);
-      st_f(static_cast<T*>(p.dv_s) + off + dd, dvs[d]);
-      st_f(static_cast<T*>(p.dv_c) + off + dd, dvc[d]);
-    }
-  }
+  float v[R * D / kLanes];
+  lane_sum<R, D>(dv, lane, v);
+  write_rows<T, R, D>(v, lane, static_cast<T*>(path ? p.dv_c : p.dv_s) + head, D, j0 + g * R, p.T, 1.f, nullptr, nullptr);
+  lane_sum<R, D>(dk, lane, v);
+  write_rows<T, R, D>(v, lane, static_cast<T*>(path ? p.dk_c : p.dk_s) + head, D, j0 + g * R, p.T, 1.f, cos_tab, sin_tab);
 }
+
+}  // namespace
 
 // ------------------------------------------------------------------------------------------------ launchers
 static SimtParams make_params(const AttnArgs& a) {
   SimtParams p{};
   p.q_s = a.q_s; p.k_s = a.k_s; p.v_s = a.v_s; p.q_c = a.q_c; p.k_c = a.k_c; p.v_c = a.v_c;
-  p.bits = a.meta.bits; p.bitsT = a.meta.bitsT; p.kpad = a.meta.kpad;
+  p.bits = a.meta.bits; p.bitsT = a.meta.bitsT; p.kpad = a.meta.kpad; p.cls = a.meta.cls;
   p.cos_tab = a.rope ? a.rope_cos : nullptr;
   p.sin_tab = a.rope ? a.rope_sin : nullptr;
   p.out = a.out; p.lse = a.lse; p.d_out = a.d_out;
   p.dq_s = a.dq_s; p.dk_s = a.dk_s; p.dv_s = a.dv_s; p.dq_c = a.dq_c; p.dk_c = a.dk_c; p.dv_c = a.dv_c;
   p.delta = static_cast<float*>(a.workspace);
-  p.B = a.B; p.H = a.H; p.T = a.T; p.TW = a.meta.TW;
+  p.B = a.B; p.H = a.H; p.T = a.T; p.TW = a.meta.TW; p.NT = a.meta.NT;
   p.scale = a.scale;
-  p.sqrt_sm = a.sqrt_softmax ? 1 : 0;
   p.o_row = out_row_stride(a);
   p.o_bh = out_bh_stride(a);
   return p;
@@ -393,38 +529,44 @@ static SimtParams make_params(const AttnArgs& a) {
 
 size_t simt_bwd_workspace_bytes(int B, int H, int T, int D) { return align256(size_t(B) * H * T * sizeof(float)); }
 
-template <typename T, int D>
+template <typename T, int D, bool SQ>
 static cudaError_t fwd_t(const AttnArgs& a) {
-  constexpr int R = kSimtThreads / (D / 8);
-  dim3 grid((a.T + R - 1) / R, a.B * a.H);
-  attn_fwd_simt_kernel<T, D><<<grid, kSimtThreads, 0, a.stream>>>(make_params(a));
+  constexpr int rows = kGroups * fwd_rows<D>(), bytes = fwd_smem<D>();
+  constexpr auto kern = attn_fwd_simt_kernel<T, D, SQ>;
+  if (cudaError_t e = opt_in_smem<kern>(bytes); e != cudaSuccess) return e;
+  kern<<<dim3((a.T + rows - 1) / rows, a.B * a.H), kSimtThreads, bytes, a.stream>>>(make_params(a));
   count_launches(1);
   return cudaGetLastError();
 }
 
-template <typename T, int D>
+template <typename T, int D, bool SQ>
 static cudaError_t bwd_t(const AttnArgs& a) {
-  constexpr int R = kSimtThreads / (D / 8);
-  dim3 grid((a.T + R - 1) / R, a.B * a.H);
-  SimtParams p = make_params(a);
-  attn_bwd_dq_simt_kernel<T, D><<<grid, kSimtThreads, 0, a.stream>>>(p);
-  attn_bwd_dkv_simt_kernel<T, D><<<grid, kSimtThreads, 0, a.stream>>>(p);
+  constexpr int q_rows = kGroups * fwd_rows<D>(), k_rows = kGroups * dkv_rows<D>();
+  constexpr auto kq = attn_bwd_dq_simt_kernel<T, D, SQ>;
+  constexpr auto kkv = attn_bwd_dkv_simt_kernel<T, D, SQ>;
+  cudaError_t e = opt_in_smem<kq>(dq_smem<D>());
+  if (e == cudaSuccess) e = opt_in_smem<kkv>(dkv_smem<D>());
+  if (e != cudaSuccess) return e;
+  const SimtParams p = make_params(a);
+  kq<<<dim3((a.T + q_rows - 1) / q_rows, a.B * a.H, 2), kSimtThreads, dq_smem<D>(), a.stream>>>(p);
+  kkv<<<dim3((a.T + k_rows - 1) / k_rows, a.B * a.H, 2), kSimtThreads, dkv_smem<D>(), a.stream>>>(p);
   count_launches(2);
   return cudaGetLastError();
 }
 
+#define MINTB_SIMT_CASE(FN, TT, DD) return a.sqrt_softmax ? FN<TT, DD, true>(a) : FN<TT, DD, false>(a)
 #define MINTB_SIMT_DISPATCH(FN)                                                        \
   if (a.dtype == MINTB_F32) {                                                          \
     switch (a.D) {                                                                     \
-      case 16: return FN<float, 16>(a);                                                \
-      case 32: return FN<float, 32>(a);                                                \
-      case 64: return FN<float, 64>(a);                                                \
+      case 16: MINTB_SIMT_CASE(FN, float, 16);                                         \
+      case 32: MINTB_SIMT_CASE(FN, float, 32);                                         \
+      case 64: MINTB_SIMT_CASE(FN, float, 64);                                         \
     }                                                                                  \
   } else {                                                                             \
     switch (a.D) {                                                                     \
-      case 16: return FN<__nv_bfloat16, 16>(a);                                        \
-      case 32: return FN<__nv_bfloat16, 32>(a);                                        \
-      case 64: return FN<__nv_bfloat16, 64>(a);                                        \
+      case 16: MINTB_SIMT_CASE(FN, __nv_bfloat16, 16);                                 \
+      case 32: MINTB_SIMT_CASE(FN, __nv_bfloat16, 32);                                 \
+      case 64: MINTB_SIMT_CASE(FN, __nv_bfloat16, 64);                                 \
     }                                                                                  \
   }                                                                                    \
   return cudaErrorInvalidValue;
