@@ -284,6 +284,11 @@ MINTB_API size_t mintb_add_layernorm_bwd_workspace_bytes(int rows, int E);
 MINTB_API int mintb_add_layernorm_bwd(const void* dy, const void* ds_in, const void* x, const void* r, float a, float b,
                                       const void* gamma, int param_dtype, const float* stats, void* dx, void* dr, float* dgamma,
                                       float* dbeta, void* workspace, size_t workspace_bytes, int rows, int E, void* stream);
+/* Operands of n projections with LoRA adapters (bf16; w: host array of n device pointers to W [out][in]; delta [n][out][in] = B A;
+ * b [n][out][r]): merged[n][out][in] = W + scaling delta, rounded to bf16 after each step, and, when b_diag is given,
+ * b_diag[n][out][n r] = B of projection i in columns i r .. (i + 1) r, else zero: one operand for the gradients of every A. */
+MINTB_API int mintb_lora_operands(const void* const* w, const void* delta, const void* b, int n, int out, int in, int r, float scaling,
+                                  void* merged, void* b_diag, void* stream);
 /* mintb_add_layernorm_bwd with dgamma and dbeta written as `grad_dtype` (f32 or bf16); ds_apart: ds_in is another gradient of the
  * same input, added to dx = a ds after that has been rounded to bf16 (dr does not see it) */
 MINTB_API int mintb_add_layernorm_bwd_typed(const void* dy, const void* ds_in, int ds_apart, const void* x, const void* r, float a, float b,

@@ -58,6 +58,7 @@ PROTOTYPES = {
     "mintb_add_layernorm_bwd_workspace_bytes": (c_size_t, [c_int, c_int]),
     "mintb_add_layernorm_bwd": (c_int, [_P, _P, _P, _P, c_float, c_float, _P, c_int, _P, _P, _P, _P, _P, _P, c_size_t, c_int,
                                         c_int, _P]),
+    "mintb_lora_operands": (c_int, [_P, _P, _P, c_int, c_int, c_int, c_int, c_float, _P, _P, _P]),
     "mintb_add_layernorm_bwd_typed": (c_int, [_P, _P, c_int, _P, _P, c_float, c_float, _P, c_int, _P, _P, _P, _P, _P, c_int, _P, c_size_t, c_int,
                                               c_int, _P]),
     "mintb_bias_grad_workspace_bytes": (c_size_t, [c_int, c_int]),

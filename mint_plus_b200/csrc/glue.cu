@@ -673,6 +673,43 @@ __global__ void __launch_bounds__(256) qkv_grad_pack_kernel(const __nv_bfloat16*
   }
 }
 
+// ------------------------------------------------------------------------------------------------ LoRA operands
+constexpr int kLoraMax = 8;   // projections per launch
+struct LoraParams {
+  const __nv_bfloat16* w[kLoraMax];   // W [out][in]
+  const __nv_bfloat16 *delta, *b;     // B A [n][out][in], B [n][out][r]
+  __nv_bfloat16* merged;              // [n][out][in]
+  __nv_bfloat16* b_diag;              // [n][out][n r]: B of projection i in columns i r .. (i + 1) r, zeros elsewhere; may be null
+  int n, out, in, r;
+  float scaling;
+};
+
+// merged = W + scaling (B A), each step rounded to bf16 as the tensor expression rounds it, and b_diag, the B's as the operand of one
+// product that forms g B of all projections (r a multiple of eight).  Eight values per thread; HBM-bound.
+__global__ void __launch_bounds__(256) lora_operands_kernel(LoraParams p) {
+  ptx::griddep_wait();
+  ptx::griddep_launch();
+  const size_t idx = size_t(blockIdx.x) * 256 + threadIdx.x;
+  const size_t per_w = size_t(p.out) * p.in / 8, n_w = p.n * per_w;
+  if (idx < n_w) {
+    const size_t at = idx * 8;
+    float w[8], d[8];
+    unpack8(__ldg(reinterpret_cast<const uint4*>(p.w[idx / per_w]) + idx % per_w), w);
+    unpack8(__ldg(reinterpret_cast<const uint4*>(p.delta + at)), d);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) w[j] += __bfloat162float(__float2bfloat16_rn(p.scaling * d[j]));
+    *reinterpret_cast<uint4*>(p.merged + at) = pack8(w);
+  } else if (p.b_diag != nullptr) {
+    const int nr = p.n * p.r;
+    const size_t k = idx - n_w;
+    if (k >= size_t(p.n) * p.out * nr / 8) return;
+    const int row = int(k / (nr / 8)), c = int(k % (nr / 8)) * 8, i = row / p.out;
+    uint4 v = make_uint4(0u, 0u, 0u, 0u);
+    if (c / p.r == i) v = __ldg(reinterpret_cast<const uint4*>(p.b + size_t(row) * p.r + c % p.r));
+    *reinterpret_cast<uint4*>(p.b_diag + size_t(row) * nr + c) = v;
+  }
+}
+
 int fail(const char* what, cudaError_t e) {
   set_error("%s: %s", what, cudaGetErrorString(e));
   return MINTB_ECUDA;
@@ -694,6 +731,28 @@ int ln_bwd_grid_max(int rows) {
 extern "C" {
 
 using namespace mintb;
+
+int mintb_lora_operands(const void* const* w, const void* delta, const void* b, int n, int out, int in, int r, float scaling, void* merged,
+                        void* b_diag, void* stream) {
+  bool ok = w != nullptr && delta != nullptr && merged != nullptr && n > 0 && n <= kLoraMax && out > 0 && in > 0 && in % 8 == 0 &&
+            (b_diag == nullptr || (b != nullptr && r > 0 && r % 8 == 0));
+  LoraParams p{};
+  for (int i = 0; ok && i < n; ++i) {
+    p.w[i] = static_cast<const __nv_bfloat16*>(w[i]);
+    ok = w[i] != nullptr && (reinterpret_cast<uintptr_t>(w[i]) & 15) == 0;
+  }
+  if (!ok) {
+    set_error("mintb_lora_operands: 1 to 8 16-byte aligned weights, delta, merged, in a multiple of 8; b and r a multiple of 8 with b_diag");
+    return MINTB_EINVAL;
+  }
+  p.delta = static_cast<const __nv_bfloat16*>(delta); p.b = static_cast<const __nv_bfloat16*>(b);
+  p.merged = static_cast<__nv_bfloat16*>(merged); p.b_diag = static_cast<__nv_bfloat16*>(b_diag);
+  p.n = n; p.out = out; p.in = in; p.r = r; p.scaling = scaling;
+  const size_t vec = size_t(n) * out * in / 8 + (b_diag != nullptr ? size_t(n) * out * n * r / 8 : 0);
+  const cudaError_t e = launch_dependent(lora_operands_kernel, dim3(unsigned((vec + 255) / 256)), dim3(256), 0, static_cast<cudaStream_t>(stream), p);
+  count_launches(1);
+  return e == cudaSuccess ? MINTB_OK : fail("mintb_lora_operands launch", e);
+}
 
 int mintb_add_layernorm_fwd_q(const void* x, const void* r, float a, float b, const void* gamma, const void* beta, int param_dtype,
                               void* s_out, void* y_out, float* stats, int rows, int E, float eps, void* q_out, float q_inv_scale,

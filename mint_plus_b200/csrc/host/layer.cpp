@@ -11,7 +11,7 @@ namespace {
 
 // Positions in LayerPlan::params.
 struct Where {
-  int64_t ws, bs, wc, bc, wo, bo, w1, b1, w2, b2, g1, be1, g2, be2, n;
+  int64_t ws, bs, wc, bc, wo, bo, w1, b1, w2, b2, g1, be1, g2, be2, la, lb, n;   // la, lb: seven A's, seven B's
   explicit Where(const LayerPlan& p) {
     int64_t k = 0;
     ws = k; k += p.n_self;
@@ -22,11 +22,13 @@ struct Where {
     g1 = be1 = -1;
     if (!p.mu) { g1 = k++; be1 = k++; }
     g2 = k++; be2 = k++;
+    la = lb = -1;
+    if (p.lora_r > 0) { la = k; lb = k + 7; k += 14; }
     n = k;
   }
 };
 
-enum Saved { kX, kXq, kStats1, kQ0, kQ1, kQ2, kQ3, kQ4, kQ5, kOut, kLse, kO, kX1, kH2, kStats2, kZ, kA, kY2, kNumSaved };
+enum Saved { kX, kXq, kStats1, kQ0, kQ1, kQ2, kQ3, kQ4, kQ5, kOut, kLse, kO, kX1, kH2, kStats2, kZ, kA, kY2, kMerged, kARows, kBDiag, kNumSaved };
 
 }  // namespace
 
@@ -80,6 +82,24 @@ std::tuple<Tensor, OptTensor> LayerPlan::forward(const Tensor& x_in, const OptTe
     }
     const Tensor& op = fp8 ? hq : h;
 
+    // adapters: the products run on merged weights, [6E][E] of both pathways and [E][E] of the output projection
+    Tensor merged, qkv6_op = qkv6, out_op = out.w;
+    if (lora_r > 0) {
+      const void* w[7];
+      for (int i = 0; i < 7; ++i) w[i] = ptr(params[i < 3 ? at.ws + i : i < 6 ? at.wc + i - 3 : at.wo]);
+      const Tensor a_all = at::stack(at::TensorList(params).slice(at.la, 7)), b_all = at::stack(at::TensorList(params).slice(at.lb, 7));
+      const Tensor delta = at::bmm(b_all, a_all);
+      merged = e.empty({7 * E, E}, at::kBFloat16);
+      if (grad) {
+        keep_t[kARows] = a_all.view({7 * lora_r, E});
+        keep_t[kBDiag] = e.empty({7 * E, 7 * lora_r}, at::kBFloat16);
+        keep_t[kMerged] = merged;
+      }
+      check(mintb_lora_operands(w, ptr(delta), ptr(b_all), 7, E, E, lora_r, float(lora_scaling), ptr(merged), ptr(keep_t[kBDiag]), e.stream), "mintb_lora_operands");
+      qkv6_op = merged;   // (its first 6E rows)
+      out_op = merged.narrow(0, 6 * E, E);
+    }
+
     // q, k, v of both pathways, head-major, the self pathway rotated.  Packed: positions without a token are not written, and keys
     // there are masked but still multiplied by a zero probability, so they must hold finite numbers.
     AttnInputs a;
@@ -87,8 +107,8 @@ std::tuple<Tensor, OptTensor> LayerPlan::forward(const Tensor& x_in, const OptTe
     for (int k = 0; k < 6; ++k) a.q[k] = all.select(0, k);
     const int32_t* map = packed ? batch.rows32.data_ptr<int32_t>() : nullptr;
     const int in_dt = fp8 ? MINTB_E4M3 : MINTB_BF16;
-    if (qkv6.defined()) {
-      check(mintb_qkv2_fwd(ptr(op), ptr(qkv6), ptr(bias6), ptr(a.q[0]), ptr(a.q[1]), ptr(a.q[2]), ptr(a.q[3]), ptr(a.q[4]), ptr(a.q[5]), T, B, H, D, in_dt,
+    if (qkv6_op.defined()) {
+      check(mintb_qkv2_fwd(ptr(op), ptr(qkv6_op), ptr(bias6), ptr(a.q[0]), ptr(a.q[1]), ptr(a.q[2]), ptr(a.q[3]), ptr(a.q[4]), ptr(a.q[5]), T, B, H, D, in_dt,
                            param_dt(bias6, "bias"), float(qkv_self.alpha()), float(qkv_cross.alpha()), 1.f, fptr(batch.cos), fptr(batch.sin), map, rows, e.stream,
                            e.status),
             "mintb_qkv2_fwd");
@@ -111,8 +131,8 @@ std::tuple<Tensor, OptTensor> LayerPlan::forward(const Tensor& x_in, const OptTe
     // output projection with the residual sum in its epilogue
     Product po;
     po.x = fp8 ? quantize(o, out.x_scale) : o;
-    po.w = out.w; po.bias = params[at.bo]; po.alpha = out.alpha();
-    auto [x1, x1q] = linear_res_fwd(po, x, keep, add, fp8 && mu ? fc1.x_scale : 0.0);
+    po.w = out_op; po.bias = params[at.bo]; po.alpha = out.alpha();
+    auto [x1, x1q] = linear_res_fwd(po, x, keep, add, fp8 && mu ? fc1.x_scale : 0.0, lora_r > 0);
 
     Tensor h2 = x1, h2q = x1q;
     if (!mu) {
@@ -160,7 +180,8 @@ std::tuple<Tensor, OptTensor> LayerPlan::forward(const Tensor& x_in, const OptTe
     for (int k = 0; k < kNumSaved; ++k)
       if (keep_t[k].defined()) node->saved[k] = SavedVariable(keep_t[k], false);
     if (!fp8)
-      for (const Tensor& t : {qkv_self.w, qkv_cross.w, out.w, fc1.w, fc2.w}) node->weights.emplace_back(t, false);
+      for (const Tensor& t : {qkv_self.w, qkv_cross.w, out.w, fc1.w, fc2.w})
+        if (t.defined()) node->weights.emplace_back(t, false);
   }
   return {y, y8.defined() ? OptTensor(y8) : OptTensor()};
 }
@@ -234,13 +255,30 @@ variable_list LayerNode::apply(variable_list&& grads) {
       d1 = g.dx;
     }
   }
+  // adapters (shared products: every A, every B and their gradients in one operand each; the seven projections are self q, k, v,
+  // cross q, k, v and out, whose inputs and output gradients differ, so out has products of its own on the same operands)
+  const int64_t r = plan.lora_r;
+  Operand w_out = plan.out, os = plan.qkv_self, oc = plan.qkv_cross;
+  if (r > 0) {
+    os.w = s[kMerged].narrow(0, 0, 3 * E);
+    oc.w = s[kMerged].narrow(0, 3 * E, 3 * E);
+    w_out.w = s[kMerged].narrow(0, 6 * E, E);
+  }
+  const bool lora_out = r > 0 && (wants(at.la + 6) || wants(at.lb + 6)), lora_qkv = r > 0 && (any(at.la, 6) || any(at.lb, 6));
   // output projection: its result entered the sum times `add`
   Tensor d_attn;
   {
-    auto [go, dbo] = operand(plan.out, d1, Tensor(), bias_dt(at.bo));
+    auto [go, dbo] = operand(w_out, d1, Tensor(), bias_dt(at.bo));
     if (dbo.defined()) give(at.bo, plan.add == 1.0 ? dbo : dbo * plan.add);
-    if (wants(at.wo)) give(at.wo, wgrad(go, s[kO], a_w(plan.out) * plan.add, w_dt(at.wo)));
-    d_attn = dgrad(go, plan.out.w, a_in(plan.out) * plan.add);
+    if (wants(at.wo)) give(at.wo, wgrad(go, s[kO], a_w(w_out) * plan.add, w_dt(at.wo)));
+    if (lora_out) {   // dB = s g^T (x A^T), dA = s (g B)^T x
+      Product xa;
+      xa.x = s[kO];
+      xa.w = s[kARows].narrow(0, 6 * r, r);
+      if (wants(at.lb + 6)) give(at.lb + 6, wgrad(go, linear_fwd(xa).first, plan.lora_scaling, at::kBFloat16));
+      if (wants(at.la + 6)) give(at.la + 6, wgrad(dgrad(go, plan.params[at.lb + 6], 1.0), s[kO], plan.lora_scaling, at::kBFloat16));
+    }
+    d_attn = dgrad(go, w_out.w, a_in(w_out) * plan.add);
   }
   if (packed) d_attn = at::zeros({T * B, E}, d_attn.options()).index_copy_(0, batch.rows64, d_attn);
   AttnInputs a;
@@ -253,7 +291,6 @@ variable_list LayerNode::apply(variable_list&& grads) {
 
   // both projections read the same rows: their input gradients are one product over the concatenated reduction, so the e5m2 casts
   // take scales that give them one multiplier
-  Operand os = plan.qkv_self, oc = plan.qkv_cross;
   if (fp8) settle(os, [&] { return std::max(amax(g[0]), amax(g[1]) / ((os.w_scale * os.out_scale) / (oc.w_scale * oc.out_scale))); });
   if (fp8) oc.grad_scale = os.grad_scale * (os.w_scale * os.out_scale) / (oc.w_scale * oc.out_scale);
   auto [gs, dbs] = operand(os, g[0], Tensor(), bias_dt(at.bs, plan.n_self));
@@ -262,6 +299,28 @@ variable_list LayerNode::apply(variable_list&& grads) {
   give_rows(at.bc, plan.n_cross, dbc);
   if (any(at.ws, plan.n_self)) give_rows(at.ws, plan.n_self, wgrad(gs, s[kXq], a_w(os), w_dt(at.ws)));
   if (any(at.wc, plan.n_cross)) give_rows(at.wc, plan.n_cross, wgrad(gc, s[kXq], a_w(oc), w_dt(at.wc)));
+  if (lora_qkv) {
+    const Tensor& h = s[kXq];
+    const int64_t n = 7 * r;   // columns of the shared products (those of `out` come out as zero and are not used)
+    if (any(at.lb, 6)) {
+      Product xa;
+      xa.x = h;
+      xa.w = s[kARows];
+      const Tensor t = linear_fwd(xa).first;                           // x A^T of every projection
+      for (int p = 0; p < 2; ++p) {                                    // [3E][n], of which the diagonal blocks count
+        const Tensor db = wgrad(p ? gc : gs, t, plan.lora_scaling, at::kBFloat16);
+        const Tensor blocks = db.as_strided({3, E, r}, {E * n + r, n, 1}, 3 * p * r).contiguous();
+        for (int i = 0; i < 3; ++i)
+          if (wants(at.lb + 3 * p + i)) res[at.lb + 3 * p + i + 1] = blocks.select(0, i);
+      }
+    }
+    if (any(at.la, 6)) {
+      const Tensor gb = dgrad(gs, s[kBDiag].narrow(0, 0, 3 * E), 1.0, gc, s[kBDiag].narrow(0, 3 * E, 3 * E));   // g B of every projection
+      const Tensor da = wgrad(gb, h, plan.lora_scaling, at::kBFloat16);                                        // [n][E]
+      for (int i = 0; i < 6; ++i)
+        if (wants(at.la + i)) res[at.la + i + 1] = da.narrow(0, i * r, r);
+    }
+  }
   if (mu) {
     if (task_should_compute_output(0)) res[0] = dgrad(gs, os.w, a_in(os), gc, oc.w, d1, plan.keep).view(shape);
   } else if (task_should_compute_output(0) || p1) {

@@ -39,6 +39,9 @@ struct LayerPlan {
   std::vector<Tensor> params;
   int64_t n_self = 1, n_cross = 1;
   Operand qkv_self, qkv_cross, out, fc1, fc2;   // qkv operands [3E][E], rows [Q; K; V]
+  // frozen projections with adapters: params ends with A and B of self q, k, v, cross q, k, v and out; the operands are formed per call
+  int64_t lora_r = 0;
+  double lora_scaling = 1.0;
   Tensor qkv6, bias6;                           // both pathways in one operand, when one product serves them
   Tensor bias_self, bias_cross;                 // [3E] biases of separate products
 

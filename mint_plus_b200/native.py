@@ -1,9 +1,9 @@
 """Lays the two-pathway layers out for the C++ host side (csrc/host/layer.cpp): which parameters and operands a layer's forward
 and backward pass take, formed once and kept on the layer until one of them changes.
 
-A layer is served here when it is what the builders make: bf16 activations on the GPU, nn.Linear projections with bf16 weights or
-Fp8Linear ones throughout, LayerNorms with parameters, the fused attention.  Everything else (adapters, wrapped projections, mixed
-kinds) stays on the modules' own path.
+A layer is served here when it is what the builders make: bf16 activations on the GPU, nn.Linear projections with bf16 weights
+(with or without LoRA adapters on a frozen base) or Fp8Linear ones throughout, LayerNorms with parameters, the fused attention.
+Everything else (wrapped projections, mixed kinds) stays on the modules' own path.
 """
 from __future__ import annotations
 
@@ -50,12 +50,23 @@ def _attn_mods(attn):
 
 def _build(layer, mu: bool, keep: float, add: float) -> Optional[_Plan]:
     from . import modules_plus as mp
+    from .lora import LoRALinear
     from .mu_scaling import Fp8Linear, fused_fp8_weight
     sa, ma, ff = layer.self_attn, layer.multimer_attn, layer.feed_forward
     ms, mc = _attn_mods(sa), _attn_mods(ma)
     if ms is None or mc is None or sa._modules.get("out_proj") is None:
         return None
     one = [sa.out_proj, ff.fc1, ff.fc2]
+    adapters = None
+    if all(type(m) is LoRALinear for m in ms + mc + one[:1]):
+        adapters = ms + mc + one[:1]
+        if len(ms) != 3 or len(mc) != 3 or len({(m.r, m.scaling) for m in adapters}) != 1 or adapters[0].r % 8 or sa.embed_dim % 8 or \
+                12 * sa.embed_dim ** 2 > mp._QKV6_MAX_BYTES or any(isinstance(m.dropout, nn.Dropout) or type(m.base) is not nn.Linear for m in adapters):
+            return None
+        ms, mc, one = [m.base for m in ms], [m.base for m in mc], [one[0].base] + one[1:]
+        if any(p.dtype != torch.bfloat16 or not p.is_contiguous() for m in adapters for p in (m.lora_A, m.lora_B)) or \
+                any(p.requires_grad for m in ms + mc + one[:1] for p in m.parameters()):
+            return None
     linears = ms + mc + one
     fp8 = type(linears[0]) is Fp8Linear
     if any(type(m) is not (Fp8Linear if fp8 else nn.Linear) for m in linears):
@@ -80,6 +91,10 @@ def _build(layer, mu: bool, keep: float, add: float) -> Optional[_Plan]:
         p.slots += [(m._modules, n, m._modules.get(n)) for n in names]
     for m in linears + norms:
         p.slots += [(m._parameters, "weight", m._parameters.get("weight")), (m._parameters, "bias", m._parameters.get("bias"))]
+
+    for m in adapters or ():
+        p.slots += [(m._modules, n, m._modules.get(n)) for n in ("base", "dropout")] + [(m._parameters, n, m._parameters.get(n)) for n in ("lora_A", "lora_B")]
+        p.slots += [(m.__dict__, "scaling", m.__dict__.get("scaling"))]
 
     def watch(t):
         if t is not None:
@@ -107,10 +122,14 @@ def _build(layer, mu: bool, keep: float, add: float) -> Optional[_Plan]:
         else:
             p.can_grad, p.x_scale = True, 0.0
             w_s, w_c = ((m[0].weight.detach() if len(m) == 1 else None) for m in (ms, mc))
-            if w_s is None or w_c is None or 12 * E * E <= mp._QKV6_MAX_BYTES:
+            if adapters is None and (w_s is None or w_c is None or 12 * E * E <= mp._QKV6_MAX_BYTES):
                 for m in ms + mc:
                     watch(m.weight)
-        if mp.FUSE_QKV6 and 6 * E * E * (1 if fp8 else 2) <= mp._QKV6_MAX_BYTES and bias_s == bias_c:
+        if adapters is not None:
+            if bias_s != bias_c:
+                return None
+            bias6 = torch.cat([m.bias.detach().float() for m in ms + mc]) if bias_s else None
+        elif mp.FUSE_QKV6 and 6 * E * E * (1 if fp8 else 2) <= mp._QKV6_MAX_BYTES and bias_s == bias_c:
             # both pathways' projections as one product that reads x once; a larger [6E][E] operand pushes the activation rows out
             # of L2 between column tiles (measured slower)
             if fp8:
@@ -123,20 +142,23 @@ def _build(layer, mu: bool, keep: float, add: float) -> Optional[_Plan]:
         elif not fp8:
             w_s = torch.cat([m.weight.detach() for m in ms]) if w_s is None else w_s
             w_c = torch.cat([m.weight.detach() for m in mc]) if w_c is None else w_c
-        if qkv6 is None:
+        if qkv6 is None and adapters is None:
             b_self = (ms[0].bias.detach() if len(ms) == 1 else torch.cat([m.bias.detach() for m in ms])) if bias_s else None
             b_cross = (mc[0].bias.detach() if len(mc) == 1 else torch.cat([m.bias.detach() for m in mc])) if bias_c else None
         for m in ms + mc:
             watch(m.bias)
         if not fp8:
-            op_s, op_c = L.host().Operand(w_s), L.host().Operand(w_c)
+            op_s, op_c = (L.host().Operand(w) for w in (w_s, w_c)) if adapters is None else (L.host().Operand(None), L.host().Operand(None))
             o, f1, f2 = (L.host().Operand(m.weight) for m in one)
     params = [m.weight for m in ms] + [m.bias for m in ms] + [m.weight for m in mc] + [m.bias for m in mc]
     for m in one + norms:
         params += [m.weight, m.bias]
+    if adapters is not None:
+        params += [m.lora_A for m in adapters] + [m.lora_B for m in adapters]
     p.native = L.host().LayerPlan(mu=mu, fp8=fp8, sqrt_softmax=bool(layer._use_sqrt_softmax), H=H, D=sa.head_dim, scale=sa.scaling, keep=keep, add=add,
                                   eps1=norms[0].eps, eps2=norms[-1].eps, params=params, n_self=len(ms), n_cross=len(mc), qkv_self=op_s, qkv_cross=op_c,
-                                  out=o, fc1=f1, fc2=f2, qkv6=qkv6, bias6=bias6, bias_self=b_self, bias_cross=b_cross)
+                                  out=o, fc1=f1, fc2=f2, qkv6=qkv6, bias6=bias6, bias_self=b_self, bias_cross=b_cross,
+                                  lora_r=adapters[0].r if adapters else 0, lora_scaling=adapters[0].scaling if adapters else 1.0)
     p.slots += [(layer.__dict__, k, layer.__dict__.get(k)) for k in ("_use_sqrt_softmax", "_tau_f")]
     p.rot = sa.rot_emb
     return p

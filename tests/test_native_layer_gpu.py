@@ -7,6 +7,7 @@ import torch
 
 import mint_plus_b200 as M
 from mint_plus_b200 import modules_plus, native, ops
+from mint_plus_b200.lora import apply_lora
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -25,6 +26,13 @@ def make_layer(kind):
         if n.endswith("bias") or "norm" in n:
             torch.nn.init.normal_(p, 1.0 if n.endswith("norm.weight") else 0.0, 0.1)
     layer = layer.to(DEV).to(torch.bfloat16)
+    if kind == "lora":
+        wrap = torch.nn.Module()
+        wrap.layers = torch.nn.ModuleList([layer])
+        apply_lora(wrap, r=8, alpha=16.0)
+        for n, p in layer.named_parameters():
+            if n.endswith("lora_B"):
+                torch.nn.init.normal_(p, 0.0, 0.1)
     if kind.endswith("fp8"):
         wrap = torch.nn.Module()
         wrap.layers = torch.nn.ModuleList([layer])
@@ -64,7 +72,7 @@ def close(a, b, tol):
 
 
 @pytest.mark.parametrize("kind,T,B,two_products", [("base", 70, 3, False), ("base", 129, 1, True), ("plus", 64, 2, False), ("plus", 200, 2, True), ("mu", 65, 2, False),
-                                                   ("mu_fp8", 130, 3, False), ("mu_fp8", 33, 1, True), ("base_fp8", 96, 2, False)])
+                                                   ("mu_fp8", 130, 3, False), ("mu_fp8", 33, 1, True), ("base_fp8", 96, 2, False), ("lora", 150, 2, False), ("lora", 61, 1, False)])
 def test_layer_equals_the_composed_operators(kind, T, B, two_products, monkeypatch):
     if two_products:
         monkeypatch.setattr(modules_plus, "_QKV6_MAX_BYTES", 0)
