@@ -7,6 +7,7 @@ of this package — the layers get `chain_ids` and derive the compact mask metad
 """
 from __future__ import annotations
 
+import time
 from typing import Callable, Dict, List, Optional
 
 import torch
@@ -64,6 +65,19 @@ class Alphabet:
 
     def encode(self, sequence: str) -> List[int]:
         return [self.tok_to_idx.get(ch, self.unk_idx) for ch in sequence]
+
+
+_free_seen = {}     # device index -> (free bytes, when)
+
+
+def _driver_free(device: torch.device, need: float) -> int:
+    """Free bytes on the device.  The driver takes milliseconds to answer, so an answer of the last second stands where `need` is far
+    from it."""
+    seen = _free_seen.get(device.index)
+    now = time.monotonic()
+    if seen is None or now - seen[1] > 1.0 or need > 0.2 * seen[0]:
+        seen = _free_seen[device.index] = (torch.cuda.mem_get_info(device)[0], now)
+    return seen[0]
 
 
 class MINT(nn.Module):
@@ -205,10 +219,7 @@ class MINT(nn.Module):
         need = per_layer * len(self.layers)
         from . import _lib
         cached = _lib.host().cached_free_bytes(x.device.index)        # held by the allocator and free: reusable
-        if need <= 0.7 * cached:
-            return False                                              # (asking the driver takes it milliseconds)
-        free, _ = torch.cuda.mem_get_info(x.device)
-        return need > 0.7 * (free + cached)
+        return need > 0.7 * cached and need > 0.7 * (_driver_free(x.device, need) + cached)
 
     @classmethod
     def from_config(cls, model_size: str, fp8: bool = False, use_erf_gelu: bool = False) -> "MINT":
