@@ -98,20 +98,27 @@ inline size_t grad_h_stride(const AttnArgs& a) { return a.grad_rowmajor ? size_t
 
 void set_error(const char* fmt, ...);
 // Launch `kern` so that it may start while the kernel before it in the stream is still running (programmatic dependent
-// launch); the kernel calls ptx::griddep_wait() before it touches anything that kernel writes.
+// launch); the kernel calls ptx::griddep_wait() before it touches anything that kernel writes.  `cluster` neighbouring CTAs form a cluster.
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_dependent(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+inline cudaError_t launch_dependent_clusters(int cluster, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = unsigned(cluster);
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
+}
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_dependent(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+  return launch_dependent_clusters(1, kern, grid, block, smem, stream, static_cast<Args&&>(args)...);
 }
 // Lets `Kern` use `bytes` of dynamic shared memory on the current device; asks the driver once per device.
 int current_device();   // of the calling thread, or -1

@@ -25,10 +25,11 @@ constexpr int kABytes = kGM * kSlabBytes;
 constexpr int kGStageOutBytes = 32 * 64 + 32 * 32;   // one epilogue warp's staging: 32 rows x 32 bf16 columns, then 32 rows x 32 e4m3 columns, for bulk stores
 constexpr int kGTileRing = 4;   // tile numbers travel from the loading warp to the other roles through a ring this deep
 // A narrower tile needs less of the ring per slab and has less work to hide a slab's latency behind: more stages.
-template <int BN>
+template <int BN, bool PAIR>
 struct GemmCfg {
-  static constexpr int kStages = BN == 256 ? 4 : BN == 128 ? 6 : 8;
-  static constexpr int kBBytes = BN * kSlabBytes, kStageBytes = kABytes + kBBytes;
+  static constexpr int kStages = PAIR ? 6 : BN == 256 ? 4 : BN == 128 ? 6 : 8;
+  static constexpr int kBRows = PAIR ? BN / 2 : BN;   // rows of W this CTA loads
+  static constexpr int kBBytes = kBRows * kSlabBytes, kStageBytes = kABytes + kBBytes;
   static constexpr size_t kSmem = 1024 + size_t(kStages) * kStageBytes + kGEpiWarps * kGStageOutBytes + 256 + 2 * BN * sizeof(float);
 };
 
@@ -117,11 +118,13 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
 }
 
 // EPI: epilogue kind; HD: head_dim of the head-major epilogue (0 otherwise); BN: tile columns
-template <int EPI, int HD, int BN>
+template <int EPI, int HD, int BN, bool PAIR>
 __global__ void __launch_bounds__(kGThreads, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                const __grid_constant__ CUtensorMap map_out, const __grid_constant__ CUtensorMap map_pre, GemmParams p) {
-  constexpr int kGN = BN, kGStages = GemmCfg<BN>::kStages, kGStageBytes = GemmCfg<BN>::kStageBytes;
+  using Cfg = GemmCfg<BN, PAIR>;
+  constexpr int kGN = BN, kGStages = Cfg::kStages, kGStageBytes = Cfg::kStageBytes;
+  constexpr int kTileM = PAIR ? 2 * kGM : kGM;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   unsigned char* s_out = smem + size_t(kGStages) * kGStageBytes;   // [epilogue warp][32 rows][64 B], 64B swizzle
@@ -138,20 +141,24 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   static_assert((2 * kGStages + 4 + 2 * kGTileRing) * 8 + 8 + kGTileRing * 4 <= 256, "barrier area of the shared-memory tail");
 
   const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
-  const int tiles_m = (p.M + kGM - 1) / kGM, tiles_n = (p.N + kGN - 1) / kGN;
+  const int rank = PAIR ? int(cluster_rank()) : 0;   // CTA 0 of a pair draws the tiles and issues the products
+  const int tiles_m = (p.M + kTileM - 1) / kTileM, tiles_n = (p.N + kGN - 1) / kGN;
   const int n_tiles = tiles_m * tiles_n;
   const int elems_per_slab = p.in_dtype == MINTB_E4M3 ? 128 : 64;
   const int n_slabs = (p.K + elems_per_slab - 1) / elems_per_slab;
 
   if (tid == 0) {
     for (int s = 0; s < kGStages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-    for (int s = 0; s < 2; ++s) { mbar_init(&acc_full[s], 1); mbar_init(&acc_empty[s], kGEpiThreads); }
-    for (int s = 0; s < kGTileRing; ++s) { mbar_init(&tr_full[s], 1); mbar_init(&tr_empty[s], 1 + kGEpiWarps); }
+    for (int s = 0; s < 2; ++s) { mbar_init(&acc_full[s], 1); mbar_init(&acc_empty[s], PAIR ? 2 * kGEpiWarps : kGEpiThreads); }
+    for (int s = 0; s < kGTileRing; ++s) { mbar_init(&tr_full[s], 1); mbar_init(&tr_empty[s], PAIR ? 2 + 2 * kGEpiWarps : 1 + kGEpiWarps); }
     fence_mbar_init();
   }
-  if (warp == 1) { tmem_alloc(tmem_slot, 2 * BN); tmem_relinquish(); }
+  if (warp == 1) {
+    if constexpr (PAIR) { tmem_alloc_pair(tmem_slot, 2 * BN); tmem_relinquish_pair(); }
+    else { tmem_alloc(tmem_slot, 2 * BN); tmem_relinquish(); }
+  }
   tc_fence_before();
-  __syncthreads();
+  if constexpr (PAIR) cluster_sync(); else __syncthreads();
   tc_fence_after();
   // The next kernel may set itself up while this one runs: from here on only, because its CTAs may take tensor memory that a CTA of
   // this grid has yet to allocate, and then wait for this grid; and after the wait, so that a kernel may count on everything before
@@ -167,33 +174,63 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       // Tiles are drawn from the launch's work counter (the first one is the CTA's own number), so a CTA that shares its SM
       // with another kernel for a while - a collective of the gradient exchange, say - simply takes fewer tiles instead of
       // holding the whole grid up.  The tile numbers reach the other roles through a small ring.
+      // Of a pair, CTA 0 draws for both and writes the number into both rings; each CTA loads its own rows of x and its half of
+      // the tile's rows of W, and all the bytes are counted on CTA 0's barrier.
       uint32_t stage = 0, phase = 0, n_drawn = 0;
       bool ok = true;
       for (;;) {
         const uint32_t slot = n_drawn % kGTileRing;
-        ok = mbar_wait(&tr_empty[slot], ((n_drawn / kGTileRing) & 1) ^ 1, p.status, 0x705);
-        if (!ok) break;
-        int t = n_drawn == 0 ? int(blockIdx.x) : int(gridDim.x) + atomicAdd(p.sched, 1);
-        if (t >= n_tiles) t = -1;
-        tile_ring[slot] = t;
-        mbar_arrive(&tr_full[slot]);
+        int t;
+        if (!PAIR || rank == 0) {
+          const uint32_t parity = ((n_drawn / kGTileRing) & 1) ^ 1;
+          ok = PAIR ? mbar_wait_cluster(&tr_empty[slot], parity, p.status, 0x705) : mbar_wait(&tr_empty[slot], parity, p.status, 0x705);
+          if (!ok) break;
+          const int n_workers = int(gridDim.x) / (PAIR ? 2 : 1);
+          t = n_drawn == 0 ? int(blockIdx.x) / (PAIR ? 2 : 1) : n_workers + atomicAdd(p.sched, 1);
+          if (t >= n_tiles) t = -1;
+          tile_ring[slot] = t;
+          mbar_arrive(&tr_full[slot]);
+          if constexpr (PAIR) {
+            cluster_store(cluster_addr(&tile_ring[slot], 1), t);
+            cluster_arrive(cluster_addr(&tr_full[slot], 1));
+          }
+        } else {
+          ok = mbar_wait_cluster(&tr_full[slot], (n_drawn / kGTileRing) & 1, p.status, 0x708);
+          if (!ok) break;
+          t = tile_ring[slot];
+          cluster_arrive(cluster_addr(&tr_empty[slot], 0));
+        }
         ++n_drawn;
         if (t < 0) break;
-        const int m0 = (t / tiles_n) * kGM, n0 = (t % tiles_n) * kGN;
+        const int m0 = (t / tiles_n) * kTileM + rank * kGM, n0 = (t % tiles_n) * kGN + rank * Cfg::kBRows;
         for (int kb = 0; kb < n_slabs; ++kb) {
           ok = mbar_wait(&empty[stage], phase ^ 1, p.status, 0x701);
           if (!ok) break;
           unsigned char* a = smem + size_t(stage) * kGStageBytes;
-          mbar_expect_tx(&full[stage], kGStageBytes);
-          tma_load_2d(a, &map_a, &full[stage], kb * elems_per_slab, m0);
-          tma_load_2d(a + kABytes, &map_b, &full[stage], kb * elems_per_slab, n0);
+          if constexpr (PAIR) {
+            if (rank == 0) mbar_expect_tx(&full[stage], 2 * kGStageBytes);
+            const uint32_t bar = cluster_addr(&full[stage], 0);
+            tma_load_2d_pair(a, &map_a, bar, kb * elems_per_slab, m0);
+            tma_load_2d_pair(a + kABytes, &map_b, bar, kb * elems_per_slab, n0);
+          } else {
+            mbar_expect_tx(&full[stage], kGStageBytes);
+            tma_load_2d(a, &map_a, &full[stage], kb * elems_per_slab, m0);
+            tma_load_2d(a + kABytes, &map_b, &full[stage], kb * elems_per_slab, n0);
+          }
           if (++stage == kGStages) { stage = 0; phase ^= 1; }
         }
         if (!ok) break;
       }
-      leave_tile_counter(p.sched, int(gridDim.x));
+      // The products of a pair report to both CTAs: neither leaves before the last report on each of its stages has arrived.
+      if constexpr (PAIR)
+        for (int i = 0; i < kGStages && ok; ++i) {
+          ok = mbar_wait(&empty[stage], phase ^ 1, p.status, 0x709);
+          if (++stage == kGStages) { stage = 0; phase ^= 1; }
+        }
+      if (rank == 0) leave_tile_counter(p.sched, int(gridDim.x) / (PAIR ? 2 : 1));
     }
   } else if (warp == 1) {
+    if (rank == 0) {
     // All lanes run the loop and one elected lane issues: with warp-uniform control flow and operands the descriptors stay
     // in uniform registers, which is what tcgen05.mma reads; issued from a single-lane region every instruction first has
     // to move its operands there, and at 8-bit rates (one 128 x 256 x 32-byte instruction per 128 cycles) the issuing
@@ -203,7 +240,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       return __all_sync(0xffffffffu, mbar_wait(bar, parity, p.status, code));
     };
     const bool f8 = p.in_dtype == MINTB_E4M3;
-    const uint32_t idesc = f8 ? idesc_e4m3(kGM, kGN) : idesc_bf16(kGM, kGN, false, false);
+    const uint32_t idesc = f8 ? idesc_e4m3(kTileM, kGN) : idesc_bf16(kTileM, kGN, false, false);
     constexpr uint32_t kHi = desc_hi32(8 * kSlabBytes, kSw128);
     const uint32_t a_lo0 = desc_addr32(__shfl_sync(0xffffffffu, smem_u32(smem), 0)) + desc_lbo32(16);
     const uint32_t tbase_u = __shfl_sync(0xffffffffu, tbase, 0);
@@ -217,7 +254,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       if (leader) mbar_arrive(&tr_empty[slot]);
       ++n_seen;
       if (t < 0) break;
-      ok = wait_all(&acc_empty[ab], ab_phase ^ 1, 0x702);
+      ok = PAIR ? __all_sync(0xffffffffu, mbar_wait_cluster(&acc_empty[ab], ab_phase ^ 1, p.status, 0x702)) : wait_all(&acc_empty[ab], ab_phase ^ 1, 0x702);
       if (!ok) break;
       tc_fence_after();
       const uint32_t d = tbase_u + ab * kGN;
@@ -227,22 +264,33 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         tc_fence_after();
         const uint32_t a_lo = a_lo0 + stage * (kGStageBytes >> 4), b_lo = a_lo + (kABytes >> 4);
         if (leader) {
-          if (f8) {
+          if constexpr (PAIR) {
+            if (f8) {
+#pragma unroll
+              for (int k = 0; k < 4; ++k) umma_ss_pair<true>(d, make_desc(kHi, a_lo + 2 * k), make_desc(kHi, b_lo + 2 * k), idesc, kb > 0 || k > 0);
+            } else {
+#pragma unroll
+              for (int k = 0; k < 4; ++k) umma_ss_pair<false>(d, make_desc(kHi, a_lo + 2 * k), make_desc(kHi, b_lo + 2 * k), idesc, kb > 0 || k > 0);
+            }
+          } else if (f8) {
 #pragma unroll
             for (int k = 0; k < 4; ++k) umma_ss_f8(d, make_desc(kHi, a_lo + 2 * k), make_desc(kHi, b_lo + 2 * k), idesc, kb > 0 || k > 0);
           } else {
 #pragma unroll
             for (int k = 0; k < 4; ++k) umma_ss(d, make_desc(kHi, a_lo + 2 * k), make_desc(kHi, b_lo + 2 * k), idesc, kb > 0 || k > 0);
           }
-          umma_commit(&empty[stage]);
+          if constexpr (PAIR) umma_commit_pair(&empty[stage]); else umma_commit(&empty[stage]);
         }
         __syncwarp();
         if (++stage == kGStages) { stage = 0; phase ^= 1; }
       }
       if (!ok) break;
-      if (leader) umma_commit(&acc_full[ab]);
+      if (leader) {
+        if constexpr (PAIR) umma_commit_pair(&acc_full[ab]); else umma_commit(&acc_full[ab]);
+      }
       __syncwarp();
       if (++ab == 2) { ab = 0; ab_phase ^= 1; }
+    }
     }
   } else {
     // eight warps: warp w works on TMEM lanes 32 (w % 4) ... (the quarter it may access) and on column half (w - 2) / 4
@@ -328,14 +376,17 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     bool ok = true;
     for (;;) {
       const uint32_t slot = n_seen % kGTileRing;
-      ok = mbar_wait(&tr_full[slot], (n_seen / kGTileRing) & 1, p.status, 0x707);
+      ok = PAIR ? mbar_wait_cluster(&tr_full[slot], (n_seen / kGTileRing) & 1, p.status, 0x707)
+                : mbar_wait(&tr_full[slot], (n_seen / kGTileRing) & 1, p.status, 0x707);
       if (!ok) break;
       const int t = tile_ring[slot];
       __syncwarp();
-      if (lane == 0) mbar_arrive(&tr_empty[slot]);
+      if (lane == 0) {
+        if constexpr (PAIR) cluster_arrive(cluster_addr(&tr_empty[slot], 0)); else mbar_arrive(&tr_empty[slot]);
+      }
       ++n_seen;
       if (t < 0) break;
-      const int m0 = (t / tiles_n) * kGM, n0 = (t % tiles_n) * kGN;
+      const int m0 = (t / tiles_n) * kTileM + rank * kGM, n0 = (t % tiles_n) * kGN;
       const int m = m0 + row;
       float* bias_t = s_bias + ab * kGN;
       for (int j = et; j < kGN; j += kGEpiThreads) bias_t[j] = (p.bias != nullptr && n0 + j < p.N) ? load_bias(p.bias, p.bias_dtype, n0 + j) : 0.f;
@@ -585,16 +636,21 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         tmem_ld_wait();   // (a load issued ahead of a chunk that was not processed)
       }
       tc_fence_before();
-      mbar_arrive(&acc_empty[ab]);
+      if constexpr (PAIR) {
+        __syncwarp();
+        if (lane == 0) cluster_arrive(cluster_addr(&acc_empty[ab], 0));
+      } else {
+        mbar_arrive(&acc_empty[ab]);
+      }
       if (++ab == 2) { ab = 0; ab_phase ^= 1; }
     }
     if (lane == 0) bulk_wait_all();   // (a dependent kernel may already be waiting for this grid)
   }
   tc_fence_before();
-  __syncthreads();
+  if constexpr (PAIR) cluster_sync(); else __syncthreads();
   if (warp == 1) {
     __syncwarp();
-    tmem_dealloc(tbase, 2 * BN);
+    if constexpr (PAIR) tmem_dealloc_pair(tbase, 2 * BN); else tmem_dealloc(tbase, 2 * BN);
   }
 }
 
@@ -681,6 +737,12 @@ static bool gemm_out_map_f8(CUtensorMap* m, const void* ptr, int rows, int N) {
 // and 200 cycles at 256, 128 and 64 columns: the narrow ones are bound by the operand traffic into shared memory) plus filling
 // the ring and draining the last tile.  Whole-batch products come out at 256; M = 497 against N = K = 1280 (e4m3) at 64: 20 tiles on 148 SMs
 // and 15.9 us before, 80 tiles and 8.6 us now.
+//
+// A pair's 256 x 256 tile needs two thirds of a single CTA's operand traffic per product (32 KB instead of 48 KB per slab and SM, which
+// is what limits the 128 x 256 tile, and the power that goes with it), but its tiles are handed over between two SMs: at 10
+// slabs per tile it loses 8 % (M32768 N2560 K640 bf16: 92 -> 100 us), at 20 it is even, at 40 and more it gains: M16384 N15360 K2560 bf16
+// 1074 -> 921 us, M16384 N2560 K10240 615 -> 550 us, e4m3 M32768 N1280 K5120 154 -> 145 us.
+constexpr int kPairTile = 512, kPairMinSlabs = 32;
 static int pick_tile(int M, int N, int n_slabs, int sms) {
   const long long tm = (M + kGM - 1) / kGM;
   int best = 256;
@@ -690,17 +752,23 @@ static int pick_tile(int M, int N, int n_slabs, int sms) {
     const long long cost = rounds * n_slabs * (bn == 256 ? 512 : bn == 128 ? 280 : 200) + 1500 + 8 * bn;
     if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = bn; }
   }
+  if (n_slabs >= kPairMinSlabs) {
+    const long long rounds = ((tm + 1) / 2 * ((N + 255) / 256) + sms / 2 - 1) / (sms / 2);
+    if (rounds * n_slabs * 470 + 1500 + 8 * 256 < best_cost) best = kPairTile;
+  }
   return best;
 }
 
-template <int EPI, int HD, int BN>
+template <int EPI, int HD, int BN, bool PAIR>
 static int launch_gemm_t(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mo, const CUtensorMap& mp, GemmParams& p, int sms, cudaStream_t stream) {
-  constexpr auto kern = gemm_tc_kernel<EPI, HD, BN>;
-  cudaError_t e = opt_in_smem<kern>(int(GemmCfg<BN>::kSmem));
+  constexpr auto kern = gemm_tc_kernel<EPI, HD, BN, PAIR>;
+  cudaError_t e = opt_in_smem<kern>(int(GemmCfg<BN, PAIR>::kSmem));
   if (e != cudaSuccess) { set_error("cudaFuncSetAttribute: %s", cudaGetErrorString(e)); return MINTB_ECUDA; }
-  const int tiles = ((p.M + kGM - 1) / kGM) * ((p.N + BN - 1) / BN);
+  constexpr int kTileM = PAIR ? 2 * kGM : kGM;
+  const int tiles = ((p.M + kTileM - 1) / kTileM) * ((p.N + BN - 1) / BN);
+  const int workers = PAIR ? sms / 2 : sms, grid = (tiles < workers ? tiles : workers) * (PAIR ? 2 : 1);
   if (int rc = next_tile_counter(&p.sched); rc != MINTB_OK) return rc;
-  e = launch_dependent(kern, dim3(tiles < sms ? tiles : sms), dim3(kGThreads), GemmCfg<BN>::kSmem, stream, ma, mb, mo, mp, p);
+  e = launch_dependent_clusters(PAIR ? 2 : 1, kern, dim3(grid), dim3(kGThreads), GemmCfg<BN, PAIR>::kSmem, stream, ma, mb, mo, mp, p);
   count_launches(1);
   if (e != cudaSuccess) { set_error("gemm launch: %s", cudaGetErrorString(e)); return MINTB_ECUDA; }
   return MINTB_OK;
@@ -711,8 +779,8 @@ int launch_gemm(const GemmParams& p_in, const void* x, const void* w, cudaStream
   CUtensorMap ma, mb;
   const int sms = sm_count();
   const int per_slab = p.in_dtype == MINTB_E4M3 ? 128 : 64;
-  const int bn = pick_tile(p.M, p.N, (p.K + per_slab - 1) / per_slab, sms);
-  if (!gemm_map(&ma, x, p.M, p.K, p.in_dtype, kGM) || !gemm_map(&mb, w, p.N, p.K, p.in_dtype, bn)) {
+  const int tile = pick_tile(p.M, p.N, (p.K + per_slab - 1) / per_slab, sms);
+  if (!gemm_map(&ma, x, p.M, p.K, p.in_dtype, kGM) || !gemm_map(&mb, w, p.N, p.K, p.in_dtype, tile == kPairTile ? 128 : tile)) {
     set_error("mintb gemm: cuTensorMapEncodeTiled failed");
     return MINTB_ECUDA;
   }
@@ -738,9 +806,10 @@ int launch_gemm(const GemmParams& p_in, const void* x, const void* w, cudaStream
   }
   p.alt_stores = (p.use_bulk_f8 && p.use_bulk_store && p.preact != nullptr) ? 1 : 0;
 #define MINTB_GEMM_TILE(EPI, HD)                                                              \
-  return bn == 256 ? launch_gemm_t<EPI, HD, 256>(ma, mb, mo, mp, p, sms, stream)              \
-       : bn == 128 ? launch_gemm_t<EPI, HD, 128>(ma, mb, mo, mp, p, sms, stream)              \
-                   : launch_gemm_t<EPI, HD, 64>(ma, mb, mo, mp, p, sms, stream)
+  return tile == kPairTile ? launch_gemm_t<EPI, HD, 256, true>(ma, mb, mo, mp, p, sms, stream)  \
+       : tile == 256       ? launch_gemm_t<EPI, HD, 256, false>(ma, mb, mo, mp, p, sms, stream) \
+       : tile == 128       ? launch_gemm_t<EPI, HD, 128, false>(ma, mb, mo, mp, p, sms, stream) \
+                           : launch_gemm_t<EPI, HD, 64, false>(ma, mb, mo, mp, p, sms, stream)
   if (p.epilogue == kEpiBias) MINTB_GEMM_TILE(kEpiBias, 0);
   if (p.epilogue == kEpiBiasGelu) MINTB_GEMM_TILE(kEpiBiasGelu, 0);
   if (p.D == 16) MINTB_GEMM_TILE(kEpiHeadMajor, 16);
