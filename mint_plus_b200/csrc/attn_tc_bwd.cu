@@ -16,6 +16,8 @@
 #include "common.cuh"
 #include "ptx.cuh"
 
+#include <type_traits>
+
 namespace mintb {
 
 using namespace ptx;
@@ -268,7 +270,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
   constexpr int kBwdThreads = Cfg::kThreads, kComputeThreads = 32 * Cfg::kCW;
   constexpr int kColDK = Cfg::kColDK, kColDV = Cfg::kColDV, kColDQ = Cfg::kColDQ, kColBuf = Cfg::kColBuf, kAcc = Cfg::kAcc;
   extern __shared__ unsigned char smem_raw[];
-  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  unsigned char* smem = align_smem_1024(smem_raw);
   unsigned char* sK = smem;
   unsigned char* sV = sK + Cfg::kTileBytes;
   unsigned char* sQ = sV + Cfg::kTileBytes;                          // [stage][0: Q_i, 1: dO_i]
@@ -571,7 +573,8 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
     const uint32_t lane_base = uint32_t(quarter * 32) << 16;
     const uint32_t tBuf = tbase + lane_base + kColBuf;   // + 128 * buffer + 16 * vg: S^T columns of this thread; dP^T 64 further
     const bool key_valid = kj < p.T && !((p.kpad[size_t(b) * p.TW + krow / 32] >> (krow % 32)) & 1u);
-    const uint32_t* mrow = p.bitsT + (size_t(b) * p.T + krow) * p.TW;
+    const uint32_t* mrow = p.bitsT + (size_t(b) * p.T + krow) * p.TW + grp / 2;   // words grp / 2 and 2 + grp / 2 of a tile's four
+    const int mshift = 16 * (grp & 1);
     const uint32_t flip = path == 0 ? 0xffffu : 0u;   // keep-bit = mask bit XOR flip
     const uint64_t c22 = pack2(p.scale_log2, p.scale_log2);
     bool ok = true;
@@ -609,11 +612,23 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
       return true;
     };
 
+    // Mask bits of a tile for this key row (four words); asked for one tile ahead, so that a mixed tile does not wait for them.
+    auto next_active = [&](int i) {
+      while (i < nqt && tq[i] == 0) ++i;
+      return i;
+    };
+    auto tile_mask = [&](int i) {   // bits of this thread's 16 queries in the two halves
+      if (!(i < nqt && (tq[i] & 2))) return make_ushort2(0xffffu, 0xffffu);
+      const uint32_t a = __ldg(mrow + 4 * i), b = __ldg(mrow + 4 * i + 2);
+      return make_ushort2((unsigned short)((a >> mshift) ^ flip), (unsigned short)((b >> mshift) ^ flip));
+    };
     int prev_tile = -1;
-    for (int i = 0; i < nqt && ok; ++i) {
-      const uint8_t f = tq[i];
-      if (f == 0) continue;
-      // mask bits of the tile for this key row: half `sub`, 16-column group vg -> word 2 sub + vg / 2, bits 16 (vg & 1)...
+    int i = next_active(0), i_next;
+    ushort2 mask = tile_mask(i), mask_next;
+    const uint32_t ds_addr = smem_u32(sDS) + swizzled_offset(r, 2 * grp * kVPG, 128);   // (the other chunk of a group of 16 columns: bit 4 flipped)
+    for (; i < nqt && ok; i = i_next, mask = mask_next) {
+      i_next = next_active(i + 1);
+      mask_next = tile_mask(i_next);
 #pragma unroll 1
       for (int sub = 0; sub < 2 && ok; ++sub) {
         ok = mbar_wait(&sdp_full[br.pos], br.phase, p.status, 0x602);
@@ -624,50 +639,58 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
         }
         if (it == 0 && sub == 0 && grp >= 2) __nanosleep(kBwdStaggerNs);
         tc_fence_after();
-        unsigned char* ds_row = sDS + size_t(it % kNDq) * Cfg::kDsBytes + size_t(sub) * Cfg::kDsBlock;
+        const uint32_t ds_row = ds_addr + uint32_t(it % kNDq) * Cfg::kDsBytes + uint32_t(sub) * Cfg::kDsBlock;
 #pragma unroll
         for (int v = 0; v < kVPG; ++v) {
           const int vg = grp * kVPG + v;
-          // statistics of this thread's 16 queries, from the copy that arrived in shared memory with the query tile
+          // statistics of this thread's 16 queries, (nl0, nl1, nd0, nd1) per pair, from the copy that arrived in shared memory with the query tile
           const float4* st = reinterpret_cast<const float4*>(sStats + size_t(sr.pos) * Cfg::kStatBytes) + (sub * kHalf + 16 * vg) / 2;
-          float4 sq[8];
-#pragma unroll
-          for (int j = 0; j < 8; ++j) sq[j] = st[j];
-          uint32_t keep = 0xffffu;
-          if (f & 2) keep = ((__ldg(mrow + 4 * i + 2 * sub + vg / 2) >> (16 * (vg & 1))) & 0xffffu) ^ flip;
+          uint32_t keep = sub == 0 ? mask.x : mask.y;
           if (!key_valid) keep = 0u;
-          const bool all = keep == 0xffffu;
           const uint32_t tS = tBuf + br.pos * 128 + 16 * vg;
           uint32_t sv[16], dpv[16];
           tmem_ld16(tS, sv);
           tmem_ld16(tS + 64, dpv);
           tmem_ld_wait();
           uint32_t pp[8], dd[8];
+          // Straight-line code for each of the two cases: a test inside the loop would cut it into blocks that end in
+          // reconvergence points, and the exponentials of one pair of queries could not overlap those of the next.
+          auto elements = [&](auto masked) {
 #pragma unroll
-          for (int j = 0; j < 16; j += 2) {
-            const float4 q2 = sq[j / 2];   // (nl0, nl1, nd0, nd1)
-            float p0, p1;
-            unpack2(ffma2(pack2(__uint_as_float(sv[j]), __uint_as_float(sv[j + 1])), c22, pack2(q2.x, q2.y)), p0, p1);
-            p0 = bwd_ex2(p0);
-            p1 = bwd_ex2(p1);
-            if (!all) {
-              if (!((keep >> j) & 1u)) p0 = 0.f;
-              if (!((keep >> (j + 1)) & 1u)) p1 = 0.f;
+            for (int j = 0; j < 16; j += 2) {
+              const float4 q2 = st[j / 2];
+              float p0, p1;
+              unpack2(ffma2(pack2(__uint_as_float(sv[j]), __uint_as_float(sv[j + 1])), c22, pack2(q2.x, q2.y)), p0, p1);
+              p0 = bwd_ex2(p0);
+              p1 = bwd_ex2(p1);
+              if (decltype(masked)::value) {
+                p0 = (keep >> j) & 1u ? p0 : 0.f;
+                p1 = (keep >> (j + 1)) & 1u ? p1 : 0.f;
+              }
+              float d0, d1;
+              const uint64_t p2 = pack2(p0, p1), dp2 = pack2(__uint_as_float(dpv[j]), __uint_as_float(dpv[j + 1])), nd2 = pack2(q2.z, q2.w);
+              if (SQ)   // r = sqrt(p) is what p0, p1 hold: dS = r (dP / 2 - r delta / 2), and r itself multiplies dO in dV
+                unpack2(fmul2(p2, ffma2(p2, nd2, fmul2(dp2, pack2(0.5f, 0.5f)))), d0, d1);
+              else      // dS = p (dP - delta)
+                unpack2(fmul2(p2, fadd2(dp2, nd2)), d0, d1);
+              pp[j / 2] = bwd_pack(p0, p1);
+              dd[j / 2] = bwd_pack(d0, d1);
             }
-            float d0, d1;
-            const uint64_t p2 = pack2(p0, p1), dp2 = pack2(__uint_as_float(dpv[j]), __uint_as_float(dpv[j + 1])), nd2 = pack2(q2.z, q2.w);
-            if (SQ)   // r = sqrt(p) is what p0, p1 hold: dS = r (dP / 2 - r delta / 2), and r itself multiplies dO in dV
-              unpack2(fmul2(p2, ffma2(p2, nd2, fmul2(dp2, pack2(0.5f, 0.5f)))), d0, d1);
-            else      // dS = p (dP - delta)
-              unpack2(fmul2(p2, fadd2(dp2, nd2)), d0, d1);
-            pp[j / 2] = bwd_pack(p0, p1);
-            dd[j / 2] = bwd_pack(d0, d1);
+          };
+          if (__all_sync(0xffffffffu, keep == 0xffffu)) {
+            elements(std::false_type{});
+          } else if (__all_sync(0xffffffffu, keep == 0u)) {   // the other side of a chain boundary, or padding
+#pragma unroll
+            for (int j = 0; j < 8; ++j) pp[j] = dd[j] = 0u;
+          } else {
+            elements(std::true_type{});
           }
           tmem_st8(tS, pp);         // P^T over the S^T columns this thread has read
           tmem_st8(tS + 64, dd);    // dS^T likewise
           // and dS into shared memory for the dQ product: 2 chunks of 8 queries in block `sub` of the dS tile
-          *reinterpret_cast<uint4*>(ds_row + swizzled_offset(r, 2 * vg, 128)) = make_uint4(dd[0], dd[1], dd[2], dd[3]);
-          *reinterpret_cast<uint4*>(ds_row + swizzled_offset(r, 2 * vg + 1, 128)) = make_uint4(dd[4], dd[5], dd[6], dd[7]);
+          const uint32_t ds_at = kVPG == 1 ? ds_row : ds_row ^ (v * 32);
+          smem_store16(ds_at, dd[0], dd[1], dd[2], dd[3]);
+          smem_store16(ds_at ^ 16u, dd[4], dd[5], dd[6], dd[7]);
         }
         tmem_st_wait();
         fence_proxy_async_smem();

@@ -108,7 +108,7 @@ gemm_bwd_kernel(const __grid_constant__ CUtensorMap map_a1, const __grid_constan
                 const __grid_constant__ CUtensorMap map_out, BwdGemmParams p) {
   constexpr int kBN = BN, kBStages = BwdGemmCfg<BN>::kStages, kBStageBytes = BwdGemmCfg<BN>::kStageBytes;
   extern __shared__ unsigned char smem_raw[];
-  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  unsigned char* smem = align_smem_1024(smem_raw);
   unsigned char* s_out = smem + size_t(kBStages) * kBStageBytes;   // [epilogue warp][32 rows][128 B]
   unsigned char* tail = s_out + kBEpiWarps * kBOutStageBytes;
   uint64_t* full = reinterpret_cast<uint64_t*>(tail);   // [kBStages]

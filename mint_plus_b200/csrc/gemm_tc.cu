@@ -126,7 +126,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   constexpr int kGN = BN, kGStages = Cfg::kStages, kGStageBytes = Cfg::kStageBytes;
   constexpr int kTileM = PAIR ? 2 * kGM : kGM;
   extern __shared__ unsigned char smem_raw[];
-  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  unsigned char* smem = align_smem_1024(smem_raw);
   unsigned char* s_out = smem + size_t(kGStages) * kGStageBytes;   // [epilogue warp][32 rows][64 B], 64B swizzle
   unsigned char* tail = s_out + kGEpiWarps * kGStageOutBytes;
   uint64_t* full = reinterpret_cast<uint64_t*>(tail);   // [kGStages]

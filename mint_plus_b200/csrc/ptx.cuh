@@ -11,6 +11,14 @@ namespace ptx {
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 
+// The first 1024-byte boundary of the dynamic shared memory, as an offset from its start: rounding the pointer itself through an
+// integer would make it a generic address, and every later load and store through it a generic (slower) access.
+__device__ __forceinline__ unsigned char* align_smem_1024(unsigned char* raw) { return raw + ((0u - smem_u32(raw)) & 1023u); }
+
+__device__ __forceinline__ void smem_store16(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred;
   asm volatile(
