@@ -25,7 +25,6 @@ using namespace ptx;
 constexpr int kBwdTile = 128;       // keys per CTA and queries per step
 constexpr int kHalf = 64;           // queries per compute group
 constexpr int kBwdMaxTiles = 256;   // T <= 32768
-constexpr unsigned kBwdStaggerNs = 250;   // initial offset between the two pairs of compute groups
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -100,9 +99,6 @@ __device__ __forceinline__ uint64_t fmul2(uint64_t a, uint64_t b) {
   uint64_t r;
   asm("mul.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
-}
-__device__ __forceinline__ void named_barrier(int id, int nthreads) {
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
 
 // ------------------------------------------------------------------------------------------------ pre / post passes
@@ -215,22 +211,32 @@ struct BwdCfg {
   static constexpr int kDsBytes = 2 * kDsBlock;
   // One CTA per SM, 16 compute warps, all 512 TMEM columns: dK, dV, two dQ tiles, then two (head_dim 64) or three
   // (head_dim <= 32) buffers of {S^T half (64 columns), dP^T half (64 columns)}; the third buffer lets the products run
-  // two halves ahead of the compute warps.
+  // ahead of the compute warps.
   static constexpr int kCW = 16;                                // compute warps
-  static constexpr int kThreads = 128 + 32 * kCW;
+  static constexpr int kThreads = 128 + 32 * kCW;               // + three MMA issuers and the loading warp
   static constexpr int kNBuf = D <= 32 ? 3 : 2;
   static constexpr int kNDq = 2;                                // dQ tiles in TMEM == dS tiles in shared memory
-  static constexpr int kQStages = D <= 32 ? 3 : 2;              // stages of {Q_i, dO_i}
+  static constexpr int kQStages = D <= 32 ? 4 : 2;              // stages of {Q_i, dO_i} (a power of two)
+  static constexpr int kKv = D <= 32 ? 2 : 1;                   // key tiles {K, V} in shared memory
   static constexpr int kAcc = D <= 32 ? 32 : 64;                // columns reserved per accumulator
   static constexpr int kColDK = 0, kColDV = kAcc, kColDQ = 2 * kAcc, kColBuf = (2 + kNDq) * kAcc;
   static constexpr uint32_t kTmemCols = 512;
-  static constexpr int kVPG = 16 / kCW;                         // 16-column query groups per thread and half
   static constexpr int kDqWarpBytes = 32 * (D / 4) * 4;          // staging of one warp's dQ slice: 32 queries x D/4 fp32 columns
   static constexpr int kDqStageBytes = kCW * kDqWarpBytes;
   static constexpr int kStatBytes = 128 * 8;                     // softmax statistics of one query tile: 128 x (-lse log2 e, -delta)
-  static constexpr size_t kSmemBytes =
-      1024 + 2 * kTileBytes + size_t(kQStages) * 2 * kTileBytes + size_t(kNDq) * kDsBytes + kDqStageBytes + kQStages * kStatBytes + 4096;
+  static constexpr size_t kSmemBytes = 1024 + size_t(kKv) * 2 * kTileBytes + size_t(kQStages) * 2 * kTileBytes + size_t(kNDq) * kDsBytes +
+                                       kDqStageBytes + kQStages * kStatBytes + 2560;
 };
+
+// One work item - the dK, dV of a key tile in one pathway - as the loading warp hands it to the other roles.
+struct BwdPlan {
+  int n;                           // query tiles with pairs of the pathway; 0: no more items
+  int kt, bh, path;
+  uint32_t kpad[4];                // padding bits of the tile's 128 keys
+  uint16_t tiles[kBwdMaxTiles];    // their numbers, kMixed set where the tile needs the chain mask
+};
+constexpr uint16_t kMixed = 0x8000;
+constexpr int kPlans = 4;          // the one being computed, the one whose gradients have yet to leave, and two ahead
 
 struct BwdParams {
   const uint32_t *bitsT, *kpad;
@@ -247,6 +253,8 @@ struct BwdParams {
   size_t g_row, g_b, g_h;          // element strides of dk / dv: between keys, batch entries, heads
   const int32_t* token_row;        // row of the row-major gradient matrices per token t * B + b (negative: none), or null
   int B;
+  int n_items;                     // key tiles x (batch, head) x 2 pathways
+  int* sched;                      // work counter pair of this launch (common.cuh)
 };
 
 // ring counter with phase bit: position in [0, N), phase flips on wrap
@@ -258,6 +266,12 @@ struct Ring {
   }
 };
 
+// Persistent CTAs, one per SM.  What limits the kernel is the chain load - product - exponentials - product of a query tile and,
+// with the few tiles a key tile has (1 to 16), what a key tile costs beside them: as one CTA per key tile that was 13 700 cycles at
+// head_dim 32 and 20 900 at 64 (set-up and loads until the first exponential 4700, last dQ tile and gradients out 5000 to 10 000,
+// next CTA 2000 to 3000) against 2200 and 3100 cycles per query tile.  Here barriers and TMEM are set up once; the loading warp
+// plans and loads the next key tile while the current one is computed; and a key tile's last dQ tile and its dK, dV leave after the
+// compute warps have handed the next key tile's first half to the tensor cores.
 template <int D, bool SQ>
 __global__ void __launch_bounds__(BwdCfg<D>::kThreads, 1)
 attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_constant__ CUtensorMap map_ks,
@@ -266,145 +280,64 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
                    const __grid_constant__ CUtensorMap map_do, const __grid_constant__ CUtensorMap map_dq_s,
                    const __grid_constant__ CUtensorMap map_dq_c, BwdParams p) {
   using Cfg = BwdCfg<D>;
-  constexpr int RB = Cfg::kRowBytes, kNBuf = Cfg::kNBuf, kQStages = Cfg::kQStages, kNDq = Cfg::kNDq, kVPG = Cfg::kVPG;
-  constexpr int kBwdThreads = Cfg::kThreads, kComputeThreads = 32 * Cfg::kCW;
+  constexpr int RB = Cfg::kRowBytes, kNBuf = Cfg::kNBuf, kQStages = Cfg::kQStages, kNDq = Cfg::kNDq, kKv = Cfg::kKv;
   constexpr int kColDK = Cfg::kColDK, kColDV = Cfg::kColDV, kColDQ = Cfg::kColDQ, kColBuf = Cfg::kColBuf, kAcc = Cfg::kAcc;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = align_smem_1024(smem_raw);
-  unsigned char* sK = smem;
-  unsigned char* sV = sK + Cfg::kTileBytes;
-  unsigned char* sQ = sV + Cfg::kTileBytes;                          // [stage][0: Q_i, 1: dO_i]
+  unsigned char* sKV = smem;                                         // [key tile][0: K, 1: V]
+  unsigned char* sQ = sKV + size_t(kKv) * 2 * Cfg::kTileBytes;       // [stage][0: Q_i, 1: dO_i]
   unsigned char* sDS = sQ + size_t(kQStages) * 2 * Cfg::kTileBytes;  // [buf][half][128 rows x 128 B]
   unsigned char* sDqStage = sDS + size_t(kNDq) * Cfg::kDsBytes;      // [compute warp][32 queries][D/4 fp32], swizzled
   unsigned char* sStats = sDqStage + Cfg::kDqStageBytes;             // [stage][64] x (nl0, nl1, nd0, nd1), loaded with the query tile
   unsigned char* tail = sStats + size_t(kQStages) * Cfg::kStatBytes;
   uint64_t* bars = reinterpret_cast<uint64_t*>(tail);
-  uint64_t* kv_full = bars;            // 1
-  uint64_t* acc_full = bars + 1;       // 1
-  uint64_t* q_full = bars + 2;         // [3]
-  uint64_t* q_empty = bars + 5;        // [3]
-  uint64_t* sdp_full = bars + 8;       // [3 buffers]
-  uint64_t* pds_full = bars + 11;      // [3 buffers]
-  uint64_t* buf_free = bars + 14;      // [3 buffers]
-  uint64_t* dq_full = bars + 17;       // [2]
-  uint64_t* dq_empty = bars + 19;      // [2]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 21);
-  uint8_t* tq = reinterpret_cast<uint8_t*>(tmem_slot + 2);  // per query tile: 0 skip, else 1 | (needs chain mask) << 1 | (pad) << 2
+  uint64_t* plan_full = bars;           // [4]
+  uint64_t* plan_empty = bars + 4;      // [4]
+  uint64_t* kv_full = bars + 8;         // [2]
+  uint64_t* kv_empty = bars + 10;       // [2]
+  uint64_t* q_full = bars + 12;         // [4] Q_i and dO_i
+  uint64_t* st_full = bars + 16;        // [4] the statistics
+  uint64_t* q_empty = bars + 20;        // [4]
+  uint64_t* sdp_full = bars + 24;       // [3 buffers]
+  uint64_t* pds_full = bars + 27;       // [3 buffers]
+  uint64_t* buf_free = bars + 30;       // [3 buffers]
+  uint64_t* dq_full = bars + 33;        // [2]
+  uint64_t* dq_empty = bars + 35;       // [2]
+  uint64_t* acc_full = bars + 37;
+  uint64_t* acc_empty = bars + 38;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 39);
+  BwdPlan* plans = reinterpret_cast<BwdPlan*>(bars + 40);            // [kPlans]
+  static_assert(40 * 8 + kPlans * sizeof(BwdPlan) <= 2560, "tail of the shared memory");
 
   const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
-  const int kt = blockIdx.x, bh = blockIdx.y, path = blockIdx.z, b = bh / p.H;
-  const int k0 = kt * kBwdTile;
-  const int nqt = (p.T + kBwdTile - 1) / kBwdTile;
-  const uint8_t want = path == 0 ? kHasIntra : kHasInter;
-
-  const CUtensorMap* mq = path == 0 ? &map_qs : &map_qc;
-  const CUtensorMap* mk = path == 0 ? &map_ks : &map_kc;
-  const CUtensorMap* mv = path == 0 ? &map_vs : &map_vc;
-
-  // the gradients of a key tile without a single pair of this pathway are zero
-  auto write_zero_gradients = [&]() {
-    for (int idx = tid; idx < kBwdTile * (D / 8); idx += kBwdThreads) {
-      const int row = idx / (D / 8), vec = idx % (D / 8);
-      if (k0 + row < p.T) {
-        size_t base = size_t(k0 + row) * p.g_row + size_t(b) * p.g_b;
-        if (p.token_row != nullptr) {
-          const int tr = __ldg(p.token_row + size_t(k0 + row) * p.B + b);
-          if (tr < 0) continue;
-          base = size_t(tr) * p.g_b;
-        }
-        const size_t off = base + size_t(bh % p.H) * p.g_h + vec * 8;
-        *reinterpret_cast<uint4*>(p.dk[path] + off) = make_uint4(0u, 0u, 0u, 0u);
-        *reinterpret_cast<uint4*>(p.dv[path] + off) = make_uint4(0u, 0u, 0u, 0u);
-      }
-    }
-  };
-  // Every key of the tile padded (padded batches have many such tiles): leave before any barrier, TMEM or copy is set up.
-  {
-    const uint32_t* w = p.kpad + size_t(b) * p.TW + 4 * kt;
-    if ((w[0] & w[1] & w[2] & w[3]) == 0xffffffffu) {   // uniform over the CTA
-      write_zero_gradients();
-      return;
-    }
-  }
   if (tid == 0) {
-    mbar_init(kv_full, 1);
-    mbar_init(acc_full, 2);
-    for (int s = 0; s < 3; ++s) {
-      mbar_init(&q_full[s], 1); mbar_init(&q_empty[s], 2);      // released by the dV and the dK stream
-      mbar_init(&sdp_full[s], 1); mbar_init(&pds_full[s], kComputeThreads);
-      mbar_init(&buf_free[s], 2);                                // dV and dK of a half have read P^T, dS^T
+    for (int s = 0; s < 4; ++s) {
+      mbar_init(&plan_full[s], 1); mbar_init(&plan_empty[s], 3 + Cfg::kCW);   // three MMA issuers and every compute warp read a plan
+      mbar_init(&q_full[s], 1); mbar_init(&st_full[s], 1); mbar_init(&q_empty[s], 1);
     }
-    for (int s = 0; s < 2; ++s) { mbar_init(&dq_full[s], 1); mbar_init(&dq_empty[s], kComputeThreads); }
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&kv_full[s], 1); mbar_init(&kv_empty[s], 2);                   // released by the S / dP and the dQ stream
+      mbar_init(&dq_full[s], 1); mbar_init(&dq_empty[s], 32 * Cfg::kCW);
+    }
+    for (int s = 0; s < 3; ++s) {
+      mbar_init(&sdp_full[s], 1); mbar_init(&pds_full[s], 32 * Cfg::kCW / 2);
+      mbar_init(&buf_free[s], 2);                                // dV and dK of a half have read P^T, dS^T; the dQ stream has seen it
+    }
+    mbar_init(acc_full, 1); mbar_init(acc_empty, Cfg::kCW);
     fence_mbar_init();
-    // K and V of the tile do not depend on the query-tile scan below: their copies run while it does
-    prefetch_tensormap(mk); prefetch_tensormap(mv);
-    mbar_expect_tx(kv_full, 2 * Cfg::kTileBytes);
-    tma_load_3d(sK, mk, kv_full, 0, k0, bh);
-    tma_load_3d(sV, mv, kv_full, 0, k0, bh);
   }
   if (warp == 1) { tmem_alloc(tmem_slot, Cfg::kTmemCols); tmem_relinquish(); }
-
-  int any_active = 0;
-  uint8_t my_flag = 0;   // flag of query tile `tid` (the loop below runs at most once per thread: nqt <= kBwdMaxTiles < kBwdThreads)
-  for (int i = tid; i < nqt; i += kBwdThreads) {
-    uint8_t c = 0;
-#pragma unroll
-    for (int a = 0; a < 2; ++a)
-#pragma unroll
-      for (int e = 0; e < 2; ++e)
-        if (2 * i + a < p.NT && 2 * kt + e < p.NT) c |= p.cls[(size_t(b) * p.NT + 2 * i + a) * p.NT + 2 * kt + e];
-    uint8_t f = 0;
-    if (c & want) f = 1 | (((c & 3) == 3) ? 2 : 0) | ((c & kHasPad) ? 4 : 0);
-    if (p.skip_pad_queries) {   // the padding bits describe positions: words 4 i .. 4 i + 3 cover the queries of tile i
-      const uint32_t* w = p.kpad + size_t(b) * p.TW + 4 * i;
-      if ((w[0] & w[1] & w[2] & w[3]) == 0xffffffffu) f = 0;
-    }
-    tq[i] = f;
-    any_active |= f;
-    my_flag = f;
-  }
-  // The first query tile's Q and dO do not wait for the CTA-wide barrier below: warp 0 holds the flags of tiles 0..31 and
-  // requests the first tile with work among them at once (the copy of its statistics follows after the wait for the pass
-  // before this kernel).  A TMA round trip is about as long as the whole set-up, so the first products start that much
-  // earlier.  Warp 0 remembers the tile; its loading loop then skips these two copies.
-  int early_q = -1;
-  if (warp == 0) {
-    const unsigned act = __ballot_sync(0xffffffffu, my_flag != 0);
-    if (act != 0u) {
-      early_q = __ffs(act) - 1;
-      if (lane == 0) {   // the thread that initialised the barriers
-        prefetch_tensormap(mq); prefetch_tensormap(&map_do);
-        mbar_expect_tx(&q_full[0], 2 * Cfg::kTileBytes + Cfg::kStatBytes);
-        tma_load_3d(sQ, mq, &q_full[0], 0, early_q * kBwdTile, bh);
-        if (p.do_seq_first) tma_load_3d(sQ + Cfg::kTileBytes, &map_do, &q_full[0], 0, bh, early_q * kBwdTile);
-        else tma_load_3d(sQ + Cfg::kTileBytes, &map_do, &q_full[0], 0, early_q * kBwdTile, bh);
-      }
-    }
-  }
   tc_fence_before();
-  any_active = __syncthreads_or(any_active);
+  __syncthreads();
   tc_fence_after();
-  // Up to here nothing that the pass before this kernel writes (the statistics, the cleared dQ accumulators) has been
-  // touched, so all of it may overlap that pass; from here on it has to be complete.  The pass after this kernel (the dQ
-  // conversion) may be scheduled once every CTA has come this far; it waits for the whole grid itself.
-  griddep_wait();
-  if (tid == 0) griddep_launch();
-  const uint32_t tbase = *tmem_slot;
-  if (any_active == 0) {
-    // no query tile holds a pair of this pathway (every query on the other side of the mask): zero gradients; the copies of
-    // K and V must have landed and TMEM must be given back before the CTA leaves
-    write_zero_gradients();
-    if (tid == 0) mbar_wait(kv_full, 0, p.status, 0x500);
-    __syncthreads();
-    if (warp == 1) {
-      __syncwarp();
-      tmem_dealloc(tbase, Cfg::kTmemCols);
-    }
-    return;
+  // The loading warp plans its first key tile and requests what no recent pass has written before it waits for the pass before this
+  // kernel (the statistics, the cleared dQ accumulators); nothing else here happens before that wait.  The pass after this kernel
+  // (the dQ conversion) may be scheduled once every CTA has come this far; it waits for the whole grid itself.
+  if (warp != 3) {
+    griddep_wait();
+    if (tid == 0) griddep_launch();
   }
-  int n_active = 0;
-  for (int i = 0; i < nqt; ++i) n_active += tq[i] != 0;
-  n_active = __shfl_sync(0xffffffffu, n_active, 0);   // the same in every thread; the shuffle lets the compiler know it
+  const uint32_t tbase = *tmem_slot;
   // The MMA warps below run their loops with all lanes and let one elected lane issue: with warp-uniform control flow and
   // operands the descriptors stay in uniform registers, which is what tcgen05.mma reads; issued from a divergent single-lane
   // region every instruction first has to move its operands there.
@@ -412,28 +345,137 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
     return __all_sync(0xffffffffu, mbar_wait(bar, parity, p.status, code));
   };
   const uint32_t tbase_u = __shfl_sync(0xffffffffu, tbase, 0);
-  const int n_sub = 2 * n_active;   // 64-query halves, numbered u = 2 * tile + half; half u lives in buffer u % kNBuf
 
-  if (warp == 1) {
+  if (warp == 3) {
+    // ---------------------------------------------------------------- plans and TMA loads
+    const int nqt = (p.T + kBwdTile - 1) / kBwdTile, nkt = nqt;
+    Ring<kPlans> pr;
+    Ring<kKv> kr;
+    Ring<kQStages> lr;
+    bool ok = true;
+    for (int n = 0; ok; ++n) {
+      int item = 0;
+      if (lane == 0) item = n == 0 ? int(blockIdx.x) : int(gridDim.x) + atomicAdd(p.sched, 1);
+      item = __shfl_sync(0xffffffffu, item, 0);
+      if (item >= p.n_items) break;
+      const int kt = item % nkt, bh = (item / nkt) % (p.B * p.H), path = item / (nkt * p.B * p.H), b = bh / p.H;
+      const int k0 = kt * kBwdTile;
+      const uint8_t want = path == 0 ? kHasIntra : kHasInter;
+      const uint4 kw = *reinterpret_cast<const uint4*>(p.kpad + size_t(b) * p.TW + 4 * kt);
+      ok = wait_all(&plan_empty[pr.pos], pr.phase ^ 1, 0x520);
+      if (!ok) break;
+      BwdPlan& plan = plans[pr.pos];
+      int n_act = 0;
+      if ((kw.x & kw.y & kw.z & kw.w) != 0xffffffffu)   // (every key of the tile padded: padded batches have many such tiles)
+        for (int i0 = 0; i0 < nqt; i0 += 32) {
+          const int i = i0 + lane;
+          uint8_t c = 0;
+          bool pad = false;
+          if (i < nqt) {
+#pragma unroll
+            for (int a = 0; a < 2; ++a)
+#pragma unroll
+              for (int e = 0; e < 2; ++e)
+                if (2 * i + a < p.NT && 2 * kt + e < p.NT) c |= p.cls[(size_t(b) * p.NT + 2 * i + a) * p.NT + 2 * kt + e];
+            if (p.skip_pad_queries) {   // the padding bits describe positions: words 4 i .. 4 i + 3 cover the queries of tile i
+              const uint4 w = *reinterpret_cast<const uint4*>(p.kpad + size_t(b) * p.TW + 4 * i);
+              pad = (w.x & w.y & w.z & w.w) == 0xffffffffu;
+            }
+          }
+          const bool act = (c & want) != 0 && !pad;
+          const unsigned m = __ballot_sync(0xffffffffu, act);
+          if (act) plan.tiles[n_act + __popc(m & ((1u << lane) - 1u))] = uint16_t(i | ((c & 3) == 3 ? kMixed : 0));
+          n_act += __popc(m);
+        }
+      if (n_act == 0) {   // the gradients of a key tile without a single pair of this pathway are zero
+        for (int idx = lane; idx < kBwdTile * (D / 8); idx += 32) {
+          const int row = idx / (D / 8), vec = idx % (D / 8);
+          if (k0 + row < p.T) {
+            size_t base = size_t(k0 + row) * p.g_row + size_t(b) * p.g_b;
+            if (p.token_row != nullptr) {
+              const int tr = __ldg(p.token_row + size_t(k0 + row) * p.B + b);
+              if (tr < 0) continue;
+              base = size_t(tr) * p.g_b;
+            }
+            const size_t off = base + size_t(bh % p.H) * p.g_h + vec * 8;
+            *reinterpret_cast<uint4*>(p.dk[path] + off) = make_uint4(0u, 0u, 0u, 0u);
+            *reinterpret_cast<uint4*>(p.dv[path] + off) = make_uint4(0u, 0u, 0u, 0u);
+          }
+        }
+        continue;
+      }
+      if (lane == 0) {
+        plan.n = n_act; plan.kt = kt; plan.bh = bh; plan.path = path;
+        plan.kpad[0] = kw.x; plan.kpad[1] = kw.y; plan.kpad[2] = kw.z; plan.kpad[3] = kw.w;
+      }
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(&plan_full[pr.pos]);
+        const CUtensorMap* mq = path == 0 ? &map_qs : &map_qc;
+        const CUtensorMap* mk = path == 0 ? &map_ks : &map_kc;
+        const CUtensorMap* mv = path == 0 ? &map_vs : &map_vc;
+        ok = mbar_wait(&kv_empty[kr.pos], kr.phase ^ 1, p.status, 0x521);
+        if (ok) {
+          unsigned char* kv = sKV + size_t(kr.pos) * 2 * Cfg::kTileBytes;
+          mbar_expect_tx(&kv_full[kr.pos], 2 * Cfg::kTileBytes);
+          tma_load_3d(kv, mk, &kv_full[kr.pos], 0, k0, bh);
+          tma_load_3d(kv + Cfg::kTileBytes, mv, &kv_full[kr.pos], 0, k0, bh);
+        }
+        for (int t = 0; t < n_act && ok; ++t) {
+          const int i = plan.tiles[t] & (kMixed - 1);
+          ok = mbar_wait(&q_empty[lr.pos], lr.phase ^ 1, p.status, 0x525);
+          if (!ok) break;
+          unsigned char* dst = sQ + size_t(lr.pos) * 2 * Cfg::kTileBytes;
+          mbar_expect_tx(&q_full[lr.pos], 2 * Cfg::kTileBytes);
+          tma_load_3d(dst, mq, &q_full[lr.pos], 0, i * kBwdTile, bh);
+          if (p.do_seq_first) tma_load_3d(dst + Cfg::kTileBytes, &map_do, &q_full[lr.pos], 0, bh, i * kBwdTile);
+          else tma_load_3d(dst + Cfg::kTileBytes, &map_do, &q_full[lr.pos], 0, i * kBwdTile, bh);
+          if (t == 0) griddep_wait();   // (returns at once from the second time on)
+          mbar_expect_tx(&st_full[lr.pos], Cfg::kStatBytes);
+          bulk_load_1d(sStats + size_t(lr.pos) * Cfg::kStatBytes, p.stats + size_t(bh) * p.Tpad + size_t(i) * kBwdTile, Cfg::kStatBytes,
+                       &st_full[lr.pos]);
+          lr.advance();
+        }
+      }
+      ok = __shfl_sync(0xffffffffu, int(ok), 0) != 0;
+      pr.advance();
+      kr.advance();
+    }
+    if (ok) ok = wait_all(&plan_empty[pr.pos], pr.phase ^ 1, 0x526);
+    if (ok && lane == 0) {
+      plans[pr.pos].n = 0;
+      mbar_arrive(&plan_full[pr.pos]);
+    }
+    if (lane == 0) leave_tile_counter(p.sched, int(gridDim.x));
+    griddep_wait();
+  } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA stream A: S^T = K Q^T and dP^T = V dO^T
     // Issuing one tcgen05.mma costs its thread some 50 cycles whatever the tile size, and at small head sizes the
-    // products are tiny, so the four families of products are issued by four warps in parallel (disjoint accumulators).
-    if (n_active > 0) {
-      const bool leader = elect_one();
-      constexpr uint32_t idesc_s = idesc_bf16(kBwdTile, kHalf, false, false);   // M = 128 keys, N = 64 queries
-      constexpr uint32_t kHi = desc_hi32(8 * RB, swizzle_for_row_bytes(RB));
-      constexpr uint32_t kLbo = desc_lbo32(16);
-      const uint32_t k_lo = desc_addr32(__shfl_sync(0xffffffffu, smem_u32(sK), 0)) + kLbo;
-      const uint32_t v_lo = desc_addr32(__shfl_sync(0xffffffffu, smem_u32(sV), 0)) + kLbo;
-      const uint32_t q_lo = desc_addr32(__shfl_sync(0xffffffffu, smem_u32(sQ), 0)) + kLbo;
-      constexpr uint32_t kTileU = Cfg::kTileBytes >> 4, kHalfU = (kHalf * RB) >> 4;
-      bool ok = wait_all(kv_full, 0, 0x501);
-      Ring<kQStages> qr;     // query tile of the half being issued
-      Ring<kNBuf> ib;        // buffer of the half being issued
-      Ring<kNBuf> wb;        // buffer whose release is awaited next
-      auto issue_sdp = [&](int u) -> bool {   // both products of half u
+    // products are tiny, so the products are issued by three warps in parallel (disjoint accumulators).
+    const bool leader = elect_one();
+    constexpr uint32_t idesc_s = idesc_bf16(kBwdTile, kHalf, false, false);   // M = 128 keys, N = 64 queries
+    constexpr uint32_t kHi = desc_hi32(8 * RB, swizzle_for_row_bytes(RB));
+    constexpr uint32_t kLbo = desc_lbo32(16);
+    const uint32_t k_lo0 = desc_addr32(__shfl_sync(0xffffffffu, smem_u32(sKV), 0)) + kLbo;
+    const uint32_t q_lo = desc_addr32(__shfl_sync(0xffffffffu, smem_u32(sQ), 0)) + kLbo;
+    constexpr uint32_t kTileU = Cfg::kTileBytes >> 4, kHalfU = (kHalf * RB) >> 4;
+    bool ok = true;
+    Ring<kPlans> pr;
+    Ring<kKv> kr;
+    Ring<kQStages> qr;     // query tile of the half being issued
+    Ring<kNBuf> ib;        // its buffer
+    for (;;) {
+      ok = wait_all(&plan_full[pr.pos], pr.phase, 0x501);
+      if (!ok) break;
+      const int n = __shfl_sync(0xffffffffu, plans[pr.pos].n, 0);
+      if (n == 0) break;
+      ok = wait_all(&kv_full[kr.pos], kr.phase, 0x502);
+      const uint32_t k_lo = k_lo0 + kr.pos * 2 * kTileU, v_lo = k_lo + kTileU;
+      for (int u = 0; u < 2 * n && ok; ++u) {
         const int h = u & 1;
-        if (h == 0 && !wait_all(&q_full[qr.pos], qr.phase, 0x502)) return false;
+        ok = wait_all(&buf_free[ib.pos], ib.phase ^ 1, 0x505);
+        if (ok && h == 0) ok = wait_all(&q_full[qr.pos], qr.phase, 0x503);
+        if (!ok) break;
         tc_fence_after();
         const uint32_t qs = q_lo + qr.pos * 2 * kTileU + h * kHalfU;
         const uint32_t dos = qs + kTileU;
@@ -448,44 +490,48 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
         __syncwarp();
         ib.advance();
         if (h == 1) qr.advance();
-        return true;
-      };
-      int issued = 0;
-      for (; issued < kNBuf && issued < n_sub && ok; ++issued) ok = issue_sdp(issued);
-      for (int u = 0; issued < n_sub && ok; ++u, ++issued) {
-        ok = wait_all(&buf_free[wb.pos], wb.phase, 0x505);   // dV and dK of half u have consumed P^T, dS^T
-        if (!ok) break;
-        wb.advance();
-        ok = issue_sdp(issued);
       }
+      if (!ok) break;
+      if (leader) {
+        umma_commit(&kv_empty[kr.pos]);
+        mbar_arrive(&plan_empty[pr.pos]);
+      }
+      __syncwarp();
+      pr.advance();
+      kr.advance();
     }
-  } else if (warp == 2 || warp == 3) {
-    // ---------------------------------------------------------------- MMA streams V and K: dV += P^T dO, dK += dS^T Q
-    if (n_active > 0) {
-      const bool leader = elect_one();
-      constexpr uint32_t idesc_acc = idesc_bf16(kBwdTile, D, false, true);      // A from TMEM, B rows of dO / Q (N = D contiguous)
-      constexpr uint32_t kHi = desc_hi32(8 * RB, swizzle_for_row_bytes(RB));
-      constexpr uint32_t kLbo = desc_lbo32(8 * RB);
-      constexpr uint32_t kTileU = Cfg::kTileBytes >> 4, kHalfU = (kHalf * RB) >> 4, kStep = (16 * RB) >> 4;
-      const bool is_v = __shfl_sync(0xffffffffu, warp, 0) == 2;
-      // dV reads P^T (over S^T) and dO; dK reads dS^T (over dP^T, 64 columns further) and Q
-      const uint32_t b_lo = desc_addr32(__shfl_sync(0xffffffffu, smem_u32(sQ), 0)) + kLbo + (is_v ? kTileU : 0u);
-      const uint32_t a_col = tbase_u + kColBuf + (is_v ? 0u : 64u);
-      const uint32_t d_col = tbase_u + (is_v ? kColDV : kColDK);
-      bool ok = true;
-      Ring<kQStages> qr;
-      Ring<kNBuf> br;
-      for (int it = 0; it < n_active && ok; ++it) {
+  } else if (warp == 2) {
+    // ---------------------------------------------------------------- MMA stream B: dV += P^T dO, dK += dS^T Q
+    const bool leader = elect_one();
+    constexpr uint32_t idesc_acc = idesc_bf16(kBwdTile, D, false, true);      // A from TMEM, B rows of dO / Q (N = D contiguous)
+    constexpr uint32_t kHi = desc_hi32(8 * RB, swizzle_for_row_bytes(RB));
+    constexpr uint32_t kTileU = Cfg::kTileBytes >> 4, kHalfU = (kHalf * RB) >> 4, kStep = (16 * RB) >> 4;
+    const uint32_t q_lo = desc_addr32(__shfl_sync(0xffffffffu, smem_u32(sQ), 0)) + desc_lbo32(8 * RB);
+    bool ok = true;
+    Ring<kPlans> pr;
+    Ring<1> ar;            // the accumulators, given back once the previous key tile's values have been read
+    Ring<kQStages> qr;
+    Ring<kNBuf> br;
+    for (;;) {
+      ok = wait_all(&plan_full[pr.pos], pr.phase, 0x510);
+      if (!ok) break;
+      const int n = __shfl_sync(0xffffffffu, plans[pr.pos].n, 0);
+      if (n == 0) break;
+      ok = wait_all(acc_empty, ar.phase ^ 1, 0x513);
+      for (int it = 0; it < n && ok; ++it) {
         ok = wait_all(&q_full[qr.pos], qr.phase, 0x511);
         for (int h = 0; h < 2 && ok; ++h) {
           ok = wait_all(&pds_full[br.pos], br.phase, 0x512);
           if (!ok) break;
           tc_fence_after();
-          const uint32_t rows = b_lo + qr.pos * 2 * kTileU + h * kHalfU;
+          const uint32_t q = q_lo + qr.pos * 2 * kTileU + h * kHalfU, d_o = q + kTileU;
+          const uint32_t pt = tbase_u + kColBuf + br.pos * 128, ds = pt + 64;   // P^T lies over S^T, dS^T over dP^T
           if (leader) {
 #pragma unroll
-            for (int k = 0; k < kHalf / 16; ++k)
-              umma_ts(d_col, a_col + br.pos * 128 + k * 16, make_desc(kHi, rows + k * kStep), idesc_acc, it > 0 || h > 0 || k > 0);
+            for (int k = 0; k < kHalf / 16; ++k) {
+              umma_ts(tbase_u + kColDV, pt + k * 16, make_desc(kHi, d_o + k * kStep), idesc_acc, it > 0 || h > 0 || k > 0);
+              umma_ts(tbase_u + kColDK, ds + k * 16, make_desc(kHi, q + k * kStep), idesc_acc, it > 0 || h > 0 || k > 0);
+            }
             umma_commit(&buf_free[br.pos]);
           }
           __syncwarp();
@@ -495,109 +541,102 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
         __syncwarp();
         qr.advance();
       }
-      if (ok && leader) umma_commit(acc_full);
-    }
-  } else if (warp == 0) {
-    // ---------------------------------------------------------------- TMA loads and MMA stream Q: dQ tile = dS K
-    // One thread does both: it loads K, V and the first query tiles, then per tile issues the dQ product and
-    // refills the stage that tile has just released with the tile kQStages steps ahead.
-    if (n_active > 0) {
-      const bool leader = elect_one();
-      constexpr uint32_t idesc_dq = idesc_bf16(kBwdTile, D, true, true);        // A = dS (queries contiguous), B = K (D contiguous)
-      constexpr uint32_t kHiA = desc_hi32(8 * 128, kSw128), kHiB = desc_hi32(8 * RB, swizzle_for_row_bytes(RB));
-      const uint32_t ds_lo = desc_addr32(__shfl_sync(0xffffffffu, smem_u32(sDS), 0)) + desc_lbo32(Cfg::kDsBlock);
-      const uint32_t kb_lo = desc_addr32(__shfl_sync(0xffffffffu, smem_u32(sK), 0)) + desc_lbo32(8 * RB);
-      constexpr uint32_t kDsU = Cfg::kDsBytes >> 4, kAStep = (16 * 128) >> 4, kBStep = (16 * RB) >> 4;
-      if (leader) { prefetch_tensormap(mq); prefetch_tensormap(&map_do); }      // (K and V were requested before the query-tile scan)
-      int next_q = 0;        // next query tile index to look at (the elected lane's copy is the one that counts)
-      Ring<kQStages> lr;     // stage the next load goes to (likewise)
-      auto load_next = [&]() {   // issue the loads of the next active query tile; called by the elected lane only
-        while (next_q < nqt && tq[next_q] == 0) ++next_q;
-        if (next_q >= nqt) return;
-        unsigned char* dst = sQ + size_t(lr.pos) * 2 * Cfg::kTileBytes;
-        const bool early = next_q == early_q;   // Q and dO of this tile (the first one, stage 0) were requested during the set-up
-        if (!early) mbar_expect_tx(&q_full[lr.pos], 2 * Cfg::kTileBytes + Cfg::kStatBytes);
-        bulk_load_1d(sStats + size_t(lr.pos) * Cfg::kStatBytes, p.stats + size_t(bh) * p.Tpad + size_t(next_q) * kBwdTile,
-                     Cfg::kStatBytes, &q_full[lr.pos]);
-        if (!early) {
-          tma_load_3d(dst, mq, &q_full[lr.pos], 0, next_q * kBwdTile, bh);
-          if (p.do_seq_first) tma_load_3d(dst + Cfg::kTileBytes, &map_do, &q_full[lr.pos], 0, bh, next_q * kBwdTile);
-          else tma_load_3d(dst + Cfg::kTileBytes, &map_do, &q_full[lr.pos], 0, next_q * kBwdTile, bh);
-        }
-        ++next_q;
-        lr.advance();
-      };
+      if (!ok) break;
       if (leader) {
-        for (int s = 0; s < kQStages; ++s) load_next();
+        umma_commit(acc_full);
+        mbar_arrive(&plan_empty[pr.pos]);
       }
       __syncwarp();
-      bool ok = wait_all(kv_full, 0, 0x521);
-      Ring<kNBuf> br;        // buffers of the two halves of the tile
-      Ring<kQStages> er;     // stage released by the tile
-      for (int it = 0; it < n_active && ok; ++it) {
-        ok = wait_all(&pds_full[br.pos], br.phase, 0x522);
-        br.advance();
-        if (ok) ok = wait_all(&pds_full[br.pos], br.phase, 0x523);
-        br.advance();
-        if (ok) ok = wait_all(&dq_empty[it % kNDq], ((it / kNDq) & 1) ^ 1, 0x524);   // buffer drained kNDq tiles ago
+      pr.advance();
+      ar.advance();
+    }
+  } else if (warp == 0) {
+    // ---------------------------------------------------------------- MMA stream Q: dQ tile = dS K
+    const bool leader = elect_one();
+    constexpr uint32_t idesc_dq = idesc_bf16(kBwdTile, D, true, true);        // A = dS (queries contiguous), B = K (D contiguous)
+    constexpr uint32_t kHiA = desc_hi32(8 * 128, kSw128), kHiB = desc_hi32(8 * RB, swizzle_for_row_bytes(RB));
+    const uint32_t ds_lo = desc_addr32(__shfl_sync(0xffffffffu, smem_u32(sDS), 0)) + desc_lbo32(Cfg::kDsBlock);
+    const uint32_t kb_lo0 = desc_addr32(__shfl_sync(0xffffffffu, smem_u32(sKV), 0)) + desc_lbo32(8 * RB);
+    constexpr uint32_t kDsU = Cfg::kDsBytes >> 4, kAStep = (16 * 128) >> 4, kBStep = (16 * RB) >> 4, kTileU = Cfg::kTileBytes >> 4;
+    bool ok = true;
+    Ring<kPlans> pr;
+    Ring<kKv> kr;
+    Ring<kNBuf> br;        // buffers of the two halves of the tile
+    Ring<kNDq> dr;
+    for (;;) {
+      ok = wait_all(&plan_full[pr.pos], pr.phase, 0x527);
+      if (!ok) break;
+      const int n = __shfl_sync(0xffffffffu, plans[pr.pos].n, 0);
+      if (n == 0) break;
+      ok = wait_all(&kv_full[kr.pos], kr.phase, 0x528);
+      const uint32_t kb_lo = kb_lo0 + kr.pos * 2 * kTileU;
+      for (int it = 0; it < n && ok; ++it) {
+        for (int h = 0; h < 2 && ok; ++h) {
+          ok = wait_all(&pds_full[br.pos], br.phase, 0x522);
+          // (its arrival keeps the buffer from being filled again, twice, before this warp has looked)
+          if (ok && leader) mbar_arrive(&buf_free[br.pos]);
+          br.advance();
+        }
+        if (ok) ok = wait_all(&dq_empty[dr.pos], dr.phase ^ 1, 0x524);   // tile drained kNDq tiles ago
         if (!ok) break;
         tc_fence_after();
-        const uint32_t a_lo = ds_lo + uint32_t(it % kNDq) * kDsU;
+        const uint32_t a_lo = ds_lo + dr.pos * kDsU;
         if (leader) {
 #pragma unroll
           for (int k = 0; k < kBwdTile / 16; ++k)
-            umma_ss(tbase_u + kColDQ + (it % kNDq) * kAcc, make_desc(kHiA, a_lo + k * kAStep), make_desc(kHiB, kb_lo + k * kBStep), idesc_dq, k > 0);
-          umma_commit(&dq_full[it % kNDq]);
+            umma_ss(tbase_u + kColDQ + dr.pos * kAcc, make_desc(kHiA, a_lo + k * kAStep), make_desc(kHiB, kb_lo + k * kBStep), idesc_dq, k > 0);
+          umma_commit(&dq_full[dr.pos]);
         }
         __syncwarp();
-        if (it + kQStages < n_active) {   // this tile's stage is released by its dV and dK streams
-          ok = wait_all(&q_empty[er.pos], er.phase, 0x525);
-          if (ok && leader) load_next();
-          __syncwarp();
-        }
-        er.advance();
+        dr.advance();
       }
+      if (!ok) break;
+      if (leader) {
+        umma_commit(&kv_empty[kr.pos]);
+        mbar_arrive(&plan_empty[pr.pos]);
+      }
+      __syncwarp();
+      pr.advance();
+      kr.advance();
     }
   } else {
     // ---------------------------------------------------------------- compute warps (lane = key row)
-    // 16 warps work on ONE 64-query half at a time: thread = key row x 16 query columns (group grp = 0..3).  The
-    // products run up to kNBuf halves ahead, and groups 2,3 start a fraction of a half later than groups 0,1 so that the
-    // exp2-heavy part of one pair of groups overlaps the TMEM traffic and barrier work of the other.
-    // Everything here is elementwise: no exchange between threads.
-    const int cwp = warp - 4;                     // 0..kCW-1
-    const int grp = cwp / 4;                      // physical group; it covers the 16-column groups vg = grp * kVPG + v
+    // 8 warps work on each of the two 64-query halves of a tile: thread = key row x 32 query columns, so that the chain from
+    // the wait to the arrival is paid once per 32 exponentials and the two sets of warps fill each other's waits (16 warps on
+    // one half after the other, 16 columns each: 249 -> 228 us at B8 H20 T1024 D32).  Everything is elementwise: no exchange
+    // between threads.
+    constexpr int hD = D / 2, NC = D / 4;
+    const int cwp = warp - 4;                     // 0..15
+    const int grp = cwp / 4;                      // pair (half, 32 columns of it); also the warp's share of dQ and of the gradients
+    const int sub = grp / 2, c32 = grp & 1;
     const int quarter = warp % 4;
     const int r = quarter * 32 + lane;            // key row in the tile == TMEM lane
-    const int kj = k0 + r;
-    const int krow = kj < p.T ? kj : p.T - 1;
     const uint32_t lane_base = uint32_t(quarter * 32) << 16;
-    const uint32_t tBuf = tbase + lane_base + kColBuf;   // + 128 * buffer + 16 * vg: S^T columns of this thread; dP^T 64 further
-    const bool key_valid = kj < p.T && !((p.kpad[size_t(b) * p.TW + krow / 32] >> (krow % 32)) & 1u);
-    const uint32_t* mrow = p.bitsT + (size_t(b) * p.T + krow) * p.TW + grp / 2;   // words grp / 2 and 2 + grp / 2 of a tile's four
-    const int mshift = 16 * (grp & 1);
-    const uint32_t flip = path == 0 ? 0xffffu : 0u;   // keep-bit = mask bit XOR flip
+    const uint32_t tBuf = tbase + lane_base + kColBuf + 32 * c32;   // + 128 * buffer: S^T columns of this thread; dP^T 64 further
+    const uint32_t ds_addr = smem_u32(sDS) + uint32_t(sub) * Cfg::kDsBlock + swizzled_offset(r, 4 * c32, 128);
     const uint64_t c22 = pack2(p.scale_log2, p.scale_log2);
+    unsigned char* my_stage = sDqStage + size_t(cwp) * Cfg::kDqWarpBytes;
     bool ok = true;
-    int it = 0;
-    Ring<kNBuf> br;
-    Ring<kQStages> sr;     // stage that holds the current tile's statistics
+    Ring<kNBuf> br;        // buffer of this warp's half: every other one
+    if (sub == 1) br.advance();
+    // The other rings follow from two counts (registers are what this loop is short of, so it also reads the plans' fields again
+    // rather than keep them): query tiles handed to the tensor cores so far, and key tiles.
+    uint32_t g = 0, m = 0;
 
     // dQ of a tile leaves through shared memory: each compute warp stages its 32 queries x NC columns and one lane adds
     // them to the fp32 accumulator in HBM with ONE bulk reduction (instead of a 16-byte atomic per thread and 4 columns).
-    const CUtensorMap* mdq = path == 0 ? &map_dq_s : &map_dq_c;
-    unsigned char* my_stage = sDqStage + size_t(cwp) * Cfg::kDqWarpBytes;
-    auto drain_dq = [&](int jt, int qtile) -> bool {   // add dQ of active tile jt (query tile qtile) to HBM
-      if (!mbar_wait(&dq_full[jt % kNDq], (jt / kNDq) & 1, p.status, 0x601)) return false;
+    auto drain_dq = [&](const BwdPlan& plan, int it, uint32_t g) -> bool {   // add dQ of the plan's tile `it`, number g of all, to HBM
+      const uint32_t xb = g % kNDq;
+      if (!wait_all(&dq_full[xb], (g / kNDq) & 1u, 0x601)) return false;
       tc_fence_after();
-      constexpr int NC = D / 4 * kVPG;   // columns per thread
       constexpr int kRowB = NC * 4;      // bytes per staged row: 64, 32 or 16
       uint32_t v[NC];
-      tmem_ld_n<NC>(tbase + lane_base + kColDQ + (jt % kNDq) * kAcc + grp * NC, v);
+      tmem_ld_n<NC>(tbase + lane_base + kColDQ + xb * kAcc + grp * NC, v);
       if (lane == 0) bulk_wait_read_all();   // the previous reduction of this warp has read the staging rows
       __syncwarp();
       tmem_ld_wait();
       tc_fence_before();
-      mbar_arrive(&dq_empty[jt % kNDq]);
+      mbar_arrive(&dq_empty[xb]);
 #pragma unroll
       for (int e = 0; e < NC; e += 4) {
         const uint32_t off = kRowB == 16 ? uint32_t(lane) * 16u : swizzled_offset(lane, e / 4, kRowB);
@@ -605,199 +644,225 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
       }
       fence_proxy_async_smem();
       __syncwarp();
-      if (lane == 0 && qtile * kBwdTile + quarter * 32 < p.T) {   // rows past T inside the box are dropped by the copy engine
-        tma_reduce_add_3d(mdq, my_stage, grp * NC, qtile * kBwdTile + quarter * 32, bh);
-        bulk_commit_group();
+      if (lane == 0) {
+        const int row = (plan.tiles[it] & (kMixed - 1)) * kBwdTile + quarter * 32;
+        if (row < p.T) {   // rows past T inside the box are dropped by the copy engine
+          tma_reduce_add_3d(plan.path == 0 ? &map_dq_s : &map_dq_c, my_stage, grp * NC, row, plan.bh);
+          bulk_commit_group();
+        }
       }
       return true;
     };
 
-    // Mask bits of a tile for this key row (four words); asked for one tile ahead, so that a mixed tile does not wait for them.
-    auto next_active = [&](int i) {
-      while (i < nqt && tq[i] == 0) ++i;
-      return i;
-    };
-    auto tile_mask = [&](int i) {   // bits of this thread's 16 queries in the two halves
-      if (!(i < nqt && (tq[i] & 2))) return make_ushort2(0xffffu, 0xffffu);
-      const uint32_t a = __ldg(mrow + 4 * i), b = __ldg(mrow + 4 * i + 2);
-      return make_ushort2((unsigned short)((a >> mshift) ^ flip), (unsigned short)((b >> mshift) ^ flip));
-    };
-    int prev_tile = -1;
-    int i = next_active(0), i_next;
-    ushort2 mask = tile_mask(i), mask_next;
-    const uint32_t ds_addr = smem_u32(sDS) + swizzled_offset(r, 2 * grp * kVPG, 128);   // (the other chunk of a group of 16 columns: bit 4 flipped)
-    for (; i < nqt && ok; i = i_next, mask = mask_next) {
-      i_next = next_active(i + 1);
-      mask_next = tile_mask(i_next);
-#pragma unroll 1
-      for (int sub = 0; sub < 2 && ok; ++sub) {
-        ok = mbar_wait(&sdp_full[br.pos], br.phase, p.status, 0x602);
-        if (!ok) break;
-        if (sub == 0) {   // the tile's loads have landed long ago (its products are done): this only orders the reads below
-          ok = mbar_wait(&q_full[sr.pos], sr.phase, p.status, 0x604);
-          if (!ok) break;
+    // What is left of a key tile: the last dQ tile, then dK (scaled, un-rotated for the self pathway) and dV.  Groups 0, 1 take dK:
+    // the columns [NC half, + NC) and the ones the rotation pairs them with, hD further; groups 2, 3 half of dV's columns each.
+    // The rotation's table rows are read with whole rows per group of lanes and turned in shared memory: a row per lane took one
+    // 128-byte line per lane and instruction, 7000 cycles of a key tile at head_dim 64 against 2300 without rotation.
+    auto finish_item = [&](const BwdPlan& plan, uint32_t m, uint32_t g) -> bool {   // plan number m, whose last tile is number g
+      const int k0 = plan.kt * kBwdTile, kj = k0 + r, bh = plan.bh, b = bh / p.H, path = plan.path;
+      const bool is_dk = grp < 2;
+      const int half = grp & 1;
+      const bool rot = is_dk && path == 0 && p.cos_tab != nullptr;
+      constexpr int kLpr = NC / 4;   // lanes per table row: 4, 2 or 1
+      float4 tc[kLpr], ts[kLpr];
+      if (rot) {
+#pragma unroll
+        for (int i = 0; i < kLpr; ++i) {
+          const int row = k0 + quarter * 32 + i * (32 / kLpr) + lane / kLpr;
+          const size_t at = size_t(row < p.T ? row : p.T - 1) * hD + half * NC + (lane % kLpr) * 4;
+          tc[i] = __ldg(reinterpret_cast<const float4*>(p.cos_tab + at));
+          ts[i] = __ldg(reinterpret_cast<const float4*>(p.sin_tab + at));
         }
-        if (it == 0 && sub == 0 && grp >= 2) __nanosleep(kBwdStaggerNs);
-        tc_fence_after();
-        const uint32_t ds_row = ds_addr + uint32_t(it % kNDq) * Cfg::kDsBytes + uint32_t(sub) * Cfg::kDsBlock;
-#pragma unroll
-        for (int v = 0; v < kVPG; ++v) {
-          const int vg = grp * kVPG + v;
-          // statistics of this thread's 16 queries, (nl0, nl1, nd0, nd1) per pair, from the copy that arrived in shared memory with the query tile
-          const float4* st = reinterpret_cast<const float4*>(sStats + size_t(sr.pos) * Cfg::kStatBytes) + (sub * kHalf + 16 * vg) / 2;
-          uint32_t keep = sub == 0 ? mask.x : mask.y;
-          if (!key_valid) keep = 0u;
-          const uint32_t tS = tBuf + br.pos * 128 + 16 * vg;
-          uint32_t sv[16], dpv[16];
-          tmem_ld16(tS, sv);
-          tmem_ld16(tS + 64, dpv);
-          tmem_ld_wait();
-          uint32_t pp[8], dd[8];
-          // Straight-line code for each of the two cases: a test inside the loop would cut it into blocks that end in
-          // reconvergence points, and the exponentials of one pair of queries could not overlap those of the next.
-          auto elements = [&](auto masked) {
-#pragma unroll
-            for (int j = 0; j < 16; j += 2) {
-              const float4 q2 = st[j / 2];
-              float p0, p1;
-              unpack2(ffma2(pack2(__uint_as_float(sv[j]), __uint_as_float(sv[j + 1])), c22, pack2(q2.x, q2.y)), p0, p1);
-              p0 = bwd_ex2(p0);
-              p1 = bwd_ex2(p1);
-              if (decltype(masked)::value) {
-                p0 = (keep >> j) & 1u ? p0 : 0.f;
-                p1 = (keep >> (j + 1)) & 1u ? p1 : 0.f;
-              }
-              float d0, d1;
-              const uint64_t p2 = pack2(p0, p1), dp2 = pack2(__uint_as_float(dpv[j]), __uint_as_float(dpv[j + 1])), nd2 = pack2(q2.z, q2.w);
-              if (SQ)   // r = sqrt(p) is what p0, p1 hold: dS = r (dP / 2 - r delta / 2), and r itself multiplies dO in dV
-                unpack2(fmul2(p2, ffma2(p2, nd2, fmul2(dp2, pack2(0.5f, 0.5f)))), d0, d1);
-              else      // dS = p (dP - delta)
-                unpack2(fmul2(p2, fadd2(dp2, nd2)), d0, d1);
-              pp[j / 2] = bwd_pack(p0, p1);
-              dd[j / 2] = bwd_pack(d0, d1);
-            }
-          };
-          if (__all_sync(0xffffffffu, keep == 0xffffu)) {
-            elements(std::false_type{});
-          } else if (__all_sync(0xffffffffu, keep == 0u)) {   // the other side of a chain boundary, or padding
-#pragma unroll
-            for (int j = 0; j < 8; ++j) pp[j] = dd[j] = 0u;
-          } else {
-            elements(std::true_type{});
-          }
-          tmem_st8(tS, pp);         // P^T over the S^T columns this thread has read
-          tmem_st8(tS + 64, dd);    // dS^T likewise
-          // and dS into shared memory for the dQ product: 2 chunks of 8 queries in block `sub` of the dS tile
-          const uint32_t ds_at = kVPG == 1 ? ds_row : ds_row ^ (v * 32);
-          smem_store16(ds_at, dd[0], dd[1], dd[2], dd[3]);
-          smem_store16(ds_at ^ 16u, dd[4], dd[5], dd[6], dd[7]);
-        }
-        tmem_st_wait();
-        fence_proxy_async_smem();
-        tc_fence_before();
-        mbar_arrive(&pds_full[br.pos]);
-        br.advance();
       }
-      if (!ok) break;
-      if (prev_tile >= 0) ok = drain_dq(it - 1, prev_tile);
-      prev_tile = i;
-      sr.advance();
-      ++it;
-    }
-    if (ok && prev_tile >= 0) ok = drain_dq(it - 1, prev_tile);
-    if (lane == 0) bulk_wait_read_all();   // the reductions have read their staging rows (their additions may still be under way)
-
-    // ---- epilogue: 16-column groups vg 0,1 write the two column halves of dK (scaled, un-rotated for the self pathway),
-    //      vg 2,3 those of dV
-    if (n_active > 0) {
-      if (ok) ok = mbar_wait(acc_full, 0, p.status, 0x603);
+      // element offset of this thread's row in dk / dv, negative when the key has no row (past T, or dropped token)
+      long long row_off = -1;
+      if (kj < p.T) {
+        row_off = static_cast<long long>(size_t(kj) * p.g_row + size_t(b) * p.g_b);
+        if (p.token_row != nullptr) {
+          const int tr = __ldg(p.token_row + size_t(kj) * p.B + b);
+          row_off = tr < 0 ? -1 : static_cast<long long>(size_t(tr) * p.g_b);
+        }
+        if (row_off >= 0) row_off += static_cast<long long>(size_t(bh % p.H) * p.g_h);
+      }
+      if (!drain_dq(plan, plan.n - 1, g)) return false;
+      if (lane == 0) bulk_wait_read_all();   // the staging rows of the dQ reduction are reused below
+      __syncwarp();
+      if (rot) {
+        auto turn = [&](float4 (&x)[kLpr]) {   // this lane's row of the 32 that the warp has loaded
+          if constexpr (kLpr > 1) {
+#pragma unroll
+            for (int i = 0; i < kLpr; ++i)
+              *reinterpret_cast<float4*>(my_stage + swizzled_offset(i * (32 / kLpr) + lane / kLpr, lane % kLpr, NC * 4)) = x[i];
+            __syncwarp();
+#pragma unroll
+            for (int i = 0; i < kLpr; ++i) x[i] = *reinterpret_cast<const float4*>(my_stage + swizzled_offset(lane, i, NC * 4));
+            __syncwarp();
+          }
+        };
+        turn(tc);
+        turn(ts);
+      }
+      if (!wait_all(acc_full, m & 1u, 0x603)) return false;
       tc_fence_after();
-    }
-    ok = __all_sync(0xffffffffu, ok);   // the stores below exchange rows between the lanes of the warp
-    if (ok) {
-      constexpr int hD = D / 2;
-      constexpr int kPieces = hD / 8;   // 16-byte pieces of a thread's half row: 4, 2 or 1
-      if (kPieces > 1) {                // the staging rows of the dQ reductions are reused below
-        if (lane == 0) bulk_wait_read_all();
+      const int col0 = is_dk ? half * NC : half * hD, col1 = is_dk ? hD + half * NC : half * hD + NC;
+      uint32_t t0[NC], t1[NC];
+      {
+        const uint32_t src = tbase + lane_base + (is_dk ? kColDK : kColDV);
+        tmem_ld_n<NC>(src + col0, t0);
+        tmem_ld_n<NC>(src + col1, t1);
+        tmem_ld_wait();
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(acc_empty);
+      float o0[NC], o1[NC];
+      const float mul = is_dk ? p.scale : 1.f;
+      if (rot) {   // R^T: dx_lo = dy_lo c + dy_hi s, dx_hi = dy_hi c - dy_lo s
+#pragma unroll
+        for (int i = 0; i < kLpr; ++i) {
+          const float cv[4] = {tc[i].x, tc[i].y, tc[i].z, tc[i].w}, sv[4] = {ts[i].x, ts[i].y, ts[i].z, ts[i].w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float lo = __uint_as_float(t0[4 * i + e]), hi = __uint_as_float(t1[4 * i + e]);
+            o0[4 * i + e] = (lo * cv[e] + hi * sv[e]) * mul;
+            o1[4 * i + e] = (hi * cv[e] - lo * sv[e]) * mul;
+          }
+        }
+      } else {
+#pragma unroll
+        for (int d = 0; d < NC; ++d) {
+          o0[d] = __uint_as_float(t0[d]) * mul;
+          o1[d] = __uint_as_float(t1[d]) * mul;
+        }
+      }
+      __nv_bfloat16* base = is_dk ? p.dk[path] : p.dv[path];
+      if constexpr (NC == 4) {
+        if (row_off >= 0) {
+          *reinterpret_cast<uint2*>(base + row_off + col0) = make_uint2(bwd_pack(o0[0], o0[1]), bwd_pack(o0[2], o0[3]));
+          *reinterpret_cast<uint2*>(base + row_off + col1) = make_uint2(bwd_pack(o1[0], o1[1]), bwd_pack(o1[2], o1[3]));
+        }
+      } else {
+        // Rows of different keys lie far apart (row-major gradients) or 2 D elements apart: staged per warp and read back so
+        // that the neighbouring lanes that write one row's pieces cover whole runs of it.
+        constexpr int kPieces = hD / 8, kRowB = hD * 2;   // 16-byte pieces of a row, 4 or 2: half of them from each column range
+#pragma unroll
+        for (int j = 0; j < NC; j += 8) {
+          *reinterpret_cast<uint4*>(my_stage + swizzled_offset(lane, j / 8, kRowB)) =
+              make_uint4(bwd_pack(o0[j], o0[j + 1]), bwd_pack(o0[j + 2], o0[j + 3]), bwd_pack(o0[j + 4], o0[j + 5]), bwd_pack(o0[j + 6], o0[j + 7]));
+          *reinterpret_cast<uint4*>(my_stage + swizzled_offset(lane, (NC + j) / 8, kRowB)) =
+              make_uint4(bwd_pack(o1[j], o1[j + 1]), bwd_pack(o1[j + 2], o1[j + 3]), bwd_pack(o1[j + 4], o1[j + 5]), bwd_pack(o1[j + 6], o1[j + 7]));
+        }
+        __syncwarp();
+        const int piece = lane % kPieces;
+        const int col = piece < kPieces / 2 ? col0 + piece * 8 : col1 + (piece - kPieces / 2) * 8;
+#pragma unroll
+        for (int i = 0; i < kPieces; ++i) {
+          const int row = i * (32 / kPieces) + lane / kPieces;
+          const long long ro = __shfl_sync(0xffffffffu, row_off, row);
+          const uint4 q = *reinterpret_cast<const uint4*>(my_stage + swizzled_offset(row, piece, kRowB));
+          if (ro >= 0) *reinterpret_cast<uint4*>(base + ro + col) = q;
+        }
         __syncwarp();
       }
+      return true;
+    };
+
+    for (;; ++m) {
+      ok = wait_all(&plan_full[m % kPlans], (m / kPlans) & 1u, 0x600);
+      if (!ok) break;
+      const BwdPlan& plan = plans[m % kPlans];
+      const int n = plan.n;
+      // Which of the thread's 32 queries of tile `it` its key belongs to; asked for one tile ahead, so that a mixed tile does
+      // not wait for its mask words.
+      auto tile_mask = [&](int it) -> uint32_t {
+        const uint32_t e = plan.tiles[it];
+        if (plan.kt * kBwdTile + r >= p.T || ((plan.kpad[quarter] >> lane) & 1u)) return 0u;
+        if (!(e & kMixed)) return 0xffffffffu;
+        const uint32_t bits = __ldg(p.bitsT + (size_t(plan.bh / p.H) * p.T + plan.kt * kBwdTile + r) * p.TW + 4 * (e & (kMixed - 1)) + grp);
+        return plan.path == 0 ? ~bits : bits;
+      };
+      uint32_t mask = n > 0 ? tile_mask(0) : 0u;
+      // (one more round without a tile after the last key tile: its gradients leave there)
+      for (int it = 0; it < (n > 0 ? n : 1) && ok; ++it) {
+        if (n > 0) {
+          const uint32_t mask_next = it + 1 < n ? tile_mask(it + 1) : 0u;
+          ok = wait_all(&st_full[g % kQStages], (g / kQStages) & 1u, 0x604);
+          if (ok) ok = wait_all(&sdp_full[br.pos], br.phase, 0x602);
+          if (!ok) break;
+          tc_fence_after();
+          const uint32_t ds_row = ds_addr + (g % kNDq) * Cfg::kDsBytes;
 #pragma unroll
-      for (int v = 0; v < kVPG; ++v) {
-        const int vg = grp * kVPG + v;
-        const bool is_dk = vg < 2;
-        const int half_col = vg & 1;
-        float lo[hD], hi[hD];   // lower / upper half of the row (dK needs both for the rotation; dV only its own)
-        if (n_active > 0) {
-          const uint32_t src = tbase + lane_base + (is_dk ? kColDK : kColDV);
-          uint32_t t0[hD], t1[hD];
-          if (is_dk || half_col == 0) tmem_ld_n<hD>(src, t0);
-          if (is_dk || half_col == 1) tmem_ld_n<hD>(src + hD, t1);
-          tmem_ld_wait();
+          for (int v = 0; v < 2; ++v) {
+            // statistics of this thread's 16 queries, (nl0, nl1, nd0, nd1) per pair, from the copy that arrived in shared memory with the query tile
+            const float4* st = reinterpret_cast<const float4*>(sStats + (g % kQStages) * Cfg::kStatBytes) + (sub * kHalf + 32 * c32 + 16 * v) / 2;
+            const uint32_t keep = (mask >> (16 * v)) & 0xffffu;
+            const uint32_t tS = tBuf + br.pos * 128 + 16 * v;
+            uint32_t sv[16], dpv[16];
+            tmem_ld16(tS, sv);
+            tmem_ld16(tS + 64, dpv);
+            tmem_ld_wait();
+            uint32_t pp[8], dd[8];
+            // Straight-line code for each of the two cases: a test inside the loop would cut it into blocks that end in
+            // reconvergence points, and the exponentials of one pair of queries could not overlap those of the next.
+            auto elements = [&](auto masked) {
 #pragma unroll
-          for (int j = 0; j < hD; ++j) { lo[j] = __uint_as_float(t0[j]); hi[j] = __uint_as_float(t1[j]); }
-        } else {
+              for (int j = 0; j < 16; j += 2) {
+                const float4 q2 = st[j / 2];
+                float p0, p1;
+                unpack2(ffma2(pack2(__uint_as_float(sv[j]), __uint_as_float(sv[j + 1])), c22, pack2(q2.x, q2.y)), p0, p1);
+                p0 = bwd_ex2(p0);
+                p1 = bwd_ex2(p1);
+                if (decltype(masked)::value) {
+                  p0 = (keep >> j) & 1u ? p0 : 0.f;
+                  p1 = (keep >> (j + 1)) & 1u ? p1 : 0.f;
+                }
+                float d0, d1;
+                const uint64_t p2 = pack2(p0, p1), dp2 = pack2(__uint_as_float(dpv[j]), __uint_as_float(dpv[j + 1])), nd2 = pack2(q2.z, q2.w);
+                if (SQ)   // r = sqrt(p) is what p0, p1 hold: dS = r (dP / 2 - r delta / 2), and r itself multiplies dO in dV
+                  unpack2(fmul2(p2, ffma2(p2, nd2, fmul2(dp2, pack2(0.5f, 0.5f)))), d0, d1);
+                else      // dS = p (dP - delta)
+                  unpack2(fmul2(p2, fadd2(dp2, nd2)), d0, d1);
+                pp[j / 2] = bwd_pack(p0, p1);
+                dd[j / 2] = bwd_pack(d0, d1);
+              }
+            };
+            if (__all_sync(0xffffffffu, keep == 0xffffu)) {
+              elements(std::false_type{});
+            } else if (__all_sync(0xffffffffu, keep == 0u)) {   // the other side of a chain boundary, or padding
 #pragma unroll
-          for (int j = 0; j < hD; ++j) lo[j] = hi[j] = 0.f;
-        }
-        // element offset of this thread's half row in dk / dv, negative when the key has no row (past T, or dropped token)
-        long long row_off = -1;
-        if (kj < p.T) {
-          row_off = static_cast<long long>(size_t(kj) * p.g_row + size_t(b) * p.g_b);
-          if (p.token_row != nullptr) {
-            const int tr = __ldg(p.token_row + size_t(kj) * p.B + b);
-            row_off = tr < 0 ? -1 : static_cast<long long>(size_t(tr) * p.g_b);
-          }
-          if (row_off >= 0) row_off += static_cast<long long>(size_t(bh % p.H) * p.g_h + half_col * hD);
-        }
-        float outv[hD];
-        if (is_dk) {
-          const bool rot = path == 0 && p.cos_tab != nullptr;
-          if (rot) {   // R^T: dx_lo = dy_lo c + dy_hi s, dx_hi = dy_hi c - dy_lo s; table rows read 16 bytes at a time
-            const float4* c4 = reinterpret_cast<const float4*>(p.cos_tab + size_t(krow) * hD);
-            const float4* s4 = reinterpret_cast<const float4*>(p.sin_tab + size_t(krow) * hD);
-#pragma unroll
-            for (int d = 0; d < hD; d += 4) {
-              const float4 cs = __ldg(c4 + d / 4), sn = __ldg(s4 + d / 4);
-              const float cv[4] = {cs.x, cs.y, cs.z, cs.w}, sv4[4] = {sn.x, sn.y, sn.z, sn.w};
-#pragma unroll
-              for (int e = 0; e < 4; ++e)
-                outv[d + e] = (half_col == 0 ? lo[d + e] * cv[e] + hi[d + e] * sv4[e] : hi[d + e] * cv[e] - lo[d + e] * sv4[e]) * p.scale;
+              for (int j = 0; j < 8; ++j) pp[j] = dd[j] = 0u;
+            } else {
+              elements(std::true_type{});
             }
-          } else {
-#pragma unroll
-            for (int d = 0; d < hD; ++d) outv[d] = (half_col == 0 ? lo[d] : hi[d]) * p.scale;
+            tmem_st8(tS, pp);         // P^T over the S^T columns this thread has read
+            tmem_st8(tS + 64, dd);    // dS^T likewise
+            // and dS into shared memory for the dQ product: 2 chunks of 8 queries in block `sub` of the dS tile
+            const uint32_t ds_at = ds_row ^ (v * 32);
+            smem_store16(ds_at, dd[0], dd[1], dd[2], dd[3]);
+            smem_store16(ds_at ^ 16u, dd[4], dd[5], dd[6], dd[7]);
           }
-        } else {
-#pragma unroll
-          for (int d = 0; d < hD; ++d) outv[d] = half_col == 0 ? lo[d] : hi[d];
+          tmem_st_wait();
+          fence_proxy_async_smem();
+          tc_fence_before();
+          mbar_arrive(&pds_full[br.pos]);
+          br.advance();
+          br.advance();
+          mask = mask_next;
+          ++g;
         }
-        __nv_bfloat16* base = is_dk ? p.dk[path] : p.dv[path];
-        if constexpr (kPieces == 1) {
-          if (row_off >= 0)
-            *reinterpret_cast<uint4*>(base + row_off) = make_uint4(bwd_pack(outv[0], outv[1]), bwd_pack(outv[2], outv[3]),
-                                                                   bwd_pack(outv[4], outv[5]), bwd_pack(outv[6], outv[7]));
-        } else {
-          // Rows of different keys lie far apart (row-major gradients) or 2 hD elements apart: staged per warp and read back
-          // so that kPieces neighbouring lanes write one row's contiguous 16 hD bytes, a store instruction covers whole runs.
-          constexpr int kRowB = hD * 2;   // 64 or 32 bytes
-#pragma unroll
-          for (int j = 0; j < hD; j += 8)
-            *reinterpret_cast<uint4*>(my_stage + swizzled_offset(lane, j / 8, kRowB)) =
-                make_uint4(bwd_pack(outv[j], outv[j + 1]), bwd_pack(outv[j + 2], outv[j + 3]), bwd_pack(outv[j + 4], outv[j + 5]),
-                           bwd_pack(outv[j + 6], outv[j + 7]));
+        // the tile before this one: of the same key tile, or the last one of the key tile before
+        if (it > 0) {
+          ok = drain_dq(plan, it - 1, g - 2);
+        } else if (m > 0) {
+          const BwdPlan& before = plans[(m - 1) % kPlans];
+          ok = finish_item(before, m - 1, n > 0 ? g - 2 : g - 1);
           __syncwarp();
-          const int piece = lane % kPieces;
-#pragma unroll
-          for (int i = 0; i < kPieces; ++i) {
-            const int r = i * (32 / kPieces) + lane / kPieces;
-            const long long ro = __shfl_sync(0xffffffffu, row_off, r);
-            const uint4 q = *reinterpret_cast<const uint4*>(my_stage + swizzled_offset(r, piece, kRowB));
-            if (ro >= 0) *reinterpret_cast<uint4*>(base + ro + piece * 8) = q;
-          }
-          __syncwarp();
+          if (lane == 0) mbar_arrive(&plan_empty[(m - 1) % kPlans]);
         }
       }
+      if (!ok || n == 0) break;
     }
+    if (lane == 0) bulk_wait_read_all();   // the reductions have read their staging rows (their additions may still be under way)
   }
   tc_fence_before();
   __syncthreads();
@@ -855,7 +920,9 @@ static int bwd_tc_t(const AttnArgs& a, const void* q_s, const void* k_s, const f
   p.skip_pad_queries = a.skip_pad_queries ? 1 : 0;
   p.g_row = grad_row_stride(a); p.g_b = grad_b_stride(a); p.g_h = grad_h_stride(a);
   p.token_row = a.token_row; p.B = a.B;
-  dim3 grid((a.T + kBwdTile - 1) / kBwdTile, BH, 2);
+  p.n_items = (a.T + kBwdTile - 1) / kBwdTile * BH * 2;
+  if (int rc = next_tile_counter(&p.sched); rc != MINTB_OK) return rc;
+  const dim3 grid(unsigned(p.n_items < sm_count() ? p.n_items : sm_count()));
   e = launch_dependent(attn_bwd_tc_kernel<D, SQ>, grid, dim3(Cfg::kThreads), Cfg::kSmemBytes, a.stream, mqs, mks, mvs, mqc, mkc, mvc, mdo, mdq_s, mdq_c, p);
   count_launches(1);
   if (e == cudaSuccess) e = cudaGetLastError();
