@@ -55,16 +55,17 @@ static bool bwd_make_map(CUtensorMap* m, const void* ptr, int D, int T, int BH, 
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// fp32 dQ accumulator [BH][T][D] as a reduction target: box = (D / 4 columns, 32 rows, 1), i.e. what one compute warp
-// drains from TMEM per query tile.
+// fp32 dQ accumulator [BH][T][D] as a reduction target: box = (up to 32 columns, 32 rows, 1), a warp's share of a query tile
+// or half of it.  The copy engine works off a box row by row: quarter rows of four warps made it, with 512 of them per tile,
+// slower than the products (2000 cycles of a tile's 2800).
 static bool bwd_make_dq_map(CUtensorMap* m, const void* ptr, int D, int T, int BH) {
   EncodeTiledFn fn = bwd_encode_fn();
   if (fn == nullptr) return false;
   cuuint64_t dims[3] = {cuuint64_t(D), cuuint64_t(T), cuuint64_t(BH)};
   cuuint64_t strides[2] = {cuuint64_t(D) * 4, cuuint64_t(T) * D * 4};
-  cuuint32_t box[3] = {cuuint32_t(D / 4), 32, 1};
+  cuuint32_t box[3] = {cuuint32_t(D < 32 ? D : 32), 32, 1};
   cuuint32_t es[3] = {1, 1, 1};
-  CUtensorMapSwizzle sw = D == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : D == 32 ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_NONE;
+  CUtensorMapSwizzle sw = D >= 32 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B;
   return fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void*>(ptr), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
             CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
@@ -213,25 +214,27 @@ struct BwdCfg {
   // (head_dim <= 32) buffers of {S^T half (64 columns), dP^T half (64 columns)}; the third buffer lets the products run
   // ahead of the compute warps.
   static constexpr int kCW = 16;                                // compute warps
-  static constexpr int kThreads = 128 + 32 * kCW;               // + three MMA issuers and the loading warp
+  static constexpr int kThreads = 256 + 32 * kCW;               // + three MMA issuers, the loading warp, four warps for the results
   static constexpr int kNBuf = D <= 32 ? 3 : 2;
   static constexpr int kNDq = 2;                                // dQ tiles in TMEM == dS tiles in shared memory
   static constexpr int kQStages = D <= 32 ? 4 : 2;              // stages of {Q_i, dO_i} (a power of two)
-  static constexpr int kKv = D <= 32 ? 2 : 1;                   // key tiles {K, V} in shared memory
+  static constexpr int kK = 2, kV = D <= 32 ? 2 : 1;            // key tiles in shared memory (V's is free a tile earlier than K's)
   static constexpr int kAcc = D <= 32 ? 32 : 64;                // columns reserved per accumulator
   static constexpr int kColDK = 0, kColDV = kAcc, kColDQ = 2 * kAcc, kColBuf = (2 + kNDq) * kAcc;
   static constexpr uint32_t kTmemCols = 512;
-  static constexpr int kDqWarpBytes = 32 * (D / 4) * 4;          // staging of one warp's dQ slice: 32 queries x D/4 fp32 columns
-  static constexpr int kDqStageBytes = kCW * kDqWarpBytes;
+  static constexpr int kDqCols = D < 32 ? D : 32;               // columns of one dQ box: 32 rows x kDqCols
+  static constexpr int kDqStages = D <= 32 ? 2 : 1;
+  static constexpr int kDqQuarterBytes = 32 * D * 4;            // staging of the 32 queries of one TMEM quarter
   static constexpr int kStatBytes = 128 * 8;                     // softmax statistics of one query tile: 128 x (-lse log2 e, -delta)
-  static constexpr size_t kSmemBytes = 1024 + size_t(kKv) * 2 * kTileBytes + size_t(kQStages) * 2 * kTileBytes + size_t(kNDq) * kDsBytes +
-                                       kDqStageBytes + kQStages * kStatBytes + 2560;
+  static constexpr size_t kSmemBytes = 1024 + size_t(kK + kV) * kTileBytes + size_t(kQStages) * 2 * kTileBytes + size_t(kNDq) * kDsBytes +
+                                       size_t(kDqStages) * 4 * kDqQuarterBytes + kQStages * kStatBytes + 3072;
 };
 
 // One work item - the dK, dV of a key tile in one pathway - as the loading warp hands it to the other roles.
 struct BwdPlan {
   int n;                           // query tiles with pairs of the pathway; 0: no more items
   int kt, bh, path;
+  uint32_t flip;                   // a query belongs to the pathway where mask bit XOR flip
   uint32_t kpad[4];                // padding bits of the tile's 128 keys
   uint16_t tiles[kBwdMaxTiles];    // their numbers, kMixed set where the tile needs the chain mask
 };
@@ -280,50 +283,54 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
                    const __grid_constant__ CUtensorMap map_do, const __grid_constant__ CUtensorMap map_dq_s,
                    const __grid_constant__ CUtensorMap map_dq_c, BwdParams p) {
   using Cfg = BwdCfg<D>;
-  constexpr int RB = Cfg::kRowBytes, kNBuf = Cfg::kNBuf, kQStages = Cfg::kQStages, kNDq = Cfg::kNDq, kKv = Cfg::kKv;
+  constexpr int RB = Cfg::kRowBytes, kNBuf = Cfg::kNBuf, kQStages = Cfg::kQStages, kNDq = Cfg::kNDq, kK = Cfg::kK, kV = Cfg::kV;
   constexpr int kColDK = Cfg::kColDK, kColDV = Cfg::kColDV, kColDQ = Cfg::kColDQ, kColBuf = Cfg::kColBuf, kAcc = Cfg::kAcc;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = align_smem_1024(smem_raw);
-  unsigned char* sKV = smem;                                         // [key tile][0: K, 1: V]
-  unsigned char* sQ = sKV + size_t(kKv) * 2 * Cfg::kTileBytes;       // [stage][0: Q_i, 1: dO_i]
+  unsigned char* sK = smem;                                          // [kK]
+  unsigned char* sV = sK + size_t(kK) * Cfg::kTileBytes;             // [kV]
+  unsigned char* sQ = sV + size_t(kV) * Cfg::kTileBytes;             // [stage][0: Q_i, 1: dO_i]
   unsigned char* sDS = sQ + size_t(kQStages) * 2 * Cfg::kTileBytes;  // [buf][half][128 rows x 128 B]
-  unsigned char* sDqStage = sDS + size_t(kNDq) * Cfg::kDsBytes;      // [compute warp][32 queries][D/4 fp32], swizzled
-  unsigned char* sStats = sDqStage + Cfg::kDqStageBytes;             // [stage][64] x (nl0, nl1, nd0, nd1), loaded with the query tile
+  unsigned char* sDqStage = sDS + size_t(kNDq) * Cfg::kDsBytes;      // [stage][quarter][column box][32 queries][kDqCols fp32], swizzled
+  unsigned char* sStats = sDqStage + size_t(Cfg::kDqStages) * 4 * Cfg::kDqQuarterBytes;   // [stage][64] x (nl0, nl1, nd0, nd1), loaded with the query tile
   unsigned char* tail = sStats + size_t(kQStages) * Cfg::kStatBytes;
   uint64_t* bars = reinterpret_cast<uint64_t*>(tail);
   uint64_t* plan_full = bars;           // [4]
   uint64_t* plan_empty = bars + 4;      // [4]
-  uint64_t* kv_full = bars + 8;         // [2]
-  uint64_t* kv_empty = bars + 10;       // [2]
-  uint64_t* q_full = bars + 12;         // [4] Q_i and dO_i
-  uint64_t* st_full = bars + 16;        // [4] the statistics
-  uint64_t* q_empty = bars + 20;        // [4]
-  uint64_t* sdp_full = bars + 24;       // [3 buffers]
-  uint64_t* pds_full = bars + 27;       // [3 buffers]
-  uint64_t* buf_free = bars + 30;       // [3 buffers]
-  uint64_t* dq_full = bars + 33;        // [2]
-  uint64_t* dq_empty = bars + 35;       // [2]
-  uint64_t* acc_full = bars + 37;
-  uint64_t* acc_empty = bars + 38;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 39);
-  BwdPlan* plans = reinterpret_cast<BwdPlan*>(bars + 40);            // [kPlans]
-  static_assert(40 * 8 + kPlans * sizeof(BwdPlan) <= 2560, "tail of the shared memory");
+  uint64_t* k_full = bars + 8;          // [2]
+  uint64_t* k_empty = bars + 10;        // [2]
+  uint64_t* v_full = bars + 12;         // [2]
+  uint64_t* v_empty = bars + 14;        // [2]
+  uint64_t* q_full = bars + 16;         // [4] Q_i and dO_i
+  uint64_t* st_full = bars + 20;        // [4] the statistics
+  uint64_t* q_empty = bars + 24;        // [4]
+  uint64_t* sdp_full = bars + 28;       // [3 buffers]
+  uint64_t* pds_full = bars + 31;       // [3 buffers]
+  uint64_t* buf_free = bars + 34;       // [3 buffers]
+  uint64_t* dq_full = bars + 37;        // [2]
+  uint64_t* dq_empty = bars + 39;       // [2]
+  uint64_t* acc_full = bars + 41;
+  uint64_t* acc_empty = bars + 42;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 43);
+  BwdPlan* plans = reinterpret_cast<BwdPlan*>(bars + 44);            // [kPlans]
+  static_assert(44 * 8 + kPlans * sizeof(BwdPlan) <= 3072, "tail of the shared memory");
 
   const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
   if (tid == 0) {
     for (int s = 0; s < 4; ++s) {
-      mbar_init(&plan_full[s], 1); mbar_init(&plan_empty[s], 3 + Cfg::kCW);   // three MMA issuers and every compute warp read a plan
+      mbar_init(&plan_full[s], 1); mbar_init(&plan_empty[s], 7 + Cfg::kCW);   // every warp but the loading one reads a plan
       mbar_init(&q_full[s], 1); mbar_init(&st_full[s], 1); mbar_init(&q_empty[s], 1);
     }
     for (int s = 0; s < 2; ++s) {
-      mbar_init(&kv_full[s], 1); mbar_init(&kv_empty[s], 2);                   // released by the S / dP and the dQ stream
-      mbar_init(&dq_full[s], 1); mbar_init(&dq_empty[s], 32 * Cfg::kCW);
+      mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 2);                     // released by the S / dP and the dQ stream
+      mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 1);
+      mbar_init(&dq_full[s], 1); mbar_init(&dq_empty[s], 4);                   // four warps drain a tile
     }
     for (int s = 0; s < 3; ++s) {
       mbar_init(&sdp_full[s], 1); mbar_init(&pds_full[s], 32 * Cfg::kCW / 2);
       mbar_init(&buf_free[s], 2);                                // dV and dK of a half have read P^T, dS^T; the dQ stream has seen it
     }
-    mbar_init(acc_full, 1); mbar_init(acc_empty, Cfg::kCW);
+    mbar_init(acc_full, 1); mbar_init(acc_empty, 4);
     fence_mbar_init();
   }
   if (warp == 1) { tmem_alloc(tmem_slot, Cfg::kTmemCols); tmem_relinquish(); }
@@ -350,7 +357,8 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
     // ---------------------------------------------------------------- plans and TMA loads
     const int nqt = (p.T + kBwdTile - 1) / kBwdTile, nkt = nqt;
     Ring<kPlans> pr;
-    Ring<kKv> kr;
+    Ring<kK> kr;
+    Ring<kV> vr;
     Ring<kQStages> lr;
     bool ok = true;
     for (int n = 0; ok; ++n) {
@@ -405,7 +413,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
         continue;
       }
       if (lane == 0) {
-        plan.n = n_act; plan.kt = kt; plan.bh = bh; plan.path = path;
+        plan.n = n_act; plan.kt = kt; plan.bh = bh; plan.path = path; plan.flip = path == 0 ? 0xffffffffu : 0u;
         plan.kpad[0] = kw.x; plan.kpad[1] = kw.y; plan.kpad[2] = kw.z; plan.kpad[3] = kw.w;
       }
       __syncwarp();
@@ -414,12 +422,15 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
         const CUtensorMap* mq = path == 0 ? &map_qs : &map_qc;
         const CUtensorMap* mk = path == 0 ? &map_ks : &map_kc;
         const CUtensorMap* mv = path == 0 ? &map_vs : &map_vc;
-        ok = mbar_wait(&kv_empty[kr.pos], kr.phase ^ 1, p.status, 0x521);
+        ok = mbar_wait(&k_empty[kr.pos], kr.phase ^ 1, p.status, 0x521);
         if (ok) {
-          unsigned char* kv = sKV + size_t(kr.pos) * 2 * Cfg::kTileBytes;
-          mbar_expect_tx(&kv_full[kr.pos], 2 * Cfg::kTileBytes);
-          tma_load_3d(kv, mk, &kv_full[kr.pos], 0, k0, bh);
-          tma_load_3d(kv + Cfg::kTileBytes, mv, &kv_full[kr.pos], 0, k0, bh);
+          mbar_expect_tx(&k_full[kr.pos], Cfg::kTileBytes);
+          tma_load_3d(sK + size_t(kr.pos) * Cfg::kTileBytes, mk, &k_full[kr.pos], 0, k0, bh);
+          ok = mbar_wait(&v_empty[vr.pos], vr.phase ^ 1, p.status, 0x523);
+        }
+        if (ok) {
+          mbar_expect_tx(&v_full[vr.pos], Cfg::kTileBytes);
+          tma_load_3d(sV + size_t(vr.pos) * Cfg::kTileBytes, mv, &v_full[vr.pos], 0, k0, bh);
         }
         for (int t = 0; t < n_act && ok; ++t) {
           const int i = plan.tiles[t] & (kMixed - 1);
@@ -440,6 +451,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
       ok = __shfl_sync(0xffffffffu, int(ok), 0) != 0;
       pr.advance();
       kr.advance();
+      vr.advance();
     }
     if (ok) ok = wait_all(&plan_empty[pr.pos], pr.phase ^ 1, 0x526);
     if (ok && lane == 0) {
@@ -456,12 +468,13 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
     constexpr uint32_t idesc_s = idesc_bf16(kBwdTile, kHalf, false, false);   // M = 128 keys, N = 64 queries
     constexpr uint32_t kHi = desc_hi32(8 * RB, swizzle_for_row_bytes(RB));
     constexpr uint32_t kLbo = desc_lbo32(16);
-    const uint32_t k_lo0 = desc_addr32(__shfl_sync(0xffffffffu, smem_u32(sKV), 0)) + kLbo;
+    const uint32_t k_lo0 = desc_addr32(__shfl_sync(0xffffffffu, smem_u32(sK), 0)) + kLbo, v_lo0 = desc_addr32(__shfl_sync(0xffffffffu, smem_u32(sV), 0)) + kLbo;
     const uint32_t q_lo = desc_addr32(__shfl_sync(0xffffffffu, smem_u32(sQ), 0)) + kLbo;
     constexpr uint32_t kTileU = Cfg::kTileBytes >> 4, kHalfU = (kHalf * RB) >> 4;
     bool ok = true;
     Ring<kPlans> pr;
-    Ring<kKv> kr;
+    Ring<kK> kr;
+    Ring<kV> vr;
     Ring<kQStages> qr;     // query tile of the half being issued
     Ring<kNBuf> ib;        // its buffer
     for (;;) {
@@ -469,8 +482,8 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
       if (!ok) break;
       const int n = __shfl_sync(0xffffffffu, plans[pr.pos].n, 0);
       if (n == 0) break;
-      ok = wait_all(&kv_full[kr.pos], kr.phase, 0x502);
-      const uint32_t k_lo = k_lo0 + kr.pos * 2 * kTileU, v_lo = k_lo + kTileU;
+      ok = wait_all(&k_full[kr.pos], kr.phase, 0x502);
+      const uint32_t k_lo = k_lo0 + kr.pos * kTileU, v_lo = v_lo0 + vr.pos * kTileU;
       for (int u = 0; u < 2 * n && ok; ++u) {
         const int h = u & 1;
         ok = wait_all(&buf_free[ib.pos], ib.phase ^ 1, 0x505);
@@ -483,6 +496,11 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
         if (leader) {
 #pragma unroll
           for (int k = 0; k < D / 16; ++k) umma_ss(col, make_desc(kHi, k_lo + 2 * k), make_desc(kHi, qs + 2 * k), idesc_s, k > 0);
+        }
+        __syncwarp();
+        if (u == 0) ok = wait_all(&v_full[vr.pos], vr.phase, 0x504);
+        if (!ok) break;
+        if (leader) {
 #pragma unroll
           for (int k = 0; k < D / 16; ++k) umma_ss(col + 64, make_desc(kHi, v_lo + 2 * k), make_desc(kHi, dos + 2 * k), idesc_s, k > 0);
           umma_commit(&sdp_full[ib.pos]);
@@ -493,12 +511,14 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
       }
       if (!ok) break;
       if (leader) {
-        umma_commit(&kv_empty[kr.pos]);
+        umma_commit(&k_empty[kr.pos]);
+        umma_commit(&v_empty[vr.pos]);
         mbar_arrive(&plan_empty[pr.pos]);
       }
       __syncwarp();
       pr.advance();
       kr.advance();
+      vr.advance();
     }
   } else if (warp == 2) {
     // ---------------------------------------------------------------- MMA stream B: dV += P^T dO, dK += dS^T Q
@@ -528,10 +548,11 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
           const uint32_t pt = tbase_u + kColBuf + br.pos * 128, ds = pt + 64;   // P^T lies over S^T, dS^T over dP^T
           if (leader) {
 #pragma unroll
-            for (int k = 0; k < kHalf / 16; ++k) {
+            for (int k = 0; k < kHalf / 16; ++k)
               umma_ts(tbase_u + kColDV, pt + k * 16, make_desc(kHi, d_o + k * kStep), idesc_acc, it > 0 || h > 0 || k > 0);
+#pragma unroll
+            for (int k = 0; k < kHalf / 16; ++k)
               umma_ts(tbase_u + kColDK, ds + k * 16, make_desc(kHi, q + k * kStep), idesc_acc, it > 0 || h > 0 || k > 0);
-            }
             umma_commit(&buf_free[br.pos]);
           }
           __syncwarp();
@@ -556,11 +577,11 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
     constexpr uint32_t idesc_dq = idesc_bf16(kBwdTile, D, true, true);        // A = dS (queries contiguous), B = K (D contiguous)
     constexpr uint32_t kHiA = desc_hi32(8 * 128, kSw128), kHiB = desc_hi32(8 * RB, swizzle_for_row_bytes(RB));
     const uint32_t ds_lo = desc_addr32(__shfl_sync(0xffffffffu, smem_u32(sDS), 0)) + desc_lbo32(Cfg::kDsBlock);
-    const uint32_t kb_lo0 = desc_addr32(__shfl_sync(0xffffffffu, smem_u32(sKV), 0)) + desc_lbo32(8 * RB);
+    const uint32_t kb_lo0 = desc_addr32(__shfl_sync(0xffffffffu, smem_u32(sK), 0)) + desc_lbo32(8 * RB);
     constexpr uint32_t kDsU = Cfg::kDsBytes >> 4, kAStep = (16 * 128) >> 4, kBStep = (16 * RB) >> 4, kTileU = Cfg::kTileBytes >> 4;
     bool ok = true;
     Ring<kPlans> pr;
-    Ring<kKv> kr;
+    Ring<kK> kr;
     Ring<kNBuf> br;        // buffers of the two halves of the tile
     Ring<kNDq> dr;
     for (;;) {
@@ -568,8 +589,8 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
       if (!ok) break;
       const int n = __shfl_sync(0xffffffffu, plans[pr.pos].n, 0);
       if (n == 0) break;
-      ok = wait_all(&kv_full[kr.pos], kr.phase, 0x528);
-      const uint32_t kb_lo = kb_lo0 + kr.pos * 2 * kTileU;
+      ok = wait_all(&k_full[kr.pos], kr.phase, 0x528);
+      const uint32_t kb_lo = kb_lo0 + kr.pos * kTileU;
       for (int it = 0; it < n && ok; ++it) {
         for (int h = 0; h < 2 && ok; ++h) {
           ok = wait_all(&pds_full[br.pos], br.phase, 0x522);
@@ -592,88 +613,78 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
       }
       if (!ok) break;
       if (leader) {
-        umma_commit(&kv_empty[kr.pos]);
+        umma_commit(&k_empty[kr.pos]);
         mbar_arrive(&plan_empty[pr.pos]);
       }
       __syncwarp();
       pr.advance();
       kr.advance();
     }
-  } else {
-    // ---------------------------------------------------------------- compute warps (lane = key row)
-    // 8 warps work on each of the two 64-query halves of a tile: thread = key row x 32 query columns, so that the chain from
-    // the wait to the arrival is paid once per 32 exponentials and the two sets of warps fill each other's waits (16 warps on
-    // one half after the other, 16 columns each: 249 -> 228 us at B8 H20 T1024 D32).  Everything is elementwise: no exchange
-    // between threads.
-    constexpr int hD = D / 2, NC = D / 4;
-    const int cwp = warp - 4;                     // 0..15
-    const int grp = cwp / 4;                      // pair (half, 32 columns of it); also the warp's share of dQ and of the gradients
-    const int sub = grp / 2, c32 = grp & 1;
+  } else if (warp < 8) {
+    // ---------------------------------------------------------------- results: dQ per query tile, dK and dV per key tile
+    // Four warps, one per TMEM quarter, so that the compute warps go from one half to the next: a tile's dQ costs whoever fetches
+    // it 1300 cycles, a key tile's gradients 1500 to 3000.
+    constexpr int hD = D / 2, kC = Cfg::kDqCols, kCh = hD < 16 ? hD : 16;
     const int quarter = warp % 4;
-    const int r = quarter * 32 + lane;            // key row in the tile == TMEM lane
-    const uint32_t lane_base = uint32_t(quarter * 32) << 16;
-    const uint32_t tBuf = tbase + lane_base + kColBuf + 32 * c32;   // + 128 * buffer: S^T columns of this thread; dP^T 64 further
-    const uint32_t ds_addr = smem_u32(sDS) + uint32_t(sub) * Cfg::kDsBlock + swizzled_offset(r, 4 * c32, 128);
-    const uint64_t c22 = pack2(p.scale_log2, p.scale_log2);
-    unsigned char* my_stage = sDqStage + size_t(cwp) * Cfg::kDqWarpBytes;
+    const int r = quarter * 32 + lane;            // query of a dQ tile, key of dK / dV
+    const uint32_t tq = tbase + (uint32_t(quarter * 32) << 16);
     bool ok = true;
-    Ring<kNBuf> br;        // buffer of this warp's half: every other one
-    if (sub == 1) br.advance();
-    // The other rings follow from two counts (registers are what this loop is short of, so it also reads the plans' fields again
-    // rather than keep them): query tiles handed to the tensor cores so far, and key tiles.
-    uint32_t g = 0, m = 0;
+    uint32_t t = 0, m = 0;                        // query tiles and key tiles so far
 
-    // dQ of a tile leaves through shared memory: each compute warp stages its 32 queries x NC columns and one lane adds
-    // them to the fp32 accumulator in HBM with ONE bulk reduction (instead of a 16-byte atomic per thread and 4 columns).
-    auto drain_dq = [&](const BwdPlan& plan, int it, uint32_t g) -> bool {   // add dQ of the plan's tile `it`, number g of all, to HBM
-      const uint32_t xb = g % kNDq;
-      if (!wait_all(&dq_full[xb], (g / kNDq) & 1u, 0x601)) return false;
+    // A tile's dQ goes through shared memory: a quarter's 32 queries are staged and one lane adds them to the fp32 accumulator in HBM
+    // with a bulk reduction of whole rows.
+    auto drain_dq = [&](const BwdPlan& plan, int it) -> bool {
+      const uint32_t xb = t % kNDq;
+      if (!wait_all(&dq_full[xb], (t / kNDq) & 1u, 0x601)) return false;
       tc_fence_after();
-      constexpr int kRowB = NC * 4;      // bytes per staged row: 64, 32 or 16
-      uint32_t v[NC];
-      tmem_ld_n<NC>(tbase + lane_base + kColDQ + xb * kAcc + grp * NC, v);
-      if (lane == 0) bulk_wait_read_all();   // the previous reduction of this warp has read the staging rows
-      __syncwarp();
-      tmem_ld_wait();
-      tc_fence_before();
-      mbar_arrive(&dq_empty[xb]);
-#pragma unroll
-      for (int e = 0; e < NC; e += 4) {
-        const uint32_t off = kRowB == 16 ? uint32_t(lane) * 16u : swizzled_offset(lane, e / 4, kRowB);
-        *reinterpret_cast<uint4*>(my_stage + off) = make_uint4(v[e], v[e + 1], v[e + 2], v[e + 3]);
+      unsigned char* stage = sDqStage + (4 * (t % Cfg::kDqStages) + quarter) * Cfg::kDqQuarterBytes;
+      if (lane == 0) {   // the reduction that used these rows last has read them
+        if (Cfg::kDqStages == 2) bulk_wait_read_but_one(); else bulk_wait_read_all();
       }
+      __syncwarp();
+#pragma unroll
+      for (int c = 0; c < D; c += kC) {
+        uint32_t v[kC];
+        tmem_ld_n<kC>(tq + kColDQ + xb * kAcc + c, v);
+        tmem_ld_wait();
+#pragma unroll
+        for (int e = 0; e < kC; e += 4)
+          *reinterpret_cast<uint4*>(stage + c * 128 + swizzled_offset(lane, e / 4, kC * 4)) = make_uint4(v[e], v[e + 1], v[e + 2], v[e + 3]);
+      }
+      tc_fence_before();
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) {
+        mbar_arrive(&dq_empty[xb]);
         const int row = (plan.tiles[it] & (kMixed - 1)) * kBwdTile + quarter * 32;
         if (row < p.T) {   // rows past T inside the box are dropped by the copy engine
-          tma_reduce_add_3d(plan.path == 0 ? &map_dq_s : &map_dq_c, my_stage, grp * NC, row, plan.bh);
-          bulk_commit_group();
+#pragma unroll
+          for (int c = 0; c < D; c += kC) tma_reduce_add_3d(plan.path == 0 ? &map_dq_s : &map_dq_c, stage + c * 128, c, row, plan.bh);
         }
+        bulk_commit_group();
       }
+      ++t;
       return true;
     };
 
-    // What is left of a key tile: the last dQ tile, then dK (scaled, un-rotated for the self pathway) and dV.  Groups 0, 1 take dK:
-    // the columns [NC half, + NC) and the ones the rotation pairs them with, hD further; groups 2, 3 half of dV's columns each.
-    // The rotation's table rows are read with whole rows per group of lanes and turned in shared memory: a row per lane took one
-    // 128-byte line per lane and instruction, 7000 cycles of a key tile at head_dim 64 against 2300 without rotation.
-    auto finish_item = [&](const BwdPlan& plan, uint32_t m, uint32_t g) -> bool {   // plan number m, whose last tile is number g
-      const int k0 = plan.kt * kBwdTile, kj = k0 + r, bh = plan.bh, b = bh / p.H, path = plan.path;
-      const bool is_dk = grp < 2;
-      const int half = grp & 1;
-      const bool rot = is_dk && path == 0 && p.cos_tab != nullptr;
-      constexpr int kLpr = NC / 4;   // lanes per table row: 4, 2 or 1
-      float4 tc[kLpr], ts[kLpr];
-      if (rot) {
+    // dK (scaled, un-rotated for the self pathway) and dV of a key tile; the accumulators are given back as soon as they are in
+    // registers.
+    auto store8 = [](__nv_bfloat16* dst, const float (&x)[kCh], int j) {
+      *reinterpret_cast<uint4*>(dst) = make_uint4(bwd_pack(x[j], x[j + 1]), bwd_pack(x[j + 2], x[j + 3]), bwd_pack(x[j + 4], x[j + 5]), bwd_pack(x[j + 6], x[j + 7]));
+    };
+    auto finish_item = [&](const BwdPlan& plan) -> bool {
+      const int kj = plan.kt * kBwdTile + r, bh = plan.bh, b = bh / p.H, path = plan.path;
+      const bool rot = path == 0 && p.cos_tab != nullptr;
+      const size_t tab = size_t(kj < p.T ? kj : p.T - 1) * hD;
+      float4 tc[kCh / 4], ts[kCh / 4];
+      auto load_tables = [&](int d0) {
 #pragma unroll
-        for (int i = 0; i < kLpr; ++i) {
-          const int row = k0 + quarter * 32 + i * (32 / kLpr) + lane / kLpr;
-          const size_t at = size_t(row < p.T ? row : p.T - 1) * hD + half * NC + (lane % kLpr) * 4;
-          tc[i] = __ldg(reinterpret_cast<const float4*>(p.cos_tab + at));
-          ts[i] = __ldg(reinterpret_cast<const float4*>(p.sin_tab + at));
+        for (int i = 0; i < kCh / 4; ++i) {
+          tc[i] = __ldg(reinterpret_cast<const float4*>(p.cos_tab + tab + d0) + i);
+          ts[i] = __ldg(reinterpret_cast<const float4*>(p.sin_tab + tab + d0) + i);
         }
-      }
+      };
+      if (rot) load_tables(0);
       // element offset of this thread's row in dk / dv, negative when the key has no row (past T, or dropped token)
       long long row_off = -1;
       if (kj < p.T) {
@@ -684,111 +695,113 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
         }
         if (row_off >= 0) row_off += static_cast<long long>(size_t(bh % p.H) * p.g_h);
       }
-      if (!drain_dq(plan, plan.n - 1, g)) return false;
-      if (lane == 0) bulk_wait_read_all();   // the staging rows of the dQ reduction are reused below
-      __syncwarp();
-      if (rot) {
-        auto turn = [&](float4 (&x)[kLpr]) {   // this lane's row of the 32 that the warp has loaded
-          if constexpr (kLpr > 1) {
-#pragma unroll
-            for (int i = 0; i < kLpr; ++i)
-              *reinterpret_cast<float4*>(my_stage + swizzled_offset(i * (32 / kLpr) + lane / kLpr, lane % kLpr, NC * 4)) = x[i];
-            __syncwarp();
-#pragma unroll
-            for (int i = 0; i < kLpr; ++i) x[i] = *reinterpret_cast<const float4*>(my_stage + swizzled_offset(lane, i, NC * 4));
-            __syncwarp();
-          }
-        };
-        turn(tc);
-        turn(ts);
-      }
+      __nv_bfloat16* dk = p.dk[path] + row_off;
+      __nv_bfloat16* dv = p.dv[path] + row_off;
       if (!wait_all(acc_full, m & 1u, 0x603)) return false;
       tc_fence_after();
-      const int col0 = is_dk ? half * NC : half * hD, col1 = is_dk ? hD + half * NC : half * hD + NC;
-      uint32_t t0[NC], t1[NC];
-      {
-        const uint32_t src = tbase + lane_base + (is_dk ? kColDK : kColDV);
-        tmem_ld_n<NC>(src + col0, t0);
-        tmem_ld_n<NC>(src + col1, t1);
+#pragma unroll
+      for (int d0 = 0; d0 < hD; d0 += kCh) {   // a range of columns and the one that the rotation pairs it with
+        uint32_t t0[kCh], t1[kCh];
+        float o0[kCh], o1[kCh];
+        tmem_ld_n<kCh>(tq + kColDV + d0, t0);
+        tmem_ld_n<kCh>(tq + kColDV + hD + d0, t1);
         tmem_ld_wait();
-      }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(acc_empty);
-      float o0[NC], o1[NC];
-      const float mul = is_dk ? p.scale : 1.f;
-      if (rot) {   // R^T: dx_lo = dy_lo c + dy_hi s, dx_hi = dy_hi c - dy_lo s
 #pragma unroll
-        for (int i = 0; i < kLpr; ++i) {
-          const float cv[4] = {tc[i].x, tc[i].y, tc[i].z, tc[i].w}, sv[4] = {ts[i].x, ts[i].y, ts[i].z, ts[i].w};
+        for (int d = 0; d < kCh; ++d) { o0[d] = __uint_as_float(t0[d]); o1[d] = __uint_as_float(t1[d]); }
+        if (row_off >= 0) {
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const float lo = __uint_as_float(t0[4 * i + e]), hi = __uint_as_float(t1[4 * i + e]);
-            o0[4 * i + e] = (lo * cv[e] + hi * sv[e]) * mul;
-            o1[4 * i + e] = (hi * cv[e] - lo * sv[e]) * mul;
+          for (int j = 0; j < kCh; j += 8) { store8(dv + d0 + j, o0, j); store8(dv + hD + d0 + j, o1, j); }
+        }
+        tmem_ld_n<kCh>(tq + kColDK + d0, t0);
+        tmem_ld_n<kCh>(tq + kColDK + hD + d0, t1);
+        tmem_ld_wait();
+        if (d0 + kCh == hD) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(acc_empty);
+        }
+        if (rot) {   // R^T: dx_lo = dy_lo c + dy_hi s, dx_hi = dy_hi c - dy_lo s
+#pragma unroll
+          for (int i = 0; i < kCh / 4; ++i) {
+            const float cv[4] = {tc[i].x, tc[i].y, tc[i].z, tc[i].w}, sv[4] = {ts[i].x, ts[i].y, ts[i].z, ts[i].w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const float lo = __uint_as_float(t0[4 * i + e]), hi = __uint_as_float(t1[4 * i + e]);
+              o0[4 * i + e] = (lo * cv[e] + hi * sv[e]) * p.scale;
+              o1[4 * i + e] = (hi * cv[e] - lo * sv[e]) * p.scale;
+            }
+          }
+          if (d0 + kCh < hD) load_tables(d0 + kCh);
+        } else {
+#pragma unroll
+          for (int d = 0; d < kCh; ++d) {
+            o0[d] = __uint_as_float(t0[d]) * p.scale;
+            o1[d] = __uint_as_float(t1[d]) * p.scale;
           }
         }
-      } else {
-#pragma unroll
-        for (int d = 0; d < NC; ++d) {
-          o0[d] = __uint_as_float(t0[d]) * mul;
-          o1[d] = __uint_as_float(t1[d]) * mul;
-        }
-      }
-      __nv_bfloat16* base = is_dk ? p.dk[path] : p.dv[path];
-      if constexpr (NC == 4) {
         if (row_off >= 0) {
-          *reinterpret_cast<uint2*>(base + row_off + col0) = make_uint2(bwd_pack(o0[0], o0[1]), bwd_pack(o0[2], o0[3]));
-          *reinterpret_cast<uint2*>(base + row_off + col1) = make_uint2(bwd_pack(o1[0], o1[1]), bwd_pack(o1[2], o1[3]));
-        }
-      } else {
-        // Rows of different keys lie far apart (row-major gradients) or 2 D elements apart: staged per warp and read back so
-        // that the neighbouring lanes that write one row's pieces cover whole runs of it.
-        constexpr int kPieces = hD / 8, kRowB = hD * 2;   // 16-byte pieces of a row, 4 or 2: half of them from each column range
 #pragma unroll
-        for (int j = 0; j < NC; j += 8) {
-          *reinterpret_cast<uint4*>(my_stage + swizzled_offset(lane, j / 8, kRowB)) =
-              make_uint4(bwd_pack(o0[j], o0[j + 1]), bwd_pack(o0[j + 2], o0[j + 3]), bwd_pack(o0[j + 4], o0[j + 5]), bwd_pack(o0[j + 6], o0[j + 7]));
-          *reinterpret_cast<uint4*>(my_stage + swizzled_offset(lane, (NC + j) / 8, kRowB)) =
-              make_uint4(bwd_pack(o1[j], o1[j + 1]), bwd_pack(o1[j + 2], o1[j + 3]), bwd_pack(o1[j + 4], o1[j + 5]), bwd_pack(o1[j + 6], o1[j + 7]));
+          for (int j = 0; j < kCh; j += 8) { store8(dk + d0 + j, o0, j); store8(dk + hD + d0 + j, o1, j); }
         }
-        __syncwarp();
-        const int piece = lane % kPieces;
-        const int col = piece < kPieces / 2 ? col0 + piece * 8 : col1 + (piece - kPieces / 2) * 8;
-#pragma unroll
-        for (int i = 0; i < kPieces; ++i) {
-          const int row = i * (32 / kPieces) + lane / kPieces;
-          const long long ro = __shfl_sync(0xffffffffu, row_off, row);
-          const uint4 q = *reinterpret_cast<const uint4*>(my_stage + swizzled_offset(row, piece, kRowB));
-          if (ro >= 0) *reinterpret_cast<uint4*>(base + ro + col) = q;
-        }
-        __syncwarp();
       }
       return true;
     };
 
     for (;; ++m) {
+      ok = wait_all(&plan_full[m % kPlans], (m / kPlans) & 1u, 0x607);
+      if (!ok) break;
+      const BwdPlan& plan = plans[m % kPlans];
+      const int n = plan.n;
+      if (n == 0) break;
+      for (int it = 0; it < n && ok; ++it) {
+        if (it == n - 1) ok = finish_item(plan);   // (the next key tile's products wait for the accumulators)
+        if (ok) ok = drain_dq(plan, it);
+      }
+      if (!ok) break;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&plan_empty[m % kPlans]);
+    }
+    if (lane == 0) bulk_wait_read_all();   // the reductions have read their staging rows (their additions may still be under way)
+  } else {
+    // ---------------------------------------------------------------- compute warps (lane = key row)
+    // 8 warps work on each of the two 64-query halves of a tile: thread = key row x 32 query columns, so that the chain from
+    // the wait to the arrival is paid once per 32 exponentials and the two sets of warps fill each other's waits (16 warps on
+    // one half after the other, 16 columns each: 249 -> 228 us at B8 H20 T1024 D32).  Everything is elementwise: no exchange
+    // between threads.
+    const int grp = (warp - 8) / 4;               // pair (half, 32 columns of it)
+    const int sub = grp / 2, c32 = grp & 1;
+    const int quarter = warp % 4;
+    const int r = quarter * 32 + lane;            // key row in the tile == TMEM lane
+    const uint32_t tBuf = tbase + (uint32_t(quarter * 32) << 16) + kColBuf + 32 * c32;   // + 128 * buffer: S^T columns of this thread; dP^T 64 further
+    const uint32_t ds_addr = smem_u32(sDS) + uint32_t(sub) * Cfg::kDsBlock + swizzled_offset(r, 4 * c32, 128);
+    const uint64_t c22 = pack2(p.scale_log2, p.scale_log2);
+    bool ok = true;
+    Ring<kNBuf> br;        // buffer of this warp's half: every other one
+    if (sub == 1) br.advance();
+    uint32_t g = 0, m = 0;                        // query tiles and key tiles so far
+    for (;; ++m) {
       ok = wait_all(&plan_full[m % kPlans], (m / kPlans) & 1u, 0x600);
       if (!ok) break;
       const BwdPlan& plan = plans[m % kPlans];
       const int n = plan.n;
-      // Which of the thread's 32 queries of tile `it` its key belongs to; asked for one tile ahead, so that a mixed tile does
-      // not wait for its mask words.
-      auto tile_mask = [&](int it) -> uint32_t {
+      if (n == 0) break;
+      const int kj = plan.kt * kBwdTile + r;
+      const uint32_t key_valid = kj < p.T && !((plan.kpad[quarter] >> lane) & 1u) ? 0xffffffffu : 0u;
+      // Mask word of the thread's 32 queries of tile `it`; asked for one tile ahead and not touched before it is needed, so that a
+      // mixed tile does not wait for it.
+      auto tile_bits = [&](int it) -> uint32_t {
         const uint32_t e = plan.tiles[it];
-        if (plan.kt * kBwdTile + r >= p.T || ((plan.kpad[quarter] >> lane) & 1u)) return 0u;
-        if (!(e & kMixed)) return 0xffffffffu;
-        const uint32_t bits = __ldg(p.bitsT + (size_t(plan.bh / p.H) * p.T + plan.kt * kBwdTile + r) * p.TW + 4 * (e & (kMixed - 1)) + grp);
-        return plan.path == 0 ? ~bits : bits;
+        return e & kMixed ? __ldg(p.bitsT + (size_t(plan.bh / p.H) * p.T + (kj < p.T ? kj : p.T - 1)) * p.TW + 4 * (e & (kMixed - 1)) + grp) : ~plan.flip;
       };
-      uint32_t mask = n > 0 ? tile_mask(0) : 0u;
-      // (one more round without a tile after the last key tile: its gradients leave there)
-      for (int it = 0; it < (n > 0 ? n : 1) && ok; ++it) {
-        if (n > 0) {
-          const uint32_t mask_next = it + 1 < n ? tile_mask(it + 1) : 0u;
+      uint32_t bits = tile_bits(0);
+      for (int it = 0; it < n && ok; ++it) {
+        {
+          const uint32_t bits_next = it + 1 < n ? tile_bits(it + 1) : 0u;
           ok = wait_all(&st_full[g % kQStages], (g / kQStages) & 1u, 0x604);
           if (ok) ok = wait_all(&sdp_full[br.pos], br.phase, 0x602);
+          if (ok) ok = wait_all(&dq_full[g % kNDq], ((g / kNDq) & 1u) ^ 1u, 0x606);   // the dS tile has been read (by the product of two tiles ago)
           if (!ok) break;
+          const uint32_t mask = (bits ^ plan.flip) & key_valid;
           tc_fence_after();
           const uint32_t ds_row = ds_addr + (g % kNDq) * Cfg::kDsBytes;
 #pragma unroll
@@ -847,22 +860,14 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
           mbar_arrive(&pds_full[br.pos]);
           br.advance();
           br.advance();
-          mask = mask_next;
+          bits = bits_next;
           ++g;
         }
-        // the tile before this one: of the same key tile, or the last one of the key tile before
-        if (it > 0) {
-          ok = drain_dq(plan, it - 1, g - 2);
-        } else if (m > 0) {
-          const BwdPlan& before = plans[(m - 1) % kPlans];
-          ok = finish_item(before, m - 1, n > 0 ? g - 2 : g - 1);
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&plan_empty[(m - 1) % kPlans]);
-        }
       }
-      if (!ok || n == 0) break;
+      if (!ok) break;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&plan_empty[m % kPlans]);
     }
-    if (lane == 0) bulk_wait_read_all();   // the reductions have read their staging rows (their additions may still be under way)
   }
   tc_fence_before();
   __syncthreads();
