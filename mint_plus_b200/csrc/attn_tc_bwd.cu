@@ -239,7 +239,7 @@ struct BwdPlan {
   uint16_t tiles[kBwdMaxTiles];    // their numbers, kMixed set where the tile needs the chain mask
 };
 constexpr uint16_t kMixed = 0x8000;
-constexpr int kPlans = 4;          // the one being computed, the one whose gradients have yet to leave, and two ahead
+constexpr int kPlans = 2;          // the one being computed and the next
 
 struct BwdParams {
   const uint32_t *bitsT, *kpad;
@@ -362,6 +362,10 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
     Ring<kQStages> lr;
     bool ok = true;
     for (int n = 0; ok; ++n) {
+      // An item is drawn when the one before the current one is done: drawn earlier, the items a CTA holds back at the end of the grid
+      // keep it busy while others have nothing left.
+      ok = wait_all(&plan_empty[pr.pos], pr.phase ^ 1, 0x520);
+      if (!ok) break;
       int item = 0;
       if (lane == 0) item = n == 0 ? int(blockIdx.x) : int(gridDim.x) + atomicAdd(p.sched, 1);
       item = __shfl_sync(0xffffffffu, item, 0);
@@ -370,29 +374,30 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
       const int k0 = kt * kBwdTile;
       const uint8_t want = path == 0 ? kHasIntra : kHasInter;
       const uint4 kw = *reinterpret_cast<const uint4*>(p.kpad + size_t(b) * p.TW + 4 * kt);
-      ok = wait_all(&plan_empty[pr.pos], pr.phase ^ 1, 0x520);
-      if (!ok) break;
+      // the classes of the first 32 query tiles are on their way together with the padding words
+      auto tile_class = [&](int i) -> uint32_t {
+        uint32_t c = 0;
+        if (i < nqt) {
+#pragma unroll
+          for (int a = 0; a < 2; ++a)
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+              if (2 * i + a < p.NT && 2 * kt + e < p.NT) c |= p.cls[(size_t(b) * p.NT + 2 * i + a) * p.NT + 2 * kt + e];
+          if (p.skip_pad_queries) {   // the padding bits describe positions: words 4 i .. 4 i + 3 cover the queries of tile i
+            const uint4 w = *reinterpret_cast<const uint4*>(p.kpad + size_t(b) * p.TW + 4 * i);
+            if ((w.x & w.y & w.z & w.w) == 0xffffffffu) c = 0;
+          }
+        }
+        return c;
+      };
+      uint32_t c = tile_class(lane);
       BwdPlan& plan = plans[pr.pos];
       int n_act = 0;
       if ((kw.x & kw.y & kw.z & kw.w) != 0xffffffffu)   // (every key of the tile padded: padded batches have many such tiles)
         for (int i0 = 0; i0 < nqt; i0 += 32) {
-          const int i = i0 + lane;
-          uint8_t c = 0;
-          bool pad = false;
-          if (i < nqt) {
-#pragma unroll
-            for (int a = 0; a < 2; ++a)
-#pragma unroll
-              for (int e = 0; e < 2; ++e)
-                if (2 * i + a < p.NT && 2 * kt + e < p.NT) c |= p.cls[(size_t(b) * p.NT + 2 * i + a) * p.NT + 2 * kt + e];
-            if (p.skip_pad_queries) {   // the padding bits describe positions: words 4 i .. 4 i + 3 cover the queries of tile i
-              const uint4 w = *reinterpret_cast<const uint4*>(p.kpad + size_t(b) * p.TW + 4 * i);
-              pad = (w.x & w.y & w.z & w.w) == 0xffffffffu;
-            }
-          }
-          const bool act = (c & want) != 0 && !pad;
-          const unsigned m = __ballot_sync(0xffffffffu, act);
-          if (act) plan.tiles[n_act + __popc(m & ((1u << lane) - 1u))] = uint16_t(i | ((c & 3) == 3 ? kMixed : 0));
+          if (i0 > 0) c = tile_class(i0 + lane);
+          const unsigned m = __ballot_sync(0xffffffffu, (c & want) != 0);
+          if (c & want) plan.tiles[n_act + __popc(m & ((1u << lane) - 1u))] = uint16_t((i0 + lane) | ((c & 3) == 3 ? kMixed : 0));
           n_act += __popc(m);
         }
       if (n_act == 0) {   // the gradients of a key tile without a single pair of this pathway are zero
@@ -453,8 +458,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
       kr.advance();
       vr.advance();
     }
-    if (ok) ok = wait_all(&plan_empty[pr.pos], pr.phase ^ 1, 0x526);
-    if (ok && lane == 0) {
+    if (ok && lane == 0) {   // (the slot it waited for last)
       plans[pr.pos].n = 0;
       mbar_arrive(&plan_full[pr.pos]);
     }
@@ -795,74 +799,73 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
       };
       uint32_t bits = tile_bits(0);
       for (int it = 0; it < n && ok; ++it) {
-        {
-          const uint32_t bits_next = it + 1 < n ? tile_bits(it + 1) : 0u;
-          ok = wait_all(&st_full[g % kQStages], (g / kQStages) & 1u, 0x604);
-          if (ok) ok = wait_all(&sdp_full[br.pos], br.phase, 0x602);
-          if (ok) ok = wait_all(&dq_full[g % kNDq], ((g / kNDq) & 1u) ^ 1u, 0x606);   // the dS tile has been read (by the product of two tiles ago)
-          if (!ok) break;
-          const uint32_t mask = (bits ^ plan.flip) & key_valid;
-          tc_fence_after();
-          const uint32_t ds_row = ds_addr + (g % kNDq) * Cfg::kDsBytes;
+        const uint32_t bits_next = it + 1 < n ? tile_bits(it + 1) : 0u;
+        ok = mbar_wait(&st_full[g % kQStages], (g / kQStages) & 1u, p.status, 0x604) &
+             mbar_wait(&dq_full[g % kNDq], ((g / kNDq) & 1u) ^ 1u, p.status, 0x606) &   // the dS tile has been read (by the product of two tiles ago)
+             mbar_wait(&sdp_full[br.pos], br.phase, p.status, 0x602);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        const uint32_t mask = (bits ^ plan.flip) & key_valid;
+        tc_fence_after();
+        const uint32_t ds_row = ds_addr + (g % kNDq) * Cfg::kDsBytes;
 #pragma unroll
-          for (int v = 0; v < 2; ++v) {
-            // statistics of this thread's 16 queries, (nl0, nl1, nd0, nd1) per pair, from the copy that arrived in shared memory with the query tile
-            const float4* st = reinterpret_cast<const float4*>(sStats + (g % kQStages) * Cfg::kStatBytes) + (sub * kHalf + 32 * c32 + 16 * v) / 2;
-            const uint32_t keep = (mask >> (16 * v)) & 0xffffu;
-            const uint32_t tS = tBuf + br.pos * 128 + 16 * v;
-            uint32_t sv[16], dpv[16];
-            tmem_ld16(tS, sv);
-            tmem_ld16(tS + 64, dpv);
-            tmem_ld_wait();
-            uint32_t pp[8], dd[8];
-            // Straight-line code for each of the two cases: a test inside the loop would cut it into blocks that end in
-            // reconvergence points, and the exponentials of one pair of queries could not overlap those of the next.
-            auto elements = [&](auto masked) {
+        for (int v = 0; v < 2; ++v) {
+          // statistics of this thread's 16 queries, (nl0, nl1, nd0, nd1) per pair, from the copy that arrived in shared memory with the query tile
+          const float4* st = reinterpret_cast<const float4*>(sStats + (g % kQStages) * Cfg::kStatBytes) + (sub * kHalf + 32 * c32 + 16 * v) / 2;
+          const uint32_t keep = (mask >> (16 * v)) & 0xffffu;
+          const uint32_t tS = tBuf + br.pos * 128 + 16 * v;
+          uint32_t sv[16], dpv[16];
+          tmem_ld16(tS, sv);
+          tmem_ld16(tS + 64, dpv);
+          tmem_ld_wait();
+          uint32_t pp[8], dd[8];
+          // Straight-line code for each of the two cases: a test inside the loop would cut it into blocks that end in
+          // reconvergence points, and the exponentials of one pair of queries could not overlap those of the next.
+          auto elements = [&](auto masked) {
 #pragma unroll
-              for (int j = 0; j < 16; j += 2) {
-                const float4 q2 = st[j / 2];
-                float p0, p1;
-                unpack2(ffma2(pack2(__uint_as_float(sv[j]), __uint_as_float(sv[j + 1])), c22, pack2(q2.x, q2.y)), p0, p1);
-                p0 = bwd_ex2(p0);
-                p1 = bwd_ex2(p1);
-                if (decltype(masked)::value) {
-                  p0 = (keep >> j) & 1u ? p0 : 0.f;
-                  p1 = (keep >> (j + 1)) & 1u ? p1 : 0.f;
-                }
-                float d0, d1;
-                const uint64_t p2 = pack2(p0, p1), dp2 = pack2(__uint_as_float(dpv[j]), __uint_as_float(dpv[j + 1])), nd2 = pack2(q2.z, q2.w);
-                if (SQ)   // r = sqrt(p) is what p0, p1 hold: dS = r (dP / 2 - r delta / 2), and r itself multiplies dO in dV
-                  unpack2(fmul2(p2, ffma2(p2, nd2, fmul2(dp2, pack2(0.5f, 0.5f)))), d0, d1);
-                else      // dS = p (dP - delta)
-                  unpack2(fmul2(p2, fadd2(dp2, nd2)), d0, d1);
-                pp[j / 2] = bwd_pack(p0, p1);
-                dd[j / 2] = bwd_pack(d0, d1);
+            for (int j = 0; j < 16; j += 2) {
+              const float4 q2 = st[j / 2];
+              float p0, p1;
+              unpack2(ffma2(pack2(__uint_as_float(sv[j]), __uint_as_float(sv[j + 1])), c22, pack2(q2.x, q2.y)), p0, p1);
+              p0 = bwd_ex2(p0);
+              p1 = bwd_ex2(p1);
+              if (decltype(masked)::value) {
+                p0 = (keep >> j) & 1u ? p0 : 0.f;
+                p1 = (keep >> (j + 1)) & 1u ? p1 : 0.f;
               }
-            };
-            if (__all_sync(0xffffffffu, keep == 0xffffu)) {
-              elements(std::false_type{});
-            } else if (__all_sync(0xffffffffu, keep == 0u)) {   // the other side of a chain boundary, or padding
-#pragma unroll
-              for (int j = 0; j < 8; ++j) pp[j] = dd[j] = 0u;
-            } else {
-              elements(std::true_type{});
+              float d0, d1;
+              const uint64_t p2 = pack2(p0, p1), dp2 = pack2(__uint_as_float(dpv[j]), __uint_as_float(dpv[j + 1])), nd2 = pack2(q2.z, q2.w);
+              if (SQ)   // r = sqrt(p) is what p0, p1 hold: dS = r (dP / 2 - r delta / 2), and r itself multiplies dO in dV
+                unpack2(fmul2(p2, ffma2(p2, nd2, fmul2(dp2, pack2(0.5f, 0.5f)))), d0, d1);
+              else      // dS = p (dP - delta)
+                unpack2(fmul2(p2, fadd2(dp2, nd2)), d0, d1);
+              pp[j / 2] = bwd_pack(p0, p1);
+              dd[j / 2] = bwd_pack(d0, d1);
             }
-            tmem_st8(tS, pp);         // P^T over the S^T columns this thread has read
-            tmem_st8(tS + 64, dd);    // dS^T likewise
-            // and dS into shared memory for the dQ product: 2 chunks of 8 queries in block `sub` of the dS tile
-            const uint32_t ds_at = ds_row ^ (v * 32);
-            smem_store16(ds_at, dd[0], dd[1], dd[2], dd[3]);
-            smem_store16(ds_at ^ 16u, dd[4], dd[5], dd[6], dd[7]);
+          };
+          if (__all_sync(0xffffffffu, keep == 0xffffu)) {
+            elements(std::false_type{});
+          } else if (__all_sync(0xffffffffu, keep == 0u)) {   // the other side of a chain boundary, or padding
+#pragma unroll
+            for (int j = 0; j < 8; ++j) pp[j] = dd[j] = 0u;
+          } else {
+            elements(std::true_type{});
           }
-          tmem_st_wait();
-          fence_proxy_async_smem();
-          tc_fence_before();
-          mbar_arrive(&pds_full[br.pos]);
-          br.advance();
-          br.advance();
-          bits = bits_next;
-          ++g;
+          tmem_st8(tS, pp);         // P^T over the S^T columns this thread has read
+          tmem_st8(tS + 64, dd);    // dS^T likewise
+          // and dS into shared memory for the dQ product: 2 chunks of 8 queries in block `sub` of the dS tile
+          const uint32_t ds_at = ds_row ^ (v * 32);
+          smem_store16(ds_at, dd[0], dd[1], dd[2], dd[3]);
+          smem_store16(ds_at ^ 16u, dd[4], dd[5], dd[6], dd[7]);
         }
+        tmem_st_wait();
+        fence_proxy_async_smem();
+        tc_fence_before();
+        mbar_arrive(&pds_full[br.pos]);
+        br.advance();
+        br.advance();
+        bits = bits_next;
+        ++g;
       }
       if (!ok) break;
       __syncwarp();
