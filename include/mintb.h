@@ -207,6 +207,12 @@ MINTB_API int mintb_qkv_fwd(const void* x, const void* w, const void* bias, void
                             int D, int in_dtype, int bias_dtype, float alpha, float q_scale, const float* rope_cos,
                             const float* rope_sin, const int32_t* row_map, int n_rows, void* stream, int* dev_status);
 MINTB_API int mintb_quantize_e4m3(const void* x, void* out, size_t n, float inv_scale, void* stream);
+/* mintb_linear_f32: fp32 projections on the CUDA cores, out[g] = act(x w[g]^T + bias[g]) (+ resid) for g < groups <= 6 weights of one
+ * shape [N][K] (host arrays of device pointers; bias[g] may be NULL), act = erf-GELU if `gelu`.  D > 0: head-major outputs
+ * (B,H,T,D), row m = t * B + b, column n = h * D + d (M = T * B, N = H * D, no resid); else row-major [M][N].  N and K are multiples of
+ * four, every pointer 16-byte aligned. */
+MINTB_API int mintb_linear_f32(const float* x, const float* const* w, const float* const* bias, float* const* out, const float* resid,
+                               int groups, int M, int N, int K, int gelu, int B, int T, int H, int D, void* stream);
 /* mintb_linear_res_fwd: mintb_linear_fwd without activation and with the layer's residual sum formed in the epilogue:
  * out[M][N] = res_a * resid[M][N] + res_b * (alpha * x w^T + bias) - x + out_proj(attention) of the Pre-LN layer
  * (modules.py:183-186: res_a = res_b = 1) and sqrt(1 - tau) x + sqrt(tau) out_proj(attention) of the muS layer

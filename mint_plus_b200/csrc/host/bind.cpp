@@ -48,6 +48,8 @@ PYBIND11_MODULE(_mintb_host, m) {
   m.def("mask_meta", &mask_meta, nogil);
   m.def("combine", &combine, nogil);
   m.def("linear", &linear, nogil);
+  m.def("linear_f32", &linear_f32, nogil);
+  m.def("heads_f32", &heads_f32, nogil);
   m.def("add_layernorm", &add_layernorm, nogil);
   m.def("embed", &embed, nogil);
   m.def("masked_ce", &masked_ce, nogil);

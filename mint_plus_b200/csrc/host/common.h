@@ -102,6 +102,10 @@ std::pair<Tensor, Tensor> linear_fwd(const Product& p);     // (y, pre-activatio
 // res_a resid + res_b (alpha x w^T + bias), and with quant > 0 its e4m3 copy saturate(. / quant); round_first: the projection is rounded
 // to bf16 before the sum
 std::pair<Tensor, Tensor> linear_res_fwd(const Product& p, const Tensor& resid, double res_a, double res_b, double quant, bool round_first = false);
+// fp32: act(x w^T + bias) (+ resid) of (rows, K) rows
+Tensor linear_f32(const Tensor& x, const Tensor& w, const OptTensor& bias, bool gelu, const OptTensor& resid);
+// fp32: the q, k, v projections of (T,B,E) activations, head-major: `w` and `bias` hold the weights in order, each [E][E] or [3E][E]
+std::vector<Tensor> heads_f32(const Tensor& x, const std::vector<Tensor>& w, const std::vector<OptTensor>& bias, int64_t H);
 Tensor quantize(const Tensor& x, double scale);
 // alpha (dz w + dz2 w2) + beta resid
 Tensor dgrad(const Tensor& dz, const Tensor& w, double alpha, const Tensor& dz2 = {}, const Tensor& w2 = {}, const Tensor& resid = {}, double beta = 0.0);

@@ -71,6 +71,40 @@ std::pair<Tensor, Tensor> linear_res_fwd(const Product& p, const Tensor& resid, 
   return {out, q8};
 }
 
+Tensor linear_f32(const Tensor& x, const Tensor& w, const OptTensor& bias, bool gelu, const OptTensor& resid) {
+  Env e(x);
+  const int64_t K = w.size(1), N = w.size(0), M = x.numel() / K;
+  TORCH_CHECK(x.size(-1) == K && x.is_contiguous() && w.is_contiguous(), "linear_f32: contiguous rows of the weight's width are required");
+  std::vector<int64_t> shape = x.sizes().vec();
+  shape.back() = N;
+  Tensor out = e.empty(shape, at::kFloat);
+  const Tensor b = opt(bias), r = opt(resid);
+  TORCH_CHECK(!r.defined() || (r.is_contiguous() && r.numel() == M * N), "linear_f32: the residual has the result's shape");
+  const float *wp = fptr(w), *bp = fptr(b);
+  float* op = fptr(out);
+  check(mintb_linear_f32(fptr(x), &wp, &bp, &op, fptr(r), 1, M, N, K, gelu, 1, 1, 1, 0, e.stream), "mintb_linear_f32");
+  return out;
+}
+
+std::vector<Tensor> heads_f32(const Tensor& x, const std::vector<Tensor>& w, const std::vector<OptTensor>& bias, int64_t H) {
+  Env e(x);
+  const int64_t T = x.size(0), B = x.size(1), E = x.size(2), D = E / H;
+  std::vector<const float*> wp, bp;
+  std::vector<float*> op;
+  std::vector<Tensor> out;
+  for (size_t i = 0; i < w.size(); ++i) {
+    TORCH_CHECK(x.is_contiguous() && w[i].is_contiguous() && w[i].size(1) == E && w[i].size(0) % E == 0, "heads_f32: contiguous (n E, E) weights are required");
+    for (int64_t k = 0; k < w[i].size(0) / E; ++k) {
+      wp.push_back(fptr(w[i]) + k * E * E);
+      bp.push_back(bias[i].has_value() ? fptr(*bias[i]) + k * E : nullptr);
+      out.push_back(e.empty({B, H, T, D}, at::kFloat));
+      op.push_back(fptr(out.back()));
+    }
+  }
+  check(mintb_linear_f32(fptr(x), wp.data(), bp.data(), op.data(), nullptr, int(wp.size()), T * B, E, E, 0, B, T, H, D, e.stream), "mintb_linear_f32");
+  return out;
+}
+
 Tensor quantize(const Tensor& x, double scale) {
   Env e(x);
   Tensor out = e.empty(x.sizes(), at::kFloat8_e4m3fn);

@@ -1,0 +1,222 @@
+// fp32 projections on the CUDA cores: out = act(x w^T + bias) [+ resid], x [M][K] and w [N][K] K-contiguous (nn.Linear layout).
+//
+// One launch serves up to six weights of the same shape (the q, k, v projections of both pathways read the same rows), each with an
+// output of its own, row-major or scattered head-major into (B,H,T,D).  Bound by the packed fp32 multiply-adds: a thread keeps a
+// TM x TN block of results in registers, pairs of rows in one 64-bit register, and reads TM + TN operands per k from shared memory.
+// Slabs of BK columns are turned on the way into shared memory ([k][row], rows XOR-ed by their k so that neither the stores nor the
+// reads collide) and double buffered; the next slab's global loads are in flight while one is multiplied.
+#include "common.cuh"
+#include "ptx.cuh"
+
+namespace mintb {
+namespace {
+
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ uint64_t ffma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
+struct SgemmParams {
+  const float* x;
+  const float *w[6], *bias[6];
+  float* out[6];
+  const float* resid;      // row-major [M][N] or null
+  int M, N, K, gelu;
+  int B, T, H, D;          // D > 0: head-major outputs, row m = t * B + b, column n = h * D + d
+};
+
+template <int BM, int BN, int TM, int TN, int BK, int KS>
+__global__ void __launch_bounds__(KS * (BM / TM) * (BN / TN)) sgemm_kernel(const SgemmParams p) {
+  constexpr int kThreads = (BM / TM) * (BN / TN), kTx = BN / TN;
+  constexpr int kLpr = BK / 4;                        // lanes that load one row's slab, 16 bytes each
+  constexpr int kUnit = 32 / kLpr;                    // rows a warp loads at a time: the unit of the XOR
+  constexpr int kLa = BM * kLpr / kThreads, kLb = BN * kLpr / kThreads;
+  static_assert(kLa * kThreads == BM * kLpr && kLb * kThreads == BN * kLpr && BM % 32 == 0 && BN % 32 == 0 && kUnit >= 4, "tile shape");
+  extern __shared__ float4 smem4[];
+  ptx::griddep_wait();
+  ptx::griddep_launch();
+  const int kg = threadIdx.x / kThreads, tid = threadIdx.x % kThreads, tx = tid % kTx, ty = tid / kTx;   // kg: which of the KS parts of every slab
+  constexpr int kBuf = BK * (BM + BN);
+  float* sm = reinterpret_cast<float*>(smem4) + kg * 2 * kBuf;   // [KS][2][BK][BM + BN]
+  const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN, g = blockIdx.z;
+  const float* __restrict__ x = p.x;
+  const float* __restrict__ w = p.w[g];
+  const int lc = tid % kLpr, lr = tid / kLpr;         // this thread's column chunk and first row of a slab
+  float4 ra[kLa], rb[kLb];
+  auto fetch = [&](int k0) {
+    const int k = k0 + 4 * lc;
+    const bool in_k = k < p.K;                        // (K is a multiple of four)
+#pragma unroll
+    for (int i = 0; i < kLa; ++i) {
+      const int m = m0 + lr + i * (kThreads / kLpr);
+      ra[i] = in_k && m < p.M ? __ldg(reinterpret_cast<const float4*>(x + size_t(m) * p.K + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int i = 0; i < kLb; ++i) {
+      const int n = n0 + lr + i * (kThreads / kLpr);
+      rb[i] = in_k && n < p.N ? __ldg(reinterpret_cast<const float4*>(w + size_t(n) * p.K + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  };
+  auto stash = [&](float* buf) {
+    const int sw = kUnit * lc;
+#pragma unroll
+    for (int i = 0; i < kLa; ++i) {
+      const int r = (lr + i * (kThreads / kLpr)) ^ sw;
+      float* d = buf + (4 * lc) * (BM + BN) + r;
+      d[0] = ra[i].x; d[BM + BN] = ra[i].y; d[2 * (BM + BN)] = ra[i].z; d[3 * (BM + BN)] = ra[i].w;
+    }
+#pragma unroll
+    for (int i = 0; i < kLb; ++i) {
+      const int r = (lr + i * (kThreads / kLpr)) ^ sw;
+      float* d = buf + (4 * lc) * (BM + BN) + BM + r;
+      d[0] = rb[i].x; d[BM + BN] = rb[i].y; d[2 * (BM + BN)] = rb[i].z; d[3 * (BM + BN)] = rb[i].w;
+    }
+  };
+  uint64_t acc[TM / 2][TN];
+#pragma unroll
+  for (int i = 0; i < TM / 2; ++i)
+#pragma unroll
+    for (int j = 0; j < TN; ++j) acc[i][j] = 0ull;
+  const int slabs = (p.K + KS * BK - 1) / (KS * BK);
+  fetch(kg * BK);
+  stash(sm);
+  __syncthreads();
+  for (int s = 0; s < slabs; ++s) {
+    const float* buf = sm + (s & 1) * kBuf;
+    if (s + 1 < slabs) fetch(((s + 1) * KS + kg) * BK);
+#pragma unroll
+    for (int k = 0; k < BK; ++k) {
+      const int sw = kUnit * (k / 4);
+      const float* row = buf + k * (BM + BN);
+      uint64_t a[TM / 2];
+      float b[TN];
+#pragma unroll
+      for (int i = 0; i < TM; i += 4) {
+        const float4 v = *reinterpret_cast<const float4*>(row + ((TM * ty + i) ^ sw));
+        a[i / 2] = pack2(v.x, v.y);
+        a[i / 2 + 1] = pack2(v.z, v.w);
+      }
+#pragma unroll
+      for (int j = 0; j < TN; j += 4) {
+        const float4 v = *reinterpret_cast<const float4*>(row + BM + ((4 * tx + j * kTx) ^ sw));
+        b[j] = v.x; b[j + 1] = v.y; b[j + 2] = v.z; b[j + 3] = v.w;
+      }
+#pragma unroll
+      for (int j = 0; j < TN; ++j) {
+        const uint64_t bb = pack2(b[j], b[j]);
+#pragma unroll
+        for (int i = 0; i < TM / 2; ++i) acc[i][j] = ffma2(a[i], bb, acc[i][j]);
+      }
+    }
+    if (s + 1 < slabs) stash(sm + ((s + 1) & 1) * kBuf);   // (that buffer was left by everyone before the last barrier)
+    __syncthreads();
+  }
+  if constexpr (KS > 1) {   // the parts' sums, one after the other, through the shared memory of the slabs
+    uint64_t* red = reinterpret_cast<uint64_t*>(smem4);   // [KS - 1][TM / 2 * TN][kThreads]
+    static_assert((KS - 1) * (TM / 2) * TN * kThreads * 8 <= KS * 2 * kBuf * 4, "room for the partial sums");
+    if (kg > 0) {
+#pragma unroll
+      for (int i = 0; i < TM / 2; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) red[((kg - 1) * (TM / 2) * TN + i * TN + j) * kThreads + tid] = acc[i][j];
+    }
+    __syncthreads();
+    if (kg > 0) return;
+#pragma unroll
+    for (int i = 0; i < TM / 2; ++i)
+#pragma unroll
+      for (int j = 0; j < TN; ++j)
+#pragma unroll
+        for (int q = 0; q < KS - 1; ++q) {
+          float a0, a1, b0, b1;
+          unpack2(acc[i][j], a0, a1);
+          unpack2(red[(q * (TM / 2) * TN + i * TN + j) * kThreads + tid], b0, b1);
+          acc[i][j] = pack2(a0 + b0, a1 + b1);
+        }
+  }
+  // groups of four columns: 4 tx + j kTx (N is a multiple of four)
+  float bias[TN];
+#pragma unroll
+  for (int j = 0; j < TN; j += 4) {
+    const int n = n0 + 4 * tx + j * kTx;
+    const float4 v = p.bias[g] != nullptr && n < p.N ? __ldg(reinterpret_cast<const float4*>(p.bias[g] + n)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    bias[j] = v.x; bias[j + 1] = v.y; bias[j + 2] = v.z; bias[j + 3] = v.w;
+  }
+#pragma unroll
+  for (int i = 0; i < TM; ++i) {
+    const int m = m0 + TM * ty + i;
+    if (m >= p.M) continue;
+#pragma unroll
+    for (int j = 0; j < TN; j += 4) {
+      const int n = n0 + 4 * tx + j * kTx;
+      if (n >= p.N) continue;
+      float v[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        float lo, hi;
+        unpack2(acc[i / 2][j + e], lo, hi);
+        v[e] = (i & 1 ? hi : lo) + bias[j + e];
+        if (p.gelu) v[e] = 0.5f * v[e] * (1.f + erff(v[e] * 0.70710678118654752f));
+      }
+      size_t at = size_t(m) * p.N + n;
+      if (p.D > 0) {
+        const int t = m / p.B, b = m % p.B;
+        at = ((size_t(b) * p.H + n / p.D) * p.T + t) * p.D + n % p.D;
+      }
+      if (p.resid != nullptr) {
+        const float4 r = __ldg(reinterpret_cast<const float4*>(p.resid + at));
+        v[0] += r.x; v[1] += r.y; v[2] += r.z; v[3] += r.w;
+      }
+      *reinterpret_cast<float4*>(p.out[g] + at) = make_float4(v[0], v[1], v[2], v[3]);
+    }
+  }
+}
+
+template <int BM, int BN, int TM, int TN, int BK, int KS>
+int launch_t(const SgemmParams& p, int groups, cudaStream_t s) {
+  constexpr auto kern = sgemm_kernel<BM, BN, TM, TN, BK, KS>;
+  constexpr size_t smem = size_t(KS) * 2 * BK * (BM + BN) * sizeof(float);
+  cudaError_t e = opt_in_smem<kern>(int(smem));
+  if (e == cudaSuccess)
+    e = launch_dependent(kern, dim3((p.M + BM - 1) / BM, (p.N + BN - 1) / BN, groups), dim3(KS * (BM / TM) * (BN / TN)), smem, s, p);
+  count_launches(1);
+  if (e != cudaSuccess) { set_error("sgemm launch: %s", cudaGetErrorString(e)); return MINTB_ECUDA; }
+  return MINTB_OK;
+}
+
+}  // namespace
+}  // namespace mintb
+
+using namespace mintb;
+
+extern "C" int mintb_linear_f32(const float* x, const float* const* w, const float* const* bias, float* const* out, const float* resid, int groups, int M,
+                                int N, int K, int gelu, int B, int T, int H, int D, void* stream) {
+  bool ok = x != nullptr && w != nullptr && bias != nullptr && out != nullptr && groups >= 1 && groups <= 6 && M > 0 && N > 0 && K > 0 && N % 4 == 0 && K % 4 == 0 &&
+            (D == 0 || (D % 4 == 0 && N == H * D && M == T * B && resid == nullptr)) && M <= 65535 * 32;
+  auto aligned = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
+  ok = ok && aligned(x) && aligned(resid);
+  for (int i = 0; ok && i < groups; ++i) ok = w[i] != nullptr && out[i] != nullptr && aligned(w[i]) && aligned(bias[i]) && aligned(out[i]);
+  if (!ok) {
+    set_error("mintb_linear_f32: one to six 16-byte aligned weights, N and K multiples of four, and matching head-major sizes are required");
+    return MINTB_EINVAL;
+  }
+  SgemmParams p{};
+  p.x = x; p.resid = resid; p.M = M; p.N = N; p.K = K; p.gelu = gelu; p.B = B; p.T = T; p.H = H; p.D = D;
+  for (int i = 0; i < groups; ++i) { p.w[i] = w[i]; p.bias[i] = bias[i]; p.out[i] = out[i]; }
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  // The largest tile that leaves every SM several: with fewer than about one 64 x 32 tile per SM, smaller ones whose K four parts of the
+  // CTA share (M100 N320 K1280: 29 -> 16 us); with rounds of tiles to spare, 64 x 64 (M5120 N1280 K320: 106 -> 97 us).  Against the
+  // library's products: M2048 N320 K320 26.6 -> 17.5 us, six of them 157 -> 64 us in one launch, M2048 N320 K1280 65 -> 59 us, M5120
+  // N320 K1280 101 -> 112 us (without the residual sum and its pass), M5120 N1280 K320 109 -> 97 us.
+  const long long tiles = static_cast<long long>((M + 63) / 64) * ((N + 31) / 32) * groups, sms = sm_count();
+  if (4 * tiles < 5 * sms) return launch_t<32, 32, 4, 4, 32, 4>(p, groups, s);
+  if (tiles < 14 * sms) return launch_t<64, 32, 8, 4, 32, 2>(p, groups, s);
+  return launch_t<64, 64, 8, 4, 16, 1>(p, groups, s);
+}

@@ -254,6 +254,9 @@ class _PreLnLayer(_TwoPathwayLayer):
             return x + self.feed_forward(h), attn
         if pack is not None:
             raise NotImplementedError("packed tokens need bfloat16 CUDA activations")
+        y = native.run_layer_f32(self, x, self_attn_mask, self_attn_padding_mask, chain_ids)
+        if y is not None:
+            return y, None
         residual = x
         x = self.self_attn_layer_norm(x)
         if self.use_multimer:

@@ -3,7 +3,8 @@ and backward pass take, formed once and kept on the layer until one of them chan
 
 A layer is served here when it is what the builders make: bf16 activations on the GPU, nn.Linear projections with bf16 weights
 (with or without LoRA adapters on a frozen base) or Fp8Linear ones throughout, LayerNorms with parameters, the fused attention.
-Everything else (wrapped projections, mixed kinds) stays on the modules' own path.
+Everything else (wrapped projections, mixed kinds) stays on the modules' own path; plain fp32 layers have a short one of their own at
+the end of this file.
 """
 from __future__ import annotations
 
@@ -190,3 +191,35 @@ def run_layer(layer, x, chain_mask, padding_mask, chain_ids, pack, *, mu: bool, 
     if q8 is not None:
         ops.attach_e4m3(y, q8, next_quant)
     return y
+
+
+def _plain(mod, kind, dtype=torch.float32) -> bool:
+    """`mod` is exactly a `kind` with aligned contiguous parameters of `dtype` and no hooks."""
+    return (type(mod) is kind and not mod._forward_hooks and not mod._forward_pre_hooks and
+            all(p is None or (p.is_cuda and p.dtype == dtype and p.is_contiguous() and p.data_ptr() % 16 == 0) for p in (mod.weight, mod.bias)))
+
+
+def run_layer_f32(layer, x, chain_mask, padding_mask, chain_ids):
+    """The Pre-LN layer's result for fp32 activations (T,B,E) without gradients, or None when the layer is not served here: every
+    projection one launch with bias, GELU and residual sum in its epilogue, and the six of q, k, v together with the head-major
+    layout.  (With gradients the projections stay autograd's linears, which keep what their backward pass needs.)"""
+    from . import modules_plus as mp
+    if (torch.is_grad_enabled() or not (x.is_cuda and x.dtype == torch.float32 and x.is_contiguous() and x.data_ptr() % 16 == 0) or
+            not (layer.use_multimer and layer._use_fused_multi_pathway) or layer._use_sqrt_softmax or torch.is_autocast_enabled("cuda")):
+        return None
+    sa, ma, ff = layer.self_attn, layer.multimer_attn, layer.feed_forward
+    if type(ff) is not mp.VanillaFeedForward or sa.head_dim not in (16, 32, 64) or x.numel() == 0:
+        return None
+    projections = [m for a in (sa, ma) for m in (_attn_mods(a) or [None])]
+    if not (all(m is not None and _plain(m, torch.nn.Linear) for m in (*projections, sa.out_proj, ff.fc1, ff.fc2)) and ff.fc1.out_features % 4 == 0 and
+            type(layer.self_attn_layer_norm) is type(layer.final_layer_norm) is torch.nn.LayerNorm):
+        return None
+    T, B, E = x.shape
+    host = L.host()
+    meta = mp._cached_ids_meta(chain_ids, padding_mask) if chain_ids is not None and chain_mask is None else ops.cached_mask_meta(chain_mask, padding_mask)
+    rope = sa.rot_emb is not None
+    heads = host.heads_f32(layer.self_attn_layer_norm(x), [m.weight for m in projections], [m.bias for m in projections], sa.num_heads)
+    out = ops.multimer_attention(*heads, meta=meta, rope=rope, inv_freq=sa.rot_emb.inv_freq if rope else None, scale=sa.scaling, out_seq_first=True)
+    x = host.linear_f32(out.reshape(T, B, E), sa.out_proj.weight, sa.out_proj.bias, False, x)
+    h = host.linear_f32(layer.final_layer_norm(x), ff.fc1.weight, ff.fc1.bias, True, None)
+    return host.linear_f32(h, ff.fc2.weight, ff.fc2.bias, False, x)
