@@ -285,7 +285,6 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
   __syncthreads();
   tc_fence_after();
   griddep_wait();    // the set-up above may overlap the kernel before this one; what it wrote is read from here on
-  griddep_launch();  // (the next kernel's set-up may begin: this grid's tensor memory is allocated)
   const uint32_t tbase = *tmem_slot;
 
   if (warp == 0) {
@@ -410,7 +409,10 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
       }
       ++item_no;
     }
-    if (lane == 0) leave_tile_counter(p.sched, int(gridDim.x));   // (after this CTA's last draw, whichever way the loop ended)
+    if (lane == 0) {   // after this CTA's last draw, whichever way the loop ended
+      griddep_launch();   // only now: see launch_dependent in common.cuh
+      leave_tile_counter(p.sched, int(gridDim.x));
+    }
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issuer
     // The whole warp runs this loop and one elected lane issues: with warp-uniform control flow and operands the compiler

@@ -338,11 +338,9 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
   __syncthreads();
   tc_fence_after();
   // The loading warp plans its first key tile and requests what no recent pass has written before it waits for the pass before this
-  // kernel (the statistics, the cleared dQ accumulators); nothing else here happens before that wait.  The pass after this kernel
-  // (the dQ conversion) may be scheduled once every CTA has come this far; it waits for the whole grid itself.
+  // kernel (the statistics, the cleared dQ accumulators); nothing else here happens before that wait.
   if (warp != 3) {
     griddep_wait();
-    if (tid == 0) griddep_launch();
   }
   const uint32_t tbase = *tmem_slot;
   // The MMA warps below run their loops with all lanes and let one elected lane issue: with warp-uniform control flow and
@@ -464,6 +462,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
     }
     if (lane == 0) leave_tile_counter(p.sched, int(gridDim.x));
     griddep_wait();
+    if (lane == 0) griddep_launch();   // only now: see launch_dependent in common.cuh
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA stream A: S^T = K Q^T and dP^T = V dO^T
     // Issuing one tcgen05.mma costs its thread some 50 cycles whatever the tile size, and at small head sizes the

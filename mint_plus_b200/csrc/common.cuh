@@ -99,6 +99,10 @@ inline size_t grad_h_stride(const AttnArgs& a) { return a.grad_rowmajor ? size_t
 void set_error(const char* fmt, ...);
 // Launch `kern` so that it may start while the kernel before it in the stream is still running (programmatic dependent
 // launch); the kernel calls ptx::griddep_wait() before it touches anything that kernel writes.  `cluster` neighbouring CTAs form a cluster.
+// Where that kernel lets it start (ptx::griddep_launch()): after its own wait, so that a kernel may count on everything before its direct
+// predecessor being complete; after its tensor memory is allocated, which the next kernel's CTAs might otherwise take and then wait;
+// and, in the persistent kernels, when a CTA has drawn its last unit: CTAs of the next kernel that wait on the SMs from the start cost
+// a long kernel 3 % (attention forward B8 H40 T2048 D64: 564 us per call, 549 without them).
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_dependent_clusters(int cluster, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
   cudaLaunchConfig_t cfg{};

@@ -139,7 +139,6 @@ gemm_bwd_kernel(const __grid_constant__ CUtensorMap map_a1, const __grid_constan
   __syncthreads();
   tc_fence_after();
   griddep_wait();
-  griddep_launch();   // only now: see gemm_tc_kernel
   const uint32_t tbase = *tmem_slot;
 
   if (warp == 0) {
@@ -187,6 +186,7 @@ gemm_bwd_kernel(const __grid_constant__ CUtensorMap map_a1, const __grid_constan
         }
         if (!ok) break;
       }
+      griddep_launch();   // only now: see launch_dependent in common.cuh
       leave_tile_counter(p.sched, int(gridDim.x));
     }
   } else if (warp == 1) {

@@ -160,11 +160,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   tc_fence_before();
   if constexpr (PAIR) cluster_sync(); else __syncthreads();
   tc_fence_after();
-  // The next kernel may set itself up while this one runs: from here on only, because its CTAs may take tensor memory that a CTA of
-  // this grid has yet to allocate, and then wait for this grid; and after the wait, so that a kernel may count on everything before
-  // its direct predecessor being complete.
   griddep_wait();
-  griddep_launch();
   const uint32_t tbase = *tmem_slot;
 
   if (warp == 0) {
@@ -227,6 +223,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           ok = mbar_wait(&empty[stage], phase ^ 1, p.status, 0x709);
           if (++stage == kGStages) { stage = 0; phase ^= 1; }
         }
+      griddep_launch();   // only now: see launch_dependent in common.cuh
       if (rank == 0) leave_tile_counter(p.sched, int(gridDim.x) / (PAIR ? 2 : 1));
     }
   } else if (warp == 1) {
