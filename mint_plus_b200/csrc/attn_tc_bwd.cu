@@ -1,15 +1,15 @@
 // tcgen05 backward of the combined-softmax multimer attention (bf16 in, fp32 accumulate).
 //
 // With the forward log-sum-exp known, the two pathways are independent: the self pathway contributes
-// P o ~M and the cross pathway P o M, each computed from its own Q, K, V.  The grid is
-// (key tiles of 128, batch*head, pathway); a CTA owns dK and dV of its key tile in TMEM and walks the query
-// tiles of 128 whose class holds pairs of its pathway:
+// P o ~M and the cross pathway P o M, each computed from its own Q, K, V.  Persistent CTAs, one per SM, draw work items
+// (key tile of 128, batch*head, pathway); a CTA holds dK and dV of its item in TMEM and walks the query
+// tiles of 128 whose class holds pairs of the pathway:
 //   S^T = K Q^T, dP^T = V dO^T            (lane = key, column = query; two halves of 64 queries, one TMEM buffer each)
 //   P^T = exp2(S^T c - lse), masked       dS^T = P^T o (dP^T - delta)
 //   dV += P^T dO, dK += dS^T Q            (A operands read from TMEM, aliased over S^T / dP^T)
 //   dQ_tile = dS K                        (dS through shared memory), added to an fp32 accumulator in HBM
-// Warp roles: warps 0-3 MMA issuers, one per family of products (warp 0 also issues the TMA loads), warps 4-19 compute
-// (thread = key row x 16 query columns of the half in flight).  The halves ping-pong: while one is computed the tensor pipe refills the other buffer.
+// Warp roles: warps 0-2 MMA issuers (dQ; S^T and dP^T; dV and dK), warp 3 plans the items and issues the TMA loads, warps 4-7
+// fetch and store the results (dQ per query tile, dK and dV per item), warps 8-23 compute (thread = key row x 32 query columns of one half).
 // TMEM (512 columns): dK, dV, two dQ tiles, then two (head_dim 64) or three (head_dim <= 32) buffers {S^T half, dP^T half}.
 // dQ is accumulated across CTAs with fp32 atomics, so its low-order bits depend on arrival order;
 // dK and dV are reduced inside one CTA in a fixed order.  All mbarrier waits are bounded.
@@ -23,7 +23,7 @@ namespace mintb {
 using namespace ptx;
 
 constexpr int kBwdTile = 128;       // keys per CTA and queries per step
-constexpr int kHalf = 64;           // queries per compute group
+constexpr int kHalf = 64;           // queries of a tile that eight compute warps work on
 constexpr int kBwdMaxTiles = 256;   // T <= 32768
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -273,8 +273,8 @@ struct Ring {
 // with the few tiles a key tile has (1 to 16), what a key tile costs beside them: as one CTA per key tile that was 13 700 cycles at
 // head_dim 32 and 20 900 at 64 (set-up and loads until the first exponential 4700, last dQ tile and gradients out 5000 to 10 000,
 // next CTA 2000 to 3000) against 2200 and 3100 cycles per query tile.  Here barriers and TMEM are set up once; the loading warp
-// plans and loads the next key tile while the current one is computed; and a key tile's last dQ tile and its dK, dV leave after the
-// compute warps have handed the next key tile's first half to the tensor cores.
+// plans and loads the next key tile while the current one is computed; and four warps of their own take the results away while the
+// compute warps go on with the next key tile.  B8 H20 T1024 D32: kernel 265 -> 175 us; B5 H20 T1531 D64 square root: 295 -> 250 us.
 template <int D, bool SQ>
 __global__ void __launch_bounds__(BwdCfg<D>::kThreads, 1)
 attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_constant__ CUtensorMap map_ks,

@@ -2,7 +2,8 @@
 //
 //   x [M][K] and W [N][K] are both K-contiguous (nn.Linear layout), bf16 (kind::f16) or e4m3 (kind::f8f6f4), fp32 accumulate.
 //   Persistent CTAs walk 128 x BN output tiles (N fastest, so the CTAs running together share rows of x in L2), BN = 256 where
-//   they fill the chip, 128 or 64 where fewer, larger tiles would leave most SMs idle (pick_tile below).
+//   they fill the chip, 128 or 64 where fewer, larger tiles would leave most SMs idle, and 256 x 256 tiles by pairs of CTAs where the
+//   reduction is long (pick_tile below).
 //   warp 0  TMA producer: 128-byte-wide K slabs of x (128 rows) and W (BN rows) into a ring of 4 to 8 stages, 128B swizzle
 //   warp 1  MMA issuer: four tcgen05.mma (M128 N = BN) per slab into one of two BN-column TMEM accumulators
 //   warps 2-9  epilogue: two threads per output row (one per half of the tile's columns); 32 columns at a time: alpha, bias, erf-GELU, cast, store —
@@ -732,8 +733,8 @@ static bool gemm_out_map_f8(CUtensorMap* m, const void* ptr, int rows, int N) {
 
 // The tile width that finishes first by a count of cycles on the busiest SM: rounds of the grid times the slabs of a tile (512, 280
 // and 200 cycles at 256, 128 and 64 columns: the narrow ones are bound by the operand traffic into shared memory) plus filling
-// the ring and draining the last tile.  Whole-batch products come out at 256; M = 497 against N = K = 1280 (e4m3) at 64: 20 tiles on 148 SMs
-// and 15.9 us before, 80 tiles and 8.6 us now.
+// the ring and draining the last tile.  Whole-batch products come out at 256; M = 497 against N = K = 1280 (bf16) at 64: 20 tiles on 148 SMs
+// and 13.7 us before, 80 tiles and 9.3 us now.
 //
 // A pair's 256 x 256 tile needs two thirds of a single CTA's operand traffic per product (32 KB instead of 48 KB per slab and SM, which
 // is what limits the 128 x 256 tile, and the power that goes with it), but its tiles are handed over between two SMs: at 10

@@ -124,7 +124,7 @@ struct LnParams {
 
 // MAXV: 16-byte vectors per lane (E <= MAXV * 256).  A warp owns a row and holds it packed, as it was loaded, through the passes for
 // the mean, the variance and the result: as fp32 values (and with registers for a second tensor that is not there) the wide rows
-// left 12 warps on an SM and half of the memory's rate (16384 x 2560, no residual: 72 us, 2.3 TB/s; now 34 us, 4.9 TB/s).
+// left 12 warps on an SM and half of the memory's rate (16384 x 2560, no residual, back to back: 56 us; now 39 us, 4.3 TB/s).
 template <int MAXV, bool HAS_R>
 __global__ void __launch_bounds__(kLnWarps * 32, MAXV == 10 ? 4 : (MAXV == 5 ? 6 : 8)) add_layernorm_fwd_kernel(LnParams p) {
   __shared__ __align__(16) float s_gamma[MAXV * 256], s_beta[MAXV * 256];   // the parameters as fp32, read back 16 bytes at a time
@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(kLnWarps * 32, MAXV == 10 ? 4 : (MAXV == 5 ? 6
 // by nine warp shuffles, then across the warps through a double-buffered shared-memory slot with ONE barrier per batch of rows.
 // Which tensors exist is a template argument (r, ds_in, parameter gradients), so that none costs registers that is not there, and
 // the arithmetic is packed, two columns an instruction: with all of it in one body, single values and the load of ds_in behind the
-// barrier, instructions and latency held 32768 x 640 at 2.1 TB/s (80 us; now 37 us).
+// barrier, instructions and latency held 32768 x 640 at 2.1 TB/s (75 us; now 32 us).
 #ifndef MINTB_LN_BWD_PER_SM
 #define MINTB_LN_BWD_PER_SM 3
 #endif

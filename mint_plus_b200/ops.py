@@ -526,11 +526,6 @@ def f8_output_grad(dy: torch.Tensor, z: Optional[torch.Tensor], want_db: bool, h
     return dz8, db, holder.scale
 
 
-def _gelu_erf_grad(z: torch.Tensor) -> torch.Tensor:
-    zf = z.float()
-    return 0.5 * (1.0 + torch.erf(zf * 0.7071067811865476)) + zf * torch.exp(-0.5 * zf * zf) * 0.3989422804014327
-
-
 def linear_backward(dy, x2d, w, bias, z, needs, out_scale: float = 1.0, db=None, want_dx=True):
     """Gradients of y = act(out_scale * x W^T + b): the GELU derivative and the bias gradient come from one fused pass
     (or the bias gradient is handed in as `db` by the pass that produced dy); dgrad (dz W) and wgrad (dz^T x) run on the
