@@ -255,6 +255,8 @@ MINTB_API int mintb_linear_dgrad(const void* dz, const void* w, const void* dz2,
 MINTB_API int mintb_linear_dgrad_res(const void* dz, const void* w, const void* dz2, const void* w2, void* dx, const void* resid, float beta,
                                      int M, int N, int K, int N2, int dz_dtype, int w_dtype, float alpha, void* stream, int* dev_status);
 MINTB_API size_t mintb_linear_wgrad_workspace_bytes(int N, int K, int out_dtype);
+/* what that product needs for M tokens: none where it stores its result without an fp32 sum in between */
+MINTB_API size_t mintb_linear_wgrad_needed_bytes(int M, int N, int K, int dz_dtype, int out_dtype);
 MINTB_API int mintb_linear_wgrad(const void* dz, const void* x, void* dw, void* workspace, size_t workspace_bytes, int M, int N,
                                  int K, int dz_dtype, int x_dtype, int out_dtype, float alpha, void* stream, int* dev_status);
 

@@ -523,8 +523,25 @@ extern "C" int mintb_linear_dgrad_res(const void* dz, const void* w, const void*
   return launch_bwd_gemm<kDgrad>(bn, a1, b1, a2, b2, mo, p, tiles, static_cast<cudaStream_t>(stream));
 }
 
+// How a weight gradient is formed.
+struct WgradWay { bool direct; int bn; WgradPlan plan; };
+static WgradWay plan_wgrad_way(int M, int N, int K, bool f8, int out_dtype) {
+  const int epb = f8 ? 128 : 64, sms = sm_count(), n_slabs = (M + epb - 1) / epb;
+  // Uncut, when the tiles over all tokens end before the cut reduction does with its clearing and conversion passes (about 3 us;
+  // the bulk reduction and its order are gone then too): up to about 2000 tokens for the 8M model's matrices.
+  long long direct_cost;
+  const int bn = pick_bwd_tile(N, K, n_slabs, f8, sms, &direct_cost);
+  const int tiles256 = ((N + kBM - 1) / kBM) * ((K + 255) / 256);
+  const WgradPlan plan = plan_wgrad(tiles256, n_slabs, sms);
+  return WgradWay{K % 8 == 0 && direct_cost <= plan.cost * 512 + (out_dtype == MINTB_BF16 ? 6000 : 3500), bn, plan};
+}
+
 extern "C" size_t mintb_linear_wgrad_workspace_bytes(int N, int K, int out_dtype) {
   return out_dtype == MINTB_F32 ? 0 : align256(size_t(N) * K * 4);
+}
+
+extern "C" size_t mintb_linear_wgrad_needed_bytes(int M, int N, int K, int dz_dtype, int out_dtype) {
+  return M <= 0 || N <= 0 || K <= 0 || plan_wgrad_way(M, N, K, is_f8(dz_dtype), out_dtype).direct ? 0 : mintb_linear_wgrad_workspace_bytes(N, K, out_dtype);
 }
 
 extern "C" int mintb_linear_wgrad(const void* dz, const void* x, void* dw, void* workspace, size_t workspace_bytes, int M, int N,
@@ -548,20 +565,17 @@ extern "C" int mintb_linear_wgrad(const void* dz, const void* x, void* dw, void*
     set_error("mintb_linear_wgrad: rows of dz and x must be 16-byte multiples, K a multiple of 4, and the pointers 16-byte aligned");
     return MINTB_EINVAL;
   }
-  const size_t need = mintb_linear_wgrad_workspace_bytes(N, K, out_dtype);
+  const size_t need = mintb_linear_wgrad_needed_bytes(M, N, K, dz_dtype, out_dtype);
   if (need > 0 && (workspace == nullptr || workspace_bytes < need)) {
     set_error("mintb_linear_wgrad: workspace of %zu bytes required, %zu given", need, workspace_bytes);
     return MINTB_EWORKSPACE;
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const int epb = 128 / esz, sms = sm_count(), n_slabs = (M + epb - 1) / epb;
-  // Uncut, when the tiles over all tokens end before the cut reduction does with its clearing and conversion passes (about 3 us;
-  // the bulk reduction and its order are gone then too): up to about 2000 tokens for the 8M model's matrices.
-  long long direct_cost;
-  const int bn = pick_bwd_tile(N, K, n_slabs, f8, sms, &direct_cost);
-  const int tiles256 = ((N + kBM - 1) / kBM) * ((K + 255) / 256);
-  const WgradPlan plan = plan_wgrad(tiles256, n_slabs, sms);
-  const bool direct = K % 8 == 0 && direct_cost <= plan.cost * 512 + (out_dtype == MINTB_BF16 ? 6000 : 3500);
+  const int epb = 128 / esz;
+  const WgradWay way = plan_wgrad_way(M, N, K, f8, out_dtype);
+  const bool direct = way.direct;
+  const int bn = way.bn;
+  const WgradPlan& plan = way.plan;
   float* acc = out_dtype == MINTB_F32 ? static_cast<float*>(dw) : static_cast<float*>(workspace);
   cudaError_t e = direct ? cudaSuccess : cudaMemsetAsync(acc, 0, size_t(N) * K * 4, s);
   if (e != cudaSuccess) { set_error("cudaMemsetAsync: %s", cudaGetErrorString(e)); return MINTB_ECUDA; }

@@ -127,7 +127,7 @@ Tensor wgrad(const Tensor& dz, const Tensor& x, double alpha, at::ScalarType out
   const int64_t M = dz.size(0), N = dz.size(1), K = x.size(1);
   const int odt = dt_code(out, "dw");
   Tensor dw = e.empty({N, K}, out);
-  const size_t bytes = mintb_linear_wgrad_workspace_bytes(N, K, odt);
+  const size_t bytes = mintb_linear_wgrad_needed_bytes(M, N, K, dt_code(dz.scalar_type(), "dz"), odt);
   Tensor ws = e.bytes(bytes);
   check(mintb_linear_wgrad(ptr(dz), ptr(x), ptr(dw), ptr(ws), bytes, M, N, K, dt_code(dz.scalar_type(), "dz"), dt_code(x.scalar_type(), "x"), odt,
                            float(alpha), e.stream, e.status),

@@ -97,7 +97,7 @@ std::tuple<Tensor, OptTensor> LayerPlan::forward(const Tensor& x_in, const OptTe
       }
       check(mintb_lora_operands(w, ptr(delta), ptr(b_all), 7, E, E, lora_r, float(lora_scaling), ptr(merged), ptr(keep_t[kBDiag]), e.stream), "mintb_lora_operands");
       qkv6_op = merged;   // (its first 6E rows)
-      out_op = merged.narrow(0, 6 * E, E);
+      out_op = rows_of(merged, 6 * E, E);
     }
 
     // q, k, v of both pathways, head-major, the self pathway rotated.  Packed: positions without a token are not written, and keys
@@ -206,7 +206,7 @@ variable_list LayerNode::apply(variable_list&& grads) {
     if (!g.defined()) return;
     const Tensor c = as_dtype(g, plan.params[k].scalar_type());
     for (int64_t i = 0; i < n; ++i)
-      if (wants(k + i)) res[k + i + 1] = n == 1 ? c : c.narrow(0, i * E, E);
+      if (wants(k + i)) res[k + i + 1] = n == 1 ? c : rows_of(c, i * E, E);
   };
   auto w_dt = [&](int64_t k) { return plan.params[k].scalar_type() == at::kFloat ? at::kFloat : at::kBFloat16; };
   for (auto& s : weights) s.unpack();   // raises if a weight that the products read again has been written since
@@ -260,9 +260,9 @@ variable_list LayerNode::apply(variable_list&& grads) {
   const int64_t r = plan.lora_r;
   Operand w_out = plan.out, os = plan.qkv_self, oc = plan.qkv_cross;
   if (r > 0) {
-    os.w = s[kMerged].narrow(0, 0, 3 * E);
-    oc.w = s[kMerged].narrow(0, 3 * E, 3 * E);
-    w_out.w = s[kMerged].narrow(0, 6 * E, E);
+    os.w = rows_of(s[kMerged], 0, 3 * E);
+    oc.w = rows_of(s[kMerged], 3 * E, 3 * E);
+    w_out.w = rows_of(s[kMerged], 6 * E, E);
   }
   const bool lora_out = r > 0 && (wants(at.la + 6) || wants(at.lb + 6)), lora_qkv = r > 0 && (any(at.la, 6) || any(at.lb, 6));
   // output projection: its result entered the sum times `add`
@@ -274,7 +274,7 @@ variable_list LayerNode::apply(variable_list&& grads) {
     if (lora_out) {   // dB = s g^T (x A^T), dA = s (g B)^T x
       Product xa;
       xa.x = s[kO];
-      xa.w = s[kARows].narrow(0, 6 * r, r);
+      xa.w = rows_of(s[kARows], 6 * r, r);
       if (wants(at.lb + 6)) give(at.lb + 6, wgrad(go, linear_fwd(xa).first, plan.lora_scaling, at::kBFloat16));
       if (wants(at.la + 6)) give(at.la + 6, wgrad(dgrad(go, plan.params[at.lb + 6], 1.0), s[kO], plan.lora_scaling, at::kBFloat16));
     }
@@ -315,10 +315,10 @@ variable_list LayerNode::apply(variable_list&& grads) {
       }
     }
     if (any(at.la, 6)) {
-      const Tensor gb = dgrad(gs, s[kBDiag].narrow(0, 0, 3 * E), 1.0, gc, s[kBDiag].narrow(0, 3 * E, 3 * E));   // g B of every projection
+      const Tensor gb = dgrad(gs, rows_of(s[kBDiag], 0, 3 * E), 1.0, gc, rows_of(s[kBDiag], 3 * E, 3 * E));   // g B of every projection
       const Tensor da = wgrad(gb, h, plan.lora_scaling, at::kBFloat16);                                        // [n][E]
       for (int i = 0; i < 6; ++i)
-        if (wants(at.la + i)) res[at.la + i + 1] = da.narrow(0, i * r, r);
+        if (wants(at.la + i)) res[at.la + i + 1] = rows_of(da, i * r, r);
     }
   }
   if (mu) {
