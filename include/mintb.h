@@ -340,6 +340,10 @@ MINTB_API int mintb_embed_fwd(const long long* tokens, const void* weight, void*
                               int dtype, int pad_idx, int mask_idx, int token_dropout, float mask_ratio_train, void* stream);
 MINTB_API int mintb_embed_bwd(const long long* tokens, const void* d_out, const float* row_scales, float* d_weight, int B, int T,
                               int E, int V, int dtype, int pad_idx, int mask_idx, int token_dropout, void* stream);
+/* (between the two: mintb_mlm_corrupt, the corruption of that step from its three draws of n values: target[i] (0 / 1) where tokens[i] is none of
+ * cls, eos, pad and u_target[i] < 0.15; out[i] = residue[i] for targets with u_kind[i] > 0.9, mask for u_kind[i] < 0.8, else tokens[i]) */
+MINTB_API int mintb_mlm_corrupt(const long long* tokens, const float* u_target, const float* u_kind, const long long* residue, long long* out,
+                                unsigned char* target, long long n, int cls, int eos, int pad, int mask, void* stream);
 MINTB_API int mintb_masked_ce_fwd(const void* logits, const long long* targets, const unsigned char* mask, float* lse, float* sums,
                                   int N, int ld, int V, void* stream);
 MINTB_API int mintb_masked_ce_bwd(const void* logits, const long long* targets, const unsigned char* mask, const float* lse,

@@ -194,6 +194,20 @@ __global__ void __launch_bounds__(256) masked_ce_bwd_kernel(const __nv_bfloat16*
   }
 }
 
+// The masked-language-model corruption from its three draws: a residue (not one of the special tokens) is a target where
+// u_target < 0.15; a target becomes <mask> where u_kind < 0.8 and the drawn residue where u_kind > 0.9.
+__global__ void __launch_bounds__(256) mlm_corrupt_kernel(const long long* __restrict__ tokens, const float* __restrict__ u_target, const float* __restrict__ u_kind,
+                                                          const long long* __restrict__ residue, long long* __restrict__ out, uint8_t* __restrict__ target,
+                                                          long long n, int cls, int eos, int pad, int mask) {
+  const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const long long t = tokens[i];
+  const bool tg = u_target[i] < 0.15f && t != cls && t != eos && t != pad;
+  const float k = u_kind[i];
+  out[i] = tg && k > 0.9f ? residue[i] : tg && k < 0.8f ? mask : t;
+  target[i] = tg ? 1 : 0;
+}
+
 }  // namespace
 }  // namespace mintb
 
@@ -288,4 +302,16 @@ extern "C" int mintb_masked_ce_bwd(const void* logits, const long long* targets,
   count_launches(1);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? MINTB_OK : el_fail("mintb_masked_ce_bwd launch", e);
+}
+
+extern "C" int mintb_mlm_corrupt(const long long* tokens, const float* u_target, const float* u_kind, const long long* residue, long long* out,
+                                 unsigned char* target, long long n, int cls, int eos, int pad, int mask, void* stream) {
+  if (tokens == nullptr || u_target == nullptr || u_kind == nullptr || residue == nullptr || out == nullptr || target == nullptr || n <= 0 || n > (1ll << 38)) {
+    set_error("mintb_mlm_corrupt: every pointer and a positive size are required");
+    return MINTB_EINVAL;
+  }
+  mlm_corrupt_kernel<<<unsigned((n + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(tokens, u_target, u_kind, residue, out, target, n, cls, eos, pad, mask);
+  count_launches(1);
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? MINTB_OK : el_fail("mintb_mlm_corrupt launch", e);
 }

@@ -53,6 +53,7 @@ PYBIND11_MODULE(_mintb_host, m) {
   m.def("add_layernorm", &add_layernorm, nogil);
   m.def("embed", &embed, nogil);
   m.def("masked_ce", &masked_ce, nogil);
+  m.def("mlm_corrupt", &mlm_corrupt, nogil);
 
   py::class_<Operand>(m, "Operand")
       .def(py::init([](const OptTensor& w, double w_scale, double x_scale, double out_scale, py::object holder) {

@@ -164,8 +164,23 @@ Tensor combine(const Tensor& il_, const Tensor& el_, const Tensor& mask_u8, cons
 }
 
 // ---- plain projection ---------------------------------------------------------------------------------------------------------
+// The products take rows of 16-byte multiples: a weight with other numbers of rows (the vocabulary) gets zero rows appended.
+static Tensor pad_rows(const Tensor& t, int64_t n) {
+  Env e(t);
+  auto shape = t.sizes().vec();
+  shape[0] = n;
+  Tensor out = e.empty(shape, t.scalar_type());
+  const size_t have = t.nbytes(), all = out.nbytes();
+  cudaStream_t s = static_cast<cudaStream_t>(e.stream);
+  C10_CUDA_CHECK(cudaMemcpyAsync(out.data_ptr(), t.data_ptr(), have, cudaMemcpyDeviceToDevice, s));
+  C10_CUDA_CHECK(cudaMemsetAsync(static_cast<char*>(out.data_ptr()) + have, 0, all - have, s));
+  return out;
+}
+
 struct LinearNode : public torch::autograd::Node {
   SavedVariable x, w, z;
+  Tensor padded;      // the weight with its zero rows, where it has any
+  int64_t n = 0;      // its rows without them
   std::vector<int64_t> x_shape;
   at::ScalarType w_dt = at::kBFloat16, b_dt = at::kBFloat16;
   bool has_bias = false;
@@ -174,16 +189,29 @@ struct LinearNode : public torch::autograd::Node {
     if (!grads[0].defined()) return r;
     at::NoGradGuard no_grad;
     const Tensor x2 = rows_of(x.unpack());
-    const Tensor dy = grads[0].reshape({x2.size(0), -1}).contiguous();
+    Tensor dy;
+    if (padded.defined()) {
+      auto shape = x_shape;
+      shape.back() = padded.size(0);
+      dy = at::zeros(shape, x2.options());
+      dy.narrow(-1, 0, n).copy_(grads[0]);
+      dy = dy.view({x2.size(0), -1});
+    } else {
+      dy = grads[0].reshape({x2.size(0), -1}).contiguous();
+    }
     const bool want_db = has_bias && task_should_compute_output(2);
+    const Tensor wt = as_dtype(w.unpack(), at::kBFloat16).contiguous();
     auto [dz, db] = gelu_colsum(dy, z.unpack(), want_db ? std::optional<at::ScalarType>(b_dt) : std::nullopt);
-    if (task_should_compute_output(0)) r[0] = dgrad(dz, as_dtype(w.unpack(), at::kBFloat16).contiguous(), 1.0).view(x_shape);
+    if (task_should_compute_output(0)) r[0] = dgrad(dz, padded.defined() ? padded : wt, 1.0).view(x_shape);
     if (task_should_compute_output(1)) r[1] = as_dtype(wgrad(dz, x2, 1.0, w_dt == at::kFloat ? at::kFloat : at::kBFloat16), w_dt);
     if (want_db) r[2] = db;
+    if (padded.defined())
+      for (int k = 1; k < 3; ++k)
+        if (r[k].defined()) r[k] = rows_of(r[k], 0, n);
     return r;
   }
   void release_variables() override {
-    x.reset_data(); w.reset_data(); z.reset_data();
+    x.reset_data(); w.reset_data(); z.reset_data(); padded.reset();
   }
   std::string name() const override { return "LinearBackward"; }
 };
@@ -200,11 +228,18 @@ Tensor linear(const Tensor& x, const Tensor& w, const OptTensor& bias_, bool gel
     p.bias = bias.defined() ? bias.contiguous() : bias;
     p.gelu = gelu;
     p.save_preact = node != nullptr;
+    const int64_t n = w.size(0), np = (n + 7) / 8 * 8;
+    if (np != n) {
+      p.w = pad_rows(p.w, np);
+      if (bias.defined()) p.bias = pad_rows(p.bias, np);
+      if (node) { node->padded = p.w; node->n = n; }
+    }
     Tensor out;
     std::tie(out, z) = linear_fwd(p);
     auto shape = x.sizes().vec();
-    shape.back() = w.size(0);
+    shape.back() = np;
     y = out.view(shape);
+    if (np != n) y = y.narrow(-1, 0, n);
   }
   if (node) {
     set_history(y, node);
@@ -349,6 +384,17 @@ struct MaskedCeNode : public torch::autograd::Node {
   }
   std::string name() const override { return "MaskedCrossEntropyBackward"; }
 };
+
+std::tuple<Tensor, Tensor> mlm_corrupt(const Tensor& tokens, const Tensor& u_target, const Tensor& u_kind, const Tensor& residue, int64_t cls, int64_t eos, int64_t pad,
+                                       int64_t mask) {
+  Env e(tokens);
+  Tensor out = e.empty(tokens.sizes(), at::kLong), target = e.empty(tokens.sizes(), at::kBool);
+  auto i64 = [](const Tensor& t) { return reinterpret_cast<long long*>(t.data_ptr<int64_t>()); };
+  check(mintb_mlm_corrupt(i64(tokens), fptr(u_target), fptr(u_kind), i64(residue), i64(out), reinterpret_cast<unsigned char*>(target.data_ptr<bool>()), tokens.numel(),
+                          int(cls), int(eos), int(pad), int(mask), e.stream),
+        "mintb_mlm_corrupt");
+  return {out, target};
+}
 
 Tensor masked_ce(const Tensor& logits_, const Tensor& targets_, const Tensor& target_mask) {
   const int64_t B = logits_.size(0), T = logits_.size(1), V = logits_.size(2);

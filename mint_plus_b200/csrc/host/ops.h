@@ -23,6 +23,8 @@ Tensor linear(const Tensor& x, const Tensor& w, const OptTensor& bias, bool gelu
 std::tuple<OptTensor, OptTensor, OptTensor> add_layernorm(const Tensor& x, const OptTensor& r, double a, double b, const OptTensor& gamma, const OptTensor& beta,
                                                           double eps, bool need_s, double quant);
 Tensor embed(const Tensor& tokens, const Tensor& weight, int64_t pad, int64_t mask, bool dropout, double ratio);
+std::tuple<Tensor, Tensor> mlm_corrupt(const Tensor& tokens, const Tensor& u_target, const Tensor& u_kind, const Tensor& residue, int64_t cls, int64_t eos, int64_t pad,
+                                       int64_t mask);   // (corrupted tokens, targets)
 Tensor masked_ce(const Tensor& logits, const Tensor& targets, const Tensor& target_mask);
 
 }  // namespace mintb_host

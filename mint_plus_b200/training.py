@@ -13,8 +13,14 @@ import torch.nn.functional as F
 def mlm_corrupt(tokens: torch.Tensor, cls_idx: int, eos_idx: int, padding_idx: int, mask_idx: int,
                 generator: Optional[torch.Generator] = None) -> Tuple[torch.Tensor, torch.Tensor]:
     """(corrupted tokens, boolean target mask), drawn on the tokens' device."""
-    special = tokens.eq(cls_idx) | tokens.eq(eos_idx) | tokens.eq(padding_idx)
     dev = tokens.device
+    if tokens.is_cuda and tokens.dtype == torch.int64 and tokens.numel() > 0 and torch.get_default_dtype() == torch.float32:
+        # on the GPU: the three draws, in the order below, and one launch for what follows from them (15 otherwise, 170 us of host time)
+        from . import _lib
+        u_target, u_kind = (torch.rand(tokens.shape, device=dev, generator=generator) for _ in range(2))
+        residue = torch.randint(4, 24, tokens.shape, device=dev, generator=generator)
+        return _lib.host().mlm_corrupt(tokens.contiguous(), u_target, u_kind, residue, cls_idx, eos_idx, padding_idx, mask_idx)
+    special = tokens.eq(cls_idx) | tokens.eq(eos_idx) | tokens.eq(padding_idx)
     target = (torch.rand(tokens.shape, device=dev, generator=generator) < 0.15) & ~special
     rand = torch.rand(tokens.shape, device=dev, generator=generator)
     randaa = torch.randint(4, 24, tokens.shape, device=dev, generator=generator)
