@@ -131,14 +131,14 @@ __global__ void __launch_bounds__(kLnWarps * 32, MAXV == 10 ? 4 : (MAXV == 5 ? 6
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int nvec = p.E / 8;
   const float inv_e = 1.f / float(p.E);
-  if (p.gamma != nullptr) {   // (no kernel of this library writes parameters, so they may be read ahead of the wait)
+  ptx::griddep_wait();   // (the parameters too are read behind it: the kernel before may be an optimizer's)
+  ptx::griddep_launch();
+  if (p.gamma != nullptr) {
     for (int i = threadIdx.x; i < p.E; i += kLnWarps * 32) {
       s_gamma[i] = ld_param(p.gamma, p.param_dtype, i);
       s_beta[i] = p.beta != nullptr ? ld_param(p.beta, p.param_dtype, i) : 0.f;
     }
   }
-  ptx::griddep_wait();
-  ptx::griddep_launch();
   __syncthreads();
   for (int row = blockIdx.x * kLnWarps + warp; row < p.rows; row += gridDim.x * kLnWarps) {
     const uint4* xr = reinterpret_cast<const uint4*>(p.x + size_t(row) * p.E);
@@ -274,6 +274,8 @@ __global__ void __launch_bounds__(NW * 32, MINB) add_layernorm_bwd_kernel(LnPara
   const bool live = vi < nvec;
   const float inv_e = 1.f / float(p.E);
   uint64_t gm[4], rg[PARAM ? 4 : 1], rb[PARAM ? 4 : 1];
+  ptx::griddep_wait();
+  ptx::griddep_launch();
 #pragma unroll
   for (int j = 0; j < 4; ++j)
     gm[j] = live ? pk(ld_param(p.gamma, p.param_dtype, vi * 8 + 2 * j), ld_param(p.gamma, p.param_dtype, vi * 8 + 2 * j + 1)) : pk(0.f, 0.f);
@@ -281,8 +283,6 @@ __global__ void __launch_bounds__(NW * 32, MINB) add_layernorm_bwd_kernel(LnPara
 #pragma unroll
     for (int j = 0; j < 4; ++j) rg[j] = rb[j] = pk(0.f, 0.f);
   }
-  ptx::griddep_wait();
-  ptx::griddep_launch();
   const float nb = p.b;
   int parity = 0;
   for (int row0 = blockIdx.x * kLnBwdRows; row0 < p.rows; row0 += gridDim.x * kLnBwdRows, parity ^= 1) {

@@ -226,3 +226,24 @@ def test_add_layernorm_backward_with_frozen_norm_parameters():
         grads.append((x.grad, r.grad))
         assert (norm.weight.grad is None) == frozen
     assert torch.equal(grads[0][0], grads[1][0]) and torch.equal(grads[0][1], grads[1][1])
+
+
+def test_layernorm_sees_parameters_that_the_kernel_before_wrote():
+    """No synchronisation between an in-place update of gamma and beta (a kernel of another library) and the passes that read them."""
+    E, rows = 320, 64
+    torch.manual_seed(0)
+    norm = torch.nn.LayerNorm(E).to(DEV, torch.bfloat16)
+    x = _bf(torch.randn(rows, E, device=DEV)).requires_grad_(True)
+    gy = _bf(torch.randn(rows, E, device=DEV))
+    steps = []
+    for k in range(50):
+        with torch.no_grad():
+            norm.weight.fill_(float(k % 7 + 1))
+            norm.bias.fill_(float(k % 5))
+        _, y = ops.add_layernorm(x, None, 1.0, 0.0, norm, need_s=False)
+        steps.append((k, y.detach(), torch.autograd.grad(y, x, gy)[0]))
+    n = torch.nn.functional.layer_norm(x.detach().float(), (E,))
+    dx = steps[0][2].float()                     # gamma = 1
+    for k, y, g in steps:
+        torch.testing.assert_close(y.float(), n * (k % 7 + 1) + k % 5, rtol=2e-2, atol=4e-2)
+        torch.testing.assert_close(g.float(), dx * (k % 7 + 1), rtol=2e-2, atol=4e-2 * dx.abs().max().item() * (k % 7 + 1))

@@ -1,0 +1,36 @@
+"""Dependent launches, read from the CUDA sources: a kernel that may start beside the one before it reads no global memory ahead of its
+wait."""
+import os
+import re
+
+import pytest
+
+import mint_plus_b200 as M
+
+CSRC = os.path.join(os.path.dirname(os.path.abspath(M.__file__)), "csrc")
+
+
+def kernels():
+    """(file, name, body) of every __global__ function."""
+    for f in sorted(os.listdir(CSRC)):
+        if f.endswith(".cu"):
+            src = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, f)).read())
+            src = re.sub(r"__launch_bounds__\s*\((?:[^()]|\([^()]*\))*\)", "", src)
+            for m in re.finditer(r"__global__\s+void\s+(\w+)\s*\([^;{]*\)\s*\{", src):
+                depth, i = 1, m.end()
+                while depth:
+                    depth += {"{": 1, "}": -1}.get(src[i], 0)
+                    i += 1
+                yield f, m.group(1), src[m.end():i]
+
+
+DEPENDENT = [k for k in kernels() if "griddep_wait()" in k[2]]
+
+
+@pytest.mark.parametrize("file,name,body", DEPENDENT, ids=[k[1] for k in DEPENDENT])
+def test_nothing_is_loaded_before_the_wait(file, name, body):
+    assert not re.search(r"__ldg\(|ld_param\(|ld_f\(|load_bias\(", body[:body.index("griddep_wait()")])
+
+
+def test_the_kernels_were_found():
+    assert {"add_layernorm_fwd_kernel", "add_layernorm_bwd_kernel", "gemm_tc_kernel", "attn_bwd_tc_kernel"} <= {k[1] for k in DEPENDENT}
