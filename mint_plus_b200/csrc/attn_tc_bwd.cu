@@ -764,7 +764,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
       __syncwarp();
       if (lane == 0) mbar_arrive(&plan_empty[m % kPlans]);
     }
-    if (lane == 0) bulk_wait_read_all();   // the reductions have read their staging rows (their additions may still be under way)
+    if (lane == 0) bulk_wait_all();   // the dQ conversion adds nothing to these sums: it has to find them complete (see bulk_wait_all in ptx.cuh)
   } else {
     // ---------------------------------------------------------------- compute warps (lane = key row)
     // 8 warps work on each of the two 64-query halves of a tile: thread = key row x 32 query columns, so that the chain from

@@ -324,7 +324,7 @@ gemm_bwd_kernel(const __grid_constant__ CUtensorMap map_a1, const __grid_constan
       mbar_arrive(&acc_empty[ab]);
       if (++ab == 2) { ab = 0; ab_phase ^= 1; }
     }
-    if (lane == 0) bulk_wait_all();   // (a dependent kernel may already be waiting for this grid)
+    if (lane == 0) bulk_wait_all();   // (the results are in memory before this grid ends: see ptx.cuh)
   }
   tc_fence_before();
   __syncthreads();

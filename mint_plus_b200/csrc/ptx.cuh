@@ -208,7 +208,9 @@ __device__ __forceinline__ void bulk_commit_group() { asm volatile("cp.async.bul
 __device__ __forceinline__ void bulk_wait_read_all() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 // all bulk groups of this thread except the most recent one have finished reading their shared-memory source
 __device__ __forceinline__ void bulk_wait_read_but_one() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
-// all bulk groups of this thread have completed
+// all bulk groups of this thread have completed: what they write is in global memory.  Every kernel of this library whose results leave by
+// bulk stores or reductions ends on this wait, not on the reading one: that the end of a grid drains such operations before a dependent
+// grid's griddepcontrol.wait returns is nowhere promised, and none of them counts on it.
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
 // Untiled bulk copy global -> this CTA's shared memory, completion counted in bytes on `bar`.  Both addresses 16-byte

@@ -1,5 +1,5 @@
 """Dependent launches, read from the CUDA sources: a kernel that may start beside the one before it reads no global memory ahead of its
-wait."""
+wait, and one whose results leave by bulk operations ends when they have arrived."""
 import os
 import re
 
@@ -32,5 +32,15 @@ def test_nothing_is_loaded_before_the_wait(file, name, body):
     assert not re.search(r"__ldg\(|ld_param\(|ld_f\(|load_bias\(", body[:body.index("griddep_wait()")])
 
 
+BULK = [k for k in kernels() if "bulk_commit_group()" in k[2]]
+
+
+@pytest.mark.parametrize("file,name,body", BULK, ids=[k[1] for k in BULK])
+def test_bulk_results_have_arrived_at_the_end(file, name, body):
+    waits = re.findall(r"bulk_wait_\w+\(\)", body)
+    assert waits[-1] == "bulk_wait_all()" and body.rindex("bulk_wait_all()") > body.rindex("bulk_commit_group()")
+
+
 def test_the_kernels_were_found():
+    assert {"attn_bwd_tc_kernel", "gemm_tc_kernel", "gemm_bwd_kernel"} == {k[1] for k in BULK}
     assert {"add_layernorm_fwd_kernel", "add_layernorm_bwd_kernel", "gemm_tc_kernel", "attn_bwd_tc_kernel"} <= {k[1] for k in DEPENDENT}
