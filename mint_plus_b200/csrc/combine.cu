@@ -312,8 +312,9 @@ __global__ void __launch_bounds__(32 * kWarps, 4) combine_fwd_kernel(const T* __
   constexpr int KC = Num<T>::kKeys, NV = Num<T>::kV, NP = Num<T>::kP, LD = D + 8;
   extern __shared__ __align__(16) unsigned char smem[];
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, g = lane / 4, t = lane % 4;
-  const size_t bh = blockIdx.y;
-  const int i0 = blockIdx.x * 16;
+  const unsigned tiles = (n + 15) / 16;
+  const size_t bh = blockIdx.x / tiles;
+  const int i0 = int(blockIdx.x % tiles) * 16;
   il += bh * n * n; el += bh * n * n; mask += size_t(bh / H) * n * n;
   iv += bh * n * D; ev += bh * n * D;
   __nv_bfloat16* sv = reinterpret_cast<__nv_bfloat16*>(smem) + warp * NV * KC * LD;
@@ -441,8 +442,9 @@ __global__ void __launch_bounds__(32 * kWarps, 4) combine_bwd_rows_kernel(const 
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ float red[3][kWarps][16];
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, g = lane / 4, t = lane % 4;
-  const size_t bh = blockIdx.y;
-  const int i0 = blockIdx.x * 16;
+  const unsigned tiles = (n + 15) / 16;
+  const size_t bh = blockIdx.x / tiles;
+  const int i0 = int(blockIdx.x % tiles) * 16;
   il += bh * n * n; el += bh * n * n; mask += size_t(bh / H) * n * n;
   d_il += bh * n * n; d_el += bh * n * n;
   iv += bh * n * D; ev += bh * n * D;
@@ -567,8 +569,9 @@ __global__ void __launch_bounds__(32 * kWarps, D == 64 ? 2 : 4) combine_bwd_valu
   constexpr int KB = values_keys<D>(), NV = Num<T>::kV, NP = Num<T>::kP, LD = D + 8, LP = KB + 8;
   extern __shared__ __align__(16) unsigned char smem[];
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, g = lane / 4, t = lane % 4;
-  const size_t bh = blockIdx.y;
-  const int j0 = blockIdx.x * KB;
+  const unsigned tiles = (n + KB - 1) / KB;
+  const size_t bh = blockIdx.x / tiles;
+  const int j0 = int(blockIdx.x % tiles) * KB;
   il += bh * n * n; el += bh * n * n; mask += size_t(bh / H) * n * n;
   __nv_bfloat16* sp = reinterpret_cast<__nv_bfloat16*>(smem) + warp * (NP * 16 * LP + NV * 16 * LD);
   __nv_bfloat16* sg = sp + NP * 16 * LP;
@@ -666,12 +669,18 @@ cudaError_t need_smem(K kernel, int bytes) {
   return bytes <= 48 * 1024 ? cudaSuccess : cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
 
+// One dimension for tiles and (batch, head) pairs together: a second one would end at 65535 pairs.
+unsigned blocks(int n, int rows, int B, int H) {
+  const size_t all = size_t(n + rows - 1) / rows * B * H;
+  return all <= 0x7fffffffu ? unsigned(all) : 0u;   // (a launch of none is an error)
+}
+
 template <typename T, int D, bool PAIR>
 cudaError_t fwd_t(const void* il, const void* el, const uint8_t* mask, const void* iv, const void* ev, void* out, int B, int H, int n, cudaStream_t s) {
   constexpr int bytes = fwd_smem_bytes<T, D>();
   cudaError_t e = need_smem(combine_fwd_kernel<T, D, PAIR>, bytes);
   if (e != cudaSuccess) return e;
-  combine_fwd_kernel<T, D, PAIR><<<dim3((n + 15) / 16, B * H), 32 * kWarps, bytes, s>>>(
+  combine_fwd_kernel<T, D, PAIR><<<blocks(n, 16, B, H), 32 * kWarps, bytes, s>>>(
       static_cast<const T*>(il), static_cast<const T*>(el), mask, static_cast<const T*>(iv), static_cast<const T*>(ev), static_cast<T*>(out), H, n);
   count_launches(1);
   return cudaGetLastError();
@@ -684,10 +693,10 @@ cudaError_t bwd_t(const void* il, const void* el, const uint8_t* mask, const voi
   cudaError_t e = need_smem(combine_bwd_rows_kernel<T, D, PAIR>, rows_bytes);
   if (e == cudaSuccess) e = need_smem(combine_bwd_values_kernel<T, D, PAIR>, val_bytes);
   if (e != cudaSuccess) return e;
-  combine_bwd_rows_kernel<T, D, PAIR><<<dim3((n + 15) / 16, B * H), 32 * kWarps, rows_bytes, s>>>(
+  combine_bwd_rows_kernel<T, D, PAIR><<<blocks(n, 16, B, H), 32 * kWarps, rows_bytes, s>>>(
       static_cast<const T*>(il), static_cast<const T*>(el), mask, static_cast<const T*>(iv), static_cast<const T*>(ev), static_cast<const T*>(d_out),
       static_cast<T*>(d_il), static_cast<T*>(d_el), stats, H, n);
-  combine_bwd_values_kernel<T, D, PAIR><<<dim3((n + values_keys<D>() - 1) / values_keys<D>(), B * H), 32 * kWarps, val_bytes, s>>>(
+  combine_bwd_values_kernel<T, D, PAIR><<<blocks(n, values_keys<D>(), B, H), 32 * kWarps, val_bytes, s>>>(
       static_cast<const T*>(il), static_cast<const T*>(el), mask, static_cast<const T*>(d_out), stats, static_cast<T*>(d_iv), static_cast<T*>(d_ev), H, n);
   count_launches(2);
   return cudaGetLastError();

@@ -33,3 +33,20 @@ def test_combine_tile_edges(T, D, dtype):
     for a, b in zip((out, *got), (want, *wg)):
         b = b.detach()
         assert (a.float().cpu() - b).norm() <= tol * (b.norm() + 1e-6)
+
+
+def test_combine_more_than_65535_heads():
+    """(batch, head) pairs beyond the 65535 blocks that a second grid dimension takes."""
+    B, H, T, D = 32800, 2, 3, 16
+    g = torch.Generator(DEV).manual_seed(0)
+    il, el = (torch.randn(B, H, T, T, device=DEV, generator=g).requires_grad_() for _ in range(2))
+    iv, ev = (torch.randn(B, H, T, D, device=DEV, generator=g).requires_grad_() for _ in range(2))
+    mask = torch.rand(B, T, T, device=DEV, generator=g) < 0.5
+    d = torch.randn(B, H, T, D, device=DEV, generator=g)
+    out = M.fused_multimer_combine(il, el, mask, iv, ev)
+    got = torch.autograd.grad(out, (il, el, iv, ev), d)
+    m = mask.unsqueeze(1)
+    p = torch.where(m, el, il).softmax(-1)
+    want = (p * ~m) @ iv + (p * m) @ ev
+    for a, b in zip((out, *got), (want, *torch.autograd.grad(want, (il, el, iv, ev), d))):
+        assert (a - b).norm() <= 2e-6 * b.norm()
