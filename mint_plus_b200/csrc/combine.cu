@@ -2,10 +2,11 @@
 //
 // Bound by HBM on the (B,H,T,T) logits, their gradients and the mask; the sums over keys, queries and head dimensions run on
 // the warp-level matrix instruction (16x8x16, bf16 operands, fp32 accumulators), because as scalar loops they and not the
-// memory set the pace (B2 H20 T360 D32 bf16, 47 MB, forward + backward: 996 us with one dot product per lane and key, 75 us so;
-// what remains is the latency of mask -> logits -> products in warps that live for three chunks).
+// memory set the pace (B2 H20 T360 D32 bf16, 47 MB, forward + backward as one step: 1030 us with one dot product per lane and key, 87 us
+// so; 81 with probabilities of two pieces and their exponents rounded ahead of ex2, which shows in bf16 results).  What remains is the
+// latency of mask -> logits -> products in warps that live for three chunks.
 // Operands keep their precision: a value is split into bf16 pieces (v = v0 + v1 + ...; one piece for a bf16 tensor, three for an
-// fp32 one, two / three for the fp32 probabilities) and the products of pieces that matter in fp32 are added, smallest first.
+// fp32 one and for the probabilities, which are fp32 either way) and the products of pieces that matter in fp32 are added, smallest first.
 //
 // A CTA of four warps owns 16 query rows (or one block of keys) and its warps take turns on the chunks of the other axis, each
 // with a private online-softmax state, merged in a fixed order at the end: with T / 16 * B * H CTAs even one short pair fills
@@ -20,8 +21,9 @@ namespace {
 constexpr int kWarps = 4;
 
 template <typename T> struct Num;
-template <> struct Num<__nv_bfloat16> { static constexpr int kV = 1, kP = 2, kKeys = 32; };   // pieces of a tensor / of a probability
-template <> struct Num<float> { static constexpr int kV = 3, kP = 3, kKeys = 32; };
+template <> struct Num<__nv_bfloat16> { static constexpr int kV = 1, kKeys = 32; };   // pieces of a tensor
+template <> struct Num<float> { static constexpr int kV = 3, kKeys = 32; };
+constexpr int kP = 3;   // pieces of a probability: fp32 whatever the tensors are
 
 __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   uint32_t r;
@@ -239,18 +241,6 @@ __device__ __forceinline__ void keep(float (&out)[N][4], const float (&s)[N][4],
     for (int e = 0; e < 4; ++e) out[nt][e] = (sel >> (4 * nt + e)) & 1u ? s[nt][e] : 0.f;
 }
 
-// exp(s - ref), for which bf16 logits take the hardware's exp2 as it is (2 ulp of fp32).
-template <typename T>
-__device__ __forceinline__ float exp_from(float s, float ref) {
-  if constexpr (Num<T>::kV == 1) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"((s - ref) * kLog2e));
-    return y;
-  } else {
-    return expf(s - ref);
-  }
-}
-
 // c += a b summed over the pieces whose product reaches fp32, smallest first.  B fragments of piece `q` come from frag(q).
 template <int NA, int NB, typename F>
 __device__ __forceinline__ void mma_pieces(float (&c)[4], const uint32_t (&a)[NA][4], F frag) {
@@ -309,7 +299,7 @@ constexpr int fwd_smem_bytes() {
 template <typename T, int D, bool PAIR>
 __global__ void __launch_bounds__(32 * kWarps, 4) combine_fwd_kernel(const T* __restrict__ il, const T* __restrict__ el, const uint8_t* __restrict__ mask,
                                                                   const T* __restrict__ iv, const T* __restrict__ ev, T* __restrict__ out, int H, int n) {
-  constexpr int KC = Num<T>::kKeys, NV = Num<T>::kV, NP = Num<T>::kP, LD = D + 8;
+  constexpr int KC = Num<T>::kKeys, NV = Num<T>::kV, NP = kP, LD = D + 8;
   extern __shared__ __align__(16) unsigned char smem[];
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, g = lane / 4, t = lane % 4;
   const unsigned tiles = (n + 15) / 16;
@@ -347,7 +337,7 @@ __global__ void __launch_bounds__(32 * kWarps, 4) combine_fwd_kernel(const T* __
       for (int nt = 0; nt < KC / 8; ++nt)
 #pragma unroll
         for (int e = 2 * h; e < 2 * h + 2; ++e) {
-          s[nt][e] = exp_from<T>(s[nt][e], ref);
+          s[nt][e] = expf(s[nt][e] - ref);
           l[h] += s[nt][e];
         }
     }
@@ -499,7 +489,7 @@ __global__ void __launch_bounds__(32 * kWarps, 4) combine_bwd_rows_kernel(const 
       for (int nt = 0; nt < KC / 8; ++nt)
 #pragma unroll
         for (int e = 2 * h; e < 2 * h + 2; ++e) {
-          const float p = exp_from<T>(s[nt][e], ref);
+          const float p = expf(s[nt][e] - ref);
           l[h] += p;
           dl[h] = fmaf(p, dp[nt][e], dl[h]);
         }
@@ -544,8 +534,8 @@ __global__ void __launch_bounds__(32 * kWarps, 4) combine_bwd_rows_kernel(const 
         const uint32_t in = blk.edge ? (blk.inside >> (4 * nt + 2 * h)) & 3u : 3u;
         if (in == 0) continue;
         const size_t off = size_t(i0 + g + 8 * h) * n + j0 + 8 * nt + 2 * t;
-        const float a = exp_from<T>(s[nt][2 * h], ref[h]) * inv[h] * (dp[nt][2 * h] - delta[h]);
-        const float b = exp_from<T>(s[nt][2 * h + 1], ref[h]) * inv[h] * (dp[nt][2 * h + 1] - delta[h]);
+        const float a = expf(s[nt][2 * h] - ref[h]) * inv[h] * (dp[nt][2 * h] - delta[h]);
+        const float b = expf(s[nt][2 * h + 1] - ref[h]) * inv[h] * (dp[nt][2 * h + 1] - delta[h]);
         st_pair<PAIR>(d_il + off, (x & 1u) ? 0.f : a, (x & 2u) ? 0.f : b, (in & 2u) != 0);
         st_pair<PAIR>(d_el + off, (x & 1u) ? a : 0.f, (x & 2u) ? b : 0.f, (in & 2u) != 0);
       }
@@ -558,7 +548,7 @@ __global__ void __launch_bounds__(32 * kWarps, 4) combine_bwd_rows_kernel(const 
 template <int D> constexpr int values_keys() { return 32; }
 template <typename T, int D>
 constexpr int values_smem_bytes() {
-  constexpr int w = kWarps * (Num<T>::kP * 16 * (values_keys<D>() + 8) + Num<T>::kV * 16 * (D + 8)) * 2, r = 2 * values_keys<D>() * D * 4;
+  constexpr int w = kWarps * (kP * 16 * (values_keys<D>() + 8) + Num<T>::kV * 16 * (D + 8)) * 2, r = 2 * values_keys<D>() * D * 4;
   return w > r ? w : r;
 }
 
@@ -566,7 +556,7 @@ template <typename T, int D, bool PAIR>
 __global__ void __launch_bounds__(32 * kWarps, D == 64 ? 2 : 4) combine_bwd_values_kernel(const T* __restrict__ il, const T* __restrict__ el, const uint8_t* __restrict__ mask,
                                                                          const T* __restrict__ dO, const float* __restrict__ stats, T* __restrict__ d_iv,
                                                                          T* __restrict__ d_ev, int H, int n) {
-  constexpr int KB = values_keys<D>(), NV = Num<T>::kV, NP = Num<T>::kP, LD = D + 8, LP = KB + 8;
+  constexpr int KB = values_keys<D>(), NV = Num<T>::kV, NP = kP, LD = D + 8, LP = KB + 8;
   extern __shared__ __align__(16) unsigned char smem[];
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, g = lane / 4, t = lane % 4;
   const unsigned tiles = (n + KB - 1) / KB;
@@ -600,7 +590,7 @@ __global__ void __launch_bounds__(32 * kWarps, D == 64 ? 2 : 4) combine_bwd_valu
 #pragma unroll
       for (int nt = 0; nt < KB / 8; ++nt)
 #pragma unroll
-        for (int e = 2 * h; e < 2 * h + 2; ++e) s[nt][e] = exp_from<T>(s[nt][e], st.x) * st.y;
+        for (int e = 2 * h; e < 2 * h + 2; ++e) s[nt][e] = expf(s[nt][e] - st.x) * st.y;
     }
 #pragma unroll
     for (int path = 0; path < 2; ++path) {

@@ -50,3 +50,39 @@ def test_combine_more_than_65535_heads():
     want = (p * ~m) @ iv + (p * m) @ ev
     for a, b in zip((out, *got), (want, *torch.autograd.grad(want, (il, el, iv, ev), d))):
         assert (a - b).norm() <= 2e-6 * b.norm()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("far", [False, True])
+def test_combine_keeps_fp32_probabilities(dtype, far):
+    """Sums whose terms cancel to about 1e-5 of their size show an error of the probabilities 1e5 times enlarged, in a bf16 result too.
+    `far`: the keys that carry the values lie 40 and more below the row maximum, where a rounded exponent counts most."""
+    B, H, T, D = 2, 2, 66, 16
+    g = torch.Generator().manual_seed(7)
+    value = torch.ones(T)
+    value[1::2] = -1.0
+    if far:     # two groups at logits -50 and -50 + k/8, with the bf16 value that comes closest to cancelling the first group's
+        off = torch.arange(1, 81).double() / 8
+        miss = (torch.exp(off) * torch.exp(-off).bfloat16().double() - 1).abs()
+        k = miss.argmin()
+        value[1::2] = -torch.exp(-off[k]).bfloat16().float()
+        s = torch.full((B, H, T, T), -50.0)
+        s[..., 1::2] += off[k].float()
+        el = s.clone()
+    else:
+        s, el = (1e-4 * torch.randn(B, H, T, T, generator=g) for _ in range(2))
+    s[..., :2] = el[..., :2] = 0.0
+    value[:2] = 0.0
+    v = value[:, None].expand(B, H, T, D)
+    mask = ((torch.arange(T)[:, None] + torch.arange(T)[None, :] // 2) % 3 == 0).expand(B, T, T)
+    il, el, iv, ev = (t.to(dtype) for t in (s, el, v, v))
+    m = mask.unsqueeze(1)
+    p = torch.where(m, el, il).double().softmax(-1)
+    want = (p * ~m) @ iv.double() + (p * m) @ ev.double()
+    size = p @ iv.double().abs()
+    out = M.fused_multimer_combine(*(t.to(DEV) for t in (il, el, mask, iv, ev))).double().cpu()
+    # a term is off by a few roundings of fp32: all of a group alike (far) 4 x 2^-24 at most, else some 2 x 2^-24 each, 64 of them with
+    # either sign, an eighth of that in the sum; a bf16 result rounds by 2^-9 on top
+    cancel = (want.norm() / size.norm()).item()
+    bound = (4.0 if far else 0.25) * 2.0 ** -24 / cancel + (2.0 ** -9 if dtype == torch.bfloat16 else 0.0)
+    assert (out - want).norm() <= bound * want.norm()
