@@ -289,6 +289,95 @@ __device__ __forceinline__ float quad_sum(float v) {
 // ends as 0 / 0 = NaN, as the softmax of an all -inf row does in PyTorch.
 __device__ __forceinline__ float finite_or_zero(float m) { return m == -INFINITY ? 0.f : m; }
 
+// ------------------------------------------------------------------------------------------------ values that cannot be split
+// Infinities, and finite values that round up to one in bf16, do not survive the split (inf - inf).  A sum that has met one ends up not
+// finite and stays so: it is looked at once, at the end, and a warp that finds such a sum forms its share again in fp32, from the
+// elements that the pathways select.  The walks in pieces pay nothing for it; functions of their own, so that they keep their registers.
+template <int N>
+__device__ __forceinline__ bool all_finite(const float (&c)[N][4]) {
+  float t = 0.f;
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) t = fmaf(c[i][e], 0.f, t);
+  return !__any_sync(0xffffffffu, t != 0.f);   // (a NaN is not 0)
+}
+
+// The matrices of one (batch, head): logits, mask, values, and dO [n][D] or null.
+template <typename T>
+struct Matrices {
+  const T *il, *el;
+  const uint8_t* mask;
+  const T *iv, *ev, *dO;
+  int n;
+  __device__ __forceinline__ bool cross(int i, int j) const { return mask[size_t(i) * n + j] != 0; }
+  __device__ __forceinline__ float p(int i, int j, float ref) const { return expf(ld_f((cross(i, j) ? el : il) + size_t(i) * n + j) - ref); }
+  template <int D>
+  __device__ __forceinline__ float dp(int i, int j) const {
+    const T *a = dO + size_t(i) * D, *b = (cross(i, j) ? ev : iv) + size_t(j) * D;
+    float x = 0.f;
+#pragma unroll 1
+    for (int d = 0; d < D; ++d) x = fmaf(ld_f(a + d), ld_f(b + d), x);
+    return x;
+  }
+};
+
+// Forward: acc[D / 8][4] of this lane over the warp's chunks of KC keys, under the row maxima m.
+template <typename T, int D, int KC>
+__device__ __noinline__ void exact_forward(const Matrices<T> x, int i0, float m0, float m1, float* acc) {
+  const int warp = threadIdx.x / 32, g = threadIdx.x % 32 / 4, t = threadIdx.x % 4;
+  for (int k = 0; k < D / 2; ++k) acc[k] = 0.f;
+  for (int h = 0; h < 2; ++h) {
+    const int i = i0 + g + 8 * h;
+    const float ref = finite_or_zero(h ? m1 : m0);
+    for (int j0 = warp * KC; i < x.n && j0 < x.n; j0 += kWarps * KC)
+      for (int j = j0; j < min(j0 + KC, x.n); ++j) {
+        const float p = x.p(i, j, ref);
+        const T* v = (x.cross(i, j) ? x.ev : x.iv) + size_t(j) * D + 2 * t;
+        for (int d = 0; d < D / 8; ++d)
+          for (int e = 0; e < 2; ++e) acc[4 * d + 2 * h + e] = fmaf(p, ld_f(v + 8 * d + e), acc[4 * d + 2 * h + e]);
+      }
+  }
+}
+
+// Backward, this lane's elements of the warp's chunks (rows g and g + 8, columns 8 nt + 2 t and the next): sum_j p dP of row h ...
+template <typename T, int D, int KC>
+__device__ __noinline__ float exact_delta(const Matrices<T> x, int i0, int h, float m) {
+  const int warp = threadIdx.x / 32, g = threadIdx.x % 32 / 4, t = threadIdx.x % 4, i = i0 + g + 8 * h;
+  float sum = 0.f;
+  for (int j0 = warp * KC; i < x.n && j0 < x.n; j0 += kWarps * KC)
+    for (int j = j0 + 2 * t; j < min(j0 + KC, x.n); j += j % 2 ? 7 : 1) sum = fmaf(x.p(i, j, finite_or_zero(m)), x.template dp<D>(i, j), sum);
+  return sum;
+}
+// ... and dS = p / l (dP - delta).
+template <typename T, int D, int KC>
+__device__ __noinline__ void exact_logit_grads(const Matrices<T> x, int i0, int h, float ref, float inv, float delta, T* d_il, T* d_el) {
+  const int warp = threadIdx.x / 32, g = threadIdx.x % 32 / 4, t = threadIdx.x % 4, i = i0 + g + 8 * h;
+  for (int j0 = warp * KC; i < x.n && j0 < x.n; j0 += kWarps * KC)
+    for (int j = j0 + 2 * t; j < min(j0 + KC, x.n); j += j % 2 ? 7 : 1) {
+      const float ds = x.p(i, j, ref) * inv * (x.template dp<D>(i, j) - delta);
+      st_f(d_il + size_t(i) * x.n + j, x.cross(i, j) ? 0.f : ds);
+      st_f(d_el + size_t(i) * x.n + j, x.cross(i, j) ? ds : 0.f);
+    }
+}
+
+// Backward: acc[pathway][KB / 16][D / 8][4] of this lane over the warp's rows.
+template <typename T, int D, int KB>
+__device__ __noinline__ void exact_value_grads(const Matrices<T> x, int j0, const float* stats, float* acc) {
+  const int warp = threadIdx.x / 32, g = threadIdx.x % 32 / 4, t = threadIdx.x % 4;
+  for (int k = 0; k < KB * D / 16; ++k) acc[k] = 0.f;
+  for (int i0 = warp * 16; i0 < x.n; i0 += kWarps * 16)
+    for (int i = i0; i < min(i0 + 16, x.n); ++i)
+      for (int k = 0; k < KB / 8; ++k) {
+        const int j = j0 + 8 * k + g;
+        if (j >= x.n) break;
+        const float p = x.p(i, j, stats[2 * i]) * stats[2 * i + 1];
+        float* a = acc + ((x.cross(i, j) ? KB / 16 : 0) + k / 2) * D / 2 + 2 * (k % 2);
+        for (int d = 0; d < D / 8; ++d)
+          for (int e = 0; e < 2; ++e) a[4 * d + e] = fmaf(p, ld_f(x.dO + size_t(i) * D + 8 * d + 2 * t + e), a[4 * d + e]);
+      }
+}
+
 // ------------------------------------------------------------------------------------------------ forward
 template <typename T, int D>
 constexpr int fwd_smem_bytes() {
@@ -388,6 +477,14 @@ __global__ void __launch_bounds__(32 * kWarps, 4) combine_fwd_kernel(const T* __
         for (int e = 0; e < 4; ++e) acc[d][e] += part[d][e];
     }
   }
+  if (!all_finite(acc)) {
+    float again[D / 2];
+    exact_forward<T, D, KC>({il, el, mask, iv, ev, nullptr, n}, i0, m[0], m[1], again);
+#pragma unroll
+    for (int d = 0; d < D / 8; ++d)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[d][e] = again[4 * d + e];
+  }
   // merge the four warps' states: [warp][16][D] accumulators, then maxima and row sums
   l[0] = quad_sum(l[0]);
   l[1] = quad_sum(l[1]);
@@ -437,11 +534,11 @@ __global__ void __launch_bounds__(32 * kWarps, 4) combine_bwd_rows_kernel(const 
   const int i0 = int(blockIdx.x % tiles) * 16;
   il += bh * n * n; el += bh * n * n; mask += size_t(bh / H) * n * n;
   d_il += bh * n * n; d_el += bh * n * n;
-  iv += bh * n * D; ev += bh * n * D;
+  iv += bh * n * D; ev += bh * n * D; dO += bh * n * D;
   __nv_bfloat16* sv = reinterpret_cast<__nv_bfloat16*>(smem) + warp * NV * KC * LD;
 
   uint32_t go[D / 16][NV][4];
-  stage<T, D, 16>(dO + bh * n * D, i0, n, sv, lane);
+  stage<T, D, 16>(dO, i0, n, sv, lane);
   staged();
 #pragma unroll
   for (int k = 0; k < D / 16; ++k)
@@ -495,6 +592,13 @@ __global__ void __launch_bounds__(32 * kWarps, 4) combine_bwd_rows_kernel(const 
         }
     }
   }
+  // (values of one piece are not split)
+  const Matrices<T> x{il, el, mask, iv, ev, dO, n};
+  const bool exact = NV > 1 && __any_sync(0xffffffffu, dl[0] * 0.f != 0.f || dl[1] * 0.f != 0.f);
+  if (exact) {
+    dl[0] = exact_delta<T, D, KC>(x, i0, 0, m[0]);
+    dl[1] = exact_delta<T, D, KC>(x, i0, 1, m[1]);
+  }
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     l[h] = quad_sum(l[h]);
@@ -522,6 +626,10 @@ __global__ void __launch_bounds__(32 * kWarps, 4) combine_bwd_rows_kernel(const 
       stats[(bh * n + i0 + r) * 2] = ref[h];
       stats[(bh * n + i0 + r) * 2 + 1] = inv[h];
     }
+  }
+  if (exact) {
+    for (int h = 0; h < 2; ++h) exact_logit_grads<T, D, KC>(x, i0, h, h ? ref[1] : ref[0], h ? inv[1] : inv[0], h ? delta[1] : delta[0], d_il, d_el);
+    return;
   }
   for (int j0 = warp * KC; j0 < n; j0 += kWarps * KC) {
     float s[KC / 8][4], dp[KC / 8][4];
@@ -563,6 +671,7 @@ __global__ void __launch_bounds__(32 * kWarps, D == 64 ? 2 : 4) combine_bwd_valu
   const size_t bh = blockIdx.x / tiles;
   const int j0 = int(blockIdx.x % tiles) * KB;
   il += bh * n * n; el += bh * n * n; mask += size_t(bh / H) * n * n;
+  dO += bh * n * D; stats += bh * n * 2;
   __nv_bfloat16* sp = reinterpret_cast<__nv_bfloat16*>(smem) + warp * (NP * 16 * LP + NV * 16 * LD);
   __nv_bfloat16* sg = sp + NP * 16 * LP;
 
@@ -580,13 +689,13 @@ __global__ void __launch_bounds__(32 * kWarps, D == 64 ? 2 : 4) combine_bwd_valu
     float s[KB / 8][4];
     Block<T, KB, PAIR> blk;
     __syncwarp();
-    stage<T, D, 16>(dO + bh * n * D, i0, n, sg, lane);
+    stage<T, D, 16>(dO, i0, n, sg, lane);
     blk.load_mask(mask, i0, j0, n, lane);
     blk.load_logits(il, el, i0, j0, n, lane, s);
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       const int i = i0 + g + 8 * h;
-      const float2 st = i < n ? *reinterpret_cast<const float2*>(stats + (bh * n + i) * 2) : make_float2(0.f, 0.f);
+      const float2 st = i < n ? *reinterpret_cast<const float2*>(stats + size_t(i) * 2) : make_float2(0.f, 0.f);
 #pragma unroll
       for (int nt = 0; nt < KB / 8; ++nt)
 #pragma unroll
@@ -628,6 +737,23 @@ __global__ void __launch_bounds__(32 * kWarps, D == 64 ? 2 : 4) combine_bwd_valu
         }
       }
     }
+  }
+  bool finite = true;
+#pragma unroll
+  for (int p = 0; p < 2; ++p)
+#pragma unroll
+    for (int k = 0; k < KB / 16; ++k) finite = all_finite(acc[p][k]) && finite;
+  if (!finite) {
+    float again[KB * D / 16];
+    exact_value_grads<T, D, KB>({il, el, mask, nullptr, nullptr, dO, n}, j0, stats, again);
+#pragma unroll
+    for (int p = 0; p < 2; ++p)
+#pragma unroll
+      for (int k = 0; k < KB / 16; ++k)
+#pragma unroll
+        for (int d = 0; d < D / 8; ++d)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) acc[p][k][d][e] = again[((p * KB / 16 + k) * D / 8 + d) * 4 + e];
   }
   __syncthreads();
   float* red = reinterpret_cast<float*>(smem);   // [2][KB][D], the warps' sums added in turn

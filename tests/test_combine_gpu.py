@@ -86,3 +86,44 @@ def test_combine_keeps_fp32_probabilities(dtype, far):
     cancel = (want.norm() / size.norm()).item()
     bound = (4.0 if far else 0.25) * 2.0 ** -24 / cancel + (2.0 ** -9 if dtype == torch.bfloat16 else 0.0)
     assert (out - want).norm() <= bound * want.norm()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("D", [16, 32, 64])
+@pytest.mark.parametrize("value", [float("inf"), -3.4e38])
+def test_combine_infinite_and_largest_values(dtype, D, value):
+    """Infinities and values at the end of the range reach the rows and dimensions that they belong to, as sums in fp32 have them."""
+    B, H, T = 1, 2, 70
+    g = torch.Generator().manual_seed(D)
+    il, el = (torch.randn(B, H, T, T, generator=g).to(dtype) for _ in range(2))
+    iv, ev, d = (torch.randn(B, H, T, D, generator=g).to(dtype) for _ in range(3))
+    mask = torch.rand(B, T, T, generator=g) < 0.5
+    mask[:, :20] = False
+    iv[0, 0, 3, 5] = value
+    ev[0, 1, T - 1, D - 1] = value
+    d[0, 1, 33, 2] = value
+
+    def exact(il, el, iv, ev, d):
+        # sums over the selected elements alone, as the operator defines them
+        m = mask.unsqueeze(1)
+        p = torch.where(m, el, il).softmax(-1)
+        sel = lambda a, keep: torch.where(keep.unsqueeze(-1), a, torch.zeros((), dtype=a.dtype))
+        v = torch.where(m.unsqueeze(-1), ev.unsqueeze(-3), iv.unsqueeze(-3))              # (B,H,T,T,D): the value that (i, j) takes
+        out = (p.unsqueeze(-1) * v).sum(-2)
+        dp = (d.unsqueeze(-2) * v).sum(-1)
+        ds = p * (dp - (p * dp).sum(-1, keepdim=True))
+        g = p.unsqueeze(-1) * d.unsqueeze(-2)
+        return [out, ds.masked_fill(m, 0.0), ds.masked_fill(~m, 0.0), sel(g, (~m).expand_as(p)).sum(-3), sel(g, m.expand_as(p)).sum(-3)]
+
+    want = exact(*[t.float() for t in (il, el, iv, ev, d)])
+    leaves = [t.to(DEV).requires_grad_() for t in (il, el, iv, ev)]
+    out = M.fused_multimer_combine(leaves[0], leaves[1], mask.to(DEV), leaves[2], leaves[3])
+    got = [out, *torch.autograd.grad(out, leaves, d.to(DEV))]
+    for a, b in zip(got, want):
+        b = b.to(dtype).float()                                                            # (beyond bf16's range: infinite there)
+        a = a.float().cpu()
+        assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a.isinf(), b.isinf()) and torch.equal(a[a.isinf()], b[b.isinf()])
+        f = b.isfinite()
+        big = b.abs() > 1e30
+        assert torch.allclose(a[f & big], b[f & big], rtol=1e-2)
+        assert (a[f & ~big] - b[f & ~big]).norm() <= (2e-6 if dtype == torch.float32 else 6e-3) * b[f & ~big].norm()
