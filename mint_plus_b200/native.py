@@ -19,11 +19,14 @@ from . import ops
 
 class _Plan:
     """The native plan of a layer and what it was made from: `slots` are (dict, key, object) that must still hold that object,
-    `tensors` (tensor, address, version) whose contents were copied into an operand."""
+    `tensors` (tensor, address, version) whose contents were copied into an operand, `fixed` the layer's own settings.  The layer keeps
+    its plan and the plan nothing of the layer's own dictionary: a dropped layer dies at once, weights and copies with it."""
 
-    __slots__ = ("native", "slots", "tensors", "can_grad", "x_scale", "rot")
+    __slots__ = ("native", "slots", "tensors", "fixed", "can_grad", "x_scale", "rot")
 
-    def valid(self) -> bool:
+    def valid(self, fixed) -> bool:
+        if self.fixed != fixed:
+            return False
         for d, k, o in self.slots:
             if d.get(k) is not o:
                 return False
@@ -49,7 +52,7 @@ def _attn_mods(attn):
     return None if any(m is None for m in mods) else mods
 
 
-def _build(layer, mu: bool, keep: float, add: float) -> Optional[_Plan]:
+def _build(layer, mu: bool, fixed) -> Optional[_Plan]:
     from . import modules_plus as mp
     from .lora import LoRALinear
     from .mu_scaling import Fp8Linear, fused_fp8_weight
@@ -83,10 +86,11 @@ def _build(layer, mu: bool, keep: float, add: float) -> Optional[_Plan]:
            or (m.bias is not None and (m.bias.dtype not in params_dt or not m.bias.is_contiguous())) for m in linears):
         return None
     E, H = sa.embed_dim, sa.num_heads
+    keep, add, sqrt_softmax = fixed
     bias_s, bias_c = ms[0].bias is not None, mc[0].bias is not None
 
     p = _Plan()
-    p.slots, p.tensors = [], []
+    p.slots, p.tensors, p.fixed = [], [], fixed
     for m, names in ((layer, ("self_attn", "multimer_attn", "feed_forward", "final_layer_norm") + (() if mu else ("self_attn_layer_norm",))),
                      (sa, _ATTN_CHILDREN), (ma, _ATTN_CHILDREN), (ff, ("fc1", "fc2"))):
         p.slots += [(m._modules, n, m._modules.get(n)) for n in names]
@@ -156,11 +160,10 @@ def _build(layer, mu: bool, keep: float, add: float) -> Optional[_Plan]:
         params += [m.weight, m.bias]
     if adapters is not None:
         params += [m.lora_A for m in adapters] + [m.lora_B for m in adapters]
-    p.native = L.host().LayerPlan(mu=mu, fp8=fp8, sqrt_softmax=bool(layer._use_sqrt_softmax), H=H, D=sa.head_dim, scale=sa.scaling, keep=keep, add=add,
+    p.native = L.host().LayerPlan(mu=mu, fp8=fp8, sqrt_softmax=sqrt_softmax, H=H, D=sa.head_dim, scale=sa.scaling, keep=keep, add=add,
                                   eps1=norms[0].eps, eps2=norms[-1].eps, params=params, n_self=len(ms), n_cross=len(mc), qkv_self=op_s, qkv_cross=op_c,
                                   out=o, fc1=f1, fc2=f2, qkv6=qkv6, bias6=bias6, bias_self=b_self, bias_cross=b_cross,
                                   lora_r=adapters[0].r if adapters else 0, lora_scaling=adapters[0].scaling if adapters else 1.0)
-    p.slots += [(layer.__dict__, k, layer.__dict__.get(k)) for k in ("_use_sqrt_softmax", "_tau_f")]
     p.rot = sa.rot_emb
     return p
 
@@ -171,10 +174,11 @@ def run_layer(layer, x, chain_mask, padding_mask, chain_ids, pack, *, mu: bool, 
     if not (x.is_cuda and x.dtype == torch.bfloat16 and layer.use_multimer and layer._use_fused_multi_pathway and mp.FUSE_OUT_RESIDUAL):
         return None
     plan = layer.__dict__.get("_native_plan")
-    if plan is None or not plan.valid():
+    fixed = (keep, add, bool(layer._use_sqrt_softmax))
+    if plan is None or not plan.valid(fixed):
         if layer.self_attn.head_dim not in (16, 32, 64):
             return None
-        plan = _build(layer, mu, keep, add)
+        plan = _build(layer, mu, fixed)
         layer.__dict__["_native_plan"] = plan
         if plan is None:
             return None

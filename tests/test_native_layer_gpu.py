@@ -1,6 +1,8 @@
 """The layers as the C++ host side runs them (one autograd node over the launches) against the same layers composed from the
 operators: values, input and parameter gradients, for every kind of layer it serves; operands follow the parameters."""
 import copy
+import gc
+import weakref
 
 import pytest
 import torch
@@ -141,3 +143,23 @@ def test_checkpointed_layer_gives_the_same_gradients():
     y, _ = checkpoint(layer, xr, use_reentrant=False, self_attn_padding_mask=pad, chain_ids=ids)
     y.backward(gy)
     close([y.detach(), xr.grad] + [p.grad for p in layer.parameters()], want, 1e-3)
+
+
+def values(layer, x, ids, pad):
+    with torch.no_grad():
+        return layer(x, self_attn_padding_mask=pad, chain_ids=ids)[0]
+
+
+@pytest.mark.parametrize("kind", ["base", "plus", "mu_fp8", "lora"])
+def test_a_dropped_layer_frees_its_weights_at_once(kind):
+    layer = make_layer(kind)
+    values(layer, *batch(64, 2))
+    assert layer._native_plan is not None
+    gc.collect()
+    gc.disable()
+    try:
+        w = weakref.ref(layer.feed_forward.fc1.weight)
+        del layer
+        assert w() is None
+    finally:
+        gc.enable()
