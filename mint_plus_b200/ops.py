@@ -8,6 +8,7 @@ import weakref
 from typing import Optional, Tuple
 
 import torch
+from torch.utils.weak import WeakIdKeyDictionary
 
 from . import _lib as L
 
@@ -126,8 +127,8 @@ def cached_mask_meta(chain_mask: torch.Tensor, key_padding_mask: Optional[torch.
 
 
 # ----------------------------------------------------------------------------------------------- RoPE tables
-_rope_cache = {}
-_ROPE_TABLES = 256
+_rope_cache = WeakIdKeyDictionary()      # inv_freq buffer -> its tables; they go when it goes
+_rope_default = {}                       # (D, device) -> the tables of the default frequencies
 
 
 def default_inv_freq(D: int, device) -> torch.Tensor:
@@ -137,13 +138,15 @@ def default_inv_freq(D: int, device) -> torch.Tensor:
 
 def rope_tables(T: int, D: int, device,
                 inv_freq: Optional[torch.Tensor] = None) -> Tuple[torch.Tensor, torch.Tensor, Optional[torch.Tensor]]:
-    """(cos, sin, inv_freq): the cos/sin tables (T, D/2) fp32 on `device`, cached per (T, D, device, inv_freq contents); the
-    third entry is the caller's inv_freq (None for the default frequencies), held so that the cache key stays valid."""
+    """(cos, sin, inv_freq): the cos/sin tables (T, D/2) fp32 on `device`, kept with the buffer `inv_freq` (the default frequencies
+    without one) for as long as it lives and holds what they were made from."""
     device = torch.device(device)
-    key = (D, device.index, inv_freq.data_ptr() if inv_freq is not None else 0, inv_freq._version if inv_freq is not None else 0)
-    hit = _rope_cache.get(key)
-    if hit is not None and T in hit[3]:
-        return hit[3][T]
+    made_from = (D, device.index) if inv_freq is None else (D, device.index, inv_freq.data_ptr(), inv_freq._version)
+    hit = _rope_default.get(made_from) if inv_freq is None else _rope_cache.get(inv_freq)
+    if hit is not None and hit[3] != made_from:
+        hit = None
+    if hit is not None and T in hit[2]:
+        return (*hit[2][T], inv_freq)
     if hit is None or T > hit[0].shape[0]:
         # row t depends on t alone, so the table of the longest length seen so far serves the shorter ones
         rows = (T + 255) // 256 * 256
@@ -154,13 +157,15 @@ def rope_tables(T: int, D: int, device,
         sin = torch.empty_like(cos)
         with _on(device):
             L.check(L.lib().mintb_rope_tables(_ptr(inv), _ptr(cos), _ptr(sin), rows, D, _stream()), "rope_tables")
-        while len(_rope_cache) >= _ROPE_TABLES:      # every layer of a model brings its own inv_freq buffer
-            _rope_cache.pop(next(iter(_rope_cache)), None)
-        hit = _rope_cache[key] = (cos, sin, inv_freq, {})   # keeps the buffer alive so its address cannot be reused under this key
-    if len(hit[3]) >= 64:
-        hit[3].clear()
-    hit[3][T] = out = (hit[0][:T], hit[1][:T], inv_freq)
-    return out
+        hit = (cos, sin, {}, made_from)
+        if inv_freq is None:
+            _rope_default[made_from] = hit
+        else:
+            _rope_cache[inv_freq] = hit
+    if len(hit[2]) >= 64:
+        hit[2].clear()
+    hit[2][T] = (hit[0][:T], hit[1][:T])
+    return (*hit[2][T], inv_freq)
 
 
 # ----------------------------------------------------------------------------------------------- attention

@@ -163,3 +163,18 @@ def test_a_dropped_layer_frees_its_weights_at_once(kind):
         assert w() is None
     finally:
         gc.enable()
+
+
+def test_rotary_tables_live_as_long_as_their_frequencies():
+    inv = ops.default_inv_freq(32, DEV)
+    before = torch.cuda.memory_allocated()
+    tabs = ops.rope_tables(300, 32, DEV, inv)
+    assert ops.rope_tables(200, 32, DEV, inv)[0].data_ptr() == tabs[0].data_ptr()
+    longer = ops.rope_tables(600, 32, DEV, inv)
+    torch.testing.assert_close(longer[0][:300], tabs[0])
+    torch.testing.assert_close(longer[1], torch.outer(torch.arange(600, device=DEV).float(), inv).sin(), rtol=0, atol=1e-4)
+    assert torch.cuda.memory_allocated() > before
+    inv.mul_(0.5)
+    torch.testing.assert_close(ops.rope_tables(9, 32, DEV, inv)[1], torch.outer(torch.arange(9, device=DEV).float(), inv).sin(), rtol=0, atol=1e-6)
+    del tabs, longer, inv
+    assert torch.cuda.memory_allocated() < before
