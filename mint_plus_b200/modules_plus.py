@@ -215,6 +215,11 @@ class _TwoPathwayLayer(nn.Module):
         return self._multimer_attention_plus(x, chain_mask, padding_mask)
 
 
+# what the C++ host side computes in their place (native.py): a layer whose methods are others runs through them
+OWN_CODE = frozenset((VanillaFeedForward.forward, _TwoPathwayLayer._multimer_attention_superfused, _TwoPathwayLayer._multimer_attention_plus,
+                      MultiHeadAttention.project_qkv_4d, MultiHeadAttention._project_qkv, MultimerAttention.project_qkv_4d))
+
+
 class _PreLnLayer(_TwoPathwayLayer):
     """x -> LN -> attention -> +residual -> LN -> FFN -> +residual (modules.py:179-195, modules_plus.py:72-96)."""
 

@@ -2,7 +2,8 @@
 and backward pass take, formed once and kept on the layer until one of them changes.
 
 A layer is served here when it is what the builders make: bf16 activations on the GPU, nn.Linear projections with bf16 weights
-(with or without LoRA adapters on a frozen base) or Fp8Linear ones throughout, LayerNorms with parameters, the fused attention.
+(with or without LoRA adapters on a frozen base) or Fp8Linear ones throughout, LayerNorms with parameters, the fused attention, a
+VanillaFeedForward, and none of the methods that this file stands in for overridden.
 Everything else (wrapped projections, mixed kinds) stays on the modules' own path; plain fp32 layers have a short one of their own at
 the end of this file.
 """
@@ -52,13 +53,18 @@ def _attn_mods(attn):
     return None if any(m is None for m in mods) else mods
 
 
+def _own(mp, obj, *names) -> bool:
+    """These methods of `obj` are the package's, overridden neither in a subclass nor on the instance nor patched."""
+    return all(getattr(getattr(obj, n, None), "__func__", None) in mp.OWN_CODE for n in names)
+
+
 def _build(layer, mu: bool, fixed) -> Optional[_Plan]:
     from . import modules_plus as mp
     from .lora import LoRALinear
     from .mu_scaling import Fp8Linear, fused_fp8_weight
     sa, ma, ff = layer.self_attn, layer.multimer_attn, layer.feed_forward
     ms, mc = _attn_mods(sa), _attn_mods(ma)
-    if ms is None or mc is None or sa._modules.get("out_proj") is None:
+    if ms is None or mc is None or sa._modules.get("out_proj") is None or type(ff) is not mp.VanillaFeedForward:
         return None
     one = [sa.out_proj, ff.fc1, ff.fc2]
     adapters = None
@@ -171,7 +177,8 @@ def _build(layer, mu: bool, fixed) -> Optional[_Plan]:
 def run_layer(layer, x, chain_mask, padding_mask, chain_ids, pack, *, mu: bool, keep: float, add: float, next_quant=None):
     """The layer's result for x (T,B,E) (or the packed rows of one), or None when the layer is not served here."""
     from . import modules_plus as mp
-    if not (x.is_cuda and x.dtype == torch.bfloat16 and layer.use_multimer and layer._use_fused_multi_pathway and mp.FUSE_OUT_RESIDUAL):
+    if not (x.is_cuda and x.dtype == torch.bfloat16 and layer.use_multimer and layer._use_fused_multi_pathway and mp.FUSE_OUT_RESIDUAL and
+            _own(mp, layer, "_multimer_attention_superfused") and _own(mp, layer.feed_forward, "forward")):
         return None
     plan = layer.__dict__.get("_native_plan")
     fixed = (keep, add, bool(layer._use_sqrt_softmax))
@@ -213,6 +220,9 @@ def run_layer_f32(layer, x, chain_mask, padding_mask, chain_ids):
         return None
     sa, ma, ff = layer.self_attn, layer.multimer_attn, layer.feed_forward
     if type(ff) is not mp.VanillaFeedForward or sa.head_dim not in (16, 32, 64) or x.numel() == 0:
+        return None
+    if not (_own(mp, layer, "_multimer_attention_plus", "_multimer_attention_superfused") and _own(mp, ff, "forward") and
+            all(_own(mp, a, "project_qkv_4d") and (not hasattr(a, "_project_qkv") or _own(mp, a, "_project_qkv")) for a in (sa, ma))):
         return None
     projections = [m for a in (sa, ma) for m in (_attn_mods(a) or [None])]
     if not (all(m is not None and _plain(m, torch.nn.Linear) for m in (*projections, sa.out_proj, ff.fc1, ff.fc2)) and ff.fc1.out_features % 4 == 0 and

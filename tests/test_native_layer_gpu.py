@@ -178,3 +178,54 @@ def test_rotary_tables_live_as_long_as_their_frequencies():
     torch.testing.assert_close(ops.rope_tables(9, 32, DEV, inv)[1], torch.outer(torch.arange(9, device=DEV).float(), inv).sin(), rtol=0, atol=1e-6)
     del tabs, longer, inv
     assert torch.cuda.memory_allocated() < before
+
+
+def equal_to_composed(layer, x, ids, pad, monkeypatch, tol=1e-2):
+    got = values(layer, x, ids, pad)
+    with monkeypatch.context() as m:
+        m.setattr(native, "run_layer", lambda *a, **k: None)
+        m.setattr(native, "run_layer_f32", lambda *a, **k: None)
+        want = values(layer, x, ids, pad)
+    assert (got.float() - want.float()).norm() <= tol * want.float().norm()
+    return got
+
+
+class _Relu(torch.nn.Module):
+    def __init__(self, ff):
+        super().__init__()
+        self.fc1, self.fc2 = ff.fc1, ff.fc2
+
+    def forward(self, x):
+        return self.fc2(torch.relu(self.fc1(x)))
+
+
+class _Doubled(M.VanillaFeedForward):
+    def forward(self, x):
+        return 2 * super().forward(x)
+
+
+class _Attn(M.TransformerLayer_MINT_plus):
+    def _multimer_attention_superfused(self, x, *a, residual=None, **k):
+        y, _ = super()._multimer_attention_superfused(x, *a, residual=residual, **k)
+        return 3 * y, None
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("what", ["relu", "subclass", "instance", "attention"])
+def test_modules_that_compute_something_else_keep_their_results(what, dtype, monkeypatch):
+    layer = make_layer("plus").to(dtype)
+    x, ids, pad = batch(70, 2)
+    x = x.to(dtype)
+    values(layer, x, ids, pad)                      # a layer that has been served before
+    plain = values(layer, x, ids, pad)
+    if what == "relu":
+        layer.feed_forward = _Relu(layer.feed_forward)
+    elif what == "subclass":
+        layer.feed_forward.__class__ = _Doubled
+    elif what == "instance":
+        own = layer.feed_forward.forward
+        layer.feed_forward.forward = lambda h: 2 * own(h)
+    else:
+        layer.__class__ = _Attn
+    got = equal_to_composed(layer, x, ids, pad, monkeypatch)
+    assert (got - plain).abs().max() > 0.1
