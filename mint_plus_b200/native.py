@@ -13,6 +13,7 @@ from typing import Optional
 
 import torch
 from torch import nn
+from torch.nn.modules.module import _has_any_global_hook as _any_global_hook
 
 from . import _lib as L
 from . import ops
@@ -20,10 +21,11 @@ from . import ops
 
 class _Plan:
     """The native plan of a layer and what it was made from: `slots` are (dict, key, object) that must still hold that object,
-    `tensors` (tensor, address, version) whose contents were copied into an operand, `fixed` the layer's own settings.  The layer keeps
+    `tensors` (tensor, address, version) whose contents were copied into an operand, `fixed` the layer's own settings; `hooks` are the hook
+    dictionaries of the modules that would be called otherwise: while one is filled the layer runs through the modules.  The layer keeps
     its plan and the plan nothing of the layer's own dictionary: a dropped layer dies at once, weights and copies with it."""
 
-    __slots__ = ("native", "slots", "tensors", "fixed", "can_grad", "x_scale", "rot")
+    __slots__ = ("native", "slots", "tensors", "fixed", "hooks", "can_grad", "x_scale", "rot")
 
     def valid(self, fixed) -> bool:
         if self.fixed != fixed:
@@ -56,6 +58,10 @@ def _attn_mods(attn):
 def _own(mp, obj, *names) -> bool:
     """These methods of `obj` are the package's, overridden neither in a subclass nor on the instance nor patched."""
     return all(getattr(getattr(obj, n, None), "__func__", None) in mp.OWN_CODE for n in names)
+
+
+def _hooks(mod):
+    return [mod._forward_hooks, mod._forward_pre_hooks, mod._backward_hooks, mod._backward_pre_hooks]
 
 
 def _build(layer, mu: bool, fixed) -> Optional[_Plan]:
@@ -103,6 +109,10 @@ def _build(layer, mu: bool, fixed) -> Optional[_Plan]:
     for m in linears + norms:
         p.slots += [(m._parameters, "weight", m._parameters.get("weight")), (m._parameters, "bias", m._parameters.get("bias"))]
 
+    p.hooks = _hooks(ff)
+    if adapters is not None:
+        p.hooks += _hooks(adapters[-1])
+        p.slots += [(adapters[-1].__dict__, "forward", None)]
     for m in adapters or ():
         p.slots += [(m._modules, n, m._modules.get(n)) for n in ("base", "dropout")] + [(m._parameters, n, m._parameters.get(n)) for n in ("lora_A", "lora_B")]
         p.slots += [(m.__dict__, "scaling", m.__dict__.get("scaling"))]
@@ -189,7 +199,7 @@ def run_layer(layer, x, chain_mask, padding_mask, chain_ids, pack, *, mu: bool, 
         layer.__dict__["_native_plan"] = plan
         if plan is None:
             return None
-    if not plan.can_grad and torch.is_grad_enabled():
+    if (not plan.can_grad and torch.is_grad_enabled()) or any(plan.hooks) or _any_global_hook():
         return None
     T, B = (pack.T, pack.B) if pack is not None else (x.shape[0], x.shape[1])
     meta = mp._cached_ids_meta(chain_ids, padding_mask) if chain_ids is not None and chain_mask is None else ops.cached_mask_meta(chain_mask, padding_mask)
@@ -206,7 +216,7 @@ def run_layer(layer, x, chain_mask, padding_mask, chain_ids, pack, *, mu: bool, 
 
 def _plain(mod, kind, dtype=torch.float32) -> bool:
     """`mod` is exactly a `kind` with aligned contiguous parameters of `dtype` and no hooks."""
-    return (type(mod) is kind and not mod._forward_hooks and not mod._forward_pre_hooks and
+    return (type(mod) is kind and not any(_hooks(mod)) and "forward" not in mod.__dict__ and
             all(p is None or (p.is_cuda and p.dtype == dtype and p.is_contiguous() and p.data_ptr() % 16 == 0) for p in (mod.weight, mod.bias)))
 
 
@@ -220,6 +230,8 @@ def run_layer_f32(layer, x, chain_mask, padding_mask, chain_ids):
         return None
     sa, ma, ff = layer.self_attn, layer.multimer_attn, layer.feed_forward
     if type(ff) is not mp.VanillaFeedForward or sa.head_dim not in (16, 32, 64) or x.numel() == 0:
+        return None
+    if any(_hooks(ff)) or _any_global_hook():
         return None
     if not (_own(mp, layer, "_multimer_attention_plus", "_multimer_attention_superfused") and _own(mp, ff, "forward") and
             all(_own(mp, a, "project_qkv_4d") and (not hasattr(a, "_project_qkv") or _own(mp, a, "_project_qkv")) for a in (sa, ma))):

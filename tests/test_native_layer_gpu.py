@@ -229,3 +229,40 @@ def test_modules_that_compute_something_else_keep_their_results(what, dtype, mon
         layer.__class__ = _Attn
     got = equal_to_composed(layer, x, ids, pad, monkeypatch)
     assert (got - plain).abs().max() > 0.1
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("where", ["block", "global"])
+def test_hooks_fire(where, dtype):
+    layer = make_layer("plus").to(dtype)
+    x, ids, pad = batch(70, 2)
+    x = x.to(dtype)
+    plain = values(layer, x, ids, pad)
+    seen = []
+    if where == "block":
+        h = layer.feed_forward.register_forward_hook(lambda m, i, o: seen.append(m) or 2 * o)
+    else:
+        h = torch.nn.modules.module.register_module_forward_hook(lambda m, i, o: (seen.append(m), 2 * o)[1] if m is layer.feed_forward else None)
+    got = values(layer, x, ids, pad)
+    h.remove()
+    assert seen == [layer.feed_forward] and (got - plain).abs().max() > 0.1
+    assert torch.equal(values(layer, x, ids, pad), plain)
+
+
+def test_backward_hook_of_the_block_fires():
+    layer = make_layer("plus")
+    x, ids, pad = batch(70, 2)
+    seen = []
+    layer.feed_forward.register_full_backward_hook(lambda m, gi, go: seen.append(m))
+    run(layer, x, ids, pad, torch.randn_like(x))
+    assert seen == [layer.feed_forward]
+
+
+def test_hooks_of_a_wrapped_output_projection_fire():
+    layer = make_layer("lora")
+    x, ids, pad = batch(70, 2)
+    values(layer, x, ids, pad)
+    seen = []
+    layer.self_attn.out_proj.register_forward_hook(lambda m, i, o: seen.append(m))
+    values(layer, x, ids, pad)
+    assert seen == [layer.self_attn.out_proj]
