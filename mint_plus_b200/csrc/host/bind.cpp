@@ -68,21 +68,23 @@ PYBIND11_MODULE(_mintb_host, m) {
   py::class_<LayerPlan>(m, "LayerPlan")
       .def(py::init([](bool mu, bool fp8, bool sqrt_softmax, int64_t H, int64_t D, double scale, double keep, double add, double eps1, double eps2,
                        const std::vector<OptTensor>& params, int64_t n_self, int64_t n_cross, const Operand& qkv_self, const Operand& qkv_cross, const Operand& out,
-                       const Operand& fc1, const Operand& fc2, const OptTensor& qkv6, const OptTensor& bias6, const OptTensor& bias_self, const OptTensor& bias_cross, int64_t lora_r, double lora_scaling) {
+                       const Operand& fc1, const Operand& fc2, bool joint, const OptTensor& qkv6, int64_t lora_r, double lora_scaling) {
              LayerPlan p;
              p.lora_r = lora_r; p.lora_scaling = lora_scaling;
              p.mu = mu; p.fp8 = fp8; p.sqrt_softmax = sqrt_softmax; p.H = H; p.D = D; p.scale = scale; p.keep = keep; p.add = add; p.eps1 = eps1; p.eps2 = eps2;
              for (const OptTensor& t : params) p.params.push_back(opt(t));
              p.n_self = n_self; p.n_cross = n_cross; p.qkv_self = qkv_self; p.qkv_cross = qkv_cross; p.out = out; p.fc1 = fc1; p.fc2 = fc2;
-             p.qkv6 = opt(qkv6); p.bias6 = opt(bias6); p.bias_self = opt(bias_self); p.bias_cross = opt(bias_cross);
+             p.joint = joint; p.qkv6 = opt(qkv6);
+             p.form();
              return p;
            }),
            py::kw_only(), py::arg("mu"), py::arg("fp8"), py::arg("sqrt_softmax"), py::arg("H"), py::arg("D"), py::arg("scale"), py::arg("keep"), py::arg("add"),
            py::arg("eps1"), py::arg("eps2"), py::arg("params"), py::arg("n_self"), py::arg("n_cross"), py::arg("qkv_self"), py::arg("qkv_cross"), py::arg("out"),
-           py::arg("fc1"), py::arg("fc2"), py::arg("qkv6"), py::arg("bias6"), py::arg("bias_self"), py::arg("bias_cross"),
+           py::arg("fc1"), py::arg("fc2"), py::arg("joint"), py::arg("qkv6"),
            py::arg("lora_r") = 0, py::arg("lora_scaling") = 1.0)
+      .def("as_laid_out", &LayerPlan::as_laid_out)
       .def("forward",
-           [](LayerPlan& p, const Tensor& x, const OptTensor& xq, int64_t T, int64_t B, const Tensor& meta, const OptTensor& cos, const OptTensor& sin,
+           [](const LayerPlan& p, const Tensor& x, const OptTensor& xq, int64_t T, int64_t B, const Tensor& meta, const OptTensor& cos, const OptTensor& sin,
               const OptTensor& rows32, const OptTensor& rows64, const OptTensor& inv32, double next_quant) {
              return p.forward(x, xq, Batch{T, B, meta, opt(cos), opt(sin), opt(rows32), opt(rows64), opt(inv32)}, next_quant);
            },

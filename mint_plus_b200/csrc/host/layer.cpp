@@ -50,9 +50,79 @@ struct LayerNode : public torch::autograd::Node {
   std::string name() const override { return "TransformerLayerBackward"; }
 };
 
-std::tuple<Tensor, OptTensor> LayerPlan::forward(const Tensor& x_in, const OptTensor& xq_in, const Batch& batch, double next_quant) {
+static uint32_t version_of(const Tensor& t) { return t.is_inference() ? 0 : uint32_t(t._version()); }
+
+// The vectors in one piece; in fp32 where their types differ.
+static Tensor concatenated(at::TensorList parts) {
+  for (const Tensor& t : parts)
+    if (!t.defined()) return Tensor();
+  for (const Tensor& t : parts)
+    if (t.scalar_type() != parts[0].scalar_type()) {
+      std::vector<Tensor> f;
+      for (const Tensor& u : parts) f.push_back(u.to(at::kFloat));
+      return at::cat(f);
+    }
+  return parts.size() == 1 ? parts[0] : at::cat(parts);
+}
+
+void LayerPlan::form() {
   const Where at(*this);
   TORCH_CHECK(int64_t(params.size()) == at.n, "a layer plan needs ", at.n, " parameters, got ", params.size());
+  at::AutoDispatchBelowADInplaceOrView below;
+  const at::TensorList all(params);
+  const at::TensorList ws = all.slice(at.ws, n_self), wc = all.slice(at.wc, n_cross), bs = all.slice(at.bs, n_self), bc = all.slice(at.bc, n_cross);
+  const int64_t E = H * D;
+  auto both = [](at::TensorList a, at::TensorList b) {
+    std::vector<Tensor> v = a.vec();
+    v.insert(v.end(), b.begin(), b.end());
+    return concatenated(v);
+  };
+  if (joint && !fp8) {
+    qkv6 = both(ws, wc);
+    qkv_self.w = rows_of(qkv6, 0, 3 * E);
+    qkv_cross.w = rows_of(qkv6, 3 * E, 3 * E);
+  } else if (!fp8 && lora_r == 0) {
+    qkv_self.w = concatenated(ws);
+    qkv_cross.w = concatenated(wc);
+  }
+  if (joint || lora_r > 0) {
+    bias6 = both(bs, bc);
+  } else {
+    bias_self = concatenated(bs);
+    bias_cross = concatenated(bc);
+  }
+  stamps.clear();
+  for (int64_t k = 0; k < at.n; ++k) {
+    const Tensor& t = params[k];
+    const bool weight = k == at.wo || k == at.w1 || k == at.w2 || k < at.bs || (k >= at.wc && k < at.bc);
+    const bool qkv = k < at.wo, copied = fp8 ? weight || (joint && qkv) : joint && qkv;
+    stamps.push_back(t.defined() ? Stamp{t.scalar_type(), copied, t.data_ptr(), version_of(t)} : Stamp{at::kFloat, false, nullptr, 0});
+  }
+}
+
+bool LayerPlan::as_laid_out() const {
+  for (size_t k = 0; k < params.size(); ++k) {
+    const Tensor& t = params[k];
+    if (!t.defined()) continue;
+    const Stamp& s = stamps[k];
+    if (t.scalar_type() != s.dtype || !t.is_contiguous() || !t.is_cuda()) return false;
+    if (s.copied && (t.data_ptr() != s.data || version_of(t) != s.version)) return false;
+  }
+  return true;
+}
+
+std::tuple<Tensor, OptTensor> LayerPlan::forward(const Tensor& x, const OptTensor& xq, const Batch& batch, double next_quant) const {
+  // Separate projections too large to be kept in a joint copy, their biases, and a frozen base's biases are joined in every call.
+  if (!joint && (lora_r > 0 || n_self > 1 || n_cross > 1)) {
+    LayerPlan now = *this;
+    now.form();
+    return now.run(x, xq, batch, next_quant);
+  }
+  return run(x, xq, batch, next_quant);
+}
+
+std::tuple<Tensor, OptTensor> LayerPlan::run(const Tensor& x_in, const OptTensor& xq_in, const Batch& batch, double next_quant) const {
+  const Where at(*this);
   std::vector<Tensor> inputs;
   inputs.reserve(at.n + 1);
   inputs.push_back(x_in);

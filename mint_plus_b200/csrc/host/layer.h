@@ -28,24 +28,40 @@ struct Batch {
 };
 
 // A two-pathway transformer layer laid out for calling: its parameters and the operands formed from them.  The Python layer builds
-// one and keeps it until a parameter or an operand it was made from changes.
+// one and keeps it while as_laid_out() finds the parameters as they were.
 struct LayerPlan {
   bool mu = false;      // x = keep x + add attn(x); x = LN(keep x + add ffn(x)); else x += attn(LN(x)); x += ffn(LN(x))
   bool fp8 = false, sqrt_softmax = false;
   int64_t H = 0, D = 0;
   double scale = 1.0, keep = 1.0, add = 1.0, eps1 = 0.0, eps2 = 0.0;
   // parameters: self q/k/v weights (one fused or three), their biases, the cross pathway's, then out, fc1, fc2 (weight, bias) and the
-  // norms (gamma, beta): the first one on Pre-LN layers only.  An absent bias is undefined.
+  // norms (gamma, beta): the first one on Pre-LN layers only.  An absent bias is undefined.  They are the module's own tensors, so a
+  // product that reads one directly follows whatever is written to it or put in its place.
   std::vector<Tensor> params;
   int64_t n_self = 1, n_cross = 1;
   Operand qkv_self, qkv_cross, out, fc1, fc2;   // qkv operands [3E][E], rows [Q; K; V]
   // frozen projections with adapters: params ends with A and B of self q, k, v, cross q, k, v and out; the operands are formed per call
   int64_t lora_r = 0;
   double lora_scaling = 1.0;
-  Tensor qkv6, bias6;                           // both pathways in one operand, when one product serves them
+  bool joint = false;                           // both pathways' projections are one product: on
+  Tensor qkv6, bias6;                           // this operand, a copy that is kept while its sources stand
   Tensor bias_self, bias_cross;                 // [3E] biases of separate products
 
-  std::tuple<Tensor, OptTensor> forward(const Tensor& x, const OptTensor& xq, const Batch& batch, double next_quant);
+  // Forms what is copied from the parameters (not the e4m3 weights, which Python hands in) and notes what it was copied from.
+  void form();
+  // The parameters are what the plan was laid out for, and those behind a kept copy have not been written or replaced.
+  bool as_laid_out() const;
+  std::tuple<Tensor, OptTensor> forward(const Tensor& x, const OptTensor& xq, const Batch& batch, double next_quant) const;
+
+ private:
+  struct Stamp {
+    at::ScalarType dtype;
+    bool copied;        // a kept copy depends on it
+    const void* data;
+    uint32_t version;
+  };
+  std::vector<Stamp> stamps;   // one for each parameter
+  std::tuple<Tensor, OptTensor> run(const Tensor& x, const OptTensor& xq, const Batch& batch, double next_quant) const;
 };
 
 }  // namespace mintb_host

@@ -20,12 +20,12 @@ from . import ops
 
 
 class _Plan:
-    """The native plan of a layer and what it was made from: `slots` are (dict, key, object) that must still hold that object,
-    `tensors` (tensor, address, version) whose contents were copied into an operand, `fixed` the layer's own settings; `hooks` are the hook
+    """The native plan of a layer and what it was made from: `slots` are (dict, key, object) that must still hold that object
+    (the contents behind the copied operands the native plan watches), `fixed` the layer's own settings; `hooks` are the hook
     dictionaries of the modules that would be called otherwise: while one is filled the layer runs through the modules.  The layer keeps
     its plan and the plan nothing of the layer's own dictionary: a dropped layer dies at once, weights and copies with it."""
 
-    __slots__ = ("native", "slots", "tensors", "fixed", "hooks", "can_grad", "x_scale", "rot")
+    __slots__ = ("native", "slots", "fixed", "hooks", "can_grad", "x_scale", "rot")
 
     def valid(self, fixed) -> bool:
         if self.fixed != fixed:
@@ -33,10 +33,7 @@ class _Plan:
         for d, k, o in self.slots:
             if d.get(k) is not o:
                 return False
-        for t, p, v in self.tensors:
-            if t._version != v or t.data_ptr() != p:
-                return False
-        return True
+        return self.native.as_laid_out()
 
     # copies of a model lay their layers out themselves
     def __deepcopy__(self, memo):
@@ -102,12 +99,13 @@ def _build(layer, mu: bool, fixed) -> Optional[_Plan]:
     bias_s, bias_c = ms[0].bias is not None, mc[0].bias is not None
 
     p = _Plan()
-    p.slots, p.tensors, p.fixed = [], [], fixed
+    p.slots, p.fixed = [], fixed
     for m, names in ((layer, ("self_attn", "multimer_attn", "feed_forward", "final_layer_norm") + (() if mu else ("self_attn_layer_norm",))),
                      (sa, _ATTN_CHILDREN), (ma, _ATTN_CHILDREN), (ff, ("fc1", "fc2"))):
         p.slots += [(m._modules, n, m._modules.get(n)) for n in names]
     for m in linears + norms:
         p.slots += [(m._parameters, "weight", m._parameters.get("weight")), (m._parameters, "bias", m._parameters.get("bias"))]
+    p.slots += [(sa.__dict__, k, sa.__dict__.get(k)) for k in ("scaling", "num_heads", "head_dim")] + [(n.__dict__, "eps", n.eps) for n in norms]
 
     p.hooks = _hooks(ff)
     if adapters is not None:
@@ -117,60 +115,33 @@ def _build(layer, mu: bool, fixed) -> Optional[_Plan]:
         p.slots += [(m._modules, n, m._modules.get(n)) for n in ("base", "dropout")] + [(m._parameters, n, m._parameters.get(n)) for n in ("lora_A", "lora_B")]
         p.slots += [(m.__dict__, "scaling", m.__dict__.get("scaling"))]
 
-    def watch(t):
-        if t is not None:
-            p.tensors.append((t, t.data_ptr(), t._version))
-
-    with torch.no_grad():
-        qkv6 = bias6 = b_self = b_cross = None
-        if fp8:
-            f8s, f8c = fused_fp8_weight(sa, ms), fused_fp8_weight(ma, mc)
-            if f8s[2] != f8c[2]:
-                return None          # one cast of the input serves both products
-            holders = [f8s[4], one[0].grad_scale, one[1].grad_scale, one[2].grad_scale]
-            p.can_grad = all(m.fp8_grads for m in linears)
-            op_s = L.host().Operand(f8s[0], f8s[1], f8s[2], f8s[3], holders[0])
-            op_c = L.host().Operand(f8c[0], f8c[1], f8c[2], f8c[3])
-            wq = [m._quantized_weight() for m in one]
-            o, f1, f2 = (L.host().Operand(w, s, m.x_scale, m.out_scale, h) for (w, s), m, h in zip(wq, one, holders[1:]))
-            for m in linears:
-                watch(m.weight)
-                p.slots += [(m.__dict__, k, m.__dict__.get(k)) for k in ("_wq", "x_scale", "out_scale", "fp8_grads", "grad_scale")]
-            p.slots += [(h.__dict__, "scale", h.scale) for h in holders if h is not None]
-            p.slots += [(a.__dict__, "_fp8_qkv_grad_scale", a.__dict__.get("_fp8_qkv_grad_scale")) for a in (sa, ma)]
-            w_s, w_c = f8s[0], f8c[0]
-            p.x_scale = f8s[2]
-        else:
-            p.can_grad, p.x_scale = True, 0.0
-            w_s, w_c = ((m[0].weight.detach() if len(m) == 1 else None) for m in (ms, mc))
-            if adapters is None and (w_s is None or w_c is None or 12 * E * E <= mp._QKV6_MAX_BYTES):
-                for m in ms + mc:
-                    watch(m.weight)
-        if adapters is not None:
-            if bias_s != bias_c:
-                return None
-            bias6 = torch.cat([m.bias.detach().float() for m in ms + mc]) if bias_s else None
-        elif mp.FUSE_QKV6 and 6 * E * E * (1 if fp8 else 2) <= mp._QKV6_MAX_BYTES and bias_s == bias_c:
-            # both pathways' projections as one product that reads x once; a larger [6E][E] operand pushes the activation rows out
-            # of L2 between column tiles (measured slower)
-            if fp8:
-                qkv6 = torch.cat([w_s.view(torch.uint8), w_c.view(torch.uint8)]).view(torch.float8_e4m3fn)
-            else:
-                qkv6 = torch.cat([m.weight.detach() for m in ms + mc])
-            w_s, w_c = qkv6[:3 * E], qkv6[3 * E:]
-            if bias_s:
-                bias6 = torch.cat([m.bias.detach().float() for m in ms + mc])
-        elif not fp8:
-            w_s = torch.cat([m.weight.detach() for m in ms]) if w_s is None else w_s
-            w_c = torch.cat([m.weight.detach() for m in mc]) if w_c is None else w_c
-        if qkv6 is None and adapters is None:
-            b_self = (ms[0].bias.detach() if len(ms) == 1 else torch.cat([m.bias.detach() for m in ms])) if bias_s else None
-            b_cross = (mc[0].bias.detach() if len(mc) == 1 else torch.cat([m.bias.detach() for m in mc])) if bias_c else None
-        for m in ms + mc:
-            watch(m.bias)
-        if not fp8:
-            op_s, op_c = (L.host().Operand(w) for w in (w_s, w_c)) if adapters is None else (L.host().Operand(None), L.host().Operand(None))
-            o, f1, f2 = (L.host().Operand(m.weight) for m in one)
+    # both pathways' projections as one product that reads x once; a larger [6E][E] operand pushes the activation rows out of L2 between
+    # column tiles (measured slower)
+    joint = adapters is None and mp.FUSE_QKV6 and 6 * E * E * (1 if fp8 else 2) <= mp._QKV6_MAX_BYTES and bias_s == bias_c
+    qkv6 = None
+    if fp8:
+        f8s, f8c = fused_fp8_weight(sa, ms), fused_fp8_weight(ma, mc)
+        if f8s[2] != f8c[2]:
+            return None          # one cast of the input serves both products
+        holders = [f8s[4], one[0].grad_scale, one[1].grad_scale, one[2].grad_scale]
+        p.can_grad = all(m.fp8_grads for m in linears)
+        op_s = L.host().Operand(f8s[0], f8s[1], f8s[2], f8s[3], holders[0])
+        op_c = L.host().Operand(f8c[0], f8c[1], f8c[2], f8c[3])
+        wq = [m._quantized_weight() for m in one]
+        o, f1, f2 = (L.host().Operand(w, s, m.x_scale, m.out_scale, h) for (w, s), m, h in zip(wq, one, holders[1:]))
+        for m in linears:
+            p.slots += [(m.__dict__, k, m.__dict__.get(k)) for k in ("_wq", "x_scale", "out_scale", "fp8_grads", "grad_scale")]
+        p.slots += [(h.__dict__, "scale", h.scale) for h in holders if h is not None]
+        p.slots += [(a.__dict__, "_fp8_qkv_grad_scale", a.__dict__.get("_fp8_qkv_grad_scale")) for a in (sa, ma)]
+        p.x_scale = f8s[2]
+        if joint:
+            qkv6 = torch.cat([f8s[0].view(torch.uint8), f8c[0].view(torch.uint8)]).view(torch.float8_e4m3fn)
+    else:
+        p.can_grad, p.x_scale = True, 0.0
+        if adapters is not None and bias_s != bias_c:
+            return None
+        op_s = op_c = L.host().Operand(None)
+        o, f1, f2 = (L.host().Operand(m.weight) for m in one)
     params = [m.weight for m in ms] + [m.bias for m in ms] + [m.weight for m in mc] + [m.bias for m in mc]
     for m in one + norms:
         params += [m.weight, m.bias]
@@ -178,8 +149,7 @@ def _build(layer, mu: bool, fixed) -> Optional[_Plan]:
         params += [m.lora_A for m in adapters] + [m.lora_B for m in adapters]
     p.native = L.host().LayerPlan(mu=mu, fp8=fp8, sqrt_softmax=sqrt_softmax, H=H, D=sa.head_dim, scale=sa.scaling, keep=keep, add=add,
                                   eps1=norms[0].eps, eps2=norms[-1].eps, params=params, n_self=len(ms), n_cross=len(mc), qkv_self=op_s, qkv_cross=op_c,
-                                  out=o, fc1=f1, fc2=f2, qkv6=qkv6, bias6=bias6, bias_self=b_self, bias_cross=b_cross,
-                                  lora_r=adapters[0].r if adapters else 0, lora_scaling=adapters[0].scaling if adapters else 1.0)
+                                  out=o, fc1=f1, fc2=f2, joint=joint, qkv6=qkv6, lora_r=adapters[0].r if adapters else 0, lora_scaling=adapters[0].scaling if adapters else 1.0)
     p.rot = sa.rot_emb
     return p
 

@@ -266,3 +266,33 @@ def test_hooks_of_a_wrapped_output_projection_fire():
     layer.self_attn.out_proj.register_forward_hook(lambda m, i, o: seen.append(m))
     values(layer, x, ids, pad)
     assert seen == [layer.self_attn.out_proj]
+
+
+@pytest.mark.parametrize("kind,how", [("plus", "data"), ("base", "data"), ("base", "data_copy"), ("plus", "bias_data"), ("plus", "dtype")])
+def test_weights_replaced_through_data_are_followed(kind, how, monkeypatch):
+    monkeypatch.setattr(modules_plus, "_QKV6_MAX_BYTES", 0)
+    layer = make_layer(kind)
+    x, ids, pad = batch(64, 2)
+    before = values(layer, x, ids, pad)
+    sa = layer.self_attn
+    w = (sa.fused_qkv if kind == "plus" else sa.q_proj).weight
+    if how == "data":
+        w.data = -w.data
+    elif how == "data_copy":
+        w.data.mul_(-1)
+    elif how == "bias_data":
+        sa.fused_qkv.bias.data = sa.fused_qkv.bias.data + 1
+    else:
+        layer.feed_forward.fc1.weight.data = -layer.feed_forward.fc1.weight.data.float()
+    got = equal_to_composed(layer, x, ids, pad, monkeypatch)
+    assert (got - before).abs().max() > 0.05
+
+
+def test_a_changed_logit_scale_is_followed(monkeypatch):
+    layer = make_layer("plus")
+    x, ids, pad = batch(64, 2)
+    before = values(layer, x, ids, pad)
+    layer.self_attn.scaling = 3.0
+    layer.final_layer_norm.eps = 0.5
+    got = equal_to_composed(layer, x, ids, pad, monkeypatch)
+    assert (got - before).abs().max() > 0.05
