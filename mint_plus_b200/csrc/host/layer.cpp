@@ -37,6 +37,7 @@ struct LayerNode : public torch::autograd::Node {
   Batch batch;
   SavedVariable saved[kNumSaved];
   std::vector<SavedVariable> weights;   // what the bf16 products read again
+  SavedVariable gamma1, gamma2, b_out;  // parameters that are read again: the norms' gammas, B of the output projection's adapter
   std::vector<int64_t> shape;
   double xq_scale = 1.0;
 
@@ -44,6 +45,9 @@ struct LayerNode : public torch::autograd::Node {
   void release_variables() override {
     for (auto& s : saved) s.reset_data();
     for (auto& s : weights) s.reset_data();
+    gamma1.reset_data();
+    gamma2.reset_data();
+    b_out.reset_data();
     plan = LayerPlan();
     batch = Batch();
   }
@@ -249,6 +253,9 @@ std::tuple<Tensor, OptTensor> LayerPlan::run(const Tensor& x_in, const OptTensor
     keep_t[kX] = x_in;
     for (int k = 0; k < kNumSaved; ++k)
       if (keep_t[k].defined()) node->saved[k] = SavedVariable(keep_t[k], false);
+    if (!mu) node->gamma1 = SavedVariable(params[at.g1], false);
+    node->gamma2 = SavedVariable(params[at.g2], false);
+    if (lora_r > 0) node->b_out = SavedVariable(params[at.lb + 6], false);
     if (!fp8)
       for (const Tensor& t : {qkv_self.w, qkv_cross.w, out.w, fc1.w, fc2.w})
         if (t.defined()) node->weights.emplace_back(t, false);
@@ -279,7 +286,9 @@ variable_list LayerNode::apply(variable_list&& grads) {
       if (wants(k + i)) res[k + i + 1] = n == 1 ? c : rows_of(c, i * E, E);
   };
   auto w_dt = [&](int64_t k) { return plan.params[k].scalar_type() == at::kFloat ? at::kFloat : at::kBFloat16; };
-  for (auto& s : weights) s.unpack();   // raises if a weight that the products read again has been written since
+  // unpacking raises if a parameter that is read again has been written since
+  for (auto& s : weights) s.unpack();
+  const Tensor g1v = gamma1.unpack(), g2v = gamma2.unpack(), b_outv = b_out.unpack();
   Tensor s[kNumSaved];
   for (int k = 0; k < kNumSaved; ++k) s[k] = saved[k].unpack();
   const Tensor x = s[kX].reshape({-1, E}).contiguous(), gy = grads[0].reshape({-1, E}).contiguous();
@@ -303,7 +312,7 @@ variable_list LayerNode::apply(variable_list&& grads) {
 
   Tensor d_ffn = gy, d1;   // gradients of the FFN's result and of the first residual sum
   if (mu) {
-    NormGrad g = add_layernorm_bwd(gy, Tensor(), s[kX1], s[kY2], plan.keep, plan.add, plan.params[at.g2], s[kStats2], p2);
+    NormGrad g = add_layernorm_bwd(gy, Tensor(), s[kX1], s[kY2], plan.keep, plan.add, g2v, s[kStats2], p2);
     if (p2) { give(at.g2, g.dgamma); give(at.be2, g.dbeta); }
     d1 = g.dx;
     d_ffn = g.dr;
@@ -320,7 +329,7 @@ variable_list LayerNode::apply(variable_list&& grads) {
       d1 = dgrad(g1, plan.fc1.w, a_in(plan.fc1), Tensor(), Tensor(), d1, 1.0);   // both ways into the first residual sum
     } else {
       Tensor dh2 = dgrad(g1, plan.fc1.w, a_in(plan.fc1));
-      NormGrad g = add_layernorm_bwd(dh2, gy, s[kX1], Tensor(), 1.0, 0.0, plan.params[at.g2], s[kStats2], p2, true);
+      NormGrad g = add_layernorm_bwd(dh2, gy, s[kX1], Tensor(), 1.0, 0.0, g2v, s[kStats2], p2, true);
       if (p2) { give(at.g2, g.dgamma); give(at.be2, g.dbeta); }
       d1 = g.dx;
     }
@@ -346,7 +355,7 @@ variable_list LayerNode::apply(variable_list&& grads) {
       xa.x = s[kO];
       xa.w = rows_of(s[kARows], 6 * r, r);
       if (wants(at.lb + 6)) give(at.lb + 6, wgrad(go, linear_fwd(xa).first, plan.lora_scaling, at::kBFloat16));
-      if (wants(at.la + 6)) give(at.la + 6, wgrad(dgrad(go, plan.params[at.lb + 6], 1.0), s[kO], plan.lora_scaling, at::kBFloat16));
+      if (wants(at.la + 6)) give(at.la + 6, wgrad(dgrad(go, b_outv, 1.0), s[kO], plan.lora_scaling, at::kBFloat16));
     }
     d_attn = dgrad(go, w_out.w, a_in(w_out) * plan.add);
   }
@@ -395,7 +404,7 @@ variable_list LayerNode::apply(variable_list&& grads) {
     if (task_should_compute_output(0)) res[0] = dgrad(gs, os.w, a_in(os), gc, oc.w, d1, plan.keep).view(shape);
   } else if (task_should_compute_output(0) || p1) {
     Tensor dh = dgrad(gs, os.w, a_in(os), gc, oc.w);
-    NormGrad n = add_layernorm_bwd(dh, d1, x, Tensor(), 1.0, 0.0, plan.params[at.g1], s[kStats1], p1, true);
+    NormGrad n = add_layernorm_bwd(dh, d1, x, Tensor(), 1.0, 0.0, g1v, s[kStats1], p1, true);
     if (p1) { give(at.g1, n.dgamma); give(at.be1, n.dbeta); }
     res[0] = n.dx.view(shape);
   }

@@ -296,3 +296,15 @@ def test_a_changed_logit_scale_is_followed(monkeypatch):
     layer.final_layer_norm.eps = 0.5
     got = equal_to_composed(layer, x, ids, pad, monkeypatch)
     assert (got - before).abs().max() > 0.05
+
+
+@pytest.mark.parametrize("kind,name", [("plus", "self_attn_layer_norm.weight"), ("plus", "final_layer_norm.weight"), ("mu_fp8", "final_layer_norm.weight"),
+                                       ("lora", "self_attn.out_proj.lora_B"), ("plus", "feed_forward.fc1.weight")])
+def test_a_parameter_written_before_the_backward_pass_raises(kind, name):
+    layer = make_layer(kind)
+    x, ids, pad = batch(64, 2)
+    y, _ = layer(x.clone().requires_grad_(), self_attn_padding_mask=pad, chain_ids=ids)
+    with torch.no_grad():
+        dict(layer.named_parameters())[name].mul_(2)
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        y.sum().backward()
