@@ -40,6 +40,7 @@ PYBIND11_MODULE(_mintb_host, m) {
   m.def("set_failure_class", [](py::object c) { g_failure = c.release().ptr(); });
   m.def("dev_status", &dev_status);
   m.def("cached_free_bytes", &cached_free_bytes);
+  m.def("capture_id", &capture_id);
   auto nogil = py::call_guard<py::gil_scoped_release>();
   m.def("attention",
         [](const Tensor& q0, const Tensor& q1, const Tensor& q2, const Tensor& q3, const Tensor& q4, const Tensor& q5, const Tensor& meta, const OptTensor& cos,

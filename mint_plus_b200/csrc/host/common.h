@@ -124,6 +124,8 @@ std::pair<Tensor, Tensor> gelu_colsum(const Tensor& dy, const Tensor& z, std::op
 std::pair<Tensor, Tensor> gelu_colsum_f8(const Tensor& dy, const Tensor& z, std::optional<at::ScalarType> db_dt, double scale);
 // Bytes that the caching allocator holds on the device without using them.
 int64_t cached_free_bytes(int device);
+// The capture that the current stream of the tensor's device is in, 0 if none.
+uint64_t capture_id(const Tensor& t);
 
 struct NormOut {
   Tensor s, y, stats, q8;

@@ -202,4 +202,11 @@ int64_t cached_free_bytes(int device) {
   return stats.reserved_bytes[all].current - stats.allocated_bytes[all].current;
 }
 
+uint64_t capture_id(const Tensor& t) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  C10_CUDA_CHECK(cudaStreamGetCaptureInfo(at::cuda::getCurrentCUDAStream(t.device().index()).stream(), &status, &id));
+  return status == cudaStreamCaptureStatusNone ? 0 : id;
+}
+
 }  // namespace mintb_host

@@ -116,8 +116,10 @@ bool LayerPlan::as_laid_out() const {
 }
 
 std::tuple<Tensor, OptTensor> LayerPlan::forward(const Tensor& x, const OptTensor& xq, const Batch& batch, double next_quant) const {
-  // Separate projections too large to be kept in a joint copy, their biases, and a frozen base's biases are joined in every call.
-  if (!joint && (lora_r > 0 || n_self > 1 || n_cross > 1)) {
+  // Separate projections too large to be kept in a joint copy, their biases, and a frozen base's biases are joined in every call.  A
+  // captured call joins everything itself, so that its replays follow the weights and hold the copies in the graph's own memory.
+  c10::cuda::CUDAGuard guard(x.device());
+  if ((!fp8 && capture_id(x) != 0) || (!joint && (lora_r > 0 || n_self > 1 || n_cross > 1))) {
     LayerPlan now = *this;
     now.form();
     return now.run(x, xq, batch, next_quant);

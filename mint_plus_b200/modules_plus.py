@@ -119,7 +119,9 @@ def _fused6_operands(layer, ops_s, ops_c):
         return None       # a [6E][E] operand this large pushes the activation rows out of L2 between column tiles (measured slower)
     key = tuple((p.data_ptr(), p._version) for p in _qkv_params(layer.self_attn) + _qkv_params(layer.multimer_attn)) + (f8_s is not None,)
     cached = getattr(layer, "_qkv6_cache", None)
-    if cached is not None and cached[0] == key:
+    # a captured call forms its own bf16 copy, so that the replays follow the weights (e4m3 copies are those of the capture)
+    capturing = ops.capture_id(w_s) != 0
+    if cached is not None and cached[0] == key and (f8_s is not None or not capturing):
         return cached[1], cached[2]
     with torch.no_grad():
         if f8_s is not None:
@@ -127,7 +129,8 @@ def _fused6_operands(layer, ops_s, ops_c):
         else:
             w6 = torch.cat([w_s.detach().to(torch.bfloat16), w_c.detach().to(torch.bfloat16)], dim=0)
         b6 = torch.cat([b_s.detach().float(), b_c.detach().float()], dim=0) if b_s is not None else None
-    layer._qkv6_cache = (key, w6, b6)
+    if not capturing:
+        layer._qkv6_cache = (key, w6, b6)
     return w6, b6
 
 
@@ -294,11 +297,12 @@ _ids_meta_cache = []
 
 
 def _cached_ids_meta(chain_ids, padding_mask):
-    for ids, ver, pad, meta in _ids_meta_cache:
-        if ids is chain_ids and ver == chain_ids._version and pad is padding_mask:
+    capture = ops.capture_id(chain_ids)
+    for ids, ver, pad, cap, meta in _ids_meta_cache:
+        if ids is chain_ids and ver == chain_ids._version and pad is padding_mask and cap == capture:
             return meta
     meta = ops.mask_meta_from_chain_ids(chain_ids, padding_mask)
-    _ids_meta_cache.insert(0, (chain_ids, chain_ids._version, padding_mask, meta))
+    _ids_meta_cache.insert(0, (chain_ids, chain_ids._version, padding_mask, capture, meta))
     del _ids_meta_cache[2:]
     return meta
 

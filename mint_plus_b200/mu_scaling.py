@@ -233,7 +233,8 @@ def fused_fp8_weight(owner: nn.Module, mods):
         w = torch.cat([m.weight.detach() for m in mods], dim=0)
         w_scale = max(m._quantized_weight()[1] for m in mods)   # amax of the concatenation / 448; a host read only where a copy is stale
         cached = (key, ops.quantize_e4m3(w.to(torch.bfloat16).contiguous(), w_scale), w_scale)
-        owner._fp8_qkv_cache = cached
+        if not ops.capture_id(w):     # (what a capture forms exists in its replays only)
+            owner._fp8_qkv_cache = cached
     return cached[1], cached[2], max(m.x_scale for m in mods), mods[0].out_scale, (owner._fp8_qkv_grad_scale if f8_grads else None)
 
 

@@ -25,7 +25,7 @@ class _Plan:
     dictionaries of the modules that would be called otherwise: while one is filled the layer runs through the modules.  The layer keeps
     its plan and the plan nothing of the layer's own dictionary: a dropped layer dies at once, weights and copies with it."""
 
-    __slots__ = ("native", "slots", "fixed", "hooks", "can_grad", "x_scale", "rot")
+    __slots__ = ("native", "slots", "fixed", "hooks", "can_grad", "x_scale", "rot", "block")
 
     def valid(self, fixed) -> bool:
         if self.fixed != fixed:
@@ -107,7 +107,7 @@ def _build(layer, mu: bool, fixed) -> Optional[_Plan]:
         p.slots += [(m._parameters, "weight", m._parameters.get("weight")), (m._parameters, "bias", m._parameters.get("bias"))]
     p.slots += [(sa.__dict__, k, sa.__dict__.get(k)) for k in ("scaling", "num_heads", "head_dim")] + [(n.__dict__, "eps", n.eps) for n in norms]
 
-    p.hooks = _hooks(ff)
+    p.block, p.hooks = ff, _hooks(ff)
     if adapters is not None:
         p.hooks += _hooks(adapters[-1])
         p.slots += [(adapters[-1].__dict__, "forward", None)]
@@ -158,7 +158,7 @@ def run_layer(layer, x, chain_mask, padding_mask, chain_ids, pack, *, mu: bool, 
     """The layer's result for x (T,B,E) (or the packed rows of one), or None when the layer is not served here."""
     from . import modules_plus as mp
     if not (x.is_cuda and x.dtype == torch.bfloat16 and layer.use_multimer and layer._use_fused_multi_pathway and mp.FUSE_OUT_RESIDUAL and
-            _own(mp, layer, "_multimer_attention_superfused") and _own(mp, layer.feed_forward, "forward")):
+            getattr(layer._multimer_attention_superfused, "__func__", None) in mp.OWN_CODE):
         return None
     plan = layer.__dict__.get("_native_plan")
     fixed = (keep, add, bool(layer._use_sqrt_softmax))
@@ -166,10 +166,12 @@ def run_layer(layer, x, chain_mask, padding_mask, chain_ids, pack, *, mu: bool, 
         if layer.self_attn.head_dim not in (16, 32, 64):
             return None
         plan = _build(layer, mu, fixed)
-        layer.__dict__["_native_plan"] = plan
+        if not ops.capture_id(x):     # (what a capture forms exists in its replays only)
+            layer.__dict__["_native_plan"] = plan
         if plan is None:
             return None
-    if (not plan.can_grad and torch.is_grad_enabled()) or any(plan.hooks) or _any_global_hook():
+    if ((not plan.can_grad and torch.is_grad_enabled()) or any(plan.hooks) or _any_global_hook() or
+            getattr(plan.block.forward, "__func__", None) not in mp.OWN_CODE):
         return None
     T, B = (pack.T, pack.B) if pack is not None else (x.shape[0], x.shape[1])
     meta = mp._cached_ids_meta(chain_ids, padding_mask) if chain_ids is not None and chain_mask is None else ops.cached_mask_meta(chain_mask, padding_mask)

@@ -105,14 +105,21 @@ def mask_meta_from_mask(chain_mask: torch.Tensor, key_padding_mask: Optional[tor
     return MaskMeta(buf, B, T)
 
 
-_meta_cache = []  # [(weakref(mask), version, weakref(pad) | None, pad version, MaskMeta)], newest first
+def capture_id(t: torch.Tensor) -> int:
+    """Which stream capture a call on `t` belongs to, 0 outside one.  What a capture forms exists in its replays only, and a replay
+    has to form anew what depends on the contents of its inputs: metadata is shared within one capture, or outside of any."""
+    return L.host().capture_id(t) if t.is_cuda and torch.cuda.is_current_stream_capturing() else 0
+
+
+_meta_cache = []  # [(weakref(mask), version, weakref(pad) | None, pad version, capture, MaskMeta)], newest first
 
 
 def cached_mask_meta(chain_mask: torch.Tensor, key_padding_mask: Optional[torch.Tensor] = None) -> MaskMeta:
     """Metadata for a (B,T,T) mask, reused while the same tensor objects are passed again (every layer of a
     forward pass receives the same mask, esm2.py:124-132)."""
-    for ref_m, ver_m, ref_p, ver_p, meta in _meta_cache:
-        if ref_m() is chain_mask and ver_m == chain_mask._version:
+    capture = capture_id(chain_mask)
+    for ref_m, ver_m, ref_p, ver_p, cap, meta in _meta_cache:
+        if ref_m() is chain_mask and ver_m == chain_mask._version and cap == capture:
             if key_padding_mask is None and ref_p is None:
                 return meta
             if key_padding_mask is not None and ref_p is not None and ref_p() is key_padding_mask \
@@ -121,7 +128,7 @@ def cached_mask_meta(chain_mask: torch.Tensor, key_padding_mask: Optional[torch.
     meta = mask_meta_from_mask(chain_mask, key_padding_mask)
     _meta_cache.insert(0, (weakref.ref(chain_mask), chain_mask._version,
                            None if key_padding_mask is None else weakref.ref(key_padding_mask),
-                           0 if key_padding_mask is None else key_padding_mask._version, meta))
+                           0 if key_padding_mask is None else key_padding_mask._version, capture, meta))
     del _meta_cache[4:]
     return meta
 
@@ -139,7 +146,8 @@ def default_inv_freq(D: int, device) -> torch.Tensor:
 def rope_tables(T: int, D: int, device,
                 inv_freq: Optional[torch.Tensor] = None) -> Tuple[torch.Tensor, torch.Tensor, Optional[torch.Tensor]]:
     """(cos, sin, inv_freq): the cos/sin tables (T, D/2) fp32 on `device`, kept with the buffer `inv_freq` (the default frequencies
-    without one) for as long as it lives and holds what they were made from."""
+    without one) for as long as it lives and holds what they were made from.  A table that a longer one replaces is kept as well: a
+    captured graph may read it (lengths at least double, so all of them together are no more than twice the longest)."""
     device = torch.device(device)
     made_from = (D, device.index) if inv_freq is None else (D, device.index, inv_freq.data_ptr(), inv_freq._version)
     hit = _rope_default.get(made_from) if inv_freq is None else _rope_cache.get(inv_freq)
@@ -149,7 +157,7 @@ def rope_tables(T: int, D: int, device,
         return (*hit[2][T], inv_freq)
     if hit is None or T > hit[0].shape[0]:
         # row t depends on t alone, so the table of the longest length seen so far serves the shorter ones
-        rows = (T + 255) // 256 * 256
+        rows = max((T + 255) // 256 * 256, 0 if hit is None else 2 * hit[0].shape[0])
         inv = default_inv_freq(D, device) if inv_freq is None else inv_freq.detach().to(device=device, dtype=torch.float32).contiguous()
         if inv.numel() != D // 2:
             raise ValueError(f"inv_freq must have D/2 = {D // 2} entries")
@@ -157,7 +165,9 @@ def rope_tables(T: int, D: int, device,
         sin = torch.empty_like(cos)
         with _on(device):
             L.check(L.lib().mintb_rope_tables(_ptr(inv), _ptr(cos), _ptr(sin), rows, D, _stream()), "rope_tables")
-        hit = (cos, sin, {}, made_from)
+        hit = (cos, sin, {}, made_from, hit)
+        if capture_id(cos):     # (what a capture forms exists in its replays only)
+            return cos[:T], sin[:T], inv_freq
         if inv_freq is None:
             _rope_default[made_from] = hit
         else:

@@ -52,7 +52,8 @@ class GraphedTrainStep:
     replay overwrites).  The gradients are in `p.grad` of the parameters afterwards, at the same addresses every step.
 
     What the graph freezes: every value the library hands to its kernels by value at capture time.  For bf16 models there
-    is none that changes; for FP8 models the per-tensor scales of the capture are replayed, so a loop that updates the
+    is none that changes, and the copies that join weights are made inside the graph, so a replay follows an optimizer step;
+    for FP8 models the e4m3 weights and per-tensor scales of the capture are replayed, so a loop that updates the
     weights has to run eagerly (or re-capture after `Fp8WeightScaler.refresh()`).  The MLM corruption is drawn by the
     device generator inside the graph and differs from replay to replay, as in eager mode.  Before constructing one, drop
     every reference to losses of earlier eager steps: a live autograd graph keeps its gradient-accumulation nodes bound to
@@ -77,6 +78,8 @@ class GraphedTrainStep:
         self.graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(self.graph):
             self.loss = self._body()
+        # e4m3 copies that the graph reads and the model would drop when its weights change
+        self._copies = [m.__dict__.get(k) for m in model.modules() for k in ("_native_plan", "_wq", "_fp8_qkv_cache", "_qkv6_cache")]
 
     def _body(self) -> torch.Tensor:
         for p in self.params:

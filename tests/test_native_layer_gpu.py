@@ -308,3 +308,98 @@ def test_a_parameter_written_before_the_backward_pass_raises(kind, name):
         dict(layer.named_parameters())[name].mul_(2)
     with pytest.raises(RuntimeError, match="modified by an inplace operation"):
         y.sum().backward()
+
+
+def captured(layer, x, ids, pad, gy):
+    """(graph, [result, input gradient, parameter gradients], input) of one forward and backward pass, captured."""
+    x = x.clone().requires_grad_()
+
+    def step():
+        x.grad = None
+        for p in layer.parameters():
+            p.grad = None
+        y, _ = layer(x, self_attn_padding_mask=pad, chain_ids=ids)
+        y.backward(gy)
+        return y.detach()
+
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        for _ in range(2):
+            step()
+    torch.cuda.current_stream().wait_stream(side)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        y = step()
+    return g, [y, x.grad] + [p.grad for p in layer.parameters() if p.grad is not None], x
+
+
+@pytest.mark.parametrize("kind,two", [("base", False), ("base", True), ("plus", False), ("plus", True), ("lora", False), ("mu", False)])
+@pytest.mark.parametrize("served", [True, False])
+def test_a_replayed_step_follows_its_weights(kind, two, served, monkeypatch):
+    if two:
+        monkeypatch.setattr(modules_plus, "_QKV6_MAX_BYTES", 0)
+    if not served:
+        monkeypatch.setattr(native, "run_layer", lambda *a, **k: None)
+    layer = make_layer(kind)
+    x, ids, pad = batch(70, 3)
+    gy = torch.randn(70, 3, E, device=DEV, generator=torch.Generator(DEV).manual_seed(1)).bfloat16()
+    g, out, held = captured(layer, x, ids, pad, gy)
+    with torch.no_grad():
+        for p in layer.parameters():
+            p.mul_(-0.5)
+    junk = run(layer, x, ids, pad, gy)                       # an eager step between replays makes operands of its own
+    del junk
+    junk = [torch.full((1 << 18,), float("nan"), device=DEV) for _ in range(64)]     # (into whatever it freed)
+    # p.grad of the graph were dropped by run(): the buffers in `out` still are what a replay writes
+    g.replay()
+    got = [t.clone() for t in out]
+    del junk
+    twin = copy.deepcopy(layer)
+    close(got, run(twin, x, ids, pad, gy), 1e-2)
+
+
+def test_a_replayed_step_keeps_its_rotary_tables():
+    layer = make_layer("plus")
+    x, ids, pad = batch(70, 3)
+    gy = torch.randn(70, 3, E, device=DEV).bfloat16()
+    g, out, held = captured(layer, x, ids, pad, gy)
+    g.replay()
+    want = [t.clone() for t in out]
+    xl, il, pl = batch(900, 1)
+    values(layer, xl, il, pl)                                # a longer table takes the place of the shorter
+    junk = [torch.full((1 << 12,), float("nan"), device=DEV) for _ in range(256)]
+    g.replay()
+    close([t.clone() for t in out], want, 1e-3)
+    del junk
+
+
+def test_a_replay_builds_the_metadata_of_its_own_inputs():
+    """Chain ids and padding written into the captured step's input tensors after a warm-up on the same tensors."""
+    layer = make_layer("plus")
+    x, ids, pad = batch(70, 3)
+    gy = torch.randn(70, 3, E, device=DEV).bfloat16()
+    g, out, held = captured(layer, x, ids, pad, gy)
+    with torch.no_grad():
+        ids.copy_(1 - ids.flip(1))
+        pad.copy_(pad.roll(1, 0))
+    g.replay()
+    close([t.clone() for t in out], run(layer, x, ids.clone(), pad.clone(), gy), 1e-3)
+
+
+def test_a_captured_fp8_step_keeps_its_weights():
+    """The model drops and re-forms its e4m3 copies (and the plans made from them) between two replays."""
+    torch.manual_seed(0)
+    model = M.build_mint_mu("8M", num_layers=2, use_fp8=True, embed_dim=128, attention_heads=4).to(DEV).to(torch.bfloat16).train()
+    tokens = torch.randint(4, 24, (3, 90), device=DEV)
+    ids = (torch.arange(90, device=DEV) > 40).long().expand(3, 90).contiguous()
+    step = M.GraphedTrainStep(model, tokens, ids)
+    torch.cuda.manual_seed(5)
+    want = step(tokens, ids).item()
+    M.refresh_fp8_weights(model)
+    M.shared_step(model, (tokens, ids))[0].backward()
+    junk = [torch.full((n,), 0x7F, dtype=torch.uint8, device=DEV) for n in (1 << 14, 1 << 15, 3 << 14, 1 << 16, 3 << 15) for _ in range(40)]
+    torch.cuda.manual_seed(5)
+    assert step(tokens, ids).item() == pytest.approx(want, rel=1e-3)
+    del junk
