@@ -33,6 +33,7 @@ __device__ __forceinline__ bool elect_one() {
 // be scheduled as soon as every CTA of this grid has said so or has finished.  Kernels of this library call it after their own
 // griddep_wait(), so at any time everything before a kernel's direct predecessor is complete.
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 __device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ---------------------------------------------------------------------------------------------- mbarrier

@@ -247,3 +247,20 @@ def test_layernorm_sees_parameters_that_the_kernel_before_wrote():
     for k, y, g in steps:
         torch.testing.assert_close(y.float(), n * (k % 7 + 1) + k % 5, rtol=2e-2, atol=4e-2)
         torch.testing.assert_close(g.float(), dx * (k % 7 + 1), rtol=2e-2, atol=4e-2 * dx.abs().max().item() * (k % 7 + 1))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("E,rows", [(8, 1), (72, 5), (1280, 3), (2560, 700)])
+@pytest.mark.parametrize("off,bias", [(0, True), (1, True), (8, False)])
+def test_layernorm_parameters_of_any_type_and_alignment(dtype, E, rows, off, bias):
+    """Parameters as views into a flat buffer, on and off a 16-byte boundary, with and without beta."""
+    torch.manual_seed(E + off)
+    flat = torch.randn(2, E + off, device=DEV).to(dtype)
+    norm = torch.nn.LayerNorm(E, bias=bias).to(DEV)
+    norm.weight = torch.nn.Parameter(flat[0, off:])
+    if bias:
+        norm.bias = torch.nn.Parameter(flat[1, off:])
+    x = _bf(torch.randn(rows, E, device=DEV))
+    _, y = ops.add_layernorm(x, None, 1.0, 0.0, norm, need_s=False)
+    ref = torch.nn.functional.layer_norm(x.float(), (E,), norm.weight.float(), norm.bias.float() if bias else None, norm.eps)
+    torch.testing.assert_close(y.float(), ref, rtol=1e-2, atol=1e-2)
