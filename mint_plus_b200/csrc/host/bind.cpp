@@ -83,7 +83,8 @@ PYBIND11_MODULE(_mintb_host, m) {
            py::arg("eps1"), py::arg("eps2"), py::arg("params"), py::arg("n_self"), py::arg("n_cross"), py::arg("qkv_self"), py::arg("qkv_cross"), py::arg("out"),
            py::arg("fc1"), py::arg("fc2"), py::arg("joint"), py::arg("qkv6"),
            py::arg("lora_r") = 0, py::arg("lora_scaling") = 1.0)
-      .def("as_laid_out", &LayerPlan::as_laid_out)
+      .def("state", &LayerPlan::state)
+      .def("refreshed", &LayerPlan::refreshed)
       .def("forward",
            [](const LayerPlan& p, const Tensor& x, const OptTensor& xq, int64_t T, int64_t B, const Tensor& meta, const OptTensor& cos, const OptTensor& sin,
               const OptTensor& rows32, const OptTensor& rows64, const OptTensor& inv32, double next_quant) {

@@ -104,15 +104,23 @@ void LayerPlan::form() {
   }
 }
 
-bool LayerPlan::as_laid_out() const {
+int LayerPlan::state() const {
+  bool written = false;
   for (size_t k = 0; k < params.size(); ++k) {
     const Tensor& t = params[k];
     if (!t.defined()) continue;
     const Stamp& s = stamps[k];
-    if (t.scalar_type() != s.dtype || !t.is_contiguous() || !t.is_cuda()) return false;
-    if (s.copied && (t.data_ptr() != s.data || version_of(t) != s.version)) return false;
+    if (t.scalar_type() != s.dtype || !t.is_contiguous() || !t.is_cuda()) return kOther;
+    written = written || (s.copied && (t.data_ptr() != s.data || version_of(t) != s.version));
   }
-  return true;
+  return !written ? kCurrent : fp8 ? kOther : kWritten;
+}
+
+LayerPlan LayerPlan::refreshed() const {
+  c10::cuda::CUDAGuard guard(params[0].device());
+  LayerPlan p = *this;
+  p.form();
+  return p;
 }
 
 std::tuple<Tensor, OptTensor> LayerPlan::forward(const Tensor& x, const OptTensor& xq, const Batch& batch, double next_quant) const {

@@ -28,7 +28,7 @@ struct Batch {
 };
 
 // A two-pathway transformer layer laid out for calling: its parameters and the operands formed from them.  The Python layer builds
-// one and keeps it while as_laid_out() finds the parameters as they were.
+// one and keeps it while state() finds the parameters what they were.
 struct LayerPlan {
   bool mu = false;      // x = keep x + add attn(x); x = LN(keep x + add ffn(x)); else x += attn(LN(x)); x += ffn(LN(x))
   bool fp8 = false, sqrt_softmax = false;
@@ -49,8 +49,11 @@ struct LayerPlan {
 
   // Forms what is copied from the parameters (not the e4m3 weights, which Python hands in) and notes what it was copied from.
   void form();
-  // The parameters are what the plan was laid out for, and those behind a kept copy have not been written or replaced.
-  bool as_laid_out() const;
+  // kCurrent; kWritten: a parameter behind a kept copy has been written or replaced since, and form() takes it in; kOther: the plan was
+  // laid out for something else (another type, or e4m3 copies of weights that have changed).
+  enum State { kCurrent, kWritten, kOther };
+  int state() const;
+  LayerPlan refreshed() const;   // (a plan of its own: calls under way keep theirs)
   std::tuple<Tensor, OptTensor> forward(const Tensor& x, const OptTensor& xq, const Batch& batch, double next_quant) const;
 
  private:

@@ -33,7 +33,10 @@ class _Plan:
         for d, k, o in self.slots:
             if d.get(k) is not o:
                 return False
-        return self.native.as_laid_out()
+        state = self.native.state()
+        if state == 1 and not torch.cuda.is_current_stream_capturing():     # (a captured call joins its weights itself)
+            self.native = self.native.refreshed()
+        return state < 2
 
     # copies of a model lay their layers out themselves
     def __deepcopy__(self, memo):

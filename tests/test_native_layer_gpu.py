@@ -127,6 +127,23 @@ def test_operands_follow_the_parameters(kind):
         assert not torch.equal(layer(x, **kw)[0], changed)
 
 
+@pytest.mark.parametrize("kind", ["base", "plus", "mu", "lora"])
+def test_an_update_of_every_parameter_keeps_the_plan(kind):
+    """A training loop changes all weights in each step: the copies are formed again, the layer is not laid out anew."""
+    layer = make_layer(kind)
+    x, ids, pad = batch(80, 2)
+    gy = torch.randn_like(x)
+    run(layer, x, ids, pad, gy)
+    plan = layer._native_plan
+    for _ in range(2):
+        with torch.no_grad():
+            for p in layer.parameters():
+                p.add_(0.05 * torch.randn_like(p))
+        got = run(layer, x, ids, pad, gy)
+        assert layer._native_plan is plan
+        close(got, run(copy.deepcopy(layer), x, ids, pad, gy), 1e-3)
+
+
 def make_twin_value(twin, x, kw):
     twin.__dict__["_native_plan"] = None
     return twin(x, **kw)[0]
