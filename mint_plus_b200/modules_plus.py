@@ -40,7 +40,7 @@ def _linear_res(mod, x, resid, a, b, quant_scale=None):
     """a * resid + b * mod(x) for bf16 CUDA tensors: in the projection's GEMM epilogue for nn.Linear / Fp8Linear, as a
     separate fused pass for wrapped projections (e.g. LoRA adapters)."""
     from .mu_scaling import Fp8Linear
-    if isinstance(mod, Fp8Linear):
+    if isinstance(mod, Fp8Linear) and not mod._observing:
         return mod.forward_res(x, resid, a, b, quant_scale)
     if type(mod) is nn.Linear:
         return ops.linear_res(x, mod.weight, mod.bias, resid, a, b, quant_scale)
@@ -64,7 +64,7 @@ class VanillaFeedForward(nn.Module):
         # (F.gelu's default is the exact erf form too, so both flags give the same function)
         if x.is_cuda and x.dtype == torch.bfloat16:
             from .mu_scaling import Fp8Linear, fp8_ffn
-            if isinstance(self.fc1, Fp8Linear) and isinstance(self.fc2, Fp8Linear):
+            if isinstance(self.fc1, Fp8Linear) and isinstance(self.fc2, Fp8Linear) and not self.fc1._observing:
                 return fp8_ffn(self.fc1, self.fc2, x)    # fc1 hands gelu(.) to fc2 as e4m3: no bf16 copy, no cast pass
             return _linear(self.fc2, _linear(self.fc1, x, gelu=True))
         x = gelu_erf(self.fc1(x)) if self.use_erf_gelu else F.gelu(self.fc1(x))
@@ -86,6 +86,8 @@ def _qkv_operands(attn):
         lora = (torch.stack([m.lora_A for m in mods]), torch.stack([m.lora_B for m in mods]), mods[0].scaling)
         return w, b, None, lora
     if all(isinstance(m, Fp8Linear) for m in mods):
+        if any(m._observing for m in mods):
+            return None
         kind = "fp8"
     elif all(type(m) is nn.Linear for m in mods):
         kind = "bf16"

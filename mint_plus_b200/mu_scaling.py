@@ -146,6 +146,8 @@ class _Fp8FfnFn(torch.autograd.Function):
 class Fp8Linear(nn.Module):
     """Drop-in for nn.Linear (same `weight`, `bias`, `in_features`, `out_features`) computing in e4m3 on the GPU."""
 
+    _observing = False      # while set (by `calibrate_fp8`) the layers call the module instead of fusing its product with its neighbours
+
     def __init__(self, in_features: int, out_features: int, bias: bool = True, x_scale: float = 1.0):
         super().__init__()
         self.in_features, self.out_features = in_features, out_features
@@ -330,6 +332,7 @@ def apply_fp8_to_model(model: nn.Module, static_scale: bool = True, keep_embed_i
 def calibrate_fp8(model: nn.Module, *forward_args, margin: float = 1.0, **forward_kwargs) -> nn.Module:
     """Run one forward pass and set every Fp8Linear's activation scale to amax(input) * margin / 448."""
     hooks, seen = [], {}
+    packed = getattr(model, "pack_padding", False)
 
     def pre_hook(mod, args):
         seen[mod] = max(seen.get(mod, 0.0), float(args[0].detach().abs().amax()))
@@ -337,11 +340,18 @@ def calibrate_fp8(model: nn.Module, *forward_args, margin: float = 1.0, **forwar
     for m in model.modules():
         if isinstance(m, Fp8Linear):
             hooks.append(m.register_forward_pre_hook(pre_hook))
+            m._observing = True
+    if packed:
+        model.pack_padding = False
     try:
         model(*forward_args, **forward_kwargs)
     finally:
         for h in hooks:
             h.remove()
+        for m in model.modules():
+            m.__dict__.pop("_observing", None)
+        if packed:
+            model.pack_padding = True
     for m, amax in seen.items():
         m.x_scale = max(amax * margin, 1e-12) / E4M3_MAX
     return model

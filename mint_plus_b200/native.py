@@ -85,7 +85,7 @@ def _build(layer, mu: bool, fixed) -> Optional[_Plan]:
             return None
     linears = ms + mc + one
     fp8 = type(linears[0]) is Fp8Linear
-    if any(type(m) is not (Fp8Linear if fp8 else nn.Linear) for m in linears):
+    if any(type(m) is not (Fp8Linear if fp8 else nn.Linear) for m in linears) or (fp8 and any(m._observing for m in linears)):
         return None
     for mods in (ms, mc):
         if len({m.bias is None for m in mods}) != 1 or len({m.weight.dtype for m in mods}) != 1:
@@ -133,7 +133,7 @@ def _build(layer, mu: bool, fixed) -> Optional[_Plan]:
         wq = [m._quantized_weight() for m in one]
         o, f1, f2 = (L.host().Operand(w, s, m.x_scale, m.out_scale, h) for (w, s), m, h in zip(wq, one, holders[1:]))
         for m in linears:
-            p.slots += [(m.__dict__, k, m.__dict__.get(k)) for k in ("_wq", "x_scale", "out_scale", "fp8_grads", "grad_scale")]
+            p.slots += [(m.__dict__, k, m.__dict__.get(k)) for k in ("_wq", "x_scale", "out_scale", "fp8_grads", "grad_scale", "_observing")]
         p.slots += [(h.__dict__, "scale", h.scale) for h in holders if h is not None]
         p.slots += [(a.__dict__, "_fp8_qkv_grad_scale", a.__dict__.get("_fp8_qkv_grad_scale")) for a in (sa, ma)]
         p.x_scale = f8s[2]
