@@ -241,15 +241,17 @@ def fused_fp8_weight(owner: nn.Module, mods):
 
 
 def refresh_fp8_weights(model: nn.Module) -> nn.Module:
-    """Drop every cached e4m3 weight copy of `model`, so that the next forward pass casts the master weights again.
+    """Drop every cached copy of weights of `model` (e4m3 copies, the layers' joint QKV operands), so that the next forward pass forms
+    them from the master weights again.
     The caches notice in-place updates of a Parameter (optimizer steps, `weight.copy_`), which bump its version counter;
     writes through `weight.data` (sharded or apex-style optimizers, broadcasts into `.data`) do not - call this after such
     a write, or the forward pass keeps multiplying by the old e4m3 weights."""
     for m in model.modules():
         if isinstance(m, Fp8Linear):
             m._wq, m._wq_key = None, None
-        if getattr(m, "_fp8_qkv_cache", None) is not None:
-            m._fp8_qkv_cache = None
+        for k in ("_fp8_qkv_cache", "_qkv6_cache", "_native_plan"):
+            if getattr(m, k, None) is not None:
+                setattr(m, k, None)
     return model
 
 

@@ -305,6 +305,19 @@ def test_weights_replaced_through_data_are_followed(kind, how, monkeypatch):
     assert (got - before).abs().max() > 0.05
 
 
+@pytest.mark.parametrize("kind", ["base", "mu_fp8"])
+def test_refresh_takes_in_writes_that_leave_no_trace(kind, monkeypatch):
+    """In-place writes through .data, which neither move a weight nor count as a version, into a joint copy and e4m3 copies."""
+    layer = make_layer(kind)
+    x, ids, pad = batch(64, 2)
+    before = values(layer, x, ids, pad)
+    for m in (layer.self_attn.q_proj, layer.multimer_attn.v_proj, layer.feed_forward.fc1):
+        m.weight.data.mul_(-1)
+    M.refresh_fp8_weights(layer)
+    got = equal_to_composed(layer, x, ids, pad, monkeypatch)
+    assert torch.equal(got, values(copy.deepcopy(layer), x, ids, pad)) and (got - before).abs().max() > 0.05
+
+
 def test_a_changed_logit_scale_is_followed(monkeypatch):
     layer = make_layer("plus")
     x, ids, pad = batch(64, 2)
