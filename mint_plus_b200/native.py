@@ -4,8 +4,14 @@ and backward pass take, formed once and kept on the layer until one of them chan
 A layer is served here when it is what the builders make: bf16 activations on the GPU, nn.Linear projections with bf16 weights
 (with or without LoRA adapters on a frozen base) or Fp8Linear ones throughout, LayerNorms with parameters, the fused attention, a
 VanillaFeedForward, and none of the methods that this file stands in for overridden.
-Everything else (wrapped projections, mixed kinds) stays on the modules' own path; plain fp32 layers have a short one of their own at
-the end of this file.
+
+The modules' own path (modules_plus.py, mu_scaling.py on the operators of ops.py) serves the rest, and has to stay for it:
+* layers with fp32 weights under bf16 activations, RMSNorm, mixed kinds of projections or foreign ones, blocks and attentions of a subclass;
+* LoRA with dropout, on fused or on some projections only, of a rank that is no multiple of eight, on trainable bases or above 1870 columns;
+* FP8 layers without 8-bit gradients while gradients are on, or whose pathways have different activation scales, and calibration;
+* layers while hooks are registered on their block or a wrapped output projection, or module-wide ones;
+* MINTB_FUSE_OUT_RESIDUAL=0, the materialised-logits combine, single-pathway layers;
+* everything in fp32 with gradients: run_layer_f32 at the end of this file serves plain fp32 Pre-LN layers without them.
 """
 from __future__ import annotations
 
