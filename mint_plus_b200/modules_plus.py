@@ -299,13 +299,15 @@ _ids_meta_cache = []
 
 
 def _cached_ids_meta(chain_ids, padding_mask):
-    capture = ops.capture_id(chain_ids)
-    for ids, ver, pad, cap, meta in _ids_meta_cache:
-        if ids is chain_ids and ver == chain_ids._version and pad is padding_mask and cap == capture:
-            return meta
+    capture, ver = ops.capture_id(chain_ids), ops.versions(chain_ids, padding_mask)
+    if ver is not None:
+        for ids, pad, v, cap, meta in _ids_meta_cache:
+            if ids is chain_ids and pad is padding_mask and v == ver and cap == capture:
+                return meta
     meta = ops.mask_meta_from_chain_ids(chain_ids, padding_mask)
-    _ids_meta_cache.insert(0, (chain_ids, chain_ids._version, padding_mask, capture, meta))
-    del _ids_meta_cache[2:]
+    if ver is not None:
+        _ids_meta_cache.insert(0, (chain_ids, padding_mask, ver, capture, meta))
+        del _ids_meta_cache[2:]
     return meta
 
 

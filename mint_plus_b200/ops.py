@@ -111,25 +111,28 @@ def capture_id(t: torch.Tensor) -> int:
     return L.host().capture_id(t) if t.is_cuda and torch.cuda.is_current_stream_capturing() else 0
 
 
-_meta_cache = []  # [(weakref(mask), version, weakref(pad) | None, pad version, capture, MaskMeta)], newest first
+def versions(*tensors) -> Optional[tuple]:
+    """What tells that these tensors (or None) have been written in place; None where one of them, made in inference mode, does not count."""
+    if any(t is not None and t.is_inference() for t in tensors):
+        return None
+    return tuple(0 if t is None else t._version for t in tensors)
+
+
+_meta_cache = []  # [(weakref(mask), weakref(pad) | None, their versions, capture, MaskMeta)], newest first
 
 
 def cached_mask_meta(chain_mask: torch.Tensor, key_padding_mask: Optional[torch.Tensor] = None) -> MaskMeta:
     """Metadata for a (B,T,T) mask, reused while the same tensor objects are passed again (every layer of a
     forward pass receives the same mask, esm2.py:124-132)."""
-    capture = capture_id(chain_mask)
-    for ref_m, ver_m, ref_p, ver_p, cap, meta in _meta_cache:
-        if ref_m() is chain_mask and ver_m == chain_mask._version and cap == capture:
-            if key_padding_mask is None and ref_p is None:
-                return meta
-            if key_padding_mask is not None and ref_p is not None and ref_p() is key_padding_mask \
-                    and ver_p == key_padding_mask._version:
+    capture, ver = capture_id(chain_mask), versions(chain_mask, key_padding_mask)
+    if ver is not None:
+        for ref_m, ref_p, v, cap, meta in _meta_cache:
+            if v == ver and cap == capture and ref_m() is chain_mask and (ref_p is None if key_padding_mask is None else ref_p is not None and ref_p() is key_padding_mask):
                 return meta
     meta = mask_meta_from_mask(chain_mask, key_padding_mask)
-    _meta_cache.insert(0, (weakref.ref(chain_mask), chain_mask._version,
-                           None if key_padding_mask is None else weakref.ref(key_padding_mask),
-                           0 if key_padding_mask is None else key_padding_mask._version, capture, meta))
-    del _meta_cache[4:]
+    if ver is not None:
+        _meta_cache.insert(0, (weakref.ref(chain_mask), None if key_padding_mask is None else weakref.ref(key_padding_mask), ver, capture, meta))
+        del _meta_cache[4:]
     return meta
 
 

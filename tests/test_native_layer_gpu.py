@@ -458,3 +458,17 @@ def test_calibration_measures_the_inputs_of_every_projection(packed):
     with torch.no_grad():
         after = twin(tokens, ids)["logits"]
     assert twin.layers[0]._native_plan is not None and not torch.equal(before, after)
+
+
+@pytest.mark.parametrize("mode", [torch.no_grad, torch.inference_mode])
+def test_masks_written_in_place_are_noticed(mode):
+    """Chain ids and padding in static buffers, changed between two calls of a layer."""
+    layer = make_layer("plus")
+    x, ids, pad = batch(70, 3)
+    with mode():
+        ids, pad = ids.clone(), pad.clone()
+        for change in (lambda: pad.copy_(pad.roll(1, 0)), lambda: ids.copy_(1 - ids.flip(1))):
+            before = values(layer, x, ids, pad)
+            change()
+            got = values(layer, x, ids, pad)
+            assert torch.equal(got, values(layer, x, ids.clone(), pad.clone())) and not torch.equal(got, before)
