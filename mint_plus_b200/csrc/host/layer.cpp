@@ -72,6 +72,7 @@ static Tensor concatenated(at::TensorList parts) {
 void LayerPlan::form() {
   const Where at(*this);
   TORCH_CHECK(int64_t(params.size()) == at.n, "a layer plan needs ", at.n, " parameters, got ", params.size());
+  c10::InferenceMode normal(false);   // (copies that a pass in inference mode leaves serve the training step after it)
   at::AutoDispatchBelowADInplaceOrView below;
   const at::TensorList all(params);
   const at::TensorList ws = all.slice(at.ws, n_self), wc = all.slice(at.wc, n_cross), bs = all.slice(at.bs, n_self), bc = all.slice(at.bc, n_cross);
@@ -111,7 +112,8 @@ int LayerPlan::state() const {
     if (!t.defined()) continue;
     const Stamp& s = stamps[k];
     if (t.scalar_type() != s.dtype || !t.is_contiguous() || !t.is_cuda()) return kOther;
-    written = written || (s.copied && (t.data_ptr() != s.data || version_of(t) != s.version));
+    // (a parameter made in inference mode does not count its writes: its copies are formed in every call)
+    written = written || (s.copied && (t.data_ptr() != s.data || t.is_inference() || version_of(t) != s.version));
   }
   return !written ? kCurrent : fp8 ? kOther : kWritten;
 }
@@ -127,6 +129,11 @@ std::tuple<Tensor, OptTensor> LayerPlan::forward(const Tensor& x, const OptTenso
   // Separate projections too large to be kept in a joint copy, their biases, and a frozen base's biases are joined in every call.  A
   // captured call joins everything itself, so that its replays follow the weights and hold the copies in the graph's own memory.
   c10::cuda::CUDAGuard guard(x.device());
+  if (c10::InferenceMode::is_enabled()) {   // results as tensors that count their writes: the e4m3 copy beside one is valid until the next
+    c10::InferenceMode normal(false);
+    at::NoGradGuard no_grad;
+    return forward(x, xq, batch, next_quant);
+  }
   if ((!fp8 && capture_id(x) != 0) || (!joint && (lora_r > 0 || n_self > 1 || n_cross > 1))) {
     LayerPlan now = *this;
     now.form();

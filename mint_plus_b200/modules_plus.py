@@ -125,7 +125,7 @@ def _fused6_operands(layer, ops_s, ops_c):
     capturing = ops.capture_id(w_s) != 0
     if cached is not None and cached[0] == key and (f8_s is not None or not capturing):
         return cached[1], cached[2]
-    with torch.no_grad():
+    with ops.normal_tensors():
         if f8_s is not None:
             w6 = torch.cat([f8_s[0].view(torch.uint8), f8_c[0].view(torch.uint8)], dim=0).view(torch.float8_e4m3fn)
         else:

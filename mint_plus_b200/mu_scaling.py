@@ -174,10 +174,11 @@ class Fp8Linear(nn.Module):
     def _quantized_weight(self):
         key = (self.weight.data_ptr(), self.weight._version, self.weight.device)
         if self._wq is None or self._wq_key != key:
-            w = self.weight.detach()
-            amax = float(w.abs().amax())                      # host sync, only when the weight has changed
-            self._w_scale = max(amax, 1e-12) / E4M3_MAX
-            self._wq = ops.quantize_e4m3(w.to(torch.bfloat16).contiguous(), self._w_scale)
+            with ops.normal_tensors():
+                w = self.weight.detach()
+                amax = float(w.abs().amax())                  # host sync, only when the weight has changed
+                self._w_scale = max(amax, 1e-12) / E4M3_MAX
+                self._wq = ops.quantize_e4m3(w.to(torch.bfloat16).contiguous(), self._w_scale)
             self._wq_key = key
         return self._wq, self._w_scale
 
@@ -232,9 +233,10 @@ def fused_fp8_weight(owner: nn.Module, mods):
     key = tuple((m.weight.data_ptr(), m.weight._version) for m in mods)
     cached = getattr(owner, "_fp8_qkv_cache", None)
     if cached is None or cached[0] != key:
-        w = torch.cat([m.weight.detach() for m in mods], dim=0)
         w_scale = max(m._quantized_weight()[1] for m in mods)   # amax of the concatenation / 448; a host read only where a copy is stale
-        cached = (key, ops.quantize_e4m3(w.to(torch.bfloat16).contiguous(), w_scale), w_scale)
+        with ops.normal_tensors():
+            w = torch.cat([m.weight.detach() for m in mods], dim=0)
+            cached = (key, ops.quantize_e4m3(w.to(torch.bfloat16).contiguous(), w_scale), w_scale)
         if not ops.capture_id(w):     # (what a capture forms exists in its replays only)
             owner._fp8_qkv_cache = cached
     return cached[1], cached[2], max(m.x_scale for m in mods), mods[0].out_scale, (owner._fp8_qkv_grad_scale if f8_grads else None)
@@ -272,10 +274,12 @@ class Fp8WeightScaler:
         self._host = None
         self._event = None
 
-    @torch.no_grad()
     def refresh(self) -> None:
-        if not self.mods:
-            return
+        if self.mods:
+            with ops.normal_tensors():
+                self._refresh()
+
+    def _refresh(self) -> None:
         ws = [m.weight.detach() for m in self.mods]
         amax = torch.stack([a.float() for a in torch._foreach_norm(ws, float("inf"))])
         if self._host is None:

@@ -144,7 +144,8 @@ def _build(layer, mu: bool, fixed) -> Optional[_Plan]:
         p.slots += [(a.__dict__, "_fp8_qkv_grad_scale", a.__dict__.get("_fp8_qkv_grad_scale")) for a in (sa, ma)]
         p.x_scale = f8s[2]
         if joint:
-            qkv6 = torch.cat([f8s[0].view(torch.uint8), f8c[0].view(torch.uint8)]).view(torch.float8_e4m3fn)
+            with ops.normal_tensors():
+                qkv6 = torch.cat([f8s[0].view(torch.uint8), f8c[0].view(torch.uint8)]).view(torch.float8_e4m3fn)
     else:
         p.can_grad, p.x_scale = True, 0.0
         if adapters is not None and bias_s != bias_c:

@@ -4,6 +4,7 @@ every computation runs in the CUDA library (there is no eager fallback).
 """
 from __future__ import annotations
 
+import contextlib
 import weakref
 from typing import Optional, Tuple
 
@@ -111,6 +112,13 @@ def capture_id(t: torch.Tensor) -> int:
     return L.host().capture_id(t) if t.is_cuda and torch.cuda.is_current_stream_capturing() else 0
 
 
+@contextlib.contextmanager
+def normal_tensors():
+    """What is kept from one call for the next is made outside inference mode: its tensors cannot be saved for a backward pass."""
+    with torch.inference_mode(False), torch.no_grad():
+        yield
+
+
 def versions(*tensors) -> Optional[tuple]:
     """What tells that these tensors (or None) have been written in place; None where one of them, made in inference mode, does not count."""
     if any(t is not None and t.is_inference() for t in tensors):
@@ -152,20 +160,22 @@ def rope_tables(T: int, D: int, device,
     without one) for as long as it lives and holds what they were made from.  A table that a longer one replaces is kept as well: a
     captured graph may read it (lengths at least double, so all of them together are no more than twice the longest)."""
     device = torch.device(device)
-    made_from = (D, device.index) if inv_freq is None else (D, device.index, inv_freq.data_ptr(), inv_freq._version)
+    ver = versions(inv_freq)
+    made_from = (D, device.index) if inv_freq is None else (D, device.index, inv_freq.data_ptr(), ver)
     hit = _rope_default.get(made_from) if inv_freq is None else _rope_cache.get(inv_freq)
-    if hit is not None and hit[3] != made_from:
+    if hit is not None and (hit[3] != made_from or ver is None):
         hit = None
     if hit is not None and T in hit[2]:
         return (*hit[2][T], inv_freq)
     if hit is None or T > hit[0].shape[0]:
         # row t depends on t alone, so the table of the longest length seen so far serves the shorter ones
         rows = max((T + 255) // 256 * 256, 0 if hit is None else 2 * hit[0].shape[0])
-        inv = default_inv_freq(D, device) if inv_freq is None else inv_freq.detach().to(device=device, dtype=torch.float32).contiguous()
-        if inv.numel() != D // 2:
-            raise ValueError(f"inv_freq must have D/2 = {D // 2} entries")
-        cos = torch.empty(rows, D // 2, dtype=torch.float32, device=device)
-        sin = torch.empty_like(cos)
+        with normal_tensors():
+            inv = default_inv_freq(D, device) if inv_freq is None else inv_freq.detach().to(device=device, dtype=torch.float32).contiguous()
+            if inv.numel() != D // 2:
+                raise ValueError(f"inv_freq must have D/2 = {D // 2} entries")
+            cos = torch.empty(rows, D // 2, dtype=torch.float32, device=device)
+            sin = torch.empty_like(cos)
         with _on(device):
             L.check(L.lib().mintb_rope_tables(_ptr(inv), _ptr(cos), _ptr(sin), rows, D, _stream()), "rope_tables")
         hit = (cos, sin, {}, made_from, hit)
@@ -177,7 +187,8 @@ def rope_tables(T: int, D: int, device,
             _rope_cache[inv_freq] = hit
     if len(hit[2]) >= 64:
         hit[2].clear()
-    hit[2][T] = (hit[0][:T], hit[1][:T])
+    with normal_tensors():
+        hit[2][T] = (hit[0][:T], hit[1][:T])
     return (*hit[2][T], inv_freq)
 
 
@@ -367,8 +378,10 @@ def quantize_e4m3(x: torch.Tensor, scale: float) -> torch.Tensor:
 
 def attach_e4m3(t: torch.Tensor, q8: torch.Tensor, scale: float) -> None:
     """Hand the e4m3 copy of `t` (cast with `scale`) to whoever receives `t` next: the copy rides on the tensor object itself.
-    The pass that produced `t` (a fused residual + LayerNorm) wrote it for the e4m3 projections that read `t` next."""
-    t._mintb_e4m3 = (q8, float(scale), t._version)
+    The pass that produced `t` (a fused residual + LayerNorm) wrote it for the e4m3 projections that read `t` next.  A tensor of
+    inference mode, which does not count its writes, carries none."""
+    if not t.is_inference():
+        t._mintb_e4m3 = (q8, float(scale), t._version)
 
 
 def attached_e4m3(t: torch.Tensor, scale: float) -> Optional[torch.Tensor]:

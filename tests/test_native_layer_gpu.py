@@ -472,3 +472,37 @@ def test_masks_written_in_place_are_noticed(mode):
             change()
             got = values(layer, x, ids, pad)
             assert torch.equal(got, values(layer, x, ids.clone(), pad.clone())) and not torch.equal(got, before)
+
+
+@pytest.mark.parametrize("kind", ["base", "plus", "mu", "lora", "mu_fp8", "base_fp8"])
+@pytest.mark.parametrize("served", [True, False])
+def test_training_goes_on_after_a_pass_in_inference_mode(kind, served, monkeypatch):
+    """What a validation pass under torch.inference_mode leaves behind serves the training step that follows it."""
+    if not served:
+        monkeypatch.setattr(native, "run_layer", lambda *a, **k: None)
+    layer = make_layer(kind)
+    x, ids, pad = batch(80, 2)
+    gy = torch.randn_like(x)
+    with torch.inference_mode():
+        first = layer(x, self_attn_padding_mask=pad, chain_ids=ids)[0].clone()
+    got = run(layer, x, ids, pad, gy)
+    assert torch.equal(got[0], first)
+    close(got, run(copy.deepcopy(layer), x, ids, pad, gy), 1e-3)
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+def test_a_model_in_inference_mode(fp8):
+    """Same logits as without gradients, whatever mode the batch was made in, and a training step afterwards."""
+    torch.manual_seed(0)
+    model = M.build_mint_mu("8M", num_layers=3, use_fp8=fp8, embed_dim=128, attention_heads=4).to(DEV).to(torch.bfloat16)
+    tokens = torch.randint(4, 24, (2, 60), device=DEV)
+    ids = (torch.arange(60, device=DEV) > 30).long().expand(2, 60).contiguous()
+    model.eval()
+    with torch.inference_mode():
+        got = model(tokens, ids)["logits"].clone()
+        assert torch.equal(model(tokens.clone(), ids.clone())["logits"], got)
+    with torch.no_grad():
+        assert torch.equal(model(tokens, ids)["logits"], got)
+    model.train()
+    M.shared_step(model, (tokens, ids))[0].backward()
+    assert all(p.grad is not None and p.grad.isfinite().all() for p in model.parameters())
