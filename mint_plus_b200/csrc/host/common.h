@@ -137,9 +137,15 @@ struct NormGrad {
 NormGrad add_layernorm_bwd(const Tensor& dy, const Tensor& ds, const Tensor& x, const Tensor& r, double a, double b, const Tensor& gamma, const Tensor& stats,
                            bool want_params, bool ds_apart = false);   // ds_apart: ds is added to the rounded dx
 
+// The operators have no forward-mode derivative: a tangent on an input is an error and not dropped.
+inline void no_tangent(const Tensor& t) {
+  TORCH_CHECK_NOT_IMPLEMENTED(!t.defined() || !t._fw_grad(0).defined(), "mint_plus_b200 operators have no forward-mode derivative");
+}
+
 // Which inputs of a call want gradients, as a node of the autograd graph; nullptr when none does.
 template <typename N>
 std::shared_ptr<N> make_node(const std::vector<Tensor>& inputs) {
+  for (const Tensor& t : inputs) no_tangent(t);
   if (!at::GradMode::is_enabled()) return nullptr;
   bool any = false;
   for (const Tensor& t : inputs) any = any || (t.defined() && t.requires_grad());

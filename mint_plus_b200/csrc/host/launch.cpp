@@ -72,6 +72,7 @@ std::pair<Tensor, Tensor> linear_res_fwd(const Product& p, const Tensor& resid, 
 }
 
 Tensor linear_f32(const Tensor& x, const Tensor& w, const OptTensor& bias, bool gelu, const OptTensor& resid) {
+  for (const Tensor& t : {x, w, opt(bias), opt(resid)}) no_tangent(t);
   Env e(x);
   const int64_t K = w.size(1), N = w.size(0), M = x.numel() / K;
   TORCH_CHECK(x.size(-1) == K && x.is_contiguous() && w.is_contiguous(), "linear_f32: contiguous rows of the weight's width are required");
@@ -92,7 +93,10 @@ std::vector<Tensor> heads_f32(const Tensor& x, const std::vector<Tensor>& w, con
   std::vector<const float*> wp, bp;
   std::vector<float*> op;
   std::vector<Tensor> out;
+  no_tangent(x);
   for (size_t i = 0; i < w.size(); ++i) {
+    no_tangent(w[i]);
+    no_tangent(opt(bias[i]));
     TORCH_CHECK(x.is_contiguous() && w[i].is_contiguous() && w[i].size(1) == E && w[i].size(0) % E == 0, "heads_f32: contiguous (n E, E) weights are required");
     for (int64_t k = 0; k < w[i].size(0) / E; ++k) {
       wp.push_back(fptr(w[i]) + k * E * E);

@@ -506,3 +506,26 @@ def test_a_model_in_inference_mode(fp8):
     model.train()
     M.shared_step(model, (tokens, ids))[0].backward()
     assert all(p.grad is not None and p.grad.isfinite().all() for p in model.parameters())
+
+
+@pytest.mark.parametrize("what", ["attention", "combine", "linear", "norm", "layer", "layer_f32", "loss"])
+@pytest.mark.parametrize("grad", [True, False])
+def test_a_tangent_is_refused(what, grad):
+    """The operators have no forward-mode derivative; a tangent that was dropped would read as zero."""
+    from torch.autograd import forward_ad as fw
+    x, ids, pad = batch(32, 2)
+    layer = make_layer("plus")
+    meta = M.mask_meta_from_chain_ids(ids, pad)
+    with fw.dual_level(), torch.set_grad_enabled(grad):
+        dual = lambda t: fw.make_dual(t, torch.ones_like(t))
+        heads = [torch.randn(2, H, 32, E // H, device=DEV).bfloat16() for _ in range(6)]
+        logits = torch.randn(2, 3, 32, 32, device=DEV)
+        call = {"attention": lambda: M.multimer_attention(*heads[:5], dual(heads[5]), meta=meta),
+                "combine": lambda: M.fused_multimer_combine(dual(logits), logits, torch.zeros(2, 32, 32, dtype=torch.bool, device=DEV), *[torch.randn(2, 3, 32, 16, device=DEV)] * 2),
+                "linear": lambda: ops.linear(dual(x), layer.feed_forward.fc1.weight, layer.feed_forward.fc1.bias),
+                "norm": lambda: ops.add_layernorm(dual(x), None, 1.0, 0.0, layer.final_layer_norm),
+                "layer": lambda: layer(dual(x), self_attn_padding_mask=pad, chain_ids=ids),
+                "layer_f32": lambda: layer.float()(dual(x.float()), self_attn_padding_mask=pad, chain_ids=ids),
+                "loss": lambda: ops.masked_cross_entropy(dual(torch.randn(2, 32, 40, device=DEV).bfloat16()), ids, ~pad)}[what]
+        with pytest.raises(NotImplementedError):
+            call()
