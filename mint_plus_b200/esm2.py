@@ -131,12 +131,12 @@ class MINT(nn.Module):
     def forward(self, tokens: torch.Tensor, chain_ids: Optional[torch.Tensor] = None,
                 repr_layers: List[int] = []) -> Dict[str, torch.Tensor]:
         assert tokens.ndim == 2
-        with torch.inference_mode(False):       # (the layers share metadata of these two while their versions stand)
-            padding_mask = tokens.eq(self.padding_idx)                # B, T
-            if chain_ids is None:
-                chain_ids = torch.zeros_like(tokens)
-            elif chain_ids.is_inference():
-                chain_ids = chain_ids.clone()
+        padding_mask = tokens.eq(self.padding_idx)                    # B, T
+        if chain_ids is None:
+            chain_ids = torch.zeros_like(tokens)
+        if padding_mask.is_inference() or chain_ids.is_inference():
+            with torch.inference_mode(False):   # the layers share metadata of these two while their versions stand: tensors that have one
+                padding_mask, chain_ids = padding_mask.clone(), chain_ids.clone()
         self_attn_mask = None
         if self._needs_dense_mask():
             self_attn_mask = ~torch.eq(chain_ids.unsqueeze(-1), chain_ids.unsqueeze(-2))      # B, T, T; True = other chain

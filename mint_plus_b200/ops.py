@@ -9,7 +9,6 @@ import weakref
 from typing import Optional, Tuple
 
 import torch
-from torch.utils.weak import WeakIdKeyDictionary
 
 from . import _lib as L
 
@@ -119,11 +118,12 @@ def normal_tensors():
         yield
 
 
-def versions(*tensors) -> Optional[tuple]:
-    """What tells that these tensors (or None) have been written in place; None where one of them, made in inference mode, does not count."""
-    if any(t is not None and t.is_inference() for t in tensors):
+def versions(a: torch.Tensor, b: Optional[torch.Tensor] = None) -> Optional[tuple]:
+    """What tells that these tensors have been written in place; None where one of them, made in inference mode, does not count."""
+    try:
+        return (a._version, 0 if b is None else b._version)
+    except RuntimeError:
         return None
-    return tuple(0 if t is None else t._version for t in tensors)
 
 
 _meta_cache = []  # [(weakref(mask), weakref(pad) | None, their versions, capture, MaskMeta)], newest first
@@ -145,7 +145,7 @@ def cached_mask_meta(chain_mask: torch.Tensor, key_padding_mask: Optional[torch.
 
 
 # ----------------------------------------------------------------------------------------------- RoPE tables
-_rope_cache = WeakIdKeyDictionary()      # inv_freq buffer -> its tables; they go when it goes
+_rope_cache = {}                         # id of an inv_freq buffer -> (weak reference to it, its tables); they go when it goes
 _rope_default = {}                       # (D, device) -> the tables of the default frequencies
 
 
@@ -160,11 +160,15 @@ def rope_tables(T: int, D: int, device,
     without one) for as long as it lives and holds what they were made from.  A table that a longer one replaces is kept as well: a
     captured graph may read it (lengths at least double, so all of them together are no more than twice the longest)."""
     device = torch.device(device)
-    ver = versions(inv_freq)
-    made_from = (D, device.index) if inv_freq is None else (D, device.index, inv_freq.data_ptr(), ver)
-    hit = _rope_default.get(made_from) if inv_freq is None else _rope_cache.get(inv_freq)
-    if hit is not None and (hit[3] != made_from or ver is None):
-        hit = None
+    if inv_freq is None:
+        made_from = (D, device.index)
+        hit = _rope_default.get(made_from)
+    else:
+        ver = versions(inv_freq)
+        made_from = (D, device.index, inv_freq.data_ptr(), ver)
+        ref, hit = _rope_cache.get(id(inv_freq), (None, None))
+        if hit is not None and (ref() is not inv_freq or hit[3] != made_from or ver is None):
+            hit = None
     if hit is not None and T in hit[2]:
         return (*hit[2][T], inv_freq)
     if hit is None or T > hit[0].shape[0]:
@@ -184,7 +188,8 @@ def rope_tables(T: int, D: int, device,
         if inv_freq is None:
             _rope_default[made_from] = hit
         else:
-            _rope_cache[inv_freq] = hit
+            key = id(inv_freq)
+            _rope_cache[key] = (weakref.ref(inv_freq, lambda r: _rope_cache.pop(key) if _rope_cache.get(key, (None,))[0] is r else None), hit)
     if len(hit[2]) >= 64:
         hit[2].clear()
     with normal_tensors():
