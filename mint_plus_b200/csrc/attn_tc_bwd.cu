@@ -70,6 +70,18 @@ static bool bwd_make_dq_map(CUtensorMap* m, const void* ptr, int D, int T, int B
             CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// mask words, key-major: [B][T][TW] with a box of the 4 words (128 queries) of 128 keys
+static bool bwd_make_bits_map(CUtensorMap* m, const void* ptr, int TW, int T, int B) {
+  EncodeTiledFn fn = bwd_encode_fn();
+  if (fn == nullptr) return false;
+  cuuint64_t dims[3] = {cuuint64_t(TW), cuuint64_t(T), cuuint64_t(B)};
+  cuuint64_t strides[2] = {cuuint64_t(TW) * 4, cuuint64_t(T) * TW * 4};
+  cuuint32_t box[3] = {4, cuuint32_t(kBwdTile), 1};
+  cuuint32_t es[3] = {1, 1, 1};
+  return fn(m, CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, const_cast<void*>(ptr), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 __device__ __forceinline__ float bwd_ex2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -226,23 +238,32 @@ struct BwdCfg {
   static constexpr int kDqStages = D <= 32 ? 2 : 1;
   static constexpr int kDqQuarterBytes = 32 * D * 4;            // staging of the 32 queries of one TMEM quarter
   static constexpr int kStatBytes = 128 * 8;                     // softmax statistics of one query tile: 128 x (-lse log2 e, -delta)
+  static constexpr int kMaskBytes = kBwdTile * 16;               // mask words of one tile: 128 keys x 128 queries
   static constexpr size_t kSmemBytes = 1024 + size_t(kK + kV) * kTileBytes + size_t(kQStages) * 2 * kTileBytes + size_t(kNDq) * kDsBytes +
-                                       size_t(kDqStages) * 4 * kDqQuarterBytes + kQStages * kStatBytes + 3072;
+                                       size_t(kDqStages) * 4 * kDqQuarterBytes + kQStages * (kStatBytes + kMaskBytes) + 3072;
 };
 
 // One work item - the dK, dV of a key tile in one pathway - as the loading warp hands it to the other roles.
 struct BwdPlan {
   int n;                           // query tiles with pairs of the pathway; 0: no more items
   int kt, bh, path;
-  uint32_t flip;                   // a query belongs to the pathway where mask bit XOR flip
-  uint32_t kpad[4];                // padding bits of the tile's 128 keys
   uint16_t tiles[kBwdMaxTiles];    // their numbers, kMixed set where the tile needs the chain mask
 };
 constexpr uint16_t kMixed = 0x8000;
 constexpr int kPlans = 2;          // the one being computed and the next
 
+// What the compute warps have to know of a tile, beside its statistics and mask words in the same stage: they work through one stream
+// of tiles and never look at the items they belong to.
+struct BwdTile {
+  uint32_t flags;
+  uint32_t flip;                   // a query belongs to the pathway where mask bit XOR flip
+  uint32_t unused[2];
+  uint32_t kpad[4];                // padding bits of the tile's 128 keys
+};
+constexpr uint32_t kTileEnd = 1, kTileMasked = 2, kTileMixed = 4;   // no more tiles; some pairs do not count; the mask words were loaded
+
 struct BwdParams {
-  const uint32_t *bitsT, *kpad;
+  const uint32_t* kpad;
   const uint8_t* cls;
   const float2* stats;             // [B*H][Tpad / 2] x (nl0, nl1, nd0, nd1): -lse * log2 e and -delta of two queries, Tpad = T rounded up to 128
   const float *cos_tab, *sin_tab;  // null without rope
@@ -275,13 +296,18 @@ struct Ring {
 // next CTA 2000 to 3000) against 2200 and 3100 cycles per query tile.  Here barriers and TMEM are set up once; the loading warp
 // plans and loads the next key tile while the current one is computed; and four warps of their own take the results away while the
 // compute warps go on with the next key tile.  B8 H20 T1024 D32: kernel 265 -> 175 us; B5 H20 T1531 D64 square root: 295 -> 250 us.
+// The compute warps do not know of key tiles: the loading warp puts a descriptor of each tile, its statistics and, by TMA, its mask words
+// into the tile's stage, and one barrier stands for all of it and the products (three waits, a plan and a mask word from global memory
+// before: 175 -> 160 us).  The roles' code is kept short, for with 24 warps in seven roles the kernel waits for instructions (the waits in
+// ptx.cuh, loops of the result warps not unrolled): -> 130 us; at D64 250 -> 235, where a buffer's round through the products and back
+// (1700 of the tile's 5400 cycles) takes the rest.
 template <int D, bool SQ>
 __global__ void __launch_bounds__(BwdCfg<D>::kThreads, 1)
 attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_constant__ CUtensorMap map_ks,
                    const __grid_constant__ CUtensorMap map_vs, const __grid_constant__ CUtensorMap map_qc,
                    const __grid_constant__ CUtensorMap map_kc, const __grid_constant__ CUtensorMap map_vc,
                    const __grid_constant__ CUtensorMap map_do, const __grid_constant__ CUtensorMap map_dq_s,
-                   const __grid_constant__ CUtensorMap map_dq_c, BwdParams p) {
+                   const __grid_constant__ CUtensorMap map_dq_c, const __grid_constant__ CUtensorMap map_bits, BwdParams p) {
   using Cfg = BwdCfg<D>;
   constexpr int RB = Cfg::kRowBytes, kNBuf = Cfg::kNBuf, kQStages = Cfg::kQStages, kNDq = Cfg::kNDq, kK = Cfg::kK, kV = Cfg::kV;
   constexpr int kColDK = Cfg::kColDK, kColDV = Cfg::kColDV, kColDQ = Cfg::kColDQ, kColBuf = Cfg::kColBuf, kAcc = Cfg::kAcc;
@@ -293,7 +319,8 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
   unsigned char* sDS = sQ + size_t(kQStages) * 2 * Cfg::kTileBytes;  // [buf][half][128 rows x 128 B]
   unsigned char* sDqStage = sDS + size_t(kNDq) * Cfg::kDsBytes;      // [stage][quarter][column box][32 queries][kDqCols fp32], swizzled
   unsigned char* sStats = sDqStage + size_t(Cfg::kDqStages) * 4 * Cfg::kDqQuarterBytes;   // [stage][64] x (nl0, nl1, nd0, nd1), loaded with the query tile
-  unsigned char* tail = sStats + size_t(kQStages) * Cfg::kStatBytes;
+  unsigned char* sMask = sStats + size_t(kQStages) * Cfg::kStatBytes;    // [stage][128 keys][4 words], loaded likewise for tiles that need it
+  unsigned char* tail = sMask + size_t(kQStages) * Cfg::kMaskBytes;
   uint64_t* bars = reinterpret_cast<uint64_t*>(tail);
   uint64_t* plan_full = bars;           // [4]
   uint64_t* plan_empty = bars + 4;      // [4]
@@ -301,8 +328,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
   uint64_t* k_empty = bars + 10;        // [2]
   uint64_t* v_full = bars + 12;         // [2]
   uint64_t* v_empty = bars + 14;        // [2]
-  uint64_t* q_full = bars + 16;         // [4] Q_i and dO_i
-  uint64_t* st_full = bars + 20;        // [4] the statistics
+  uint64_t* q_full = bars + 16;         // [4] Q_i and dO_i, statistics, mask words and descriptor
   uint64_t* q_empty = bars + 24;        // [4]
   uint64_t* sdp_full = bars + 28;       // [3 buffers]
   uint64_t* pds_full = bars + 31;       // [3 buffers]
@@ -312,14 +338,15 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
   uint64_t* acc_full = bars + 41;
   uint64_t* acc_empty = bars + 42;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 43);
-  BwdPlan* plans = reinterpret_cast<BwdPlan*>(bars + 44);            // [kPlans]
-  static_assert(44 * 8 + kPlans * sizeof(BwdPlan) <= 3072, "tail of the shared memory");
+  BwdTile* descs = reinterpret_cast<BwdTile*>(bars + 44);            // [4], one per stage
+  BwdPlan* plans = reinterpret_cast<BwdPlan*>(descs + 4);            // [kPlans]
+  static_assert(44 * 8 + 4 * sizeof(BwdTile) + kPlans * sizeof(BwdPlan) <= 3072, "tail of the shared memory");
 
   const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
   if (tid == 0) {
     for (int s = 0; s < 4; ++s) {
-      mbar_init(&plan_full[s], 1); mbar_init(&plan_empty[s], 7 + Cfg::kCW);   // every warp but the loading one reads a plan
-      mbar_init(&q_full[s], 1); mbar_init(&st_full[s], 1); mbar_init(&q_empty[s], 1);
+      mbar_init(&plan_full[s], 1); mbar_init(&plan_empty[s], 7);   // the issuing and the result warps read a plan
+      mbar_init(&q_full[s], 1); mbar_init(&q_empty[s], 1);
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 2);                     // released by the S / dP and the dQ stream
@@ -327,7 +354,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
       mbar_init(&dq_full[s], 1); mbar_init(&dq_empty[s], 4);                   // four warps drain a tile
     }
     for (int s = 0; s < 3; ++s) {
-      mbar_init(&sdp_full[s], 1); mbar_init(&pds_full[s], 32 * Cfg::kCW / 2);
+      mbar_init(&sdp_full[s], 2); mbar_init(&pds_full[s], 32 * Cfg::kCW / 2);
       mbar_init(&buf_free[s], 2);                                // dV and dK of a half have read P^T, dS^T; the dQ stream has seen it
     }
     mbar_init(acc_full, 1); mbar_init(acc_empty, 4);
@@ -347,7 +374,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
   // operands the descriptors stay in uniform registers, which is what tcgen05.mma reads; issued from a divergent single-lane
   // region every instruction first has to move its operands there.
   auto wait_all = [&](uint64_t* bar, uint32_t parity, int code) -> bool {
-    return __all_sync(0xffffffffu, mbar_wait(bar, parity, p.status, code));
+    return __all_sync(0xffffffffu, mbar_wait_tight(bar, parity, p.status, code));
   };
   const uint32_t tbase_u = __shfl_sync(0xffffffffu, tbase, 0);
 
@@ -416,8 +443,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
         continue;
       }
       if (lane == 0) {
-        plan.n = n_act; plan.kt = kt; plan.bh = bh; plan.path = path; plan.flip = path == 0 ? 0xffffffffu : 0u;
-        plan.kpad[0] = kw.x; plan.kpad[1] = kw.y; plan.kpad[2] = kw.z; plan.kpad[3] = kw.w;
+        plan.n = n_act; plan.kt = kt; plan.bh = bh; plan.path = path;
       }
       __syncwarp();
       if (lane == 0) {
@@ -425,29 +451,34 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
         const CUtensorMap* mq = path == 0 ? &map_qs : &map_qc;
         const CUtensorMap* mk = path == 0 ? &map_ks : &map_kc;
         const CUtensorMap* mv = path == 0 ? &map_vs : &map_vc;
-        ok = mbar_wait(&k_empty[kr.pos], kr.phase ^ 1, p.status, 0x521);
+        ok = mbar_wait_tight(&k_empty[kr.pos], kr.phase ^ 1, p.status, 0x521);
         if (ok) {
           mbar_expect_tx(&k_full[kr.pos], Cfg::kTileBytes);
           tma_load_3d(sK + size_t(kr.pos) * Cfg::kTileBytes, mk, &k_full[kr.pos], 0, k0, bh);
-          ok = mbar_wait(&v_empty[vr.pos], vr.phase ^ 1, p.status, 0x523);
+          ok = mbar_wait_tight(&v_empty[vr.pos], vr.phase ^ 1, p.status, 0x523);
         }
         if (ok) {
           mbar_expect_tx(&v_full[vr.pos], Cfg::kTileBytes);
           tma_load_3d(sV + size_t(vr.pos) * Cfg::kTileBytes, mv, &v_full[vr.pos], 0, k0, bh);
         }
         for (int t = 0; t < n_act && ok; ++t) {
+          const bool mixed = (plan.tiles[t] & kMixed) != 0;
           const int i = plan.tiles[t] & (kMixed - 1);
-          ok = mbar_wait(&q_empty[lr.pos], lr.phase ^ 1, p.status, 0x525);
+          ok = mbar_wait_tight(&q_empty[lr.pos], lr.phase ^ 1, p.status, 0x525);
           if (!ok) break;
+          BwdTile& tile = descs[lr.pos];
+          tile.flags = mixed ? kTileMixed | kTileMasked : (kw.x | kw.y | kw.z | kw.w) != 0 ? kTileMasked : 0u;
+          tile.flip = path == 0 ? 0xffffffffu : 0u;
+          *reinterpret_cast<uint4*>(tile.kpad) = kw;
           unsigned char* dst = sQ + size_t(lr.pos) * 2 * Cfg::kTileBytes;
-          mbar_expect_tx(&q_full[lr.pos], 2 * Cfg::kTileBytes);
+          mbar_expect_tx(&q_full[lr.pos], 2 * Cfg::kTileBytes + Cfg::kStatBytes + (mixed ? Cfg::kMaskBytes : 0));
+          if (mixed) tma_load_3d(sMask + size_t(lr.pos) * Cfg::kMaskBytes, &map_bits, &q_full[lr.pos], 4 * i, k0, b);
           tma_load_3d(dst, mq, &q_full[lr.pos], 0, i * kBwdTile, bh);
           if (p.do_seq_first) tma_load_3d(dst + Cfg::kTileBytes, &map_do, &q_full[lr.pos], 0, bh, i * kBwdTile);
           else tma_load_3d(dst + Cfg::kTileBytes, &map_do, &q_full[lr.pos], 0, i * kBwdTile, bh);
           if (t == 0) griddep_wait();   // (returns at once from the second time on)
-          mbar_expect_tx(&st_full[lr.pos], Cfg::kStatBytes);
           bulk_load_1d(sStats + size_t(lr.pos) * Cfg::kStatBytes, p.stats + size_t(bh) * p.Tpad + size_t(i) * kBwdTile, Cfg::kStatBytes,
-                       &st_full[lr.pos]);
+                       &q_full[lr.pos]);
           lr.advance();
         }
       }
@@ -459,6 +490,10 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
     if (ok && lane == 0) {   // (the slot it waited for last)
       plans[pr.pos].n = 0;
       mbar_arrive(&plan_full[pr.pos]);
+      if (mbar_wait_tight(&q_empty[lr.pos], lr.phase ^ 1, p.status, 0x526)) {   // the stream of tiles ends with one more descriptor
+        descs[lr.pos].flags = kTileEnd;
+        mbar_arrive(&q_full[lr.pos]);
+      }
     }
     if (lane == 0) leave_tile_counter(p.sched, int(gridDim.x));
     griddep_wait();
@@ -484,7 +519,15 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
       ok = wait_all(&plan_full[pr.pos], pr.phase, 0x501);
       if (!ok) break;
       const int n = __shfl_sync(0xffffffffu, plans[pr.pos].n, 0);
-      if (n == 0) break;
+      if (n == 0) {   // hand the last descriptor to both sets of compute warps
+        ok = wait_all(&q_full[qr.pos], qr.phase, 0x506);
+        for (int u = 0; u < 2 && ok; ++u) {
+          ok = wait_all(&buf_free[ib.pos], ib.phase ^ 1, 0x507);
+          if (ok && leader) { mbar_arrive(&sdp_full[ib.pos]); mbar_arrive(&sdp_full[ib.pos]); }
+          ib.advance();
+        }
+        break;
+      }
       ok = wait_all(&k_full[kr.pos], kr.phase, 0x502);
       const uint32_t k_lo = k_lo0 + kr.pos * kTileU, v_lo = v_lo0 + vr.pos * kTileU;
       for (int u = 0; u < 2 * n && ok; ++u) {
@@ -507,6 +550,9 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
 #pragma unroll
           for (int k = 0; k < D / 16; ++k) umma_ss(col + 64, make_desc(kHi, v_lo + 2 * k), make_desc(kHi, dos + 2 * k), idesc_s, k > 0);
           umma_commit(&sdp_full[ib.pos]);
+          // The compute warps wait on sdp_full alone: its second arrival passes on that the tile's statistics, mask words and
+          // descriptor are there (a wait costs a warp some 150 cycles even when it has nothing to wait for).
+          mbar_arrive(&sdp_full[ib.pos]);
         }
         __syncwarp();
         ib.advance();
@@ -645,7 +691,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
         if (Cfg::kDqStages == 2) bulk_wait_read_but_one(); else bulk_wait_read_all();
       }
       __syncwarp();
-#pragma unroll
+#pragma unroll 1
       for (int c = 0; c < D; c += kC) {
         uint32_t v[kC];
         tmem_ld_n<kC>(tq + kColDQ + xb * kAcc + c, v);
@@ -702,7 +748,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
       __nv_bfloat16* dv = p.dv[path] + row_off;
       if (!wait_all(acc_full, m & 1u, 0x603)) return false;
       tc_fence_after();
-#pragma unroll
+#pragma unroll 1
       for (int d0 = 0; d0 < hD; d0 += kCh) {   // a range of columns and the one that the rotation pairs it with
         uint32_t t0[kCh], t1[kCh];
         float o0[kCh], o1[kCh];
@@ -778,33 +824,22 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
     const uint32_t tBuf = tbase + (uint32_t(quarter * 32) << 16) + kColBuf + 32 * c32;   // + 128 * buffer: S^T columns of this thread; dP^T 64 further
     const uint32_t ds_addr = smem_u32(sDS) + uint32_t(sub) * Cfg::kDsBlock + swizzled_offset(r, 4 * c32, 128);
     const uint64_t c22 = pack2(p.scale_log2, p.scale_log2);
-    bool ok = true;
     Ring<kNBuf> br;        // buffer of this warp's half: every other one
     if (sub == 1) br.advance();
-    uint32_t g = 0, m = 0;                        // query tiles and key tiles so far
-    for (;; ++m) {
-      ok = wait_all(&plan_full[m % kPlans], (m / kPlans) & 1u, 0x600);
-      if (!ok) break;
-      const BwdPlan& plan = plans[m % kPlans];
-      const int n = plan.n;
-      if (n == 0) break;
-      const int kj = plan.kt * kBwdTile + r;
-      const uint32_t key_valid = kj < p.T && !((plan.kpad[quarter] >> lane) & 1u) ? 0xffffffffu : 0u;
-      // Mask word of the thread's 32 queries of tile `it`; asked for one tile ahead and not touched before it is needed, so that a
-      // mixed tile does not wait for it.
-      auto tile_bits = [&](int it) -> uint32_t {
-        const uint32_t e = plan.tiles[it];
-        return e & kMixed ? __ldg(p.bitsT + (size_t(plan.bh / p.H) * p.T + (kj < p.T ? kj : p.T - 1)) * p.TW + 4 * (e & (kMixed - 1)) + grp) : ~plan.flip;
-      };
-      uint32_t bits = tile_bits(0);
-      for (int it = 0; it < n && ok; ++it) {
-        const uint32_t bits_next = it + 1 < n ? tile_bits(it + 1) : 0u;
-        ok = mbar_wait(&st_full[g % kQStages], (g / kQStages) & 1u, p.status, 0x604) &
-             mbar_wait(&dq_full[g % kNDq], ((g / kNDq) & 1u) ^ 1u, p.status, 0x606) &   // the dS tile has been read (by the product of two tiles ago)
-             mbar_wait(&sdp_full[br.pos], br.phase, p.status, 0x602);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
-        const uint32_t mask = (bits ^ plan.flip) & key_valid;
+    bool ok = true;
+    bool seen = false;     // the wait for the next half has been over before it began
+    for (uint32_t g = 0;; ++g) {   // query tiles
+        if (!__all_sync(0xffffffffu, seen) && !wait_all(&sdp_full[br.pos], br.phase, 0x602)) break;
+        // the dS tile has been read (by the product of two tiles ago): looked at now, needed behind the first exponentials
+        const bool ds_free = mbar_test_wait(&dq_full[g % kNDq], ((g / kNDq) & 1u) ^ 1u);
+        const BwdTile& tile = descs[g % kQStages];
+        const uint32_t flags = tile.flags;
+        if (flags & kTileEnd) break;
+        uint32_t mask = 0xffffffffu;
+        if (flags & kTileMasked) {
+          const uint32_t bits = flags & kTileMixed ? reinterpret_cast<const uint32_t*>(sMask + (g % kQStages) * Cfg::kMaskBytes)[4 * r + grp] : ~tile.flip;
+          mask = (bits ^ tile.flip) & ((tile.kpad[quarter] >> lane) & 1u ? 0u : 0xffffffffu);
+        }
         tc_fence_after();
         const uint32_t ds_row = ds_addr + (g % kNDq) * Cfg::kDsBytes;
 #pragma unroll
@@ -842,13 +877,17 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
               dd[j / 2] = bwd_pack(d0, d1);
             }
           };
-          if (__all_sync(0xffffffffu, keep == 0xffffu)) {
+          if (!(flags & kTileMasked) || __all_sync(0xffffffffu, keep == 0xffffu)) {
             elements(std::false_type{});
           } else if (__all_sync(0xffffffffu, keep == 0u)) {   // the other side of a chain boundary, or padding
 #pragma unroll
             for (int j = 0; j < 8; ++j) pp[j] = dd[j] = 0u;
           } else {
             elements(std::true_type{});
+          }
+          if (v == 0 && !__all_sync(0xffffffffu, ds_free)) {
+            ok = wait_all(&dq_full[g % kNDq], ((g / kNDq) & 1u) ^ 1u, 0x606);
+            if (!ok) break;
           }
           tmem_st8(tS, pp);         // P^T over the S^T columns this thread has read
           tmem_st8(tS + 64, dd);    // dS^T likewise
@@ -857,18 +896,14 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
           smem_store16(ds_at, dd[0], dd[1], dd[2], dd[3]);
           smem_store16(ds_at ^ 16u, dd[4], dd[5], dd[6], dd[7]);
         }
+        if (!ok) break;
         tmem_st_wait();
         fence_proxy_async_smem();
         tc_fence_before();
         mbar_arrive(&pds_full[br.pos]);
         br.advance();
         br.advance();
-        bits = bits_next;
-        ++g;
-      }
-      if (!ok) break;
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&plan_empty[m % kPlans]);
+        seen = mbar_test_wait(&sdp_full[br.pos], br.phase);
     }
   }
   tc_fence_before();
@@ -904,7 +939,11 @@ static int bwd_tc_t(const AttnArgs& a, const void* q_s, const void* k_s, const f
     set_error("mintb_attn_bwd: cuTensorMapEncodeTiled failed");
     return MINTB_ECUDA;
   }
-  CUtensorMap mdq_s, mdq_c;
+  CUtensorMap mdq_s, mdq_c, mbits;
+  if (!bwd_make_bits_map(&mbits, a.meta.bitsT, a.meta.TW, a.T, a.B)) {
+    set_error("mintb_attn_bwd: cuTensorMapEncodeTiled failed for the mask words");
+    return MINTB_ECUDA;
+  }
   if (!bwd_make_dq_map(&mdq_s, acc_s, D, a.T, BH) || !bwd_make_dq_map(&mdq_c, acc_c, D, a.T, BH)) {
     set_error("mintb_attn_bwd: cuTensorMapEncodeTiled failed for the dQ accumulators");
     return MINTB_ECUDA;
@@ -912,7 +951,7 @@ static int bwd_tc_t(const AttnArgs& a, const void* q_s, const void* k_s, const f
   cudaError_t e = opt_in_smem<attn_bwd_tc_kernel<D, SQ>>(int(Cfg::kSmemBytes));
   if (e != cudaSuccess) { set_error("cudaFuncSetAttribute: %s", cudaGetErrorString(e)); return MINTB_ECUDA; }
   BwdParams p{};
-  p.bitsT = a.meta.bitsT; p.kpad = a.meta.kpad; p.cls = a.meta.cls;
+  p.kpad = a.meta.kpad; p.cls = a.meta.cls;
   p.stats = stats;
   p.cos_tab = a.rope ? a.rope_cos : nullptr;
   p.sin_tab = a.rope ? a.rope_sin : nullptr;
@@ -930,7 +969,7 @@ static int bwd_tc_t(const AttnArgs& a, const void* q_s, const void* k_s, const f
   p.n_items = (a.T + kBwdTile - 1) / kBwdTile * BH * 2;
   if (int rc = next_tile_counter(&p.sched); rc != MINTB_OK) return rc;
   const dim3 grid(unsigned(p.n_items < sm_count() ? p.n_items : sm_count()));
-  e = launch_dependent(attn_bwd_tc_kernel<D, SQ>, grid, dim3(Cfg::kThreads), Cfg::kSmemBytes, a.stream, mqs, mks, mvs, mqc, mkc, mvc, mdo, mdq_s, mdq_c, p);
+  e = launch_dependent(attn_bwd_tc_kernel<D, SQ>, grid, dim3(Cfg::kThreads), Cfg::kSmemBytes, a.stream, mqs, mks, mvs, mqc, mkc, mvc, mdo, mdq_s, mdq_c, mbits, p);
   count_launches(1);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) { set_error("attention backward launch: %s", cudaGetErrorString(e)); return MINTB_ECUDA; }
