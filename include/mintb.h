@@ -213,6 +213,14 @@ MINTB_API int mintb_quantize_e4m3(const void* x, void* out, size_t n, float inv_
  * four, every pointer 16-byte aligned. */
 MINTB_API int mintb_linear_f32(const float* x, const float* const* w, const float* const* bias, float* const* out, const float* resid,
                                int groups, int M, int N, int K, int gelu, int B, int T, int H, int D, void* stream);
+/* mintb_linear_f32_tc: the same on the tensor cores, each fp32 number as three bf16 pieces, in the same precision.  `workspace` holds
+ * the pieces of x and the weights (mintb_linear_f32_tc_workspace_bytes, 256-byte aligned); without one the product is formed on the
+ * CUDA cores.  mintb_linear_f32_needed_bytes: the workspace where the tensor cores are faster, 0 where they are not. */
+MINTB_API size_t mintb_linear_f32_tc_workspace_bytes(int groups, int M, int N, int K);
+MINTB_API size_t mintb_linear_f32_needed_bytes(int groups, int M, int N, int K);
+MINTB_API int mintb_linear_f32_tc(const float* x, const float* const* w, const float* const* bias, float* const* out, const float* resid,
+                                  int groups, int M, int N, int K, int gelu, int B, int T, int H, int D, void* workspace,
+                                  size_t workspace_bytes, void* stream, int* dev_status);
 /* mintb_linear_res_fwd: mintb_linear_fwd without activation and with the layer's residual sum formed in the epilogue:
  * out[M][N] = res_a * resid[M][N] + res_b * (alpha * x w^T + bias) - x + out_proj(attention) of the Pre-LN layer
  * (modules.py:183-186: res_a = res_b = 1) and sqrt(1 - tau) x + sqrt(tau) out_proj(attention) of the muS layer

@@ -41,6 +41,9 @@ PROTOTYPES = {
     "mintb_attn_bwd_rows": (c_int, [_P] * 6 + [_P, _P, _P, _P, _P, _P] + [_P] * 6 + [_P, c_size_t, c_int, c_int, c_int, c_int,
                                     c_int, c_uint, c_float, _P, _P, _P]),
     "mintb_linear_f32": (c_int, [_P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _P]),
+    "mintb_linear_f32_tc_workspace_bytes": (c_size_t, [c_int, c_int, c_int, c_int]),
+    "mintb_linear_f32_needed_bytes": (c_size_t, [c_int, c_int, c_int, c_int]),
+    "mintb_linear_f32_tc": (c_int, [_P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _P, c_size_t, _P, _P]),
     "mintb_linear_fwd": (c_int, [_P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float, _P, _P]),
     "mintb_qkv_fwd": (c_int, [_P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float, _P, _P, _P, c_int,
                               _P, _P]),

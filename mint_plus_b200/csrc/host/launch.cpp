@@ -71,6 +71,14 @@ std::pair<Tensor, Tensor> linear_res_fwd(const Product& p, const Tensor& resid, 
   return {out, q8};
 }
 
+// fp32 products, on the tensor cores where they are faster
+static void product_f32(const Env& e, const float* x, const float* const* w, const float* const* bias, float* const* out, const float* resid, int groups, int64_t M,
+                        int64_t N, int64_t K, bool gelu, int64_t B, int64_t T, int64_t H, int64_t D) {
+  const size_t n = M > INT32_MAX ? 0 : mintb_linear_f32_needed_bytes(groups, int(M), int(N), int(K));
+  const Tensor ws = e.bytes(n);
+  check(mintb_linear_f32_tc(x, w, bias, out, resid, groups, M, N, K, gelu, B, T, H, D, n ? ws.data_ptr() : nullptr, n, e.stream, e.status), "mintb_linear_f32");
+}
+
 Tensor linear_f32(const Tensor& x, const Tensor& w, const OptTensor& bias, bool gelu, const OptTensor& resid) {
   for (const Tensor& t : {x, w, opt(bias), opt(resid)}) no_tangent(t);
   Env e(x);
@@ -83,7 +91,7 @@ Tensor linear_f32(const Tensor& x, const Tensor& w, const OptTensor& bias, bool 
   TORCH_CHECK(!r.defined() || (r.is_contiguous() && r.numel() == M * N), "linear_f32: the residual has the result's shape");
   const float *wp = fptr(w), *bp = fptr(b);
   float* op = fptr(out);
-  check(mintb_linear_f32(fptr(x), &wp, &bp, &op, fptr(r), 1, M, N, K, gelu, 1, 1, 1, 0, e.stream), "mintb_linear_f32");
+  product_f32(e, fptr(x), &wp, &bp, &op, fptr(r), 1, M, N, K, gelu, 1, 1, 1, 0);
   return out;
 }
 
@@ -105,7 +113,7 @@ std::vector<Tensor> heads_f32(const Tensor& x, const std::vector<Tensor>& w, con
       op.push_back(fptr(out.back()));
     }
   }
-  check(mintb_linear_f32(fptr(x), wp.data(), bp.data(), op.data(), nullptr, int(wp.size()), T * B, E, E, 0, B, T, H, D, e.stream), "mintb_linear_f32");
+  product_f32(e, fptr(x), wp.data(), bp.data(), op.data(), nullptr, int(wp.size()), T * B, E, E, false, B, T, H, D);
   return out;
 }
 

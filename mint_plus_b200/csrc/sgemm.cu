@@ -5,8 +5,8 @@
 // TM x TN block of results in registers, pairs of rows in one 64-bit register, and reads TM + TN operands per k from shared memory.
 // Slabs of BK columns are turned on the way into shared memory ([k][row], rows XOR-ed by their k so that neither the stores nor the
 // reads collide) and double buffered; the next slab's global loads are in flight while one is multiplied.
-#include "common.cuh"
 #include "ptx.cuh"
+#include "sgemm.cuh"
 
 namespace mintb {
 namespace {
@@ -22,15 +22,6 @@ __device__ __forceinline__ uint64_t ffma2(uint64_t a, uint64_t b, uint64_t c) {
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
   return r;
 }
-
-struct SgemmParams {
-  const float* x;
-  const float *w[6], *bias[6];
-  float* out[6];
-  const float* resid;      // row-major [M][N] or null
-  int M, N, K, gelu;
-  int B, T, H, D;          // D > 0: head-major outputs, row m = t * B + b, column n = h * D + d
-};
 
 template <int BM, int BN, int TM, int TN, int BK, int KS>
 __global__ void __launch_bounds__(KS * (BM / TM) * (BN / TN)) sgemm_kernel(const SgemmParams p) {
@@ -196,21 +187,24 @@ int launch_t(const SgemmParams& p, int groups, cudaStream_t s) {
 
 using namespace mintb;
 
-extern "C" int mintb_linear_f32(const float* x, const float* const* w, const float* const* bias, float* const* out, const float* resid, int groups, int M,
-                                int N, int K, int gelu, int B, int T, int H, int D, void* stream) {
+static int sgemm_args(SgemmParams& p, const char* who, const float* x, const float* const* w, const float* const* bias, float* const* out, const float* resid, int groups,
+                      int M, int N, int K, int gelu, int B, int T, int H, int D) {
   bool ok = x != nullptr && w != nullptr && bias != nullptr && out != nullptr && groups >= 1 && groups <= 6 && M > 0 && N > 0 && K > 0 && N % 4 == 0 && K % 4 == 0 &&
             (D == 0 || (D % 4 == 0 && N == H * D && M == T * B && resid == nullptr)) && M <= 65535 * 32;
   auto aligned = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
   ok = ok && aligned(x) && aligned(resid);
   for (int i = 0; ok && i < groups; ++i) ok = w[i] != nullptr && out[i] != nullptr && aligned(w[i]) && aligned(bias[i]) && aligned(out[i]);
   if (!ok) {
-    set_error("mintb_linear_f32: one to six 16-byte aligned weights, N and K multiples of four, and matching head-major sizes are required");
+    set_error("%s: one to six 16-byte aligned weights, N and K multiples of four, and matching head-major sizes are required", who);
     return MINTB_EINVAL;
   }
-  SgemmParams p{};
   p.x = x; p.resid = resid; p.M = M; p.N = N; p.K = K; p.gelu = gelu; p.B = B; p.T = T; p.H = H; p.D = D;
   for (int i = 0; i < groups; ++i) { p.w[i] = w[i]; p.bias[i] = bias[i]; p.out[i] = out[i]; }
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  return MINTB_OK;
+}
+
+static int launch_sgemm_simt(const SgemmParams& p, int groups, cudaStream_t s) {
+  const int M = p.M, N = p.N;
   // The largest tile that leaves every SM several: with fewer than about one 64 x 32 tile per SM, smaller ones whose K four parts of the
   // CTA share (M100 N320 K1280: 29 -> 16 us); with rounds of tiles to spare, 64 x 64 (M5120 N1280 K320: 106 -> 97 us).  Against the
   // library's products: M2048 N320 K320 26.6 -> 17.5 us, six of them 157 -> 64 us in one launch, M2048 N320 K1280 65 -> 59 us, M5120
@@ -219,4 +213,31 @@ extern "C" int mintb_linear_f32(const float* x, const float* const* w, const flo
   if (4 * tiles < 5 * sms) return launch_t<32, 32, 4, 4, 32, 4>(p, groups, s);
   if (tiles < 14 * sms) return launch_t<64, 32, 8, 4, 32, 2>(p, groups, s);
   return launch_t<64, 64, 8, 4, 16, 1>(p, groups, s);
+}
+
+extern "C" int mintb_linear_f32(const float* x, const float* const* w, const float* const* bias, float* const* out, const float* resid, int groups, int M,
+                                int N, int K, int gelu, int B, int T, int H, int D, void* stream) {
+  SgemmParams p{};
+  if (int rc = sgemm_args(p, "mintb_linear_f32", x, w, bias, out, resid, groups, M, N, K, gelu, B, T, H, D); rc != MINTB_OK) return rc;
+  return launch_sgemm_simt(p, groups, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" size_t mintb_linear_f32_tc_workspace_bytes(int groups, int M, int N, int K) {
+  return groups > 0 && M > 0 && N > 0 && K > 0 ? sgemm_tc_workspace_bytes(groups, M, N, K) : 0;
+}
+
+extern "C" size_t mintb_linear_f32_needed_bytes(int groups, int M, int N, int K) {
+  return groups > 0 && M > 0 && N > 0 && K > 0 && sgemm_tc_wins(groups, M, N, K) ? sgemm_tc_workspace_bytes(groups, M, N, K) : 0;
+}
+
+extern "C" int mintb_linear_f32_tc(const float* x, const float* const* w, const float* const* bias, float* const* out, const float* resid, int groups, int M,
+                                   int N, int K, int gelu, int B, int T, int H, int D, void* workspace, size_t workspace_bytes, void* stream, int* dev_status) {
+  SgemmParams p{};
+  if (int rc = sgemm_args(p, "mintb_linear_f32_tc", x, w, bias, out, resid, groups, M, N, K, gelu, B, T, H, D); rc != MINTB_OK) return rc;
+  if (workspace == nullptr) return launch_sgemm_simt(p, groups, static_cast<cudaStream_t>(stream));
+  if ((reinterpret_cast<uintptr_t>(workspace) & 255) != 0 || workspace_bytes < sgemm_tc_workspace_bytes(groups, M, N, K)) {
+    set_error("mintb_linear_f32_tc: %zu bytes of workspace on a 256-byte boundary are required", sgemm_tc_workspace_bytes(groups, M, N, K));
+    return MINTB_EWORKSPACE;
+  }
+  return launch_sgemm_tc(p, groups, workspace, static_cast<cudaStream_t>(stream), dev_status);
 }

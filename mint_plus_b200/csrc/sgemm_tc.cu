@@ -1,0 +1,346 @@
+// fp32 projections on the tensor cores: out = act(x w^T + bias) [+ resid] for up to six weights of one shape, in fp32 precision.
+//
+// Every fp32 operand is the sum of three bf16 numbers (8 bits of the mantissa each), and six of the nine products of the pieces make up
+// the fp32 product to 2^-25: 128 x 128 results of 32 columns are twelve tcgen05.mma of 64 cycles, where the CUDA cores need 4096 cycles.
+// A first pass writes the pieces of x and of the weights (6 bytes a number, read back from L2): split by the warps of the product kernel
+// instead, each tile of x once per tile of columns, 32 columns took 2000 cycles (M2048 N320 K320, six weights: 30.5 us; the CUDA cores
+// 63, this 26.4).  With one tile a CTA it is the products that bound it (980 cycles per 32 columns), with many the pieces' way from L2.
+// The accumulation inside tcgen05.mma truncates: measured against fp64 on 512 x 512 results of N(0, 1) operands, the error relative to
+// the result is 2.4e-8 after one product of 16 columns (fp32 fma chain: 2.2e-8), 3.9e-8 after two (3.5e-8), but 2.9e-7 after 20
+// (7.2e-8), nearly all of it towards zero.  So an accumulator in TMEM holds one slab of 32 columns, the small products first, and the
+// slabs are summed in registers, rounding to nearest.  Error of whole projections against fp64: 6.6e-8 at K = 320 and 9.6e-8 at 1280,
+// with the fma chains of sgemm.cu 1.2e-7 to 2.3e-7 and 2.3e-7 to 3.2e-7.
+//
+// Persistent CTAs, one per SM: warps 0-7 sum the slabs and finish the tile (two per TMEM lane quarter, half of the columns each), warp 8
+// issues the products, warp 9 the TMA loads; four accumulators let the products run on while a tile is finished.
+// A result that is not finite is formed again as a plain fp32 dot product: an infinite operand, or one that rounds to infinity as bf16,
+// has no pieces.
+#include "ptx.cuh"
+#include "sgemm.cuh"
+
+namespace mintb {
+namespace {
+
+using namespace ptx;
+
+constexpr int kBM = 128, kBK = 64, kSum = 32;   // rows; columns of a stage; columns of an accumulator
+constexpr int kSumWarps = 8;
+constexpr int kThreads = 32 * (kSumWarps + 2);
+constexpr int kAccs = 4;
+
+template <int BN>
+struct TcCfg {
+  static constexpr int kStages = 2;
+  static constexpr int kPieceA = kBM * 128, kPieceB = BN * 128;           // one piece of a slab: rows of 64 bf16
+  static constexpr int kStageBytes = 3 * (kPieceA + kPieceB);              // [A hi | A mid | A lo | B hi | B mid | B lo]
+  static constexpr int kCols = BN / 2;                                     // columns of a tile per summing thread
+  static constexpr size_t kSmemBytes = 1024 + size_t(kStages) * kStageBytes + kSumWarps * 4096 + 256;
+};
+
+__device__ __forceinline__ uint32_t cvt2(float lo, float hi) {
+  uint32_t r;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+  return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t pair(uint32_t lo, uint32_t hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));
+  return r;
+}
+// the bf16 pair nearest to (a, b), which keeps what is left over
+__device__ __forceinline__ uint32_t take_piece(float& a, float& b) {
+  const uint32_t h = cvt2(a, b);
+  a -= __uint_as_float(h << 16);
+  b -= __uint_as_float(h & 0xffff0000u);
+  return h;
+}
+
+struct SplitParams {
+  const float *x, *w[6];
+  __nv_bfloat16 *px, *pw;   // pieces [3][M][Kp] and [3][groups N][Kp]
+  int M, N, groups, K, Kp;
+};
+
+// Eight numbers a thread: 32 bytes in, 16 bytes to each of the three pieces.  Bound by the launch and the L2 (M2048 K320 with six weights
+// of N320: 5.2 MB in, 7.8 MB out).
+__global__ void __launch_bounds__(256) sgemm_split_kernel(const SplitParams p) {
+  griddep_wait();
+  griddep_launch();
+  const int chunks = p.Kp / 8;
+  const size_t idx = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  size_t row = idx / chunks;
+  const int k = int(idx % chunks) * 8;
+  const size_t rows_w = size_t(p.groups) * p.N;
+  if (row >= p.M + rows_w) return;
+  const bool is_w = row >= size_t(p.M);
+  const float* src = p.x + row * p.K;
+  if (is_w) {
+    row -= p.M;
+    src = p.w[row / p.N] + (row % p.N) * p.K;
+  }
+  const size_t piece = (is_w ? rows_w : size_t(p.M)) * p.Kp;
+  __nv_bfloat16* dst = (is_w ? p.pw : p.px) + row * p.Kp + k;
+  float4 a = __ldg(reinterpret_cast<const float4*>(src + k));   // (K is a multiple of four)
+  float4 b = k + 4 < p.K ? __ldg(reinterpret_cast<const float4*>(src + k + 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+  for (int q = 0; q < 3; ++q)
+    *reinterpret_cast<uint4*>(dst + q * piece) = make_uint4(take_piece(a.x, a.y), take_piece(a.z, a.w), take_piece(b.x, b.y), take_piece(b.z, b.w));
+}
+
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                                  const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+// pieces [3][rows][Kp] as (K, rows, 3), box of 64 columns and `box_rows` rows; columns past K and rows past the end read as zero
+bool piece_map(CUtensorMap* m, const void* ptr, int K, int Kp, size_t rows, int box_rows) {
+  static const EncodeTiledFn fn = [] {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess) p = nullptr;
+    return reinterpret_cast<EncodeTiledFn>(p);
+  }();
+  if (fn == nullptr) return false;
+  cuuint64_t dims[3] = {cuuint64_t(K), cuuint64_t(rows), 3}, strides[2] = {cuuint64_t(Kp) * 2, cuuint64_t(rows) * Kp * 2};
+  cuuint32_t box[3] = {kBK, cuuint32_t(box_rows), 1}, es[3] = {1, 1, 1};
+  return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <int BN>
+__global__ void __launch_bounds__(kThreads, 1)
+sgemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
+                                                               const __grid_constant__ SgemmParams p, int n_total, int m_tiles, int n_tiles_all, int* status) {
+  using Cfg = TcCfg<BN>;
+  constexpr int kStages = Cfg::kStages, kCols = Cfg::kCols;
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* smem = align_smem_1024(smem_raw);
+  unsigned char* staging = smem + kStages * Cfg::kStageBytes;             // [summing warp][32 rows][128 B]
+  uint64_t* full = reinterpret_cast<uint64_t*>(staging + kSumWarps * 4096);   // [kStages] loads -> products
+  uint64_t* empty = full + kStages;                                        // [kStages] products -> loads
+  uint64_t* acc_full = empty + kStages;                                    // [kAccs] products -> summing warps
+  uint64_t* acc_free = acc_full + kAccs;                                   // [kAccs] summing warps -> products
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_free + kAccs);
+  const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+  if (tid == 0) {
+    for (int s = 0; s < kStages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+    for (int s = 0; s < kAccs; ++s) { mbar_init(&acc_full[s], 1); mbar_init(&acc_free[s], kSumWarps); }
+    fence_mbar_init();
+  }
+  if (warp == kSumWarps) { tmem_alloc(tmem_slot, kAccs * BN); tmem_relinquish(); }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  griddep_wait();
+  const uint32_t tbase = *tmem_slot;
+  const int slabs = (p.K + kBK - 1) / kBK, sums = (p.K + kSum - 1) / kSum;
+
+  const int n_tiles = int(blockIdx.x) < n_tiles_all ? (n_tiles_all - 1 - int(blockIdx.x)) / int(gridDim.x) + 1 : 0;
+  const uint32_t total = uint32_t(n_tiles) * slabs;
+
+  if (warp > kSumWarps) {
+    // ---------------------------------------------------------------- loads
+    if (lane == 0) {
+      int tile = blockIdx.x, k = 0;
+      for (uint32_t it = 0; it < total; ++it) {
+        const uint32_t stage = it % kStages;
+        if (!mbar_wait(&empty[stage], ((it / kStages) & 1) ^ 1, status, 0x701)) break;
+        const int m0 = tile % m_tiles * kBM, n0 = tile / m_tiles * BN;
+        unsigned char* dst = smem + stage * Cfg::kStageBytes;
+        mbar_expect_tx(&full[stage], Cfg::kStageBytes);
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+          tma_load_3d(dst + q * Cfg::kPieceA, &map_x, &full[stage], k, m0, q);
+          tma_load_3d(dst + 3 * Cfg::kPieceA + q * Cfg::kPieceB, &map_w, &full[stage], k, n0, q);
+        }
+        k += kBK;
+        if (k >= p.K) {
+          k = 0;
+          tile += gridDim.x;
+        }
+      }
+      griddep_launch();
+    }
+  } else if (warp == kSumWarps) {
+    // ---------------------------------------------------------------- products
+    const bool leader = elect_one();
+    constexpr uint32_t idesc = idesc_bf16(kBM, BN, false, false);
+    constexpr uint32_t kHi = desc_hi32(8 * 128, kSw128);
+    const uint32_t lo0 = desc_addr32(__shfl_sync(0xffffffffu, smem_u32(smem), 0)) + desc_lbo32(16);
+    const uint32_t tb = __shfl_sync(0xffffffffu, tbase, 0);
+    constexpr uint32_t kA = Cfg::kPieceA >> 4, kB = Cfg::kPieceB >> 4;
+    uint32_t n_acc = 0;
+    int s = 0;                                // slab of the tile
+    bool ok = true;
+    for (uint32_t it = 0; it < total && ok; ++it) {
+      const uint32_t stage = it % kStages;
+      ok = __all_sync(0xffffffffu, mbar_wait(&full[stage], (it / kStages) & 1, status, 0x703));
+      const uint32_t a0 = lo0 + stage * (Cfg::kStageBytes >> 4), b0 = a0 + 3 * kA;
+      const int parts = sums - 2 * s < 2 ? 1 : 2;
+      for (int h = 0; h < parts && ok; ++h, ++n_acc) {
+        const uint32_t acc = n_acc % kAccs;
+        ok = __all_sync(0xffffffffu, mbar_wait(&acc_free[acc], ((n_acc / kAccs) & 1) ^ 1, status, 0x702));
+        if (!ok) break;
+        tc_fence_after();
+        if (leader) {
+          // pieces 0 (high) to 2 (low), the smallest products first
+          constexpr int kPa[6] = {0, 2, 1, 0, 1, 0}, kPb[6] = {2, 0, 1, 1, 0, 0};
+#pragma unroll
+          for (int q = 0; q < 6; ++q)
+#pragma unroll
+            for (int k = 0; k < kSum / 16; ++k)
+              umma_ss(tb + acc * BN, make_desc(kHi, a0 + kPa[q] * kA + 4 * h + 2 * k), make_desc(kHi, b0 + kPb[q] * kB + 4 * h + 2 * k), idesc, q > 0 || k > 0);
+          if (h + 1 == parts) umma_commit(&empty[stage]);
+          umma_commit(&acc_full[acc]);
+        }
+        __syncwarp();
+      }
+      if (++s == slabs) s = 0;
+    }
+  } else {
+    // ---------------------------------------------------------------- sums of the slabs, results
+    const int quarter = warp % 4, half = warp / 4;
+    const uint32_t tq = tbase + (uint32_t(quarter * 32) << 16) + half * kCols;
+    unsigned char* stg = staging + warp * 4096;
+    uint32_t it = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < n_tiles_all && ok; tile += gridDim.x) {
+      uint64_t sum[kCols / 2];
+#pragma unroll
+      for (int j = 0; j < kCols / 2; ++j) sum[j] = 0ull;
+      for (int s = 0; s < sums; ++s, ++it) {
+        const uint32_t acc = it % kAccs;
+        ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[acc], (it / kAccs) & 1, status, 0x704));
+        if (!ok) break;
+        tc_fence_after();
+        uint32_t r[kCols / 32][32];
+#pragma unroll
+        for (int c = 0; c < kCols / 32; ++c) tmem_ld32(tq + acc * BN + 32 * c, r[c]);
+        tmem_ld_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&acc_free[acc]);
+#pragma unroll
+        for (int c = 0; c < kCols / 32; ++c)
+#pragma unroll
+          for (int j = 0; j < 16; ++j) sum[16 * c + j] = add2(sum[16 * c + j], pair(r[c][2 * j], r[c][2 * j + 1]));
+      }
+      if (!ok) break;
+      // 32 columns at a time through shared memory, so that eight lanes write 128 bytes of a row
+      const int m0 = tile % m_tiles * kBM + quarter * 32, n0 = tile / m_tiles * BN + half * kCols;
+#pragma unroll
+      for (int c = 0; c < kCols; c += 32) {
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const ulonglong2 two = make_ulonglong2(sum[c / 2 + 2 * j], sum[c / 2 + 2 * j + 1]);
+          *reinterpret_cast<ulonglong2*>(stg + swizzled_offset(lane, j, 128)) = two;
+        }
+        __syncwarp();
+        const int ng = n0 + c + 4 * (lane % 8);
+        if (ng >= n_total) continue;
+        const int g = ng / p.N, n = ng % p.N;
+        const float4 bias = p.bias[g] != nullptr ? __ldg(reinterpret_cast<const float4*>(p.bias[g] + n)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float* wrow = p.w[g] + size_t(n) * p.K;
+        float* out = p.out[g];
+        size_t col = n;
+        if (p.D > 0) col = size_t(n / p.D) * p.T * p.D + n % p.D;
+#pragma unroll 1
+        for (int r0 = 0; r0 < 32; r0 += 4) {
+          const int row = r0 + lane / 8, m = m0 + row;
+          if (m >= p.M) break;
+          const float4 q = *reinterpret_cast<const float4*>(stg + swizzled_offset(row, lane % 8, 128));
+          float y[4] = {q.x, q.y, q.z, q.w};
+          const float b[4] = {bias.x, bias.y, bias.z, bias.w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            if (!(fabsf(y[e]) <= 3.402823466e38f)) {
+              float d = 0.f;
+#pragma unroll 1
+              for (int k = 0; k < p.K; ++k) d = fmaf(p.x[size_t(m) * p.K + k], wrow[size_t(e) * p.K + k], d);
+              y[e] = d;
+            }
+            y[e] += b[e];
+            if (p.gelu) y[e] = 0.5f * y[e] * (1.f + erff(y[e] * 0.70710678118654752f));
+          }
+          size_t o = size_t(m) * p.N + col;
+          if (p.D > 0) {
+            const int t = m / p.B, bb = m % p.B;
+            o = (size_t(bb) * p.H * p.T + t) * p.D + col;
+          }
+          if (p.resid != nullptr) {
+            const float4 r = __ldg(reinterpret_cast<const float4*>(p.resid + o));
+            y[0] += r.x; y[1] += r.y; y[2] += r.z; y[3] += r.w;
+          }
+          *reinterpret_cast<float4*>(out + o) = make_float4(y[0], y[1], y[2], y[3]);
+        }
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == kSumWarps) {
+    __syncwarp();
+    tmem_dealloc(tbase, kAccs * BN);
+  }
+}
+
+int padded_k(int K) { return (K + 7) & ~7; }   // rows of the pieces start on 16 bytes
+
+template <int BN>
+int launch_tc_t(const SgemmParams& p, int groups, void* workspace, cudaStream_t s, int* status) {
+  constexpr auto kern = sgemm_tc_kernel<BN>;
+  const int n_total = groups * p.N, m_tiles = (p.M + kBM - 1) / kBM, tiles = m_tiles * ((n_total + BN - 1) / BN), Kp = padded_k(p.K);
+  SplitParams sp{};
+  sp.x = p.x; sp.M = p.M; sp.N = p.N; sp.groups = groups; sp.K = p.K; sp.Kp = Kp;
+  for (int i = 0; i < groups; ++i) sp.w[i] = p.w[i];
+  sp.px = static_cast<__nv_bfloat16*>(workspace);
+  sp.pw = sp.px + align256(size_t(p.M) * Kp * 6) / 2;
+  CUtensorMap mx, mw;
+  if (!piece_map(&mx, sp.px, p.K, Kp, size_t(p.M), kBM) || !piece_map(&mw, sp.pw, p.K, Kp, size_t(n_total), BN)) {
+    set_error("mintb_linear_f32_tc: cuTensorMapEncodeTiled failed");
+    return MINTB_ECUDA;
+  }
+  cudaError_t e = opt_in_smem<kern>(int(TcCfg<BN>::kSmemBytes));
+  const size_t units = (size_t(p.M) + n_total) * (Kp / 8);
+  if (e == cudaSuccess) e = launch_dependent(sgemm_split_kernel, dim3(unsigned((units + 255) / 256)), dim3(256), 0, s, sp);
+  if (e == cudaSuccess)
+    e = launch_dependent(kern, dim3(unsigned(tiles < sm_count() ? tiles : sm_count())), dim3(kThreads), TcCfg<BN>::kSmemBytes, s, mx, mw, p, n_total, m_tiles, tiles, status);
+  count_launches(2);
+  if (e != cudaSuccess) { set_error("sgemm launch: %s", cudaGetErrorString(e)); return MINTB_ECUDA; }
+  return MINTB_OK;
+}
+
+}  // namespace
+
+size_t sgemm_tc_workspace_bytes(int groups, int M, int N, int K) {
+  return align256(size_t(M) * padded_k(K) * 6) + align256(size_t(groups) * N * padded_k(K) * 6);
+}
+
+// Nanoseconds of the product with 128 x BN tiles, as measured: the passes' ends, then per 32 columns the rounds of twelve products on the
+// busiest SM or the pieces of all tiles from L2 (6.3 TB/s), whichever is longer.
+static long long tc_ns(int groups, int M, int N, int K, bool wide) {
+  const long long tiles = static_cast<long long>((M + kBM - 1) / kBM) * ((groups * N + (wide ? 127 : 63)) / (wide ? 128 : 64)), sms = sm_count();
+  const long long mma = (tiles + sms - 1) / sms * (wide ? 520 : 440), l2 = tiles * (wide ? 760 : 570) / 100;
+  return (wide ? 8400 : 6200) + (K + kSum - 1) / kSum * (mma > l2 ? mma : l2);
+}
+
+// Where the tensor cores win: M2048 K320 six weights of N320 63.4 -> 26.4 us, N320 16.9 -> 11.9, N1280 44.6 -> 22.5, K1280 N320
+// 58.2 -> 28.9; M5120 143 -> 50, 31 -> 18, 95 -> 37, 111 -> 47.  Few tiles or a short x leave them to the CUDA cores, whose time goes
+// with the multiply-adds (13.3 per ps) or the length of one sum: M700 N320 K320 8.8 us (10.6), M100 N320 K1280 14.9 (23.8),
+// M700 N320 K1280 24.7 (25.1).
+bool sgemm_tc_wins(int groups, int M, int N, int K) {
+  const long long work = static_cast<long long>(M) * N * K * groups / 13300, chain = static_cast<long long>(K) * 10;
+  const long long wide = tc_ns(groups, M, N, K, true), narrow = tc_ns(groups, M, N, K, false), simt = 2300 + (work > chain ? work : chain);
+  return 11 * (wide < narrow ? wide : narrow) < 10 * simt;
+}
+
+int launch_sgemm_tc(const SgemmParams& p, int groups, void* workspace, cudaStream_t s, int* status) {
+  if (tc_ns(groups, p.M, p.N, p.K, true) <= tc_ns(groups, p.M, p.N, p.K, false)) return launch_tc_t<128>(p, groups, workspace, s, status);
+  return launch_tc_t<64>(p, groups, workspace, s, status);
+}
+
+}  // namespace mintb

@@ -1,5 +1,7 @@
 """fp32 projections at the edges of their tiles (32 / 64 rows and columns, slabs of 16 to 128 columns) against float64, and the layer that
 runs on them against the same layer with gradients on, whose projections are autograd's."""
+import ctypes
+
 import pytest
 import torch
 
@@ -36,3 +38,38 @@ def test_layer_f32(fused, T, B, H, D):
     ref, _ = layer(x, self_attn_padding_mask=pad, chain_ids=chain_ids)
     assert ref.requires_grad
     torch.testing.assert_close(y, ref.detach(), rtol=2e-5, atol=2e-5)
+
+
+@pytest.mark.parametrize("m,n,k,groups,d", [(1, 4, 4, 1, 0), (128, 64, 32, 1, 0), (129, 68, 36, 2, 0), (300, 320, 324, 6, 16), (700, 100, 1284, 3, 0), (20000, 32, 64, 1, 32)])
+def test_linear_f32_on_the_tensor_cores(m, n, k, groups, d):
+    """Edges of the 128 x 128 / 64 tiles, of the slabs of 32 and 64 columns and between the weights; errors as those of fp32 sums.  What
+    has no bf16 pieces - infinities, NaN, values next to the largest fp32 number - gives what the CUDA cores give."""
+    torch.manual_seed(0)
+    lib = _lib.lib()
+    x = torch.randn(m, k, device="cuda")
+    ws = [torch.randn(n, k, device="cuda") * k ** -0.5 for _ in range(groups)]
+    bs = [torch.randn(n, device="cuda") for _ in range(groups)]
+
+    def run(x, tensor_cores):
+        outs = [torch.full((m, n), -7.0, device="cuda") for _ in range(groups)]
+        size = lib.mintb_linear_f32_tc_workspace_bytes(groups, m, n, k)
+        work = torch.empty(size, dtype=torch.uint8, device="cuda") if tensor_cores else None
+        arr = ctypes.c_void_p * groups
+        rc = lib.mintb_linear_f32_tc(x.data_ptr(), arr(*[w.data_ptr() for w in ws]), arr(*[b.data_ptr() for b in bs]), arr(*[o.data_ptr() for o in outs]), None,
+                                     groups, m, n, k, 0, 1, m, n // d if d else 1, d, work.data_ptr() if tensor_cores else None, size if tensor_cores else 0,
+                                     torch.cuda.current_stream().cuda_stream, None)
+        assert rc == 0
+        torch.cuda.synchronize()
+        return torch.stack([o.view(n // d, m, d).transpose(0, 1).reshape(m, n) if d else o for o in outs])
+
+    got, simt = run(x, True), run(x, False)
+    ref = torch.stack([x.double() @ w.double().T + b.double() for w, b in zip(ws, bs)])
+    torch.testing.assert_close(got.double(), ref, rtol=2e-6, atol=2e-6)
+    # no further off than the fma chains; a sum of a few terms is off by its last rounding, half a unit of 2^-23, either way
+    assert (got - ref).norm() <= max(1.2 * (simt - ref).norm(), 2.0 ** -24 * ref.norm())
+    x[m // 2, k // 2], x[0, 0], x[m - 1, k - 1] = 3.4e38, float("inf"), float("nan")
+    ws[0][n // 2, k // 2] = -float("inf")
+    got, simt = run(x, True), run(x, False)
+    bad = ~simt.isfinite()
+    assert bad.any() and torch.equal(got.isnan(), simt.isnan()) and torch.equal(got[bad & ~simt.isnan()], simt[bad & ~simt.isnan()])
+    torch.testing.assert_close(got[~bad], simt[~bad], rtol=1e-5, atol=4e-6)
