@@ -12,7 +12,7 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libmintb.so")
-SOURCES = ["api.cu", "prep.cu", "attn_simt.cu", "sgemm.cu", "sgemm_tc.cu", "attn_tc.cu", "attn_tc_bwd.cu", "gemm_tc.cu", "gemm_bwd.cu", "combine.cu", "glue.cu", "embed_loss.cu", "selftest.cu"]
+SOURCES = ["api.cu", "prep.cu", "attn_simt.cu", "attn_f32.cu", "sgemm.cu", "sgemm_tc.cu", "attn_tc.cu", "attn_tc_bwd.cu", "gemm_tc.cu", "gemm_bwd.cu", "combine.cu", "glue.cu", "embed_loss.cu", "selftest.cu"]
 HOST = os.path.join(CSRC, "host")
 HOST_LIB = os.path.join(HERE, "_mintb_host.so")
 HOST_SOURCES = ["launch.cpp", "ops.cpp", "layer.cpp", "bind.cpp"]

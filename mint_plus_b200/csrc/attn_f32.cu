@@ -1,0 +1,687 @@
+// fp32 attention (forward, dQ, dK/dV) of head_dim 16 and 32 with its contractions on the warp-level matrix instruction, in fp32 precision.
+//
+// Every fp32 operand - and the probabilities and dS, which are formed in fp32 - is the sum of three bf16 numbers, and six of the nine
+// products of the pieces make up the fp32 product to 2^-25.  The instruction's accumulation truncates, so an accumulator takes the six
+// products of 16 columns, the smallest first, and what spans more columns is summed outside, rounding to nearest.
+// As loops of packed multiply-adds (attn_simt.cu) the contractions and the shared-memory reads that feed them took nearly all of the time:
+// B4 H20 T401 D16 forward + backward 208 -> 126 us, D32 446 -> 219, B4 H20 T640 D16 forward 105 -> 70.  What is left is spread: the
+// matrix pipe 29 to 43 % busy, the splitting, and the wait for a tile to be staged (more warps at fewer registers: no faster).
+// Error against fp64 as that of the fma chains: at T401 D16 1.2e-7 (out), 3.6e-7 (dQ, dK), 3.3e-7 (dV) against 1.2e-7, 3.6e-7, 3.5e-7.
+//
+// A CTA of four warps owns 64 rows (queries in forward and dQ, keys in dK/dV; one row of the class table) and walks the tiles of 64 along
+// the other axis; a warp keeps the pieces of its 16 rows in registers.  Results are in a fixed order: no atomics.
+// Rows with a result that is not finite are formed again in plain fp32: an infinite value, or one that rounds to infinity as bf16, has
+// no pieces.
+#include "simt.cuh"
+
+namespace mintb {
+namespace {
+
+constexpr int kWarps = 4, kThreads = 32 * kWarps, kTile = 64;
+static_assert(kTile == kClassTile && kTile == 16 * kWarps, "a CTA's rows and a tile of the other axis are entries of the class table");
+
+typedef __nv_bfloat16 bf16;
+
+template <int D>
+struct Cfg {
+  static constexpr int LD = D + 8;                    // the 16-byte pad makes the eight rows of an ldmatrix start in different banks
+  static constexpr int kPiece = kTile * LD;           // elements of one piece of a tile
+  static constexpr int kBuf = 3 * kPiece;
+};
+
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ uint32_t pack2(float lo, float hi) {
+  uint32_t r;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+  return r;
+}
+// the three bf16 pieces of the pair (a, b), most significant first
+__device__ __forceinline__ void split(float a, float b, uint32_t (&out)[3]) {
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    out[k] = pack2(a, b);
+    if (k < 2) {
+      a -= __uint_as_float(out[k] << 16);
+      b -= __uint_as_float(out[k] & 0xffff0000u);
+    }
+  }
+}
+__device__ __forceinline__ void mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+template <bool TRANS>
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], const bf16* p) {
+  const uint32_t a = uint32_t(__cvta_generic_to_shared(p));
+  if constexpr (TRANS)
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
+  else
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
+}
+__device__ __forceinline__ float4 ldg4(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
+
+// The pairs of pieces whose products count, the smallest first.
+__host__ __device__ constexpr int piece_a(int q) { return q == 0 ? 2 : q == 2 || q == 3 ? 1 : 0; }
+__host__ __device__ constexpr int piece_b(int q) { return q == 1 ? 2 : q == 2 || q == 4 ? 1 : 0; }
+
+// Rows [r0, r0 + 64) of x[T][..] as pieces dst[3][64][LD] (zeros past T), rotated when tables are given:
+// y[d] = x[d] cos - x[d+h] sin (d < h), y[d] = x[d] cos + x[d-h] sin (d >= h)   (rotary_embedding.py:16-24).
+template <int D>
+__device__ __forceinline__ void stage(const float* __restrict__ x, size_t row_stride, int r0, int Tlen, const float* __restrict__ cos_tab,
+                                      const float* __restrict__ sin_tab, bf16* __restrict__ dst) {
+  constexpr int h = D / 2, PER = h / 4;
+#pragma unroll
+  for (int i0 = 0; i0 < kTile * PER; i0 += kThreads) {
+    const int i = i0 + threadIdx.x, r = i / PER, c = i % PER * 4, t = r0 + r;
+    float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
+    if (t < Tlen) {
+      lo = ldg4(x + size_t(t) * row_stride + c);
+      hi = ldg4(x + size_t(t) * row_stride + c + h);
+      if (cos_tab != nullptr) {
+        const float4 cs = ldg4(cos_tab + size_t(t) * h + c), sn = ldg4(sin_tab + size_t(t) * h + c);
+        const float4 a = lo, b = hi;
+        lo = make_float4(a.x * cs.x - b.x * sn.x, a.y * cs.y - b.y * sn.y, a.z * cs.z - b.z * sn.z, a.w * cs.w - b.w * sn.w);
+        hi = make_float4(b.x * cs.x + a.x * sn.x, b.y * cs.y + a.y * sn.y, b.z * cs.z + a.z * sn.z, b.w * cs.w + a.w * sn.w);
+      }
+    }
+    uint32_t p0[3], p1[3];
+    bf16* row = dst + r * Cfg<D>::LD + c;
+    split(lo.x, lo.y, p0); split(lo.z, lo.w, p1);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) *reinterpret_cast<uint2*>(row + q * Cfg<D>::kPiece) = make_uint2(p0[q], p1[q]);
+    split(hi.x, hi.y, p0); split(hi.z, hi.w, p1);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) *reinterpret_cast<uint2*>(row + h + q * Cfg<D>::kPiece) = make_uint2(p0[q], p1[q]);
+  }
+}
+
+// This warp's 16 rows of a staged tile as the left operand: [piece][16 columns of d][register].
+template <int D>
+__device__ __forceinline__ void left_rows(uint32_t (&a)[3][D / 16][4], const bf16* tile, int warp, int lane) {
+#pragma unroll
+  for (int q = 0; q < 3; ++q)
+#pragma unroll
+    for (int k = 0; k < D / 16; ++k) ldsm4<false>(a[q][k], tile + q * Cfg<D>::kPiece + (16 * warp + lane % 8 + 8 * ((lane / 8) & 1)) * Cfg<D>::LD + 16 * k + 8 * (lane / 16));
+}
+// c[j][..] = the warp's rows . rows [16 g, 16 g + 16) of a staged tile, in the accumulator layout: lane (r, t) holds rows r and r + 8,
+// columns 8 j + 2 t and the next.
+template <int D>
+__device__ __forceinline__ void dots(float (&c)[2][4], const uint32_t (&a)[3][D / 16][4], const bf16* tile, int g, int lane) {
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) c[j][e] = 0.f;
+  uint32_t b[3][D / 16][4];
+#pragma unroll
+  for (int q = 0; q < 3; ++q)
+#pragma unroll
+    for (int k = 0; k < D / 16; ++k) ldsm4<false>(b[q][k], tile + q * Cfg<D>::kPiece + (16 * g + lane % 8 + 8 * (lane / 16)) * Cfg<D>::LD + 16 * k + 8 * ((lane / 8) & 1));
+#pragma unroll
+  for (int q = 0; q < 6; ++q)
+#pragma unroll
+    for (int k = 0; k < D / 16; ++k)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) mma(c[j], a[piece_a(q)][k], b[piece_b(q)][k][2 * j], b[piece_b(q)][k][2 * j + 1]);
+}
+// acc += w . rows [16 g, 16 g + 16) of a staged tile, w (16 x 16, accumulator layout) split into pieces here
+template <int D>
+__device__ __forceinline__ void axpy(float (&acc)[D / 8][4], const float (&w)[2][4], const bf16* tile, int g, int lane) {
+  uint32_t a[3][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    uint32_t s[3];
+    split(w[i / 2][2 * (i % 2)], w[i / 2][2 * (i % 2) + 1], s);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) a[q][i] = s[q];
+  }
+#pragma unroll
+  for (int d = 0; d < D / 16; ++d) {
+    uint32_t b[3][4];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) ldsm4<true>(b[q], tile + q * Cfg<D>::kPiece + (16 * g + lane % 8 + 8 * ((lane / 8) & 1)) * Cfg<D>::LD + 16 * d + 8 * (lane / 16));
+    float o[2][4];
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) o[j][e] = 0.f;
+#pragma unroll
+    for (int q = 0; q < 6; ++q)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) mma(o[j], a[piece_a(q)], b[piece_b(q)][2 * j], b[piece_b(q)][2 * j + 1]);
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[2 * d + j][e] += o[j][e];
+  }
+}
+
+template <int N>
+__device__ __forceinline__ void clear(float (&v)[N][4]) {
+#pragma unroll
+  for (int n = 0; n < N; ++n)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) v[n][e] = 0.f;
+}
+// A tile's sums are formed by themselves before they are added to the whole: a tenth less error at T = 400 than one chain of 16-column sums.
+template <int N>
+__device__ __forceinline__ void add(float (&v)[N][4], const float (&w)[N][4]) {
+#pragma unroll
+  for (int n = 0; n < N; ++n)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) v[n][e] += w[n][e];
+}
+
+__device__ __forceinline__ float quad_sum(float v) {   // over the four lanes of a row
+  v += __shfl_xor_sync(0xffffffffu, v, 1);
+  return v + __shfl_xor_sync(0xffffffffu, v, 2);
+}
+__device__ __forceinline__ float quad_max(float v) {
+  v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 1));
+  return fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 2));
+}
+__device__ __forceinline__ float warp_sum(float v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+template <int N>
+__device__ __forceinline__ bool finite(const float (&v)[N][4], int h) {   // rows r (h = 0) and r + 8
+  bool ok = true;
+#pragma unroll
+  for (int i = 0; i < N; ++i) ok = ok && fabsf(v[i][2 * h]) <= 3.402823466e38f && fabsf(v[i][2 * h + 1]) <= 3.402823466e38f;
+  return ok;
+}
+// bit r: row r of the warp's 16 has a value that is not finite
+__device__ __forceinline__ uint32_t bad_rows(bool bad_lo, bool bad_hi) {
+  const uint32_t lo = __ballot_sync(0xffffffffu, bad_lo), hi = __ballot_sync(0xffffffffu, bad_hi);
+  uint32_t rows = 0;
+#pragma unroll
+  for (int r = 0; r < 8; ++r) rows |= ((lo >> (4 * r)) & 15u ? 1u << r : 0u) | ((hi >> (4 * r)) & 15u ? 256u << r : 0u);
+  return rows;
+}
+// element d of row t, rotated when tables are given (plain fp32 paths, lane d; 0 past D)
+template <int D>
+__device__ __forceinline__ float rotated(const float* row, int t, const float* cos_tab, const float* sin_tab, int d) {
+  constexpr int h = D / 2;
+  if (d >= D) return 0.f;
+  if (cos_tab == nullptr) return __ldg(row + d);
+  const float c = __ldg(cos_tab + size_t(t) * h + d % h), s = __ldg(sin_tab + size_t(t) * h + d % h);
+  return d < h ? __ldg(row + d) * c - __ldg(row + d + h) * s : __ldg(row + d) * c + __ldg(row + d - h) * s;
+}
+__device__ __forceinline__ bool bit_of(const uint32_t* words, int i) { return (__ldg(words + i / 32) >> (i % 32)) & 1u; }
+
+// dst[..] = f * acc (un-rotated when tables are given: R^T: dx_lo = dy_lo c + dy_hi s, dx_hi = dy_hi c - dy_lo s) for rows r and r + 8;
+// the partner dimension, half a row away, is in the same lane.
+template <int D>
+__device__ __forceinline__ void write_rows(float (&acc)[D / 8][4], float* base, int row0, int Tlen, int lane, float f, const float* cos_tab, const float* sin_tab) {
+  constexpr int h = D / 2;
+#pragma unroll
+  for (int hh = 0; hh < 2; ++hh) {
+    const int t = row0 + lane / 4 + 8 * hh;
+    if (t >= Tlen) continue;
+#pragma unroll
+    for (int n = 0; n < D / 16; ++n) {
+      float2 lo = make_float2(acc[n][2 * hh], acc[n][2 * hh + 1]), hi = make_float2(acc[n + D / 16][2 * hh], acc[n + D / 16][2 * hh + 1]);
+      const int d = 8 * n + 2 * (lane % 4);
+      if (cos_tab != nullptr) {
+        const float2 c = __ldg(reinterpret_cast<const float2*>(cos_tab + size_t(t) * h + d)), s = __ldg(reinterpret_cast<const float2*>(sin_tab + size_t(t) * h + d));
+        const float2 a = lo, b = hi;
+        lo = make_float2(a.x * c.x + b.x * s.x, a.y * c.y + b.y * s.y);
+        hi = make_float2(b.x * c.x - a.x * s.x, b.y * c.y - a.y * s.y);
+      }
+      *reinterpret_cast<float2*>(base + size_t(t) * D + d) = make_float2(lo.x * f, lo.y * f);
+      *reinterpret_cast<float2*>(base + size_t(t) * D + d + h) = make_float2(hi.x * f, hi.y * f);
+    }
+  }
+}
+template <int D>
+__device__ __forceinline__ void write_row(float v, float* base, int t, int lane, float f, const float* cos_tab, const float* sin_tab) {   // plain paths: lane d
+  constexpr int h = D / 2;
+  const float o = __shfl_xor_sync(0xffffffffu, v, h);
+  if (lane >= D) return;
+  if (cos_tab != nullptr) {
+    const float c = __ldg(cos_tab + size_t(t) * h + lane % h), s = __ldg(sin_tab + size_t(t) * h + lane % h);
+    v = lane < h ? v * c + o * s : v * c - o * s;
+  }
+  base[size_t(t) * D + lane] = v * f;
+}
+
+// ------------------------------------------------------------------------------------------------ forward
+template <int D, bool SQ>
+__global__ void __launch_bounds__(kThreads) attn_fwd_f32_kernel(const __grid_constant__ SimtParams p) {
+  constexpr int kBuf = Cfg<D>::kBuf;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  bf16 *sk_s = reinterpret_cast<bf16*>(smem_raw), *sv_s = sk_s + kBuf, *sk_c = sv_s + kBuf, *sv_c = sk_c + kBuf;
+  const int bh = blockIdx.y, b = bh / p.H, i0 = blockIdx.x * kTile;
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, t2 = 2 * (lane % 4);
+  const size_t head = size_t(bh) * p.T * D;
+  const float *q_s = static_cast<const float*>(p.q_s) + head, *q_c = static_cast<const float*>(p.q_c) + head, *k_s = static_cast<const float*>(p.k_s) + head,
+              *k_c = static_cast<const float*>(p.k_c) + head, *v_s = static_cast<const float*>(p.v_s) + head, *v_c = static_cast<const float*>(p.v_c) + head;
+  stage<D>(q_s, D, i0, p.T, p.cos_tab, p.sin_tab, sk_s);
+  stage<D>(q_c, D, i0, p.T, nullptr, nullptr, sk_c);
+  __syncthreads();
+  uint32_t aq_s[3][D / 16][4], aq_c[3][D / 16][4];
+  left_rows<D>(aq_s, sk_s, warp, lane);
+  left_rows<D>(aq_c, sk_c, warp, lane);
+  const float c2 = p.scale * kLog2e;
+  float o[D / 8][4], m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
+#pragma unroll
+  for (int n = 0; n < D / 8; ++n)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) o[n][e] = 0.f;
+  const int row = i0 + 16 * warp + lane / 4;
+  const uint32_t* mrow[2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {   // rows past T compute on zeros and are not stored
+    const int i = row + 8 * h;
+    mrow[h] = p.bits + (size_t(b) * p.T + (i < p.T ? i : p.T - 1)) * p.TW;
+  }
+  const uint8_t* cls = p.cls + (size_t(b) * p.NT + blockIdx.x) * p.NT;
+
+  for (int kt = 0; kt < p.NT; ++kt) {
+    const uint8_t c = cls[kt];
+    const bool intra = c & kHasIntra, inter = c & kHasInter;
+    if (!intra && !inter) continue;   // block-uniform: every key of the tile is padded
+    const int j0 = kt * kTile;
+    __syncthreads();
+    if (intra) {
+      stage<D>(k_s, D, j0, p.T, p.cos_tab, p.sin_tab, sk_s);
+      stage<D>(v_s, D, j0, p.T, nullptr, nullptr, sv_s);
+    }
+    if (inter) {
+      stage<D>(k_c, D, j0, p.T, nullptr, nullptr, sk_c);
+      stage<D>(v_c, D, j0, p.T, nullptr, nullptr, sv_c);
+    }
+    uint32_t cross[2][2], pad[2];
+#pragma unroll
+    for (int w = 0; w < 2; ++w) {
+      pad[w] = (c & kHasPad) ? __ldg(p.kpad + size_t(b) * p.TW + 2 * kt + w) : 0u;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) cross[h][w] = intra && inter ? __ldg(mrow[h] + 2 * kt + w) : inter ? 0xffffffffu : 0u;
+    }
+    __syncthreads();
+    float s[8][4];
+    bool any_i[4], any_x[4];   // of the warp's rows against 16 keys
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      const uint32_t x0 = (cross[0][g / 2] >> (16 * (g % 2))) & 0xffffu, x1 = (cross[1][g / 2] >> (16 * (g % 2))) & 0xffffu;
+      any_i[g] = __any_sync(0xffffffffu, (x0 & x1) != 0xffffu);
+      any_x[g] = __any_sync(0xffffffffu, (x0 | x1) != 0u);
+      float u[2][4];
+      if (any_i[g]) dots<D>(u, aq_s, sk_s, g, lane);
+      if (any_x[g]) {
+        float x[2][4];
+        dots<D>(x, aq_c, sk_c, g, lane);
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            if (!any_i[g] || (((e < 2 ? x0 : x1) >> (8 * j + t2 + e % 2)) & 1u)) u[j][e] = x[j][e];
+      }
+      const uint32_t pw = (pad[g / 2] >> (16 * (g % 2))) & 0xffffu;
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s[2 * g + j][e] = (pw >> (8 * j + t2 + e % 2)) & 1u ? -INFINITY : u[j][e] * c2;
+    }
+    float alpha[2];
+    bool grown = false;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float mx = fmaxf(s[0][2 * h], s[0][2 * h + 1]);
+#pragma unroll
+      for (int n = 1; n < 8; ++n) mx = fmaxf(mx, fmaxf(s[n][2 * h], s[n][2 * h + 1]));
+      const float m_new = fmaxf(m[h], quad_max(mx));
+      // square-root softmax accumulates sqrt(p) v: the terms are exp2((s - m) / 2), the row sum stays sum exp2(s - m)
+      alpha[h] = m_new == m[h] ? 1.f : ex2(m[h] - m_new);
+      grown = grown || m_new != m[h];
+      m[h] = m_new;
+      const float ref = m_new == -INFINITY ? 0.f : m_new;   // (only padded keys so far)
+      float sum[2] = {0.f, 0.f};
+#pragma unroll
+      for (int n = 0; n < 8; ++n)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          float& x = s[n][2 * h + e];
+          x = ex2(SQ ? 0.5f * (x - ref) : x - ref);
+          sum[e] = SQ ? fmaf(x, x, sum[e]) : sum[e] + x;
+        }
+      l[h] = fmaf(l[h], alpha[h], sum[0] + sum[1]);
+    }
+    if (__any_sync(0xffffffffu, grown)) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const float f = SQ ? sqrtf(alpha[h]) : alpha[h];
+#pragma unroll
+        for (int n = 0; n < D / 8; ++n) { o[n][2 * h] *= f; o[n][2 * h + 1] *= f; }
+      }
+    }
+    float ot[D / 8][4];
+    clear(ot);
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      float w[2][4];
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) w[j][e] = s[2 * g + j][e];
+      if (any_i[g] && any_x[g]) {
+        float x[2][4];
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const bool is_x = (cross[e / 2][g / 2] >> (16 * (g % 2) + 8 * j + t2 + e % 2)) & 1u;
+            x[j][e] = is_x ? w[j][e] : 0.f;
+            if (is_x) w[j][e] = 0.f;
+          }
+        axpy<D>(ot, x, sv_c, g, lane);
+      }
+      axpy<D>(ot, w, any_i[g] ? sv_s : sv_c, g, lane);
+    }
+    add(o, ot);
+  }
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int i = row + 8 * h;
+    const float lt = quad_sum(l[h]);
+    // A row whose keys are all padded gives 0/0 = NaN, as the softmax of an all -inf row does in PyTorch.
+    const float inv = SQ ? rsqrtf(lt) : 1.f / lt;
+#pragma unroll
+    for (int n = 0; n < D / 8; ++n) {
+      o[n][2 * h] *= inv;
+      o[n][2 * h + 1] *= inv;
+      if (i < p.T)
+        *reinterpret_cast<float2*>(static_cast<float*>(p.out) + size_t(bh) * p.o_bh + size_t(i) * p.o_row + 8 * n + t2) = make_float2(o[n][2 * h], o[n][2 * h + 1]);
+    }
+    if (i < p.T && lane % 4 == 0) p.lse[size_t(bh) * p.T + i] = (m[h] + log2f(lt)) * kLn2;
+  }
+  uint32_t bad = bad_rows(!finite(o, 0), !finite(o, 1));
+  for (; bad != 0; bad &= bad - 1) {
+    const int i = i0 + 16 * warp + __ffs(bad) - 1;
+    if (i >= p.T) break;
+    const float qs = rotated<D>(q_s + size_t(i) * D, i, p.cos_tab, p.sin_tab, lane), qc = rotated<D>(q_c + size_t(i) * D, i, nullptr, nullptr, lane);
+    float acc = 0.f, mr = -INFINITY, lr = 0.f;
+#pragma unroll 1
+    for (int j = 0; j < p.T; ++j) {
+      if (bit_of(p.kpad + size_t(b) * p.TW, j)) continue;
+      const bool x = bit_of(p.bits + (size_t(b) * p.T + i) * p.TW, j);
+      const float k = x ? rotated<D>(k_c + size_t(j) * D, j, nullptr, nullptr, lane) : rotated<D>(k_s + size_t(j) * D, j, p.cos_tab, p.sin_tab, lane);
+      const float v = rotated<D>((x ? v_c : v_s) + size_t(j) * D, j, nullptr, nullptr, lane);
+      const float sj = warp_sum(lane < D ? (x ? qc : qs) * k : 0.f) * c2, m_new = fmaxf(mr, sj);
+      const float al = m_new == mr ? 1.f : ex2(mr - m_new), ref = m_new == -INFINITY ? 0.f : m_new, w = ex2(SQ ? 0.5f * (sj - ref) : sj - ref);
+      mr = m_new;
+      lr = lr * al + (SQ ? w * w : w);
+      acc = acc * (SQ ? sqrtf(al) : al) + w * v;
+    }
+    if (lane < D) static_cast<float*>(p.out)[size_t(bh) * p.o_bh + size_t(i) * p.o_row + lane] = acc * (SQ ? rsqrtf(lr) : 1.f / lr);
+    if (lane == 0) p.lse[size_t(bh) * p.T + i] = (mr + log2f(lr)) * kLn2;
+  }
+}
+
+// ds from the scaled logit relative to lse, x = s c - lse log2 e:  softmax: w = p, ds = p (dp - delta).
+// Square-root softmax: w = sqrt(p), ds = w (dp - w delta) / 2.
+template <bool SQ>
+__device__ __forceinline__ void grads(float x, float dp, float delta, float& w, float& ds) {
+  w = ex2(SQ ? 0.5f * x : x);
+  ds = SQ ? 0.5f * w * (dp - w * delta) : w * (dp - delta);
+}
+
+// ------------------------------------------------------------------------------------------------ dQ (+ delta)
+// Of one pathway (blockIdx.z).  delta_i = dO_i . O_i;  dq~ = sum over the pathway's keys of ds k~(j);  dq_self = scale R^T dq~, dq_cross = scale dq~.
+template <int D, bool SQ>
+__global__ void __launch_bounds__(kThreads) attn_bwd_dq_f32_kernel(const __grid_constant__ SimtParams p) {
+  constexpr int kBuf = Cfg<D>::kBuf;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  bf16 *sk = reinterpret_cast<bf16*>(smem_raw), *sv = sk + kBuf;
+  const bool path = blockIdx.z != 0;   // cross
+  const int bh = blockIdx.y, b = bh / p.H, i0 = blockIdx.x * kTile;
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, t2 = 2 * (lane % 4);
+  const size_t head = size_t(bh) * p.T * D;
+  const float *cos_tab = path ? nullptr : p.cos_tab, *sin_tab = path ? nullptr : p.sin_tab;
+  const float *q_g = static_cast<const float*>(path ? p.q_c : p.q_s) + head, *k_g = static_cast<const float*>(path ? p.k_c : p.k_s) + head,
+              *v_g = static_cast<const float*>(path ? p.v_c : p.v_s) + head, *dO = static_cast<const float*>(p.d_out) + size_t(bh) * p.o_bh,
+              *o = static_cast<const float*>(p.out) + size_t(bh) * p.o_bh;
+  float* dq = static_cast<float*>(path ? p.dq_c : p.dq_s) + head;
+  stage<D>(q_g, D, i0, p.T, cos_tab, sin_tab, sk);
+  stage<D>(dO, p.o_row, i0, p.T, nullptr, nullptr, sv);
+  __syncthreads();
+  uint32_t aq[3][D / 16][4], ag[3][D / 16][4];
+  left_rows<D>(aq, sk, warp, lane);
+  left_rows<D>(ag, sv, warp, lane);
+  const float c2 = p.scale * kLog2e;
+  float acc[D / 8][4], delta[2], lse2[2];
+#pragma unroll
+  for (int n = 0; n < D / 8; ++n)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[n][e] = 0.f;
+  const int row = i0 + 16 * warp + lane / 4;
+  const uint32_t* mrow[2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int i = row + 8 * h, ic = i < p.T ? i : p.T - 1;
+    float part = 0.f;
+#pragma unroll
+    for (int d = lane % 4; d < D; d += 4) part = fmaf(__ldg(dO + size_t(ic) * p.o_row + d), __ldg(o + size_t(ic) * p.o_row + d), part);
+    delta[h] = quad_sum(part);
+    lse2[h] = __ldg(p.lse + size_t(bh) * p.T + ic) * kLog2e;
+    if (!path && lane % 4 == 0 && i < p.T) p.delta[size_t(bh) * p.T + i] = delta[h];
+    mrow[h] = p.bits + (size_t(b) * p.T + ic) * p.TW;
+  }
+  const uint8_t* cls = p.cls + (size_t(b) * p.NT + blockIdx.x) * p.NT;
+  const uint8_t mine = path ? kHasInter : kHasIntra, other = path ? kHasIntra : kHasInter;
+
+  for (int kt = 0; kt < p.NT; ++kt) {
+    const uint8_t c = cls[kt];
+    if (!(c & mine)) continue;
+    const int j0 = kt * kTile;
+    __syncthreads();
+    stage<D>(k_g, D, j0, p.T, cos_tab, sin_tab, sk);
+    stage<D>(v_g, D, j0, p.T, nullptr, nullptr, sv);
+    uint32_t drop[2][2];   // keys of the row that are padded or belong to the other pathway
+#pragma unroll
+    for (int w = 0; w < 2; ++w) {
+      const uint32_t pad = (c & kHasPad) ? __ldg(p.kpad + size_t(b) * p.TW + 2 * kt + w) : 0u;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const uint32_t bits = c & other ? __ldg(mrow[h] + 2 * kt + w) : 0u;
+        drop[h][w] = pad | (c & other ? (path ? ~bits : bits) : 0u);
+      }
+    }
+    __syncthreads();
+    float at[D / 8][4];
+    clear(at);
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      const uint32_t d0 = (drop[0][g / 2] >> (16 * (g % 2))) & 0xffffu, d1 = (drop[1][g / 2] >> (16 * (g % 2))) & 0xffffu;
+      if (__all_sync(0xffffffffu, (d0 & d1) == 0xffffu)) continue;
+      float s[2][4], dp[2][4];
+      dots<D>(s, aq, sk, g, lane);
+      dots<D>(dp, ag, sv, g, lane);
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          float w, ds;
+          grads<SQ>(s[j][e] * c2 - lse2[e / 2], dp[j][e], delta[e / 2], w, ds);
+          s[j][e] = ((e < 2 ? d0 : d1) >> (8 * j + t2 + e % 2)) & 1u ? 0.f : ds;
+        }
+      axpy<D>(at, s, sk, g, lane);
+    }
+    add(acc, at);
+  }
+  uint32_t bad = bad_rows(!finite(acc, 0), !finite(acc, 1));
+  write_rows<D>(acc, dq, i0 + 16 * warp, p.T, lane, p.scale, cos_tab, sin_tab);
+  __syncwarp();
+  for (; bad != 0; bad &= bad - 1) {
+    const int r = __ffs(bad) - 1, i = i0 + 16 * warp + r;
+    if (i >= p.T) break;
+    const float q = rotated<D>(q_g + size_t(i) * D, i, cos_tab, sin_tab, lane), go = rotated<D>(dO + size_t(i) * p.o_row, i, nullptr, nullptr, lane);
+    const float l2 = __shfl_sync(0xffffffffu, r < 8 ? lse2[0] : lse2[1], 4 * (r % 8)), de = __shfl_sync(0xffffffffu, r < 8 ? delta[0] : delta[1], 4 * (r % 8));
+    float a = 0.f;
+#pragma unroll 1
+    for (int j = 0; j < p.T; ++j) {
+      if (bit_of(p.kpad + size_t(b) * p.TW, j) || bit_of(p.bits + (size_t(b) * p.T + i) * p.TW, j) != path) continue;
+      const float k = rotated<D>(k_g + size_t(j) * D, j, cos_tab, sin_tab, lane), v = rotated<D>(v_g + size_t(j) * D, j, nullptr, nullptr, lane);
+      float w, ds;
+      grads<SQ>(warp_sum(lane < D ? q * k : 0.f) * c2 - l2, warp_sum(lane < D ? go * v : 0.f), de, w, ds);
+      a = fmaf(ds, k, a);
+    }
+    write_row<D>(a, dq, i, lane, p.scale, cos_tab, sin_tab);
+  }
+}
+
+// ------------------------------------------------------------------------------------------------ dK, dV
+// Of one pathway, per key row j, over query tiles:  dv += w dO_i;  dk~ += ds scale q~(i).
+template <int D, bool SQ>
+__global__ void __launch_bounds__(kThreads) attn_bwd_dkv_f32_kernel(const __grid_constant__ SimtParams p) {
+  constexpr int kBuf = Cfg<D>::kBuf;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  bf16 *sq = reinterpret_cast<bf16*>(smem_raw), *sg = sq + kBuf;
+  float *slse2 = reinterpret_cast<float*>(sg + kBuf), *sdelta = slse2 + kTile;
+  const bool path = blockIdx.z != 0;
+  const int bh = blockIdx.y, b = bh / p.H, j0 = blockIdx.x * kTile;
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, t2 = 2 * (lane % 4);
+  const size_t head = size_t(bh) * p.T * D;
+  const float *cos_tab = path ? nullptr : p.cos_tab, *sin_tab = path ? nullptr : p.sin_tab;
+  const float *q_g = static_cast<const float*>(path ? p.q_c : p.q_s) + head, *k_g = static_cast<const float*>(path ? p.k_c : p.k_s) + head,
+              *v_g = static_cast<const float*>(path ? p.v_c : p.v_s) + head, *dO = static_cast<const float*>(p.d_out) + size_t(bh) * p.o_bh;
+  float *dk_g = static_cast<float*>(path ? p.dk_c : p.dk_s) + head, *dv_g = static_cast<float*>(path ? p.dv_c : p.dv_s) + head;
+  stage<D>(k_g, D, j0, p.T, cos_tab, sin_tab, sq);
+  stage<D>(v_g, D, j0, p.T, nullptr, nullptr, sg);
+  __syncthreads();
+  uint32_t ak[3][D / 16][4], av[3][D / 16][4];
+  left_rows<D>(ak, sq, warp, lane);
+  left_rows<D>(av, sg, warp, lane);
+  const float c2 = p.scale * kLog2e;
+  float dk[D / 8][4], dv[D / 8][4];
+#pragma unroll
+  for (int n = 0; n < D / 8; ++n)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) dk[n][e] = dv[n][e] = 0.f;
+  const int row = j0 + 16 * warp + lane / 4;
+  const uint32_t* mrow[2];
+  bool dead[2];   // padded keys have probability zero
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int j = row + 8 * h, jc = j < p.T ? j : p.T - 1;
+    dead[h] = j >= p.T || bit_of(p.kpad + size_t(b) * p.TW, jc);
+    mrow[h] = p.bitsT + (size_t(b) * p.T + jc) * p.TW;
+  }
+  const uint8_t* cls = p.cls + size_t(b) * p.NT * p.NT + blockIdx.x;
+  const uint8_t mine = path ? kHasInter : kHasIntra, other = path ? kHasIntra : kHasInter;
+
+  for (int qt = 0; qt < p.NT; ++qt) {
+    const uint8_t c = cls[size_t(qt) * p.NT];
+    if (!(c & mine)) continue;
+    const int i0 = qt * kTile;
+    __syncthreads();
+    stage<D>(q_g, D, i0, p.T, cos_tab, sin_tab, sq);
+    stage<D>(dO, p.o_row, i0, p.T, nullptr, nullptr, sg);
+    if (threadIdx.x < kTile) {
+      const int i = i0 + threadIdx.x;
+      slse2[threadIdx.x] = i < p.T ? __ldg(p.lse + size_t(bh) * p.T + i) * kLog2e : INFINITY;  // p = exp2(-inf) = 0
+      sdelta[threadIdx.x] = i < p.T ? __ldg(p.delta + size_t(bh) * p.T + i) : 0.f;
+    }
+    uint32_t drop[2][2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int w = 0; w < 2; ++w) {
+        const uint32_t bits = c & other ? __ldg(mrow[h] + 2 * qt + w) : 0u;
+        drop[h][w] = dead[h] ? 0xffffffffu : c & other ? (path ? ~bits : bits) : 0u;
+      }
+    __syncthreads();
+    float vt[D / 8][4], kt[D / 8][4];
+    clear(vt);
+    clear(kt);
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      const uint32_t d0 = (drop[0][g / 2] >> (16 * (g % 2))) & 0xffffu, d1 = (drop[1][g / 2] >> (16 * (g % 2))) & 0xffffu;
+      if (__all_sync(0xffffffffu, (d0 & d1) == 0xffffu)) continue;
+      float s[2][4], dp[2][4];
+      dots<D>(s, ak, sq, g, lane);
+      dots<D>(dp, av, sg, g, lane);
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const float2 lse2 = *reinterpret_cast<const float2*>(slse2 + 16 * g + 8 * j + t2), delta = *reinterpret_cast<const float2*>(sdelta + 16 * g + 8 * j + t2);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          float w, ds;
+          grads<SQ>(s[j][e] * c2 - (e % 2 ? lse2.y : lse2.x), dp[j][e], e % 2 ? delta.y : delta.x, w, ds);
+          const bool no = ((e < 2 ? d0 : d1) >> (8 * j + t2 + e % 2)) & 1u;
+          s[j][e] = no ? 0.f : w;            // (w multiplies dO in dV: p for the softmax, sqrt(p) for the square-root softmax)
+          dp[j][e] = no ? 0.f : ds * p.scale;
+        }
+      }
+      axpy<D>(vt, s, sg, g, lane);
+      axpy<D>(kt, dp, sq, g, lane);
+    }
+    add(dv, vt);
+    add(dk, kt);
+  }
+  uint32_t bad = bad_rows(!finite(dk, 0) || !finite(dv, 0), !finite(dk, 1) || !finite(dv, 1));
+  write_rows<D>(dv, dv_g, j0 + 16 * warp, p.T, lane, 1.f, nullptr, nullptr);
+  write_rows<D>(dk, dk_g, j0 + 16 * warp, p.T, lane, 1.f, cos_tab, sin_tab);
+  __syncwarp();
+  for (; bad != 0; bad &= bad - 1) {
+    const int j = j0 + 16 * warp + __ffs(bad) - 1;
+    if (j >= p.T) break;
+    const float k = rotated<D>(k_g + size_t(j) * D, j, cos_tab, sin_tab, lane), v = rotated<D>(v_g + size_t(j) * D, j, nullptr, nullptr, lane);
+    float a = 0.f, av1 = 0.f;
+    const bool none = bit_of(p.kpad + size_t(b) * p.TW, j);
+#pragma unroll 1
+    for (int i = 0; i < p.T && !none; ++i) {
+      if (bit_of(p.bitsT + (size_t(b) * p.T + j) * p.TW, i) != path) continue;
+      const float q = rotated<D>(q_g + size_t(i) * D, i, cos_tab, sin_tab, lane), go = rotated<D>(dO + size_t(i) * p.o_row, i, nullptr, nullptr, lane);
+      float w, ds;
+      grads<SQ>(warp_sum(lane < D ? q * k : 0.f) * c2 - __ldg(p.lse + size_t(bh) * p.T + i) * kLog2e, warp_sum(lane < D ? go * v : 0.f), __ldg(p.delta + size_t(bh) * p.T + i), w, ds);
+      av1 = fmaf(w, go, av1);
+      a = fmaf(ds * p.scale, q, a);
+    }
+    write_row<D>(av1, dv_g, j, lane, 1.f, nullptr, nullptr);
+    write_row<D>(a, dk_g, j, lane, 1.f, cos_tab, sin_tab);
+  }
+}
+
+template <int D, bool SQ>
+cudaError_t fwd_t(const SimtParams& p, cudaStream_t s) {
+  constexpr auto kern = attn_fwd_f32_kernel<D, SQ>;
+  constexpr int bytes = 4 * Cfg<D>::kBuf * 2;
+  if (cudaError_t e = opt_in_smem<kern>(bytes); e != cudaSuccess) return e;
+  kern<<<dim3((p.T + kTile - 1) / kTile, p.B * p.H), kThreads, bytes, s>>>(p);
+  count_launches(1);
+  return cudaGetLastError();
+}
+template <int D, bool SQ>
+cudaError_t bwd_t(const SimtParams& p, cudaStream_t s) {
+  constexpr auto kq = attn_bwd_dq_f32_kernel<D, SQ>;
+  constexpr auto kkv = attn_bwd_dkv_f32_kernel<D, SQ>;
+  constexpr int q_bytes = 2 * Cfg<D>::kBuf * 2, kv_bytes = q_bytes + 2 * kTile * 4;
+  cudaError_t e = opt_in_smem<kq>(q_bytes);
+  if (e == cudaSuccess) e = opt_in_smem<kkv>(kv_bytes);
+  if (e != cudaSuccess) return e;
+  const dim3 grid((p.T + kTile - 1) / kTile, p.B * p.H, 2);
+  kq<<<grid, kThreads, q_bytes, s>>>(p);
+  kkv<<<grid, kThreads, kv_bytes, s>>>(p);
+  count_launches(2);
+  return cudaGetLastError();
+}
+
+}  // namespace
+
+cudaError_t launch_attn_fwd_f32(const SimtParams& p, int D, bool sq, cudaStream_t s) {
+  if (D == 16) return sq ? fwd_t<16, true>(p, s) : fwd_t<16, false>(p, s);
+  return sq ? fwd_t<32, true>(p, s) : fwd_t<32, false>(p, s);
+}
+cudaError_t launch_attn_bwd_f32(const SimtParams& p, int D, bool sq, cudaStream_t s) {
+  if (D == 16) return sq ? bwd_t<16, true>(p, s) : bwd_t<16, false>(p, s);
+  return sq ? bwd_t<32, true>(p, s) : bwd_t<32, false>(p, s);
+}
+
+}  // namespace mintb

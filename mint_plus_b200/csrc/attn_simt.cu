@@ -1,7 +1,7 @@
 // fp32 CUDA-core kernels for the combined-softmax multimer attention (forward, dQ, dK/dV).
 //
-// They serve the fp32 configuration (agreement with the PyTorch path to ~1e-6), and bf16 tensors where a caller asks for fp32
-// arithmetic.  Every result is produced in a fixed order: no atomics.
+// They serve fp32 tensors of head_dim 64 (attn_f32.cu has the others; agreement with the PyTorch path to ~1e-6), and bf16 tensors where
+// a caller asks for fp32 arithmetic.  Every result is produced in a fixed order: no atomics.
 //
 // Bound by the fp32 multiply-adds: 2 D per query, key in the forward pass, 7 D in the backward pass.  A block of 128 threads is
 // 8 row groups x 16 column lanes: a thread owns R rows (queries in forward and dQ, keys in dK/dV) and, of every tile of 64 along
@@ -13,7 +13,7 @@
 //
 // The backward kernels run per pathway (grid dimension): with the log-sum-exp known a pathway's gradients involve only its own
 // pairs, and one pathway's accumulators fit the registers.  Tiles are skipped or restricted to a pathway by the 64 x 64 class table.
-#include "common.cuh"
+#include "simt.cuh"
 
 namespace mintb {
 
@@ -22,21 +22,6 @@ constexpr int kLanes = 16;            // column lanes
 constexpr int kGroups = 8;            // row groups
 constexpr int kSimtTile = 64;         // columns per tile: four per lane, and the granularity of the class table
 static_assert(kSimtTile == kClassTile, "a tile is one entry of the class table");
-
-struct SimtParams {
-  const void *q_s, *k_s, *v_s, *q_c, *k_c, *v_c;
-  const uint32_t *bits, *bitsT, *kpad;
-  const uint8_t* cls;
-  const float *cos_tab, *sin_tab;
-  void* out;
-  float* lse;
-  const void* d_out;
-  void *dq_s, *dk_s, *dv_s, *dq_c, *dk_c, *dv_c;
-  float* delta;  // [B][H][T]
-  int B, H, T, TW, NT;
-  float scale;
-  size_t o_row, o_bh;   // element strides of out and d_out: between queries, between (batch, head) pairs
-};
 
 namespace {
 
@@ -558,8 +543,6 @@ static cudaError_t bwd_t(const AttnArgs& a) {
 #define MINTB_SIMT_DISPATCH(FN)                                                        \
   if (a.dtype == MINTB_F32) {                                                          \
     switch (a.D) {                                                                     \
-      case 16: MINTB_SIMT_CASE(FN, float, 16);                                         \
-      case 32: MINTB_SIMT_CASE(FN, float, 32);                                         \
       case 64: MINTB_SIMT_CASE(FN, float, 64);                                         \
     }                                                                                  \
   } else {                                                                             \
@@ -571,7 +554,16 @@ static cudaError_t bwd_t(const AttnArgs& a) {
   }                                                                                    \
   return cudaErrorInvalidValue;
 
-cudaError_t launch_attn_fwd_simt(const AttnArgs& a) { MINTB_SIMT_DISPATCH(fwd_t) }
-cudaError_t launch_attn_bwd_simt(const AttnArgs& a) { MINTB_SIMT_DISPATCH(bwd_t) }
+// fp32 tensors of head_dim 16 and 32 are served by attn_f32.cu, whatever the size
+static bool on_tensor_cores(const AttnArgs& a) { return a.dtype == MINTB_F32 && a.D != 64; }
+
+cudaError_t launch_attn_fwd_simt(const AttnArgs& a) {
+  if (on_tensor_cores(a)) return launch_attn_fwd_f32(make_params(a), a.D, a.sqrt_softmax, a.stream);
+  MINTB_SIMT_DISPATCH(fwd_t)
+}
+cudaError_t launch_attn_bwd_simt(const AttnArgs& a) {
+  if (on_tensor_cores(a)) return launch_attn_bwd_f32(make_params(a), a.D, a.sqrt_softmax, a.stream);
+  MINTB_SIMT_DISPATCH(bwd_t)
+}
 
 }  // namespace mintb

@@ -331,8 +331,10 @@ static long long tc_ns(int groups, int M, int N, int K, bool wide) {
 // Where the tensor cores win: M2048 K320 six weights of N320 63.4 -> 26.4 us, N320 16.9 -> 11.9, N1280 44.6 -> 22.5, K1280 N320
 // 58.2 -> 28.9; M5120 143 -> 50, 31 -> 18, 95 -> 37, 111 -> 47.  Few tiles or a short x leave them to the CUDA cores, whose time goes
 // with the multiply-adds (13.3 per ps) or the length of one sum: M700 N320 K320 8.8 us (10.6), M100 N320 K1280 14.9 (23.8),
-// M700 N320 K1280 24.7 (25.1).
+// M700 N320 K1280 24.7 (25.1).  Below a thousand rows a model's pass waits for the host, which the second launch costs 6 us (8M model,
+// B3 T112: 796 us, 871 with the products that would be faster here).
 bool sgemm_tc_wins(int groups, int M, int N, int K) {
+  if (M < 1024) return false;
   const long long work = static_cast<long long>(M) * N * K * groups / 13300, chain = static_cast<long long>(K) * 10;
   const long long wide = tc_ns(groups, M, N, K, true), narrow = tc_ns(groups, M, N, K, false), simt = 2300 + (work > chain ? work : chain);
   return 11 * (wide < narrow ? wide : narrow) < 10 * simt;

@@ -1,0 +1,27 @@
+// What the fp32 attention kernels (attn_simt.cu, attn_f32.cu) share.
+#pragma once
+
+#include "common.cuh"
+
+namespace mintb {
+
+struct SimtParams {
+  const void *q_s, *k_s, *v_s, *q_c, *k_c, *v_c;
+  const uint32_t *bits, *bitsT, *kpad;
+  const uint8_t* cls;
+  const float *cos_tab, *sin_tab;
+  void* out;
+  float* lse;
+  const void* d_out;
+  void *dq_s, *dk_s, *dv_s, *dq_c, *dk_c, *dv_c;
+  float* delta;  // [B][H][T]
+  int B, H, T, TW, NT;
+  float scale;
+  size_t o_row, o_bh;   // element strides of out and d_out: between queries, between (batch, head) pairs
+};
+
+// attn_f32.cu: fp32 tensors of head_dim 16 and 32
+cudaError_t launch_attn_fwd_f32(const SimtParams& p, int D, bool sqrt_softmax, cudaStream_t s);
+cudaError_t launch_attn_bwd_f32(const SimtParams& p, int D, bool sqrt_softmax, cudaStream_t s);
+
+}  // namespace mintb

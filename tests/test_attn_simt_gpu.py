@@ -31,3 +31,37 @@ def test_fp32_attention_tile_edges(T, D, sqrt_softmax):
     got = torch.autograd.grad(out, leaves, grad.cuda())
     for a, b in zip((out, *got), (want, *wg)):
         assert (a.detach().cpu() - b).norm() <= 4e-6 * b.norm() + 3e-6
+
+
+@pytest.mark.parametrize("D", [16, 32])
+def test_fp32_attention_values_without_bf16_pieces(D):
+    """Infinite values and values that round to infinity as bf16 act on the rows and keys that fp32 arithmetic lets them act on."""
+    B, H, T = 1, 2, 150
+    g = torch.Generator().manual_seed(D)
+    qs, ks, vs, qc, kc, vc, go = [torch.randn(B, H, T, D, generator=g) for _ in range(7)]
+    ids = (torch.arange(T) >= 70).long()[None]
+    x = O.chain_mask_from_ids(ids)[:, None]                   # cross pathway
+    vs[0, 0, 5, 3], vc[0, 0, 140, 2], vs[0, 1, 149, 0] = float("inf"), -float("inf"), 3.4e38
+    kc[0, 1, 20, 1] = 3.4e38                                  # logits of +-1e38: a row's only key, or none of its keys
+    qs[0, 1, 100, 4], ks[0, 1, 75, 4] = 3.4e38, 3.4e38        # their product overflows
+    go[0, 0, 80, 7] = float("inf")
+    s = torch.where(x, qc @ kc.transpose(-1, -2), qs @ ks.transpose(-1, -2)) * D ** -0.5      # fp32: overflows where the kernel's does
+    p = torch.softmax(s.double(), -1)
+    # a weight of zero takes an infinite value's row nowhere but to NaN, in its own pathway only
+    term = lambda w, v: (w[..., None] * v).sum(-2)
+    want = term(torch.where(x, 0.0, p), torch.where(x[..., None], 0.0, vs.double()[:, :, None])) + term(torch.where(x, p, 0.0), torch.where(x[..., None], vc.double()[:, :, None], 0.0))
+    leaves = [t.cuda().requires_grad_() for t in (qs, ks, vs, qc, kc, vc)]
+    out = M.multimer_attention(*leaves, chain_ids=ids.cuda(), rope=False)
+    got = out.detach().cpu()
+    want = want.float()
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
+    ok = want.isfinite()
+    torch.testing.assert_close(got[ok], want[ok], rtol=1e-5, atol=1e-5)
+    assert not ok.all() and ok.float().mean() > 0.5
+    dv = torch.autograd.grad(out, (leaves[2], leaves[5]), go.cuda())
+    for d, sel in zip(dv, (~x, x)):                           # dV reads the probabilities and dO alone
+        w = torch.where(sel, p, 0.0)
+        ref = term(w.transpose(-1, -2), torch.where(sel.transpose(-1, -2)[..., None], go.double()[:, :, None], 0.0)).float()
+        d = d.cpu()
+        assert torch.equal(d.isfinite(), ref.isfinite()) and not ref.isfinite().all()
+        torch.testing.assert_close(d[ref.isfinite()], ref[ref.isfinite()], rtol=1e-5, atol=1e-5)
