@@ -557,7 +557,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
 
     // rescale this thread's O accumulator by alpha (rare: the running maximum grew by more than the threshold)
     auto rescale_o = [&](float alpha) {
-#pragma unroll
+#pragma unroll 1
       for (int c0 = 0; c0 < D; c0 += 16) {
         uint32_t o[16];
         tmem_ld16(tO + c0, o);
@@ -739,8 +739,9 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
           const float inv = SQ ? rsqrtf(l_all) : 1.f / l_all;
           const float f_self = (SQ ? ex2(0.5f * (m_ref - m_all)) : w_self) * inv;
           const float f_other = (SQ ? ex2(0.5f * (m_other - m_all)) : w_other) * inv;
-          constexpr int CH = NC > 16 ? 16 : NC;   // columns per pass (keeps the register footprint small)
-#pragma unroll
+          // A short loop: code that runs once per item has to be fetched anew each time, at some 100 cycles for eight instructions.
+          constexpr int CH = 8;
+#pragma unroll 1
           for (int c0 = 0; c0 < NC; c0 += CH) {
             uint32_t oa[CH], ob[CH];
             tmem_ld_n<CH>(tO + ch * NC + c0, oa);                                                              // own accumulator

@@ -24,6 +24,7 @@ constexpr int kGEpiWarps = 8, kGEpiThreads = 32 * kGEpiWarps, kGThreads = 64 + k
 constexpr int kSlabBytes = 128;                       // bytes of K per stage and row (64 bf16 or 128 e4m3)
 constexpr int kABytes = kGM * kSlabBytes;
 constexpr int kGStageOutBytes = 32 * 64 + 32 * 32;   // one epilogue warp's staging: 32 rows x 32 bf16 columns, then 32 rows x 32 e4m3 columns, for bulk stores
+constexpr int kPrefetchRows = 8;   // row tiles up to which the weights are prefetched
 constexpr int kGTileRing = 4;   // tile numbers travel from the loading warp to the other roles through a ring this deep
 // A narrower tile needs less of the ring per slab and has less work to hide a slab's latency behind: more stages.
 template <int BN, bool PAIR>
@@ -148,6 +149,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   const int elems_per_slab = p.in_dtype == MINTB_E4M3 ? 128 : 64;
   const int n_slabs = (p.K + elems_per_slab - 1) / elems_per_slab;
 
+  // With few rows the weights come from HBM and are used once: they are on their way to L2 while the kernel before this one still runs.
+  // (A prefetch delivers nothing: what that kernel writes is read behind the wait below, weights included.)
+  if (warp == 0 && lane == 0 && tiles_m <= kPrefetchRows && int(blockIdx.x) < tiles_n * (PAIR ? 2 : 1)) {
+    const int n0 = int(blockIdx.x) / (PAIR ? 2 : 1) * kGN + rank * Cfg::kBRows;
+    for (int kb = 0; kb < n_slabs; ++kb) tma_prefetch_2d(&map_b, kb * elems_per_slab, n0);
+  }
   if (tid == 0) {
     for (int s = 0; s < kGStages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
     for (int s = 0; s < 2; ++s) { mbar_init(&acc_full[s], 1); mbar_init(&acc_empty[s], PAIR ? 2 * kGEpiWarps : kGEpiThreads); }
