@@ -70,6 +70,12 @@ int next_tile_counter(int** out) {
   return MINTB_OK;
 }
 
+void bind_context() {
+  static thread_local bool bound = false;
+  if (bound) return;
+  int dev = 0;
+  bound = cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess;
+}
 int current_device() {
   int dev = -1;
   return cudaGetDevice(&dev) == cudaSuccess ? dev : -1;

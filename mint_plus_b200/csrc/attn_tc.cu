@@ -38,6 +38,7 @@ static EncodeTiledFn encode_fn() {
     if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess) p = nullptr;
     return reinterpret_cast<EncodeTiledFn>(p);
   }();
+  bind_context();
   return fn;
 }
 

@@ -37,6 +37,7 @@ static EncodeTiledFn bwd_encode_fn() {
     if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess) p = nullptr;
     return reinterpret_cast<EncodeTiledFn>(p);
   }();
+  bind_context();
   return fn;
 }
 

@@ -136,6 +136,9 @@ inline cudaError_t opt_in_smem(int bytes) {
   return e;
 }
 int sm_count();         // of the current device
+// Makes the current device's context the calling thread's, which encoding a tensor map asks for and a thread's first runtime call does: a
+// backward pass may begin, on a thread of its own, with a product.
+void bind_context();
 void count_launches(int n);  // process-wide tally of kernels launched by this library
 
 // Work counters of the persistent kernels.  A launch takes the next {next unit, CTAs that have left} pair of a pool in the

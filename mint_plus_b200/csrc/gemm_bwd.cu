@@ -334,6 +334,160 @@ gemm_bwd_kernel(const __grid_constant__ CUtensorMap map_a1, const __grid_constan
   }
 }
 
+// ------------------------------------------------------------------------------------------------ weight gradients of a layer
+// Up to kGroup products dw = alpha dz^T x over the same tokens in one launch, each tile's reduction uncut, with the column sums of dz (the
+// bias gradients) as a further product of sixteen columns against ones.  For short batches, whose products are a few tiles each and whose
+// time is launches: five products and four passes of column sums of a layer of the 8M model (B4 T330) are one launch of 205 tiles.  64
+// columns a tile, since the tokens of a tile are short and the tiles few; alpha is not for the column sums.
+constexpr int kGroup = 6, kGroupBN = 64, kOnesCols = 16, kOnesBytes = 16 * 128;
+struct WgradGroup {
+  CUtensorMap a[kGroup], b[kGroup];
+  __nv_bfloat16 *dw[kGroup], *db[kGroup];   // db null: not wanted
+  int rows[kGroup], cols[kGroup], first[kGroup + 1];   // first: number of the product's first tile
+  float alpha[kGroup];
+  int n, red;
+  int* status;
+};
+
+__global__ void __launch_bounds__(kBThreads, 1) wgrad_group_kernel(const __grid_constant__ WgradGroup p) {
+  using Cfg = BwdGemmCfg<kGroupBN>;
+  constexpr int kStages = Cfg::kStages, kStageBytes = Cfg::kStageBytes, kAccCols = kGroupBN + kOnesCols;
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* smem = align_smem_1024(smem_raw);
+  unsigned char* ones = smem + size_t(kStages) * kStageBytes;      // 16 rows of 128 bytes, whatever the swizzle
+  uint64_t* full = reinterpret_cast<uint64_t*>(ones + kOnesBytes);
+  uint64_t* empty = full + kStages;
+  uint64_t* acc_full = empty + kStages;   // [2]
+  uint64_t* acc_empty = acc_full + 2;     // [2]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+  const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+  const int n_tiles = p.first[p.n], n_slabs = (p.red + 63) / 64;
+  if (tid == 0) {
+    for (int s = 0; s < kStages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+    for (int s = 0; s < 2; ++s) { mbar_init(&acc_full[s], 1); mbar_init(&acc_empty[s], kBEpiWarps); }
+    fence_mbar_init();
+  }
+  if (warp == 1) { tmem_alloc(tmem_slot, 256); tmem_relinquish(); }
+  for (int i = tid; i < kOnesBytes / 4; i += kBThreads) reinterpret_cast<uint32_t*>(ones)[i] = 0x3f803f80u;
+  fence_proxy_async_smem();
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  griddep_wait();
+  const uint32_t tbase = *tmem_slot;
+  struct Tile { int g, m0, n0; };
+  auto tile_at = [&](int t) {
+    Tile x{0, 0, 0};
+    while (t >= p.first[x.g + 1]) ++x.g;
+    const int tiles_n = (p.cols[x.g] + kGroupBN - 1) / kGroupBN, i = t - p.first[x.g];
+    x.m0 = i / tiles_n * kBM;
+    x.n0 = i % tiles_n * kGroupBN;
+    return x;
+  };
+
+  if (warp == 0) {
+    if (lane == 0) {
+      uint32_t stage = 0, phase = 0;
+      bool ok = true;
+      for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
+        const Tile x = tile_at(t);
+        for (int kb = 0; kb < n_slabs; ++kb) {
+          ok = mbar_wait(&empty[stage], phase ^ 1, p.status, 0x811);
+          if (!ok) break;
+          unsigned char* a = smem + size_t(stage) * kStageBytes;
+          mbar_expect_tx(&full[stage], kStageBytes);
+          for (int blk = 0; blk < kBM / 64; ++blk) tma_load_2d(a + blk * 64 * 128, &p.a[x.g], &full[stage], x.m0 + blk * 64, kb * 64);
+          tma_load_2d(a + kBABytes, &p.b[x.g], &full[stage], x.n0, kb * 64);
+          if (++stage == kStages) { stage = 0; phase ^= 1; }
+        }
+      }
+      griddep_launch();
+    }
+  } else if (warp == 1) {
+    const bool leader = elect_one();
+    auto wait_all = [&](uint64_t* bar, uint32_t parity, int code) -> bool {
+      return __all_sync(0xffffffffu, mbar_wait(bar, parity, p.status, code));
+    };
+    constexpr uint32_t kHi = desc_hi32(8 * 128, kSw128), kLbo = desc_lbo32(64 * 128), kStep = (16u * 128u) >> 4;
+    constexpr uint32_t idesc = idesc_bf16(kBM, kGroupBN, true, true), idesc_ones = idesc_bf16(kBM, kOnesCols, true, true);
+    const uint32_t lo0 = desc_addr32(__shfl_sync(0xffffffffu, smem_u32(smem), 0)) + kLbo;
+    const uint32_t ones_lo = desc_addr32(__shfl_sync(0xffffffffu, smem_u32(ones), 0)) + kLbo;
+    const uint32_t tb = __shfl_sync(0xffffffffu, tbase, 0);
+    uint32_t stage = 0, phase = 0, ab = 0, ab_phase = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
+      const Tile x = tile_at(t);
+      const bool sums = x.n0 == 0 && p.db[x.g] != nullptr;
+      ok = wait_all(&acc_empty[ab], ab_phase ^ 1, 0x812);
+      if (!ok) break;
+      tc_fence_after();
+      const uint32_t d = tb + ab * 128;
+      for (int kb = 0; kb < n_slabs; ++kb) {
+        ok = wait_all(&full[stage], phase, 0x813);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t a_lo = lo0 + stage * (kStageBytes >> 4), b_lo = a_lo + (kBABytes >> 4);
+        if (leader) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const uint64_t da = make_desc(kHi, a_lo + k * kStep);
+            umma_ss(d, da, make_desc(kHi, b_lo + k * kStep), idesc, kb > 0 || k > 0);
+            if (sums) umma_ss(d + kGroupBN, da, make_desc(kHi, ones_lo), idesc_ones, kb > 0 || k > 0);
+          }
+          umma_commit(&empty[stage]);
+        }
+        __syncwarp();
+        if (++stage == kStages) { stage = 0; phase ^= 1; }
+      }
+      if (!ok) break;
+      if (leader) umma_commit(&acc_full[ab]);
+      __syncwarp();
+      if (++ab == 2) { ab = 0; ab_phase ^= 1; }
+    }
+  } else {
+    const int quarter = warp % 4, chalf = (warp - 2) / 4;   // TMEM lanes and half of the tile's columns
+    uint32_t ab = 0, ab_phase = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; t < n_tiles; t += gridDim.x) {
+      const Tile x = tile_at(t);
+      ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[ab], ab_phase, p.status, 0x814));
+      if (!ok) break;
+      tc_fence_after();
+      const uint32_t tacc = tbase + (uint32_t(quarter * 32) << 16) + ab * 128;
+      const int row = x.m0 + quarter * 32 + lane, c0 = chalf * 32;
+      const float alpha = p.alpha[x.g];
+      uint32_t r[32], sum[4];
+      const bool sums = x.n0 == 0 && p.db[x.g] != nullptr && chalf == 0;
+      tmem_ld32(tacc + c0, r);
+      if (sums) tmem_ld4(tacc + kGroupBN, sum);
+      tmem_ld_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&acc_empty[ab]);
+      if (row < p.rows[x.g]) {   // (64 bytes of a row per lane: the results are small)
+        if (sums) p.db[x.g][row] = __float2bfloat16_rn(__uint_as_float(sum[0]));
+        const int cols = p.cols[x.g];
+        __nv_bfloat16* dst = p.dw[x.g] + size_t(row) * cols + x.n0 + c0;
+#pragma unroll
+        for (int j = 0; j < 32; j += 8)
+          if (x.n0 + c0 + j < cols)   // (columns come in multiples of eight)
+            *reinterpret_cast<uint4*>(dst + j) =
+                make_uint4(bwd_pack_bf16x2(__uint_as_float(r[j]) * alpha, __uint_as_float(r[j + 1]) * alpha),
+                           bwd_pack_bf16x2(__uint_as_float(r[j + 2]) * alpha, __uint_as_float(r[j + 3]) * alpha),
+                           bwd_pack_bf16x2(__uint_as_float(r[j + 4]) * alpha, __uint_as_float(r[j + 5]) * alpha),
+                           bwd_pack_bf16x2(__uint_as_float(r[j + 6]) * alpha, __uint_as_float(r[j + 7]) * alpha));
+      }
+      if (++ab == 2) { ab = 0; ab_phase ^= 1; }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    __syncwarp();
+    tmem_dealloc(tbase, 256);
+  }
+}
+
 // out[i] = bf16(acc[i]): the fp32 sum of the wgrad units as the bf16 gradient; 8 elements per thread.
 __global__ void __launch_bounds__(256) wgrad_convert_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ out, size_t n) {
   griddep_wait();
@@ -361,6 +515,7 @@ static EncodeTiledFn bwd_gemm_encode_fn() {
     if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess) p = nullptr;
     return reinterpret_cast<EncodeTiledFn>(p);
   }();
+  bind_context();
   return fn;
 }
 
@@ -608,5 +763,45 @@ extern "C" int mintb_linear_wgrad(const void* dz, const void* x, void* dw, void*
     count_launches(1);
     if (e != cudaSuccess) { set_error("wgrad convert launch: %s", cudaGetErrorString(e)); return MINTB_ECUDA; }
   }
+  return MINTB_OK;
+}
+
+// Worth one launch where every product would run uncut by itself.  8M model, B4 T330: a layer's nine launches of 93 us together, one of
+// 15 us; the training step's kernels 1490 -> 1100 us (with the attention's gains), the step, which waits for the host, 2460 -> 2295 us.
+extern "C" int mintb_linear_wgrad_group_wins(int n, int M, const int* N, const int* K) {
+  if (n < 2 || n > kGroup || M <= 0 || N == nullptr || K == nullptr) return 0;
+  for (int i = 0; i < n; ++i)
+    if (N[i] <= 0 || K[i] <= 0 || N[i] % 8 || K[i] % 8 || !plan_wgrad_way(M, N[i], K[i], false, MINTB_BF16).direct) return 0;
+  return 1;
+}
+
+extern "C" int mintb_linear_wgrad_group(const void* const* dz, const void* const* x, void* const* dw, void* const* db, const int* N, const int* K, const float* alpha,
+                                        int n, int M, void* stream, int* dev_status) {
+  bool ok = dz != nullptr && x != nullptr && dw != nullptr && db != nullptr && N != nullptr && K != nullptr && alpha != nullptr && n >= 1 && n <= kGroup && M > 0;
+  for (int i = 0; ok && i < n; ++i)
+    ok = dz[i] != nullptr && x[i] != nullptr && dw[i] != nullptr && N[i] > 0 && K[i] > 0 && N[i] % 8 == 0 && K[i] % 8 == 0 && bwd_aligned16(dz[i]) && bwd_aligned16(x[i]) &&
+         bwd_aligned16(dw[i]);
+  if (!ok) {
+    set_error("mintb_linear_wgrad_group: one to %d products of 16-byte aligned bf16 matrices, N and K multiples of eight, are required", kGroup);
+    return MINTB_EINVAL;
+  }
+  WgradGroup p{};
+  p.n = n; p.red = M; p.status = dev_status;
+  for (int i = 0; i < n; ++i) {
+    if (!operand_map(&p.a[i], dz[i], M, N[i], 2, 64) || !operand_map(&p.b[i], x[i], M, K[i], 2, 64)) {
+      set_error("mintb_linear_wgrad_group: cuTensorMapEncodeTiled failed");
+      return MINTB_ECUDA;
+    }
+    p.dw[i] = static_cast<__nv_bfloat16*>(dw[i]);
+    p.db[i] = static_cast<__nv_bfloat16*>(db[i]);
+    p.rows[i] = N[i]; p.cols[i] = K[i]; p.alpha[i] = alpha[i];
+    p.first[i + 1] = p.first[i] + (N[i] + kBM - 1) / kBM * ((K[i] + kGroupBN - 1) / kGroupBN);
+  }
+  constexpr size_t smem = BwdGemmCfg<kGroupBN>::kSmem + kOnesBytes;
+  cudaError_t e = opt_in_smem<wgrad_group_kernel>(int(smem));
+  const int sms = sm_count(), tiles = p.first[n];
+  if (e == cudaSuccess) e = launch_dependent(wgrad_group_kernel, dim3(unsigned(tiles < sms ? tiles : sms)), dim3(kBThreads), smem, static_cast<cudaStream_t>(stream), p);
+  count_launches(1);
+  if (e != cudaSuccess) { set_error("wgrad group launch: %s", cudaGetErrorString(e)); return MINTB_ECUDA; }
   return MINTB_OK;
 }

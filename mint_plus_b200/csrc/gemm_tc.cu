@@ -697,6 +697,7 @@ static EncodeTiledFn gemm_encode_fn() {
     if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess) p = nullptr;
     return reinterpret_cast<EncodeTiledFn>(p);
   }();
+  bind_context();
   return fn;
 }
 

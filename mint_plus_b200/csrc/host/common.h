@@ -118,6 +118,14 @@ Tensor quantize(const Tensor& x, double scale);
 // alpha (dz w + dz2 w2) + beta resid
 Tensor dgrad(const Tensor& dz, const Tensor& w, double alpha, const Tensor& dz2 = {}, const Tensor& w2 = {}, const Tensor& resid = {}, double beta = 0.0);
 Tensor wgrad(const Tensor& dz, const Tensor& x, double alpha, at::ScalarType out);
+// Weight gradients of several projections over the same tokens, formed by one launch: dw = alpha dz^T x, db (where wanted) the column
+// sums of dz, in bf16.
+struct WeightGrad {
+  Tensor dz, x, dw, db;
+  double alpha = 1.0;
+  bool want_db = false;
+};
+void wgrad_group(std::vector<WeightGrad>& items);
 // (dz, db): dz = dy gelu'(z) (dy itself without z) in bf16, db its column sums in the given type (none: not wanted)
 std::pair<Tensor, Tensor> gelu_colsum(const Tensor& dy, const Tensor& z, std::optional<at::ScalarType> db_dt);
 // (dz in e5m2, db)

@@ -147,6 +147,27 @@ Tensor wgrad(const Tensor& dz, const Tensor& x, double alpha, at::ScalarType out
   return dw;
 }
 
+void wgrad_group(std::vector<WeightGrad>& items) {
+  if (items.empty()) return;
+  Env e(items[0].dz);
+  constexpr size_t kMost = 6;
+  TORCH_CHECK(items.size() <= kMost, "wgrad_group: at most six products");
+  const void *dz[kMost], *x[kMost];
+  void *dw[kMost], *db[kMost];
+  int N[kMost], K[kMost];
+  float alpha[kMost];
+  for (size_t i = 0; i < items.size(); ++i) {
+    WeightGrad& w = items[i];
+    TORCH_CHECK(w.dz.scalar_type() == at::kBFloat16 && w.x.scalar_type() == at::kBFloat16 && w.dz.size(0) == items[0].dz.size(0), "wgrad_group: bf16 rows of the same tokens");
+    N[i] = int(w.dz.size(1));
+    K[i] = int(w.x.size(1));
+    w.dw = e.empty({N[i], K[i]}, at::kBFloat16);
+    if (w.want_db) w.db = e.empty({N[i]}, at::kBFloat16);
+    dz[i] = ptr(w.dz); x[i] = ptr(w.x); dw[i] = ptr(w.dw); db[i] = ptr(w.db); alpha[i] = float(w.alpha);
+  }
+  check(mintb_linear_wgrad_group(dz, x, dw, db, N, K, alpha, int(items.size()), int(items[0].dz.size(0)), e.stream, e.status), "mintb_linear_wgrad_group");
+}
+
 static std::pair<Tensor, Tensor> bias_pass(const Tensor& dy, const Tensor& z, std::optional<at::ScalarType> db_dt, double f8_scale) {
   Env e(dy);
   const int64_t M = dy.size(0), N = dy.size(1);

@@ -327,6 +327,40 @@ variable_list LayerNode::apply(variable_list&& grads) {
   auto a_in = [&](const Operand& o) { return fp8 ? o.grad_scale * o.w_scale * o.out_scale : 1.0; };
   auto a_w = [&](const Operand& o) { return fp8 ? o.grad_scale * o.x_scale * o.out_scale : 1.0; };
 
+  // The weight gradients of a short batch are formed together at the end, with the bias gradients that go with them.
+  struct Later { int64_t kw, nw, kb, nb; double db_factor; };
+  std::vector<WeightGrad> group;
+  std::vector<Later> later;
+  bool grouped = false;
+  if (!fp8 && plan.lora_r == 0) {
+    const int64_t F = s[kA].size(1);
+    int N[5], K[5], n = 0;
+    bool bf16 = true;
+    auto count = [&](int64_t k, int64_t m, int64_t rows, int64_t cols) {
+      if (!any(k, m)) return;
+      bf16 = bf16 && plan.params[k].scalar_type() == at::kBFloat16;
+      N[n] = int(rows);
+      K[n++] = int(cols);
+    };
+    count(at.w2, 1, E, F);
+    count(at.w1, 1, F, E);
+    count(at.wo, 1, E, E);
+    count(at.ws, plan.n_self, 3 * E, E);
+    count(at.wc, plan.n_cross, 3 * E, E);
+    grouped = bf16 && x.size(0) <= INT32_MAX && mintb_linear_wgrad_group_wins(n, int(x.size(0)), N, K) != 0;
+  }
+  // Whether the bias gradient of a projection comes with its weight gradient; and one projection's weight gradient.
+  auto with_w = [&](int64_t kw, int64_t nw, int64_t kb, int64_t nb) { return grouped && any(kw, nw) && any(kb, nb) && plan.params[kb].scalar_type() == at::kBFloat16; };
+  auto weight_grad = [&](int64_t kw, int64_t nw, int64_t kb, int64_t nb, const Tensor& g, const Tensor& in, double alpha, double db_factor = 1.0) {
+    if (!any(kw, nw)) return;
+    if (!grouped) return give_rows(kw, nw, wgrad(g, in, alpha, w_dt(kw)));
+    WeightGrad w;
+    w.dz = g; w.x = in; w.alpha = alpha; w.want_db = with_w(kw, nw, kb, nb);
+    group.push_back(w);
+    later.push_back({kw, nw, kb, nb, db_factor});
+  };
+  auto bias_dt_apart = [&](int64_t kw, int64_t nw, int64_t kb, int64_t nb) { return with_w(kw, nw, kb, nb) ? std::nullopt : bias_dt(kb, nb); };
+
   Tensor d_ffn = gy, d1;   // gradients of the FFN's result and of the first residual sum
   if (mu) {
     NormGrad g = add_layernorm_bwd(gy, Tensor(), s[kX1], s[kY2], plan.keep, plan.add, g2v, s[kStats2], p2);
@@ -335,13 +369,13 @@ variable_list LayerNode::apply(variable_list&& grads) {
     d_ffn = g.dr;
   }
   {
-    auto [g2, db2] = operand(plan.fc2, d_ffn, Tensor(), bias_dt(at.b2));
+    auto [g2, db2] = operand(plan.fc2, d_ffn, Tensor(), bias_dt_apart(at.w2, 1, at.b2, 1));
     give(at.b2, db2);
-    if (wants(at.w2)) give(at.w2, wgrad(g2, s[kA], a_w(plan.fc2), w_dt(at.w2)));
+    weight_grad(at.w2, 1, at.b2, 1, g2, s[kA], a_w(plan.fc2));
     Tensor da = dgrad(g2, plan.fc2.w, a_in(plan.fc2));
-    auto [g1, db1] = operand(plan.fc1, da, s[kZ], bias_dt(at.b1));
+    auto [g1, db1] = operand(plan.fc1, da, s[kZ], bias_dt_apart(at.w1, 1, at.b1, 1));
     give(at.b1, db1);
-    if (wants(at.w1)) give(at.w1, wgrad(g1, s[kH2], a_w(plan.fc1), w_dt(at.w1)));
+    weight_grad(at.w1, 1, at.b1, 1, g1, s[kH2], a_w(plan.fc1));
     if (mu) {
       d1 = dgrad(g1, plan.fc1.w, a_in(plan.fc1), Tensor(), Tensor(), d1, 1.0);   // both ways into the first residual sum
     } else {
@@ -364,9 +398,9 @@ variable_list LayerNode::apply(variable_list&& grads) {
   // output projection: its result entered the sum times `add`
   Tensor d_attn;
   {
-    auto [go, dbo] = operand(w_out, d1, Tensor(), bias_dt(at.bo));
+    auto [go, dbo] = operand(w_out, d1, Tensor(), bias_dt_apart(at.wo, 1, at.bo, 1));
     if (dbo.defined()) give(at.bo, plan.add == 1.0 ? dbo : dbo * plan.add);
-    if (wants(at.wo)) give(at.wo, wgrad(go, s[kO], a_w(w_out) * plan.add, w_dt(at.wo)));
+    weight_grad(at.wo, 1, at.bo, 1, go, s[kO], a_w(w_out) * plan.add, plan.add);
     if (lora_out) {   // dB = s g^T (x A^T), dA = s (g B)^T x
       Product xa;
       xa.x = s[kO];
@@ -389,12 +423,17 @@ variable_list LayerNode::apply(variable_list&& grads) {
   // take scales that give them one multiplier
   if (fp8) settle(os, [&] { return std::max(amax(g[0]), amax(g[1]) / ((os.w_scale * os.out_scale) / (oc.w_scale * oc.out_scale))); });
   if (fp8) oc.grad_scale = os.grad_scale * (os.w_scale * os.out_scale) / (oc.w_scale * oc.out_scale);
-  auto [gs, dbs] = operand(os, g[0], Tensor(), bias_dt(at.bs, plan.n_self));
-  auto [gc, dbc] = operand(oc, g[1], Tensor(), bias_dt(at.bc, plan.n_cross));
+  auto [gs, dbs] = operand(os, g[0], Tensor(), bias_dt_apart(at.ws, plan.n_self, at.bs, plan.n_self));
+  auto [gc, dbc] = operand(oc, g[1], Tensor(), bias_dt_apart(at.wc, plan.n_cross, at.bc, plan.n_cross));
   give_rows(at.bs, plan.n_self, dbs);
   give_rows(at.bc, plan.n_cross, dbc);
-  if (any(at.ws, plan.n_self)) give_rows(at.ws, plan.n_self, wgrad(gs, s[kXq], a_w(os), w_dt(at.ws)));
-  if (any(at.wc, plan.n_cross)) give_rows(at.wc, plan.n_cross, wgrad(gc, s[kXq], a_w(oc), w_dt(at.wc)));
+  weight_grad(at.ws, plan.n_self, at.bs, plan.n_self, gs, s[kXq], a_w(os));
+  weight_grad(at.wc, plan.n_cross, at.bc, plan.n_cross, gc, s[kXq], a_w(oc));
+  wgrad_group(group);
+  for (size_t i = 0; i < group.size(); ++i) {
+    give_rows(later[i].kw, later[i].nw, group[i].dw);
+    if (group[i].db.defined()) give_rows(later[i].kb, later[i].nb, later[i].db_factor == 1.0 ? group[i].db : group[i].db * later[i].db_factor);
+  }
   if (lora_qkv) {
     const Tensor& h = s[kXq];
     const int64_t n = 7 * r;   // columns of the shared products (those of `out` come out as zero and are not used)

@@ -104,6 +104,7 @@ bool piece_map(CUtensorMap* m, const void* ptr, int K, int Kp, size_t rows, int 
     return reinterpret_cast<EncodeTiledFn>(p);
   }();
   if (fn == nullptr) return false;
+  bind_context();
   cuuint64_t dims[3] = {cuuint64_t(K), cuuint64_t(rows), 3}, strides[2] = {cuuint64_t(Kp) * 2, cuuint64_t(rows) * Kp * 2};
   cuuint32_t box[3] = {kBK, cuuint32_t(box_rows), 1}, es[3] = {1, 1, 1};
   return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,

@@ -98,3 +98,47 @@ def test_backward_gemms_reject_bad_arguments():
         ops.gemm_dgrad(a, torch.zeros(24, 12, dtype=torch.bfloat16, device=DEV))            # K * 2 not a 16-byte multiple
     with pytest.raises((TypeError, NotImplementedError)):
         ops.gemm_dgrad(a, torch.zeros(24, 16, dtype=torch.float8_e4m3fn, device=DEV))       # mixed bf16 / 8-bit
+
+
+@pytest.mark.parametrize("M,shapes", [(1, [(8, 8), (64, 72)]), (64, [(128, 64), (136, 8)]), (330, [(960, 320), (320, 1280), (1280, 320), (320, 320), (960, 320), (24, 136)]),
+                                      (1987, [(320, 320), (256, 128)])])
+def test_wgrad_group(M, shapes):
+    """Weight gradients of several projections and their bias gradients in one launch, at the edges of the 128 x 64 tiles and of the slabs
+    of 64 tokens, more tiles than CTAs: the weight gradients are those of the single products, the column sums those of fp32 sums."""
+    import ctypes
+    from mint_plus_b200 import _lib as L
+    g = torch.Generator().manual_seed(M)
+    n = len(shapes)
+    dz = [_rand((M, a), g).to(DEV) for a, _ in shapes]
+    x = [_rand((M, b), g).to(DEV) for _, b in shapes]
+    dw = [torch.full(s, 7.0, device=DEV, dtype=torch.bfloat16) for s in shapes]
+    db = [torch.full((a,), 7.0, device=DEV, dtype=torch.bfloat16) if i != 1 else None for i, (a, _) in enumerate(shapes)]
+    alpha = [0.5 + i for i in range(n)]
+    arr = lambda ts: (ctypes.c_void_p * n)(*[None if t is None else t.data_ptr() for t in ts])
+    ints = lambda k: (ctypes.c_int * n)(*[s[k] for s in shapes])
+    rc = L.lib().mintb_linear_wgrad_group(arr(dz), arr(x), arr(dw), arr(db), ints(0), ints(1), (ctypes.c_float * n)(*alpha), n, M,
+                                          torch.cuda.current_stream().cuda_stream, None)
+    assert rc == 0, L.lib().mintb_last_error()
+    for i in range(n):
+        single = ops.gemm_wgrad(dz[i], x[i], alpha=alpha[i])
+        want = alpha[i] * (dz[i].double().t() @ x[i].double())
+        # bf16 results of fp32 sums: half a bf16 step, and the sums' own roundings where terms cancel
+        tol = 2.0 ** -8 * want.abs() + M * 2.0 ** -23 * want.abs().max()
+        assert ((dw[i].double() - want).abs() <= tol).all() and ((single.double() - want).abs() <= tol + 1e-3 * want.abs().max()).all()
+        if db[i] is not None:
+            sums = dz[i].double().sum(0)
+            assert ((db[i].double() - sums).abs() <= 2.0 ** -8 * sums.abs() + M * 2.0 ** -23 * dz[i].double().abs().sum(0)).all()
+
+
+def test_a_thread_may_begin_with_a_product():
+    """The first CUDA call of a thread is an encoded tensor map: its context has to be current by then."""
+    import threading
+    g = torch.Generator().manual_seed(3)
+    dz, w = _rand((64, 64), g).to(DEV), _rand((64, 128), g).to(DEV)
+    want = ops.gemm_dgrad(dz, w)
+    torch.empty_like(want)       # (leaves a block for the thread's result in the allocator's cache)
+    got = []
+    t = threading.Thread(target=lambda: got.append(ops.gemm_dgrad(dz, w)))
+    t.start()
+    t.join()
+    assert torch.equal(got[0], want)
