@@ -121,6 +121,13 @@ MINTB_API int mintb_attn_fwd(const void* q_self, const void* k_self, const void*
                    const float* rope_sin, void* out, float* lse, void* workspace, size_t workspace_bytes, int B,
                    int H, int T, int D, int dtype, unsigned flags, float scale, void* stream, int* dev_status);
 
+/* mintb_mask_meta_from_chain_ids (`ids64`: 64-bit ids) into `meta`, then mintb_attn_fwd on it; with in-kernel RoPE on the bf16 kernels the
+ * metadata and the rotated copies are formed by one launch. */
+MINTB_API int mintb_attn_fwd_ids(const void* chain_ids, int ids64, const uint8_t* key_pad, void* meta, const void* q_self, const void* k_self,
+                                 const void* v_self, const void* q_cross, const void* k_cross, const void* v_cross, const float* rope_cos,
+                                 const float* rope_sin, void* out, float* lse, void* workspace, size_t workspace_bytes, int B, int H, int T,
+                                 int D, int dtype, unsigned flags, float scale, void* stream, int* dev_status);
+
 /* No-allocation forward.  It has no counterpart in the reference.  Some callers of this library cannot allocate device
  * memory at the point where they call it: code that runs while a CUDA graph is being captured, real-time or
  * fixed-memory-budget hosts that forbid cudaMalloc after start-up, and host languages whose bindings hand over

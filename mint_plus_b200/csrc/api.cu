@@ -301,6 +301,31 @@ int mintb_attn_fwd(const void* q_self, const void* k_self, const void* v_self, c
   return e == cudaSuccess ? MINTB_OK : cuda_fail(e, "attention forward launch");
 }
 
+int mintb_attn_fwd_ids(const void* chain_ids, int ids64, const uint8_t* key_pad, void* meta, const void* q_self, const void* k_self, const void* v_self,
+                       const void* q_cross, const void* k_cross, const void* v_cross, const float* rope_cos, const float* rope_sin, void* out, float* lse,
+                       void* workspace, size_t workspace_bytes, int B, int H, int T, int D, int dtype, unsigned flags, float scale, void* stream, int* dev_status) {
+  const bool together = check_shape(B, H, T, D, dtype, "mintb_attn_fwd_ids") == MINTB_OK && use_tc(D, dtype, flags) && (flags & MINTB_FLAG_ROPE) &&
+                        !(flags & MINTB_FLAG_QK_PREROTATED) && chain_ids != nullptr;
+  if (!together) {
+    if (int rc = meta_from_chain_ids(chain_ids, ids64 != 0, key_pad, meta, B, T, stream); rc != MINTB_OK) return rc;
+    return mintb_attn_fwd(q_self, k_self, v_self, q_cross, k_cross, v_cross, meta, rope_cos, rope_sin, out, lse, workspace, workspace_bytes, B, H, T, D, dtype, flags, scale,
+                          stream, dev_status);
+  }
+  AttnArgs a{};
+  const size_t need = mintb_attn_fwd_workspace_bytes(B, H, T, D, dtype, flags);
+  int rc = fill_common(a, "mintb_attn_fwd_ids", q_self, k_self, v_self, q_cross, k_cross, v_cross, meta, rope_cos, rope_sin, workspace, workspace_bytes, need, B, H, T, D, dtype,
+                       flags, scale, stream, dev_status);
+  if (rc != MINTB_OK) return rc;
+  if (out == nullptr || lse == nullptr || !aligned(out, 16)) {
+    set_error("mintb_attn_fwd_ids: out (16-byte aligned) and lse are required");
+    return MINTB_EINVAL;
+  }
+  a.out = out;
+  a.lse = lse;
+  a.chain_ids = chain_ids; a.ids64 = ids64 != 0; a.key_pad = key_pad; a.meta_buf = meta;
+  return launch_attn_fwd_tc(a);
+}
+
 int mintb_attn_bwd_rows(const void* q_self, const void* k_self, const void* v_self, const void* q_cross,
                         const void* k_cross, const void* v_cross, const void* meta, const float* rope_cos,
                         const float* rope_sin, const void* out, const float* lse, const void* d_out, void* dq_self,

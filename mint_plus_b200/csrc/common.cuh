@@ -85,6 +85,10 @@ struct AttnArgs {
   float scale;
   cudaStream_t stream;
   int* dev_status;
+  const void* chain_ids;             // forward: the mask metadata is still to be formed from these (null: it is there) ...
+  bool ids64;
+  const uint8_t* key_pad;
+  void* meta_buf;                    // ... here
 };
 
 // element strides of out / d_out: row (query) stride and (batch, head) stride
@@ -163,6 +167,7 @@ cudaError_t launch_meta_from_chain_ids(const void* chain_ids, bool ids64, const 
                                        cudaStream_t s);
 cudaError_t launch_meta_from_mask(const uint8_t* mask, const uint8_t* key_pad, void* meta, int B, int T,
                                   cudaStream_t s);
+cudaError_t launch_prepare(const AttnArgs& a, __nv_bfloat16* qr, __nv_bfloat16* kr);   // metadata and the rotated Q_self, K_self
 cudaError_t launch_rope_tables(const float* inv_freq, float* cos_tab, float* sin_tab, int T, int D, cudaStream_t s);
 
 // attn_simt.cu — fp32 CUDA-core kernels (any dtype in, fp32 arithmetic)

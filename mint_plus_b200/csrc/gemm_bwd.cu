@@ -351,7 +351,7 @@ struct WgradGroup {
 
 __global__ void __launch_bounds__(kBThreads, 1) wgrad_group_kernel(const __grid_constant__ WgradGroup p) {
   using Cfg = BwdGemmCfg<kGroupBN>;
-  constexpr int kStages = Cfg::kStages, kStageBytes = Cfg::kStageBytes, kAccCols = kGroupBN + kOnesCols;
+  constexpr int kStages = Cfg::kStages, kStageBytes = Cfg::kStageBytes;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = align_smem_1024(smem_raw);
   unsigned char* ones = smem + size_t(kStages) * kStageBytes;      // 16 rows of 128 bytes, whatever the swizzle

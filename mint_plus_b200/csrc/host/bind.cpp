@@ -46,6 +46,12 @@ PYBIND11_MODULE(_mintb_host, m) {
         [](const Tensor& q0, const Tensor& q1, const Tensor& q2, const Tensor& q3, const Tensor& q4, const Tensor& q5, const Tensor& meta, const OptTensor& cos,
            const OptTensor& sin, double scale, int64_t flags) { return attention({q0, q1, q2, q3, q4, q5}, meta, cos, sin, scale, flags); },
         nogil);
+  m.def("attention_ids",
+        [](const Tensor& q0, const Tensor& q1, const Tensor& q2, const Tensor& q3, const Tensor& q4, const Tensor& q5, const Tensor& chain_ids, const OptTensor& key_pad,
+           const OptTensor& cos, const OptTensor& sin, double scale, int64_t flags) {
+          return attention({q0, q1, q2, q3, q4, q5}, Tensor(), cos, sin, scale, flags, chain_ids, key_pad);
+        },
+        nogil);
   m.def("mask_meta", &mask_meta, nogil);
   m.def("combine", &combine, nogil);
   m.def("linear", &linear, nogil);

@@ -93,6 +93,7 @@ struct AttnInputs {   // (B,H,T,D) projections and what goes with them
   Tensor meta, cos, sin;
   double scale;
   unsigned flags;
+  Tensor ids, pad;    // forward: `meta` is still to be filled from these chain ids and this key padding (bytes)
 };
 struct AttnResult {
   Tensor out, lse;

@@ -40,9 +40,15 @@ AttnResult attn_fwd(const AttnInputs& a, bool for_backward) {
   const bool keep = for_backward && (a.flags & MINTB_FLAG_ROPE) && !(a.flags & MINTB_FLAG_QK_PREROTATED);
   if (keep) bytes = std::max(bytes, mintb_attn_bwd_workspace_bytes(B, H, T, D, dt, a.flags));
   Tensor ws = e.bytes(bytes);
-  check(mintb_attn_fwd(ptr(a.q[0]), ptr(a.q[1]), ptr(a.q[2]), ptr(a.q[3]), ptr(a.q[4]), ptr(a.q[5]), ptr(a.meta), fptr(a.cos), fptr(a.sin), ptr(r.out),
-                       fptr(r.lse), ptr(ws), bytes, B, H, T, D, dt, a.flags, float(a.scale), e.stream, e.status),
-        "mintb_attn_fwd");
+  if (a.ids.defined())
+    check(mintb_attn_fwd_ids(ptr(a.ids), a.ids.scalar_type() == at::kLong, static_cast<uint8_t*>(ptr(a.pad)), ptr(a.meta), ptr(a.q[0]), ptr(a.q[1]), ptr(a.q[2]),
+                             ptr(a.q[3]), ptr(a.q[4]), ptr(a.q[5]), fptr(a.cos), fptr(a.sin), ptr(r.out), fptr(r.lse), ptr(ws), bytes, B, H, T, D, dt, a.flags,
+                             float(a.scale), e.stream, e.status),
+          "mintb_attn_fwd");
+  else
+    check(mintb_attn_fwd(ptr(a.q[0]), ptr(a.q[1]), ptr(a.q[2]), ptr(a.q[3]), ptr(a.q[4]), ptr(a.q[5]), ptr(a.meta), fptr(a.cos), fptr(a.sin), ptr(r.out),
+                         fptr(r.lse), ptr(ws), bytes, B, H, T, D, dt, a.flags, float(a.scale), e.stream, e.status),
+          "mintb_attn_fwd");
   if (keep) r.ws = ws;
   return r;
 }

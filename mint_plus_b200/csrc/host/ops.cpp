@@ -72,11 +72,11 @@ struct AttentionNode : public torch::autograd::Node {
   std::string name() const override { return "MultimerAttentionBackward"; }
 };
 
-Tensor mask_meta(const Tensor& chain_ids, const OptTensor& key_pad) {
+// Chain ids and key padding as the metadata kernels read them.
+static std::pair<Tensor, Tensor> mask_inputs(const Tensor& chain_ids, const OptTensor& key_pad) {
   at::NoGradGuard no_grad;
   TORCH_CHECK(chain_ids.is_cuda(), "mint_plus_b200 operators run on CUDA tensors only (no CPU fallback)");
   TORCH_CHECK_VALUE(chain_ids.dim() == 2, "chain_ids must be (B, T)");
-  const int64_t B = chain_ids.size(0), T = chain_ids.size(1);
   Tensor ids = chain_ids.scalar_type() == at::kLong || chain_ids.scalar_type() == at::kInt ? chain_ids.contiguous() : chain_ids.to(at::kInt).contiguous();
   Tensor pad = opt(key_pad);
   if (pad.defined()) {
@@ -85,6 +85,13 @@ Tensor mask_meta(const Tensor& chain_ids, const OptTensor& key_pad) {
     pad = pad.contiguous();
     pad = pad.scalar_type() == at::kBool ? pad.view(at::kByte) : pad.to(at::kByte);
   }
+  return {ids, pad};
+}
+
+Tensor mask_meta(const Tensor& chain_ids, const OptTensor& key_pad) {
+  at::NoGradGuard no_grad;
+  auto [ids, pad] = mask_inputs(chain_ids, key_pad);
+  const int64_t B = ids.size(0), T = ids.size(1);
   Env e(ids);
   Tensor buf = e.bytes(mintb_mask_meta_bytes(B, T));
   if (ids.scalar_type() == at::kLong)
@@ -94,7 +101,8 @@ Tensor mask_meta(const Tensor& chain_ids, const OptTensor& key_pad) {
   return buf;
 }
 
-Tensor attention(std::array<Tensor, 6> qkv, const Tensor& meta, const OptTensor& cos, const OptTensor& sin, double scale, int64_t flags) {
+Tensor attention(std::array<Tensor, 6> qkv, const Tensor& meta, const OptTensor& cos, const OptTensor& sin, double scale, int64_t flags, const OptTensor& chain_ids,
+                 const OptTensor& key_pad) {
   for (const Tensor& t : qkv) TORCH_CHECK(t.is_cuda(), "mint_plus_b200 operators run on CUDA tensors only (no CPU fallback)");
   for (const Tensor& t : qkv)
     TORCH_CHECK_VALUE(t.dim() == 4 && t.sizes() == qkv[0].sizes(), "q/k/v of both pathways must share one (B, H, T, D) shape");
@@ -105,6 +113,10 @@ Tensor attention(std::array<Tensor, 6> qkv, const Tensor& meta, const OptTensor&
   std::vector<Tensor> in(6);
   for (int k = 0; k < 6; ++k) a.q[k] = in[k] = qkv[k].contiguous();
   a.meta = meta; a.cos = opt(cos); a.sin = opt(sin); a.scale = scale; a.flags = unsigned(flags);
+  if (chain_ids.has_value()) {   // (of the batch of q, on its device: the caller has looked)
+    std::tie(a.ids, a.pad) = mask_inputs(*chain_ids, key_pad);
+    a.meta = Env(a.ids).bytes(mintb_mask_meta_bytes(int(a.ids.size(0)), int(a.ids.size(1))));
+  }
   auto node = make_node<AttentionNode>(in);
   AttnResult r = attn_fwd(a, node != nullptr);
   if (node) {
@@ -112,7 +124,7 @@ Tensor attention(std::array<Tensor, 6> qkv, const Tensor& meta, const OptTensor&
     for (int k = 0; k < 6; ++k) node->q[k] = SavedVariable(a.q[k], false);
     node->out = SavedVariable(r.out, true);
     node->lse = SavedVariable(r.lse, false); node->ws = SavedVariable(r.ws, false);
-    node->meta = meta; node->cos = a.cos; node->sin = a.sin;
+    node->meta = a.meta; node->cos = a.cos; node->sin = a.sin;
     node->scale = scale; node->flags = a.flags;
   }
   return r.out;

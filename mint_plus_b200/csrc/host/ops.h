@@ -17,7 +17,9 @@ std::array<Tensor, 6> attn_bwd(const AttnInputs& a, const Tensor& out, const Ten
 
 // Metadata blob of a (B,T) batch from chain ids and (optionally) padded keys.
 Tensor mask_meta(const Tensor& chain_ids, const OptTensor& key_pad);
-Tensor attention(std::array<Tensor, 6> qkv, const Tensor& meta, const OptTensor& cos, const OptTensor& sin, double scale, int64_t flags);
+// (with chain_ids the metadata is formed here and `meta` is not read)
+Tensor attention(std::array<Tensor, 6> qkv, const Tensor& meta, const OptTensor& cos, const OptTensor& sin, double scale, int64_t flags, const OptTensor& chain_ids = {},
+                 const OptTensor& key_pad = {});
 Tensor combine(const Tensor& il, const Tensor& el, const Tensor& mask_u8, const Tensor& iv, const Tensor& ev);
 Tensor linear(const Tensor& x, const Tensor& w, const OptTensor& bias, bool gelu);
 std::tuple<OptTensor, OptTensor, OptTensor> add_layernorm(const Tensor& x, const OptTensor& r, double a, double b, const OptTensor& gamma, const OptTensor& beta,

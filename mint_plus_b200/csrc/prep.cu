@@ -1,5 +1,6 @@
 // Mask metadata and RoPE tables: small memory-bound kernels run once per batch.
-#include "common.cuh"
+#include "ptx.cuh"
+#include "rope.cuh"
 
 namespace mintb {
 
@@ -9,11 +10,10 @@ namespace mintb {
 // copies of the bits (B16 T2048: 34 MB, 245 us with 32 compares per thread and word, three launches and two casts before; 12 us).
 // The relation is symmetric, so the key-major copy (bitsT) holds the same words.
 template <typename Id>
-__global__ void __launch_bounds__(256) meta_from_chain_ids_kernel(const Id* __restrict__ chain_ids, const uint8_t* __restrict__ key_pad,
-                                                                  uint32_t* __restrict__ bits, uint32_t* __restrict__ bitsT, uint32_t* __restrict__ kpad,
-                                                                  uint8_t* __restrict__ cls, int T, int TW, int NT) {
+__device__ __forceinline__ void meta_rows(int b, int qt, const Id* __restrict__ chain_ids, const uint8_t* __restrict__ key_pad, uint32_t* __restrict__ bits,
+                                          uint32_t* __restrict__ bitsT, uint32_t* __restrict__ kpad, uint8_t* __restrict__ cls, int T, int TW, int NT) {
   __shared__ uint32_t s_seen[2][32];   // of the word group: keys that some row of the tile meets in its own / in another chain
-  const int b = blockIdx.x, qt = blockIdx.y, warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   chain_ids += size_t(b) * T;
   for (int w0 = 0; w0 < TW; w0 += 32) {
     const int nw = min(32, TW - w0);
@@ -64,6 +64,28 @@ __global__ void __launch_bounds__(256) meta_from_chain_ids_kernel(const Id* __re
     }
     __syncthreads();
   }
+}
+
+template <typename Id>
+__global__ void __launch_bounds__(256) meta_from_chain_ids_kernel(const Id* __restrict__ chain_ids, const uint8_t* __restrict__ key_pad,
+                                                                  uint32_t* __restrict__ bits, uint32_t* __restrict__ bitsT, uint32_t* __restrict__ kpad,
+                                                                  uint8_t* __restrict__ cls, int T, int TW, int NT) {
+  meta_rows(blockIdx.x, blockIdx.y, chain_ids, key_pad, bits, bitsT, kpad, cls, T, TW, NT);
+}
+
+// The same with the rotation of the self pathway's Q and K, by further CTAs of the launch: what an attention call on chain ids and raw
+// projections has to have done before it starts.  For short pairs, where a launch is what either costs (B1 H20 T187 D16: 18.6 us a call with
+// two, 14.7 with one).
+template <typename Id>
+__global__ void __launch_bounds__(256) prepare_kernel(const Id* __restrict__ chain_ids, const uint8_t* __restrict__ key_pad, uint32_t* __restrict__ bits,
+                                                      uint32_t* __restrict__ bitsT, uint32_t* __restrict__ kpad, uint8_t* __restrict__ cls, int B, int T, int TW, int NT,
+                                                      const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k, __nv_bfloat16* __restrict__ qr,
+                                                      __nv_bfloat16* __restrict__ kr, const float* __restrict__ cos_tab, const float* __restrict__ sin_tab, size_t rows, int D) {
+  ptx::griddep_wait();
+  ptx::griddep_launch();
+  const unsigned n = unsigned(B) * NT;
+  if (blockIdx.x < n) meta_rows(int(blockIdx.x) % B, int(blockIdx.x) / B, chain_ids, key_pad, bits, bitsT, kpad, cls, T, TW, NT);
+  else rope_rotate_part(size_t(blockIdx.x - n) * blockDim.x + threadIdx.x, q, k, qr, kr, cos_tab, sin_tab, rows, T, D);
 }
 
 // Arbitrary (B,T,T) mask: row-major words, and the transposed relation for the key-major copy.
@@ -159,6 +181,25 @@ cudaError_t launch_meta_from_chain_ids(const void* chain_ids, bool ids64, const 
     meta_from_chain_ids_kernel<int32_t><<<grid, 256, 0, s>>>(static_cast<const int32_t*>(chain_ids), key_pad, bits, bitsT, kpad, cls, T, L.TW, L.NT);
   count_launches(1);
   return cudaGetLastError();
+}
+
+cudaError_t launch_prepare(const AttnArgs& a, __nv_bfloat16* qr, __nv_bfloat16* kr) {
+  const MetaLayout L = meta_layout(a.B, a.T);
+  char* p = static_cast<char*>(a.meta_buf);
+  uint32_t* bits = reinterpret_cast<uint32_t*>(p + L.off_bits);
+  uint32_t* bitsT = reinterpret_cast<uint32_t*>(p + L.off_bitsT);
+  uint32_t* kpad = reinterpret_cast<uint32_t*>(p + L.off_kpad);
+  uint8_t* cls = reinterpret_cast<uint8_t*>(p + L.off_cls);
+  const size_t rows = size_t(a.B) * a.H * a.T, parts = rows * (a.D / 16);
+  const dim3 grid(unsigned(a.B) * L.NT + unsigned((parts + 255) / 256));
+  auto launch = [&](auto kern, auto ids) {
+    return launch_dependent(kern, grid, dim3(256), 0, a.stream, ids, a.key_pad, bits, bitsT, kpad, cls, a.B, a.T, L.TW, L.NT, static_cast<const __nv_bfloat16*>(a.q_s),
+                            static_cast<const __nv_bfloat16*>(a.k_s), qr, kr, a.rope_cos, a.rope_sin, rows, a.D);
+  };
+  const cudaError_t e = a.ids64 ? launch(prepare_kernel<long long>, static_cast<const long long*>(a.chain_ids))
+                                : launch(prepare_kernel<int32_t>, static_cast<const int32_t*>(a.chain_ids));
+  count_launches(1);
+  return e == cudaSuccess ? cudaGetLastError() : e;
 }
 
 cudaError_t launch_meta_from_mask(const uint8_t* mask, const uint8_t* key_pad, void* meta, int B, int T,

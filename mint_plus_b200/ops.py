@@ -304,14 +304,19 @@ def multimer_attention(q_self, k_self, v_self, q_cross, k_cross, v_cross, *, met
     if q_self.dim() != 4:
         raise ValueError("q/k/v of both pathways must share one (B, H, T, D) shape")
     B, H, T, D = q_self.shape
-    if meta is None:
+    # chain ids of these very rows: metadata and rotation in one launch (below)
+    together = (meta is None and chain_mask is None and chain_ids is not None and rope and grad_rowmajor_tabs is None
+                and chain_ids.shape == (B, T) and chain_ids.device == q_self.device)
+    if together:
+        pass
+    elif meta is None:
         if (chain_ids is None) == (chain_mask is None):
             raise ValueError("give exactly one of meta, chain_ids, chain_mask")
         meta = mask_meta_from_chain_ids(chain_ids, key_padding_mask) if chain_ids is not None \
             else cached_mask_meta(chain_mask, key_padding_mask)
     elif chain_ids is not None or chain_mask is not None or key_padding_mask is not None:
         raise ValueError("meta already carries the chain and padding masks")
-    if meta.B != B or meta.T != T:
+    if not together and (meta.B != B or meta.T != T):
         raise ValueError(f"mask metadata is for (B, T) = ({meta.B}, {meta.T}), tensors have ({B}, {T})")
     flags = ((L.FLAG_ROPE if rope else 0) | (L.FLAG_SQRT_SOFTMAX if sqrt_softmax else 0) | (L.FLAG_FORCE_SIMT if force_simt else 0)
              | (L.FLAG_OUT_SEQ_FIRST if out_seq_first else 0) | (L.FLAG_SKIP_PAD_QUERIES if skip_pad_queries else 0))
@@ -325,6 +330,8 @@ def multimer_attention(q_self, k_self, v_self, q_cross, k_cross, v_cross, *, met
         if any(t.shape != q_self.shape for t in ts):
             raise ValueError("q/k/v of both pathways must share one (B, H, T, D) shape")
         return _MultimerAttentionFn.apply(*(t.contiguous() for t in ts), meta, cos, sin, float(scale), int(flags), grad_rowmajor_tabs)
+    if together:
+        return L.host().attention_ids(*ts, chain_ids, key_padding_mask, cos, sin, scale, flags)
     return L.host().attention(*ts, meta.buf, cos, sin, scale, flags)
 
 
