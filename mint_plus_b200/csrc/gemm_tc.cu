@@ -150,10 +150,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   const int n_slabs = (p.K + elems_per_slab - 1) / elems_per_slab;
 
   // With few rows the weights come from HBM and are used once: they are on their way to L2 while the kernel before this one still runs.
-  // (A prefetch delivers nothing: what that kernel writes is read behind the wait below, weights included.)
+  // (A prefetch delivers nothing: what that kernel writes is read behind the wait below, weights included.)  Two rings' worth: all slabs
+  // of a long reduction hold up the loads behind them (36 x 2560 model, 12 layers, one pair of T128: 1777 us without, 1843 with all, 1771
+  // so; T700 2590, 2660, 2576; FP8 650M model T497 2366, 2346, 2336).
   if (warp == 0 && lane == 0 && tiles_m <= kPrefetchRows && int(blockIdx.x) < tiles_n * (PAIR ? 2 : 1)) {
     const int n0 = int(blockIdx.x) / (PAIR ? 2 : 1) * kGN + rank * Cfg::kBRows;
-    for (int kb = 0; kb < n_slabs; ++kb) tma_prefetch_2d(&map_b, kb * elems_per_slab, n0);
+    for (int kb = 0; kb < min(n_slabs, 2 * kGStages); ++kb) tma_prefetch_2d(&map_b, kb * elems_per_slab, n0);
   }
   if (tid == 0) {
     for (int s = 0; s < kGStages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
