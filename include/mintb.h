@@ -121,6 +121,13 @@ MINTB_API int mintb_attn_fwd(const void* q_self, const void* k_self, const void*
                    const float* rope_sin, void* out, float* lse, void* workspace, size_t workspace_bytes, int B,
                    int H, int T, int D, int dtype, unsigned flags, float scale, void* stream, int* dev_status);
 
+/* mintb_attn_fwd of bf16 tensors that leaves `out` a second time in out_e4m3, as sat(out * inv_scale) of the rounded values: the 8-bit
+ * operand of the output projection. */
+MINTB_API int mintb_attn_fwd_e4m3(const void* q_self, const void* k_self, const void* v_self, const void* q_cross, const void* k_cross,
+                                  const void* v_cross, const void* meta, const float* rope_cos, const float* rope_sin, void* out, float* lse,
+                                  void* workspace, size_t workspace_bytes, int B, int H, int T, int D, unsigned flags, float scale,
+                                  void* out_e4m3, float inv_scale, void* stream, int* dev_status);
+
 /* mintb_mask_meta_from_chain_ids (`ids64`: 64-bit ids) into `meta`, then mintb_attn_fwd on it; with in-kernel RoPE on the bf16 kernels the
  * metadata and the rotated copies are formed by one launch. */
 MINTB_API int mintb_attn_fwd_ids(const void* chain_ids, int ids64, const uint8_t* key_pad, void* meta, const void* q_self, const void* k_self,

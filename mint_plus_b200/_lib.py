@@ -33,6 +33,7 @@ PROTOTYPES = {
     "mintb_attn_fwd_workspace_bytes": (c_size_t, [c_int, c_int, c_int, c_int, c_int, c_uint]),
     "mintb_attn_fwd": (c_int, [_P] * 6 + [_P, _P, _P, _P, _P, _P, c_size_t, c_int, c_int, c_int, c_int, c_int, c_uint,
                                c_float, _P, _P]),
+    "mintb_attn_fwd_e4m3": (c_int, [_P] * 6 + [_P, _P, _P, _P, _P, _P, c_size_t, c_int, c_int, c_int, c_int, c_uint, c_float, _P, c_float, _P, _P]),
     "mintb_attn_fwd_ids": (c_int, [_P, c_int, _P, _P] + [_P] * 6 + [_P, _P, _P, _P, _P, c_size_t, c_int, c_int, c_int, c_int, c_int, c_uint, c_float, _P, _P]),
     "mintb_attn_fwd_static": (c_int, [_P] * 6 + [_P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_uint, c_float, _P,
                                       _P]),

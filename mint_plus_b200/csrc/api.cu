@@ -281,10 +281,9 @@ int check_attn_args(AttnArgs& a, const char* who, const void* q_s, const void* k
 
 extern "C" {
 
-int mintb_attn_fwd(const void* q_self, const void* k_self, const void* v_self, const void* q_cross,
-                   const void* k_cross, const void* v_cross, const void* meta, const float* rope_cos,
-                   const float* rope_sin, void* out, float* lse, void* workspace, size_t workspace_bytes, int B,
-                   int H, int T, int D, int dtype, unsigned flags, float scale, void* stream, int* dev_status) {
+static int attn_fwd_any(const void* q_self, const void* k_self, const void* v_self, const void* q_cross, const void* k_cross, const void* v_cross,
+                        const void* meta, const float* rope_cos, const float* rope_sin, void* out, float* lse, void* workspace, size_t workspace_bytes,
+                        int B, int H, int T, int D, int dtype, unsigned flags, float scale, void* out_e4m3, float inv_scale, void* stream, int* dev_status) {
   AttnArgs a{};
   size_t need = mintb_attn_fwd_workspace_bytes(B, H, T, D, dtype, flags);
   int rc = fill_common(a, "mintb_attn_fwd", q_self, k_self, v_self, q_cross, k_cross, v_cross, meta, rope_cos,
@@ -296,9 +295,34 @@ int mintb_attn_fwd(const void* q_self, const void* k_self, const void* v_self, c
   }
   a.out = out;
   a.lse = lse;
+  a.out_e4m3 = out_e4m3;
+  a.out_e4m3_inv = inv_scale;
   if (use_tc(D, dtype, flags)) return launch_attn_fwd_tc(a);
   cudaError_t e = launch_attn_fwd_simt(a);
   return e == cudaSuccess ? MINTB_OK : cuda_fail(e, "attention forward launch");
+}
+
+int mintb_attn_fwd(const void* q_self, const void* k_self, const void* v_self, const void* q_cross,
+                   const void* k_cross, const void* v_cross, const void* meta, const float* rope_cos,
+                   const float* rope_sin, void* out, float* lse, void* workspace, size_t workspace_bytes, int B,
+                   int H, int T, int D, int dtype, unsigned flags, float scale, void* stream, int* dev_status) {
+  return attn_fwd_any(q_self, k_self, v_self, q_cross, k_cross, v_cross, meta, rope_cos, rope_sin, out, lse, workspace, workspace_bytes, B, H, T, D, dtype, flags, scale,
+                      nullptr, 0.f, stream, dev_status);
+}
+
+int mintb_attn_fwd_e4m3(const void* q_self, const void* k_self, const void* v_self, const void* q_cross, const void* k_cross, const void* v_cross, const void* meta,
+                        const float* rope_cos, const float* rope_sin, void* out, float* lse, void* workspace, size_t workspace_bytes, int B, int H, int T, int D,
+                        unsigned flags, float scale, void* out_e4m3, float inv_scale, void* stream, int* dev_status) {
+  if (out_e4m3 == nullptr || !aligned(out_e4m3, 16)) {
+    set_error("mintb_attn_fwd_e4m3: out_e4m3 (16-byte aligned) is required");
+    return MINTB_EINVAL;
+  }
+  if (!use_tc(D, MINTB_BF16, flags)) {
+    set_error("mintb_attn_fwd_e4m3: the bf16 tensor-core kernels only (head size 16, 32 or 64)");
+    return MINTB_EUNSUPPORTED;
+  }
+  return attn_fwd_any(q_self, k_self, v_self, q_cross, k_cross, v_cross, meta, rope_cos, rope_sin, out, lse, workspace, workspace_bytes, B, H, T, D, MINTB_BF16, flags, scale,
+                      out_e4m3, inv_scale, stream, dev_status);
 }
 
 int mintb_attn_fwd_ids(const void* chain_ids, int ids64, const uint8_t* key_pad, void* meta, const void* q_self, const void* k_self, const void* v_self,

@@ -11,6 +11,8 @@
 // S is released as soon as the softmax threads have read it, so the next Q K^T overlaps this entry's exponentials;
 // a mixed entry holds the self logits in the low half of S and the cross logits in the high half.
 // Every wait on an mbarrier is bounded; on expiry the role records a code in *dev_status and unwinds.
+#include <cuda_fp8.h>
+
 #include <algorithm>
 #include <mutex>
 
@@ -122,6 +124,16 @@ struct FwdCfg {
   static constexpr size_t kSmemBytes = 1024 /*align slack*/ + 2 * kQBytes + size_t(kStages) * kStageBytes + 8192 /*tail: barriers, items, statistics, two entry lists*/;
 };
 
+// eight bf16 numbers, times inv, as e4m3: saturated, NaN stays NaN
+__device__ __forceinline__ uint2 e4m3_of_bf16(uint4 w, float inv) {
+  const uint32_t in[4] = {w.x, w.y, w.z, w.w};
+  uint32_t h[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    h[j] = __nv_cvt_float2_to_fp8x2(make_float2(__uint_as_float(in[j] << 16) * inv, __uint_as_float(in[j] & 0xffff0000u) * inv), __NV_SATFINITE, __NV_E4M3);
+  return make_uint2(h[0] | h[1] << 16, h[2] | h[3] << 16);
+}
+
 struct FwdParams {
   const uint32_t *bits, *kpad;
   const uint8_t* cls;
@@ -134,6 +146,8 @@ struct FwdParams {
   int skip_pad_queries;                   // leave out query tiles that hold only padded positions
   int* sched;                             // work counter pair of this launch (common.cuh)
   int NQ, n_items;                        // query tiles per (batch, head); items = NQ * B * H
+  unsigned char* out8;                    // `out` once more in e4m3, sat(out * out8_inv), in the same layout; may be null
+  float out8_inv;
   int BH, group;                          // (batch, head) pairs; how many of them take their query tiles in turn (see attn_fwd_tc_kernel)
 };
 
@@ -712,7 +726,10 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
           if (qi < p.T) {   // no unpadded key at all: NaN, as the softmax of an all -inf row gives in the PyTorch path
             const uint32_t nan2 = 0x7FC07FC0u;
 #pragma unroll
-            for (int d = 0; d < NC; d += 8) *reinterpret_cast<uint4*>(orow + d) = make_uint4(nan2, nan2, nan2, nan2);
+            for (int d = 0; d < NC; d += 8) {
+              *reinterpret_cast<uint4*>(orow + d) = make_uint4(nan2, nan2, nan2, nan2);
+              if (p.out8 != nullptr) *reinterpret_cast<uint2*>(p.out8 + (orow - p.out) + d) = make_uint2(0x7F7F7F7Fu, 0x7F7F7F7Fu);
+            }
             if (ch == 0) p.lse[size_t(bh) * p.T + qi] = -INFINITY;
           }
         } else {
@@ -726,6 +743,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
           const float f_other = (SQ ? ex2(0.5f * (m_other - m_all)) : w_other) * inv;
           // A short loop: code that runs once per item has to be fetched anew each time, at some 100 cycles for eight instructions.
           constexpr int CH = 8;
+          uint2 q_low = make_uint2(0, 0);
 #pragma unroll 1
           for (int c0 = 0; c0 < NC; c0 += CH) {
             uint32_t oa[CH], ob[CH];
@@ -742,9 +760,17 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_cons
                 v[j] = a + bb;
               }
 #pragma unroll
-              for (int j = 0; j < CH; j += 8)
-                *reinterpret_cast<uint4*>(orow + c0 + j) = make_uint4(pack_bf16(v[j], v[j + 1]), pack_bf16(v[j + 2], v[j + 3]),
-                                                                      pack_bf16(v[j + 4], v[j + 5]), pack_bf16(v[j + 6], v[j + 7]));
+              for (int j = 0; j < CH; j += 8) {
+                const uint4 w = make_uint4(pack_bf16(v[j], v[j + 1]), pack_bf16(v[j + 2], v[j + 3]), pack_bf16(v[j + 4], v[j + 5]), pack_bf16(v[j + 6], v[j + 7]));
+                *reinterpret_cast<uint4*>(orow + c0 + j) = w;
+                if (p.out8 != nullptr) {   // the 8-bit operand of the output projection, from the rounded values, sixteen at a time where there are as many
+                  const uint2 q = e4m3_of_bf16(w, p.out8_inv);
+                  unsigned char* at = p.out8 + (orow - p.out) + c0;
+                  if (NC == 8) *reinterpret_cast<uint2*>(at) = q;
+                  else if (c0 & 8) *reinterpret_cast<uint4*>(at - 8) = make_uint4(q_low.x, q_low.y, q.x, q.y);
+                  q_low = q;
+                }
+              }
             }
           }
           if (qi < p.T) {
@@ -801,7 +827,7 @@ static int fwd_tc_t(const AttnArgs& a, const void* q_s, const void* k_s) {
   const int group = (BH + n_groups - 1) / n_groups;   // of like size: the end is sorted within the last group only
   FwdParams p{a.meta.bits, a.meta.kpad, a.meta.cls, static_cast<__nv_bfloat16*>(a.out), a.lse, a.H, a.T, a.meta.TW, a.meta.NT,
               a.scale * kLog2e, a.dev_status, out_row_stride(a), out_bh_stride(a), a.skip_pad_queries ? 1 : 0,
-              sched, NQ, int(n_items), BH, group};
+              sched, NQ, int(n_items), static_cast<unsigned char*>(a.out_e4m3), a.out_e4m3_inv, BH, group};
   const int n_ctas = 2 * sm_count();   // two persistent CTAs per SM
   const unsigned grid = unsigned(n_items < n_ctas ? n_items : n_ctas);
   cudaError_t e = launch_dependent(attn_fwd_tc_kernel<D, SQ>, dim3(grid), dim3(kTcThreads), Cfg::kSmemBytes, a.stream, mqs, mks, mvs, mqc, mkc, mvc, p);

@@ -89,6 +89,8 @@ struct AttnArgs {
   bool ids64;
   const uint8_t* key_pad;
   void* meta_buf;                    // ... here
+  void* out_e4m3;                    // forward: `out` once more in e4m3, sat(out * out_e4m3_inv) (null: not wanted)
+  float out_e4m3_inv;
 };
 
 // element strides of out / d_out: row (query) stride and (batch, head) stride

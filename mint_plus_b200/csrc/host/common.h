@@ -97,9 +97,10 @@ struct AttnInputs {   // (B,H,T,D) projections and what goes with them
 };
 struct AttnResult {
   Tensor out, lse;
+  Tensor q8;          // `out` in e4m3, where asked for
   Tensor ws;          // workspace holding the rotated copies the backward pass starts from, where asked for
 };
-AttnResult attn_fwd(const AttnInputs& a, bool for_backward);
+AttnResult attn_fwd(const AttnInputs& a, bool for_backward, double q8_scale = 0.0);   // q8_scale > 0 (bf16): with the e4m3 copy
 
 struct Product {      // y = act(alpha x w^T + bias) and its variants
   Tensor x, w, bias;

@@ -26,7 +26,7 @@ int* Env::status_ptr(int device) {
   return p;
 }
 
-AttnResult attn_fwd(const AttnInputs& a, bool for_backward) {
+AttnResult attn_fwd(const AttnInputs& a, bool for_backward, double q8_scale) {
   const Tensor& q = a.q[0];
   const int64_t B = q.size(0), H = q.size(1), T = q.size(2), D = q.size(3);
   const int dt = dt_code(q.scalar_type(), "q");
@@ -45,7 +45,12 @@ AttnResult attn_fwd(const AttnInputs& a, bool for_backward) {
                              ptr(a.q[3]), ptr(a.q[4]), ptr(a.q[5]), fptr(a.cos), fptr(a.sin), ptr(r.out), fptr(r.lse), ptr(ws), bytes, B, H, T, D, dt, a.flags,
                              float(a.scale), e.stream, e.status),
           "mintb_attn_fwd");
-  else
+  else if (q8_scale > 0) {
+    r.q8 = e.empty(r.out.sizes(), at::kFloat8_e4m3fn);
+    check(mintb_attn_fwd_e4m3(ptr(a.q[0]), ptr(a.q[1]), ptr(a.q[2]), ptr(a.q[3]), ptr(a.q[4]), ptr(a.q[5]), ptr(a.meta), fptr(a.cos), fptr(a.sin), ptr(r.out),
+                              fptr(r.lse), ptr(ws), bytes, B, H, T, D, a.flags, float(a.scale), ptr(r.q8), float(1.0 / q8_scale), e.stream, e.status),
+          "mintb_attn_fwd_e4m3");
+  } else
     check(mintb_attn_fwd(ptr(a.q[0]), ptr(a.q[1]), ptr(a.q[2]), ptr(a.q[3]), ptr(a.q[4]), ptr(a.q[5]), ptr(a.meta), fptr(a.cos), fptr(a.sin), ptr(r.out),
                          fptr(r.lse), ptr(ws), bytes, B, H, T, D, dt, a.flags, float(a.scale), e.stream, e.status),
           "mintb_attn_fwd");

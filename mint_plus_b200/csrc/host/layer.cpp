@@ -142,6 +142,8 @@ std::tuple<Tensor, OptTensor> LayerPlan::forward(const Tensor& x, const OptTenso
   return run(x, xq, batch, next_quant);
 }
 
+constexpr int64_t kFewPositions = 4096;
+
 std::tuple<Tensor, OptTensor> LayerPlan::run(const Tensor& x_in, const OptTensor& xq_in, const Batch& batch, double next_quant) const {
   const Where at(*this);
   std::vector<Tensor> inputs;
@@ -215,13 +217,17 @@ std::tuple<Tensor, OptTensor> LayerPlan::run(const Tensor& x_in, const OptTensor
     a.meta = batch.meta;
     a.scale = scale;
     a.flags = MINTB_FLAG_OUT_SEQ_FIRST | (sqrt_softmax ? MINTB_FLAG_SQRT_SOFTMAX : 0) | (packed ? MINTB_FLAG_SKIP_PAD_QUERIES : 0);
-    AttnResult attn = attn_fwd(a, false);
-    Tensor o = attn.out.view({T * B, E});
+    // The output projection's 8-bit operand: of few positions from the attention kernel itself, one launch less (33 muS layers at E 1280,
+    // 128 tokens 2047 -> 2006 us, 497 2329 -> 2295, 1988 3775 -> 3752, 3976 6299 -> 6277, but 7952 10910 -> 10954); of many by a pass, because
+    // the epilogue's scattered stores cost as much (32768 tokens: 18 us of the pass's 22).
+    const bool q8 = fp8 && T * B <= kFewPositions;
+    AttnResult attn = attn_fwd(a, false, q8 ? out.x_scale : 0.0);
+    Tensor o = (q8 ? attn.q8.view(at::kByte) : attn.out).view({T * B, E});
     if (packed) o = o.index_select(0, batch.rows64);
 
     // output projection with the residual sum in its epilogue
     Product po;
-    po.x = fp8 ? quantize(o, out.x_scale) : o;
+    po.x = q8 ? o.view(at::kFloat8_e4m3fn) : fp8 ? quantize(o, out.x_scale) : o;
     po.w = out_op; po.bias = params[at.bo]; po.alpha = out.alpha();
     auto [x1, x1q] = linear_res_fwd(po, x, keep, add, fp8 && mu ? fc1.x_scale : 0.0, lora_r > 0);
 
